@@ -115,7 +115,7 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
 // leave the decode-regime kernels for the tcgen05 kernel (tris_set_grouped_tc_min_rows).
 int grouped_tc_min_rows();
 int route_rows_hint(const TrisRouteView* route);
-int launch_tiled_dump(const TrisProjView* proj, int32_t* dense_out, void* weights_out, cudaStream_t stream);
+int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t stream);
 int combine_routed_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,
                         int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream, bool pdl);
 int launch_router_route(const float* logits, int num_tokens, int num_experts, int top_k, int norm, int m_tile,
@@ -141,6 +141,16 @@ __device__ __forceinline__ void mma_m16n8k16(float (&c)[4], uint32_t a0, uint32_
       "{%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// One lane's value for the whole warp, in a form the compiler knows to be uniform.  The operands of a
+// tcgen05.mma live in uniform registers: with operands it cannot prove uniform it spends some thirty
+// instructions per MMA on moving them there.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
 // Programmatic dependent launch: wait for the producer grid's memory to be visible /
@@ -184,6 +194,16 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// The same, returning whether `pred` held on any of the threads.
+__device__ __forceinline__ bool named_barrier_or(int id, int nthreads, bool pred) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(id), "r"(nthreads), "r"(static_cast<int>(pred))
+      : "memory");
+  return any != 0;
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -223,6 +243,38 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
       if (mbar_try_wait(bar, parity)) return true;
     if (global_timer_ns() - t0 > 1000000000ull) return false;
   }
+}
+
+__device__ __forceinline__ uint32_t global_timer_lo() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+  return t;
+}
+// The same in few instructions and registers (~1 s as well).
+__device__ __forceinline__ bool mbar_wait_lean(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint32_t t0 = global_timer_lo();
+#pragma unroll 1
+  do {
+    if (mbar_try_wait(bar, parity)) return true;
+  } while (global_timer_lo() - t0 < 1000000000u);
+  return false;
+}
+// The same by a whole warp, with one answer for all lanes (collective instructions may follow).
+// kSleepNs > 0: naps between polls, for a role that waits long and must not take issue slots from the
+// roles it waits for.
+template <int kSleepNs = 0>
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+  const uint32_t t0 = global_timer_lo();
+  bool in_time;
+#pragma unroll 1
+  do {
+    if (kSleepNs > 0) __nanosleep(kSleepNs);
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    in_time = __all_sync(0xFFFFFFFFu, global_timer_lo() - t0 < 1000000000u);
+  } while (in_time);
+  return false;
 }
 
 }  // namespace tris

@@ -496,17 +496,6 @@ static int pick_ksplit(const TrisProjView* proj, const TrisRouteView* route, int
   return 1;
 }
 
-// Rows per segment (the launch's estimate) up to which the tile-record kernel is used.  It multiplies
-// 32 rows per pass and re-unpacks the weights for every pass; from ~64 rows per segment on, the
-// plane-staging kernel (64 rows per pass) and, beyond grouped_tc_min_rows(), the tcgen05 kernel do
-// less work per row.
-static int tiled_max_rows() { return std::min(64, grouped_tc_min_rows()); }
-// Above that, up to the tcgen05 threshold, the tile-record kernel that keeps a chunk's unpacked weights in
-// registers across row passes takes single-chunk projections (rank <= 256).
-static bool tiled_takes(const TrisProjView& v, int rows) {
-  return rows <= tiled_max_rows() || (v.rank <= 256 && rows <= grouped_tc_min_rows());
-}
-
 // Rows per activation tile: sized for the typical segment (mean + 4 sigma of a balanced
 // router), never above the caller's bound; longer segments take several passes.
 static int rows_hint(const TrisRouteView* route) { return route_rows_hint(route); }
@@ -563,7 +552,6 @@ extern "C" int tris_block_gr_decode(const TrisProjView* proj, int32_t* dense_out
   int st = validate_proj(proj, "tris_block_gr_decode", true);
   if (st != TRIS_OK) return st;
   TRIS_REQUIRE(proj->use_block_gr && dense_out, TRIS_ERR_INVALID_ARG, "tris_block_gr_decode: needs a block-GR payload and an output");
-  if (proj_has_tile_records(*proj)) return launch_tiled_dump(proj, dense_out, nullptr, static_cast<cudaStream_t>(stream));
   const int pr = (proj->rank + 31) / 32;
   dim3 grid(ceil_div(proj->out_features, 128), ceil_div(pr, KC), proj->num_experts);
   const size_t smem = sizeof(TileSmem<1, 1>);
@@ -576,7 +564,7 @@ extern "C" int tris_compact3_dequantize(const TrisProjView* proj, void* weights_
   int st = validate_proj(proj, "tris_compact3_dequantize", true);
   if (st != TRIS_OK) return st;
   TRIS_REQUIRE(weights_out_f16, TRIS_ERR_INVALID_ARG, "tris_compact3_dequantize: null output");
-  if (proj_has_tile_records(*proj)) return launch_tiled_dump(proj, nullptr, weights_out_f16, static_cast<cudaStream_t>(stream));
+  if (proj_has_tile_records(*proj)) return launch_tiled_dump(proj, weights_out_f16, static_cast<cudaStream_t>(stream));
   const int pr = (proj->rank + 31) / 32;
   dim3 grid(ceil_div(proj->out_features, 128), ceil_div(pr, KC), proj->num_experts);
   const size_t smem = sizeof(TileSmem<1, 1>);
@@ -584,20 +572,6 @@ extern "C" int tris_compact3_dequantize(const TrisProjView* proj, void* weights_
   compact3_dump_kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
       *proj, nullptr, static_cast<__half*>(weights_out_f16), nullptr);
   return check_cuda(cudaGetLastError(), "compact3_dump_kernel launch");
-}
-
-// Tile-record form of the tcgen05 kernel: lane-order activation rows, single-chunk projections, segments
-// above the tensor-core threshold.
-static bool umma_records_applicable(const TrisProjView& v, const GroupedArgs& a, bool lane_order, int rows) {
-  const int stride = a.hidden_stride > 0 ? a.hidden_stride : v.rank;
-  return lane_order && rows > grouped_tc_min_rows() && v.rank % 32 == 0 && v.rank <= 256 && stride % 8 == 0 && stride >= v.rank;
-}
-static void fill_record_slots(GroupedArgs& a) {
-  const int rec = std::max(a.proj[0].max_record_bytes, a.proj[1].max_record_bytes);
-  a.rec_slot_bytes = ((rec + 15) & ~15) + 16;
-  a.col_slot_bytes = std::max(a.proj[0].col_record_bytes, a.proj[1].col_record_bytes);
-  a.hidden_lane_order = 1;
-  a.ksplit = 1;
 }
 
 int tris::grouped_forward_impl(const TrisProjView* proj, const TrisRouteView* route, const void* hidden_f16,
@@ -610,22 +584,12 @@ int tris::grouped_forward_impl(const TrisProjView* proj, const TrisRouteView* ro
   if (st != TRIS_OK) return st;
   if (a.num_segments == 0 || a.num_rows == 0) return TRIS_OK;
   const bool lane_order = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER) != 0;
-  TRIS_REQUIRE(!lane_order || (proj_has_tile_records(*proj) && !a.hidden_interleaved), TRIS_ERR_INVALID_ARG,
-               "tris_grouped_forward: lane-order activations need a projection with tile records");
-  const bool col_scaled = route->hidden_col_scale != nullptr;
-  TRIS_REQUIRE(!col_scaled || (proj_has_tile_records(*proj) && !a.hidden_interleaved && !lane_order), TRIS_ERR_UNSUPPORTED,
-               "tris_grouped_forward: hidden_col_scale needs tile records and row-major activations");
-  if (proj_has_tile_records(*proj) && !a.hidden_interleaved && umma_records_applicable(*proj, a, lane_order, rows_hint(route))) {
-    if (a.hidden_stride <= 0) a.hidden_stride = proj->rank;
-    a.proj[0] = a.proj[1] = *proj;
-    a.hidden[0] = a.hidden[1] = static_cast<const __half*>(hidden_f16);
-    a.out[0] = a.out[1] = static_cast<__half*>(out_f16);
-    a.weights_before_wait = opts.pdl && opts.weights_before_wait;
-    fill_record_slots(a);
-    return launch_grouped_umma(a, 1, EPI_STORE, stream, opts.pdl);
-  }
-  if (proj_has_tile_records(*proj) && !a.hidden_interleaved && (lane_order || col_scaled || tiled_takes(*proj, rows_hint(route))))
+  TRIS_REQUIRE(!(lane_order && a.hidden_interleaved), TRIS_ERR_INVALID_ARG, "tris_grouped_forward: two column orders named");
+  if (proj_has_tile_records(*proj))
     return launch_grouped_tiled(proj, nullptr, route, hidden_f16, nullptr, out_f16, nullptr, 0, rows_hint(route), stream, opts);
+  TRIS_REQUIRE(!lane_order, TRIS_ERR_INVALID_ARG, "tris_grouped_forward: lane-order activations need a projection with tile records");
+  TRIS_REQUIRE(route->hidden_col_scale == nullptr, TRIS_ERR_UNSUPPORTED,
+               "tris_grouped_forward: hidden_col_scale needs tile records and row-major activations");
   TRIS_REQUIRE(!a.hidden_interleaved || proj->rank % 32 == 0, TRIS_ERR_INVALID_ARG,
                "tris_grouped_forward: pair-interleaved activations need rank % 32 == 0");
   if (a.hidden_stride <= 0) a.hidden_stride = proj->rank;
@@ -644,16 +608,11 @@ int tris::grouped_forward_impl(const TrisProjView* proj, const TrisRouteView* ro
 
 extern "C" int tris_grouped_hidden_layout(const TrisProjView* proj_a, const TrisProjView* proj_b, int32_t num_rows,
                                           int32_t num_segments, int32_t max_rows_per_segment) {
+  (void)num_rows, (void)num_segments, (void)max_rows_per_segment;
   if (proj_a == nullptr || proj_a->rank % 32 != 0) return TRIS_OUT_F16;
-  TrisRouteView route{};
-  route.num_rows = num_rows;
-  route.num_segments = num_segments;
-  route.max_rows_per_segment = max_rows_per_segment;
+  // the tile-record kernels read rows as they are, the plane-staging kernels pair-interleaved ones
   const bool records = proj_has_tile_records(*proj_a) && (proj_b == nullptr || proj_has_tile_records(*proj_b));
-  // single-chunk projections with records read lane order at every size (decode kernels, the register-cached
-  // kernel, the tile-record form of the tcgen05 kernel); larger ranks only where the decode kernels take them
-  return (records && (proj_a->rank <= 256 || tiled_takes(*proj_a, route_rows_hint(&route)))) ? TRIS_OUT_F16_LANE_ORDER
-                                                                                             : TRIS_OUT_F16_PAIR_INTERLEAVED;
+  return records ? TRIS_OUT_F16 : TRIS_OUT_F16_PAIR_INTERLEAVED;
 }
 
 extern "C" int tris_grouped_forward(const TrisProjView* proj, const TrisRouteView* route, const void* hidden_f16,
@@ -684,27 +643,13 @@ int tris::grouped_pair_forward_impl(const TrisProjView* proj_a, const TrisProjVi
   if (st != TRIS_OK) return st;
   if (a.num_segments == 0 || a.num_rows == 0) return TRIS_OK;
   const bool lane_order = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER) != 0;
-  const bool records = proj_has_tile_records(*proj_a) && proj_has_tile_records(*proj_b);
-  TRIS_REQUIRE(!lane_order || (records && !a.hidden_interleaved), TRIS_ERR_INVALID_ARG,
-               "tris_grouped_pair_forward: lane-order activations need projections with tile records");
-  const bool col_scaled = route->hidden_col_scale != nullptr;
-  TRIS_REQUIRE(!col_scaled || (records && !a.hidden_interleaved && !lane_order), TRIS_ERR_UNSUPPORTED,
-               "tris_grouped_pair_forward: hidden_col_scale needs tile records and row-major activations");
-  if (records && !a.hidden_interleaved && umma_records_applicable(*proj_a, a, lane_order, rows_hint(route))) {
-    if (a.hidden_stride <= 0) a.hidden_stride = proj_a->rank;
-    a.proj[0] = *proj_a;
-    a.proj[1] = *proj_b;
-    a.hidden[0] = static_cast<const __half*>(hidden_a_f16);
-    a.hidden[1] = static_cast<const __half*>(hidden_b_f16);
-    a.out[0] = static_cast<__half*>(out_a_f16);
-    a.out[1] = static_cast<__half*>(out_b_f16);
-    a.weights_before_wait = opts.pdl && opts.weights_before_wait;
-    fill_record_slots(a);
-    return launch_grouped_umma(a, 2, fuse_silu_mul ? EPI_SILU_MUL : EPI_STORE, stream, opts.pdl);
-  }
-  if (records && !a.hidden_interleaved && (lane_order || col_scaled || tiled_takes(*proj_a, rows_hint(route))))
+  TRIS_REQUIRE(!(lane_order && a.hidden_interleaved), TRIS_ERR_INVALID_ARG, "tris_grouped_pair_forward: two column orders named");
+  if (proj_has_tile_records(*proj_a) && proj_has_tile_records(*proj_b))
     return launch_grouped_tiled(proj_a, proj_b, route, hidden_a_f16, hidden_b_f16, out_a_f16, out_b_f16, fuse_silu_mul ? 2 : 1,
                                 rows_hint(route), stream, opts);
+  TRIS_REQUIRE(!lane_order, TRIS_ERR_INVALID_ARG, "tris_grouped_pair_forward: lane-order activations need projections with tile records");
+  TRIS_REQUIRE(route->hidden_col_scale == nullptr, TRIS_ERR_UNSUPPORTED,
+               "tris_grouped_pair_forward: hidden_col_scale needs tile records and row-major activations");
   TRIS_REQUIRE(!a.hidden_interleaved || proj_a->rank % 32 == 0, TRIS_ERR_INVALID_ARG,
                "tris_grouped_pair_forward: pair-interleaved activations need rank % 32 == 0");
   if (a.hidden_stride <= 0) a.hidden_stride = proj_a->rank;

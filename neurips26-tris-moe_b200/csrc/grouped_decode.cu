@@ -1,0 +1,411 @@
+// Grouped compact3 dequant-matmul over tile records for segments of few rows (decode), on mma.sync.
+//
+// A warp owns 32 outputs of one projection and multiplies them with up to 8 NT activation rows.  Lane
+// (g, t) takes code word t of output rows g, g + 8, g + 16, g + 24: 16 columns of each of a 64-column slice,
+// loaded coalesced (128 bytes per load) and straight from the record, since they are used once.  Unpacked,
+// they are the lane's A fragments of four m16n8k16 steps if step j's K positions are columns
+// 16t + 4j .. + 3, which the B side follows: a lane's activations of a slice are 32 contiguous bytes.  No
+// weight passes through shared memory or TMEM, and the warps of a CTA meet only where activation rows
+// are staged and where gate meets up.
+// tcgen05 tiles have 128 outputs and take their A from TMEM: allocation, stores and the hand-over to
+// the issuing thread cost more than the unpack at a few rows per weight.  What bounds this kernel:
+// instruction issue, and next to it the shared-memory / L1 data path (scale tables and activations are
+// re-read by every warp; 32 outputs per warp instead of 16 halve that).
+//
+// CTAs are small (four warps, seven CTAs per SM) so that the units of a decode batch are resident at
+// once and SMs are evenly loaded.  With few units the columns are split over KS warps (partial sums
+// added through shared memory): whole 128-column chunks over KS = 2, 64-column halves over KS = 4 and 8.
+#include "grouped_tiled.cuh"
+
+namespace tris {
+namespace tr {
+
+constexpr int kDecOut = 32;                                                  // outputs of a warp
+constexpr int dec_warps(int proj, int ks) { return proj * ks > 4 ? proj * ks : 4; }
+constexpr int dec_groups(int proj, int ks) { return dec_warps(proj, ks) / (proj * ks); }
+constexpr int dec_stage_cols(int ks) { return ks == 8 ? 512 : 256; }        // columns staged at a time
+constexpr int dec_row_bytes(int ks) { return 2 * dec_stage_cols(ks) + 16; }  // odd multiple of 16: conflict-free
+constexpr int dec_buf_bytes(int nt, int ks) { return 8 * nt * dec_row_bytes(ks); }
+
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
+  return d;
+}
+
+// Two half2 (columns 2i .. 2i + 3 of a code word) of one output; c = {d, nd} scale words of the two pairs.
+__device__ __forceinline__ void unpack_two(uint32_t w, int i, const uint4& c, const RowScales& rs, uint32_t& a, uint32_t& b) {
+  const uint32_t t0 = w << i, t1 = w << (i + 1);
+  const uint32_t d0 = h2_as_u32(__hmul2_rn(u32_as_h2(c.x), rs.rd)), n0 = h2_as_u32(__hmul2_rn(u32_as_h2(c.y), rs.rn));
+  const uint32_t d1 = h2_as_u32(__hmul2_rn(u32_as_h2(c.z), rs.rd)), n1 = h2_as_u32(__hmul2_rn(u32_as_h2(c.w), rs.rn));
+  a = flip_by_sign(lop3_select(d0, n0, prmt(t0, 0u, 0xAA88u)), t0);
+  b = flip_by_sign(lop3_select(d1, n1, prmt(t1, 0u, 0xAA88u)), t1);
+}
+
+// grid (groups of 32 * dec_groups outputs, segments)
+template <int NT, int MODE, int KS>
+__global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), (NT <= 3 ? 28 : 24) / dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS))
+    grouped_decode_kernel(const __grid_constant__ TiledArgs args) {
+  constexpr bool DUAL = MODE != MODE_SINGLE;
+  constexpr int P = DUAL ? 2 : 1;
+  constexpr int NW = dec_warps(P, KS), OG = dec_groups(P, KS), kThreads = 32 * NW;
+  constexpr bool HALF = KS >= 4;                         // a warp takes one half of a chunk
+  constexpr int CS = HALF ? KS / 2 : KS;                 // chunks are dealt to CS warps
+  constexpr int kCols = dec_stage_cols(KS), kRow = dec_row_bytes(KS), kBuf = dec_buf_bytes(NT, KS);
+  constexpr int kGroupChunks = kCols / kChunkCols;
+  extern __shared__ uint4 smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);    // [buffer][set][row]
+
+  if (!args.weights_before_wait) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+  const int seg = blockIdx.y;
+  const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
+  if (seg >= nseg) return;
+  const int expert = args.expert_ids[seg];
+  const int row_begin = args.segment_offsets[seg], row_end = min(args.segment_offsets[seg + 1], args.num_rows);
+  if (expert < 0 || expert >= args.num_experts || row_end <= row_begin) return;
+
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int p = DUAL ? warp & 1 : 0, og = (warp / P) % OG, ks = warp / (P * OG);
+  const int hs = HALF ? (ks & 1) : 0, first_chunk = HALF ? (ks >> 1) : ks;
+  const int o0 = (blockIdx.x * OG + og) * kDecOut, tile = o0 / kTileOut;
+  const bool mine = o0 < args.out_features;
+  const int row = o0 % kTileOut + g;                     // this lane's outputs inside the tile: row + 8 i
+
+  const TrisProjView& v = args.proj[p];
+  const int rec_bytes = v.max_record_bytes, col_bytes = v.col_record_bytes;
+  const int sal_off = record_slices(args.rank) * kSliceBytes, scale_off = sal_off + v.max_sal_words * kStepBytes;
+  // records of the tile and the expert from chunk 0 on; `rec` at this lane's row
+  const uint8_t* rec = static_cast<const uint8_t*>(v.tile_records) +
+                       static_cast<size_t>((expert * args.tiles + tile) * args.chunks) * static_cast<size_t>(rec_bytes) + row * 4;
+  const uint8_t* col = static_cast<const uint8_t*>(v.col_records) + static_cast<size_t>(expert * args.chunks) * static_cast<size_t>(col_bytes);
+  auto load_codes = [&](int c, int sl, uint32_t (&w)[4]) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + sl * kSliceBytes + row * 12) + t;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __ldg(src + 32 * i);
+  };
+  auto load_ns_scales = [&](int c, int slot, uint32_t (&w)[4]) {  // second words of the row_pack3 entries
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + scale_off + slot * kSlotBytes + row * 4) + 1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __ldg(src + 16 * i);
+  };
+  // Codes and scales of the next slice are in registers before they are needed.  The tables of a chunk and the
+  // salient words of its tile are brought to L1 one chunk ahead, by plain loads (one line per lane) whose
+  // values are dropped when the chunk is reached.
+  uint32_t touched = 0u;
+  auto touch_chunk = [&](int c) {
+    const uint8_t* at = nullptr;
+    if (lane < 16) {
+      if (lane * 128 < col_bytes) at = col + c * col_bytes + lane * 128;
+    } else if (lane - 16 < v.max_sal_words) {
+      at = rec + c * rec_bytes + sal_off + (lane - 16) * kStepBytes - g * 4;
+    }
+    if (at) touched = __ldg(reinterpret_cast<const uint32_t*>(at));
+  };
+  uint32_t codes[4] = {0u, 0u, 0u, 0u}, scales[4] = {0u, 0u, 0u, 0u};
+  auto first_loads = [&]() {
+    if (mine && first_chunk < args.chunks) {
+      load_codes(first_chunk, hs < record_slices(args.rank) ? hs : 0, codes);
+      load_ns_scales(first_chunk, 0, scales);
+      touch_chunk(first_chunk);
+    }
+  };
+  first_loads();
+  if (args.weights_before_wait) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+
+  const int groups = (args.rank + kCols - 1) / kCols;
+#pragma unroll 1
+  for (int r0 = row_begin; r0 < row_end; r0 += 8 * NT) {
+    const int rows = min(8 * NT, row_end - r0);
+    float acc[2][NT][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[m][nt][c] = 0.f;
+
+    // Activation rows of group gr into buffer gr & 1, zero up to a multiple of 64 columns.
+    auto stage = [&](int gr) {
+      const int c0 = gr * kCols, cols = min(kCols, args.rank - c0);
+      const int pieces = ((cols + kSliceCols - 1) / kSliceCols) * (kSliceCols / 8);
+      constexpr int kPieces = kCols / 8;
+      const int piece = tid % kPieces, left = cols - 8 * piece;
+      if (piece < pieces) {
+        uint8_t* d = sm + (gr & 1) * args.num_sets * kBuf + (tid / kPieces) * kRow + piece * 16;
+        const __half* from0 = args.hidden[0] + (left > 0 ? c0 + 8 * piece : 0);
+        const __half* from1 = args.hidden[1] + (left > 0 ? c0 + 8 * piece : 0);
+#pragma unroll 2
+        for (int n = tid / kPieces; n < rows; n += kThreads / kPieces, d += kThreads / kPieces * kRow) {
+          const int src = args.row_gather ? args.row_gather[r0 + n] : r0 + n;
+          const size_t off = static_cast<size_t>(src) * args.hidden_stride;
+          if (args.hidden_vec) {
+            cp_async_16(d, from0 + off, left > 0);
+            if (P == 2 && args.num_sets == 2) cp_async_16(d + kBuf, from1 + off, left > 0);
+          } else {
+            *reinterpret_cast<uint4*>(d) = read_piece(args, args.hidden[0] + off + c0, c0, piece, left);
+            if (P == 2 && args.num_sets == 2) *reinterpret_cast<uint4*>(d + kBuf) = read_piece(args, args.hidden[1] + off + c0, c0, piece, left);
+          }
+        }
+      }
+      cp_async_commit();
+    };
+    if (r0 != row_begin) {
+      first_loads();
+      __syncthreads();  // the previous pass has read its rows and partial sums
+    }
+    stage(0);
+#pragma unroll 1
+    for (int gr = 0; gr < groups; ++gr) {
+      cp_async_wait<0>();
+      __syncthreads();
+      if (gr + 1 < groups) stage(gr + 1);  // the other buffer was read before the barrier
+      if (!mine) continue;
+      const uint8_t* rows_buf = sm + ((gr & 1) * args.num_sets + (args.num_sets == 2 ? p : 0)) * kBuf + g * kRow;
+      const int c_end = min(args.chunks, (gr + 1) * kGroupChunks);
+#pragma unroll 1
+      for (int c = gr * kGroupChunks + first_chunk; c < c_end; c += CS) {
+        const uint8_t* ccol = col + c * col_bytes;
+        const int cols = args.rank - c * kChunkCols;   // from here on
+        const bool more = c + CS < args.chunks;
+        const uint32_t counts = __ldg(reinterpret_cast<const uint32_t*>(ccol) + 1);  // ColHeader: slots, steps << 8
+        const bool several = (counts & 0xFFu) > 1u;     // row-scale slots in the chunk (groups of fewer than 128 columns)
+        const uint8_t* x_base = rows_buf + (c % kGroupChunks) * (kChunkCols * 2);
+        asm volatile("" ::"r"(touched));
+        if (more) touch_chunk(c + CS);
+        RowScales rs[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rs[i] = row_scales_ns(make_uint2(0u, scales[i]));
+#pragma unroll
+        for (int s = 0; s < (HALF ? 1 : 2); ++s) {
+          const int sl = HALF ? hs : s;
+          if (sl * kSliceCols < cols) {
+            uint32_t cur[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cur[i] = codes[i];
+            if (!HALF && s == 0 && cols > kSliceCols) {
+              load_codes(c, 1, codes);
+            } else if (more) {
+              load_codes(c + CS, HALF && hs * kSliceCols + CS * kChunkCols < cols ? hs : 0, codes);
+              load_ns_scales(c + CS, 0, scales);
+            }
+            if (several) {
+              uint32_t w[4];
+              load_ns_scales(c, ccol[8 + 2 * sl + (t >> 1)], w);  // ColHeader.slot_of_row of the lane's packed row
+#pragma unroll
+              for (int i = 0; i < 4; ++i) rs[i] = row_scales_ns(make_uint2(0u, w[i]));
+            }
+            const uint4* ct = reinterpret_cast<const uint4*>(ccol + kColHdrBytes) + sl * 16 + t;
+            const uint8_t* x = x_base + sl * (kSliceCols * 2) + t * 32;
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              uint4 b[NT];
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) b[nt] = *reinterpret_cast<const uint4*>(x + nt * 8 * kRow + jj * 16);
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const uint4 cs = __ldg(ct + (2 * jj + j) * 4);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                  uint32_t a0, a1, a2, a3;
+                  unpack_two(cur[2 * m], 4 * jj + 2 * j, cs, rs[2 * m], a0, a2);
+                  unpack_two(cur[2 * m + 1], 4 * jj + 2 * j, cs, rs[2 * m + 1], a1, a3);
+#pragma unroll
+                  for (int nt = 0; nt < NT; ++nt)
+                    mma_m16n8k16(acc[m][nt], a0, a1, a2, a3, j ? b[nt].z : b[nt].x, j ? b[nt].w : b[nt].y);
+                }
+              }
+            }
+          }
+        }
+        // salient steps: lane t takes pairs 2t, 2t + 1 of the step's 16 columns
+        const int steps = static_cast<int>((counts >> 8) & 0xFFu);
+#pragma unroll 1
+        for (int st = hs; st < steps; st += HALF ? 2 : 1) {
+          const uint8_t* ent = ccol + kColHdrBytes + kColTabBytes + st * kColStepBytes;
+          const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + sal_off + st * kStepBytes);
+          const int slot = several ? ccol[12 + st] : 0;  // ColHeader.step_slot
+          const uint32_t* rsrc = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + scale_off + slot * kSlotBytes + row * 4);
+          const uint4 cs = __ldg(reinterpret_cast<const uint4*>(ent) + t);
+          const uint2 at = __ldg(reinterpret_cast<const uint2*>(ent + 64) + t);
+          uint32_t w[4], rp[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            w[i] = __ldg(wsrc + 8 * i) << (2 * t);
+            rp[i] = __ldg(rsrc + 16 * i);
+          }
+          uint32_t b[NT][2];
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            auto ld = [&](uint32_t cc) -> uint32_t { return *reinterpret_cast<const uint16_t*>(x_base + 2 * cc + nt * 8 * kRow); };
+            b[nt][0] = prmt(ld(at.x & 0xFFFFu), ld(at.x >> 16), 0x5410u);
+            b[nt][1] = prmt(ld(at.y & 0xFFFFu), ld(at.y >> 16), 0x5410u);
+          }
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            uint32_t a[2][2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const __half2 r1 = u32_as_h2(prmt(rp[2 * m + h], 0u, 0x1010u)), r2 = u32_as_h2(prmt(rp[2 * m + h], 0u, 0x3232u));
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                const uint32_t tt = w[2 * m + h] << i;
+                const uint32_t p1 = flip_by_sign(h2_as_u32(__hmul2_rn(u32_as_h2(i ? cs.z : cs.x), r1)), tt);
+                const uint32_t p2 = flip_by_sign(h2_as_u32(__hmul2_rn(u32_as_h2(i ? cs.w : cs.y), r2)), tt << 8);
+                a[h][i] = h2_as_u32(__hadd2_rn(u32_as_h2(p1), u32_as_h2(p2)));
+              }
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) mma_m16n8k16(acc[m][nt], a[0][0], a[1][0], a[0][1], a[1][1], b[nt][0], b[nt][1]);
+          }
+        }
+      }
+    }
+
+    // Output scale and bias act on the whole sum: applied to the first part, the bias once.
+    if (mine && (v.output_scale || v.bias)) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const size_t at = static_cast<size_t>(expert) * args.out_features + min(o0 + g + 8 * i, args.out_features - 1);
+        const float scale = v.output_scale ? __half2float(static_cast<const __half*>(v.output_scale)[at]) : 1.f;
+        const float bias = v.bias && ks == 0 ? __half2float(static_cast<const __half*>(v.bias)[at]) : 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) acc[i >> 1][nt][2 * (i & 1) + e] = acc[i >> 1][nt][2 * (i & 1) + e] * scale + bias;
+      }
+    }
+    // Partial sums meet: 16 outputs m of a pair of warps are finished by the gate warp (m = 0) or the up warp
+    // (m = 1) for SiLU(gate) * up, by each projection's own warp otherwise; always by the ks = 0 warp.
+    float up[NT][4];
+    if constexpr (KS > 1 || MODE == MODE_DUAL_SILU) {
+      float4* part = reinterpret_cast<float4*>(sm);
+      auto slot_of = [&](int pp, int kk, int m, int nt) { return part + (((((pp * KS + kk) * OG + og) * 2 + m) * NT + nt) * 32 + lane); };
+      __syncthreads();  // every warp is done with the activation rows
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        if (ks == 0 && (MODE != MODE_DUAL_SILU || m == p)) continue;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) *slot_of(p, ks, m, nt) = make_float4(acc[m][nt][0], acc[m][nt][1], acc[m][nt][2], acc[m][nt][3]);
+      }
+      __syncthreads();
+      if (ks > 0) continue;
+      auto add = [&](float (&x)[4], const float4* q) {
+        const float4 y = *q;
+        x[0] += y.x;
+        x[1] += y.y;
+        x[2] += y.z;
+        x[3] += y.w;
+      };
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        if constexpr (MODE == MODE_DUAL_SILU) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (p) acc[0][nt][e] = acc[1][nt][e];  // the finished half is m = p
+            up[nt][e] = 0.f;
+          }
+#pragma unroll
+          for (int k = 1; k < KS; ++k) add(acc[0][nt], slot_of(p, k, p, nt));
+#pragma unroll
+          for (int k = 0; k < KS; ++k) add(up[nt], slot_of(p ^ 1, k, p, nt));
+        } else {
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int k = 1; k < KS; ++k) add(acc[m][nt], slot_of(p, k, m, nt));
+        }
+      }
+    }
+    if (!mine) continue;
+
+    // epilogue: a 16-output half holds {(output g, row 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1)}
+    constexpr int kHalves = MODE == MODE_DUAL_SILU ? 1 : 2;
+#pragma unroll
+    for (int m = 0; m < kHalves; ++m) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        if (nt * 8 < rows) {
+          float y[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            y[e] = acc[m][nt][e];
+            if constexpr (MODE == MODE_DUAL_SILU) {
+              const float gate = p ? up[nt][e] : y[e], lin = p ? y[e] : up[nt][e];
+              y[e] = __fdividef(gate, 1.f + __expf(-gate)) * lin;
+            }
+          }
+          // transposed: this lane holds row g, outputs 2t, 2t + 1 (lo) and 8 + 2t, 9 + 2t (hi); neighbours swap one
+          // so that each stores four outputs
+          const uint32_t lo = transpose_8x8(h2_as_u32(__floats2half2_rn(y[0], y[1])));
+          const uint32_t hi = transpose_8x8(h2_as_u32(__floats2half2_rn(y[2], y[3])));
+          const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, (t & 1) ? lo : hi, 1);
+          const uint2 w = (t & 1) ? make_uint2(other, hi) : make_uint2(lo, other);
+          const int n = nt * 8 + g;
+          const int orow = n >= rows ? -1 : (args.out_scatter ? args.out_scatter[r0 + n] : r0 + n);
+          if (orow >= 0) {
+            const int o = o0 + 16 * (MODE == MODE_DUAL_SILU ? p : m) + ((t & 1) ? 8 : 0) + 2 * (t & 2);
+            __half* dst = args.out[MODE == MODE_DUAL_STORE ? p : 0] + static_cast<size_t>(orow) * args.out_features + o;
+            if (args.quad_store) {
+              if (o < args.out_features) *reinterpret_cast<uint2*>(dst) = w;
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (o + i < args.out_features)
+                  dst[i] = __ushort_as_half(static_cast<unsigned short>((i & 2 ? w.y : w.x) >> (16 * (i & 1))));
+            }
+          }
+          __syncwarp();  // the transposes need the warp together
+        }
+      }
+    }
+  }
+}
+
+template <int NT, int MODE, int KS>
+static int launch_decode(const TiledArgs& args, cudaStream_t stream, bool pdl) {
+  const int bufs = args.rank > dec_stage_cols(KS) ? 2 : 1;
+  constexpr int P = MODE == MODE_SINGLE ? 1 : 2;
+  const int part = (KS > 1 || MODE == MODE_DUAL_SILU) ? dec_warps(P, KS) * 2 * NT * 512 : 0;
+  const size_t smem = std::max(bufs * args.num_sets * dec_buf_bytes(NT, KS), part);
+  auto kernel = grouped_decode_kernel<NT, MODE, KS>;
+  static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
+  int st = configure_smem(kernel, smem, configured);
+  if (st != TRIS_OK) return st;
+  return check_cuda(launch_kernel(kernel, dim3(ceil_div(args.out_features, kDecOut * dec_groups(P, KS)), args.num_segments), dim3(32 * dec_warps(P, KS)),
+                                  smem, stream, pdl, 1, args),
+                    "grouped_decode_kernel launch");
+}
+
+template <int NT, int MODE>
+static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) {
+  // Fewer than 14 warps per SM: split the columns, as far as there are columns to split
+  const long long warps = static_cast<long long>(ceil_div(args.out_features, kDecOut)) * args.num_segments * (MODE == MODE_SINGLE ? 1 : 2);
+  const int slices = ceil_div(args.rank, kSliceCols), want = 14 * sm_count();
+  if (warps * 4 < want && slices >= 16) return launch_decode<NT, MODE, 8>(args, stream, pdl);
+  if (warps * 2 < want && slices >= 4) return launch_decode<NT, MODE, 4>(args, stream, pdl);
+  if (warps < want && slices >= 4) return launch_decode<NT, MODE, 2>(args, stream, pdl);
+  return launch_decode<NT, MODE, 1>(args, stream, pdl);
+}
+
+template <int MODE>
+static int dispatch_decode(const TiledArgs& args, int typical_rows, cudaStream_t stream, bool pdl) {
+  if (typical_rows <= 8) return dispatch_split<1, MODE>(args, stream, pdl);
+  if (typical_rows <= 16) return dispatch_split<2, MODE>(args, stream, pdl);
+  if (typical_rows <= 24) return dispatch_split<3, MODE>(args, stream, pdl);
+  return dispatch_split<4, MODE>(args, stream, pdl);
+}
+
+int launch_grouped_decode(const TiledArgs& args, int mode, int typical_rows, cudaStream_t stream, bool pdl) {
+  if (mode == MODE_SINGLE) return dispatch_decode<MODE_SINGLE>(args, typical_rows, stream, pdl);
+  if (mode == MODE_DUAL_SILU) return dispatch_decode<MODE_DUAL_SILU>(args, typical_rows, stream, pdl);
+  return dispatch_decode<MODE_DUAL_STORE>(args, typical_rows, stream, pdl);
+}
+
+}  // namespace tr
+}  // namespace tris

@@ -1,881 +1,633 @@
-// Grouped compact3 dequant-matmul over tile records (decode / skinny regime), and the dump
+// Grouped compact3 dequant-matmul over tile records, on the tcgen05 tensor cores, and the dump
 // kernel the parity tests use.  See tile_records.cuh for the record layout and the unpack.
 //
-// Work unit = one expert segment x two tile records: the gate and the up tile of the same 64
-// outputs (dual launch), or two neighbouring 64-output tiles of one projection.  A CTA has 8
-// warps; warp w works on record w / 4, outputs 16 * (w % 4) .. +15.  Per unit:
-//   1. two threads fetch the two tile records and their column records, one bulk copy each
-//      (cp.async.bulk completing on an mbarrier);
-//   2. every warp Golomb-Rice decodes one block-GR block (32 lanes = 32 indexed sub-streams)
-//      into the g_map plane in shared memory;
-//   3. activation rows arrive by bulk copies (one per row, issued by eight lanes of every warp);
-//      the activations of the salient columns are gathered into rows of their own;
-//   4. every warp unpacks its weights straight into m16n8k16 A fragments and multiplies them
-//      with the staged rows, fp32 accumulation; then the short salient pass;
-//   5. results go through shared memory and leave as 16-byte stores.
-// No dequantised weight leaves registers.
+// Work unit = one expert segment x two output tiles of 128: the gate and the up tile of the same
+// outputs (dual launch), or two neighbouring tiles of one projection.  A pass multiplies up to N rows
+// of the segment; it walks the columns in chunks of 128, and a (pass, chunk) is an "item".  One
+// persistent CTA per SM, its warps specialised so that the phases of consecutive items overlap:
 //
-// Two kernels share this code.  grouped_tiled_persistent_kernel (projections of at most 256
-// columns: one chunk) runs a fixed number of CTAs per SM, each walking units blockIdx.x,
-// blockIdx.x + gridDim.x, ...; the records of the next unit are fetched into the other half of
-// a two-stage ring while the current unit is decoded and multiplied, so the fetch latency
-// (route entry -> descriptor -> DRAM) is paid once per CTA instead of once per unit.
-// grouped_tiled_kernel (any number of chunks) runs one CTA per unit and loops over the chunks.
-// Waits on mbarriers are bounded; a time-out is reported through the route's status word and
-// the CTA leaves without storing results.
+//   loader (4 warps)     activation rows and column records of an item to shared memory (cp.async,
+//                        a ring of stages), then the activations of the salient columns gathered
+//                        into K columns of their own;
+//   unpack (16 warps)    four warpgroups, one thread per output row: warpgroup (r, h) takes tile r of
+//                        every second item.  A thread loads the code words of its own row straight from
+//                        the record (coalesced, used once, so they never touch shared memory), unpacks
+//                        64 columns to fp16 and writes them to its TMEM lane (tcgen05.st; two slots per
+//                        warpgroup);
+//   MMA (2 warps)        one per tile: tcgen05.mma with the weights from TMEM and the activations from shared memory
+//                        into TMEM accumulators [128 outputs][rows];
+//   epilogue (8 warps)   accumulators -> scale / bias or SiLU(gate) * up -> fp16 rows.
+//
+// No dequantised weight leaves the SM.  What bounds it: instruction issue, of which the unpack is the
+// larger part (3.9 lane-instructions per weight, against 16 for unpacking to mma.sync fragments
+// with the Golomb-Rice decode in the loop).
+// Waits on mbarriers are bounded; a time-out is reported through the route's status word and the
+// CTA leaves.
 #include <math.h>
 
-#include <algorithm>
-#include <atomic>
-
-#include "tile_records.cuh"
+#include "grouped_tiled.cuh"
 
 namespace tris {
 namespace tr {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = 8;
-constexpr int kOutTileRowBytes = 144;  // 64 halves + 16 bytes: rows 2t of the four t land in four bank groups
-enum { MODE_SINGLE = 0, MODE_DUAL_STORE = 1, MODE_DUAL_SILU = 2 };
-
-struct TiledArgs {
-  TrisProjView proj[2];
-  const __half* hidden[2];
-  __half* out[2];
-  const int32_t* expert_ids;
-  const int32_t* segment_offsets;
-  const int32_t* num_segments_dev;
-  const int32_t* row_gather;
-  const int32_t* out_scatter;
-  int32_t* status;
-  int32_t num_segments;
-  int32_t num_rows;
-  int32_t hidden_lane_order;    // activation rows already in lane order (else row-major)
-  int32_t hidden_stride;        // halves between activation rows
-  int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
-  int32_t rec_slot_bytes;       // shared-memory bytes reserved per tile record (16 bytes of slack included)
-  int32_t col_slot_bytes;
-  int32_t sal_slots;            // salient words reserved per activation set
-  const __half* col_scale;      // optional [rank]: activation rows are multiplied by it while staged (row-major rows only)
+constexpr int kUnpackWarps = 16, kLoadWarps = 4, kMmaWarps = 2;
+// Warps of a CTA by role.  The narrow passes of decode need one epilogue warpgroup; with eight warps fewer
+// than 32 every thread may use 72 registers, which is what the unpack wants.
+template <int N>
+struct Roles {
+  static constexpr int kEpiWarps = N <= 64 ? 4 : 8;
+  static constexpr int kEpi0 = kUnpackWarps, kLoad0 = kEpi0 + kEpiWarps, kMma0 = kLoad0 + kLoadWarps;
+  static constexpr int kThreads = (kMma0 + kMmaWarps) * 32;
 };
+constexpr int kMaxStages = 4;
+constexpr int kDBase = 4 * 2 * kACols;       // accumulators behind the four warpgroups' two slots
+constexpr int kBarBytes = 512;
+constexpr int kRowIdxBytes = 2 * 128 * 4;
 
-// Shared-memory carve-up: [mbarriers 64][stages x (2 records + NH column records)][2 g_map planes]
-// [salient rows NH x sal_slots x NT*8 x 64][activation rows NH x NT*8 x 576]
-struct SmemLayout {
-  int stage_bytes, gmap_off, hsal_off, hrows_off, total;
+// One stage: [column records][activation rows: K-major core matrices, [column / 8][N rows][16 B]][salient
+// activations, the same form, per projection]
+struct StageLayout {
+  int col_bytes, rows_off, rows_bytes, sal_off, sal_bytes, total;
 };
-__host__ __device__ inline SmemLayout smem_layout(int rec_slot, int col_slot, int sal_slots, int nh, int nt, int stages) {
-  SmemLayout l;
-  l.stage_bytes = 2 * rec_slot + nh * col_slot;
-  l.gmap_off = 64 + stages * l.stage_bytes;
-  l.hsal_off = l.gmap_off + 2 * 2048;
-  l.hrows_off = l.hsal_off + nh * sal_slots * nt * 8 * 64;
-  l.total = l.hrows_off + nh * nt * 8 * kHiddenRowBytes;
+__host__ __device__ inline StageLayout stage_layout(int max_steps, int ncol, int nset, int n) {
+  StageLayout l;
+  l.col_bytes = kColHdrBytes + kColTabBytes + max_steps * kColStepBytes;
+  l.rows_off = (ncol * l.col_bytes + 127) & ~127;
+  l.rows_bytes = n * kChunkCols * 2;
+  l.sal_off = l.rows_off + nset * l.rows_bytes;
+  l.sal_bytes = max_steps * n * 32;
+  l.total = l.sal_off + ncol * l.sal_bytes;
   return l;
 }
 
-// One lane moves nbytes global -> shared: a bulk copy when both ends are 16-byte aligned and the
-// size is a multiple of 16, plain loads otherwise.  Returns the bytes the mbarrier must expect.
-__device__ __forceinline__ uint32_t lane_copy_bytes(void* dst, const void* src, int nbytes, uint64_t* bar) {
-  if (nbytes <= 0) return 0;
-  if (((reinterpret_cast<uintptr_t>(src) | smem_u32(dst) | static_cast<uint32_t>(nbytes)) & 15u) == 0) {
-    bulk_g2s(dst, src, static_cast<uint32_t>(nbytes), bar);
-    return static_cast<uint32_t>(nbytes);
-  }
-  for (int i = 0; i < nbytes; i += 2)
-    *reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(dst) + i) = *reinterpret_cast<const uint16_t*>(static_cast<const uint8_t*>(src) + i);
-  return 0;
-}
-
-// Activation rows of a pass into hrows[set][row]; row_src(n) = source row or -1.  Lane-order
-// rows are copied as they are (lanes 0-7 of every warp issue one bulk copy per round); row-major
-// rows are re-ordered by all threads.  Lane 0 of every warp arrives on `bar`.
-template <int NT, int NH, typename RowSrc>
-__device__ __forceinline__ void issue_hidden(uint8_t* hrows, const __half* const* hidden, int rank, int p0, int nrows,
-                                             bool lane_order, int row_stride, uint64_t* bar, RowSrc row_src,
-                                             const __half* col_scale = nullptr) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c0 = 32 * p0;
-  const int ncols = min(256, rank - c0);
-  uint32_t bytes = 0;
-  if (lane_order && lane < 8) {
-    fence_proxy_async();
-    for (int i = warp * 8 + lane; i < NH * nrows; i += kWarps * 8) {
-      const int set = (NH == 2 && i >= nrows) ? 1 : 0;
-      const int n = i - set * nrows;
-      const int src = row_src(n);
-      if (src >= 0)
-        bytes += lane_copy_bytes(hrows + (set * NT * 8 + n) * kHiddenRowBytes,
-                                 hidden[set] + static_cast<size_t>(src) * row_stride + c0, 2 * ncols, bar);
+// Every role walks the same sequence: a CTA owns a contiguous range of units, and the units of one segment in
+// it form a run; for every pass over the segment's rows, for every tile of the run, for every chunk: an item.
+// The activation rows of a pass are staged once per run when all their chunks fit the ring (`reuse`),
+// otherwise a run is one tile.  The route entries of the next run are loaded while the current one is
+// worked on.
+template <int N>
+struct Walker {
+  int u, u_end, nseg;
+  int x, x_begin, x_end, expert, row_end, r0, c;
+  int next_x, next_expert, next_begin, next_end;
+  __device__ __forceinline__ void peek(const TiledArgs& args, int unit) {
+    if (unit >= u_end) return;
+    const int q = unit / args.units_x;
+    next_x = unit - q * args.units_x;
+    int seg = q, z = 0;  // row split: part z takes the passes z, z + row_split, ...
+    if (args.row_split > 1) {
+      z = q / nseg;
+      seg = q - z * nseg;
     }
+    next_expert = args.expert_ids[seg];
+    next_begin = args.segment_offsets[seg] + z * N;
+    next_end = args.segment_offsets[seg + 1];
   }
-  bytes = __reduce_add_sync(0xFFFFFFFFu, bytes);
-  if (lane == 0) {
-    if (bytes) mbar_arrive_expect_tx(bar, bytes);
-    else mbar_arrive(bar);
+  __device__ __forceinline__ void start(const TiledArgs& args) {
+    nseg = args.num_segments_dev ? min(warp_uniform(*args.num_segments_dev), args.num_segments) : args.num_segments;
+    const int total = nseg * args.units_x * args.row_split, per = total / gridDim.x, extra = total - per * gridDim.x;
+    const int b = blockIdx.x;
+    u = b * per + min(b, extra);
+    u_end = u + per + (b < extra ? 1 : 0);
+    peek(args, u);
+    load(args);
   }
-  if (lane_order) return;
-  const int items = NH * nrows * 32;  // 8 columns per item
-  for (int i = threadIdx.x; i < items; i += kThreads) {
-    const int j8 = i & 31, n = (i >> 5) % nrows, set = i / (32 * nrows);
-    const int col = c0 + 8 * j8;
-    const int src = row_src(n);
-    __half vals[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) vals[u] = __ushort_as_half(0);
-    if (src >= 0 && col < rank) {
-      const __half* rowp = hidden[set] + static_cast<size_t>(src) * row_stride + col;
-      if (col + 8 <= rank && (reinterpret_cast<uintptr_t>(rowp) & 15u) == 0) {
-        *reinterpret_cast<uint4*>(vals) = *reinterpret_cast<const uint4*>(rowp);
-      } else {
-        for (int u = 0; u < 8 && col + u < rank; ++u) vals[u] = rowp[u];
-      }
-    }
-    if (col_scale && src >= 0) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (col + u < rank) vals[u] = __hmul(vals[u], col_scale[col + u]);
-    }
-    __half* dst = reinterpret_cast<__half*>(hrows + (set * NT * 8 + n) * kHiddenRowBytes);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int j = 8 * j8 + u;
-      dst[(j & ~31) + lane_order_pos(j & 31)] = vals[u];
+  __device__ __forceinline__ bool valid() const { return u < u_end; }
+  __device__ __forceinline__ void load(const TiledArgs& args) {  // first item of the run at u, or of the next one that has rows
+    while (u < u_end) {
+      x = x_begin = next_x;  // (next_x comes from u; the loaded values are made uniform here, where they are first needed)
+      x_end = args.reuse ? min(args.units_x, x_begin + (u_end - u)) : x_begin + 1;
+      expert = warp_uniform(next_expert);
+      r0 = warp_uniform(next_begin);
+      row_end = min(warp_uniform(next_end), args.num_rows);
+      c = 0;
+      peek(args, u + (x_end - x_begin));
+      if (expert >= 0 && expert < args.num_experts && r0 < row_end) return;
+      u += x_end - x_begin;
     }
   }
-}
-
-// Gathers the activations of the salient columns into rows of their own, hsal[set][word][row]
-// (64 bytes: the word's 32 slots in lane order), so that the salient pass loads its B fragments
-// like the main loop does.  All threads; col(set) = the staged column record of that set.
-template <int NT, int NH, typename ColOf>
-__device__ __forceinline__ void gather_salient(uint8_t* hsal, const uint8_t* hrows, int nrows, int sal_slots, ColOf col_of) {
-#pragma unroll
-  for (int set = 0; set < NH; ++set) {
-    const uint8_t* col = col_of(set);
-    const int words = min(static_cast<int>(reinterpret_cast<const ColHeader*>(col)->sal_words), sal_slots);
-    for (int q = 0; q < words; ++q) {
-      for (int i = threadIdx.x; i < nrows * 4; i += kThreads) {
-        const int t = i & 3, n = i >> 2;
-        const uint4 pos = *reinterpret_cast<const uint4*>(col + kColHdrBytes + kColTabBytes + q * kSalEntryBytes + t * 16);
-        const uint8_t* rp = hrows + (set * NT * 8 + n) * kHiddenRowBytes;
-        auto ld = [&](uint32_t off) { return static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(rp + off)); };
-        uint4 v;
-        v.x = ld(pos.x & 0xFFFFu) | (ld(pos.x >> 16) << 16);
-        v.y = ld(pos.y & 0xFFFFu) | (ld(pos.y >> 16) << 16);
-        v.z = ld(pos.z & 0xFFFFu) | (ld(pos.z >> 16) << 16);
-        v.w = ld(pos.w & 0xFFFFu) | (ld(pos.w >> 16) << 16);
-        *reinterpret_cast<uint4*>(hsal + (((set * sal_slots + q) * NT * 8 + n) * 4 + t) * 16) = v;
-      }
-    }
+  __device__ __forceinline__ int rows() const { return min(N, row_end - r0); }
+  __device__ __forceinline__ void next_pass(const TiledArgs& args) {
+    c = 0;
+    x = x_begin;
+    r0 += args.row_split * N;
+    if (r0 < row_end) return;
+    u += x_end - x_begin;
+    load(args);
   }
-}
-
-// ---- main loop of one 256-column chunk ----------------------------------------------------------
-// NTC (compile time) = live 8-row tiles of this pass.  The packed rows are walked slot by slot
-// (runs of rows that share their row scales), so the inner loop has no branch but its own.
-// Second pass of a chunk: the salient columns, compacted into 32-slot "salient words" whose
-// activations gather_salient put into hsal.
-template <int NT, int NTC>
-__device__ __forceinline__ void sal_chunk_n(const StagedTile& st, const uint8_t* hsal_set, int out_local, int lane,
-                                            float (&acc)[NT][4]) {
-  const int g = lane >> 2, t = lane & 3;
-  const ColHeader* ch = reinterpret_cast<const ColHeader*>(st.col);
-  const int sal_words = ch->sal_words;
-  const uint8_t* s_base = hsal_set + g * 64 + t * 16;
-  const LaneShifts ls = lane_shifts(t);
-  for (int q = 0; q < sal_words; ++q) {
-    uint32_t a[2][4];
-    unpack_fragments_sal(st, q, out_local, lane, ls, a);
-#pragma unroll
-    for (int nt = 0; nt < NTC; ++nt) {
-      const uint4 hv = *reinterpret_cast<const uint4*>(s_base + (q * NT + nt) * 8 * 64);
-      mma_m16n8k16(acc[nt], a[0][0], a[1][0], a[0][1], a[1][1], hv.x, hv.y);
-      mma_m16n8k16(acc[nt], a[0][2], a[1][2], a[0][3], a[1][3], hv.z, hv.w);
-    }
+  __device__ __forceinline__ void next_tile(const TiledArgs& args) {
+    c = 0;
+    if (++x == x_end) next_pass(args);
   }
-}
-
-template <int NT, int NTC>
-__device__ __forceinline__ void main_chunk_n(const StagedTile& st, const uint8_t* hrows_set, const uint8_t* hsal_set,
-                                             int out_local, int lane, float (&acc)[NT][4]) {
-  const int g = lane >> 2, t = lane & 3;
-  const uint8_t* h_base = hrows_set + g * kHiddenRowBytes + t * 16;
-  const ColHeader* ch = reinterpret_cast<const ColHeader*>(st.col);
-  const int num_slots = ch->num_slots;
-  const LaneShifts ls = lane_shifts(t);
-  int p = 0;
-  for (int slot = 0; slot < num_slots; ++slot) {
-    const int p_end = ch->slot_end[slot];
-    const RowScalesNs rs = load_row_scales_ns(st, slot, out_local, lane);
-#pragma unroll 2
-    for (; p < p_end; ++p) {
-      uint32_t a[2][4];
-      unpack_fragments_ns(st, p, out_local, lane, rs, ls, a);
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) {
-        const uint4 hv = *reinterpret_cast<const uint4*>(h_base + nt * 8 * kHiddenRowBytes + p * 64);
-        mma_m16n8k16(acc[nt], a[0][0], a[1][0], a[0][1], a[1][1], hv.x, hv.y);
-        mma_m16n8k16(acc[nt], a[0][2], a[1][2], a[0][3], a[1][3], hv.z, hv.w);
-      }
-    }
+  __device__ __forceinline__ void next(const TiledArgs& args) {
+    if (++c == args.chunks) next_tile(args);
   }
-  sal_chunk_n<NT, NTC>(st, hsal_set, out_local, lane, acc);
-}
-
-template <int NT>
-__device__ __forceinline__ void main_chunk(const StagedTile& st, const uint8_t* hrows_set, const uint8_t* hsal_set,
-                                           int out_local, int lane, int nt_count, float (&acc)[NT][4]) {
-  if (NT == 1 || nt_count == 1) main_chunk_n<NT, 1>(st, hrows_set, hsal_set, out_local, lane, acc);
-  else if (NT == 2 || nt_count == 2) main_chunk_n<NT, (NT >= 2 ? 2 : NT)>(st, hrows_set, hsal_set, out_local, lane, acc);
-  else if (NT == 3 || nt_count == 3) main_chunk_n<NT, (NT >= 3 ? 3 : NT)>(st, hrows_set, hsal_set, out_local, lane, acc);
-  else main_chunk_n<NT, NT>(st, hrows_set, hsal_set, out_local, lane, acc);
-}
-
-// ---- weights of a chunk kept in registers across row passes (segments of many rows) ------------------
-// A warp owns 16 outputs x 256 columns = 64 half2 per lane: unpacked once per unit, after which a
-// row pass costs only the activation loads and the MMAs.  Returns the packed rows of the chunk.
-__device__ __forceinline__ int unpack_chunk_ns(const StagedTile& st, int out_local, int lane, uint32_t (&a)[kChunkRows][2][4]) {
-  const ColHeader* ch = reinterpret_cast<const ColHeader*>(st.col);
-  const int num_slots = ch->num_slots;
-  const int p_total = num_slots > 0 ? min(static_cast<int>(ch->slot_end[num_slots - 1]), kChunkRows) : 0;
-  int slot = 0;
-  RowScalesNs rs = load_row_scales_ns(st, 0, out_local, lane);
-  const LaneShifts ls = lane_shifts(lane & 3);
-#pragma unroll
-  for (int p = 0; p < kChunkRows; ++p) {
-    if (p < p_total) {
-      while (slot + 1 < num_slots && p >= ch->slot_end[slot]) {
-        ++slot;
-        rs = load_row_scales_ns(st, slot, out_local, lane);
-      }
-      unpack_fragments_ns(st, p, out_local, lane, rs, ls, a[p]);
-    } else {
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[p][h][i] = 0u;
-    }
+  __device__ __forceinline__ void next_stage(const TiledArgs& args) {  // for the role that does not look at tiles
+    if (++c == args.chunks) next_pass(args);
   }
-  return p_total;
-}
-
-template <int NT, int NTC>
-__device__ __forceinline__ void main_chunk_cached_n(const StagedTile& st, const uint32_t (&a)[kChunkRows][2][4], int p_total,
-                                                    const uint8_t* hrows_set, const uint8_t* hsal_set, int out_local, int lane,
-                                                    float (&acc)[NT][4]) {
-  const int g = lane >> 2, t = lane & 3;
-  const uint8_t* h_base = hrows_set + g * kHiddenRowBytes + t * 16;
-#pragma unroll
-  for (int p = 0; p < kChunkRows; ++p) {
-    if (p < p_total) {
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) {
-        const uint4 hv = *reinterpret_cast<const uint4*>(h_base + nt * 8 * kHiddenRowBytes + p * 64);
-        mma_m16n8k16(acc[nt], a[p][0][0], a[p][1][0], a[p][0][1], a[p][1][1], hv.x, hv.y);
-        mma_m16n8k16(acc[nt], a[p][0][2], a[p][1][2], a[p][0][3], a[p][1][3], hv.z, hv.w);
-      }
-    }
-  }
-  sal_chunk_n<NT, NTC>(st, hsal_set, out_local, lane, acc);
-}
-
-template <int NT>
-__device__ __forceinline__ void main_chunk_cached(const StagedTile& st, const uint32_t (&a)[kChunkRows][2][4], int p_total,
-                                                  const uint8_t* hrows_set, const uint8_t* hsal_set, int out_local, int lane,
-                                                  int nt_count, float (&acc)[NT][4]) {
-  if (NT == 1 || nt_count == 1) main_chunk_cached_n<NT, 1>(st, a, p_total, hrows_set, hsal_set, out_local, lane, acc);
-  else if (NT == 2 || nt_count == 2) main_chunk_cached_n<NT, (NT >= 2 ? 2 : NT)>(st, a, p_total, hrows_set, hsal_set, out_local, lane, acc);
-  else if (NT == 3 || nt_count == 3) main_chunk_cached_n<NT, (NT >= 3 ? 3 : NT)>(st, a, p_total, hrows_set, hsal_set, out_local, lane, acc);
-  else main_chunk_cached_n<NT, NT>(st, a, p_total, hrows_set, hsal_set, out_local, lane, acc);
-}
-
-// ---- epilogue of one row pass --------------------------------------------------------------------
-// acc[nt] = {(out g, row 2t), (out g, row 2t+1), (out g+8, row 2t), (out g+8, row 2t+1)}.
-// Output scale and bias; for MODE_DUAL_SILU the up warp (w + 4) hands its values to the gate warp
-// (w) through `xbuf` and the gate warp computes SiLU(gate) * up.  The fp16 results are laid out as
-// tiles [row][64 outputs] in `otile` and leave as 16-byte stores issued by all threads.  `scratch`
-// is shared memory nobody else uses until the next barrier (the activation rows of the finished
-// pass).  All threads must call; contains CTA-wide barriers.
-template <int NT, int MODE>
-__device__ __forceinline__ void finish_rows(const TiledArgs& args, uint8_t* scratch, int r, int og, bool tile_valid, int expert,
-                                            int tile0, int r0, int rows, int nt_count, float (&acc)[NT][4]) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const TrisProjView& v = args.proj[MODE == MODE_SINGLE ? 0 : r];
-  const int o_first = (tile0 + (MODE == MODE_SINGLE ? r : 0)) * kTileOut + og * 16;
-  float* xbuf = reinterpret_cast<float*>(scratch);                       // [4 og][NT][32 lanes] float4
-  uint8_t* otile = scratch + 4 * NT * 32 * 16;                           // [tile][row][144 B]
-  if (v.output_scale || v.bias) {
-    float scale[2] = {1.f, 1.f}, bias[2] = {0.f, 0.f};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int o = o_first + g + 8 * h;
-      if (o < v.out_features) {
-        if (v.output_scale) scale[h] = __half2float(static_cast<const __half*>(v.output_scale)[static_cast<size_t>(expert) * v.out_features + o]);
-        if (v.bias) bias[h] = __half2float(static_cast<const __half*>(v.bias)[static_cast<size_t>(expert) * v.out_features + o]);
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[nt][c] = acc[nt][c] * scale[c >> 1] + bias[c >> 1];
-  }
-  __syncthreads();  // every warp is done with the activation rows: they become scratch
-  if (MODE == MODE_DUAL_SILU) {
-    if (r == 1) {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-        if (nt < nt_count)
-          *reinterpret_cast<float4*>(xbuf + ((og * NT + nt) * 32 + lane) * 4) = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
-    }
-    named_barrier_sync(1 + og, 64);
-    if (r == 0) {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        if (nt >= nt_count) continue;
-        const float4 u = *reinterpret_cast<const float4*>(xbuf + ((og * NT + nt) * 32 + lane) * 4);
-        const float up[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[nt][c] = __fdividef(acc[nt][c], 1.f + __expf(-acc[nt][c])) * up[c];
-      }
-    }
-  }
-  const bool writes = tile_valid && (MODE != MODE_DUAL_SILU || r == 0);
-  if (writes) {
-    uint8_t* tile = otile + (MODE == MODE_DUAL_SILU ? 0 : r) * (NT * 8 * kOutTileRowBytes);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      if (nt >= nt_count) continue;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int n = nt * 8 + 2 * t + (c & 1);
-        const int ol = og * 16 + g + 8 * (c >> 1);
-        *reinterpret_cast<__half*>(tile + n * kOutTileRowBytes + ol * 2) = __float2half_rn(acc[nt][c]);
-      }
-    }
-  }
-  __syncthreads();
-  // 16-byte stores: item = (tile, row, 8-output piece)
-  constexpr int kTiles = (MODE == MODE_DUAL_SILU) ? 1 : 2;
-  const int items = kTiles * rows * 8;
-  for (int i = tid; i < items; i += kThreads) {
-    const int piece = i & 7;
-    const int n = (i >> 3) % rows;
-    const int tl = (kTiles == 2 && (i >> 3) >= rows) ? 1 : 0;
-    const TrisProjView& vo = args.proj[MODE == MODE_DUAL_STORE ? tl : 0];
-    const int o = (tile0 + (MODE == MODE_SINGLE ? tl : 0)) * kTileOut + piece * 8;
-    if (o >= vo.out_features) continue;
-    const int orow = args.out_scatter ? args.out_scatter[r0 + n] : r0 + n;
-    if (orow < 0) continue;
-    __half* dst = args.out[MODE == MODE_DUAL_STORE ? tl : 0] + static_cast<size_t>(orow) * vo.out_features + o;
-    const uint8_t* src = otile + tl * (NT * 8 * kOutTileRowBytes) + n * kOutTileRowBytes + piece * 16;
-    if (o + 8 <= vo.out_features && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-    } else {
-      for (int u = 0; u < 8 && o + u < vo.out_features; ++u) dst[u] = reinterpret_cast<const __half*>(src)[u];
-    }
-  }
-}
-
-struct UnitRoute {
-  int expert, row_begin, row_end;
 };
-__device__ __forceinline__ UnitRoute load_unit_route(const TiledArgs& args, int seg) {
-  UnitRoute u;
-  u.expert = args.expert_ids[seg];
-  u.row_begin = args.segment_offsets[seg];
-  u.row_end = min(args.segment_offsets[seg + 1], args.num_rows);
-  return u;
-}
-__device__ __forceinline__ bool unit_live(const TiledArgs& args, const UnitRoute& u) {
-  return u.expert >= 0 && u.expert < args.proj[0].num_experts && u.row_end > u.row_begin;
-}
 
-// ---- one CTA per unit, any number of chunks ---------------------------------------------------------
-// grid (tiles (dual) or ceil(tiles / 2) (single), segment bound)
-// One CTA per unit, four CTAs per SM (64 registers, a single record stage): measured on B200 at the OLMoE
-// shape this beats the persistent kernel below (three CTAs per SM, 80 registers, records of the next unit
-// prefetched) by 16 % per launch at batch 128 - the kernel is bound by instruction issue, and a fourth
-// resident CTA hides more latency than the prefetch does; five CTAs (48 registers, spills) are slower.
-// CACHE: single-chunk projections keep their unpacked weights in registers across the row passes of a
-// segment (64 more registers: two CTAs per SM) - the variant for prefill-sized segments.
-template <int NT, int MODE, bool CACHE>
-__global__ void __launch_bounds__(kThreads, CACHE ? 2 : 4) grouped_tiled_kernel(const __grid_constant__ TiledArgs args) {
-  constexpr bool DUAL = MODE != MODE_SINGLE;
-  constexpr int NH = DUAL ? 2 : 1;
-  extern __shared__ uint4 smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);
-  const SmemLayout L = smem_layout(args.rec_slot_bytes, args.col_slot_bytes, args.sal_slots, NH, NT, 1);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm);  // [0] records, [1] activation rows
-  uint8_t* rec_base = sm + 64;
-  uint8_t* col_base = rec_base + 2 * args.rec_slot_bytes;
-  uint32_t* gmap_base = reinterpret_cast<uint32_t*>(sm + L.gmap_off);
-  uint8_t* hsal = sm + L.hsal_off;
-  uint8_t* hrows = sm + L.hrows_off;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    mbar_init(&mbar[0], 2);
-    mbar_init(&mbar[1], kWarps);
-    fence_mbar_init();
-  }
-  reinterpret_cast<uint4*>(gmap_base)[tid] = make_uint4(0u, 0u, 0u, 0u);  // both g_map planes, for the first chunk
-  __syncthreads();
-  // Activations come from the predecessor kernel; the route arrays too, unless the caller says
-  // they are older, in which case the weight staging below overlaps the predecessor.
-  bool waited = false;
-  if (!args.weights_before_wait) {
-    pdl_wait();
-    pdl_launch_dependents();
-    waited = true;
-  }
-  const int seg = blockIdx.y;
-  const UnitRoute unit = load_unit_route(args, seg);
-  const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
-  // Row split: CTA z of a unit takes the row passes z, z + gridDim.z, ... of its segment (the launcher
-  // splits when there are fewer units than CTA slots); a CTA without a pass leaves at once.
-  // (Only the register-cached kernel is launched with gridDim.z > 1.)
-  const int row_first = unit.row_begin + (CACHE ? static_cast<int>(blockIdx.z) * (NT * 8) : 0);
-  const int row_step = (CACHE ? static_cast<int>(gridDim.z) : 1) * (NT * 8);
-  if (seg >= nseg || !unit_live(args, unit) || row_first >= unit.row_end) return;
-  const int expert = unit.expert;
-
-  const int r = warp >> 2, og = warp & 3;  // record and 16-output group of this warp
-  const int tiles = tiles_per_expert(args.proj[0].out_features);
-  const int tile0 = DUAL ? static_cast<int>(blockIdx.x) : 2 * static_cast<int>(blockIdx.x);
-  const bool tile_valid = tile0 + (DUAL ? 0 : r) < tiles;
-  const int rank = args.proj[0].rank;
-  const int chunks = num_chunks(rank);
-  const bool lane_order = args.hidden_lane_order != 0;
-
-  StagedTile st;
-  st.rec = rec_base + r * args.rec_slot_bytes;
-  st.col = col_base + (DUAL ? r : 0) * args.col_slot_bytes;
-  st.gmap = gmap_base + r * 512;
-  const uint8_t* hrows_set = hrows + (DUAL ? r : 0) * NT * 8 * kHiddenRowBytes;
-  const uint8_t* hsal_set = hsal + (DUAL ? r : 0) * args.sal_slots * NT * 8 * 64;
-  auto col_of = [&](int set) { return static_cast<const uint8_t*>(col_base + set * args.col_slot_bytes); };
-
-  int staged_chunk = -1;
-  uint32_t par_w = 0u, par_h = 0u;
-  bool dead = false;
-  uint32_t a_cache[CACHE ? kChunkRows : 1][2][4];
-  int cached_rows = -1;  // packed rows held in a_cache once the chunk has been unpacked
-  for (int r0 = row_first; r0 < unit.row_end; r0 += row_step) {
-    const int rows = min(NT * 8, unit.row_end - r0);
-    const int nt_count = (rows + 7) >> 3;
-    float acc[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[nt][c] = 0.f;
-    auto row_src = [&](int n) { return args.row_gather ? args.row_gather[r0 + n] : (r0 + n); };
-
-    for (int kc = 0; kc < chunks; ++kc) {
-      const int p0 = kc * kChunkRows;
-      // the first chunk of a unit starts right behind the set-up barrier (planes already zeroed there)
-      const bool first_iter = staged_chunk < 0;
-      if (!first_iter) __syncthreads();  // earlier consumers of the staging buffers are done
-      if (dead) break;
-      const bool need_w = staged_chunk != kc;
-      if (need_w) {
-        if (lane == 0 && warp < 2) {
-          const int rr = warp;
-          const TrisProjView& v = args.proj[DUAL ? rr : 0];
-          const int tl = tile0 + (DUAL ? 0 : rr);
-          const bool valid = tl < tiles;
-          const uint2 d = valid ? load_desc(v, expert, tl, kc) : make_uint2(0u, 0u);
-          issue_record(v, expert, kc, d, rec_base + rr * args.rec_slot_bytes,
-                       (DUAL || rr == 0) ? col_base + rr * args.col_slot_bytes : nullptr, valid, &mbar[0]);
-        }
-        if (!first_iter) reinterpret_cast<uint4*>(gmap_base)[tid] = make_uint4(0u, 0u, 0u, 0u);  // 256 threads x 16 B = both planes
-      }
-      if (waited) issue_hidden<NT, NH>(hrows, args.hidden, rank, p0, rows, lane_order, args.hidden_stride, &mbar[1], row_src, args.col_scale);
-      bool ok = true;
-      if (need_w) {
-        if (!first_iter) __syncthreads();  // planes zeroed
-        ok = mbar_wait_bounded(&mbar[0], par_w);
-        par_w ^= 1u;
-        if (ok && tile_valid) gr_decode_block(st.rec, og, const_cast<uint32_t*>(st.gmap), lane);
-        staged_chunk = kc;
-      }
-      if (!waited) {  // first pass of a CTA that staged its weights ahead of the predecessor's end
-        pdl_wait();
-        pdl_launch_dependents();
-        waited = true;
-        issue_hidden<NT, NH>(hrows, args.hidden, rank, p0, rows, lane_order, args.hidden_stride, &mbar[1], row_src, args.col_scale);
-      }
-      ok = mbar_wait_bounded(&mbar[1], par_h) && ok;
-      par_h ^= 1u;
-      if (__syncthreads_or(!ok)) {  // also publishes the decoded planes, re-ordered rows and column records
-        mbar_wait_bounded(&mbar[0], par_w ^ 1u);  // copies that may still be in flight
-        mbar_wait_bounded(&mbar[1], par_h ^ 1u);
-        if (tid == 0 && args.status) atomicExch(args.status, TRIS_ERR_TIMEOUT);
-        dead = true;
-        break;
-      }
-      gather_salient<NT, NH>(hsal, hrows, rows, args.sal_slots, col_of);
-      __syncthreads();
-      if (tile_valid) {
-        if constexpr (CACHE) {
-          if (chunks == 1) {
-            if (cached_rows < 0) cached_rows = unpack_chunk_ns(st, og * 16, lane, a_cache);
-            main_chunk_cached<NT>(st, a_cache, cached_rows, hrows_set, hsal_set, og * 16, lane, nt_count, acc);
-          } else {
-            main_chunk<NT>(st, hrows_set, hsal_set, og * 16, lane, nt_count, acc);
-          }
-        } else {
-          main_chunk<NT>(st, hrows_set, hsal_set, og * 16, lane, nt_count, acc);
-        }
-      }
+// Ring position: index and the parity of its current round.
+struct Ring {
+  int i = 0;
+  uint32_t phase = 0u;
+  __device__ __forceinline__ Ring at(int ahead, int n) const {  // ahead < n
+    Ring r = *this;
+    r.i += ahead;
+    if (r.i >= n) {
+      r.i -= n;
+      r.phase ^= 1u;
     }
-    if (dead) continue;
-    finish_rows<NT, MODE>(args, hrows, r, og, tile_valid, expert, tile0, r0, rows, nt_count, acc);
+    return r;
   }
-}
-
-// ---- persistent CTAs, records of the next unit prefetched (projections of one chunk) -----------------
-// grid (CTAs); unit u = segment * units_x + x, x = output tile (dual) or pair of tiles (single)
-template <int NT, int MODE>
-__global__ void __launch_bounds__(kThreads, 3) grouped_tiled_persistent_kernel(const __grid_constant__ TiledArgs args) {
-  constexpr bool DUAL = MODE != MODE_SINGLE;
-  constexpr int NH = DUAL ? 2 : 1;
-  extern __shared__ uint4 smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);
-  const SmemLayout L = smem_layout(args.rec_slot_bytes, args.col_slot_bytes, args.sal_slots, NH, NT, 2);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm);  // [0], [1] records of the two stages, [2] activation rows
-  uint32_t* gmap_base = reinterpret_cast<uint32_t*>(sm + L.gmap_off);
-  uint8_t* hsal = sm + L.hsal_off;
-  uint8_t* hrows = sm + L.hrows_off;
-  auto stage_rec = [&](int stage, int rr) { return sm + 64 + stage * L.stage_bytes + rr * args.rec_slot_bytes; };
-  auto stage_col = [&](int stage, int set) { return sm + 64 + stage * L.stage_bytes + 2 * args.rec_slot_bytes + set * args.col_slot_bytes; };
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    mbar_init(&mbar[0], 2);
-    mbar_init(&mbar[1], 2);
-    mbar_init(&mbar[2], kWarps);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  bool waited = false;
-  if (!args.weights_before_wait) {
-    pdl_wait();
-    pdl_launch_dependents();
-    waited = true;
-  }
-  const int tiles = tiles_per_expert(args.proj[0].out_features);
-  const int units_x = DUAL ? tiles : (tiles + 1) / 2;
-  const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
-  const int total = nseg * units_x;
-  const int G = gridDim.x;
-  int u = blockIdx.x;
-  if (u >= total) {
-    if (!waited) {
-      pdl_wait();
-      pdl_launch_dependents();
+  __device__ __forceinline__ void advance(int n) {
+    if (++i == n) {
+      i = 0;
+      phase ^= 1u;
     }
+  }
+};
+
+// One chunk of a pass's activation rows; src[n] = source row of row n.  A warp covers 8 rows x 4 pieces of
+// 16 bytes: 64 contiguous source bytes per row, conflict-free writes.  Rows that can be copied as they are
+// go by cp.async, anything else element by element; columns past the matrix read as zeros up to a
+// multiple of 16.
+template <int N>
+__device__ __forceinline__ void stage_rows(const TiledArgs& args, uint8_t* dst, const __half* hidden, const int* src, int rows, int c0, int tid) {
+  const int piece = (tid >> 5) * 4 + ((tid >> 3) & 3);
+  const int cols = min(kChunkCols, args.rank - c0), left = cols - 8 * piece;  // columns of this piece that exist
+  if (left <= -8 || (left <= 0 && !(cols & 15))) return;
+  uint8_t* d = dst + (piece * N + (tid & 7)) * 16;
+  if (args.hidden_vec) {
+    const __half* from = hidden + (left > 0 ? c0 + 8 * piece : 0);
+#pragma unroll 2
+    for (int n = tid & 7; n < rows; n += 8, d += 128)
+      cp_async_16(d, from + static_cast<size_t>(src[n]) * args.hidden_stride, left > 0);
     return;
   }
-  const int r = warp >> 2, og = warp & 3;
-  const int rank = args.proj[0].rank;
-  const bool lane_order = args.hidden_lane_order != 0;
-  const bool issuer = lane == 0 && warp < 2;  // fetches record `warp` of every unit
-  const TrisProjView& iv = args.proj[DUAL ? (warp & 1) : 0];
-
-  auto tile_of = [&](int unit, int rr) { const int x = unit % units_x; return DUAL ? x : 2 * x + rr; };
-  auto fetch = [&](int unit, int expert, uint2 d, int stage) {  // issuer only
-    const int rr = warp;
-    const bool valid = tile_of(unit, rr) < tiles && expert >= 0 && expert < args.proj[0].num_experts;
-    issue_record(iv, expert, 0, d, stage_rec(stage, rr), (DUAL || rr == 0) ? stage_col(stage, rr) : nullptr, valid, &mbar[stage]);
-  };
-  auto desc_of = [&](int unit, int expert) {  // issuer only
-    const int tl = tile_of(unit, warp);
-    if (tl >= tiles || expert < 0 || expert >= args.proj[0].num_experts) return make_uint2(0u, 0u);
-    return load_desc(iv, expert, tl, 0);
-  };
-
-  // pipeline fill: unit u in flight, descriptor of u + G and expert of u + 2G in registers
-  UnitRoute cur = load_unit_route(args, u / units_x);
-  int e1 = -1, e2 = -1;
-  uint2 d1 = make_uint2(0u, 0u);
-  if (issuer) {
-    fetch(u, cur.expert, desc_of(u, cur.expert), 0);
-    if (u + G < total) {
-      e1 = args.expert_ids[(u + G) / units_x];
-      d1 = desc_of(u + G, e1);
-    }
-    if (u + 2 * G < total) e2 = args.expert_ids[(u + 2 * G) / units_x];
+#pragma unroll 1
+  for (int n = tid & 7; n < rows; n += 8, d += 128) {
+    *reinterpret_cast<uint4*>(d) = read_piece(args, hidden + c0 + static_cast<size_t>(src[n]) * args.hidden_stride, c0, piece, left);
   }
-  UnitRoute nxt = cur;
-  if (u + G < total) nxt = load_unit_route(args, (u + G) / units_x);
+}
 
-  uint32_t par_h = 0u;
-  bool dead = false;
-  for (int it = 0;; ++it) {
-    const int stage = it & 1;
-    __syncthreads();  // the previous unit is finished: its stage, the planes and the activation rows are free
-    if (issuer) {
-      if (u + G < total) fetch(u + G, e1, d1, stage ^ 1);
-      e1 = e2;
-      d1 = (u + 2 * G < total) ? desc_of(u + 2 * G, e1) : make_uint2(0u, 0u);
-      e2 = (u + 3 * G < total) ? args.expert_ids[(u + 3 * G) / units_x] : -1;
+// Activations of the salient steps of one column record, [step * 2 + half][N rows][16 B].
+template <int N>
+__device__ __forceinline__ void gather_salient(uint8_t* dst, const uint8_t* rows_smem, const uint8_t* col, int rows, int tid) {
+  const int items = reinterpret_cast<const ColHeader*>(col)->num_steps * 2 * N;
+  for (int i = tid; i < items; i += kLoadWarps * 32) {
+    const int n = i & (N - 1), kq = i / N;
+    if (n >= rows) continue;
+    const uint4 cols = *reinterpret_cast<const uint4*>(col + kColHdrBytes + kColTabBytes + (kq >> 1) * kColStepBytes + 64 + (kq & 1) * 16);
+    const uint8_t* base = rows_smem + n * 16;
+    auto ld = [&](uint32_t c) -> uint32_t { return *reinterpret_cast<const uint16_t*>(base + (c & ~7u) * (N * 2) + (c & 7u) * 2); };
+    auto pair = [&](uint32_t cc) { return ld(cc & 0xFFFFu) | (ld(cc >> 16) << 16); };
+    *reinterpret_cast<uint4*>(dst + i * 16) = make_uint4(pair(cols.x), pair(cols.y), pair(cols.z), pair(cols.w));
+  }
+}
+
+// N: activation rows per pass (the accumulators' TMEM columns).  A longer segment takes several
+// passes and unpacks its weights again for each.
+template <int N, int MODE>
+__global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(const __grid_constant__ TiledArgs args) {
+  using W = Roles<N>;
+  constexpr bool DUAL = MODE != MODE_SINGLE;
+  constexpr int NC = DUAL ? 2 : 1;
+  constexpr int kDBufs = (512 - kDBase) / (2 * N) < 4 ? (512 - kDBase) / (2 * N) : 4;
+  extern __shared__ uint4 smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);
+  uint64_t* rows_full = reinterpret_cast<uint64_t*>(sm);   // loader -> MMA
+  uint64_t* rows_empty = rows_full + kMaxStages;           // MMA (commits of both warps) -> loader
+  uint64_t* a_full = rows_empty + kMaxStages;              // [warpgroup * 2 + slot] unpack warps -> MMA
+  uint64_t* a_empty = a_full + 8;                          // MMA (commit) -> unpack
+  uint64_t* d_full = a_empty + 8;                          // MMA (commit) -> epilogue
+  uint64_t* d_empty = d_full + 4;                          // epilogue warps -> MMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 4);
+  int* src_rows = reinterpret_cast<int*>(sm + kBarBytes);  // [2][N] source rows of a pass, by pass parity
+  uint8_t* stage_base = sm + kBarBytes + kRowIdxBytes;
+
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kMaxStages; ++i) {
+      mbar_init(&rows_full[i], kLoadWarps);
+      mbar_init(&rows_empty[i], 2);
     }
-    const bool live = unit_live(args, cur);
-    const int expert = cur.expert;
-    const int tile0 = tile_of(u, 0);
-    const bool tile_valid = tile0 + (DUAL ? 0 : r) < tiles;
-    StagedTile st;
-    st.rec = stage_rec(stage, r);
-    st.col = stage_col(stage, DUAL ? r : 0);
-    st.gmap = gmap_base + r * 512;
-    const uint8_t* hrows_set = hrows + (DUAL ? r : 0) * NT * 8 * kHiddenRowBytes;
-    const uint8_t* hsal_set = hsal + (DUAL ? r : 0) * args.sal_slots * NT * 8 * 64;
-    auto col_of = [&](int set) { return static_cast<const uint8_t*>(stage_col(stage, set)); };
+    for (int i = 0; i < 8; ++i) {
+      mbar_init(&a_full[i], 4);
+      mbar_init(&a_empty[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&d_full[i], 2);
+      mbar_init(&d_empty[i], W::kEpiWarps);
+    }
+    fence_mbar_init();
+  }
+  if (warp == W::kMma0) tmem_alloc(tmem_slot, 512);  // before the dependents may start: they allocate too
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = warp_uniform(*tmem_slot);
+  const StageLayout L = stage_layout(args.max_steps, NC, args.num_sets, N);
+  bool ok = true;
 
-    reinterpret_cast<uint4*>(gmap_base)[tid] = make_uint4(0u, 0u, 0u, 0u);
-    int r0 = cur.row_begin;
-    int rows = live ? min(NT * 8, cur.row_end - r0) : 0;
-    auto row_src = [&](int n) { return args.row_gather ? args.row_gather[r0 + n] : (r0 + n); };
-    if (waited && live) issue_hidden<NT, NH>(hrows, args.hidden, rank, 0, rows, lane_order, args.hidden_stride, &mbar[2], row_src, args.col_scale);
-    __syncthreads();  // planes zeroed
-    bool ok = mbar_wait_bounded(&mbar[stage], (it >> 1) & 1);
-    if (ok && live && tile_valid) gr_decode_block(st.rec, og, const_cast<uint32_t*>(st.gmap), lane);
-    if (!waited) {
+  // The route and the activations come from earlier kernels.  When the route is older than the
+  // predecessor, only the loader waits for it, so weights unpack while the predecessor still runs.
+  if (!args.weights_before_wait) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+  Walker<N> w;
+
+  if (warp < kUnpackWarps) {
+    // ---- unpack ---------------------------------------------------------------------------------
+    const int wg = warp >> 2, r = wg & 1, row = threadIdx.x & 127;
+    const TrisProjView& v = args.proj[DUAL ? r : 0];
+    const int max_sal = v.max_sal_words, rec_bytes = v.max_record_bytes, col_bytes = v.col_record_bytes;
+    const int sal_off = record_slices(args.rank) * kSliceBytes, rows_off = sal_off + max_sal * kStepBytes;
+    const uint32_t tmem_a = tmem + wg * (2 * kACols) + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    uint64_t* my_full = a_full + wg * 2;
+    uint64_t* my_empty = a_empty + wg * 2;
+    Ring slot;
+    w.start(args);
+    if (wg >> 1 && w.valid()) w.next(args);  // warpgroups 2 and 3 take the odd items
+    // The column record is the same for all rows: broadcast loads through L1, where the other warps of the
+    // SM find it too.  It and the first loads of the thread's own row are requested one item ahead.
+    int nrec = -1, ncol = 0;  // record numbers
+    uint32_t touched = 0u;    // one line of the next column record per lane: a load that only brings it to L1
+    uint4 ncodes = make_uint4(0u, 0u, 0u, 0u);
+    uint2 nscale = make_uint2(0u, 0u);
+    auto record = [&](int i) { return static_cast<const uint8_t*>(v.tile_records) + static_cast<size_t>(i) * static_cast<size_t>(rec_bytes); };
+    auto column_record = [&](int i) { return static_cast<const uint8_t*>(v.col_records) + static_cast<size_t>(i) * static_cast<size_t>(col_bytes); };
+    auto fetch = [&]() {
+      const int tile = DUAL ? w.x : 2 * w.x + r;
+      nrec = -1;
+      if (!w.valid() || tile >= args.tiles) return;
+      ncol = w.expert * args.chunks + w.c;
+      nrec = (w.expert * args.tiles + tile) * args.chunks + w.c;
+      const uint8_t* rec = record(nrec);
+      if (lane * 128 < col_bytes) touched = __ldg(reinterpret_cast<const uint32_t*>(column_record(ncol) + lane * 128));
+      ncodes = ldg_stream(rec + row * 16);
+      nscale = __ldg(reinterpret_cast<const uint2*>(rec + rows_off) + row);
+    };
+    fetch();
+    while (ok && w.valid()) {
+      asm volatile("" ::"r"(touched));
+      const int irec = nrec;
+      const uint8_t* col = column_record(ncol);
+      const int slices = (min(kChunkCols, args.rank - w.c * kChunkCols) + kSliceCols - 1) / kSliceCols;
+      uint4 codes = ncodes, codes1 = ncodes;
+      const uint2 rp0 = nscale;
+      uint32_t sw0 = 0u, sw1 = 0u;
+      if (irec >= 0) {
+        const uint8_t* rec = record(irec);
+        if (slices > 1) codes1 = ldg_stream(rec + kSliceBytes + row * 16);
+        if (max_sal > 0) sw0 = __ldg(reinterpret_cast<const uint32_t*>(rec + sal_off) + row);
+        if (max_sal > 1) sw1 = __ldg(reinterpret_cast<const uint32_t*>(rec + sal_off + kStepBytes) + row);
+      }
+      w.next(args);
+      if (w.valid()) w.next(args);
+      fetch();
+      if (irec < 0) continue;
+      const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(col));  // ColHeader: counts, slots of the packed rows, slots of the steps
+      const uint32_t step_hi = __ldg(reinterpret_cast<const uint32_t*>(col) + 4);
+      auto slot_scales = [&](uint32_t sl) {
+        return sl == 0u ? rp0 : __ldg(reinterpret_cast<const uint2*>(record(irec) + rows_off + sl * kSlotBytes) + row);
+      };
+      auto publish = [&]() {
+        tmem_wait_st();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&my_full[slot.i]);
+        slot.advance(2);
+      };
+      auto wait_slot = [&]() {
+        ok = mbar_wait_warp(&my_empty[slot.i], slot.phase ^ 1u) && ok;
+        tcgen05_fence_after();
+      };
+      const uint4* ct = reinterpret_cast<const uint4*>(col + kColHdrBytes);
+      uint32_t row_slots = hdr.z;
+#pragma unroll 1
+      for (int s = 0; s < slices; ++s) {
+        wait_slot();
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {  // rolled: the unpack of 32 columns is the loop body the instruction cache holds
+          const RowScales rs = row_scales_ns(slot_scales(row_slots & 0xFFu));
+          row_slots >>= 8;
+          uint32_t a[16];
+          unpack_word(codes.x, ct, rs, a);
+          unpack_word(codes.y, ct + 1, rs, a + 8);
+          tmem_st<16>(tmem_a + slot.i * kACols + h * 16, a);
+          codes.x = codes.z;
+          codes.y = codes.w;
+          ct += 2;
+        }
+        ct += 12;
+        codes = codes1;
+        publish();
+      }
+      const int steps = static_cast<int>((hdr.y >> 8) & 0xFFu);
+      uint32_t step_slots = hdr.w;
+      const uint8_t* ent = col + kColHdrBytes + kColTabBytes;
+#pragma unroll 1
+      for (int b = 0; b < steps; b += 4) {
+        wait_slot();
+#pragma unroll 1
+        for (int st = b; st < min(steps, b + 4); ++st) {
+          const uint32_t code = st == 0 ? sw0 : (st == 1 ? sw1 : __ldg(reinterpret_cast<const uint32_t*>(record(irec) + sal_off + st * kStepBytes) + row));
+          uint32_t a[8];
+          unpack_step(code, reinterpret_cast<const uint4*>(ent), slot_scales(step_slots & 0xFFu), a);
+          tmem_st<8>(tmem_a + slot.i * kACols + (st - b) * 8, a);
+          step_slots >>= 8;
+          ent += kColStepBytes;
+        }
+        step_slots = step_hi;
+        publish();
+      }
+    }
+  } else if (warp < W::kLoad0) {
+    // ---- epilogue -------------------------------------------------------------------------------
+    const int e = (warp - W::kEpi0) >> 2;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t d_lane = tmem + kDBase + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    Ring buf;
+    for (w.start(args); w.valid(); w.next_tile(args)) {
+      const int rows = w.rows(), expert = w.expert;
+      const uint32_t d = d_lane + buf.i * (2 * N);
+      ok = mbar_wait_warp<64>(&d_full[buf.i], buf.phase);
+      if (!ok) break;
+      tcgen05_fence_after();
+      auto load_out = [&](int which, int tile, int n0, float (&y)[8]) {  // scaled and biased
+        tmem_ld<8>(d + which * N + n0, y);
+        tmem_wait_ld();
+        const TrisProjView& pv = args.proj[DUAL ? which : 0];
+        if (pv.output_scale || pv.bias) {
+          const int o = min(tile * kTileOut + row, args.out_features - 1);
+          const size_t at = static_cast<size_t>(expert) * args.out_features + o;
+          const float scale = pv.output_scale ? __half2float(static_cast<const __half*>(pv.output_scale)[at]) : 1.f;
+          const float bias = pv.bias ? __half2float(static_cast<const __half*>(pv.bias)[at]) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) y[j] = y[j] * scale + bias;
+        }
+      };
+      if constexpr (MODE == MODE_DUAL_SILU) {
+#pragma unroll 1
+        for (int n0 = e * 8; n0 < rows; n0 += 2 * W::kEpiWarps) {
+          float g[8], up[8];
+          load_out(0, w.x, n0, g);
+          load_out(1, w.x, n0, up);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) g[j] = __fdividef(g[j], 1.f + __expf(-g[j])) * up[j];
+          store_rows<8>(args, args.out[0], w.x * kTileOut + row, w.r0, n0, rows, g);
+        }
+      } else {
+#pragma unroll 1
+        for (int r = e; r < 2; r += W::kEpiWarps / 4) {
+          const int tile = DUAL ? w.x : 2 * w.x + r;
+          if (tile >= args.tiles) break;
+#pragma unroll 1
+          for (int n0 = 0; n0 < rows; n0 += 8) {
+            float y[8];
+            load_out(r, tile, n0, y);
+            store_rows<8>(args, args.out[DUAL ? r : 0], tile * kTileOut + row, w.r0, n0, rows, y);
+          }
+        }
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&d_empty[buf.i]);
+      buf.advance(kDBufs);
+    }
+  } else if (warp < W::kMma0) {
+    // ---- loader ---------------------------------------------------------------------------------
+    const int tid = threadIdx.x - W::kLoad0 * 32;
+    bool waited = !args.weights_before_wait;
+    int next_src = 0, pass = 0;  // this thread's source row of the pass the walker has reached; that pass's parity
+    auto find_row = [&]() {
+      if (w.valid() && tid < w.rows()) next_src = args.row_gather ? __ldg(args.row_gather + w.r0 + tid) : w.r0 + tid;
+    };
+    auto keep_row = [&]() { if (tid < N) src_rows[pass * N + tid] = next_src; };
+    uint32_t rows_of = 0u;  // rows of the items in flight, oldest in the low byte
+    const int ahead = args.stages - 1;
+    Ring put, get;
+    auto put_item = [&]() {
+      if (w.valid()) {
+        ok = mbar_wait_warp<32>(&rows_empty[put.i], put.phase ^ 1u) && ok;
+        uint8_t* base = stage_base + put.i * L.total;
+#pragma unroll 1
+        for (int p = 0; p < NC; ++p) {
+          const TrisProjView& pv = args.proj[p];
+          const uint8_t* src = static_cast<const uint8_t*>(pv.col_records) + static_cast<size_t>(w.expert * args.chunks + w.c) * pv.col_record_bytes;
+          for (int i = tid * 16; i < pv.col_record_bytes; i += kLoadWarps * 32 * 16) cp_async_16(base + p * L.col_bytes + i, src + i);
+        }
+        if (!waited) {
+          pdl_wait();
+          pdl_launch_dependents();
+          waited = true;
+        }
+#pragma unroll 1
+        for (int s = 0; s < args.num_sets; ++s)
+          stage_rows<N>(args, base + L.rows_off + s * L.rows_bytes, args.hidden[s], src_rows + pass * N, w.rows(), w.c * kChunkCols, tid);
+        rows_of |= static_cast<uint32_t>(w.rows()) << (8 * ahead);
+        w.next_stage(args);
+        if (w.c == 0) {
+          pass ^= 1;
+          find_row();
+        }
+        put.advance(args.stages);
+      }
+      cp_async_commit();
+      rows_of >>= 8;
+    };
+    w.start(args);
+    if (args.weights_before_wait && args.row_gather) {  // the gather list may come from the predecessor
       pdl_wait();
       pdl_launch_dependents();
       waited = true;
-      if (live) issue_hidden<NT, NH>(hrows, args.hidden, rank, 0, rows, lane_order, args.hidden_stride, &mbar[2], row_src, args.col_scale);
     }
-    for (; live;) {
-      const int nt_count = (rows + 7) >> 3;
-      ok = mbar_wait_bounded(&mbar[2], par_h) && ok;
-      par_h ^= 1u;
-      if (__syncthreads_or(!ok)) {  // also publishes the decoded planes and re-ordered rows
-        mbar_wait_bounded(&mbar[2], par_h ^ 1u);
-        dead = true;
+    find_row();
+    for (int i = 0; i < ahead; ++i) {
+      keep_row();
+      named_barrier_sync(1, kLoadWarps * 32);
+      put_item();
+    }
+    while (rows_of & 0xFFu) {
+      keep_row();
+      if (ahead == 1) cp_async_wait<0>();
+      else if (ahead == 2) cp_async_wait<1>();
+      else cp_async_wait<2>();
+      // every loader thread's copies of this item have landed (and the loader warps leave together)
+      if (named_barrier_or(1, kLoadWarps * 32, !ok)) {
+        ok = false;
         break;
       }
-      gather_salient<NT, NH>(hsal, hrows, rows, args.sal_slots, col_of);
-      __syncthreads();
-      float acc[NT][4];
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[nt][c] = 0.f;
-      if (tile_valid) main_chunk<NT>(st, hrows_set, hsal_set, og * 16, lane, nt_count, acc);
-      finish_rows<NT, MODE>(args, hrows, r, og, tile_valid, expert, tile0, r0, rows, nt_count, acc);
-      r0 += NT * 8;
-      if (r0 >= cur.row_end) break;
-      rows = min(NT * 8, cur.row_end - r0);
-      __syncthreads();  // the stores have read the scratch: the activation rows can be refilled
-      issue_hidden<NT, NH>(hrows, args.hidden, rank, 0, rows, lane_order, args.hidden_stride, &mbar[2], row_src, args.col_scale);
+      uint8_t* base = stage_base + get.i * L.total;
+      const int rows = static_cast<int>(rows_of & 0xFFu);
+#pragma unroll 1
+      for (int p = 0; p < NC; ++p)
+        gather_salient<N>(base + L.sal_off + p * L.sal_bytes, base + L.rows_off + (args.num_sets == 2 ? p : 0) * L.rows_bytes,
+                          base + p * L.col_bytes, rows, tid);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&rows_full[get.i]);
+      get.advance(args.stages);
+      put_item();
     }
-    if (__syncthreads_or(dead || !ok)) {
-      if (u + G < total) mbar_wait_bounded(&mbar[stage ^ 1], ((it + 1) >> 1) & 1);  // the prefetch in flight
-      if (tid == 0 && args.status) atomicExch(args.status, TRIS_ERR_TIMEOUT);
-      return;
+    if (!waited) {
+      pdl_wait();
+      pdl_launch_dependents();
     }
-    u += G;
-    if (u >= total) return;
-    cur = nxt;
-    if (u + G < total) nxt = load_unit_route(args, (u + G) / units_x);
+    cp_async_wait<0>();
+  } else {
+    // ---- MMA ------------------------------------------------------------------------------------
+    // A whole warp walks the items; one lane issues.  K steps of a full slice are unrolled: the operands of
+    // an MMA live in uniform registers, and moving them there one by one costs more than the MMA.
+    const int r = warp - W::kMma0;
+    Ring stage, buf, slot0, slot1;
+    uint32_t item = 0u;
+    for (w.start(args); ok && w.valid(); ++item) {
+      const int rows = w.rows(), cols = min(kChunkCols, args.rank - w.c * kChunkCols);
+      const bool first = w.c == 0, last = w.c + 1 == args.chunks;
+      const bool mine = DUAL || 2 * w.x + r < args.tiles, last_tile = w.x + 1 == w.x_end;
+      const Ring at_stage = args.reuse ? stage.at(w.c, args.stages) : stage;
+      w.next(args);  // its route loads overlap the waits below
+      const uint32_t idesc = umma_idesc_f16(kTileOut, (rows + 15) & ~15);
+      const uint32_t d = tmem + kDBase + buf.i * (2 * N) + r * N;
+      ok = mbar_wait_warp(&rows_full[at_stage.i], at_stage.phase);
+      if (ok && first) ok = mbar_wait_warp(&d_empty[buf.i], buf.phase ^ 1u);
+      if (!ok) break;
+      const uint8_t* base = stage_base + at_stage.i * L.total;
+      const int wg = static_cast<int>(item & 1u) * 2 + r;
+      Ring sl = (item & 1u) ? slot1 : slot0;
+      // one slot of weights: `n` K = 16 steps against the activations at b_addr
+      auto consume = [&](int n, uint32_t b_addr, uint32_t accumulate) {
+        const int at = wg * 2 + sl.i;
+        ok = mbar_wait_warp(&a_full[at], sl.phase) && ok;
+        tcgen05_fence_after();
+        const uint64_t desc = umma_smem_desc(b_addr, N * 16, 128);
+        const uint32_t a = tmem + at * kACols;
+        if (elect_one()) {
+          umma_f16_ts(d, a, desc, idesc, accumulate);
+          if (n == 4) {
+#pragma unroll
+            for (int j = 1; j < 4; ++j) umma_f16_ts(d, a + 8 * j, desc + j * (2 * N), idesc, 1u);
+          } else {
+            for (int j = 1; j < n; ++j) umma_f16_ts(d, a + 8 * j, desc + j * (2 * N), idesc, 1u);
+          }
+          umma_commit(&a_empty[at]);
+        }
+        sl.advance(2);
+      };
+      if (mine) {
+        const uint32_t b_rows = smem_u32(base + L.rows_off + (args.num_sets == 2 ? r : 0) * L.rows_bytes);
+        for (int s = 0; s * kSliceCols < cols && ok; ++s)
+          consume(min(kSliceCols / 16, (cols - s * kSliceCols + 15) >> 4), b_rows + s * (8 * N * 16), first && s == 0 ? 0u : 1u);
+        const int p = DUAL ? r : 0;
+        const int steps = warp_uniform(reinterpret_cast<const ColHeader*>(base + p * L.col_bytes)->num_steps);
+        const uint32_t b_sal = smem_u32(base + L.sal_off + p * L.sal_bytes);
+        for (int b = 0; b < steps && ok; b += 4) consume(min(4, steps - b), b_sal + b * (2 * N * 16), 1u);
+      }
+      if (item & 1u) slot1 = sl;
+      else slot0 = sl;
+      if (elect_one()) {
+        if (last_tile) umma_commit(&rows_empty[at_stage.i]);
+        if (last) umma_commit(&d_full[buf.i]);
+      }
+      if (last) buf.advance(kDBufs);
+      if (!args.reuse) stage.advance(args.stages);
+      else if (last && last_tile) stage = stage.at(args.chunks, args.stages);
+    }
   }
+  if (!ok && args.status) atomicExch(args.status, TRIS_ERR_TIMEOUT);
+  __syncwarp();
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  if (warp == W::kMma0) tmem_dealloc(tmem, 512);
 }
 
-// ---- dump kernel: decoded g_map words and dequantised weights from the records --------------------
-// grid (tiles, chunks, E); dense_out [E, pr, O] and weights_out [E, O, rank] may each be null
-__global__ void __launch_bounds__(kThreads) tiled_dump_kernel(TrisProjView v, int32_t* dense_out, __half* weights_out,
-                                                              int rec_slot_bytes, int32_t* status) {
+// ---- dump kernel: dequantised weights from the records -----------------------------------------------
+// grid (tiles, chunks, E), 128 threads; weights_out [E, O, rank]
+__global__ void __launch_bounds__(kTileOut) tiled_dump_kernel(TrisProjView v, __half* weights_out) {
   extern __shared__ uint4 smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm);
-  uint8_t* rec = sm + 64;
-  uint8_t* col = rec + rec_slot_bytes;
-  uint32_t* gmap = reinterpret_cast<uint32_t*>(col + v.col_record_bytes);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x, chunk = blockIdx.y, e = blockIdx.z;
-  const int o0 = tile * kTileOut, p0 = chunk * kChunkRows;
-  const int pr = (v.rank + 31) >> 5;
-  if (tid == 0) {
-    mbar_init(&mbar[0], 1);
-    fence_mbar_init();
-  }
+  uint8_t* col = reinterpret_cast<uint8_t*>(smem_raw);
+  const int row = threadIdx.x, tile = blockIdx.x, c = blockIdx.y, e = blockIdx.z;
+  const RecordGeom geo = record_geom(v);
+  const uint8_t* rec = tile_record(v, geo, e, tile, c);
+  const uint8_t* src = col_record(v, geo, e, c);
+  for (int i = row * 16; i < geo.col_bytes; i += kTileOut * 16) *reinterpret_cast<uint4*>(col + i) = *reinterpret_cast<const uint4*>(src + i);
   __syncthreads();
-  if (tid == 0) issue_record(v, e, chunk, load_desc(v, e, tile, chunk), rec, col, true, &mbar[0]);
-  if (tid < 128) reinterpret_cast<uint4*>(gmap)[tid] = make_uint4(0u, 0u, 0u, 0u);
-  __syncthreads();
-  const bool ok = mbar_wait_bounded(&mbar[0], 0u);
-  if (ok && warp < 4) gr_decode_block(rec, warp, gmap, lane);
-  if (__syncthreads_or(!ok)) {
-    mbar_wait_bounded(&mbar[0], 0u);
-    if (tid == 0 && status) atomicExch(status, TRIS_ERR_TIMEOUT);
-    return;
+  const int o = tile * kTileOut + row;
+  if (o >= v.out_features) return;
+  const ColHeader* hdr = reinterpret_cast<const ColHeader*>(col);
+  const int c0 = c * kChunkCols, cols = min(kChunkCols, v.rank - c0);
+  __half* out = weights_out + (static_cast<size_t>(e) * v.out_features + o) * v.rank + c0;
+  auto scales = [&](int slot) { return reinterpret_cast<const uint2*>(rec + geo.rows_off + slot * kSlotBytes)[row]; };
+  for (int w = 0; w < (cols + 15) / 16; ++w) {
+    uint32_t a[8];
+    unpack_word(reinterpret_cast<const uint32_t*>(rec + (w >> 2) * kSliceBytes + row * 16)[w & 3],
+                reinterpret_cast<const uint4*>(col + kColHdrBytes) + (w >> 2) * 16 + (w & 3), row_scales_ns(scales(hdr->slot_of_row[w >> 1])), a);
+    for (int i = 0; i < 16; ++i)
+      if (16 * w + i < cols) out[16 * w + i] = __ushort_as_half(static_cast<unsigned short>(a[i >> 1] >> (16 * (i & 1))));
   }
-  if (dense_out) {
-    for (int i = tid; i < kChunkRows * kTileOut; i += kThreads) {
-      const int p = i / kTileOut, o = i % kTileOut;
-      if (p0 + p < pr && o0 + o < v.out_features)
-        dense_out[(static_cast<size_t>(e) * pr + p0 + p) * v.out_features + o0 + o] = static_cast<int32_t>(gmap[i]);
-    }
-  }
-  if (!weights_out) return;
-  StagedTile st{rec, col, gmap};
-  const int g = lane >> 2, t = lane & 3;
-  const LaneShifts ls = lane_shifts(t);
-  auto store_pair = [&](int o, int col_lo, uint32_t bits) {
-    if (o >= v.out_features) return;
-    __half* row = weights_out + (static_cast<size_t>(e) * v.out_features + o) * v.rank;
-    const int ca = 32 * p0 + col_lo, cb = ca + 16;
-    if (ca < v.rank) row[ca] = __ushort_as_half(static_cast<unsigned short>(bits & 0xFFFFu));
-    if (cb < v.rank) row[cb] = __ushort_as_half(static_cast<unsigned short>(bits >> 16));
-  };
-  if (warp < 4) {
-    const ColHeader* ch = reinterpret_cast<const ColHeader*>(col);
-    int p = 0;
-    for (int slot = 0; slot < ch->num_slots; ++slot) {
-      const RowScalesNs rs = load_row_scales_ns(st, slot, warp * 16, lane);
-      for (; p < ch->slot_end[slot]; ++p) {
-        uint32_t a[2][4];
-        unpack_fragments_ns(st, p, warp * 16, lane, rs, ls, a);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) store_pair(o0 + warp * 16 + g + 8 * h, 32 * p + lane_pair_col(t, i), a[h][i]);
-      }
-    }
-  }
-  __syncthreads();  // the salient columns overwrite the +-0 the main unpack left there
-  if (warp < 4) {
-    const int sal_words = reinterpret_cast<const ColHeader*>(col)->sal_words;
-    for (int q = 0; q < sal_words; ++q) {
-      uint32_t a[2][4];
-      unpack_fragments_sal(st, q, warp * 16, lane, ls, a);
-      const uint16_t* salcol = reinterpret_cast<const uint16_t*>(col + kColHdrBytes + kColTabBytes + q * kSalEntryBytes + 192);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int o = o0 + warp * 16 + g + 8 * h;
-        if (o >= v.out_features) continue;
-        __half* row = weights_out + (static_cast<size_t>(e) * v.out_features + o) * v.rank;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int slot = lane_pair_col(t, i);
-          const unsigned c_lo = salcol[slot], c_hi = salcol[slot + 16];
-          if (c_lo != 0xFFFFu) row[32 * p0 + c_lo] = __ushort_as_half(static_cast<unsigned short>(a[h][i] & 0xFFFFu));
-          if (c_hi != 0xFFFFu) row[32 * p0 + c_hi] = __ushort_as_half(static_cast<unsigned short>(a[h][i] >> 16));
-        }
-      }
+  for (int st = 0; st < hdr->num_steps; ++st) {  // the salient columns go over the +-0 the main unpack left there
+    const uint8_t* ent = col + kColHdrBytes + kColTabBytes + st * kColStepBytes;
+    uint32_t a[8];
+    unpack_step(reinterpret_cast<const uint32_t*>(rec + geo.sal_off + st * kStepBytes)[row], reinterpret_cast<const uint4*>(ent),
+                scales(hdr->step_slot[st]), a);
+    for (int i = 0; i < 16; ++i) {
+      const unsigned at = reinterpret_cast<const uint16_t*>(ent + 64)[i];
+      if (i > 0 && at == 0u) continue;  // unused position: columns ascend, so column 0 can only come first
+      out[at] = __ushort_as_half(static_cast<unsigned short>(a[i >> 1] >> (16 * (i & 1))));
     }
   }
 }
 
 // ---- host side --------------------------------------------------------------------------------------
-// typical rows per segment up to which the persistent decode kernels are used
-constexpr int kTiledDecodeMaxRows = 64;
-
-static inline int rec_slot_bytes_for(int max_record_bytes) { return ((max_record_bytes + 15) & ~15) + 16; }
-
-static int sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
+template <int MODE>
+static size_t stage_bytes(const TiledArgs& args, int n) {
+  return stage_layout(args.max_steps, MODE == MODE_SINGLE ? 1 : 2, args.num_sets, n).total;
 }
 
-template <typename Kernel>
-static int configure_smem(Kernel kernel, size_t smem, size_t (&configured)[64]) {
-  int dev = 0;
-  TRIS_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || configured[dev] < smem) {
-    TRIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    if (dev >= 0 && dev < 64) configured[dev] = smem;
-  }
-  return TRIS_OK;
-}
-
-template <int NT, int MODE>
-static int launch_tiled(const TiledArgs& args, cudaStream_t stream, bool pdl) {
-  constexpr int NH = (MODE == MODE_SINGLE) ? 1 : 2;
-  const int tiles = tiles_per_expert(args.proj[0].out_features);
-  const int units_x = MODE == MODE_SINGLE ? (tiles + 1) / 2 : tiles;
-  const size_t smem = smem_layout(args.rec_slot_bytes, args.col_slot_bytes, args.sal_slots, NH, NT, 1).total;
-  const bool four_per_sm = 4 * (smem + 1024) <= 227 * 1024;
-  if (num_chunks(args.proj[0].rank) == 1 && !four_per_sm) {
-    // the one-CTA-per-unit kernel would not reach four CTAs per SM: persistent CTAs that prefetch the next record
-    const size_t smem2 = smem_layout(args.rec_slot_bytes, args.col_slot_bytes, args.sal_slots, NH, NT, 2).total;
-    if (smem2 <= 227 * 1024) {
-      auto kernel = grouped_tiled_persistent_kernel<NT, MODE>;
-      static size_t configured[64] = {};  // per instantiation, per device: largest size set so far
-      int st = configure_smem(kernel, smem2, configured);
-      if (st != TRIS_OK) return st;
-      const int per_sm = std::max<int>(1, std::min<size_t>(3, (227 * 1024) / (smem2 + 1024)));
-      const long long units = static_cast<long long>(units_x) * args.num_segments;
-      const int grid = static_cast<int>(std::min<long long>(units, static_cast<long long>(sm_count()) * per_sm));
-      return check_cuda(launch_kernel(kernel, dim3(grid), dim3(kThreads), smem2, stream, pdl, 1, args),
-                        "grouped_tiled_persistent_kernel launch");
-    }
-  }
-  TRIS_REQUIRE(smem <= 227 * 1024, TRIS_ERR_UNSUPPORTED, "grouped_tiled_kernel: %zu bytes of shared memory", smem);
-  auto kernel = grouped_tiled_kernel<NT, MODE, false>;
-  static size_t configured[64] = {};
-  int st = configure_smem(kernel, smem, configured);
-  if (st != TRIS_OK) return st;
-  return check_cuda(launch_kernel(kernel, dim3(units_x, args.num_segments), dim3(kThreads), smem, stream, pdl, 1, args),
-                    "grouped_tiled_kernel launch");
-}
-
-// Prefill-sized segments of a single-chunk projection: one CTA per unit, 32 rows per pass, weights
-// unpacked once per unit and kept in registers.
-// Row split of the cached kernel: with fewer units than CTA slots (two per SM) - few local experts with long
-// segments, as on an expert-parallel rank - up to `g_row_split_max` CTAs share a unit's row passes, each
-// decoding and unpacking the unit's weights for itself.
+// Row split: with fewer units than SMs - few local experts or one ordinary matrix, with long segments -
+// up to g_row_split_max CTAs share a unit's row passes, each unpacking its weights for itself.
 static std::atomic<int> g_row_split_max{4};
-static int cached_row_split(int units, int max_rows) {
+static int row_split(long long units, int max_rows, int n) {
   const int limit = g_row_split_max.load(std::memory_order_relaxed);
   if (limit <= 1 || units <= 0) return 1;
-  const int passes = (max_rows + 31) / 32;
-  return std::max(1, std::min({limit, 2 * sm_count() / units, passes}));
+  return static_cast<int>(std::max<long long>(1, std::min<long long>({limit, sm_count() / units, (max_rows + n - 1) / n})));
 }
 
-template <int MODE>
-static int launch_tiled_cached(const TiledArgs& args, int max_rows, cudaStream_t stream, bool pdl) {
-  constexpr int NH = (MODE == MODE_SINGLE) ? 1 : 2;
-  constexpr int NT = 4;
-  const int tiles = tiles_per_expert(args.proj[0].out_features);
-  const int units_x = MODE == MODE_SINGLE ? (tiles + 1) / 2 : tiles;
-  const size_t smem = smem_layout(args.rec_slot_bytes, args.col_slot_bytes, args.sal_slots, NH, NT, 1).total;
-  TRIS_REQUIRE(smem <= 227 * 1024, TRIS_ERR_UNSUPPORTED, "grouped_tiled_kernel: %zu bytes of shared memory", smem);
-  auto kernel = grouped_tiled_kernel<NT, MODE, true>;
-  static size_t configured[64] = {};
+template <int N, int MODE>
+static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {
+  const size_t stage = stage_bytes<MODE>(args, N);
+  args.stages = static_cast<int>(std::min<size_t>(kMaxStages, (kMostSmem - kBarBytes - kRowIdxBytes) / stage));
+  TRIS_REQUIRE(args.stages >= 2, TRIS_ERR_UNSUPPORTED, "grouped_tiled_kernel: %zu bytes per stage", stage);
+  args.reuse = args.chunks <= args.stages;
+  const size_t smem = kBarBytes + kRowIdxBytes + args.stages * stage;
+  auto kernel = grouped_tiled_kernel<N, MODE>;
+  static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
   int st = configure_smem(kernel, smem, configured);
   if (st != TRIS_OK) return st;
-  const int split = cached_row_split(units_x * args.num_segments, max_rows);
-  return check_cuda(launch_kernel(kernel, dim3(units_x, args.num_segments, split), dim3(kThreads), smem, stream, pdl, 1, args),
-                    "grouped_tiled_kernel (cached weights) launch");
+  const long long units = static_cast<long long>(args.units_x) * args.num_segments;
+  args.row_split = row_split(units, max_rows, N);
+  const int grid = static_cast<int>(std::min<long long>(units * args.row_split, sm_count()));
+  return check_cuda(launch_kernel(kernel, dim3(grid), dim3(Roles<N>::kThreads), smem, stream, pdl, 1, args), "grouped_tiled_kernel launch");
 }
 
 template <int MODE>
-static int dispatch_tiled(const TiledArgs& args, int max_rows, cudaStream_t stream, bool pdl) {
-  if (max_rows > kTiledDecodeMaxRows && num_chunks(args.proj[0].rank) == 1) return launch_tiled_cached<MODE>(args, max_rows, stream, pdl);
-  if (max_rows <= 8) return launch_tiled<1, MODE>(args, stream, pdl);
-  if (max_rows <= 16) return launch_tiled<2, MODE>(args, stream, pdl);
-  // 24 rows per pass also for segments of up to 64 rows: with 32 rows per pass the tile no longer fits four
-  // CTAs per SM, and four CTAs that re-unpack for a second or third pass beat three that do not (measured at
-  // 32 / 40 / 48 rows per expert: 55.9 / 63.6 / 75.6 us against 63.3 / 69.2 / 83.0 for both grouped kernels)
-  return launch_tiled<3, MODE>(args, stream, pdl);
+static int dispatch_tiled(TiledArgs& args, int max_rows, int typical_rows, cudaStream_t stream, bool pdl) {
+  args.units_x = MODE == MODE_SINGLE ? (args.tiles + 1) / 2 : args.tiles;
+  if (typical_rows <= kDecodeMaxRows) return launch_grouped_decode(args, MODE, typical_rows, stream, pdl);
+  // two stages of the widest pass have to fit shared memory (many salient columns make a stage larger)
+  if (typical_rows <= 64 || 2 * stage_bytes<MODE>(args, 128) + kBarBytes + kRowIdxBytes > kMostSmem) return launch_tiled<64, MODE>(args, max_rows, stream, pdl);
+  return launch_tiled<128, MODE>(args, max_rows, stream, pdl);
 }
 
 }  // namespace tr
 
 bool proj_has_tile_records(const TrisProjView& v) {
-  return v.tile_records != nullptr && v.tile_desc != nullptr && v.col_records != nullptr && v.use_block_gr &&
-         v.expert_slot == nullptr && v.gmap_slot == nullptr && v.col_record_bytes > 0 && v.max_record_bytes > 0;
+  return v.tile_records != nullptr && v.col_records != nullptr && v.use_block_gr && v.expert_slot == nullptr &&
+         v.gmap_slot == nullptr && v.col_record_bytes > 0 && v.max_record_bytes > 0;
 }
 
 // mode: 0 single projection, 1 gate/up pair, 2 gate/up pair with SiLU * mul
@@ -883,12 +635,12 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
                          const void* hidden_a, const void* hidden_b, void* out_a, void* out_b, int mode, int max_rows,
                          cudaStream_t stream, LaunchOpts opts) {
   using namespace tr;
-  // Rows per pass: a longer segment costs a second pass that only re-unpacks (the decoded planes
-  // stay), so size the activation tile for mean + 2 sigma of a balanced router rather than for the
-  // worst case; smaller tiles mean more resident CTAs.
-  if (route->num_segments > 0 && max_rows <= kTiledDecodeMaxRows) {
+  // Rows per pass: a longer segment costs a second pass that unpacks again, so size the pass for
+  // mean + 2 sigma of a balanced router rather than for the worst case.
+  int typical = max_rows;
+  if (route->num_segments > 0) {
     const double mean = static_cast<double>(route->num_rows) / route->num_segments;
-    max_rows = std::max(1, std::min(max_rows, static_cast<int>(ceil(mean + 2.0 * sqrt(mean)))));
+    typical = std::max(1, std::min(max_rows, static_cast<int>(ceil(mean + 2.0 * sqrt(mean)))));
   }
   TiledArgs a{};
   a.proj[0] = *proj_a;
@@ -905,30 +657,38 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   a.status = route->status_dev;
   a.num_segments = route->num_segments;
   a.num_rows = route->num_rows;
-  a.hidden_lane_order = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER) != 0;
+  a.rank = proj_a->rank;
+  a.out_features = proj_a->out_features;
+  a.num_experts = proj_a->num_experts;
+  a.tiles = tiles_per_expert(a.out_features);
+  a.chunks = num_chunks(a.rank);
+  a.max_steps = std::max(a.proj[0].max_sal_words, a.proj[1].max_sal_words);
+  a.hidden_mode = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER)
+                      ? TRIS_OUT_F16_LANE_ORDER
+                      : ((route->flags & TRIS_ROUTE_HIDDEN_PAIR_INTERLEAVED) ? TRIS_OUT_F16_PAIR_INTERLEAVED : TRIS_OUT_F16);
   a.hidden_stride = route->hidden_row_stride > 0 ? route->hidden_row_stride : proj_a->rank;
   a.weights_before_wait = opts.pdl && opts.weights_before_wait;
-  a.rec_slot_bytes = rec_slot_bytes_for(std::max(a.proj[0].max_record_bytes, a.proj[1].max_record_bytes));
-  a.col_slot_bytes = std::max(a.proj[0].col_record_bytes, a.proj[1].col_record_bytes);
-  a.sal_slots = std::max(1, std::max(a.proj[0].max_sal_words, a.proj[1].max_sal_words));
+  a.num_sets = (mode != MODE_SINGLE && a.hidden[0] != a.hidden[1]) ? 2 : 1;
   a.col_scale = static_cast<const __half*>(route->hidden_col_scale);
-  TRIS_REQUIRE(a.col_scale == nullptr || !a.hidden_lane_order, TRIS_ERR_INVALID_ARG,
+  a.hidden_vec = a.hidden_mode == TRIS_OUT_F16 && !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 &&
+                 ((reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1])) & 15u) == 0;
+  a.quad_store = proj_a->out_features % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 7u) == 0;
+  a.pair_store = proj_a->out_features % 2 == 0 &&
+                 ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 3u) == 0;
+  TRIS_REQUIRE(a.col_scale == nullptr || a.hidden_mode == TRIS_OUT_F16, TRIS_ERR_INVALID_ARG,
                "grouped (tile records): hidden_col_scale needs row-major activation rows");
-  TRIS_REQUIRE(!a.hidden_lane_order || proj_a->rank % 32 == 0, TRIS_ERR_INVALID_ARG,
-               "grouped (tile records): lane-order activations need rank %% 32 == 0");
+  TRIS_REQUIRE(a.hidden_mode == TRIS_OUT_F16 || proj_a->rank % 32 == 0, TRIS_ERR_INVALID_ARG,
+               "grouped (tile records): permuted activation rows need rank %% 32 == 0");
   TRIS_REQUIRE(a.hidden_stride >= proj_a->rank, TRIS_ERR_INVALID_ARG, "grouped (tile records): hidden_row_stride < rank");
-  if (mode == MODE_SINGLE) return dispatch_tiled<MODE_SINGLE>(a, max_rows, stream, opts.pdl);
-  if (mode == MODE_DUAL_SILU) return dispatch_tiled<MODE_DUAL_SILU>(a, max_rows, stream, opts.pdl);
-  return dispatch_tiled<MODE_DUAL_STORE>(a, max_rows, stream, opts.pdl);
+  if (mode == MODE_SINGLE) return dispatch_tiled<MODE_SINGLE>(a, max_rows, typical, stream, opts.pdl);
+  if (mode == MODE_DUAL_SILU) return dispatch_tiled<MODE_DUAL_SILU>(a, max_rows, typical, stream, opts.pdl);
+  return dispatch_tiled<MODE_DUAL_STORE>(a, max_rows, typical, stream, opts.pdl);
 }
 
-int launch_tiled_dump(const TrisProjView* proj, int32_t* dense_out, void* weights_out, cudaStream_t stream) {
+int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t stream) {
   using namespace tr;
-  const int rec_slot = rec_slot_bytes_for(proj->max_record_bytes);
-  const size_t smem = 64 + static_cast<size_t>(rec_slot) + proj->col_record_bytes + 2048;
-  TRIS_CUDA(cudaFuncSetAttribute(tiled_dump_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   dim3 grid(tiles_per_expert(proj->out_features), num_chunks(proj->rank), proj->num_experts);
-  tiled_dump_kernel<<<grid, kThreads, smem, stream>>>(*proj, dense_out, static_cast<__half*>(weights_out), rec_slot, nullptr);
+  tiled_dump_kernel<<<grid, kTileOut, proj->col_record_bytes, stream>>>(*proj, static_cast<__half*>(weights_out));
   return check_cuda(cudaGetLastError(), "tiled_dump_kernel launch");
 }
 

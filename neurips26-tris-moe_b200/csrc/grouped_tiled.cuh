@@ -1,0 +1,122 @@
+// What the two tile-record kernels share: launch arguments, result stores, host helpers.
+// grouped_decode.cu: few rows per segment, many small CTAs; grouped_tiled.cu: wide passes, persistent
+// warp-specialised CTAs.
+#pragma once
+#include <algorithm>
+#include <atomic>
+
+#include "tile_records.cuh"
+#include "umma.cuh"
+
+namespace tris {
+namespace tr {
+
+enum { MODE_SINGLE = 0, MODE_DUAL_STORE = 1, MODE_DUAL_SILU = 2 };
+
+constexpr int kACols = kSliceCols / 2;  // TMEM columns of one 64-column slice of weights
+
+struct TiledArgs {
+  TrisProjView proj[2];
+  const __half* hidden[2];
+  __half* out[2];
+  const int32_t* expert_ids;
+  const int32_t* segment_offsets;
+  const int32_t* num_segments_dev;
+  const int32_t* row_gather;
+  const int32_t* out_scatter;
+  int32_t* status;
+  int32_t num_segments;
+  int32_t num_rows;
+  int32_t rank, out_features, num_experts;  // the same for both projections
+  int32_t tiles, chunks, units_x, row_split;
+  int32_t max_steps;            // salient steps a record of either projection can have
+  int32_t hidden_mode;          // column order of the activation rows (TRIS_OUT_F16 / _PAIR_INTERLEAVED / _LANE_ORDER)
+  int32_t hidden_stride;        // halves between activation rows
+  int32_t hidden_vec;           // rows can be copied in 16-byte pieces as they are
+  int32_t num_sets;             // 2 when the two projections read different activation rows
+  int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
+  int32_t stages;               // ring depth, 2 .. kMaxStages
+  int32_t reuse;                // the chunks of a pass fit the ring: staged once for all tiles of a run
+  int32_t pair_store;           // 4-byte stores of two outputs are aligned
+  int32_t quad_store;           // 8-byte stores of four outputs are aligned
+  const __half* col_scale;      // optional [rank]: activation rows are multiplied by it while staged
+};
+
+// Eight columns (8 * piece ..) of an activation row that cannot be copied as it is; `left`: how many of them exist.
+static __device__ __noinline__ uint4 read_piece(const TiledArgs& args, const __half* chunk, int c0, int piece, int left) {
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  for (int v = 0; v < 8 && v < left; ++v) {
+    __half x = chunk[out_mode_pos(8 * piece + v, args.hidden_mode)];  // chunks start at multiples of 32 columns
+    if (args.col_scale) x = __hmul(x, args.col_scale[c0 + 8 * piece + v]);
+    w[v >> 1] |= static_cast<uint32_t>(__half_as_ushort(x)) << (16 * (v & 1));
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// COUNT consecutive rows (n0 ..) of output column o, one lane per output: neighbouring lanes swap
+// halves so that each stores two outputs of one row at once.
+template <int COUNT>
+__device__ __forceinline__ void store_rows(const TiledArgs& args, __half* out, int o, int r0, int n0, int rows, const float (&v)[COUNT]) {
+  const int odd = threadIdx.x & 1;
+  const bool in = o < args.out_features;
+  if (args.pair_store) {
+    int n = n0 + odd;
+    __half* dst = out + (o & ~1) + static_cast<size_t>(r0 + n) * args.out_features;
+    const size_t step = 2 * static_cast<size_t>(args.out_features);
+#pragma unroll
+    for (int j = 0; j < COUNT; j += 2, n += 2, dst += step) {
+      if (n0 + j >= rows) break;
+      const uint32_t p = h2_as_u32(__floats2half2_rn(v[j], v[j + 1]));
+      const uint32_t q = __shfl_xor_sync(0xFFFFFFFFu, p, 1);
+      if (n < rows && in) {
+        const uint32_t w = odd ? prmt(q, p, 0x7632u) : prmt(p, q, 0x5410u);
+        if (!args.out_scatter) {
+          *reinterpret_cast<uint32_t*>(dst) = w;
+        } else {
+          const int orow = args.out_scatter[r0 + n];
+          if (orow >= 0) *reinterpret_cast<uint32_t*>(out + (o & ~1) + static_cast<size_t>(orow) * args.out_features) = w;
+        }
+      }
+    }
+  } else if (in) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) {
+      if (n0 + j >= rows) break;
+      const int orow = args.out_scatter ? args.out_scatter[r0 + n0 + j] : r0 + n0 + j;
+      if (orow >= 0) out[static_cast<size_t>(orow) * args.out_features + o] = __float2half_rn(v[j]);
+    }
+  }
+}
+
+// ---- host helpers -----------------------------------------------------------------------------------
+inline int sm_count() {
+  static std::atomic<int> cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+template <typename Kernel>
+int configure_smem(Kernel kernel, size_t smem, std::atomic<size_t> (&configured)[64]) {
+  int dev = 0;
+  TRIS_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || configured[dev].load(std::memory_order_relaxed) < smem) {
+    TRIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (dev >= 0 && dev < 64) configured[dev].store(smem, std::memory_order_relaxed);
+  }
+  return TRIS_OK;
+}
+
+constexpr size_t kMostSmem = 227 * 1024;
+
+// Segments of up to `max_rows` rows; MODE_SINGLE, MODE_DUAL_STORE or MODE_DUAL_SILU.
+int launch_grouped_decode(const TiledArgs& args, int mode, int typical_rows, cudaStream_t stream, bool pdl);
+constexpr int kDecodeMaxRows = 32;
+
+}  // namespace tr
+}  // namespace tris

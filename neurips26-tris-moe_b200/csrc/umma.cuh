@@ -62,6 +62,48 @@ __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+template <int COUNT>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[COUNT]) {  // as tmem_ld_16, 4 or 8 columns, no wait
+  static_assert(COUNT == 4 || COUNT == 8, "columns per load");
+  uint32_t r[COUNT];
+  if constexpr (COUNT == 8)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+  else
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Registers -> TMEM: thread t of the warp writes COUNT consecutive 32-bit columns of lane (taddr.lane + t).
+// This is how a computed A operand gets to the tensor core without passing through shared memory: column
+// c of lane m holds A[m][2c], A[m][2c + 1].
+template <int COUNT>
+__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[COUNT]) {
+  static_assert(COUNT == 8 || COUNT == 16, "columns per store");
+  if constexpr (COUNT == 16)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+  else
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// A from TMEM (128 lanes, 8 columns per K = 16 step), B from shared memory.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // Starts the asynchronous copy of a ROWS x 64 fp16 tile (row-major source, 128 B per row) into
 // the core-matrix layout.  row_ptr(r) returns the source row (already offset to the chunk's
 // first column) or nullptr for a row that must read as zeros.
@@ -84,3 +126,4 @@ __device__ __forceinline__ void stage_operand_async(uint8_t* dst, const __half* 
 
 
 }  // namespace tris
+

@@ -100,7 +100,7 @@ def prepare_grouped_payload(payload: dict, device=None, gr_substreams: int = DEF
     reference tensors: the per-packed-row group table (validating ``g_idx`` as
     ``prepare_compact3_k64_groups`` does, qlinear_cuda.py:364-407) and, for block-GR
     payloads, the sub-stream index (validating offsets/meta) and the tile-major records the
-    grouped kernels read (one contiguous piece per expert, 64 outputs and 256 columns, so a
+    grouped kernels read (one contiguous piece per expert, 128 outputs and 128 columns; grouping
     tile arrives with one bulk copy; ``tile_records=False`` skips them and the kernels gather
     the tile from the E-stacked tensors).  Runs once at load time and synchronises to read the
     validation status.  Idempotent."""
@@ -178,16 +178,17 @@ def _adopt_stored_derived(payload: dict, dev, E: int, pr: int, O: int, rank: int
     packed-row groups, tile records) instead of rebuilding them; False when their shapes do not fit
     this payload (then they are dropped and everything is rebuilt and re-validated)."""
     nblk = math.ceil(pr / 2) * math.ceil(O / 64)
-    count = E * math.ceil(O / 64) * math.ceil(pr / 8)
+    chunks = math.ceil(pr / 4)
+    count = E * math.ceil(O / 128) * chunks
     idx, grp, rec, desc, col = (payload.get(k) for k in ("_tris_gr_index", "_tris_packed_row_group", "_tris_tile_records",
                                                         "_tris_tile_desc", "_tris_col_records"))
     meta = payload.get("_tris_tile_meta")
     ok = all(isinstance(t, torch.Tensor) for t in (idx, grp, rec, desc, col)) and isinstance(meta, tuple) and len(meta) == 3
     ok = ok and tuple(idx.shape) == (E, nblk, 32) and tuple(grp.shape) == (E, pr) and tuple(desc.shape) == (count + 1, 2)
-    ok = ok and col.numel() == E * math.ceil(pr / 8) * int(meta[0]) and rec.dtype == torch.uint8 and col.dtype == torch.uint8
-    if ok:
-        last = desc[count - 1].to(torch.int64)
-        ok = int((last[0] & 0xFFFFFFFF) * 16 + (last[1] & 0xFFFFFFFF)) <= rec.numel()
+    ok = ok and col.numel() == E * chunks * int(meta[0]) and rec.dtype == torch.uint8 and col.dtype == torch.uint8
+    ok = ok and rec.numel() == count * int(meta[1])
+    if ok:  # records of another layout version are rebuilt
+        ok = int(col[:4].cpu().view(torch.int32).item()) == TILE_RECORD_MAGIC
     if not ok:
         for k in ("_tris_gr_index", "_tris_packed_row_group", "_tris_tile_records", "_tris_tile_desc", "_tris_col_records",
                   "_tris_tile_meta", "_tris_derived_from_checkpoint"):
@@ -203,6 +204,13 @@ def _adopt_stored_derived(payload: dict, dev, E: int, pr: int, O: int, rank: int
     return True
 
 
+TILE_RECORD_MAGIC = 0x32305254  # layout version of the records, first word of every column record
+
+
+def _col_record_bytes(view: TrisProjView, total: int) -> int:
+    return total // (view.num_experts * math.ceil(view.rank / 128))
+
+
 def _build_tile_records(payload: dict, lib, dev) -> None:
     """Plans and fills the tile-major records of a block-GR payload (``tris_tile_records_plan`` /
     ``tris_tile_records_build``) into tensors kept in the payload dict."""
@@ -215,6 +223,7 @@ def _build_tile_records(payload: dict, lib, dev) -> None:
         _native.check(lib.tris_tile_records_plan(C.byref(view), desc.data_ptr(), info.data_ptr(), stream), "tile_records_plan")
         total, max_rec, max_sal, _ = (int(v) for v in info.cpu().tolist())
         col_total = int(lib.tris_col_record_bytes(C.byref(view), max_sal))
+        view.max_record_bytes = max_rec
         records = torch.empty((max(total, 16),), dtype=torch.uint8, device=dev)
         cols = torch.empty((max(col_total, 16),), dtype=torch.uint8, device=dev)
         _native.check(lib.tris_tile_records_build(C.byref(view), desc.data_ptr(), records.data_ptr(), cols.data_ptr(),
@@ -222,7 +231,7 @@ def _build_tile_records(payload: dict, lib, dev) -> None:
     payload["_tris_tile_records"] = records
     payload["_tris_tile_desc"] = desc
     payload["_tris_col_records"] = cols
-    payload["_tris_tile_meta"] = (64 + 1024 + 256 * max_sal, max_rec, max_sal)
+    payload["_tris_tile_meta"] = (_col_record_bytes(view, col_total), max_rec, max_sal)
 
 
 def _build_view(payload: dict, need_index: bool) -> TrisProjView:
