@@ -160,7 +160,7 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
     if (st != TRIS_OK) return st;
   }
   if (np > 0) {
-    st = launch_shared_hidden(probs, np, x, nullptr, T, layer->hidden_size, s, /*pdl=*/logits_given);
+    st = launch_shared_hidden(probs, np, x, nullptr, T, layer->hidden_size, s, /*pdl=*/logits_given, nullptr, true);
     if (st != TRIS_OK) return st;
   }
   if (packed_gu) {
@@ -196,7 +196,7 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
                                       layer->down.rank, down_mode, 0, s);
   } else {
     SkinnyProblem down{static_cast<const __half*>(layer->shared_down), w.hidden_down, layer->down.rank, down_mode};
-    st = launch_shared_hidden(&down, 1, w.mlp, nullptr, R, layer->intermediate_size, s, /*pdl=*/true);
+    st = launch_shared_hidden(&down, 1, w.mlp, nullptr, R, layer->intermediate_size, s, /*pdl=*/true, nullptr, true);
   }
   if (st != TRIS_OK) return st;
 

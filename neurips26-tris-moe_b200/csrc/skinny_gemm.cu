@@ -130,7 +130,7 @@ static int launch_skinny(const SkinnyArgs& args, int mtiles, int ksplit, cudaStr
 
 // Launches up to kMaxProblems matrices that share x.
 int launch_shared_hidden(const SkinnyProblem* probs, int num_problems, const __half* x, const int32_t* row_gather,
-                         int n, int k, cudaStream_t stream, bool pdl, const int32_t* n_dev) {
+                         int n, int k, cudaStream_t stream, bool pdl, const int32_t* n_dev, bool matrices_before_wait) {
   TRIS_REQUIRE(num_problems >= 1 && num_problems <= kMaxProblems, TRIS_ERR_INVALID_ARG, "shared hidden: bad problem count");
   TRIS_REQUIRE(n >= 0 && k > 0, TRIS_ERR_INVALID_ARG, "shared hidden: bad sizes n=%d k=%d", n, k);
   TRIS_REQUIRE((k & 7) == 0, TRIS_ERR_UNSUPPORTED, "shared hidden: in_features=%d must be a multiple of 8", k);
@@ -139,7 +139,7 @@ int launch_shared_hidden(const SkinnyProblem* probs, int num_problems, const __h
     TRIS_REQUIRE(probs[i].a && probs[i].out && probs[i].m > 0, TRIS_ERR_INVALID_ARG, "shared hidden: bad problem %d", i);
   // enough rows for a dense contraction: tcgen05 / TMEM tiles
   if (tc_gemm_applicable(n, k, x, probs, num_problems))
-    return launch_tc_gemm(probs, num_problems, x, row_gather, n, k, stream, pdl, n_dev, nullptr);
+    return launch_tc_gemm(probs, num_problems, x, row_gather, n, k, stream, pdl, n_dev, nullptr, matrices_before_wait);
   SkinnyArgs args{};
   int mtiles = 0;
   for (int i = 0; i < num_problems; ++i) {

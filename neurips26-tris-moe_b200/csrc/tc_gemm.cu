@@ -35,6 +35,7 @@ struct TcGemmArgs {
   int32_t n;
   int32_t k;
   int32_t k_per_cta;  // multiple of kTcKChunk
+  int32_t a_before_wait;  // the matrices are older than the predecessor kernel
 };
 
 constexpr int kTcStages = 4;
@@ -94,6 +95,19 @@ __device__ __forceinline__ void tc_gemm_epilogue(const TcGemmArgs& args, const S
       for (unsigned r = 0; r < 8; ++r) { acc.x += v[r].x; acc.y += v[r].y; acc.z += v[r].z; acc.w += v[r].w; }
       const int n = n0 + (4 * i4) / kTcM, mbase = m0 + (4 * i4) % kTcM;
       if (n >= n_live) continue;
+      if ((pb.m & 3) == 0 && mbase < pb.m && (pb.out_mode == TRIS_OUT_F32 || pb.out_mode == TRIS_OUT_F16)) {
+        const size_t at = static_cast<size_t>(n) * pb.m + mbase;
+        if (pb.out_mode == TRIS_OUT_F32) {
+          if ((reinterpret_cast<uintptr_t>(pb.out) & 15u) == 0) {
+            *reinterpret_cast<float4*>(static_cast<float*>(pb.out) + at) = acc;
+            continue;
+          }
+        } else if ((reinterpret_cast<uintptr_t>(pb.out) & 7u) == 0) {
+          *reinterpret_cast<uint2*>(static_cast<__half*>(pb.out) + at) =
+              make_uint2(h2_as_u32(__floats2half2_rn(acc.x, acc.y)), h2_as_u32(__floats2half2_rn(acc.z, acc.w)));
+          continue;
+        }
+      }
       const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -258,22 +272,25 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_kernel(const __grid_cons
 }
 
 // ---- TMA-fed variant ------------------------------------------------------------------------
-// Same tile, same operand layout, but a K chunk of an operand arrives with ONE tensor copy: the
-// row-major matrix [rows, K] is described to the TMA unit as a 3-D tensor (8 halves, rows, K/8)
-// with byte strides (2, 2K, 16), and a box of (8, ROWS, 8) lands in shared memory as
-// [K chunk][row][16 bytes] - exactly the K-major no-swizzle core-matrix layout the MMA reads.
-// Rows past the matrix read as zeros.  One thread issues the copies (a full/empty mbarrier pair
-// per stage), one thread the MMAs; all four warps run the epilogue.  Used when the activation
-// rows are not gathered (row_gather == nullptr).
+// Same tile, but the operands lie in shared memory in the 128-byte-swizzled K-major layout (8 rows x 128
+// bytes per atom), so that a K chunk of an operand arrives with ONE tensor copy whose rows are 128
+// contiguous bytes.  (Boxes of 16-byte rows that land in the no-swizzle core-matrix order made the copy
+// engine the limit: 1536 requests per chunk; 16384 x 1024 x 256: 75 us.)  Rows past the matrix read as
+// zeros.  One thread issues the copies (a full/empty mbarrier pair per stage), one thread the MMAs; all
+// four warps run the epilogue.  The matrix chunks of the first stages are requested before the wait for
+// the predecessor kernel when the caller says that they are older.  Used when the activation rows are not
+// gathered (row_gather == nullptr).
 struct TcTmaMaps {
   CUtensorMap a[3];
   CUtensorMap x;
 };
+constexpr int kTcRowBytes = kTcKChunk * 2;
+static_assert(kTcRowBytes == 128, "one swizzle row per operand row and chunk");
 
 template <int NTILE>
-struct alignas(128) TcTmaSmem {
-  uint8_t a[kTcStages][kTcM * kTcKChunk * 2];
-  uint8_t b[kTcStages][NTILE * kTcKChunk * 2];
+struct TcTmaSmem {  // at a 1024-byte boundary
+  uint8_t a[kTcStages][kTcM * kTcRowBytes];
+  uint8_t b[kTcStages][NTILE * kTcRowBytes];
   uint64_t full[kTcStages];
   uint64_t empty[kTcStages];
   uint64_t done;
@@ -281,20 +298,26 @@ struct alignas(128) TcTmaSmem {
   int32_t timed_out;
 };
 
-__device__ __forceinline__ void tma_load_3d(void* dst_smem, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(smem_u32(dst_smem)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
-      : "memory");
+__device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                   smem_u32(dst_smem)),
+               "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+               : "memory");
+}
+// K-major, 128-byte swizzle: 1024 bytes between 8-row groups; a K = 16 step is 32 bytes further.
+__device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t smem_addr) {
+  return static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) |
+         (2ull << 61);
 }
 
 template <int NTILE>
 __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_constant__ TcGemmArgs args,
                                                                    const __grid_constant__ TcTmaMaps maps) {
   extern __shared__ uint4 smem_raw[];
-  auto& sm = *reinterpret_cast<TcTmaSmem<NTILE>*>(smem_raw);
+  uint8_t* base = reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  auto& sm = *reinterpret_cast<TcTmaSmem<NTILE>*>(base);
   cg::cluster_group cluster = cg::this_cluster();
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
 
   int tile = blockIdx.x, pi = 0;
   while (pi + 1 < args.num_problems && tile >= (args.prob[pi].m + kTcM - 1) / kTcM) {
@@ -323,7 +346,16 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem = sm.tmem_base;
+  const uint32_t tmem = warp_uniform(sm.tmem_base);
+  constexpr uint32_t kBytes = (kTcM + NTILE) * kTcRowBytes;
+  auto load_a = [&](int i) {
+    const int s = i % kTcStages;
+    mbar_arrive_expect_tx(&sm.full[s], kBytes);
+    tma_load_2d(sm.a[s], &maps.a[pi], kbeg + i * kTcKChunk, m0, &sm.full[s]);
+  };
+  const int ahead = args.a_before_wait ? min(nchunks, kTcStages) : 0;
+  if (threadIdx.x == 0)
+    for (int i = 0; i < ahead; ++i) load_a(i);
 
   pdl_wait();  // x and n_dev come from earlier kernels
   pdl_launch_dependents();
@@ -331,45 +363,47 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
 
   if (threadIdx.x == 0) {
     // producer: one tensor copy per operand per K chunk, kTcStages chunks in flight
-    constexpr uint32_t kBytes = (kTcM + NTILE) * kTcKChunk * 2;
     for (int i = 0; i < nchunks; ++i) {
       const int s = i % kTcStages;
       if (i >= kTcStages && !mbar_wait_bounded(&sm.empty[s], ((i / kTcStages) - 1) & 1)) {
         sm.timed_out = 1;
         break;
       }
-      mbar_arrive_expect_tx(&sm.full[s], kBytes);
-      const int kc = (kbeg + i * kTcKChunk) >> 3;
-      tma_load_3d(sm.a[s], &maps.a[pi], 0, m0, kc, &sm.full[s]);
-      tma_load_3d(sm.b[s], &maps.x, 0, n0, kc, &sm.full[s]);
+      if (i >= ahead) load_a(i);
+      tma_load_2d(sm.b[s], &maps.x, kbeg + i * kTcKChunk, n0, &sm.full[s]);
     }
-  } else if (threadIdx.x == 32) {
-    // consumer: four K=16 MMAs per chunk; the commit frees the stage for the producer
-    const uint32_t idesc = umma_idesc_f16(kTcM, NTILE);
-    bool ok = true;
-    for (int i = 0; i < nchunks && ok; ++i) {
-      const int s = i % kTcStages;
-      ok = mbar_wait_bounded(&sm.full[s], (i / kTcStages) & 1);
-      if (!ok) break;
-      tcgen05_fence_after();
-      const uint32_t a_addr = smem_u32(sm.a[s]), b_addr = smem_u32(sm.b[s]);
-#pragma unroll
-      for (int j = 0; j < kTcKChunk / 16; ++j) {
-        const uint64_t da = umma_smem_desc(a_addr + j * 2 * kTcM * 16, kTcM * 16, 128);
-        const uint64_t db = umma_smem_desc(b_addr + j * 2 * NTILE * 16, NTILE * 16, 128);
-        umma_f16_ss(tmem, da, db, idesc, (i > 0 || j > 0) ? 1u : 0u);
-      }
-      umma_commit(&sm.empty[s]);
-    }
-    if (!ok) sm.timed_out = 1;
-    umma_commit(&sm.done);  // arrives once every MMA issued so far has completed
   }
   __syncwarp();
+  if (warp == 1) {
+    // consumer: four K = 16 MMAs per chunk; the commit frees the stage for the producer
+    const uint32_t idesc = umma_idesc_f16(kTcM, NTILE);
+    bool ok = true;
+    for (int i = 0; i < nchunks; ++i) {
+      const int s = i % kTcStages;
+      ok = mbar_wait_warp(&sm.full[s], (i / kTcStages) & 1);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint64_t da = umma_smem_desc_sw128(smem_u32(sm.a[s])), db = umma_smem_desc_sw128(smem_u32(sm.b[s]));
+      if (elect_one()) {
+#pragma unroll
+        for (int j = 0; j < kTcKChunk / 16; ++j) umma_f16_ss(tmem, da + 2 * j, db + 2 * j, idesc, (i > 0 || j > 0) ? 1u : 0u);
+        umma_commit(&sm.empty[s]);
+      }
+    }
+    if (elect_one()) {
+      if (!ok) sm.timed_out = 1;
+      umma_commit(&sm.done);  // arrives once every MMA issued so far has completed
+    }
+    __syncwarp();
+  }
   if (!mbar_wait_bounded(&sm.done, 0)) sm.timed_out = 1;
   tcgen05_fence_after();
   __syncthreads();
   const bool failed = sm.timed_out != 0;
-  tc_gemm_epilogue<NTILE>(args, pb, reinterpret_cast<float*>(smem_raw), tmem, failed, nchunks, m0, n0, n_live, cluster);
+  if (failed && threadIdx.x == 0)  // copies in flight must not land in a buffer that is read as the partial tile
+    for (int i = 0; i < kTcStages; ++i) mbar_wait_bounded(&sm.full[i], 0);
+  __syncthreads();
+  tc_gemm_epilogue<NTILE>(args, pb, reinterpret_cast<float*>(base), tmem, failed, nchunks, m0, n0, n_live, cluster);
 }
 
 template <int NTILE>
@@ -407,24 +441,24 @@ static EncodeTiledFn encode_tiled_fn() {
   return reinterpret_cast<EncodeTiledFn>(cached.load(std::memory_order_acquire));
 }
 
-// Describes the row-major fp16 matrix [rows, k] as (8 halves, rows, k/8) with a box of
-// (8, box_rows, 8): one copy = one 64-column chunk of box_rows rows in core-matrix order.
+// Describes the row-major fp16 matrix [rows, k]; one copy = one 64-column chunk of box_rows rows,
+// 128-byte-swizzled.
 static bool encode_operand_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr || rows <= 0) return false;
-  const cuuint64_t dims[3] = {8, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(k / 8)};
-  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(k) * 2, 16};  // bytes, dimensions 1 and 2
-  const cuuint32_t box[3] = {8, static_cast<cuuint32_t>(box_rows), 8};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};  // bytes, dimension 1
+  const cuuint32_t box[2] = {kTcKChunk, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int NTILE>
 static int launch_umma_tma(const TcGemmArgs& args, const TcTmaMaps& maps, int mtiles, int ksplit, cudaStream_t stream,
                            bool pdl) {
-  const size_t smem = std::max(sizeof(TcTmaSmem<NTILE>), static_cast<size_t>(NTILE) * kTcM * 4 + 128);
+  const size_t smem = std::max(sizeof(TcTmaSmem<NTILE>), static_cast<size_t>(NTILE) * kTcM * 4) + 1024;
   static bool configured[64] = {};
   int dev = 0;
   TRIS_CUDA(cudaGetDevice(&dev));
@@ -447,7 +481,7 @@ bool tc_gemm_applicable(int n, int k, const __half* x, const SkinnyProblem* prob
 }
 
 int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x, const int32_t* row_gather, int n,
-                   int k, cudaStream_t stream, bool pdl, const int32_t* n_dev, int32_t* status) {
+                   int k, cudaStream_t stream, bool pdl, const int32_t* n_dev, int32_t* status, bool a_before_wait) {
   TcGemmArgs args{};
   int mtiles = 0;
   for (int i = 0; i < num_problems; ++i) {
@@ -461,7 +495,9 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
   args.status = status;
   args.n = n;
   args.k = k;
-  const int ntile = n <= 2048 ? 64 : 128;
+  args.a_before_wait = pdl && a_before_wait;
+  // 128-row tiles re-read the matrices half as often; 64-row tiles give a small batch more CTAs
+  const int ntile = mtiles * ceil_div(n, 128) >= 148 ? 128 : 64;
   const int ntiles = ceil_div(n, ntile);
   int ksplit = 1;
   // split K over the cluster until the GPU is full or a CTA would get fewer than two 64-column chunks: a CTA's
@@ -472,10 +508,7 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
   if (row_gather == nullptr) {  // operands by tensor copies
     TcTmaMaps maps;
     bool ok = encode_operand_map(&maps.x, x, n, k, ntile);
-    for (int i = 0; i < 3 && ok; ++i) {
-      const SkinnyProblem& pr = probs[i < num_problems ? i : 0];
-      ok = encode_operand_map(&maps.a[i], pr.a, pr.m, k, kTcM);
-    }
+    for (int i = 0; i < num_problems && ok; ++i) ok = encode_operand_map(&maps.a[i], probs[i].a, probs[i].m, k, kTcM);
     if (ok) {
       if (ntile == 64) return launch_umma_tma<64>(args, maps, mtiles, ksplit, stream, pdl);
       return launch_umma_tma<128>(args, maps, mtiles, ksplit, stream, pdl);
