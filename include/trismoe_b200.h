@@ -109,6 +109,8 @@ typedef struct TrisProjView {
 /*
  * Grouped route on the device (QL:1328-1338).  Arrays may be padded to E (+1): segment s
  * is live when s < *num_segments_dev (or s < num_segments when num_segments_dev is NULL).
+ * expert_ids == segment_offsets == NULL with num_segments == 1 (projections with tile records only): one
+ * segment of expert 0 that holds all rows - an ordinary linear needs no route arrays.
  */
 typedef struct TrisRouteView {
   const int32_t* expert_ids;        /* [>= num_segments] expert of each segment            */

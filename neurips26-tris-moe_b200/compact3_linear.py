@@ -51,9 +51,12 @@ class Compact3Linear(nn.Module):
         self.input_scale = None if ns_vector_col is None else ns_vector_col.reshape(self.in_features).to(dev, torch.float16).contiguous()
 
     def _route(self, rows: int, device) -> dict:
-        zero = torch.zeros((1,), dtype=torch.int32, device=device)
-        route = {"expert_ids": zero, "segment_offsets": torch.tensor([0, rows], dtype=torch.int32, device=device),
-                 "_max_rows_per_segment": rows}
+        if isinstance(self.payload.get("_tris_tile_records"), torch.Tensor):
+            route = {"_one_segment": True, "_max_rows_per_segment": rows}
+        else:
+            zero = torch.zeros((1,), dtype=torch.int32, device=device)
+            route = {"expert_ids": zero, "segment_offsets": torch.tensor([0, rows], dtype=torch.int32, device=device),
+                     "_max_rows_per_segment": rows}
         if self.input_scale is not None:
             route["_hidden_col_scale"] = self.input_scale
         return route

@@ -467,8 +467,9 @@ static int dispatch_grouped(const GroupedArgs& args, int max_rows, cudaStream_t 
   return launch_grouped<NPROJ, 8, EPI>(args, stream, pdl);
 }
 
-static int fill_route(GroupedArgs& a, const TrisRouteView* route) {
-  TRIS_REQUIRE(route != nullptr && route->expert_ids && route->segment_offsets, TRIS_ERR_INVALID_ARG,
+static int fill_route(GroupedArgs& a, const TrisRouteView* route, bool records) {
+  const bool one_segment = route != nullptr && !route->expert_ids && !route->segment_offsets && route->num_segments == 1 && records;
+  TRIS_REQUIRE(one_segment || (route != nullptr && route->expert_ids && route->segment_offsets), TRIS_ERR_INVALID_ARG,
                "route: expert_ids/segment_offsets must be set");
   TRIS_REQUIRE(route->num_segments >= 0 && route->num_rows >= 0, TRIS_ERR_INVALID_ARG, "route: negative sizes");
   a.expert_ids = route->expert_ids;
@@ -580,7 +581,7 @@ int tris::grouped_forward_impl(const TrisProjView* proj, const TrisRouteView* ro
   if (st != TRIS_OK) return st;
   TRIS_REQUIRE(hidden_f16 && out_f16, TRIS_ERR_INVALID_ARG, "tris_grouped_forward: null hidden/out");
   GroupedArgs a{};
-  st = fill_route(a, route);
+  st = fill_route(a, route, proj_has_tile_records(*proj));
   if (st != TRIS_OK) return st;
   if (a.num_segments == 0 || a.num_rows == 0) return TRIS_OK;
   const bool lane_order = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER) != 0;
@@ -639,7 +640,7 @@ int tris::grouped_pair_forward_impl(const TrisProjView* proj_a, const TrisProjVi
   TRIS_REQUIRE(hidden_a_f16 && hidden_b_f16 && out_a_f16 && (fuse_silu_mul || out_b_f16), TRIS_ERR_INVALID_ARG,
                "tris_grouped_pair_forward: null hidden/out");
   GroupedArgs a{};
-  st = fill_route(a, route);
+  st = fill_route(a, route, proj_has_tile_records(*proj_a) && proj_has_tile_records(*proj_b));
   if (st != TRIS_OK) return st;
   if (a.num_segments == 0 || a.num_rows == 0) return TRIS_OK;
   const bool lane_order = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER) != 0;

@@ -63,8 +63,9 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
   const int seg = blockIdx.y;
   const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
   if (seg >= nseg) return;
-  const int expert = args.expert_ids[seg];
-  const int row_begin = args.segment_offsets[seg], row_end = min(args.segment_offsets[seg + 1], args.num_rows);
+  const int expert = args.expert_ids ? args.expert_ids[seg] : 0;  // no arrays: one segment of expert 0 with all rows
+  const int row_begin = args.expert_ids ? args.segment_offsets[seg] : 0;
+  const int row_end = args.expert_ids ? min(args.segment_offsets[seg + 1], args.num_rows) : args.num_rows;
   if (expert < 0 || expert >= args.num_experts || row_end <= row_begin) return;
 
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31, g = lane >> 2, t = lane & 3;

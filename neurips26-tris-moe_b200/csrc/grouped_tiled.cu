@@ -79,6 +79,12 @@ struct Walker {
       z = q / nseg;
       seg = q - z * nseg;
     }
+    if (!args.expert_ids) {  // one segment of expert 0 with all rows
+      next_expert = 0;
+      next_begin = z * N;
+      next_end = args.num_rows;
+      return;
+    }
     next_expert = args.expert_ids[seg];
     next_begin = args.segment_offsets[seg] + z * N;
     next_end = args.segment_offsets[seg + 1];

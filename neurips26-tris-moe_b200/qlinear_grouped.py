@@ -100,8 +100,8 @@ def prepare_grouped_payload(payload: dict, device=None, gr_substreams: int = DEF
     reference tensors: the per-packed-row group table (validating ``g_idx`` as
     ``prepare_compact3_k64_groups`` does, qlinear_cuda.py:364-407) and, for block-GR
     payloads, the sub-stream index (validating offsets/meta) and the tile-major records the
-    grouped kernels read (one contiguous piece per expert, 128 outputs and 128 columns; grouping
-    tile arrives with one bulk copy; ``tile_records=False`` skips them and the kernels gather
+    grouped kernels read (one contiguous piece per expert, 128 outputs and 128 columns, with the
+    grouping bits decoded; ``tile_records=False`` skips them and the kernels gather
     the tile from the E-stacked tensors).  Runs once at load time and synchronises to read the
     validation status.  Idempotent."""
     if payload.get("_tris_prepared") and (device is None or payload["qweight1"].device == torch.device(device)):
@@ -423,17 +423,21 @@ def _coerce_grouped_route(route_or_lengths, device, expert_ids=None):
 
 def _route_view(route: dict, num_rows: int, keep: list) -> TrisRouteView:
     rv = TrisRouteView()
-    ids = route["expert_ids"]
-    seg = route["segment_offsets"]
-    if ids.dtype != torch.int32 or not ids.is_contiguous():
-        ids = ids.to(torch.int32).contiguous()
-    if seg.dtype != torch.int32 or not seg.is_contiguous():
-        seg = seg.to(torch.int32).contiguous()
-    keep += [ids, seg]
-    rv.expert_ids = ids.data_ptr() if ids.numel() else None
-    rv.segment_offsets = seg.data_ptr()
     rv.num_segments_dev = None
-    rv.num_segments = int(ids.numel())
+    if route.get("_one_segment"):  # an ordinary linear: one expert, every row; no route arrays
+        rv.expert_ids = rv.segment_offsets = None
+        rv.num_segments = 1
+    else:
+        ids = route["expert_ids"]
+        seg = route["segment_offsets"]
+        if ids.dtype != torch.int32 or not ids.is_contiguous():
+            ids = ids.to(torch.int32).contiguous()
+        if seg.dtype != torch.int32 or not seg.is_contiguous():
+            seg = seg.to(torch.int32).contiguous()
+        keep += [ids, seg]
+        rv.expert_ids = ids.data_ptr() if ids.numel() else None
+        rv.segment_offsets = seg.data_ptr()
+        rv.num_segments = int(ids.numel())
     rv.num_rows = int(num_rows)
     rv.max_rows_per_segment = int(route.get("_max_rows_per_segment", 0) or 0)
     rv.row_gather = None
