@@ -1,20 +1,23 @@
 // Grouped compact3 dequant-matmul over tile records for segments of few rows (decode), on mma.sync.
 //
 // A warp owns 32 outputs of one projection and multiplies them with up to 8 NT activation rows.  Lane
-// (g, t) takes code word t of output rows g, g + 8, g + 16, g + 24: 16 columns of each of a 64-column slice,
-// loaded coalesced (128 bytes per load) and straight from the record, since they are used once.  Unpacked,
-// they are the lane's A fragments of four m16n8k16 steps if step j's K positions are columns
-// 16t + 4j .. + 3, which the B side follows: a lane's activations of a slice are 32 contiguous bytes.  No
-// weight passes through shared memory or TMEM, and the warps of a CTA meet only where activation rows
-// are staged and where gate meets up.
+// (g, t) takes code word t of output rows g, g + 8, g + 16, g + 24: 16 columns of each of a 64-column slice.
+// Unpacked, they are the lane's A fragments of four m16n8k16 steps if step j's K positions are columns
+// 16t + 4j .. + 3, which the B side follows: a lane's activations of a slice are 32 contiguous bytes.
+// Weights go from the code words to the MMA in registers.
 // tcgen05 tiles have 128 outputs and take their A from TMEM: allocation, stores and the hand-over to
-// the issuing thread cost more than the unpack at a few rows per weight.  What bounds this kernel:
-// instruction issue, and next to it the shared-memory / L1 data path (scale tables and activations are
-// re-read by every warp; 32 outputs per warp instead of 16 halve that).
+// the issuing thread cost more than the unpack at a few rows per weight.
 //
-// CTAs are small (four warps, seven CTAs per SM) so that the units of a decode batch are resident at
-// once and SMs are evenly loaded.  With few units the columns are split over KS warps (partial sums
-// added through shared memory): whole 128-column chunks over KS = 2, 64-column halves over KS = 4 and 8.
+// Everything a CTA reads - code words, scales, tables, activation rows - is asked for at its start by
+// cp.async and read from shared memory, so that the inner loop waits for nothing further away: with the
+// same loop on L1 / L2 loads half the stall cycles were theirs.  (Bulk copies issued by the lanes of a
+// warp serialise: 57 copies made a start of several thousand cycles.)  What bounds it now: instruction
+// issue (3.4 lane-instructions per weight plus staging and epilogue).
+//
+// CTAs are small (four warps, five to seven CTAs per SM), so that the units of a decode batch are nearly
+// all resident at once and SMs are evenly loaded.  With few units the columns are split over KS warps
+// (partial sums added through shared memory): whole 128-column chunks over KS = 2, 64-column halves over
+// KS = 4 and 8.
 #include "grouped_tiled.cuh"
 
 namespace tris {
@@ -25,7 +28,19 @@ constexpr int dec_warps(int proj, int ks) { return proj * ks > 4 ? proj * ks : 4
 constexpr int dec_groups(int proj, int ks) { return dec_warps(proj, ks) / (proj * ks); }
 constexpr int dec_stage_cols(int ks) { return ks == 8 ? 512 : 256; }        // columns staged at a time
 constexpr int dec_row_bytes(int ks) { return 2 * dec_stage_cols(ks) + 16; }  // odd multiple of 16: conflict-free
-constexpr int dec_buf_bytes(int nt, int ks) { return 8 * nt * dec_row_bytes(ks); }
+// One buffer: [projection][chunk]{sub-records of the CTA's outputs, column record}, then [set][8 NT rows]
+struct DecodeLayout {
+  int col_off, chunk_bytes, acts_off, acts_bytes, total;
+};
+__host__ __device__ inline DecodeLayout decode_layout(int max_sub_bytes, int max_steps, int nproj, int nset, int nt, int ks) {
+  DecodeLayout l;
+  l.col_off = dec_groups(nproj, ks) * max_sub_bytes;
+  l.chunk_bytes = l.col_off + col_record_bytes(max_steps);
+  l.acts_off = nproj * (dec_stage_cols(ks) / kChunkCols) * l.chunk_bytes;
+  l.acts_bytes = 8 * nt * dec_row_bytes(ks);
+  l.total = l.acts_off + nset * l.acts_bytes;
+  return l;
+}
 
 __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
   uint32_t d;
@@ -42,19 +57,21 @@ __device__ __forceinline__ void unpack_two(uint32_t w, int i, const uint4& c, co
   b = flip_by_sign(lop3_select(d1, n1, prmt(t1, 0u, 0xAA88u)), t1);
 }
 
+constexpr int dec_min_ctas(int nt, int warps) { return (nt <= 2 ? 28 : 20) / warps; }
+
 // grid (groups of 32 * dec_groups outputs, segments)
 template <int NT, int MODE, int KS>
-__global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), (NT <= 3 ? 28 : 24) / dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS))
+__global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), dec_min_ctas(NT, dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS)))
     grouped_decode_kernel(const __grid_constant__ TiledArgs args) {
   constexpr bool DUAL = MODE != MODE_SINGLE;
   constexpr int P = DUAL ? 2 : 1;
   constexpr int NW = dec_warps(P, KS), OG = dec_groups(P, KS), kThreads = 32 * NW;
   constexpr bool HALF = KS >= 4;                         // a warp takes one half of a chunk
   constexpr int CS = HALF ? KS / 2 : KS;                 // chunks are dealt to CS warps
-  constexpr int kCols = dec_stage_cols(KS), kRow = dec_row_bytes(KS), kBuf = dec_buf_bytes(NT, KS);
+  constexpr int kCols = dec_stage_cols(KS), kRow = dec_row_bytes(KS);
   constexpr int kGroupChunks = kCols / kChunkCols;
   extern __shared__ uint4 smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);    // [buffer][set][row]
+  uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);
 
   if (!args.weights_before_wait) {
     pdl_wait();
@@ -71,55 +88,66 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int p = DUAL ? warp & 1 : 0, og = (warp / P) % OG, ks = warp / (P * OG);
   const int hs = HALF ? (ks & 1) : 0, first_chunk = HALF ? (ks >> 1) : ks;
-  const int o0 = (blockIdx.x * OG + og) * kDecOut, tile = o0 / kTileOut;
+  const int cta_o = blockIdx.x * OG * kDecOut, o0 = cta_o + og * kDecOut;
   const bool mine = o0 < args.out_features;
-  const int row = o0 % kTileOut + g;                     // this lane's outputs inside the tile: row + 8 i
-
   const TrisProjView& v = args.proj[p];
-  const int rec_bytes = v.max_record_bytes, col_bytes = v.col_record_bytes;
-  const int sal_off = record_slices(args.rank) * kSliceBytes, scale_off = sal_off + v.max_sal_words * kStepBytes;
-  // records of the tile and the expert from chunk 0 on; `rec` at this lane's row
-  const uint8_t* rec = static_cast<const uint8_t*>(v.tile_records) +
-                       static_cast<size_t>((expert * args.tiles + tile) * args.chunks) * static_cast<size_t>(rec_bytes) + row * 4;
-  const uint8_t* col = static_cast<const uint8_t*>(v.col_records) + static_cast<size_t>(expert * args.chunks) * static_cast<size_t>(col_bytes);
-  auto load_codes = [&](int c, int sl, uint32_t (&w)[4]) {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + sl * kSliceBytes + row * 12) + t;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = __ldg(src + 32 * i);
-  };
-  auto load_ns_scales = [&](int c, int slot, uint32_t (&w)[4]) {  // second words of the row_pack3 entries
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + scale_off + slot * kSlotBytes + row * 4) + 1;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = __ldg(src + 16 * i);
-  };
-  // Codes and scales of the next slice are in registers before they are needed.  The tables of a chunk and the
-  // salient words of its tile are brought to L1 one chunk ahead, by plain loads (one line per lane) whose
-  // values are dropped when the chunk is reached.
-  uint32_t touched = 0u;
-  auto touch_chunk = [&](int c) {
-    const uint8_t* at = nullptr;
-    if (lane < 16) {
-      if (lane * 128 < col_bytes) at = col + c * col_bytes + lane * 128;
-    } else if (lane - 16 < v.max_sal_words) {
-      at = rec + c * rec_bytes + sal_off + (lane - 16) * kStepBytes - g * 4;
-    }
-    if (at) touched = __ldg(reinterpret_cast<const uint32_t*>(at));
-  };
-  uint32_t codes[4] = {0u, 0u, 0u, 0u}, scales[4] = {0u, 0u, 0u, 0u};
-  auto first_loads = [&]() {
-    if (mine && first_chunk < args.chunks) {
-      load_codes(first_chunk, hs < record_slices(args.rank) ? hs : 0, codes);
-      load_ns_scales(first_chunk, 0, scales);
-      touch_chunk(first_chunk);
+  const int sub_bytes = v.max_record_bytes / kSubs, sal_off = record_slices(args.rank) * kSliceBytes, rows_off = sal_off + v.max_sal_words * kStepBytes;
+  const DecodeLayout L = decode_layout(args.max_sub_bytes, args.max_steps, P, args.num_sets, NT, KS);
+  const int groups = (args.rank + kCols - 1) / kCols;
+  auto buffer = [&](int b) { return sm + b * L.total; };
+
+  // Records of column group gr: per projection and chunk one linear run each of the tile and column record.
+  auto stage_weights = [&](int gr, int b) {
+    const int chunks = min(kGroupChunks, args.chunks - gr * kGroupChunks);
+    const int tile = cta_o / kTileOut, sub = (cta_o % kTileOut) / kSubOut;
+#pragma unroll 1
+    for (int pp = 0; pp < P; ++pp) {
+      const TrisProjView& pv = args.proj[pp];
+      const int rec_bytes = pv.max_record_bytes, run = OG * (rec_bytes / kSubs), col_bytes = pv.col_record_bytes;
+      const int c = gr * kGroupChunks;
+      const uint8_t* rec = static_cast<const uint8_t*>(pv.tile_records) + sub * (rec_bytes / kSubs) +
+                           static_cast<size_t>((expert * args.tiles + tile) * args.chunks + c) * static_cast<size_t>(rec_bytes);
+      const uint8_t* col = static_cast<const uint8_t*>(pv.col_records) + static_cast<size_t>(expert * args.chunks + c) * static_cast<size_t>(col_bytes);
+      uint8_t* dst = buffer(b) + pp * kGroupChunks * L.chunk_bytes;
+#pragma unroll 1
+      for (int ch = 0; ch < chunks; ++ch, rec += rec_bytes, col += col_bytes, dst += L.chunk_bytes) {
+        for (int i = tid * 16; i < run; i += kThreads * 16) cp_async_16(dst + i, rec + i);
+        for (int i = tid * 16; i < col_bytes; i += kThreads * 16) cp_async_16(dst + L.col_off + i, col + i);
+      }
     }
   };
-  first_loads();
+  // Activation rows r0 .. of column group gr, zero up to a multiple of 64 columns.
+  auto stage_acts = [&](int gr, int b, int r0, int rows) {
+    const int c0 = gr * kCols, cols = min(kCols, args.rank - c0);
+    const int pieces = ((cols + kSliceCols - 1) / kSliceCols) * (kSliceCols / 8);
+    constexpr int kPieces = kCols / 8, kStep = kThreads / kPieces;
+    const int piece = tid % kPieces, left = cols - 8 * piece;
+    if (piece < pieces) {
+      uint8_t* d = buffer(b) + L.acts_off + (tid / kPieces) * kRow + piece * 16;
+      const int at = c0 + (left > 0 ? 8 * piece : 0);
+#pragma unroll 2
+      for (int n = tid / kPieces; n < rows; n += kStep, d += kStep * kRow) {
+        const int src = args.row_gather ? args.row_gather[r0 + n] : r0 + n;
+        const size_t off = static_cast<size_t>(src) * args.hidden_stride;
+        if (args.hidden_vec) {
+          cp_async_16(d, args.hidden[0] + off + at, left > 0);
+          if (P == 2 && args.num_sets == 2) cp_async_16(d + L.acts_bytes, args.hidden[1] + off + at, left > 0);
+        } else {
+          *reinterpret_cast<uint4*>(d) = read_piece(args, args.hidden[0] + off + c0, c0, piece, left);
+          if (P == 2 && args.num_sets == 2) *reinterpret_cast<uint4*>(d + L.acts_bytes) = read_piece(args, args.hidden[1] + off + c0, c0, piece, left);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+
+  stage_weights(0, 0);
   if (args.weights_before_wait) {
     pdl_wait();
     pdl_launch_dependents();
   }
 
-  const int groups = (args.rank + kCols - 1) / kCols;
+  int load = 0;  // column groups loaded so far
 #pragma unroll 1
   for (int r0 = row_begin; r0 < row_end; r0 += 8 * NT) {
     const int rows = min(8 * NT, row_end - r0);
@@ -130,96 +158,67 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[m][nt][c] = 0.f;
-
-    // Activation rows of group gr into buffer gr & 1, zero up to a multiple of 64 columns.
-    auto stage = [&](int gr) {
-      const int c0 = gr * kCols, cols = min(kCols, args.rank - c0);
-      const int pieces = ((cols + kSliceCols - 1) / kSliceCols) * (kSliceCols / 8);
-      constexpr int kPieces = kCols / 8;
-      const int piece = tid % kPieces, left = cols - 8 * piece;
-      if (piece < pieces) {
-        uint8_t* d = sm + (gr & 1) * args.num_sets * kBuf + (tid / kPieces) * kRow + piece * 16;
-        const __half* from0 = args.hidden[0] + (left > 0 ? c0 + 8 * piece : 0);
-        const __half* from1 = args.hidden[1] + (left > 0 ? c0 + 8 * piece : 0);
-#pragma unroll 2
-        for (int n = tid / kPieces; n < rows; n += kThreads / kPieces, d += kThreads / kPieces * kRow) {
-          const int src = args.row_gather ? args.row_gather[r0 + n] : r0 + n;
-          const size_t off = static_cast<size_t>(src) * args.hidden_stride;
-          if (args.hidden_vec) {
-            cp_async_16(d, from0 + off, left > 0);
-            if (P == 2 && args.num_sets == 2) cp_async_16(d + kBuf, from1 + off, left > 0);
-          } else {
-            *reinterpret_cast<uint4*>(d) = read_piece(args, args.hidden[0] + off + c0, c0, piece, left);
-            if (P == 2 && args.num_sets == 2) *reinterpret_cast<uint4*>(d + kBuf) = read_piece(args, args.hidden[1] + off + c0, c0, piece, left);
-          }
-        }
+    {
+      const int b = groups > 1 ? load & 1 : 0;
+      if (r0 != row_begin) {
+        __syncthreads();  // the previous pass has read its buffers and partial sums
+        stage_weights(0, b);
       }
-      cp_async_commit();
-    };
-    if (r0 != row_begin) {
-      first_loads();
-      __syncthreads();  // the previous pass has read its rows and partial sums
+      stage_acts(0, b, r0, rows);
     }
-    stage(0);
 #pragma unroll 1
-    for (int gr = 0; gr < groups; ++gr) {
+    for (int gr = 0; gr < groups; ++gr, ++load) {
+      const int b = groups > 1 ? load & 1 : 0;
       cp_async_wait<0>();
       __syncthreads();
-      if (gr + 1 < groups) stage(gr + 1);  // the other buffer was read before the barrier
+      if (gr + 1 < groups) {  // the other buffer was read before the barrier
+        stage_weights(gr + 1, b ^ 1);
+        stage_acts(gr + 1, b ^ 1, r0, rows);
+      }
       if (!mine) continue;
-      const uint8_t* rows_buf = sm + ((gr & 1) * args.num_sets + (args.num_sets == 2 ? p : 0)) * kBuf + g * kRow;
-      const int c_end = min(args.chunks, (gr + 1) * kGroupChunks);
+      const uint8_t* rows_buf = buffer(b) + L.acts_off + (args.num_sets == 2 ? p : 0) * L.acts_bytes + g * kRow;
+      const int chunks = min(kGroupChunks, args.chunks - gr * kGroupChunks);
 #pragma unroll 1
-      for (int c = gr * kGroupChunks + first_chunk; c < c_end; c += CS) {
-        const uint8_t* ccol = col + c * col_bytes;
-        const int cols = args.rank - c * kChunkCols;   // from here on
-        const bool more = c + CS < args.chunks;
-        const uint32_t counts = __ldg(reinterpret_cast<const uint32_t*>(ccol) + 1);  // ColHeader: slots, steps << 8
-        const bool several = (counts & 0xFFu) > 1u;     // row-scale slots in the chunk (groups of fewer than 128 columns)
-        const uint8_t* x_base = rows_buf + (c % kGroupChunks) * (kChunkCols * 2);
-        asm volatile("" ::"r"(touched));
-        if (more) touch_chunk(c + CS);
+      for (int ch = first_chunk; ch < chunks; ch += CS) {
+        const uint8_t* ck = buffer(b) + (p * kGroupChunks + ch) * L.chunk_bytes;
+        const uint8_t* col = ck + L.col_off;
+        const uint8_t* sub = ck + og * sub_bytes;
+        const uint8_t* scales = sub + rows_off + g * 8;
+        const uint8_t* x_base = rows_buf + ch * (kChunkCols * 2);
+        const int cols = args.rank - (gr * kGroupChunks + ch) * kChunkCols;     // from here on
+        const uint32_t counts = reinterpret_cast<const uint32_t*>(col)[1];       // ColHeader: slots, steps << 8
+        const bool several = (counts & 0xFFu) > 1u;  // row-scale slots in the chunk (groups of fewer than 128 columns)
         RowScales rs[4];
+        auto load_scales = [&](int slot) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rs[i] = row_scales_ns(make_uint2(0u, scales[i]));
+          for (int i = 0; i < 4; ++i) rs[i] = row_scales_ns(*reinterpret_cast<const uint2*>(scales + slot * kSlotBytes + i * 64));
+        };
+        load_scales(0);
+#pragma unroll 1
+        for (int sl = hs; sl < (HALF ? hs + 1 : 2) && sl * kSliceCols < cols; ++sl) {
+          if (several) load_scales(col[8 + 2 * sl + (t >> 1)]);  // ColHeader.slot_of_row of the lane's packed row
+          const uint8_t* cw = sub + sl * kSliceBytes + g * 16 + t * 4;
+          uint32_t cur[4];
 #pragma unroll
-        for (int s = 0; s < (HALF ? 1 : 2); ++s) {
-          const int sl = HALF ? hs : s;
-          if (sl * kSliceCols < cols) {
-            uint32_t cur[4];
+          for (int i = 0; i < 4; ++i) cur[i] = *reinterpret_cast<const uint32_t*>(cw + i * 128);
+          const uint4* ct = reinterpret_cast<const uint4*>(col + kColHdrBytes) + sl * 16 + t;
+          const uint8_t* x = x_base + sl * (kSliceCols * 2) + t * 32;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) cur[i] = codes[i];
-            if (!HALF && s == 0 && cols > kSliceCols) {
-              load_codes(c, 1, codes);
-            } else if (more) {
-              load_codes(c + CS, HALF && hs * kSliceCols + CS * kChunkCols < cols ? hs : 0, codes);
-              load_ns_scales(c + CS, 0, scales);
-            }
-            if (several) {
-              uint32_t w[4];
-              load_ns_scales(c, ccol[8 + 2 * sl + (t >> 1)], w);  // ColHeader.slot_of_row of the lane's packed row
+          for (int jj = 0; jj < 2; ++jj) {
+            uint4 bf[NT];
 #pragma unroll
-              for (int i = 0; i < 4; ++i) rs[i] = row_scales_ns(make_uint2(0u, w[i]));
-            }
-            const uint4* ct = reinterpret_cast<const uint4*>(ccol + kColHdrBytes) + sl * 16 + t;
-            const uint8_t* x = x_base + sl * (kSliceCols * 2) + t * 32;
+            for (int nt = 0; nt < NT; ++nt) bf[nt] = *reinterpret_cast<const uint4*>(x + nt * 8 * kRow + jj * 16);
 #pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {
-              uint4 b[NT];
+            for (int j = 0; j < 2; ++j) {
+              const uint4 cs = ct[(2 * jj + j) * 4];
 #pragma unroll
-              for (int nt = 0; nt < NT; ++nt) b[nt] = *reinterpret_cast<const uint4*>(x + nt * 8 * kRow + jj * 16);
+              for (int m = 0; m < 2; ++m) {
+                uint32_t a0, a1, a2, a3;
+                unpack_two(cur[2 * m], 4 * jj + 2 * j, cs, rs[2 * m], a0, a2);
+                unpack_two(cur[2 * m + 1], 4 * jj + 2 * j, cs, rs[2 * m + 1], a1, a3);
 #pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                const uint4 cs = __ldg(ct + (2 * jj + j) * 4);
-#pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                  uint32_t a0, a1, a2, a3;
-                  unpack_two(cur[2 * m], 4 * jj + 2 * j, cs, rs[2 * m], a0, a2);
-                  unpack_two(cur[2 * m + 1], 4 * jj + 2 * j, cs, rs[2 * m + 1], a1, a3);
-#pragma unroll
-                  for (int nt = 0; nt < NT; ++nt)
-                    mma_m16n8k16(acc[m][nt], a0, a1, a2, a3, j ? b[nt].z : b[nt].x, j ? b[nt].w : b[nt].y);
-                }
+                for (int nt = 0; nt < NT; ++nt)
+                  mma_m16n8k16(acc[m][nt], a0, a1, a2, a3, j ? bf[nt].z : bf[nt].x, j ? bf[nt].w : bf[nt].y);
               }
             }
           }
@@ -228,41 +227,36 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
         const int steps = static_cast<int>((counts >> 8) & 0xFFu);
 #pragma unroll 1
         for (int st = hs; st < steps; st += HALF ? 2 : 1) {
-          const uint8_t* ent = ccol + kColHdrBytes + kColTabBytes + st * kColStepBytes;
-          const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + sal_off + st * kStepBytes);
-          const int slot = several ? ccol[12 + st] : 0;  // ColHeader.step_slot
-          const uint32_t* rsrc = reinterpret_cast<const uint32_t*>(rec + c * rec_bytes + scale_off + slot * kSlotBytes + row * 4);
-          const uint4 cs = __ldg(reinterpret_cast<const uint4*>(ent) + t);
-          const uint2 at = __ldg(reinterpret_cast<const uint2*>(ent + 64) + t);
-          uint32_t w[4], rp[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            w[i] = __ldg(wsrc + 8 * i) << (2 * t);
-            rp[i] = __ldg(rsrc + 16 * i);
-          }
-          uint32_t b[NT][2];
+          const uint8_t* ent = col + kColHdrBytes + kColTabBytes + st * kColStepBytes;
+          const uint8_t* wsrc = sub + sal_off + st * kStepBytes + g * 4;
+          const uint8_t* rsrc = scales + (several ? col[12 + st] : 0) * kSlotBytes;  // ColHeader.step_slot
+          const uint4 cs = reinterpret_cast<const uint4*>(ent)[t];
+          const uint2 at = reinterpret_cast<const uint2*>(ent + 64)[t];
+          uint32_t bf[NT][2];
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
             auto ld = [&](uint32_t cc) -> uint32_t { return *reinterpret_cast<const uint16_t*>(x_base + 2 * cc + nt * 8 * kRow); };
-            b[nt][0] = prmt(ld(at.x & 0xFFFFu), ld(at.x >> 16), 0x5410u);
-            b[nt][1] = prmt(ld(at.y & 0xFFFFu), ld(at.y >> 16), 0x5410u);
+            bf[nt][0] = prmt(ld(at.x & 0xFFFFu), ld(at.x >> 16), 0x5410u);
+            bf[nt][1] = prmt(ld(at.y & 0xFFFFu), ld(at.y >> 16), 0x5410u);
           }
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
             uint32_t a[2][2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const __half2 r1 = u32_as_h2(prmt(rp[2 * m + h], 0u, 0x1010u)), r2 = u32_as_h2(prmt(rp[2 * m + h], 0u, 0x3232u));
+              const uint32_t w = *reinterpret_cast<const uint32_t*>(wsrc + (2 * m + h) * 32) << (2 * t);
+              const uint32_t rp = *reinterpret_cast<const uint32_t*>(rsrc + (2 * m + h) * 64);
+              const __half2 r1 = u32_as_h2(prmt(rp, 0u, 0x1010u)), r2 = u32_as_h2(prmt(rp, 0u, 0x3232u));
 #pragma unroll
               for (int i = 0; i < 2; ++i) {
-                const uint32_t tt = w[2 * m + h] << i;
+                const uint32_t tt = w << i;
                 const uint32_t p1 = flip_by_sign(h2_as_u32(__hmul2_rn(u32_as_h2(i ? cs.z : cs.x), r1)), tt);
                 const uint32_t p2 = flip_by_sign(h2_as_u32(__hmul2_rn(u32_as_h2(i ? cs.w : cs.y), r2)), tt << 8);
                 a[h][i] = h2_as_u32(__hadd2_rn(u32_as_h2(p1), u32_as_h2(p2)));
               }
             }
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) mma_m16n8k16(acc[m][nt], a[0][0], a[1][0], a[0][1], a[1][1], b[nt][0], b[nt][1]);
+            for (int nt = 0; nt < NT; ++nt) mma_m16n8k16(acc[m][nt], a[0][0], a[1][0], a[0][1], a[1][1], bf[nt][0], bf[nt][1]);
           }
         }
       }
@@ -370,10 +364,11 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
 
 template <int NT, int MODE, int KS>
 static int launch_decode(const TiledArgs& args, cudaStream_t stream, bool pdl) {
-  const int bufs = args.rank > dec_stage_cols(KS) ? 2 : 1;
   constexpr int P = MODE == MODE_SINGLE ? 1 : 2;
+  const int bufs = args.rank > dec_stage_cols(KS) ? 2 : 1;
   const int part = (KS > 1 || MODE == MODE_DUAL_SILU) ? dec_warps(P, KS) * 2 * NT * 512 : 0;
-  const size_t smem = std::max(bufs * args.num_sets * dec_buf_bytes(NT, KS), part);
+  const size_t smem = std::max(bufs * decode_layout(args.max_sub_bytes, args.max_steps, P, args.num_sets, NT, KS).total, part);
+  TRIS_REQUIRE(smem <= kMostSmem, TRIS_ERR_UNSUPPORTED, "grouped_decode_kernel: %zu bytes of shared memory", smem);
   auto kernel = grouped_decode_kernel<NT, MODE, KS>;
   static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
   int st = configure_smem(kernel, smem, configured);

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
 
   if (warp < kUnpackWarps) {
     // ---- unpack ---------------------------------------------------------------------------------
-    const int wg = warp >> 2, r = wg & 1, row = threadIdx.x & 127;
+    const int wg = warp >> 2, r = wg & 1;
     const TrisProjView& v = args.proj[DUAL ? r : 0];
     const int max_sal = v.max_sal_words, rec_bytes = v.max_record_bytes, col_bytes = v.col_record_bytes;
     const int sal_off = record_slices(args.rank) * kSliceBytes, rows_off = sal_off + max_sal * kStepBytes;
@@ -262,7 +262,10 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
     uint32_t touched = 0u;    // one line of the next column record per lane: a load that only brings it to L1
     uint4 ncodes = make_uint4(0u, 0u, 0u, 0u);
     uint2 nscale = make_uint2(0u, 0u);
-    auto record = [&](int i) { return static_cast<const uint8_t*>(v.tile_records) + static_cast<size_t>(i) * static_cast<size_t>(rec_bytes); };
+    // this warp's 32 output rows: sub-record warp % 4
+    auto record = [&](int i) {
+      return static_cast<const uint8_t*>(v.tile_records) + static_cast<size_t>(kSubs * i + (warp & 3)) * static_cast<size_t>(rec_bytes / kSubs);
+    };
     auto column_record = [&](int i) { return static_cast<const uint8_t*>(v.col_records) + static_cast<size_t>(i) * static_cast<size_t>(col_bytes); };
     auto fetch = [&]() {
       const int tile = DUAL ? w.x : 2 * w.x + r;
@@ -272,8 +275,8 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       nrec = (w.expert * args.tiles + tile) * args.chunks + w.c;
       const uint8_t* rec = record(nrec);
       if (lane * 128 < col_bytes) touched = __ldg(reinterpret_cast<const uint32_t*>(column_record(ncol) + lane * 128));
-      ncodes = ldg_stream(rec + row * 16);
-      nscale = __ldg(reinterpret_cast<const uint2*>(rec + rows_off) + row);
+      ncodes = ldg_stream(rec + lane * 16);
+      nscale = __ldg(reinterpret_cast<const uint2*>(rec + rows_off) + lane);
     };
     fetch();
     while (ok && w.valid()) {
@@ -286,9 +289,9 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       uint32_t sw0 = 0u, sw1 = 0u;
       if (irec >= 0) {
         const uint8_t* rec = record(irec);
-        if (slices > 1) codes1 = ldg_stream(rec + kSliceBytes + row * 16);
-        if (max_sal > 0) sw0 = __ldg(reinterpret_cast<const uint32_t*>(rec + sal_off) + row);
-        if (max_sal > 1) sw1 = __ldg(reinterpret_cast<const uint32_t*>(rec + sal_off + kStepBytes) + row);
+        if (slices > 1) codes1 = ldg_stream(rec + kSliceBytes + lane * 16);
+        if (max_sal > 0) sw0 = __ldg(reinterpret_cast<const uint32_t*>(rec + sal_off) + lane);
+        if (max_sal > 1) sw1 = __ldg(reinterpret_cast<const uint32_t*>(rec + sal_off + kStepBytes) + lane);
       }
       w.next(args);
       if (w.valid()) w.next(args);
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(col));  // ColHeader: counts, slots of the packed rows, slots of the steps
       const uint32_t step_hi = __ldg(reinterpret_cast<const uint32_t*>(col) + 4);
       auto slot_scales = [&](uint32_t sl) {
-        return sl == 0u ? rp0 : __ldg(reinterpret_cast<const uint2*>(record(irec) + rows_off + sl * kSlotBytes) + row);
+        return sl == 0u ? rp0 : __ldg(reinterpret_cast<const uint2*>(record(irec) + rows_off + sl * kSlotBytes) + lane);
       };
       auto publish = [&]() {
         tmem_wait_st();
@@ -339,7 +342,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
         wait_slot();
 #pragma unroll 1
         for (int st = b; st < min(steps, b + 4); ++st) {
-          const uint32_t code = st == 0 ? sw0 : (st == 1 ? sw1 : __ldg(reinterpret_cast<const uint32_t*>(record(irec) + sal_off + st * kStepBytes) + row));
+          const uint32_t code = st == 0 ? sw0 : (st == 1 ? sw1 : __ldg(reinterpret_cast<const uint32_t*>(record(irec) + sal_off + st * kStepBytes) + lane));
           uint32_t a[8];
           unpack_step(code, reinterpret_cast<const uint4*>(ent), slot_scales(step_slots & 0xFFu), a);
           tmem_st<8>(tmem_a + slot.i * kACols + (st - b) * 8, a);
@@ -558,7 +561,7 @@ __global__ void __launch_bounds__(kTileOut) tiled_dump_kernel(TrisProjView v, __
   uint8_t* col = reinterpret_cast<uint8_t*>(smem_raw);
   const int row = threadIdx.x, tile = blockIdx.x, c = blockIdx.y, e = blockIdx.z;
   const RecordGeom geo = record_geom(v);
-  const uint8_t* rec = tile_record(v, geo, e, tile, c);
+  const uint8_t* rec = tile_record(v, geo, e, tile, c) + (row >> 5) * geo.sub_bytes;
   const uint8_t* src = col_record(v, geo, e, c);
   for (int i = row * 16; i < geo.col_bytes; i += kTileOut * 16) *reinterpret_cast<uint4*>(col + i) = *reinterpret_cast<const uint4*>(src + i);
   __syncthreads();
@@ -567,10 +570,10 @@ __global__ void __launch_bounds__(kTileOut) tiled_dump_kernel(TrisProjView v, __
   const ColHeader* hdr = reinterpret_cast<const ColHeader*>(col);
   const int c0 = c * kChunkCols, cols = min(kChunkCols, v.rank - c0);
   __half* out = weights_out + (static_cast<size_t>(e) * v.out_features + o) * v.rank + c0;
-  auto scales = [&](int slot) { return reinterpret_cast<const uint2*>(rec + geo.rows_off + slot * kSlotBytes)[row]; };
+  auto scales = [&](int slot) { return reinterpret_cast<const uint2*>(rec + geo.rows_off + slot * kSlotBytes)[row & 31]; };
   for (int w = 0; w < (cols + 15) / 16; ++w) {
     uint32_t a[8];
-    unpack_word(reinterpret_cast<const uint32_t*>(rec + (w >> 2) * kSliceBytes + row * 16)[w & 3],
+    unpack_word(reinterpret_cast<const uint32_t*>(rec + (w >> 2) * kSliceBytes + (row & 31) * 16)[w & 3],
                 reinterpret_cast<const uint4*>(col + kColHdrBytes) + (w >> 2) * 16 + (w & 3), row_scales_ns(scales(hdr->slot_of_row[w >> 1])), a);
     for (int i = 0; i < 16; ++i)
       if (16 * w + i < cols) out[16 * w + i] = __ushort_as_half(static_cast<unsigned short>(a[i >> 1] >> (16 * (i & 1))));
@@ -578,7 +581,7 @@ __global__ void __launch_bounds__(kTileOut) tiled_dump_kernel(TrisProjView v, __
   for (int st = 0; st < hdr->num_steps; ++st) {  // the salient columns go over the +-0 the main unpack left there
     const uint8_t* ent = col + kColHdrBytes + kColTabBytes + st * kColStepBytes;
     uint32_t a[8];
-    unpack_step(reinterpret_cast<const uint32_t*>(rec + geo.sal_off + st * kStepBytes)[row], reinterpret_cast<const uint4*>(ent),
+    unpack_step(reinterpret_cast<const uint32_t*>(rec + geo.sal_off + st * kStepBytes)[row & 31], reinterpret_cast<const uint4*>(ent),
                 scales(hdr->step_slot[st]), a);
     for (int i = 0; i < 16; ++i) {
       const unsigned at = reinterpret_cast<const uint16_t*>(ent + 64)[i];
@@ -669,6 +672,7 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   a.tiles = tiles_per_expert(a.out_features);
   a.chunks = num_chunks(a.rank);
   a.max_steps = std::max(a.proj[0].max_sal_words, a.proj[1].max_sal_words);
+  a.max_sub_bytes = std::max(a.proj[0].max_record_bytes, a.proj[1].max_record_bytes) / kSubs;
   a.hidden_mode = (route->flags & TRIS_ROUTE_HIDDEN_LANE_ORDER)
                       ? TRIS_OUT_F16_LANE_ORDER
                       : ((route->flags & TRIS_ROUTE_HIDDEN_PAIR_INTERLEAVED) ? TRIS_OUT_F16_PAIR_INTERLEAVED : TRIS_OUT_F16);

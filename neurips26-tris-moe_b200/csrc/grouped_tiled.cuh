@@ -30,6 +30,7 @@ struct TiledArgs {
   int32_t rank, out_features, num_experts;  // the same for both projections
   int32_t tiles, chunks, units_x, row_split;
   int32_t max_steps;            // salient steps a record of either projection can have
+  int32_t max_sub_bytes;        // larger sub-record of the two projections
   int32_t hidden_mode;          // column order of the activation rows (TRIS_OUT_F16 / _PAIR_INTERLEAVED / _LANE_ORDER)
   int32_t hidden_stride;        // halves between activation rows
   int32_t hidden_vec;           // rows can be copied in 16-byte pieces as they are

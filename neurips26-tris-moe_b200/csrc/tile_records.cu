@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(128) build_tile_records_kernel(TrisProjView v,
     if (r2 < 0 || (r2 >> 5) >= v.sign2_rows) return 0u;
     return (qw2[static_cast<size_t>(r2 >> 5) * v.out_features + o] >> (r2 & 31)) & 1u;
   };
-  const int slices = record_slices(v.rank);
+  const int slices = record_slices(v.rank), sub_bytes = record_bytes(v.rank, max_steps, max_slots) / kSubs;
   // codes: item = (packed row, output); two code words each
   for (int i = tid; i < slices * 2 * kTileOut; i += blockDim.x) {
     const int p = i / kTileOut, ol = i % kTileOut, o = o0 + ol, pg = p0 + p;
@@ -194,14 +194,13 @@ __global__ void __launch_bounds__(128) build_tile_records_kernel(TrisProjView v,
       s = qw1[static_cast<size_t>(pg) * v.out_features + o];
       g = plane[(p >> 1) * 2 + (ol >> 6)][(p & 1) * 64 + (ol & 63)];
     }
-    uint32_t* dst = reinterpret_cast<uint32_t*>(rec + (p >> 1) * kSliceBytes + ol * 16) + (p & 1) * 2;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(rec + (ol >> 5) * sub_bytes + (p >> 1) * kSliceBytes + (ol & 31) * 16) + (p & 1) * 2;
     dst[0] = code_word(s & 0xFFFFu, g & 0xFFFFu);
     dst[1] = code_word(s >> 16, g >> 16);
   }
   // salient steps
-  uint32_t* sal = reinterpret_cast<uint32_t*>(rec + slices * kSliceBytes);
   for (int i = tid; i < max_steps * kTileOut; i += blockDim.x) {
-    const int step = i / kTileOut, o = o0 + i % kTileOut;
+    const int step = i / kTileOut, ol = i % kTileOut, o = o0 + ol;
     uint32_t w1 = 0u, w2 = 0u;
     if (step < plan.num_steps && o < v.out_features) {
       for (int j = 0; j < 16; ++j) {
@@ -212,17 +211,18 @@ __global__ void __launch_bounds__(128) build_tile_records_kernel(TrisProjView v,
         w2 |= sign2_bit(pg, bit, o) << j;
       }
     }
-    sal[i] = code_word(w1, ~w2);  // both bits as "negative"
+    reinterpret_cast<uint32_t*>(rec + (ol >> 5) * sub_bytes + slices * kSliceBytes + step * kStepBytes)[ol & 31] =
+        code_word(w1, ~w2);  // both bits as "negative"
   }
   // row scales
-  uint2* rows = reinterpret_cast<uint2*>(rec + slices * kSliceBytes + max_steps * kStepBytes);
   for (int i = tid; i < max_slots * kTileOut; i += blockDim.x) {
-    const int slot = i / kTileOut, o = o0 + i % kTileOut;
+    const int slot = i / kTileOut, ol = i % kTileOut, o = o0 + ol;
     const int grp = slot < kChunkRows ? slot_group[slot] : -1;
     unsigned long long w = 0ull;
     if (o < v.out_features && grp >= 0 && grp < v.num_groups)
       w = static_cast<unsigned long long>(v.row_pack3[(static_cast<size_t>(e) * v.out_features + o) * v.num_groups + grp]);
-    rows[i] = make_uint2(static_cast<uint32_t>(w), static_cast<uint32_t>(w >> 32));
+    reinterpret_cast<uint2*>(rec + (ol >> 5) * sub_bytes + slices * kSliceBytes + max_steps * kStepBytes + slot * kSlotBytes)[ol & 31] =
+        make_uint2(static_cast<uint32_t>(w), static_cast<uint32_t>(w >> 32));
   }
 }
 
@@ -286,7 +286,7 @@ extern "C" int tris_tile_records_build(const TrisProjView* proj, const uint32_t*
                TRIS_ERR_INVALID_ARG, "tris_tile_records_build: record buffers must be 16-byte aligned");
   const BuildDims d = build_dims(*proj);
   // the row-scale slots follow from the record size the plan found (max_record_bytes of the view)
-  const int slots = (proj->max_record_bytes - record_bytes(proj->rank, max_sal_words, 0)) / kSlotBytes;
+  const int slots = (proj->max_record_bytes - record_bytes(proj->rank, max_sal_words, 0)) / (kSubs * kSlotBytes);
   TRIS_REQUIRE(slots >= 1 && slots <= kChunkRows && proj->max_record_bytes == record_bytes(proj->rank, max_sal_words, slots),
                TRIS_ERR_INVALID_ARG, "tris_tile_records_build: max_record_bytes=%d of the view is not the plan's record size",
                proj->max_record_bytes);

@@ -12,12 +12,13 @@
 // sub-stream index (what a parallel decode needs): 12 % more record bytes for a quarter of the
 // instructions.
 //
-//   tile record (expert e, outputs 128*tile .. +127, columns 128*chunk .. +127), one thread per output
-//     codes   2048 B per 64-column slice: [slice][output] 16 B = 4 code words of 16 columns
-//     sal      512 B per salient step:    [step][output] 4 B = 16 salient columns, two sign bits each
-//     rows    1024 B per row-scale slot:  [slot][output] 8 B = row_pack3 word (s_r1, s_r2, ns_d, ns_nd)
+//   tile record (expert e, outputs 128*tile .. +127, columns 128*chunk .. +127): four sub-records of 32
+//   outputs each, so that any run of 32-output groups is one contiguous piece; a sub-record is
+//     codes    512 B per 64-column slice: [slice][output] 16 B = 4 code words of 16 columns
+//     sal      128 B per salient step:    [step][output] 4 B = 16 salient columns, two sign bits each
+//     rows     256 B per row-scale slot:  [slot][output] 8 B = row_pack3 word (s_r1, s_r2, ns_d, ns_nd)
 //   All records of a projection have the same size (TrisProjView.max_record_bytes), so a record is
-//   found without a table.  Every load of a warp is a contiguous 128-, 256- or 512-byte piece.
+//   found without a table.
 //
 //   column record (expert e, chunk), shared by all output tiles
 //     header    64 B  slot of every packed row, slot of every salient step
@@ -46,14 +47,15 @@ constexpr int kTileOut = 128;       // outputs per tile record = threads per unp
 constexpr int kChunkRows = 4;       // packed rows per record
 constexpr int kChunkCols = 32 * kChunkRows;
 constexpr int kSliceCols = 64;      // columns per 16-byte code group
-constexpr int kSliceBytes = kTileOut * 16;
-constexpr int kStepBytes = kTileOut * 4;
-constexpr int kSlotBytes = kTileOut * 8;
+constexpr int kSubOut = 32, kSubs = kTileOut / kSubOut;  // sub-records of a tile
+constexpr int kSliceBytes = kSubOut * 16;                // within a sub-record
+constexpr int kStepBytes = kSubOut * 4;
+constexpr int kSlotBytes = kSubOut * 8;
 constexpr int kMaxSteps = kChunkCols / 16;  // all columns salient
 constexpr int kColHdrBytes = 64;
 constexpr int kColTabBytes = kChunkCols * 4;
 constexpr int kColStepBytes = 96;
-constexpr uint32_t kColMagic = 0x32305254u;  // "TR02": layout version, checked when stored records are adopted
+constexpr uint32_t kColMagic = 0x33305254u;  // "TR03": layout version, checked when stored records are adopted
 
 struct ColHeader {                  // 64 bytes; the unpack reads the first 20 as words
   uint32_t magic;
@@ -75,7 +77,7 @@ __host__ __device__ inline int record_slices(int rank) {
   return s < kChunkCols / kSliceCols ? s : kChunkCols / kSliceCols;
 }
 __host__ __device__ inline int record_bytes(int rank, int max_steps, int max_slots) {
-  return record_slices(rank) * kSliceBytes + max_steps * kStepBytes + max_slots * kSlotBytes;
+  return kSubs * (record_slices(rank) * kSliceBytes + max_steps * kStepBytes + max_slots * kSlotBytes);
 }
 
 // ---- salient step assignment ------------------------------------------------------------------
@@ -189,17 +191,19 @@ __device__ __forceinline__ void unpack_step(uint32_t w, const uint4* sc, uint2 r
 }
 
 // ---- finding records ------------------------------------------------------------------------------
-struct RecordGeom {
-  int32_t rec_bytes, slices, chunks, tiles, sal_off, rows_off, col_bytes;
+struct RecordGeom {  // offsets inside a sub-record; rec_bytes and sub_bytes are sizes
+  int32_t rec_bytes, sub_bytes, slices, chunks, tiles, sal_off, rows_off, slots, col_bytes;
 };
 __host__ __device__ inline RecordGeom record_geom(const TrisProjView& v) {
   RecordGeom g;
   g.rec_bytes = v.max_record_bytes;
+  g.sub_bytes = v.max_record_bytes / kSubs;
   g.slices = record_slices(v.rank);
   g.chunks = num_chunks(v.rank);
   g.tiles = tiles_per_expert(v.out_features);
   g.sal_off = g.slices * kSliceBytes;
   g.rows_off = g.sal_off + v.max_sal_words * kStepBytes;
+  g.slots = (g.sub_bytes - g.rows_off) / kSlotBytes;
   g.col_bytes = v.col_record_bytes;
   return g;
 }

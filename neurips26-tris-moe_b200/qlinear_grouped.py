@@ -204,7 +204,7 @@ def _adopt_stored_derived(payload: dict, dev, E: int, pr: int, O: int, rank: int
     return True
 
 
-TILE_RECORD_MAGIC = 0x32305254  # layout version of the records, first word of every column record
+TILE_RECORD_MAGIC = 0x33305254  # layout version of the records, first word of every column record
 
 
 def _col_record_bytes(view: TrisProjView, total: int) -> int:
