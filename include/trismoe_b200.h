@@ -567,6 +567,24 @@ int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void* x_f16,
                            void* stream);
 
 /*
+ * The same launch sequence for a checkpoint with per-projection input scales and / or null-space
+ * pairs.  Index 0, 1, 2 = gate, up, down; NULL = none.  input_scale multiplies the input of a
+ * projection's backbone (fp16 [H], [H], [I]; QL:3918-3923); (x . C2_e^T) . C1_e^T is added in fp16 to
+ * the projection's output (QL:2318-2333, QL:2611-2633), before SiLU where the projection is gate or up.
+ */
+typedef struct TrisMoeLayerExtras {
+  const void* input_scale[3];
+  const TrisPacked4View* ns_c2[3];
+  const TrisPacked4View* ns_c1[3];
+} TrisMoeLayerExtras;
+
+size_t tris_moe_layer_extras_workspace_bytes(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras,
+                                             int32_t num_tokens);
+int tris_moe_layer_forward_extras(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
+                                  const float* router_logits, int32_t num_tokens, void* y_f16,
+                                  float* router_logits_out, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Same computation as tris_moe_layer_forward for callers that cannot provide a workspace
  * because they are not allowed to allocate device memory: for example a serving process
  * whose memory pool claimed the whole GPU at start-up (a later cudaMalloc fails or

@@ -98,6 +98,18 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
 bool programmatic_launch_default();
 
 // Options of the launches the fused layer path makes.
+// One 4-bit matrix against fp16 rows (packed4_gemm.cu).  w.num_experts = 0: absent.
+struct P4Problem {
+  TrisPacked4View w;
+  const __half* x;
+  __half* out;
+  int x_ld, out_ld;
+  int x_aligned;  // set by packed4_gemm_impl: rows of x start on 16-byte boundaries
+};
+int validate_packed4(const TrisPacked4View* w);
+int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRouteView* route, int num_rows, int out_mode,
+                      bool accumulate, bool silu, cudaStream_t stream);
+
 struct LaunchOpts {
   bool pdl = false;                  // programmatic dependent launch
   bool weights_before_wait = false;  // the route was complete before the predecessor kernel started

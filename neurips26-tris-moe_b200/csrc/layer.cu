@@ -5,6 +5,8 @@
 //   down backbone on the routed rows
 //   grouped down
 //   weighted combine back to token order
+// Input scales and null-space pairs (TrisMoeLayerExtras) join the same sequence: three 4-bit launches and,
+// where gate or up has a pair, SiLU*mul in the epilogue of the second one.
 #include <algorithm>
 #include <mutex>
 
@@ -28,10 +30,15 @@ struct LayerWorkspace {
   __half* mlp;
   __half* hidden_down;
   __half* down_out;
+  __half* up_out;       // gate/up outputs are kept apart where a null-space pair is added to either
+  __half* ns_hidden[2];
+  __half* scaled;
   size_t bytes;
 };
 
-static LayerWorkspace carve(const TrisMoeLayerView* L, int T, char* base) {
+static int ns_hidden_ld(const TrisPacked4View* c2) { return (c2->n + 7) & ~7; }
+
+static LayerWorkspace carve(const TrisMoeLayerView* L, int T, char* base, const TrisMoeLayerExtras* X = nullptr) {
   LayerWorkspace w{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -57,8 +64,50 @@ static LayerWorkspace carve(const TrisMoeLayerView* L, int T, char* base) {
   w.mlp = reinterpret_cast<__half*>(take(2 * R * L->intermediate_size));
   w.hidden_down = reinterpret_cast<__half*>(take(2 * R * L->down.rank));
   w.down_out = reinterpret_cast<__half*>(take(2 * R * L->hidden_size));
+  if (X != nullptr) {
+    const bool gu = X->ns_c2[0] || X->ns_c2[1];
+    w.up_out = reinterpret_cast<__half*>(take(gu ? 2 * R * L->intermediate_size : 0));
+    size_t ld[2] = {0, 0};
+    for (int i = 0; i < 3; ++i)
+      if (X->ns_c2[i]) ld[i & 1] = std::max<size_t>(ld[i & 1], ns_hidden_ld(X->ns_c2[i]));
+    for (int i = 0; i < 2; ++i) w.ns_hidden[i] = reinterpret_cast<__half*>(take(2 * R * ld[i]));
+    size_t scaled = 0;
+    if (X->input_scale[0] || X->input_scale[1]) scaled = static_cast<size_t>(T) * L->hidden_size;
+    if (X->input_scale[2]) scaled = std::max(scaled, R * static_cast<size_t>(L->intermediate_size));
+    w.scaled = reinterpret_cast<__half*>(take(2 * scaled));
+  }
   w.bytes = off;
   return w;
+}
+
+// out = x * scale, rounded to fp16 (what the separate operators feed the backbone with)
+__global__ void scale_columns_kernel(const __half* __restrict__ x, const __half* __restrict__ scale, size_t count, int cols,
+                                     __half* __restrict__ out) {
+  pdl_wait();
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count; i += static_cast<size_t>(gridDim.x) * blockDim.x)
+    out[i] = __hmul(x[i], scale[i % cols]);
+}
+
+static int launch_scale_columns(const __half* x, const void* scale, int rows, int cols, __half* out, cudaStream_t s) {
+  const size_t count = static_cast<size_t>(rows) * cols;
+  return check_cuda(launch_kernel(scale_columns_kernel, dim3(static_cast<unsigned>(std::min<size_t>((count + 255) / 256, 1184))), dim3(256), 0, s, true, 1, x,
+                                  static_cast<const __half*>(scale), count, cols, out),
+                    "scale_columns_kernel launch");
+}
+
+static int validate_extras(const TrisMoeLayerView* L, const TrisMoeLayerExtras* X) {
+  for (int i = 0; i < 3; ++i) {
+    const TrisPacked4View *c2 = X->ns_c2[i], *c1 = X->ns_c1[i];
+    TRIS_REQUIRE((c2 == nullptr) == (c1 == nullptr), TRIS_ERR_INVALID_ARG, "moe layer: null-space pair %d is incomplete", i);
+    if (c2 == nullptr) continue;
+    int st = validate_packed4(c2);
+    if (st == TRIS_OK) st = validate_packed4(c1);
+    if (st != TRIS_OK) return st;
+    const int in = i == 2 ? L->intermediate_size : L->hidden_size, out = i == 2 ? L->hidden_size : L->intermediate_size;
+    TRIS_REQUIRE(c2->k == in && c1->n == out && c1->k == c2->n && c2->num_experts == L->num_experts && c1->num_experts == L->num_experts,
+                 TRIS_ERR_INVALID_ARG, "moe layer: null-space pair %d does not match the layer", i);
+  }
+  return TRIS_OK;
 }
 
 static int validate_layer(const TrisMoeLayerView* L) {
@@ -83,6 +132,18 @@ static int validate_layer(const TrisMoeLayerView* L) {
                TRIS_ERR_INVALID_ARG, "moe layer: projection expert counts differ");
   return TRIS_OK;
 }
+
+// One or two 4-bit backbones on the same dense rows.
+static int launch_packed(const TrisPacked4View* const* w, int count, const __half* x, int rows, int cols, __half* out0, __half* out1,
+                         int out_mode, cudaStream_t s) {
+  P4Problem p[2] = {};
+  for (int i = 0; i < count; ++i) {
+    const int st = validate_packed4(w[i]);
+    if (st != TRIS_OK) return st;
+    p[i] = {*w[i], x, i ? out1 : out0, cols, w[i]->n, 0};
+  }
+  return packed4_gemm_impl(p, count, nullptr, rows, out_mode, false, false, s);
+}
 }  // namespace tris
 
 using namespace tris;
@@ -92,10 +153,11 @@ extern "C" size_t tris_moe_layer_workspace_bytes(const TrisMoeLayerView* layer, 
   return carve(layer, num_tokens, nullptr).bytes;
 }
 
-extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void* x_f16, const float* router_logits,
-                                      int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace,
-                                      size_t workspace_bytes, void* stream) {
+static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
+                         const float* router_logits, int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace,
+                         size_t workspace_bytes, void* stream) {
   int st = validate_layer(layer);
+  if (st == TRIS_OK && extras) st = validate_extras(layer, extras);
   if (st != TRIS_OK) return st;
   TRIS_REQUIRE(x_f16 && y_f16, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward: null x/y");
   TRIS_REQUIRE(num_tokens >= 0, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward: negative token count");
@@ -104,12 +166,14 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
   if (num_tokens == 0) return TRIS_OK;
   const int T = num_tokens;
   TRIS_REQUIRE(workspace != nullptr, TRIS_ERR_WORKSPACE, "tris_moe_layer_forward: null workspace");
-  LayerWorkspace w = carve(layer, T, static_cast<char*>(workspace));
+  LayerWorkspace w = carve(layer, T, static_cast<char*>(workspace), extras);
   TRIS_REQUIRE(workspace_bytes >= w.bytes, TRIS_ERR_WORKSPACE, "tris_moe_layer_forward: workspace %zu < %zu bytes",
                workspace_bytes, w.bytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int R = T * layer->top_k;
   const __half* x = static_cast<const __half*>(x_f16);
+  const void* scale_of[3] = {extras ? extras->input_scale[0] : nullptr, extras ? extras->input_scale[1] : nullptr,
+                             extras ? extras->input_scale[2] : nullptr};
 
   // Launch order.  With logits given, router + route run first, so that the grouped
   // gate/up kernel can stage its weights while the backbone GEMM is still running
@@ -132,10 +196,10 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
   SkinnyProblem probs[3];
   int np = 0;
   const bool packed_gu = layer->packed_gate && layer->packed_up;  // 4-bit backbones are read in place
-  if (!packed_gu) {
-    probs[np++] = {static_cast<const __half*>(layer->shared_gate), w.hidden_gate, layer->gate.rank, gu_mode};
-    probs[np++] = {static_cast<const __half*>(layer->shared_up), w.hidden_up, layer->up.rank, gu_mode};
-  }
+  const SkinnyProblem gu[2] = {{static_cast<const __half*>(layer->shared_gate), w.hidden_gate, layer->gate.rank, gu_mode},
+                               {static_cast<const __half*>(layer->shared_up), w.hidden_up, layer->up.rank, gu_mode}};
+  for (int i = 0; i < 2; ++i)
+    if (!packed_gu && !scale_of[i]) probs[np++] = gu[i];
   const bool logits_given = router_logits != nullptr;
   const float* logits = router_logits;
   if (logits_given) {
@@ -163,13 +227,23 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
     st = launch_shared_hidden(probs, np, x, nullptr, T, layer->hidden_size, s, /*pdl=*/logits_given, nullptr, true);
     if (st != TRIS_OK) return st;
   }
-  if (packed_gu) {
-    st = tris_packed4_grouped_forward(layer->packed_gate, nullptr, x, layer->hidden_size, T, w.hidden_gate, layer->gate.rank,
-                                      gu_mode, 0, s);
+  const TrisPacked4View* packed[2] = {layer->packed_gate, layer->packed_up};
+  if (packed_gu && !scale_of[0] && !scale_of[1]) {
+    st = launch_packed(packed, 2, x, T, layer->hidden_size, w.hidden_gate, w.hidden_up, gu_mode, s);
     if (st != TRIS_OK) return st;
-    st = tris_packed4_grouped_forward(layer->packed_up, nullptr, x, layer->hidden_size, T, w.hidden_up, layer->up.rank, gu_mode,
-                                      0, s);
-    if (st != TRIS_OK) return st;
+  } else {
+    for (int i = 0; i < 2; ++i) {  // one buffer: each backbone has read it when the next scaling starts
+      if (!packed_gu && !scale_of[i]) continue;
+      const __half* xi = x;
+      if (scale_of[i]) {
+        st = launch_scale_columns(x, scale_of[i], T, layer->hidden_size, w.scaled, s);
+        if (st != TRIS_OK) return st;
+        xi = w.scaled;
+      }
+      st = packed_gu ? launch_packed(packed + i, 1, xi, T, layer->hidden_size, i ? w.hidden_up : w.hidden_gate, nullptr, gu_mode, s)
+                     : launch_shared_hidden(&gu[i], 1, xi, nullptr, T, layer->hidden_size, s, /*pdl=*/true, nullptr, true);
+      if (st != TRIS_OK) return st;
+    }
   }
   if (!logits_given) {
     st = route_launch();
@@ -187,16 +261,45 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
   LaunchOpts opts;
   opts.pdl = true;
   opts.weights_before_wait = logits_given;
-  st = grouped_pair_forward_impl(&layer->gate, &layer->up, &route, w.hidden_gate, w.hidden_up, w.mlp, nullptr, 1, s, opts);
+  const bool ns_gu = extras && (extras->ns_c2[0] || extras->ns_c2[1]);
+  P4Problem c2[2] = {}, c1[2] = {};
+  if (ns_gu) {
+    int n2 = 0;
+    for (int i = 0; i < 2; ++i) {
+      c1[i].w.n = layer->intermediate_size;
+      c1[i].out = i ? w.up_out : w.mlp;
+      c1[i].out_ld = layer->intermediate_size;
+      if (!extras->ns_c2[i]) continue;
+      const int ld = ns_hidden_ld(extras->ns_c2[i]);
+      c2[n2++] = {*extras->ns_c2[i], x, w.ns_hidden[i], layer->hidden_size, ld, 0};
+      c1[i] = {*extras->ns_c1[i], w.ns_hidden[i], c1[i].out, ld, layer->intermediate_size, 0};
+    }
+    st = packed4_gemm_impl(c2, n2, &route, R, TRIS_OUT_F16, false, false, s);
+    if (st != TRIS_OK) return st;
+    opts.weights_before_wait = true;  // the route is older than that launch
+  }
+  st = grouped_pair_forward_impl(&layer->gate, &layer->up, &route, w.hidden_gate, w.hidden_up, w.mlp, ns_gu ? w.up_out : nullptr,
+                                 ns_gu ? 0 : 1, s, opts);
   if (st != TRIS_OK) return st;
+  if (ns_gu) {
+    TrisRouteView rows = route;
+    rows.row_gather = nullptr;
+    st = packed4_gemm_impl(c1, 2, &rows, R, TRIS_OUT_F16, true, /*silu=*/true, s);
+    if (st != TRIS_OK) return st;
+  }
 
   // down backbone on routed rows
+  const __half* mlp = w.mlp;
+  if (scale_of[2]) {
+    st = launch_scale_columns(w.mlp, scale_of[2], R, layer->intermediate_size, w.scaled, s);
+    if (st != TRIS_OK) return st;
+    mlp = w.scaled;
+  }
   if (layer->packed_down) {
-    st = tris_packed4_grouped_forward(layer->packed_down, nullptr, w.mlp, layer->intermediate_size, R, w.hidden_down,
-                                      layer->down.rank, down_mode, 0, s);
+    st = launch_packed(&layer->packed_down, 1, mlp, R, layer->intermediate_size, w.hidden_down, nullptr, down_mode, s);
   } else {
     SkinnyProblem down{static_cast<const __half*>(layer->shared_down), w.hidden_down, layer->down.rank, down_mode};
-    st = launch_shared_hidden(&down, 1, w.mlp, nullptr, R, layer->intermediate_size, s, /*pdl=*/true, nullptr, true);
+    st = launch_shared_hidden(&down, 1, mlp, nullptr, R, layer->intermediate_size, s, /*pdl=*/true, nullptr, true);
   }
   if (st != TRIS_OK) return st;
 
@@ -204,11 +307,41 @@ extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void*
   route.row_gather = nullptr;
   route.flags = route_flags(down_mode);
   opts.weights_before_wait = true;
+  P4Problem dc1 = {};
+  if (extras && extras->ns_c2[2]) {
+    const int ld = ns_hidden_ld(extras->ns_c2[2]);
+    const P4Problem dc2{*extras->ns_c2[2], w.mlp, w.ns_hidden[0], layer->intermediate_size, ld, 0};
+    dc1 = {*extras->ns_c1[2], w.ns_hidden[0], w.down_out, ld, layer->hidden_size, 0};
+    st = packed4_gemm_impl(&dc2, 1, &route, R, TRIS_OUT_F16, false, false, s);
+    if (st != TRIS_OK) return st;
+  }
   st = grouped_forward_impl(&layer->down, &route, w.hidden_down, w.down_out, s, opts);
   if (st != TRIS_OK) return st;
+  if (dc1.x != nullptr) {
+    st = packed4_gemm_impl(&dc1, 1, &route, R, TRIS_OUT_F16, true, false, s);
+    if (st != TRIS_OK) return st;
+  }
 
   // combine
   return combine_routed_impl(w.down_out, w.row_of_flat, w.weights, T, layer->top_k, layer->hidden_size, y_f16, s, true);
+}
+
+extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void* x_f16, const float* router_logits,
+                                      int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace,
+                                      size_t workspace_bytes, void* stream) {
+  return layer_forward(layer, nullptr, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, stream);
+}
+
+extern "C" size_t tris_moe_layer_extras_workspace_bytes(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, int32_t num_tokens) {
+  if (layer == nullptr || extras == nullptr || num_tokens < 0 || validate_layer(layer) != TRIS_OK || validate_extras(layer, extras) != TRIS_OK)
+    return 0;
+  return carve(layer, num_tokens, nullptr, extras).bytes;
+}
+
+extern "C" int tris_moe_layer_forward_extras(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
+                                             const float* router_logits, int32_t num_tokens, void* y_f16, float* router_logits_out,
+                                             void* workspace, size_t workspace_bytes, void* stream) {
+  return layer_forward(layer, extras, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, stream);
 }
 
 // ---- variant that allocates nothing ----------------------------------------------------------

@@ -15,195 +15,164 @@
 // Shape of the work: few activation rows (a decode batch, or the rows of one routed segment) against
 // a matrix whose bytes dominate, so the matrix is the A operand of mma.m16n8k16 (16 outputs x 16
 // inputs per instruction, 8 activation rows as the N side) and each nibble is expanded exactly once
-// per pass, in registers.  A CTA owns 16 outputs of one problem; its 8 warps split every 256-column
-// chunk of the contraction (32 columns each) and add their partial sums through shared memory.
+// per pass, in registers.  Lane (g, t) takes word row 4s + t of outputs g and g + 8 of a 32-column slice s:
+// 8 columns of each, A fragments of two K = 16 steps if step j's K positions are columns 8t + 4j .. + 3;
+// the lane's activations of the slice are then 16 contiguous bytes.  Nibbles and activations are read
+// straight from global memory (L2 / L1), up to four slices ahead, and nothing is staged.  Staging 32 KB of
+// nibbles and up to 128 KB of activation rows per CTA whatever the problem's size let one CTA fill an SM:
+// 64 segments of 5 rows, 2048 -> 64 and 64 -> 1024, took 42 us a launch and now take 12; gate and up
+// share a launch.
+// The eight warps of a CTA split the columns as far as there are slices and take further groups of 16 outputs
+// otherwise; partial sums meet in shared memory.  What bounds it: latency of a handful of dependent
+// round trips; launches.
+#include <math.h>
+
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace tris {
 
 constexpr int kP4Threads = 256;
 constexpr int kP4Warps = 8;
-constexpr int kP4TileN = 16;              // outputs per CTA
-constexpr int kP4SuperCols = 4096;        // contraction columns whose nibbles a CTA holds in shared memory at once
-constexpr int kP4SuperWords = kP4SuperCols / 8;
-constexpr int kP4RedStride = 20;          // floats per (warp, activation row) in the reduction buffer
-constexpr int kP4MaxGroups = kP4SuperCols / 32 + 1;  // groups a super chunk can touch (group size >= 32)
-// fp16 scales of 16 outputs + two zero words per group, rounded so that what follows stays 16-byte aligned
-constexpr int kP4GroupBytes = (kP4MaxGroups * (kP4TileN * 2 + 8) + 15) & ~15;
-static_assert((kP4SuperWords * kP4TileN * 4) % 16 == 0 && kP4GroupBytes % 16 == 0, "activation stages must start on 16 bytes");
-
-// activation columns per staged chunk: about 32 KB per stage (64 KB at 128 rows), two stages
-__host__ __device__ constexpr int p4_chunk_cols(int nt) { return nt == 1 ? 2048 : nt == 2 ? 1024 : nt == 4 ? 512 : 256; }
-__host__ __device__ constexpr int p4_row_halfs(int nt) { return p4_chunk_cols(nt) + 8; }  // +16 bytes: rows on different banks
-__host__ __device__ constexpr size_t p4_stage_bytes(int nt) { return static_cast<size_t>(8 * nt) * p4_row_halfs(nt) * 2; }
-__host__ __device__ constexpr size_t p4_red_bytes(int nt) { return static_cast<size_t>(kP4Warps) * 8 * nt * kP4RedStride * 4; }
-__host__ __device__ constexpr size_t p4_smem_bytes(int nt) {
-  return kP4SuperWords * kP4TileN * 4 + kP4GroupBytes + (2 * p4_stage_bytes(nt) > p4_red_bytes(nt) ? 2 * p4_stage_bytes(nt) : p4_red_bytes(nt));
-}
+constexpr int kP4TileN = 16;       // outputs of a warp
+constexpr int kP4SliceCols = 32;
+constexpr int kP4RedStride = 20;   // floats per (warp, activation row) in the reduction buffer
 
 struct P4Args {
-  TrisPacked4View w;
+  P4Problem p[2];
+  int num_problems;
   const int32_t* expert_ids;
   const int32_t* segment_offsets;
   const int32_t* num_segments_dev;
-  int num_segments;  // 0: one problem over all rows (expert 0)
   const int32_t* row_gather;
-  const __half* x;
-  int x_ld;
+  int num_segments;  // 0: no route, one matrix for all rows
+  int num_experts;
   int num_rows;
-  __half* out;
-  int out_ld;
   int out_mode;
   int accumulate;
-  int x_aligned;  // rows of x start on 16-byte boundaries
-  int w_aligned;  // rows of qweight start on 16-byte boundaries
+  int n;       // outputs of either problem, at most
+  int ksplit;  // warps that share 16 outputs: 1, 2, 4 or 8
 };
 
-__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes) : "memory");
-}
-// byte t of `word` holds the nibbles of input columns 2t (low) and 2t+1 (high): returns
+// byte i of `word` holds the nibbles of input columns 2i (low) and 2i+1 (high): returns
 // half2(fp16((q_lo - zero) * scale), fp16((q_hi - zero) * scale)); zc = 1024 + zero as half2
-__device__ __forceinline__ uint32_t p4_dequant_pair(uint32_t word, int t, __half2 zc, __half2 sc) {
-  const uint32_t b = (word >> (8 * t)) & 0xFFu;
+__device__ __forceinline__ uint32_t p4_dequant_pair(uint32_t word, int i, __half2 zc, __half2 sc) {
+  const uint32_t b = prmt(word, 0u, 0x4440u + static_cast<uint32_t>(i));
   const uint32_t v = ((b * 4097u) & 0x000F000Fu) | 0x64006400u;  // 1024 + q, exact in fp16
   return h2_as_u32(__hmul2(__hsub2(u32_as_h2(v), zc), sc));
 }
 
-template <int NT>
+// grid (groups of 16 * 8 / ksplit outputs, segments or 1, problems * CTAs that share a segment's rows)
+// kSilu: both problems belong to one CTA, the second one (up) first, and problem 0's output becomes
+// silu(gate) * up, each rounded to fp16 where separate operators would round it.
+template <int NT, bool kSilu>
 __global__ void __launch_bounds__(kP4Threads) packed4_gemm_kernel(const __grid_constant__ P4Args a) {
   constexpr int kRows = 8 * NT;
-  constexpr int kChunk = p4_chunk_cols(NT);
-  constexpr int kRowHalfs = p4_row_halfs(NT);
-  extern __shared__ __align__(16) unsigned char p4_smem[];
-  uint32_t* ws = reinterpret_cast<uint32_t*>(p4_smem);                                   // [kP4SuperWords][16] nibble words
-  __half* gsc = reinterpret_cast<__half*>(p4_smem + kP4SuperWords * kP4TileN * 4);      // [kP4MaxGroups][16] scales
-  uint32_t* gzw = reinterpret_cast<uint32_t*>(gsc + kP4MaxGroups * kP4TileN);            // [kP4MaxGroups][2] zero words
-  __half* xs = reinterpret_cast<__half*>(p4_smem + kP4SuperWords * kP4TileN * 4 + kP4GroupBytes);  // [2][kRows][kRowHalfs]
-  float* red = reinterpret_cast<float*>(xs);                                             // after the main loop
+  constexpr int kAhead = NT <= 2 ? 4 : (NT == 4 ? 2 : 1);  // slices whose loads are in flight together
+  extern __shared__ __align__(16) float red[];              // [warp][activation row][kP4RedStride]
 
   pdl_wait();  // activations (and a device-built route) come from the kernels before this one
+  pdl_launch_dependents();
   int e = 0, row0 = 0, rows = a.num_rows;
   if (a.num_segments > 0) {
     const int seg = blockIdx.y;
     const int nseg = a.num_segments_dev ? min(*a.num_segments_dev, a.num_segments) : a.num_segments;
     if (seg >= nseg) return;
     e = a.expert_ids[seg];
-    if (e < 0 || e >= a.w.num_experts) return;
+    if (e < 0 || e >= a.num_experts) return;
     row0 = a.segment_offsets[seg];
     rows = min(a.segment_offsets[seg + 1], a.num_rows) - row0;
   }
-  const int N = a.w.n_count ? a.w.n_count[e] : a.w.n;
-  const int K = a.w.k_count ? a.w.k_count[e] : a.w.k;
-  const int G = max(1, a.w.g_count ? a.w.g_count[e] : a.w.num_groups);
-  const int n0 = blockIdx.x * kP4TileN;
-  if (rows <= 0 || n0 >= N || row0 < 0) return;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int og = warp / a.ksplit, ks = warp % a.ksplit;
+  const int outs = (kP4Warps / a.ksplit) * kP4TileN;
+  const int cta_n = blockIdx.x * outs, n0 = cta_n + og * kP4TileN;
+  if (rows <= 0 || row0 < 0) return;
+  const int np = kSilu ? 1 : a.num_problems;  // problems that CTAs of their own take
+  const int first = kSilu ? a.num_problems - 1 : static_cast<int>(blockIdx.z) % np;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int n_off = a.w.n_off ? a.w.n_off[e] : 0;
-  const int g_off = a.w.g_off ? a.w.g_off[e] : 0;
-  const int32_t* qw = a.w.qweight + static_cast<size_t>(a.w.kw_off ? a.w.kw_off[e] : 0) * a.w.q_ld + n_off;
-  const int32_t* qz = a.w.qzeros + static_cast<size_t>(g_off) * a.w.z_ld + (a.w.z_off ? a.w.z_off[e] : 0);
-  const __half* sc = static_cast<const __half*>(a.w.scales) + static_cast<size_t>(g_off) * a.w.s_ld + n_off;
-  const int kwords = (K + 7) >> 3;
-  const bool quad16 = a.w_aligned && ((n_off + n0) & 3) == 0;  // 16-byte copies of four outputs' words
-
-  // stage activation rows [r0, r0 + kRows) x columns [k, k + kChunk) into stage `st`: 16-byte granules, zero past K / rows
-  auto stage_x = [&](int st, int r0, int k_begin) {
-    __half* base = xs + static_cast<size_t>(st) * kRows * kRowHalfs;
-    for (int i = tid; i < kRows * (kChunk / 8); i += kP4Threads) {
-      const int r = i / (kChunk / 8), c = i % (kChunk / 8);
-      const int k = k_begin + 8 * c;
-      const int valid = (r0 + r < rows) ? max(0, min(8, K - k)) : 0;
-      __half* dst = base + r * kRowHalfs + 8 * c;
-      if (k >= ((K + 31) & ~31)) continue;  // past the last 32-column block that holds a column: never read
-      const int src_row = valid ? (a.row_gather ? a.row_gather[row0 + r0 + r] : row0 + r0 + r) : 0;
-      const __half* src = a.x + static_cast<size_t>(src_row) * a.x_ld + k;
-      if (a.x_aligned) {
-        cp_async16_zfill(dst, valid ? src : a.x, 2 * valid);
-      } else {
-        for (int j = 0; j < 8; ++j) dst[j] = j < valid ? src[j] : __ushort_as_half(0);
-      }
-    }
-  };
-
-  for (int r0 = 0; r0 < rows; r0 += kRows) {
+  for (int r0 = (blockIdx.z / np) * kRows; r0 < rows; r0 += kRows * (gridDim.z / np)) {
+#pragma unroll 1
+  for (int pi = first; pi >= (kSilu ? 0 : first); --pi) {
+    const P4Problem& pr = a.p[pi];
+    const TrisPacked4View& w = pr.w;
+    const bool present = w.num_experts > 0;
+    const int N = w.n_count ? w.n_count[e] : w.n;
+    const int K = !present ? 0 : (w.k_count ? w.k_count[e] : w.k);
+    const int G = max(1, w.g_count ? w.g_count[e] : w.num_groups);
+    if (cta_n >= N) continue;
+    const int n_off = w.n_off ? w.n_off[e] : 0;
+    const int g_off = w.g_off ? w.g_off[e] : 0;
+    // outputs past N repeat the last one
+    const int na = min(n0 + g, N - 1), nb = min(n0 + g + 8, N - 1);
+    const int32_t* qw = w.qweight + static_cast<size_t>(w.kw_off ? w.kw_off[e] : 0) * w.q_ld + n_off;
+    const int32_t* qz = w.qzeros + static_cast<size_t>(g_off) * w.z_ld + (w.z_off ? w.z_off[e] : 0);
+    const __half* sc = static_cast<const __half*>(w.scales) + static_cast<size_t>(g_off) * w.s_ld + n_off;
+    const int kwords = (K + 7) >> 3, slices = (K + kP4SliceCols - 1) / kP4SliceCols;
+    const int per = (slices + a.ksplit - 1) / a.ksplit;
+    const int s_begin = n0 < N ? ks * per : 0, s_end = n0 < N ? min(slices, s_begin + per) : 0;
+    const int gs = w.group_size > 0 ? w.group_size : (K + kP4SliceCols);  // a multiple of 32 where there are several groups
     float acc[NT][4];
+    const __half* xr[NT];  // this lane's activation row of each tile; rows past the last repeat it
 #pragma unroll
-    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-
-    for (int kk0 = 0; kk0 < K; kk0 += kP4SuperCols) {
-      // every nibble this CTA needs for these columns, requested at once: [word row][16 outputs]
-      const int nkw = min(kP4SuperWords, kwords - (kk0 >> 3));
-      for (int i = tid; i < nkw * 4; i += kP4Threads) {
-        const int kw = i >> 2, q = i & 3;
-        const int32_t* row = qw + static_cast<size_t>((kk0 >> 3) + kw) * a.w.q_ld;
-        uint32_t* dst = ws + kw * kP4TileN + 4 * q;
-        if (quad16 && n0 + 4 * q + 3 < N) {
-          cp_async16_zfill(dst, row + n0 + 4 * q, 16);
-        } else {  // ragged edge or unaligned rows: word by word, outputs past N repeat the last one
+    for (int i = 0; i < NT; ++i) {
+      acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+      const int r = row0 + min(r0 + 8 * i + g, rows - 1);
+      xr[i] = pr.x + static_cast<size_t>(a.row_gather ? a.row_gather[r] : r) * pr.x_ld + 8 * t;
+    }
+    int grp = -1;
+    __half2 zca = {}, zcb = {}, sca = {}, scb = {};
+#pragma unroll 1
+    for (int s = s_begin; s < s_end; s += kAhead) {
+      uint32_t wa[kAhead], wb[kAhead];
+      uint4 xv[kAhead][NT];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) cp_async_4(dst + j, row + min(n0 + 4 * q + j, N - 1));
-        }
-      }
-      const int span = min(kP4SuperCols, K - kk0);
-      // scales and zero points of the groups these columns fall into (outputs past N repeat the last one)
-      const int gs = a.w.group_size > 0 ? a.w.group_size : (K + kP4SuperCols);
-      const int grp0 = min(kk0 / gs, G - 1);
-      const int ngrp = min((kk0 + span - 1) / gs, G - 1) - grp0 + 1;
-      for (int i = tid; i < ngrp * (kP4TileN + 2); i += kP4Threads) {
-        const int gi = i / (kP4TileN + 2), j = i % (kP4TileN + 2);
-        if (j < kP4TileN) {
-          gsc[gi * kP4TileN + j] = __ldg(sc + static_cast<size_t>(grp0 + gi) * a.w.s_ld + min(n0 + j, N - 1));
-        } else {
-          gzw[gi * 2 + (j - kP4TileN)] =
-              static_cast<uint32_t>(__ldg(qz + static_cast<size_t>(grp0 + gi) * a.w.z_ld + (min(n0 + 8 * (j - kP4TileN), N - 1) >> 3)));
-        }
-      }
-      const int nchunks = (span + kChunk - 1) / kChunk;
-      stage_x(0, r0, kk0);
-      cp_async_commit();
-      for (int c = 0; c < nchunks; ++c) {
-        if (c + 1 < nchunks) {
-          stage_x((c + 1) & 1, r0, kk0 + (c + 1) * kChunk);
-          cp_async_commit();
-          cp_async_wait<1>();
-        } else {
-          cp_async_wait<0>();
-        }
-        __syncthreads();
-        const __half* xb = xs + static_cast<size_t>(c & 1) * kRows * kRowHalfs;
-        for (int blk = warp; blk < kChunk / 32; blk += kP4Warps) {
-          const int kl = c * kChunk + 32 * blk;  // column inside this super chunk
-          const int kc = kk0 + kl;
-          if (kc >= K) break;
-          const int gi = min(kc / gs, G - 1) - grp0;
-          const uint32_t za = (gzw[gi * 2] >> (4 * g)) & 0xFu, zb = (gzw[gi * 2 + 1] >> (4 * g)) & 0xFu;
-          const __half2 zca = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + za + 1u)));
-          const __half2 zcb = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + zb + 1u)));
-          const __half2 sca = __half2half2(gsc[gi * kP4TileN + g]);
-          const __half2 scb = __half2half2(gsc[gi * kP4TileN + g + 8]);
-          const uint32_t* wk = ws + (kl >> 3) * kP4TileN;
+      for (int u = 0; u < kAhead; ++u) {
+        const int kw = 4 * (s + u) + t, k = 8 * kw;
+        const bool in = s + u < s_end && kw < kwords;
+        wa[u] = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + na)) : 0u;
+        wb[u] = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + nb)) : 0u;
 #pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const uint32_t a0 = p4_dequant_pair(wk[(2 * s) * kP4TileN + g], t, zca, sca);
-            const uint32_t a1 = p4_dequant_pair(wk[(2 * s) * kP4TileN + g + 8], t, zcb, scb);
-            const uint32_t a2 = p4_dequant_pair(wk[(2 * s + 1) * kP4TileN + g], t, zca, sca);
-            const uint32_t a3 = p4_dequant_pair(wk[(2 * s + 1) * kP4TileN + g + 8], t, zcb, scb);
-            const __half* xk = xb + g * kRowHalfs + 32 * blk + 16 * s + 2 * t;
+        for (int i = 0; i < NT; ++i) {
+          const __half* src = xr[i] + kP4SliceCols * (s + u);
+          xv[u][i] = make_uint4(0u, 0u, 0u, 0u);
+          if (in) {
+            if (pr.x_aligned && k + 8 <= K) {
+              xv[u][i] = *reinterpret_cast<const uint4*>(src);
+            } else {  // ragged end or unaligned rows; columns past K read as zeros
+              uint32_t h[8];
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-              const uint32_t b0 = *reinterpret_cast<const uint32_t*>(xk + i * 8 * kRowHalfs);
-              const uint32_t b1 = *reinterpret_cast<const uint32_t*>(xk + i * 8 * kRowHalfs + 8);
-              mma_m16n8k16(acc[i], a0, a1, a2, a3, b0, b1);
+              for (int j = 0; j < 8; ++j) h[j] = k + j < K ? __half_as_ushort(src[j]) : 0u;
+              xv[u][i] = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
             }
           }
         }
-        __syncthreads();  // this stage (and, after the last chunk, the nibble tile) may be overwritten now
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        if (s + u >= s_end) break;
+        const int gi = min((s + u) * kP4SliceCols / gs, G - 1);
+        if (gi != grp) {
+          grp = gi;
+          const int32_t* z = qz + static_cast<size_t>(gi) * w.z_ld;
+          const uint32_t za = (static_cast<uint32_t>(__ldg(z + (na >> 3))) >> (4 * (na & 7))) & 0xFu;
+          const uint32_t zb = (static_cast<uint32_t>(__ldg(z + (nb >> 3))) >> (4 * (nb & 7))) & 0xFu;
+          zca = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + za + 1u)));
+          zcb = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + zb + 1u)));
+          sca = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + na));
+          scb = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + nb));
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t a0 = p4_dequant_pair(wa[u], 2 * j, zca, sca), a1 = p4_dequant_pair(wb[u], 2 * j, zcb, scb);
+          const uint32_t a2 = p4_dequant_pair(wa[u], 2 * j + 1, zca, sca), a3 = p4_dequant_pair(wb[u], 2 * j + 1, zcb, scb);
+#pragma unroll
+          for (int i = 0; i < NT; ++i) mma_m16n8k16(acc[i], a0, a1, a2, a3, j ? xv[u][i].z : xv[u][i].x, j ? xv[u][i].w : xv[u][i].y);
+        }
       }
     }
-
-    // add the eight warps' partial sums: red[warp][activation row][output]
+    // add the partial sums of the warps that share 16 outputs
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       float* base = red + (warp * kRows + 8 * i + 2 * t) * kP4RedStride;
@@ -213,55 +182,55 @@ __global__ void __launch_bounds__(kP4Threads) packed4_gemm_kernel(const __grid_c
       base[kP4RedStride + g + 8] = acc[i][3];
     }
     __syncthreads();
-    for (int i = tid; i < kRows * kP4TileN; i += kP4Threads) {
-      const int r = i / kP4TileN, n = i % kP4TileN;
-      if (r0 + r >= rows || n0 + n >= N) continue;
+    for (int i = tid; i < min(kRows, rows - r0) * outs; i += kP4Threads) {
+      const int r = i / outs, j = i - r * outs, n = cta_n + j;
+      if (n >= N) continue;
+      const float* src = red + ((j / kP4TileN) * a.ksplit * kRows + r) * kP4RedStride + j % kP4TileN;
       float sum = 0.f;
-#pragma unroll
-      for (int w = 0; w < kP4Warps; ++w) sum += red[(w * kRows + r) * kP4RedStride + n];
-      __half* dst = a.out + static_cast<size_t>(row0 + r0 + r) * a.out_ld + out_mode_pos(n0 + n, a.out_mode);
+      for (int v = 0; v < a.ksplit; ++v) sum += src[v * kRows * kP4RedStride];
+      const size_t row = static_cast<size_t>(row0 + r0 + r);
+      const int col = out_mode_pos(n, a.out_mode);
+      __half* dst = pr.out + row * pr.out_ld + col;
       __half v = __float2half_rn(sum);
-      if (a.accumulate) v = __hadd(*dst, v);  // what out.add_(compensation) does in fp16
+      if (a.accumulate) v = present ? __hadd(*dst, v) : *dst;  // what out.add_(compensation) does in fp16
+      if constexpr (kSilu) {
+        if (pi == 0) {  // this thread wrote the other problem's element too
+          const float f = __half2float(v);
+          v = __hmul(__float2half_rn(f / (1.f + expf(-f))), a.p[1].out[row * a.p[1].out_ld + col]);
+        }
+      }
       *dst = v;
     }
     __syncthreads();
   }
-  pdl_launch_dependents();
+  }
 }
 
 template <int NT>
-static int launch_p4(const P4Args& args, dim3 grid, cudaStream_t stream) {
-  constexpr size_t smem = p4_smem_bytes(NT);
-  if (smem > 48 * 1024) {
-    TRIS_CUDA(cudaFuncSetAttribute(packed4_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  }
-  return check_cuda(launch_kernel(packed4_gemm_kernel<NT>, grid, dim3(kP4Threads), smem, stream, programmatic_launch_default(), 1, args),
+static int launch_p4(const P4Args& args, bool silu, dim3 grid, cudaStream_t stream, bool pdl) {
+  constexpr size_t smem = static_cast<size_t>(kP4Warps) * 8 * NT * kP4RedStride * sizeof(float);
+  static_assert(smem <= 48 * 1024, "reduction buffer");
+  return check_cuda(silu ? launch_kernel(packed4_gemm_kernel<NT, true>, grid, dim3(kP4Threads), smem, stream, pdl, 1, args)
+                         : launch_kernel(packed4_gemm_kernel<NT, false>, grid, dim3(kP4Threads), smem, stream, pdl, 1, args),
                     "packed4_gemm_kernel launch");
 }
 
-}  // namespace tris
-
-using namespace tris;
-
-extern "C" int tris_packed4_grouped_forward(const TrisPacked4View* w, const TrisRouteView* route, const void* x_f16,
-                                            int32_t x_ld, int32_t num_rows, void* out_f16, int32_t out_ld,
-                                            int32_t out_mode, int32_t accumulate, void* stream) {
-  TRIS_REQUIRE(w && x_f16 && out_f16, TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: null pointer");
-  TRIS_REQUIRE(w->qweight && w->qzeros && w->scales, TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: null matrix pointer");
-  TRIS_REQUIRE(w->n > 0 && w->k >= 0 && w->num_groups >= 0 && w->num_experts > 0 && w->q_ld > 0 && w->z_ld > 0 && w->s_ld > 0,
-               TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: bad sizes n=%d k=%d groups=%d", w->n, w->k, w->num_groups);
-  TRIS_REQUIRE(w->group_size <= 0 || w->group_size % 32 == 0 || w->num_groups <= 1, TRIS_ERR_UNSUPPORTED,
-               "tris_packed4_grouped_forward: group size %d (a multiple of 32, or a single group, is supported)", w->group_size);
-  TRIS_REQUIRE(out_mode == TRIS_OUT_F16 || out_mode == TRIS_OUT_F16_PAIR_INTERLEAVED || out_mode == TRIS_OUT_F16_LANE_ORDER,
-               TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: out_mode %d", out_mode);
-  TRIS_REQUIRE(out_mode == TRIS_OUT_F16 || w->n % 32 == 0, TRIS_ERR_INVALID_ARG,
-               "tris_packed4_grouped_forward: permuted output layouts need n %% 32 == 0");
-  TRIS_REQUIRE(x_ld >= w->k && out_ld >= w->n && num_rows >= 0, TRIS_ERR_INVALID_ARG,
-               "tris_packed4_grouped_forward: row strides x_ld=%d out_ld=%d", x_ld, out_ld);
+// One launch for one or two problems on the same rows (gate and up).  `silu`: see the kernel; needs
+// two problems with `accumulate`, of which one may be absent (num_experts = 0; its `w.n` is still read).
+int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRouteView* route, int num_rows, int out_mode,
+                      bool accumulate, bool silu, cudaStream_t stream) {
   if (num_rows == 0) return TRIS_OK;
   P4Args args{};
-  args.w = *w;
-  int hint = num_rows;
+  args.num_problems = num_problems;
+  int hint = num_rows, k = 1;
+  for (int i = 0; i < num_problems; ++i) {
+    const TrisPacked4View& w = problems[i].w;
+    args.p[i] = problems[i];
+    args.p[i].x_aligned = ((reinterpret_cast<uintptr_t>(problems[i].x) & 15u) == 0 && problems[i].x_ld % 8 == 0) ? 1 : 0;
+    args.n = std::max(args.n, w.n);
+    args.num_experts = std::max(args.num_experts, w.num_experts);
+    k = std::max(k, w.num_experts > 0 ? w.k : 0);
+  }
   if (route) {
     TRIS_REQUIRE(route->expert_ids && route->segment_offsets && route->num_segments >= 0, TRIS_ERR_INVALID_ARG,
                  "tris_packed4_grouped_forward: incomplete route");
@@ -272,22 +241,52 @@ extern "C" int tris_packed4_grouped_forward(const TrisPacked4View* w, const Tris
     args.num_segments = route->num_segments;
     args.row_gather = route->row_gather;
     if (route->max_rows_per_segment > 0) hint = std::min(hint, route->max_rows_per_segment);
+    // mean + 2 sigma of a balanced router: a longer segment takes several passes
+    const double mean = static_cast<double>(num_rows) / route->num_segments;
+    hint = std::max(1, std::min(hint, static_cast<int>(ceil(mean + 2.0 * sqrt(mean)))));
   }
-  args.x = static_cast<const __half*>(x_f16);
-  args.x_ld = x_ld;
   args.num_rows = num_rows;
-  args.out = static_cast<__half*>(out_f16);
-  args.out_ld = out_ld;
   args.out_mode = out_mode;
   args.accumulate = accumulate ? 1 : 0;
-  args.x_aligned = ((reinterpret_cast<uintptr_t>(x_f16) & 15u) == 0 && x_ld % 8 == 0) ? 1 : 0;
-  args.w_aligned = ((reinterpret_cast<uintptr_t>(w->qweight) & 15u) == 0 && w->q_ld % 4 == 0) ? 1 : 0;
-  const dim3 grid(ceil_div(w->n, kP4TileN), route ? route->num_segments : 1);
+  // eight warps share 16 outputs where there are columns for all of them, else they take more outputs
+  const int slices = ceil_div(k, kP4SliceCols);
+  args.ksplit = slices >= 8 ? 8 : (slices >= 4 ? 4 : (slices >= 2 ? 2 : 1));
+  dim3 grid(ceil_div(args.n, kP4TileN * kP4Warps / args.ksplit), route ? route->num_segments : 1);
   TRIS_REQUIRE(grid.y <= 65535u, TRIS_ERR_UNSUPPORTED, "tris_packed4_grouped_forward: more than 65535 segments");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (hint <= 8) return launch_p4<1>(args, grid, s);
-  if (hint <= 16) return launch_p4<2>(args, grid, s);
-  if (hint <= 32) return launch_p4<4>(args, grid, s);
-  if (hint <= 64) return launch_p4<8>(args, grid, s);
-  return launch_p4<16>(args, grid, s);
+  // passes of 64 rows go to CTAs of their own while that leaves four per SM
+  const unsigned np = silu ? 1u : static_cast<unsigned>(num_problems);
+  grid.z = np * std::max(1u, std::min(static_cast<unsigned>(ceil_div(hint, 64)), 592u / std::max(1u, grid.x * grid.y * np)));
+  const bool pdl = programmatic_launch_default();
+  if (hint <= 8) return launch_p4<1>(args, silu, grid, stream, pdl);
+  if (hint <= 16) return launch_p4<2>(args, silu, grid, stream, pdl);
+  if (hint <= 32) return launch_p4<4>(args, silu, grid, stream, pdl);
+  return launch_p4<8>(args, silu, grid, stream, pdl);
+}
+
+int validate_packed4(const TrisPacked4View* w) {
+  TRIS_REQUIRE(w->qweight && w->qzeros && w->scales, TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: null matrix pointer");
+  TRIS_REQUIRE(w->n > 0 && w->k >= 0 && w->num_groups >= 0 && w->num_experts > 0 && w->q_ld > 0 && w->z_ld > 0 && w->s_ld > 0,
+               TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: bad sizes n=%d k=%d groups=%d", w->n, w->k, w->num_groups);
+  TRIS_REQUIRE(w->group_size <= 0 || w->group_size % 32 == 0 || w->num_groups <= 1, TRIS_ERR_UNSUPPORTED,
+               "tris_packed4_grouped_forward: group size %d (a multiple of 32, or a single group, is supported)", w->group_size);
+  return TRIS_OK;
+}
+}  // namespace tris
+
+using namespace tris;
+
+extern "C" int tris_packed4_grouped_forward(const TrisPacked4View* w, const TrisRouteView* route, const void* x_f16,
+                                            int32_t x_ld, int32_t num_rows, void* out_f16, int32_t out_ld,
+                                            int32_t out_mode, int32_t accumulate, void* stream) {
+  TRIS_REQUIRE(w && x_f16 && out_f16, TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: null pointer");
+  const int st = validate_packed4(w);
+  if (st != TRIS_OK) return st;
+  TRIS_REQUIRE(out_mode == TRIS_OUT_F16 || out_mode == TRIS_OUT_F16_PAIR_INTERLEAVED || out_mode == TRIS_OUT_F16_LANE_ORDER,
+               TRIS_ERR_INVALID_ARG, "tris_packed4_grouped_forward: out_mode %d", out_mode);
+  TRIS_REQUIRE(out_mode == TRIS_OUT_F16 || w->n % 32 == 0, TRIS_ERR_INVALID_ARG,
+               "tris_packed4_grouped_forward: permuted output layouts need n %% 32 == 0");
+  TRIS_REQUIRE(x_ld >= w->k && out_ld >= w->n && num_rows >= 0, TRIS_ERR_INVALID_ARG,
+               "tris_packed4_grouped_forward: row strides x_ld=%d out_ld=%d", x_ld, out_ld);
+  const P4Problem problem{*w, static_cast<const __half*>(x_f16), static_cast<__half*>(out_f16), x_ld, out_ld, 0};
+  return packed4_gemm_impl(&problem, 1, route, num_rows, out_mode, accumulate != 0, false, static_cast<cudaStream_t>(stream));
 }

@@ -17,7 +17,7 @@ import torch
 from torch import nn
 
 from . import _native, envflags
-from ._native import TrisMoeLayerView
+from ._native import TrisMoeLayerExtras, TrisMoeLayerView
 from .ns_compensation import Packed4Linear
 from .qlinear_grouped import (
     build_grouped_route,
@@ -197,9 +197,27 @@ class TrisSparseMoeBlock(nn.Module):
             setattr(v, "packed_" + name, None)
         return v
 
-    def workspace(self, num_tokens: int, device) -> torch.Tensor:
+    def _layer_extras(self, dev) -> Optional[TrisMoeLayerExtras]:
+        """Input scales and null-space pairs as the native layer takes them; None where the layer has none."""
+        if not (self.input_scales or self.ns_payloads):
+            return None
+        from .ns_compensation import prepare_ns_payload
+
+        ex = TrisMoeLayerExtras()
+        for i, name in enumerate(("gate", "up", "down")):
+            if name in self.input_scales:
+                ex.input_scale[i] = self.input_scales[name].data_ptr()
+            if name in self.ns_payloads:
+                p = prepare_ns_payload(self.ns_payloads[name], dev)
+                ex.ns_c2[i], ex.ns_c1[i] = C.addressof(p["_tris_c2_view"]), C.addressof(p["_tris_c1_view"])
+        return ex
+
+    def workspace(self, num_tokens: int, device, extras: Optional[TrisMoeLayerExtras] = None) -> torch.Tensor:
         lib = _native.load()
-        need = int(lib.tris_moe_layer_workspace_bytes(C.byref(self.layer_view()), int(num_tokens)))
+        if extras is None:
+            need = int(lib.tris_moe_layer_workspace_bytes(C.byref(self.layer_view()), int(num_tokens)))
+        else:
+            need = int(lib.tris_moe_layer_extras_workspace_bytes(C.byref(self.layer_view()), C.byref(extras), int(num_tokens)))
         if need == 0 and num_tokens > 0:
             raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
         if self._workspace is None or self._workspace.numel() < need or self._workspace.device != device:
@@ -245,8 +263,9 @@ class TrisSparseMoeBlock(nn.Module):
         ``OlmoeSparseMoeBlock.forward`` (modeling_olmoe.py:1046-1105).  ``router_logits``
         (fp32 ``[T, E]``) may be passed in to skip the router linear."""
         _native.require_cuda(hidden_states, "TrisSparseMoeBlock.forward")
-        if not envflags.grouped_experts_enabled() or self.input_scales or self.ns_payloads:
-            # TRIS_GROUPED_EXPERTS=0, per-projection input scales or null-space pairs: operator by operator
+        wide_router = self.num_experts > 256 or self.top_k > 32  # more than the native router takes
+        if not envflags.grouped_experts_enabled() or (wide_router and (self.input_scales or self.ns_payloads)):
+            # TRIS_GROUPED_EXPERTS=0: operator by operator
             return self.forward_grouped_ops(hidden_states, router_logits)
         if hidden_states.dtype != torch.float16:
             raise RuntimeError(f"trismoe_b200: grouped expert kernels require float16 hidden states, got {hidden_states.dtype}")
@@ -256,6 +275,11 @@ class TrisSparseMoeBlock(nn.Module):
         T = int(x.shape[0])
         dev = x.device
         y = torch.empty_like(x)
+        extras = self._layer_extras(dev)
+        returned = router_logits
+        if extras is not None and router_logits is None:
+            # such blocks route by fp16 logits and return them
+            router_logits = returned = torch.nn.functional.linear(x, self.gate.weight)
         if router_logits is not None:
             logits = router_logits.reshape(T, self.num_experts).to(torch.float32).contiguous()
             logits_in, logits_out = logits.data_ptr(), None
@@ -263,7 +287,7 @@ class TrisSparseMoeBlock(nn.Module):
             logits = torch.empty((T, self.num_experts), dtype=torch.float32, device=dev)
             logits_in, logits_out = None, logits.data_ptr()
         if T:
-            ws = self.workspace(T, dev)
+            ws = self.workspace(T, dev, extras)
             view = self.layer_view()
             if self.packed_backbones:  # gate and up see T rows, down T * top_k
                 big = [n for n in self.packed_backbones
@@ -273,13 +297,15 @@ class TrisSparseMoeBlock(nn.Module):
                 if big:
                     view = self._expanded_layer_view(dev, big)
             with torch.cuda.device(dev):
-                _native.check(
-                    lib.tris_moe_layer_forward(C.byref(view), x.data_ptr(), logits_in, T, y.data_ptr(),
-                                               logits_out, ws.data_ptr(), ws.numel(),
-                                               torch.cuda.current_stream(dev).cuda_stream),
-                    "moe_layer_forward",
-                )
-        return y.reshape(shape), logits
+                stream = torch.cuda.current_stream(dev).cuda_stream
+                if extras is None:
+                    st = lib.tris_moe_layer_forward(C.byref(view), x.data_ptr(), logits_in, T, y.data_ptr(),
+                                                    logits_out, ws.data_ptr(), ws.numel(), stream)
+                else:
+                    st = lib.tris_moe_layer_forward_extras(C.byref(view), C.byref(extras), x.data_ptr(), logits_in, T,
+                                                           y.data_ptr(), logits_out, ws.data_ptr(), ws.numel(), stream)
+                _native.check(st, "moe_layer_forward")
+        return y.reshape(shape), logits if extras is None else returned
 
     def forward_streaming(self, hidden_states: torch.Tensor, manager, block_index: int,
                           router_logits: Optional[torch.Tensor] = None):

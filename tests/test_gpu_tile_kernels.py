@@ -1,0 +1,147 @@
+"""The tile-record kernels, the 4-bit GEMM and the backbone GEMM at the edges of their tiles and of the rules
+that choose between their variants.  Weights are fp16 values known exactly (the dequantised matrix), so the
+bound of an output is that of its sum: fp32 accumulation of products of fp16 values, then one rounding to fp16."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(w, h):
+    """|error| of fp16(sum of w * h over k terms): half an fp16 ulp of the result (or of the smallest
+    normal), plus k additions of relative error 2^-22 (truncating fp32 adds) of the sum of magnitudes."""
+    ref = h.double() @ w.double().T
+    mag = h.double().abs() @ w.double().abs().T
+    acc = h.shape[1] * 2.0 ** -22 * mag
+    return ref, acc, acc * (1 + 2.0 ** -10) + ref.abs() * 2.0 ** -11 + 2.0 ** -25
+
+
+def _assert_within(got, ref, bound):
+    worst = ((got.double() - ref).abs() / bound).max().item()
+    assert worst <= 1.0, worst
+
+
+def _payload(tm, E, O, rank, group, seed):
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(seed)
+    p = synth.pack_projection(synth.raw_projection(rng, E, O, rank, group_size=group))
+    return tm.prepare_grouped_payload(p, "cuda")
+
+
+# (outputs, rank, scale group, rows per expert): decode kernel with 8 / 4 / 2 / 1 warps per 32 outputs and 8 to 32
+# rows per pass, a segment of several passes, more columns than one stage holds; tiled kernel with 64- and
+# 128-row tiles, ragged last tile, one to five column chunks.
+GROUPED = [
+    (96, 256, 32, [1, 0, 8, 3]),
+    (97, 264, 128, [16, 9, 16]),
+    (33, 1040, 64, [2, 5]),
+    (64, 64, 32, [24, 17, 0, 23]),
+    (160, 80, 32, [70, 1, 1, 1, 1, 1, 1, 1]),
+    (1040, 64, 64, [25 + i % 8 for i in range(40)]),
+    (1031, 72, 128, [i % 5 for i in range(50)]),
+    (2080, 320, 128, [1 + i % 3 for i in range(34)]),
+    (2048, 44, 32, [1] * 34),
+    (129, 136, 32, [33, 64, 65, 1]),
+    (256, 520, 128, [129, 0, 257, 100]),
+    (90, 44, 32, [300, 40]),
+]
+
+
+@pytest.mark.parametrize("O,rank,group,lengths", GROUPED)
+def test_grouped_kernels_at_tile_edges(lib, O, rank, group, lengths):
+    import trismoe_b200 as tm
+
+    E, R = len(lengths), sum(lengths)
+    pa, pb = _payload(tm, E, O, rank, group, O + rank), _payload(tm, E, O, rank, group, O + rank + 1)
+    wa, wb = tm.dequantize_grouped_payload(pa), tm.dequantize_grouped_payload(pb)
+    g = torch.Generator().manual_seed(R)
+    ha, hb = ((0.5 * torch.randn((R, rank), generator=g)).half().cuda() for _ in range(2))
+    one = tm.run_grouped_structured_expert_forward(pa, ha, None, lengths)
+    sa, sb = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, hb, None, lengths)
+    mlp, _ = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, hb, None, lengths, fuse_silu_mul=True)
+    row = 0
+    for e, n in enumerate(lengths):
+        if n == 0:
+            continue
+        rows = slice(row, row + n)
+        row += n
+        ra, ea, ba = _bound(wa[e], ha[rows])
+        rb, eb, bb = _bound(wb[e], hb[rows])
+        _assert_within(one[rows], ra, ba)
+        _assert_within(sa[rows], ra, ba)
+        _assert_within(sb[rows], rb, bb)
+        silu = ra * torch.sigmoid(ra)
+        want = silu * rb  # |silu'| < 1.1; exponential, division and two products in fp32
+        err = 1.1 * ea * rb.abs() + silu.abs() * eb + 1.1 * ea * eb + want.abs() * (2.0 ** -11 + 2.0 ** -19) + 2.0 ** -25
+        _assert_within(mlp[rows], want, err)
+
+
+@pytest.mark.parametrize("rows,cols,group,T", [
+    (16, 32, 32, 1), (17, 40, 40, 8), (64, 64, 32, 9), (48, 96, 96, 17), (72, 128, 64, 33), (256, 264, 264, 65), (128, 2048, 128, 200),
+])
+def test_packed4_gemm_at_tile_edges(lib, rows, cols, group, T):
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    m = synth.packed4_matrix(np.random.default_rng(rows + T), rows, cols, group_size=group, scale_std=0.02)
+    lin = tm.Packed4Linear(m, "cuda")
+    w = lin(torch.eye(cols, dtype=torch.float16, device="cuda")).t()  # single products: the weights themselves
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn((T, cols + 8), generator=g).half().cuda()
+    for xi in (x[:, :cols].contiguous(), x[:, 3:3 + cols]):  # aligned rows, rows read element by element
+        ref, _, bound = _bound(w, xi)
+        _assert_within(lin(xi), ref, bound)
+
+
+@pytest.mark.parametrize("T", [1, 37, 300])
+@pytest.mark.parametrize("pairs,scales", [("gate up down", ""), ("gate", "up"), ("up", "gate down"), ("down", "gate up down"), ("", "down")])
+def test_null_space_and_input_scales_in_one_sequence(lib, T, pairs, scales):
+    """The native layer sequence against the same block composed of the reference-named operators: both
+    round gate, up, mlp and the routed rows to fp16, in the same places."""
+    import trismoe_b200 as tm
+    import trismoe_oracle as orc
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(11)
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=3)
+    E, H, I = shape.num_experts, shape.hidden_size, shape.intermediate_size
+    width = {"gate": H, "up": H, "down": I}
+    vec = {n: torch.from_numpy((1 + 0.2 * rng.standard_normal(width[n])).astype(np.float16)) for n in scales.split()}
+    blk = tm.TrisSparseMoeBlock(H, I, E, shape.top_k, shape.norm_topk_prob)
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], layer["shared_gate"], layer["shared_up"], layer["shared_down"],
+                              layer["router_weight"], device="cuda", input_scales=vec)
+
+    def pair(n):
+        out = H if n == "down" else I
+        ex = [None if r == 0 else {"c2": synth.packed4_matrix(rng, r, width[n], 64, scale_std=0.02),
+                                   "c1": synth.packed4_matrix(rng, out, r, 64, scale_std=0.02)} for r in (16, 0, 24, 16, 8, 40, 0, 16)]
+        return tm.build_grouped_ns_compensation_payload(ex, "cuda", torch.float16, width[n], out)
+
+    blk.load_ns_compensation_payloads(*(pair(n) if n in pairs.split() else None for n in ("gate", "up", "down")))
+    x = synth.synth_activations(T, H, seed=T).cuda().view(1, T, -1)
+    logits = synth.synth_router_logits(T, E, seed=T).cuda()
+    want, l_ops = blk.forward_grouped_ops(x, router_logits=logits)
+    got, l_got = blk(x, router_logits=logits)
+    assert l_got is logits and l_ops is logits
+    max_abs, mean_rel = orc.error_metrics(got.float().cpu().numpy(), want.float().cpu().numpy())
+    # routing weights stay fp32 in the sequence (fp16 in the composed operators: 2^-11), gate/up without a
+    # pair stay fp32 before SiLU (fp16 there: 2^-11 each): four roundings of 2^-11 that one side has alone
+    scale = want.float().abs().max().item()
+    assert want.abs().max() > 1e-3 and max_abs <= 8 * 2.0 ** -11 * scale and mean_rel <= 4 * 2.0 ** -11, (max_abs, mean_rel, scale)
+    _, own = blk(x)
+    assert own.dtype == torch.float16 and own.shape == (T, E)
+
+
+# 64- and 128-wide tiles of the backbone GEMM: ragged rows, outputs and columns, one to many row tiles
+@pytest.mark.parametrize("n,k,m", [(33, 64, 64), (127, 192, 72), (129, 1032, 256), (300, 2048, 136), (1025, 512, 264), (2048, 1024, 128)])
+def test_backbone_gemm_at_tile_edges(lib, n, k, m):
+    import trismoe_b200 as tm
+
+    g = torch.Generator().manual_seed(n + m)
+    x = torch.randn((n, k), generator=g).half().cuda()
+    w = (0.05 * torch.randn((m, k), generator=g)).half().cuda()
+    ref, _, bound = _bound(w, x)
+    _assert_within(tm.compute_shared_hidden(x, w), ref, bound)
