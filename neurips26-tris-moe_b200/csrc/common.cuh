@@ -130,7 +130,8 @@ int grouped_tc_min_rows();
 int route_rows_hint(const TrisRouteView* route);
 int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t stream);
 int combine_routed_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,
-                        int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream, bool pdl);
+                        int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream, bool pdl,
+                        bool indices_ready = false);
 int launch_router_route(const float* logits, int num_tokens, int num_experts, int top_k, int norm, int m_tile,
                         int32_t* selected, float* weights, int32_t* perm, int32_t* tok, int32_t* slot,
                         int32_t* row_of_flat, int32_t* expert_ids, int32_t* segment_offsets, int32_t* problem_offsets,

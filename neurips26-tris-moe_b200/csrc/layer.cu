@@ -81,8 +81,7 @@ static LayerWorkspace carve(const TrisMoeLayerView* L, int T, char* base, const 
 }
 
 // out = x * scale, rounded to fp16 (what the separate operators feed the backbone with)
-__global__ void scale_columns_kernel(const __half* __restrict__ x, const __half* __restrict__ scale, size_t count, int cols,
-                                     __half* __restrict__ out) {
+__global__ void scale_columns_kernel(const __half* x, const __half* scale, size_t count, int cols, __half* out) {
   pdl_wait();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count; i += static_cast<size_t>(gridDim.x) * blockDim.x)
     out[i] = __hmul(x[i], scale[i % cols]);
@@ -224,7 +223,8 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
     if (st != TRIS_OK) return st;
   }
   if (np > 0) {
-    st = launch_shared_hidden(probs, np, x, nullptr, T, layer->hidden_size, s, /*pdl=*/logits_given, nullptr, true);
+    // as the first launch of the sequence it may follow the kernel that wrote the matrices
+    st = launch_shared_hidden(probs, np, x, nullptr, T, layer->hidden_size, s, /*pdl=*/true, nullptr, /*matrices_before_wait=*/logits_given);
     if (st != TRIS_OK) return st;
   }
   const TrisPacked4View* packed[2] = {layer->packed_gate, layer->packed_up};
@@ -323,7 +323,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
   }
 
   // combine
-  return combine_routed_impl(w.down_out, w.row_of_flat, w.weights, T, layer->top_k, layer->hidden_size, y_f16, s, true);
+  return combine_routed_impl(w.down_out, w.row_of_flat, w.weights, T, layer->top_k, layer->hidden_size, y_f16, s, true, /*indices_ready=*/true);
 }
 
 extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void* x_f16, const float* router_logits,

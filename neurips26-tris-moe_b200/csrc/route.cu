@@ -11,66 +11,78 @@ namespace tris {
 constexpr int kRouteThreads = 1024;
 constexpr int kMaxExpertsPerLane = 8;  // experts <= 256
 
-// Softmax + top-k of one token by one warp.  Ties go to the lower expert index.
-__device__ __forceinline__ void topk_one_token(const float* __restrict__ row, int num_experts, int top_k, int norm,
-                                               int32_t* __restrict__ selected, float* __restrict__ weights, int lane) {
-  float v[kMaxExpertsPerLane];
+// Softmax + top-k of one token by one warp of which lane s keeps slot s (top_k <= 32).  Ties go to the lower
+// expert index.  Probabilities are >= 0, so their bit patterns order like the numbers and one integer
+// reduction finds a maximum, a second one the lowest expert that has it (ten shuffles with a
+// two-key compare each before).  NE = experts per lane.
+struct Pick {
+  int expert;
+  float weight;
+};
+template <int NE>
+__device__ __forceinline__ Pick topk_one_token(const float* row, int num_experts, int top_k, int norm, int lane) {
+  float v[NE];
   float mx = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < kMaxExpertsPerLane; ++i) {
+  for (int i = 0; i < NE; ++i) {
     const int e = lane + 32 * i;
     v[i] = (e < num_experts) ? row[e] : -INFINITY;
     mx = fmaxf(mx, v[i]);
   }
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
   float sum = 0.f;
+  uint32_t key[NE];  // bits + 1; 0 = absent, taken or not a number
 #pragma unroll
-  for (int i = 0; i < kMaxExpertsPerLane; ++i) {
-    const int e = lane + 32 * i;
-    v[i] = (e < num_experts) ? expf(v[i] - mx) : -1.f;  // probabilities are >= 0; -1 marks "taken/absent"
-    if (e < num_experts) sum += v[i];
+  for (int i = 0; i < NE; ++i) {
+    const bool in = lane + 32 * i < num_experts;
+    const float p = expf(v[i] - mx);
+    if (in) sum += p;
+    key[i] = in && p >= 0.f ? __float_as_uint(p) + 1u : 0u;
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
   const float inv = 1.f / sum;
   float picked_sum = 0.f;
-  float my_w = 0.f;  // lane s keeps the weight of slot s (top_k <= 32)
-  int my_e = 0;
+  Pick mine{0, 0.f};
   for (int s = 0; s < top_k; ++s) {
-    float best = -1.f;
-    int best_e = 0x7FFFFFFF;
+    uint32_t best = 0u;
 #pragma unroll
-    for (int i = 0; i < kMaxExpertsPerLane; ++i) {
-      const int e = lane + 32 * i;
-      if (v[i] > best) { best = v[i]; best_e = e; }  // ascending e inside a lane: first max wins
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-      const int oe = __shfl_xor_sync(0xFFFFFFFFu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
+    for (int i = 0; i < NE; ++i) best = max(best, key[i]);
+    best = __reduce_max_sync(0xFFFFFFFFu, best);
+    uint32_t best_e = 0x7FFFFFFFu;
 #pragma unroll
-    for (int i = 0; i < kMaxExpertsPerLane; ++i)
-      if (lane + 32 * i == best_e) v[i] = -1.f;
-    const float p = best * inv;
+    for (int i = NE - 1; i >= 0; --i)
+      if (best != 0u && key[i] == best) best_e = lane + 32 * i;
+    best_e = __reduce_min_sync(0xFFFFFFFFu, best_e);
+#pragma unroll
+    for (int i = 0; i < NE; ++i)
+      if (lane + 32 * i == best_e) key[i] = 0u;
+    const float p = (best != 0u ? __uint_as_float(best - 1u) : -1.f) * inv;
     picked_sum += p;
-    if (lane == s) { my_w = p; my_e = best_e; }
+    if (lane == s) mine = {static_cast<int>(best_e), p};
   }
-  if (lane < top_k) {
-    selected[lane] = my_e;
-    weights[lane] = norm ? my_w / picked_sum : my_w;
-  }
+  if (norm) mine.weight /= picked_sum;
+  return mine;
 }
 
 // One warp per token.
-__global__ void router_topk_kernel(const float* __restrict__ logits, int num_tokens, int num_experts, int top_k,
+template <int NE>
+__global__ void router_topk_kernel(const float* logits, int num_tokens, int num_experts, int top_k,
                                    int norm, int32_t* __restrict__ selected, float* __restrict__ weights) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= num_tokens) return;
   pdl_wait();
-  topk_one_token(logits + static_cast<size_t>(warp) * num_experts, num_experts, top_k, norm,
-                 selected + static_cast<size_t>(warp) * top_k, weights + static_cast<size_t>(warp) * top_k, lane);
+  pdl_launch_dependents();
+  const Pick pick = topk_one_token<NE>(logits + static_cast<size_t>(warp) * num_experts, num_experts, top_k, norm, lane);
+  if (lane < top_k) {
+    selected[static_cast<size_t>(warp) * top_k + lane] = pick.expert;
+    weights[static_cast<size_t>(warp) * top_k + lane] = pick.weight;
+  }
 }
+
+// kernel<experts per lane> for the expert count
+#define TRIS_BY_EXPERTS(num_experts, kernel) \
+  ((num_experts) <= 32 ? kernel<1> : (num_experts) <= 64 ? kernel<2> : (num_experts) <= 128 ? kernel<4> : kernel<8>)
 
 // The flat (token, slot) list of expert ids: entry f is base[f * stride] - offset (stride 1, offset 0 for
 // a plain [T, k] array; an exchange buffer keeps the id of slot f behind that slot's activation row and
@@ -86,7 +98,7 @@ struct SelectedIds {
 __device__ __forceinline__ void route_scan_segments(const int32_t* count, int32_t* start, int num_experts, int m_tile,
                                                     int32_t* __restrict__ expert_ids, int32_t* __restrict__ segment_offsets,
                                                     int32_t* __restrict__ problem_offsets, int32_t* __restrict__ counts_out,
-                                                    int lane) {
+                                                    int lane, bool write = true) {
     // each lane owns a contiguous run of experts; warp scan of (segments, rows, tiles)
     const int epl = (num_experts + 31) / 32;
     const int e0 = lane * epl, e1 = min(num_experts, e0 + epl);
@@ -110,14 +122,17 @@ __device__ __forceinline__ void route_scan_segments(const int32_t* count, int32_
       start[e] = r;
       const int c = count[e];
       if (c > 0) {
-        expert_ids[s] = e;
-        segment_offsets[s] = r;
-        problem_offsets[s] = t;
+        if (write) {
+          expert_ids[s] = e;
+          segment_offsets[s] = r;
+          problem_offsets[s] = t;
+        }
         r += c;
         t += (c + m_tile - 1) / m_tile;
         ++s;
       }
     }
+    if (!write) return;
     for (int q = nseg + lane; q <= num_experts; q += 32) {
       segment_offsets[q] = nrows;
       problem_offsets[q] = ntiles;
@@ -201,7 +216,7 @@ __global__ void __launch_bounds__(kRouteThreads) build_route_kernel(
     const SelectedIds selected, int num_tokens, int top_k, int num_experts, int m_tile,
     int32_t* __restrict__ perm, int32_t* __restrict__ tok, int32_t* __restrict__ slot,
     int32_t* __restrict__ row_of_flat, int32_t* __restrict__ expert_ids, int32_t* __restrict__ segment_offsets,
-    int32_t* __restrict__ problem_offsets, int32_t* __restrict__ counts_out, int sel_cap) {
+    int32_t* __restrict__ problem_offsets, int32_t* __restrict__ counts_out) {
   extern __shared__ int32_t sh[];
   pdl_wait();
   pdl_launch_dependents();
@@ -262,7 +277,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_scan_kernel(int32_t* __re
 }
 
 __global__ void __launch_bounds__(kRouteParThreads) route_place_kernel(const SelectedIds selected, int num_rows, int top_k,
-                                                                       int num_experts, const int32_t* __restrict__ start_blk,
+                                                                       int num_experts, const int32_t* start_blk,
                                                                        int32_t* __restrict__ perm, int32_t* __restrict__ tok,
                                                                        int32_t* __restrict__ slot, int32_t* __restrict__ row_of_flat) {
   constexpr int NW = kRouteParThreads / 32;
@@ -337,34 +352,136 @@ static int launch_route_parallel(const SelectedIds selected, int num_tokens, int
                     "route_place_kernel launch");
 }
 
-// Router head and route in one single-CTA launch (decode-sized batches).
-__global__ void __launch_bounds__(kRouteThreads) router_route_kernel(
-    const float* __restrict__ logits, int num_tokens, int top_k, int num_experts, int norm, int m_tile,
-    int32_t* selected, float* __restrict__ weights, int32_t* __restrict__ perm, int32_t* __restrict__ tok,
-    int32_t* __restrict__ slot, int32_t* __restrict__ row_of_flat, int32_t* __restrict__ expert_ids,
-    int32_t* __restrict__ segment_offsets, int32_t* __restrict__ problem_offsets, int32_t* __restrict__ counts_out,
-    int sel_cap) {
-  extern __shared__ int32_t sh[];
+// Router head and route together.  The experts of a token are distinct, so 32 tokens are one 32-bit mask per
+// expert, a row's place among its expert's rows of the group is the number of set bits below its token's,
+// and nothing is sorted.  Up to 32 tokens: one CTA, one warp per token, picks stay in registers.  More:
+// one CTA per 32 tokens writes picks and masks, and a second launch in which every CTA adds up the masks
+// for itself (they are a few KB) places them.  512 tokens of 64 experts: 17 us for top-k, then a
+// single-CTA counting sort of the flat list; now 6.
+struct RouteArgs {
+  const float* logits;
+  int num_tokens, top_k, num_experts, norm, m_tile;
+  int32_t* selected;
+  float* weights;
+  int32_t *perm, *tok, *slot, *row_of_flat, *expert_ids, *segment_offsets, *problem_offsets, *counts;
+  uint32_t* masks;  // [group of 32 tokens][num_experts]
+};
+
+__device__ __forceinline__ void route_place(const RouteArgs& a, int token, int slot, int e, const int32_t* start, uint32_t mask) {
+  const int f = token * a.top_k + slot;
+  if (e >= a.num_experts) {  // logits that are not numbers
+    a.row_of_flat[f] = -1;
+    return;
+  }
+  const int pos = start[e] + __popc(mask & ((1u << (token & 31)) - 1u));
+  a.perm[pos] = f;
+  a.tok[pos] = token;
+  a.slot[pos] = slot;
+  a.row_of_flat[f] = pos;
+}
+
+// kPlace: the whole route (one CTA, up to 32 tokens); otherwise the picks and masks of 32 tokens
+template <int NE, bool kPlace>
+__device__ __forceinline__ void router_group(const RouteArgs& a, uint32_t* sh) {
+  uint32_t* mask = sh;  // [E]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = a.num_experts;
+  for (int e = tid; e < E; e += blockDim.x) mask[e] = 0u;
+  __syncthreads();
   pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int tk = warp; tk < num_tokens; tk += kRouteThreads / 32)
-    topk_one_token(logits + static_cast<size_t>(tk) * num_experts, num_experts, top_k, norm,
-                   selected + static_cast<size_t>(tk) * top_k, weights + static_cast<size_t>(tk) * top_k, lane);
-  __syncthreads();  // selected[] written above is read back by every thread below
   pdl_launch_dependents();
-  build_route_body(sh, SelectedIds{selected, 1, 0}, num_tokens, top_k, num_experts, m_tile, perm, tok, slot, row_of_flat,
-                   expert_ids, segment_offsets, problem_offsets, counts_out);
+  const int token = blockIdx.x * 32 + warp;
+  Pick pick{0x7FFFFFFF, 0.f};
+  if (token < a.num_tokens) {
+    pick = topk_one_token<NE>(a.logits + static_cast<size_t>(token) * E, E, a.top_k, a.norm, lane);
+    if (lane < a.top_k) {
+      if (pick.expert < E) atomicOr(&mask[pick.expert], 1u << warp);
+      a.selected[static_cast<size_t>(token) * a.top_k + lane] = pick.expert;
+      a.weights[static_cast<size_t>(token) * a.top_k + lane] = pick.weight;
+    }
+  }
+  __syncthreads();
+  if constexpr (!kPlace) {
+    for (int e = tid; e < E; e += blockDim.x) a.masks[static_cast<size_t>(blockIdx.x) * E + e] = mask[e];
+  } else {
+    int32_t* count = reinterpret_cast<int32_t*>(sh) + E;
+    int32_t* start = count + E;
+    if (warp == 0) {
+      for (int e = lane; e < E; e += 32) count[e] = __popc(mask[e]);
+      __syncwarp();
+      route_scan_segments(count, start, E, a.m_tile, a.expert_ids, a.segment_offsets, a.problem_offsets, a.counts, lane);
+    }
+    __syncthreads();
+    if (token < a.num_tokens && lane < a.top_k) route_place(a, token, lane, pick.expert, start, pick.expert < E ? mask[pick.expert] : 0u);
+  }
+}
+template <int NE>
+__global__ void __launch_bounds__(kRouteThreads) router_route_kernel(const __grid_constant__ RouteArgs a) {
+  extern __shared__ int32_t sh[];
+  router_group<NE, true>(a, reinterpret_cast<uint32_t*>(sh));
+}
+template <int NE>
+__global__ void __launch_bounds__(kRouteThreads) router_masks_kernel(const __grid_constant__ RouteArgs a) {
+  extern __shared__ int32_t sh[];
+  router_group<NE, false>(a, reinterpret_cast<uint32_t*>(sh));
+}
+
+// grid: CTAs that share the groups of 32 tokens in runs
+__global__ void __launch_bounds__(kRouteThreads) router_place_kernel(const __grid_constant__ RouteArgs a) {
+  extern __shared__ int32_t sh[];
+  const int E = a.num_experts, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int32_t* count = sh;  // [E] rows of an expert
+  int32_t* start = sh + E;
+  int32_t* before = sh + 2 * E;  // [E] of them, those of the groups before this CTA's
+  for (int e = tid; e < 3 * E; e += kRouteThreads) sh[e] = 0;
+  __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
+  const int groups = (a.num_tokens + 31) / 32, run = (groups + gridDim.x - 1) / gridDim.x;
+  const int g0 = min(groups, static_cast<int>(blockIdx.x) * run), g1 = min(groups, g0 + run);
+  const int e = tid % E, part = tid / E, parts = kRouteThreads / E;
+  if (part < parts) {
+    int total = 0, mine = 0;
+#pragma unroll 4
+    for (int g = part; g < groups; g += parts) {
+      const int c = __popc(__ldcg(a.masks + static_cast<size_t>(g) * E + e));
+      total += c;
+      mine += g < g0 ? c : 0;
+    }
+    if (total) atomicAdd(&count[e], total);
+    if (mine) atomicAdd(&before[e], mine);
+  }
+  __syncthreads();
+  if (warp == 0)
+    route_scan_segments(count, start, E, a.m_tile, a.expert_ids, a.segment_offsets, a.problem_offsets, a.counts, lane, blockIdx.x == 0);
+  __syncthreads();
+  for (int i = tid; i < E; i += kRouteThreads) start[i] += before[i];
+  __syncthreads();
+  for (int g = g0; g < g1; ++g) {
+    const uint32_t* mask = a.masks + static_cast<size_t>(g) * E;
+    const int token = g * 32 + warp;
+    if (token < a.num_tokens && lane < a.top_k) {
+      const int x = __ldcg(a.selected + static_cast<size_t>(token) * a.top_k + lane);
+      route_place(a, token, lane, x, start, x < E ? __ldcg(mask + x) : 0u);
+    }
+    if (g + 1 == g1) break;
+    __syncthreads();
+    for (int i = tid; i < E; i += kRouteThreads) start[i] += __popc(__ldcg(mask + i));
+    __syncthreads();
+  }
 }
 
 // final[t, :] = sum_s w[t, s] * rows[row_of_flat[t*k+s], :]; one thread per 8 output halves.
-__global__ void combine_routed_kernel(const __half* __restrict__ rows, const int32_t* __restrict__ row_of_flat,
-                                      const float* __restrict__ weights, int num_tokens, int top_k, int hidden,
-                                      __half* __restrict__ out) {
+// kIndicesReady: row_of_flat and weights are older than the kernel before this one.  Not __restrict__: loads
+// from a const __restrict__ parameter may be moved above the wait.
+template <bool kIndicesReady>
+__global__ void combine_routed_kernel(const __half* rows, const int32_t* row_of_flat,
+                                      const float* weights, int num_tokens, int top_k, int hidden,
+                                      __half* out) {
   const int vec_per_row = hidden >> 3;
   const long long id = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (id >= static_cast<long long>(num_tokens) * vec_per_row) return;
   const int t = static_cast<int>(id / vec_per_row), c = static_cast<int>(id % vec_per_row) * 8;
-  pdl_wait();
+  if (!kIndicesReady) pdl_wait();
   float acc[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) acc[u] = 0.f;
@@ -377,6 +494,10 @@ __global__ void combine_routed_kernel(const __half* __restrict__ rows, const int
       const bool in = s0 + j < top_k;
       r[j] = in ? row_of_flat[t * top_k + s0 + j] : 0;
       w[j] = in ? weights[t * top_k + s0 + j] : 0.f;
+    }
+    if (s0 == 0) {
+      if (kIndicesReady) pdl_wait();
+      pdl_launch_dependents();
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
@@ -401,43 +522,36 @@ __global__ void combine_routed_kernel(const __half* __restrict__ rows, const int
   *reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * hidden + c) = o;
 }
 
-static int route_smem_bytes(int num_experts, int rows, int* sel_cap) {
-  (void)rows;
-  *sel_cap = 0;
-  return static_cast<int>((2 + kRouteThreads / 32) * num_experts * sizeof(int32_t));
-}
+static int route_smem_bytes(int num_experts) { return static_cast<int>((2 + kRouteThreads / 32) * num_experts * sizeof(int32_t)); }
 
-// Router head + route for the fused layer path: one single-CTA launch for batches of up to
-// 32 tokens (one warp per token), otherwise a token-parallel top-k launch followed by the
-// single-CTA route kernel.
+// Router head + route for the fused layer path: one launch for up to 32 tokens, two for more, or top-k and the
+// general route where `scratch` does not hold the masks.
 int launch_router_route(const float* logits, int num_tokens, int num_experts, int top_k, int norm, int m_tile,
                         int32_t* selected, float* weights, int32_t* perm, int32_t* tok, int32_t* slot,
                         int32_t* row_of_flat, int32_t* expert_ids, int32_t* segment_offsets, int32_t* problem_offsets,
                         int32_t* counts, cudaStream_t stream, int32_t* scratch, size_t scratch_bytes) {
   TRIS_REQUIRE(num_experts <= 32 * kMaxExpertsPerLane && top_k <= 32 && top_k <= num_experts, TRIS_ERR_UNSUPPORTED,
                "router: supports up to %d experts and top-32", 32 * kMaxExpertsPerLane);
-  int sel_cap = 0;
-  const int smem = route_smem_bytes(num_experts, num_tokens * top_k, &sel_cap);
-  if (num_tokens <= kRouteThreads / 32) {
-    router_route_kernel<<<1, kRouteThreads, smem, stream>>>(logits, num_tokens, top_k, num_experts, norm, m_tile,
-                                                            selected, weights, perm, tok, slot, row_of_flat,
-                                                            expert_ids, segment_offsets, problem_offsets, counts, sel_cap);
-    return check_cuda(cudaGetLastError(), "router_route_kernel launch");
+  const RouteArgs args{logits, num_tokens, top_k, num_experts, norm, m_tile, selected, weights, perm, tok, slot, row_of_flat,
+                       expert_ids, segment_offsets, problem_offsets, counts, reinterpret_cast<uint32_t*>(scratch)};
+  if (num_tokens <= 32)
+    return check_cuda(launch_kernel(TRIS_BY_EXPERTS(num_experts, router_route_kernel), dim3(1), dim3(32 * num_tokens),
+                                    3 * sizeof(int32_t) * num_experts, stream, /*pdl=*/true, 1, args),
+                      "router_route_kernel launch");
+  const int groups = ceil_div(num_tokens, 32);
+  if (scratch && scratch_bytes >= sizeof(int32_t) * static_cast<size_t>(groups) * num_experts) {
+    const int st = check_cuda(launch_kernel(TRIS_BY_EXPERTS(num_experts, router_masks_kernel), dim3(groups), dim3(kRouteThreads),
+                                            sizeof(int32_t) * num_experts, stream, /*pdl=*/true, 1, args),
+                              "router_masks_kernel launch");
+    if (st != TRIS_OK) return st;
+    return check_cuda(launch_kernel(router_place_kernel, dim3(std::min(groups, 64)), dim3(kRouteThreads), 3 * sizeof(int32_t) * num_experts,
+                                    stream, /*pdl=*/true, 1, args),
+                      "router_place_kernel launch");
   }
-  const int threads = 128;
-  router_topk_kernel<<<ceil_div(num_tokens * 32, threads), threads, 0, stream>>>(logits, num_tokens, num_experts, top_k,
-                                                                                 norm, selected, weights);
-  int st = check_cuda(cudaGetLastError(), "router_topk_kernel launch");
+  const int st = tris_router_topk(logits, num_tokens, num_experts, top_k, norm, selected, weights, stream);
   if (st != TRIS_OK) return st;
-  const int rows = num_tokens * top_k;
-  if (scratch && rows >= 4 * kRouteParChunk &&
-      scratch_bytes >= sizeof(int32_t) * static_cast<size_t>(ceil_div(rows, kRouteParChunk)) * num_experts)
-    return launch_route_parallel(SelectedIds{selected, 1, 0}, num_tokens, top_k, num_experts, m_tile, perm, tok, slot, row_of_flat,
-                                 expert_ids, segment_offsets, problem_offsets, counts, scratch, stream);
-  return check_cuda(launch_kernel(build_route_kernel, dim3(1), dim3(kRouteThreads), smem, stream, /*pdl=*/true, 1,
-                                  SelectedIds{selected, 1, 0}, num_tokens, top_k, num_experts, m_tile, perm,
-                                  tok, slot, row_of_flat, expert_ids, segment_offsets, problem_offsets, counts, sel_cap),
-                    "build_route_kernel launch");
+  return tris_build_grouped_route(selected, num_tokens, top_k, num_experts, m_tile, perm, tok, slot, row_of_flat, expert_ids,
+                                  segment_offsets, problem_offsets, counts, stream);
 }
 
 // Owner rank of an expert under the contiguous partition (sizes differ by at most one).
@@ -536,7 +650,7 @@ extern "C" int tris_router_topk(const float* router_logits, int32_t num_tokens, 
                "tris_router_topk: supports up to %d experts and top-32", 32 * kMaxExpertsPerLane);
   if (num_tokens == 0) return TRIS_OK;
   const int threads = 128;
-  return check_cuda(launch_kernel(router_topk_kernel, dim3(ceil_div(num_tokens * 32, threads)), dim3(threads), 0,
+  return check_cuda(launch_kernel(TRIS_BY_EXPERTS(num_experts, router_topk_kernel), dim3(ceil_div(num_tokens * 32, threads)), dim3(threads), 0,
                                   static_cast<cudaStream_t>(stream), programmatic_launch_default(), 1, router_logits,
                                   num_tokens, num_experts, top_k, norm_topk_prob, selected_experts, routing_weights),
                     "router_topk_kernel launch");
@@ -577,25 +691,25 @@ extern "C" int tris_build_grouped_route_ex(const int32_t* selected_experts, int3
     return launch_route_parallel(ids, num_tokens, top_k, num_experts, m_tile, perm, grouped_token_indices,
                                  grouped_slots, row_of_flat, expert_ids, segment_offsets, problem_offsets, counts, scratch,
                                  static_cast<cudaStream_t>(stream), programmatic_launch_default());
-  int sel_cap = 0;
-  const int smem = route_smem_bytes(num_experts, rows, &sel_cap);
+  const int smem = route_smem_bytes(num_experts);
   return check_cuda(launch_kernel(build_route_kernel, dim3(1), dim3(kRouteThreads), smem, static_cast<cudaStream_t>(stream),
                                   programmatic_launch_default(), 1, ids, num_tokens, top_k, num_experts, m_tile,
                                   perm, grouped_token_indices, grouped_slots, row_of_flat, expert_ids, segment_offsets,
-                                  problem_offsets, counts, sel_cap),
+                                  problem_offsets, counts),
                     "build_route_kernel launch");
 }
 
 int tris::combine_routed_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,
                               int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream,
-                              bool pdl) {
+                              bool pdl, bool indices_ready) {
   TRIS_REQUIRE(down_out_f16 && row_of_flat && routing_weights && final_f16, TRIS_ERR_INVALID_ARG, "tris_combine_routed: null pointer");
   TRIS_REQUIRE(num_tokens >= 0 && top_k > 0 && hidden_size > 0, TRIS_ERR_INVALID_ARG, "tris_combine_routed: bad sizes");
   TRIS_REQUIRE((hidden_size & 7) == 0, TRIS_ERR_UNSUPPORTED, "tris_combine_routed: hidden_size must be a multiple of 8");
   if (num_tokens == 0) return TRIS_OK;
   const long long total = static_cast<long long>(num_tokens) * (hidden_size / 8);
   const int threads = 256;
-  return check_cuda(launch_kernel(combine_routed_kernel, dim3(static_cast<unsigned>((total + threads - 1) / threads)),
+  return check_cuda(launch_kernel(indices_ready ? combine_routed_kernel<true> : combine_routed_kernel<false>,
+                                  dim3(static_cast<unsigned>((total + threads - 1) / threads)),
                                   dim3(threads), 0, stream, pdl, 1, static_cast<const __half*>(down_out_f16),
                                   row_of_flat, routing_weights, num_tokens, top_k, hidden_size,
                                   static_cast<__half*>(final_f16)),

@@ -135,6 +135,29 @@ def test_null_space_and_input_scales_in_one_sequence(lib, T, pairs, scales):
     assert own.dtype == torch.float16 and own.shape == (T, E)
 
 
+@pytest.mark.parametrize("E,k", [(8, 2), (40, 8), (72, 3), (200, 8)])
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 65, 2100])
+def test_router_and_route_of_the_layer(lib, E, k, T):
+    """One launch up to 32 tokens, two above, runs of several 32-token groups per CTA above 2048; expert counts
+    on both sides of each lane count.  An identity-like layer would hide a wrong order, so whole outputs are compared."""
+    import trismoe_b200 as tm
+    import trismoe_oracle as orc
+    from trismoe_b200 import synth
+
+    shape = synth.LayerShape(64, 64, E, k, rank=32, group_size=32)
+    layer = synth.synth_layer(shape, seed=E)
+    blk = tm.TrisSparseMoeBlock(64, 64, E, k, shape.norm_topk_prob)
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], *(10 * layer["shared_" + n] for n in ("gate", "up", "down")),
+                              layer["router_weight"], device="cuda")
+    x, logits = synth.synth_activations(T, 64, seed=T).cuda().view(1, T, 64), synth.synth_router_logits(T, E, seed=T).cuda()
+    want, _ = blk.forward_grouped_ops(x, router_logits=logits)
+    got, _ = blk(x, router_logits=logits)
+    scale = want.float().abs().max().item()
+    max_abs, mean_rel = orc.error_metrics(got.float().cpu().numpy(), want.float().cpu().numpy())
+    # what the composed operators round to fp16 and the sequence does not: gate, up, SiLU, routing weight, weighted row
+    assert scale > 1e-3 and max_abs <= 10 * 2.0 ** -11 * scale and mean_rel <= 5 * 2.0 ** -11, (max_abs, mean_rel, scale)
+
+
 # 64- and 128-wide tiles of the backbone GEMM: ragged rows, outputs and columns, one to many row tiles
 @pytest.mark.parametrize("n,k,m", [(33, 64, 64), (127, 192, 72), (129, 1032, 256), (300, 2048, 136), (1025, 512, 264), (2048, 1024, 128)])
 def test_backbone_gemm_at_tile_edges(lib, n, k, m):
