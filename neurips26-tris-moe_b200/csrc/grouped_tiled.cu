@@ -416,7 +416,10 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
     };
     auto keep_row = [&]() { if (tid < N) src_rows[pass * N + tid] = next_src; };
     uint32_t rows_of = 0u;  // rows of the items in flight, oldest in the low byte
-    const int ahead = args.stages - 1;
+    // Items requested before the oldest one in flight is handed over.  A stage of a reused pass is given back
+    // only at the run's last tile, which needs all chunks of the pass handed over: the loader must not wait
+    // for such a stage while it still holds one of the same pass back.
+    const int ahead = min(args.stages - 1, args.reuse ? args.stages - args.chunks + 1 : args.stages);
     Ring put, get;
     auto put_item = [&]() {
       if (w.valid()) {

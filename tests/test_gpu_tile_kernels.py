@@ -32,7 +32,7 @@ def _payload(tm, E, O, rank, group, seed):
 
 # (outputs, rank, scale group, rows per expert): decode kernel with 8 / 4 / 2 / 1 warps per 32 outputs and 8 to 32
 # rows per pass, a segment of several passes, more columns than one stage holds; tiled kernel with 64- and
-# 128-row tiles, ragged last tile, one to five column chunks.
+# 128-row tiles, ragged last tile, one to five column chunks, one to several tiles per CTA.
 GROUPED = [
     (96, 256, 32, [1, 0, 8, 3]),
     (97, 264, 128, [16, 9, 16]),
@@ -46,6 +46,9 @@ GROUPED = [
     (129, 136, 32, [33, 64, 65, 1]),
     (256, 520, 128, [129, 0, 257, 100]),
     (90, 44, 32, [300, 40]),
+    (1040, 320, 128, [33 + i % 32 for i in range(40)]),  # several tiles per CTA on 3 and 4 staged chunks, several passes
+    (1040, 512, 128, [70] + [33 + i % 32 for i in range(39)]),
+    (1040, 300, 128, [70 + 9 * i for i in range(24)]),
 ]
 
 
