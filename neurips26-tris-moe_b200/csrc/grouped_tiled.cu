@@ -25,6 +25,8 @@
 // CTA leaves.
 #include <math.h>
 
+#include <type_traits>
+
 #include "grouped_tiled.cuh"
 
 namespace tris {
@@ -43,20 +45,25 @@ constexpr int kMaxStages = 4;
 constexpr int kDBase = 4 * 2 * kACols;       // accumulators behind the four warpgroups' two slots
 constexpr int kBarBytes = 512;
 constexpr int kRowIdxBytes = 2 * 128 * 4;
+constexpr int kOutBytes = 2 * 2 * 16 * kTileOut * 2;         // per epilogue warpgroup two tiles of 16 rows, fp16
+constexpr int kHeadBytes = kBarBytes + kRowIdxBytes + kOutBytes + 1024;  // and the way to a 1024-byte boundary
 
-// One stage: [column records][activation rows: K-major core matrices, [column / 8][N rows][16 B]][salient
-// activations, the same form, per projection]
+// One stage: [activation rows: per 64 columns [N rows][128 B] in the 128-byte swizzle (piece p of row n at p ^ (n & 7))]
+// [salient activations per projection: K-major core matrices, [column / 8][N rows][16 B]][column records].  In the
+// swizzled form eight lanes fill one 128-byte line of shared memory from one line of global memory; as core
+// matrices the two 16-byte halves of every sector went to different lines, and staging 128 rows x 128
+// columns took 2600 cycles of 5200 an item has.
 struct StageLayout {
-  int col_bytes, rows_off, rows_bytes, sal_off, sal_bytes, total;
+  int col_bytes, col_off, rows_bytes, sal_off, sal_bytes, total;
 };
 __host__ __device__ inline StageLayout stage_layout(int max_steps, int ncol, int nset, int n) {
   StageLayout l;
   l.col_bytes = kColHdrBytes + kColTabBytes + max_steps * kColStepBytes;
-  l.rows_off = (ncol * l.col_bytes + 127) & ~127;
   l.rows_bytes = n * kChunkCols * 2;
-  l.sal_off = l.rows_off + nset * l.rows_bytes;
+  l.sal_off = nset * l.rows_bytes;
   l.sal_bytes = max_steps * n * 32;
-  l.total = l.sal_off + ncol * l.sal_bytes;
+  l.col_off = l.sal_off + ncol * l.sal_bytes;
+  l.total = (l.col_off + ncol * l.col_bytes + 1023) & ~1023;
   return l;
 }
 
@@ -68,16 +75,19 @@ __host__ __device__ inline StageLayout stage_layout(int max_steps, int ncol, int
 template <int N>
 struct Walker {
   int u, u_end, nseg;
-  int x, x_begin, x_end, expert, row_end, r0, c;
-  int next_x, next_expert, next_begin, next_end;
+  int x, x_begin, x_end, expert, row_end, r0, c, c_begin, c_end;
+  int next_x, next_expert, next_begin, next_end, next_part;
   __device__ __forceinline__ void peek(const TiledArgs& args, int unit) {
     if (unit >= u_end) return;
     const int q = unit / args.units_x;
     next_x = unit - q * args.units_x;
     int seg = q, z = 0;  // row split: part z takes the passes z, z + row_split, ...
-    if (args.row_split > 1) {
+    next_part = 0;       // column split: which part of the chunks
+    if (args.row_split * args.col_split > 1) {
       z = q / nseg;
       seg = q - z * nseg;
+      next_part = z / args.row_split;
+      z -= next_part * args.row_split;
     }
     if (!args.expert_ids) {  // one segment of expert 0 with all rows
       next_expert = 0;
@@ -91,7 +101,7 @@ struct Walker {
   }
   __device__ __forceinline__ void start(const TiledArgs& args) {
     nseg = args.num_segments_dev ? min(warp_uniform(*args.num_segments_dev), args.num_segments) : args.num_segments;
-    const int total = nseg * args.units_x * args.row_split, per = total / gridDim.x, extra = total - per * gridDim.x;
+    const int total = nseg * args.units_x * args.row_split * args.col_split, per = total / gridDim.x, extra = total - per * gridDim.x;
     const int b = blockIdx.x;
     u = b * per + min(b, extra);
     u_end = u + per + (b < extra ? 1 : 0);
@@ -106,7 +116,8 @@ struct Walker {
       expert = warp_uniform(next_expert);
       r0 = warp_uniform(next_begin);
       row_end = min(warp_uniform(next_end), args.num_rows);
-      c = 0;
+      c = c_begin = next_part * args.chunks / args.col_split;
+      c_end = (next_part + 1) * args.chunks / args.col_split;
       peek(args, u + (x_end - x_begin));
       if (expert >= 0 && expert < args.num_experts && r0 < row_end) return;
       u += x_end - x_begin;
@@ -114,7 +125,7 @@ struct Walker {
   }
   __device__ __forceinline__ int rows() const { return min(N, row_end - r0); }
   __device__ __forceinline__ void next_pass(const TiledArgs& args) {
-    c = 0;
+    c = c_begin;
     x = x_begin;
     r0 += args.row_split * N;
     if (r0 < row_end) return;
@@ -122,14 +133,14 @@ struct Walker {
     load(args);
   }
   __device__ __forceinline__ void next_tile(const TiledArgs& args) {
-    c = 0;
+    c = c_begin;
     if (++x == x_end) next_pass(args);
   }
   __device__ __forceinline__ void next(const TiledArgs& args) {
-    if (++c == args.chunks) next_tile(args);
+    if (++c == c_end) next_tile(args);
   }
   __device__ __forceinline__ void next_stage(const TiledArgs& args) {  // for the role that does not look at tiles
-    if (++c == args.chunks) next_pass(args);
+    if (++c == c_end) next_pass(args);
   }
 };
 
@@ -154,26 +165,36 @@ struct Ring {
   }
 };
 
-// One chunk of a pass's activation rows; src[n] = source row of row n.  A warp covers 8 rows x 4 pieces of
-// 16 bytes: 64 contiguous source bytes per row, conflict-free writes.  Rows that can be copied as they are
-// go by cp.async, anything else element by element; columns past the matrix read as zeros up to a
-// multiple of 16.
+// One chunk of a pass's activation rows; src[n] = source row of row n.  A warp covers 4 rows x 128
+// contiguous bytes.  Rows that can be copied as they are go by cp.async, anything else element by element;
+// columns past the matrix read as zeros up to a multiple of 16.
 template <int N>
 __device__ __forceinline__ void stage_rows(const TiledArgs& args, uint8_t* dst, const __half* hidden, const int* src, int rows, int c0, int tid) {
-  const int piece = (tid >> 5) * 4 + ((tid >> 3) & 3);
-  const int cols = min(kChunkCols, args.rank - c0), left = cols - 8 * piece;  // columns of this piece that exist
-  if (left <= -8 || (left <= 0 && !(cols & 15))) return;
-  uint8_t* d = dst + (piece * N + (tid & 7)) * 16;
-  if (args.hidden_vec) {
-    const __half* from = hidden + (left > 0 ? c0 + 8 * piece : 0);
-#pragma unroll 2
-    for (int n = tid & 7; n < rows; n += 8, d += 128)
-      cp_async_16(d, from + static_cast<size_t>(src[n]) * args.hidden_stride, left > 0);
-    return;
-  }
+  const int p = tid & 7, n0 = tid >> 3;
+  const int cols = min(kChunkCols, args.rank - c0);
+  dst += n0 * 128 + ((p ^ (n0 & 7)) << 4);
 #pragma unroll 1
-  for (int n = tid & 7; n < rows; n += 8, d += 128) {
-    *reinterpret_cast<uint4*>(d) = read_piece(args, hidden + c0 + static_cast<size_t>(src[n]) * args.hidden_stride, c0, piece, left);
+  for (int s = 0; s < 2; ++s, dst += N * 128) {
+    const int piece = 8 * s + p, left = cols - 8 * piece;  // columns of this piece that exist
+    if (left <= -8 || (left <= 0 && !(cols & 15))) return;
+    uint8_t* d = dst;
+    if (args.hidden_vec) {
+      // the row numbers of four copies first: one shared-memory round trip for all of them
+      const __half* from = hidden + (left > 0 ? c0 + 8 * piece : 0);
+#pragma unroll 1
+      for (int n = n0; n < rows; n += 64, d += 64 * 128) {
+        int r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = src[min(n + 16 * j, N - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (n + 16 * j < rows) cp_async_16(d + 16 * 128 * j, from + static_cast<size_t>(r[j]) * args.hidden_stride, left > 0);
+      }
+    } else {
+#pragma unroll 1
+      for (int n = n0; n < rows; n += 16, d += 16 * 128)
+        *reinterpret_cast<uint4*>(d) = read_piece(args, hidden + c0 + static_cast<size_t>(src[n]) * args.hidden_stride, c0, piece, left);
+    }
   }
 }
 
@@ -185,8 +206,10 @@ __device__ __forceinline__ void gather_salient(uint8_t* dst, const uint8_t* rows
     const int n = i & (N - 1), kq = i / N;
     if (n >= rows) continue;
     const uint4 cols = *reinterpret_cast<const uint4*>(col + kColHdrBytes + kColTabBytes + (kq >> 1) * kColStepBytes + 64 + (kq & 1) * 16);
-    const uint8_t* base = rows_smem + n * 16;
-    auto ld = [&](uint32_t c) -> uint32_t { return *reinterpret_cast<const uint16_t*>(base + (c & ~7u) * (N * 2) + (c & 7u) * 2); };
+    const uint8_t* base = rows_smem + n * 128;
+    auto ld = [&](uint32_t c) -> uint32_t {
+      return *reinterpret_cast<const uint16_t*>(base + (c >> 6) * (N * 128) + ((((c >> 3) ^ n) & 7u) << 4) + (c & 7u) * 2);
+    };
     auto pair = [&](uint32_t cc) { return ld(cc & 0xFFFFu) | (ld(cc >> 16) << 16); };
     *reinterpret_cast<uint4*>(dst + i * 16) = make_uint4(pair(cols.x), pair(cols.y), pair(cols.z), pair(cols.w));
   }
@@ -210,7 +233,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
   uint64_t* d_empty = d_full + 4;                          // epilogue warps -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 4);
   int* src_rows = reinterpret_cast<int*>(sm + kBarBytes);  // [2][N] source rows of a pass, by pass parity
-  uint8_t* stage_base = sm + kBarBytes + kRowIdxBytes;
+  uint8_t* stage_base = sm + ((smem_u32(sm) + kBarBytes + kRowIdxBytes + kOutBytes + 1023) & ~1023u) - smem_u32(sm);  // the swizzle counts from 1024-byte boundaries
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -355,55 +378,110 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
     }
   } else if (warp < W::kLoad0) {
     // ---- epilogue -------------------------------------------------------------------------------
+    // The buffer goes back as soon as its last accumulators are read: with rows of 128 there is one, and the
+    // MMAs of the next tiles wait for it.  Results go through shared memory, from two rows of an output per word
+    // to eight outputs of a row: 16-byte stores of whole lines.  With 4-byte stores after a shuffle, 8 rows at a
+    // time, the epilogue of a unit took 7200 cycles of the 14000 between units (2048 tokens, 64 experts).
     const int e = (warp - W::kEpi0) >> 2;
     const int row = (warp & 3) * 32 + lane;
     const uint32_t d_lane = tmem + kDBase + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    Ring buf;
-    for (w.start(args); w.valid(); w.next_tile(args)) {
-      const int rows = w.rows(), expert = w.expert;
-      const uint32_t d = d_lane + buf.i * (2 * N);
-      ok = mbar_wait_warp<64>(&d_full[buf.i], buf.phase);
-      if (!ok) break;
-      tcgen05_fence_after();
-      auto load_out = [&](int which, int tile, int n0, float (&y)[8]) {  // scaled and biased
-        tmem_ld<8>(d + which * N + n0, y);
-        tmem_wait_ld();
-        const TrisProjView& pv = args.proj[DUAL ? which : 0];
-        if (pv.output_scale || pv.bias) {
-          const int o = min(tile * kTileOut + row, args.out_features - 1);
-          const size_t at = static_cast<size_t>(expert) * args.out_features + o;
-          const float scale = pv.output_scale ? __half2float(static_cast<const __half*>(pv.output_scale)[at]) : 1.f;
-          const float bias = pv.bias ? __half2float(static_cast<const __half*>(pv.bias)[at]) : 0.f;
+    constexpr bool SILU = MODE == MODE_DUAL_SILU;
+    constexpr int kParts = W::kEpiWarps / 4;  // warpgroups: each takes one projection or tile, or (SILU) every other 16 rows
+    uint32_t* out_tile = reinterpret_cast<uint32_t*>(sm + kBarBytes + kRowIdxBytes) + e * (2 * 8 * kTileOut);
+    int flip = 0;
+    // 16 rows of a tile, as [pair of rows][output] words.  Two buffers: who writes one has passed the barrier
+    // behind its last readers.
+    auto store_tile = [&](__half* out, int tile, int r0, int n0, int rows, const float (&y)[16]) {
+      uint32_t* b = out_tile + flip * (8 * kTileOut);
+      flip ^= 1;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) y[j] = y[j] * scale + bias;
-        }
-      };
-      if constexpr (MODE == MODE_DUAL_SILU) {
-#pragma unroll 1
-        for (int n0 = e * 8; n0 < rows; n0 += 2 * W::kEpiWarps) {
-          float g[8], up[8];
-          load_out(0, w.x, n0, g);
-          load_out(1, w.x, n0, up);
+      for (int j = 0; j < 8; ++j) b[j * kTileOut + row] = h2_as_u32(__floats2half2_rn(y[2 * j], y[2 * j + 1]));
+      named_barrier_sync(2 + e, 128);
+      const int n = n0 + 2 * (row >> 4), o = tile * kTileOut + 8 * (row & 15);
+      if (n >= rows || o >= args.out_features) return;
+      const uint4* from = reinterpret_cast<const uint4*>(b + (row >> 4) * kTileOut + 8 * (row & 15));
+      const uint4 p = from[0], q = from[1];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) g[j] = __fdividef(g[j], 1.f + __expf(-g[j])) * up[j];
-          store_rows<8>(args, args.out[0], w.x * kTileOut + row, w.r0, n0, rows, g);
-        }
-      } else {
-#pragma unroll 1
-        for (int r = e; r < 2; r += W::kEpiWarps / 4) {
-          const int tile = DUAL ? w.x : 2 * w.x + r;
-          if (tile >= args.tiles) break;
-#pragma unroll 1
-          for (int n0 = 0; n0 < rows; n0 += 8) {
-            float y[8];
-            load_out(r, tile, n0, y);
-            store_rows<8>(args, args.out[DUAL ? r : 0], tile * kTileOut + row, w.r0, n0, rows, y);
-          }
+      for (int k = 0; k < 2; ++k) {
+        if (n + k >= rows) break;
+        const int to = args.out_scatter ? args.out_scatter[r0 + n + k] : r0 + n + k;
+        if (to < 0) continue;
+        const uint32_t sel = k ? 0x7632u : 0x5410u;
+        const uint4 w8 = make_uint4(prmt(p.x, p.y, sel), prmt(p.z, p.w, sel), prmt(q.x, q.y, sel), prmt(q.z, q.w, sel));
+        __half* dst = out + static_cast<size_t>(to) * args.out_features + o;
+        if (args.vec_store) {
+          *reinterpret_cast<uint4*>(dst) = w8;
+        } else {
+          const uint32_t h[4] = {w8.x, w8.y, w8.z, w8.w};
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (o + j < args.out_features) dst[j] = __ushort_as_half(static_cast<unsigned short>(h[j >> 1] >> (16 * (j & 1))));
         }
       }
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&d_empty[buf.i]);
+    };
+    Ring buf;
+    for (w.start(args); w.valid(); w.next_tile(args)) {
+      const int rows = w.rows(), expert = w.expert, x = w.x;
+      const uint32_t d = d_lane + buf.i * (2 * N);
+      ok = mbar_wait_warp<64>(&d_full[buf.i], buf.phase);
+      if (named_barrier_or(2 + e, 128, !ok)) {  // the warps of a warpgroup leave together
+        ok = false;
+        break;
+      }
+      tcgen05_fence_after();
+      const int per = (rows + 15) >> 4;  // steps of 16 rows
+      const int halves = SILU ? 1 : (DUAL || 2 * x + 1 < args.tiles ? 2 : 1);
+      const int steps = SILU ? (per + kParts - 1 - e) / kParts : (kParts == 1 ? halves * per : (e < halves ? per : 0));
+      auto give_back = [&]() {
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&d_empty[buf.i]);
+      };
+      // scale and bias of this thread's output, of either projection or tile
+      float scale[2] = {1.f, 1.f}, bias[2] = {0.f, 0.f};
+      bool scaled = false;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const TrisProjView& pv = args.proj[DUAL ? h : 0];
+        if (!(pv.output_scale || pv.bias)) continue;
+        const int o = (DUAL ? x : 2 * x + h) * kTileOut + row;
+        const size_t at = static_cast<size_t>(expert) * args.out_features + min(o, args.out_features - 1);
+        if (pv.output_scale) scale[h] = __half2float(static_cast<const __half*>(pv.output_scale)[at]);
+        if (pv.bias) bias[h] = __half2float(static_cast<const __half*>(pv.bias)[at]);
+        scaled = true;
+      }
+      auto finish = [&](int h, float* y, int count) {
+        if (!scaled) return;
+#pragma unroll
+        for (int j = 0; j < count; ++j) y[j] = y[j] * (h ? scale[1] : scale[0]) + (h ? bias[1] : bias[0]);
+      };
+#pragma unroll 1
+      for (int i = 0; i < steps; ++i) {
+        const int half = SILU ? 0 : (kParts == 1 ? i / per : e);
+        const int n0 = 16 * (SILU ? e + kParts * i : (kParts == 1 ? i - half * per : i));
+        float y[16];
+        if constexpr (SILU) {
+#pragma unroll
+          for (int k = 0; k < 16; k += 8) {
+            float g[8], up[8];
+            tmem_ld<8>(d + n0 + k, g);
+            tmem_ld<8>(d + N + n0 + k, up);
+            tmem_wait_ld();
+            finish(0, g, 8);
+            finish(1, up, 8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) y[k + j] = __fdividef(g[j], 1.f + __expf(-g[j])) * up[j];
+          }
+        } else {
+          tmem_ld<8>(d + half * N + n0, *reinterpret_cast<float(*)[8]>(&y[0]));
+          tmem_ld<8>(d + half * N + n0 + 8, *reinterpret_cast<float(*)[8]>(&y[8]));
+          tmem_wait_ld();
+          finish(half, y, 16);
+        }
+        if (i + 1 == steps) give_back();
+        store_tile(args.out[DUAL ? half : 0], DUAL ? x : 2 * x + half, w.r0, n0, rows, y);
+      }
+      if (steps == 0) give_back();
       buf.advance(kDBufs);
     }
   } else if (warp < W::kMma0) {
@@ -419,7 +497,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
     // Items requested before the oldest one in flight is handed over.  A stage of a reused pass is given back
     // only at the run's last tile, which needs all chunks of the pass handed over: the loader must not wait
     // for such a stage while it still holds one of the same pass back.
-    const int ahead = min(args.stages - 1, args.reuse ? args.stages - args.chunks + 1 : args.stages);
+    const int ahead = min(args.stages - 1, args.reuse ? args.stages - args.pass_chunks + 1 : args.stages);
     Ring put, get;
     auto put_item = [&]() {
       if (w.valid()) {
@@ -429,7 +507,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
         for (int p = 0; p < NC; ++p) {
           const TrisProjView& pv = args.proj[p];
           const uint8_t* src = static_cast<const uint8_t*>(pv.col_records) + static_cast<size_t>(w.expert * args.chunks + w.c) * pv.col_record_bytes;
-          for (int i = tid * 16; i < pv.col_record_bytes; i += kLoadWarps * 32 * 16) cp_async_16(base + p * L.col_bytes + i, src + i);
+          for (int i = tid * 16; i < pv.col_record_bytes; i += kLoadWarps * 32 * 16) cp_async_16(base + L.col_off + p * L.col_bytes + i, src + i);
         }
         if (!waited) {
           pdl_wait();
@@ -438,10 +516,10 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
         }
 #pragma unroll 1
         for (int s = 0; s < args.num_sets; ++s)
-          stage_rows<N>(args, base + L.rows_off + s * L.rows_bytes, args.hidden[s], src_rows + pass * N, w.rows(), w.c * kChunkCols, tid);
+          stage_rows<N>(args, base + s * L.rows_bytes, args.hidden[s], src_rows + pass * N, w.rows(), w.c * kChunkCols, tid);
         rows_of |= static_cast<uint32_t>(w.rows()) << (8 * ahead);
         w.next_stage(args);
-        if (w.c == 0) {
+        if (w.c == w.c_begin) {
           pass ^= 1;
           find_row();
         }
@@ -476,8 +554,8 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       const int rows = static_cast<int>(rows_of & 0xFFu);
 #pragma unroll 1
       for (int p = 0; p < NC; ++p)
-        gather_salient<N>(base + L.sal_off + p * L.sal_bytes, base + L.rows_off + (args.num_sets == 2 ? p : 0) * L.rows_bytes,
-                          base + p * L.col_bytes, rows, tid);
+        gather_salient<N>(base + L.sal_off + p * L.sal_bytes, base + (args.num_sets == 2 ? p : 0) * L.rows_bytes,
+                          base + L.col_off + p * L.col_bytes, rows, tid);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&rows_full[get.i]);
@@ -498,9 +576,10 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
     uint32_t item = 0u;
     for (w.start(args); ok && w.valid(); ++item) {
       const int rows = w.rows(), cols = min(kChunkCols, args.rank - w.c * kChunkCols);
-      const bool first = w.c == 0, last = w.c + 1 == args.chunks;
+      const bool first = w.c == w.c_begin, last = w.c + 1 == w.c_end;
+      const int pass_chunks = w.c_end - w.c_begin;
       const bool mine = DUAL || 2 * w.x + r < args.tiles, last_tile = w.x + 1 == w.x_end;
-      const Ring at_stage = args.reuse ? stage.at(w.c, args.stages) : stage;
+      const Ring at_stage = args.reuse ? stage.at(w.c - w.c_begin, args.stages) : stage;
       w.next(args);  // its route loads overlap the waits below
       const uint32_t idesc = umma_idesc_f16(kTileOut, (rows + 15) & ~15);
       const uint32_t d = tmem + kDBase + buf.i * (2 * N) + r * N;
@@ -510,33 +589,34 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       const uint8_t* base = stage_base + at_stage.i * L.total;
       const int wg = static_cast<int>(item & 1u) * 2 + r;
       Ring sl = (item & 1u) ? slot1 : slot0;
-      // one slot of weights: `n` K = 16 steps against the activations at b_addr
-      auto consume = [&](int n, uint32_t b_addr, uint32_t accumulate) {
+      // one slot of weights: `n` K = 16 steps against the activations at desc, desc + step, ..
+      auto consume = [&](int n, uint64_t desc, auto step, uint32_t accumulate) {
+        constexpr int kStep = decltype(step)::value;
         const int at = wg * 2 + sl.i;
         ok = mbar_wait_warp(&a_full[at], sl.phase) && ok;
         tcgen05_fence_after();
-        const uint64_t desc = umma_smem_desc(b_addr, N * 16, 128);
         const uint32_t a = tmem + at * kACols;
         if (elect_one()) {
           umma_f16_ts(d, a, desc, idesc, accumulate);
           if (n == 4) {
 #pragma unroll
-            for (int j = 1; j < 4; ++j) umma_f16_ts(d, a + 8 * j, desc + j * (2 * N), idesc, 1u);
+            for (int j = 1; j < 4; ++j) umma_f16_ts(d, a + 8 * j, desc + j * kStep, idesc, 1u);
           } else {
-            for (int j = 1; j < n; ++j) umma_f16_ts(d, a + 8 * j, desc + j * (2 * N), idesc, 1u);
+            for (int j = 1; j < n; ++j) umma_f16_ts(d, a + 8 * j, desc + j * kStep, idesc, 1u);
           }
           umma_commit(&a_empty[at]);
         }
         sl.advance(2);
       };
       if (mine) {
-        const uint32_t b_rows = smem_u32(base + L.rows_off + (args.num_sets == 2 ? r : 0) * L.rows_bytes);
+        const uint32_t b_rows = smem_u32(base + (args.num_sets == 2 ? r : 0) * L.rows_bytes);
         for (int s = 0; s * kSliceCols < cols && ok; ++s)
-          consume(min(kSliceCols / 16, (cols - s * kSliceCols + 15) >> 4), b_rows + s * (8 * N * 16), first && s == 0 ? 0u : 1u);
+          consume(min(kSliceCols / 16, (cols - s * kSliceCols + 15) >> 4), umma_smem_desc_sw128(b_rows + s * (N * 128)), std::integral_constant<int, 2>{},
+                  first && s == 0 ? 0u : 1u);
         const int p = DUAL ? r : 0;
-        const int steps = warp_uniform(reinterpret_cast<const ColHeader*>(base + p * L.col_bytes)->num_steps);
+        const int steps = warp_uniform(reinterpret_cast<const ColHeader*>(base + L.col_off + p * L.col_bytes)->num_steps);
         const uint32_t b_sal = smem_u32(base + L.sal_off + p * L.sal_bytes);
-        for (int b = 0; b < steps && ok; b += 4) consume(min(4, steps - b), b_sal + b * (2 * N * 16), 1u);
+        for (int b = 0; b < steps && ok; b += 4) consume(min(4, steps - b), umma_smem_desc(b_sal + b * (2 * N * 16), N * 16, 128), std::integral_constant<int, 2 * N>{}, 1u);
       }
       if (item & 1u) slot1 = sl;
       else slot0 = sl;
@@ -546,7 +626,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       }
       if (last) buf.advance(kDBufs);
       if (!args.reuse) stage.advance(args.stages);
-      else if (last && last_tile) stage = stage.at(args.chunks, args.stages);
+      else if (last && last_tile) stage = stage.at(pass_chunks, args.stages);
     }
   }
   if (!ok && args.status) atomicExch(args.status, TRIS_ERR_TIMEOUT);
@@ -612,10 +692,12 @@ static int row_split(long long units, int max_rows, int n) {
 template <int N, int MODE>
 static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {
   const size_t stage = stage_bytes<MODE>(args, N);
-  args.stages = static_cast<int>(std::min<size_t>(kMaxStages, (kMostSmem - kBarBytes - kRowIdxBytes) / stage));
+  args.stages = static_cast<int>(std::min<size_t>(kMaxStages, (kMostSmem - kHeadBytes) / stage));
   TRIS_REQUIRE(args.stages >= 2, TRIS_ERR_UNSUPPORTED, "grouped_tiled_kernel: %zu bytes per stage", stage);
-  args.reuse = args.chunks <= args.stages;
-  const size_t smem = kBarBytes + kRowIdxBytes + args.stages * stage;
+  args.pass_chunks = args.chunks;
+  args.col_split = 1;
+  args.reuse = args.pass_chunks <= args.stages;
+  const size_t smem = kHeadBytes + args.stages * stage;
   auto kernel = grouped_tiled_kernel<N, MODE>;
   static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
   int st = configure_smem(kernel, smem, configured);
@@ -631,7 +713,7 @@ static int dispatch_tiled(TiledArgs& args, int max_rows, int typical_rows, cudaS
   args.units_x = MODE == MODE_SINGLE ? (args.tiles + 1) / 2 : args.tiles;
   if (typical_rows <= kDecodeMaxRows) return launch_grouped_decode(args, MODE, typical_rows, stream, pdl);
   // two stages of the widest pass have to fit shared memory (many salient columns make a stage larger)
-  if (typical_rows <= 64 || 2 * stage_bytes<MODE>(args, 128) + kBarBytes + kRowIdxBytes > kMostSmem) return launch_tiled<64, MODE>(args, max_rows, stream, pdl);
+  if (typical_rows <= 64 || 2 * stage_bytes<MODE>(args, 128) + kHeadBytes > kMostSmem) return launch_tiled<64, MODE>(args, max_rows, stream, pdl);
   return launch_tiled<128, MODE>(args, max_rows, stream, pdl);
 }
 
@@ -686,8 +768,7 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   a.hidden_vec = a.hidden_mode == TRIS_OUT_F16 && !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 &&
                  ((reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1])) & 15u) == 0;
   a.quad_store = proj_a->out_features % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 7u) == 0;
-  a.pair_store = proj_a->out_features % 2 == 0 &&
-                 ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 3u) == 0;
+  a.vec_store = proj_a->out_features % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 15u) == 0;
   TRIS_REQUIRE(a.col_scale == nullptr || a.hidden_mode == TRIS_OUT_F16, TRIS_ERR_INVALID_ARG,
                "grouped (tile records): hidden_col_scale needs row-major activation rows");
   TRIS_REQUIRE(a.hidden_mode == TRIS_OUT_F16 || proj_a->rank % 32 == 0, TRIS_ERR_INVALID_ARG,

@@ -29,6 +29,7 @@ struct TiledArgs {
   int32_t num_rows;
   int32_t rank, out_features, num_experts;  // the same for both projections
   int32_t tiles, chunks, units_x, row_split;
+  int32_t col_split, pass_chunks;  // parts of the chunks that different CTAs take; chunks of the longest part
   int32_t max_steps;            // salient steps a record of either projection can have
   int32_t max_sub_bytes;        // larger sub-record of the two projections
   int32_t hidden_mode;          // column order of the activation rows (TRIS_OUT_F16 / _PAIR_INTERLEAVED / _LANE_ORDER)
@@ -38,7 +39,7 @@ struct TiledArgs {
   int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
   int32_t stages;               // ring depth, 2 .. kMaxStages
   int32_t reuse;                // the chunks of a pass fit the ring: staged once for all tiles of a run
-  int32_t pair_store;           // 4-byte stores of two outputs are aligned
+  int32_t vec_store;            // 16-byte stores of eight outputs are aligned
   int32_t quad_store;           // 8-byte stores of four outputs are aligned
   const __half* col_scale;      // optional [rank]: activation rows are multiplied by it while staged
 };
@@ -52,41 +53,6 @@ static __device__ __noinline__ uint4 read_piece(const TiledArgs& args, const __h
     w[v >> 1] |= static_cast<uint32_t>(__half_as_ushort(x)) << (16 * (v & 1));
   }
   return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-// COUNT consecutive rows (n0 ..) of output column o, one lane per output: neighbouring lanes swap
-// halves so that each stores two outputs of one row at once.
-template <int COUNT>
-__device__ __forceinline__ void store_rows(const TiledArgs& args, __half* out, int o, int r0, int n0, int rows, const float (&v)[COUNT]) {
-  const int odd = threadIdx.x & 1;
-  const bool in = o < args.out_features;
-  if (args.pair_store) {
-    int n = n0 + odd;
-    __half* dst = out + (o & ~1) + static_cast<size_t>(r0 + n) * args.out_features;
-    const size_t step = 2 * static_cast<size_t>(args.out_features);
-#pragma unroll
-    for (int j = 0; j < COUNT; j += 2, n += 2, dst += step) {
-      if (n0 + j >= rows) break;
-      const uint32_t p = h2_as_u32(__floats2half2_rn(v[j], v[j + 1]));
-      const uint32_t q = __shfl_xor_sync(0xFFFFFFFFu, p, 1);
-      if (n < rows && in) {
-        const uint32_t w = odd ? prmt(q, p, 0x7632u) : prmt(p, q, 0x5410u);
-        if (!args.out_scatter) {
-          *reinterpret_cast<uint32_t*>(dst) = w;
-        } else {
-          const int orow = args.out_scatter[r0 + n];
-          if (orow >= 0) *reinterpret_cast<uint32_t*>(out + (o & ~1) + static_cast<size_t>(orow) * args.out_features) = w;
-        }
-      }
-    }
-  } else if (in) {
-#pragma unroll
-    for (int j = 0; j < COUNT; ++j) {
-      if (n0 + j >= rows) break;
-      const int orow = args.out_scatter ? args.out_scatter[r0 + n0 + j] : r0 + n0 + j;
-      if (orow >= 0) out[static_cast<size_t>(orow) * args.out_features + o] = __float2half_rn(v[j]);
-    }
-  }
 }
 
 // ---- host helpers -----------------------------------------------------------------------------------

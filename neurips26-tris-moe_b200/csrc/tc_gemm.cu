@@ -304,11 +304,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* m
                "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
                : "memory");
 }
-// K-major, 128-byte swizzle: 1024 bytes between 8-row groups; a K = 16 step is 32 bytes further.
-__device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t smem_addr) {
-  return static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) |
-         (2ull << 61);
-}
 
 template <int NTILE>
 __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_constant__ TcGemmArgs args,
