@@ -517,6 +517,17 @@ int tris_page_experts(const TrisPageJob* jobs, int32_t num_jobs, const int32_t* 
                       const int32_t* num_segments_dev, int32_t num_segments, int32_t num_experts,
                       int32_t* slot_table, void* stream);
 
+/*
+ * tris_grouped_forward (proj_b NULL) and tris_grouped_pair_forward with scratch, for an ordinary matrix (a route
+ * without arrays) of more than a few rows: with it the columns of the matrix can be shared among CTAs too.  The
+ * size may be 0; a smaller or NULL workspace is valid and means less or no sharing.  16-byte aligned; free again
+ * when the launch has ended.  projections: 1 or 2 (the pair).
+ */
+size_t tris_linear_workspace_bytes(const TrisProjView* proj, int32_t projections, int32_t num_rows);
+int tris_linear_forward(const TrisProjView* proj_a, const TrisProjView* proj_b, const TrisRouteView* route,
+                        const void* hidden_a_f16, const void* hidden_b_f16, void* out_a_f16, void* out_b_f16,
+                        int32_t fuse_silu_mul, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- whole MoE block --------------------------------------------------------------- */
 
 typedef struct TrisMoeLayerView {

@@ -113,6 +113,8 @@ int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRou
 struct LaunchOpts {
   bool pdl = false;                  // programmatic dependent launch
   bool weights_before_wait = false;  // the route was complete before the predecessor kernel started
+  void* workspace = nullptr;         // scratch of the column split (grouped_split_bytes), optional
+  size_t workspace_bytes = 0;
 };
 int grouped_forward_impl(const TrisProjView* proj, const TrisRouteView* route, const void* hidden_f16, void* out_f16,
                          cudaStream_t stream, LaunchOpts opts);
@@ -128,6 +130,7 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
 // leave the decode-regime kernels for the tcgen05 kernel (tris_set_grouped_tc_min_rows).
 int grouped_tc_min_rows();
 int route_rows_hint(const TrisRouteView* route);
+size_t grouped_split_bytes(const TrisProjView* proj, int projections, int num_rows);
 int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t stream);
 int combine_routed_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,
                         int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream, bool pdl,

@@ -683,3 +683,19 @@ extern "C" int tris_grouped_pair_forward(const TrisProjView* proj_a, const TrisP
                                    fuse_silu_mul, static_cast<cudaStream_t>(stream), opts);
 }
 
+
+extern "C" size_t tris_linear_workspace_bytes(const TrisProjView* proj, int32_t projections, int32_t num_rows) {
+  return proj != nullptr && (projections == 1 || projections == 2) && num_rows > 0 ? grouped_split_bytes(proj, projections, num_rows) : 0;
+}
+
+extern "C" int tris_linear_forward(const TrisProjView* proj_a, const TrisProjView* proj_b, const TrisRouteView* route, const void* hidden_a_f16,
+                                   const void* hidden_b_f16, void* out_a_f16, void* out_b_f16, int32_t fuse_silu_mul, void* workspace,
+                                   size_t workspace_bytes, void* stream) {
+  LaunchOpts opts;
+  opts.pdl = programmatic_launch_default();
+  opts.workspace = workspace;
+  opts.workspace_bytes = workspace ? workspace_bytes : 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (proj_b == nullptr) return grouped_forward_impl(proj_a, route, hidden_a_f16, out_a_f16, s, opts);
+  return grouped_pair_forward_impl(proj_a, proj_b, route, hidden_a_f16, hidden_b_f16, out_a_f16, out_b_f16, fuse_silu_mul, s, opts);
+}

@@ -75,7 +75,7 @@ __host__ __device__ inline StageLayout stage_layout(int max_steps, int ncol, int
 template <int N>
 struct Walker {
   int u, u_end, nseg;
-  int x, x_begin, x_end, expert, row_end, r0, c, c_begin, c_end;
+  int x, x_begin, x_end, expert, row_end, r0, c, c_begin, c_end, part;
   int next_x, next_expert, next_begin, next_end, next_part;
   __device__ __forceinline__ void peek(const TiledArgs& args, int unit) {
     if (unit >= u_end) return;
@@ -116,8 +116,9 @@ struct Walker {
       expert = warp_uniform(next_expert);
       r0 = warp_uniform(next_begin);
       row_end = min(warp_uniform(next_end), args.num_rows);
-      c = c_begin = next_part * args.chunks / args.col_split;
-      c_end = (next_part + 1) * args.chunks / args.col_split;
+      part = next_part;
+      c = c_begin = part * args.chunks / args.col_split;
+      c_end = (part + 1) * args.chunks / args.col_split;
       peek(args, u + (x_end - x_begin));
       if (expert >= 0 && expert < args.num_experts && r0 < row_end) return;
       u += x_end - x_begin;
@@ -443,7 +444,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const TrisProjView& pv = args.proj[DUAL ? h : 0];
-        if (!(pv.output_scale || pv.bias)) continue;
+        if (args.partial || !(pv.output_scale || pv.bias)) continue;
         const int o = (DUAL ? x : 2 * x + h) * kTileOut + row;
         const size_t at = static_cast<size_t>(expert) * args.out_features + min(o, args.out_features - 1);
         if (pv.output_scale) scale[h] = __half2float(static_cast<const __half*>(pv.output_scale)[at]);
@@ -479,6 +480,14 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
           finish(half, y, 16);
         }
         if (i + 1 == steps) give_back();
+        if (!SILU && args.partial) {  // a part of the columns: fp32 sums, [part][projection][row][output]
+          const int o = (DUAL ? x : 2 * x + half) * kTileOut + row;
+          float* dst = args.partial + (static_cast<size_t>(w.part * NC + (DUAL ? half : 0)) * args.num_rows + w.r0 + n0) * args.out_features + o;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (n0 + j < rows && o < args.out_features) dst[static_cast<size_t>(j) * args.out_features] = y[j];
+          continue;
+        }
         store_tile(args.out[DUAL ? half : 0], DUAL ? x : 2 * x + half, w.r0, n0, rows, y);
       }
       if (steps == 0) give_back();
@@ -689,23 +698,94 @@ static int row_split(long long units, int max_rows, int n) {
   return static_cast<int>(std::max<long long>(1, std::min<long long>({limit, sm_count() / units, (max_rows + n - 1) / n})));
 }
 
+// Column split of one ordinary matrix (no experts): its units of two output tiles and its row passes together are
+// too few for the SMs, and its columns many - parts of the columns go to CTAs of their own, whose fp32 sums
+// sum_parts_kernel adds in order.  4096 columns, 512 rows: 64 units for 4096 outputs (two parts), 32 for a pair of
+// 1024 (four): 92 -> SPLIT_Q and 88 -> SPLIT_KV us.  At least two chunks per part: the sums cost 128 KB of
+// traffic a part.
+static int col_split(const TiledArgs& args, int mode, long long units) {
+  if (args.expert_ids || !args.partial || units <= 0) return 1;
+  const size_t part = sizeof(float) * static_cast<size_t>(args.num_rows) * args.out_features * (mode == MODE_SINGLE ? 1 : 2);
+  return static_cast<int>(std::max<long long>(1, std::min<long long>({args.chunks / 2, sm_count() / units, static_cast<long long>(args.partial_bytes / part)})));
+}
+
+// One thread per four outputs of a row: adds the parts, then scale, bias and SiLU * up as the epilogue would.
+template <int MODE>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ TiledArgs args) {
+  constexpr int P = MODE == MODE_SINGLE ? 1 : 2;
+  const int quads = (args.out_features + 3) / 4;
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  const int row = static_cast<int>(i / quads), o = static_cast<int>(i - static_cast<long long>(row) * quads) * 4;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (row >= args.num_rows) return;
+  const int to = args.out_scatter ? args.out_scatter[row] : row;
+  if (to < 0) return;
+  float y[P][4];
+  const bool vec = args.out_features % 4 == 0;
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) y[p][j] = 0.f;
+    for (int k = 0; k < args.col_split; ++k) {
+      const float* src = args.partial + (static_cast<size_t>(k * P + p) * args.num_rows + row) * args.out_features + o;
+      if (vec) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(src));
+        y[p][0] += v.x, y[p][1] += v.y, y[p][2] += v.z, y[p][3] += v.w;
+      } else {
+        for (int j = 0; j < 4 && o + j < args.out_features; ++j) y[p][j] += __ldcg(src + j);
+      }
+    }
+    const TrisProjView& pv = args.proj[p];
+    for (int j = 0; j < 4 && o + j < args.out_features; ++j) {
+      if (pv.output_scale) y[p][j] *= __half2float(static_cast<const __half*>(pv.output_scale)[o + j]);
+      if (pv.bias) y[p][j] += __half2float(static_cast<const __half*>(pv.bias)[o + j]);
+    }
+  }
+  if constexpr (MODE == MODE_DUAL_SILU) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) y[0][j] = __fdividef(y[0][j], 1.f + __expf(-y[0][j])) * y[1][j];
+  }
+#pragma unroll
+  for (int p = 0; p < (MODE == MODE_DUAL_STORE ? 2 : 1); ++p) {
+    __half* dst = args.out[p] + static_cast<size_t>(to) * args.out_features + o;
+    if (args.quad_store) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(h2_as_u32(__floats2half2_rn(y[p][0], y[p][1])), h2_as_u32(__floats2half2_rn(y[p][2], y[p][3])));
+    } else {
+      for (int j = 0; j < 4 && o + j < args.out_features; ++j) dst[j] = __float2half_rn(y[p][j]);
+    }
+  }
+}
+
+template <int N, int MODE>
+static int launch_main(const TiledArgs& args, int grid, size_t smem, cudaStream_t stream, bool pdl) {
+  auto kernel = grouped_tiled_kernel<N, MODE>;
+  static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
+  const int st = configure_smem(kernel, smem, configured);
+  if (st != TRIS_OK) return st;
+  return check_cuda(launch_kernel(kernel, dim3(grid), dim3(Roles<N>::kThreads), smem, stream, pdl, 1, args), "grouped_tiled_kernel launch");
+}
+
 template <int N, int MODE>
 static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {
   const size_t stage = stage_bytes<MODE>(args, N);
   args.stages = static_cast<int>(std::min<size_t>(kMaxStages, (kMostSmem - kHeadBytes) / stage));
   TRIS_REQUIRE(args.stages >= 2, TRIS_ERR_UNSUPPORTED, "grouped_tiled_kernel: %zu bytes per stage", stage);
-  args.pass_chunks = args.chunks;
-  args.col_split = 1;
-  args.reuse = args.pass_chunks <= args.stages;
   const size_t smem = kHeadBytes + args.stages * stage;
-  auto kernel = grouped_tiled_kernel<N, MODE>;
-  static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
-  int st = configure_smem(kernel, smem, configured);
-  if (st != TRIS_OK) return st;
   const long long units = static_cast<long long>(args.units_x) * args.num_segments;
   args.row_split = row_split(units, max_rows, N);
-  const int grid = static_cast<int>(std::min<long long>(units * args.row_split, sm_count()));
-  return check_cuda(launch_kernel(kernel, dim3(grid), dim3(Roles<N>::kThreads), smem, stream, pdl, 1, args), "grouped_tiled_kernel launch");
+  args.col_split = col_split(args, MODE, units * args.row_split);
+  args.pass_chunks = ceil_div(args.chunks, args.col_split);
+  args.reuse = args.pass_chunks <= args.stages;
+  if (args.col_split == 1) args.partial = nullptr;
+  const int grid = static_cast<int>(std::min<long long>(units * args.row_split * args.col_split, sm_count()));
+  if (!args.partial) return launch_main<N, MODE>(args, grid, smem, stream, pdl);
+  // parts of gate and up are stored apart; the sum kernel applies SiLU * up
+  const int st = launch_main<N, MODE == MODE_DUAL_SILU ? MODE_DUAL_STORE : MODE>(args, grid, smem, stream, pdl);
+  if (st != TRIS_OK) return st;
+  const long long quads = static_cast<long long>(args.num_rows) * ceil_div(args.out_features, 4);
+  return check_cuda(launch_kernel(sum_parts_kernel<MODE>, dim3(static_cast<unsigned>((quads + 255) / 256)), dim3(256), 0, stream, /*pdl=*/true, 1, args),
+                    "sum_parts_kernel launch");
 }
 
 template <int MODE>
@@ -764,6 +844,8 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   a.hidden_stride = route->hidden_row_stride > 0 ? route->hidden_row_stride : proj_a->rank;
   a.weights_before_wait = opts.pdl && opts.weights_before_wait;
   a.num_sets = (mode != MODE_SINGLE && a.hidden[0] != a.hidden[1]) ? 2 : 1;
+  a.partial = static_cast<float*>(opts.workspace);
+  a.partial_bytes = opts.workspace_bytes;
   a.col_scale = static_cast<const __half*>(route->hidden_col_scale);
   a.hidden_vec = a.hidden_mode == TRIS_OUT_F16 && !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 &&
                  ((reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1])) & 15u) == 0;
@@ -790,4 +872,14 @@ int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t 
 
 extern "C" int tris_set_grouped_row_split_max(int32_t ctas) {
   return tris::tr::g_row_split_max.exchange(ctas < 1 ? 1 : (ctas > 16 ? 16 : ctas), std::memory_order_relaxed);
+}
+
+// Bytes that let launch_grouped_tiled split the columns as far as it would: one part per SM-filling share.
+size_t tris::grouped_split_bytes(const TrisProjView* proj, int projections, int num_rows) {
+  using namespace tr;
+  if (!proj_has_tile_records(*proj) || num_rows <= kDecodeMaxRows || num_chunks(proj->rank) < 4) return 0;
+  const long long tiles = tiles_per_expert(proj->out_features), units = projections == 1 ? (tiles + 1) / 2 : tiles;
+  const long long row_parts = std::max<long long>(1, std::min<long long>(sm_count() / units, (num_rows + 127) / 128));
+  const long long parts = std::min<long long>(num_chunks(proj->rank) / 2, sm_count() / (units * std::min<long long>(row_parts, g_row_split_max.load(std::memory_order_relaxed))));
+  return parts <= 1 ? 0 : sizeof(float) * static_cast<size_t>(parts) * projections * num_rows * proj->out_features;
 }

@@ -41,6 +41,8 @@ struct TiledArgs {
   int32_t reuse;                // the chunks of a pass fit the ring: staged once for all tiles of a run
   int32_t vec_store;            // 16-byte stores of eight outputs are aligned
   int32_t quad_store;           // 8-byte stores of four outputs are aligned
+  float* partial;               // fp32 sums of the column parts, or null: no column split
+  size_t partial_bytes;
   const __half* col_scale;      // optional [rank]: activation rows are multiplied by it while staged
 };
 

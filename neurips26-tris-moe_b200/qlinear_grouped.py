@@ -471,6 +471,15 @@ def _route_view(route: dict, num_rows: int, keep: list) -> TrisRouteView:
     return rv
 
 
+def _linear_workspace(lib, view: TrisProjView, projections: int, rows: int, dev) -> Optional[torch.Tensor]:
+    """Scratch of an ordinary matrix whose columns are shared among CTAs; None where they are not (32 rows
+    or fewer among others: the decode kernel shares them inside a CTA)."""
+    if rows <= 32:
+        return None
+    need = int(lib.tris_linear_workspace_bytes(C.byref(view), projections, rows))
+    return torch.empty((need,), dtype=torch.uint8, device=dev) if need else None
+
+
 def _ns_payload_is_noop(ns_payload) -> bool:
     if ns_payload is None:
         return True
@@ -536,10 +545,13 @@ def run_grouped_structured_expert_forward(
     keep: list = []
     rv = _route_view(route, R, keep)
     with torch.cuda.device(hidden.device):
-        _native.check(
-            lib.tris_grouped_forward(C.byref(view), C.byref(rv), hidden.data_ptr(), out.data_ptr(), _stream_ptr(hidden.device)),
-            "grouped_forward",
-        )
+        ws = _linear_workspace(lib, view, 1, R, hidden.device) if route.get("_one_segment") else None
+        if ws is not None:
+            st = lib.tris_linear_forward(C.byref(view), None, C.byref(rv), hidden.data_ptr(), None, out.data_ptr(), None, 0, ws.data_ptr(),
+                                         ws.numel(), _stream_ptr(hidden.device))
+        else:
+            st = lib.tris_grouped_forward(C.byref(view), C.byref(rv), hidden.data_ptr(), out.data_ptr(), _stream_ptr(hidden.device))
+        _native.check(st, "grouped_forward")
     if with_ns:  # out += (x . C2^T) . C1^T of each row's expert (qlinear_cuda.py:2318-2333)
         from .ns_compensation import run_grouped_ns_compensation_forward
 
@@ -599,12 +611,15 @@ def run_grouped_structured_expert_pair_forward(
     keep: list = []
     rv = _route_view(route, R, keep)
     with torch.cuda.device(dev):
-        _native.check(
-            lib.tris_grouped_pair_forward(C.byref(va), C.byref(vb), C.byref(rv), ha.data_ptr(), hb.data_ptr(),
-                                          out_a.data_ptr(), None if out_b is None else out_b.data_ptr(),
-                                          int(bool(fuse_silu_mul)), _stream_ptr(dev)),
-            "grouped_pair_forward",
-        )
+        b_ptr = None if out_b is None else out_b.data_ptr()
+        ws = _linear_workspace(lib, va, 2, R, dev) if route.get("_one_segment") else None
+        if ws is not None:
+            st = lib.tris_linear_forward(C.byref(va), C.byref(vb), C.byref(rv), ha.data_ptr(), hb.data_ptr(), out_a.data_ptr(), b_ptr,
+                                         int(bool(fuse_silu_mul)), ws.data_ptr(), ws.numel(), _stream_ptr(dev))
+        else:
+            st = lib.tris_grouped_pair_forward(C.byref(va), C.byref(vb), C.byref(rv), ha.data_ptr(), hb.data_ptr(), out_a.data_ptr(), b_ptr,
+                                               int(bool(fuse_silu_mul)), _stream_ptr(dev))
+        _native.check(st, "grouped_pair_forward")
     if ns_a or ns_b:  # qlinear_cuda.py:2611-2633
         from .ns_compensation import run_grouped_ns_compensation_forward
 

@@ -81,6 +81,37 @@ def test_grouped_kernels_at_tile_edges(lib, O, rank, group, lengths):
         _assert_within(mlp[rows], want, err)
 
 
+@pytest.mark.parametrize("O,K,T", [(136, 520, 33), (137, 1100, 64), (1024, 2048, 65), (256, 4096, 130), (72, 8192, 300), (4096, 512, 257)])
+def test_linear_columns_shared_among_ctas(lib, O, K, T):
+    """An ordinary matrix of more than 32 rows: its columns in one to many parts, single and as a pair."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(O + K)
+    mods = []
+    for _ in range(2):
+        p = synth.pack_projection(synth.raw_projection(rng, 1, O, K, group_size=128))
+        p["output_scale"] = torch.from_numpy((1 + 0.2 * rng.standard_normal((1, O))).astype(np.float16))
+        p["has_output_scale"] = True
+        mods.append(tm.Compact3Linear(p, device="cuda"))
+    x = (0.5 * torch.randn((T, K), generator=torch.Generator().manual_seed(T))).half().cuda()
+    refs = []
+    for m in mods:
+        w = tm.dequantize_grouped_payload(m.payload)[0]
+        ref, err, _ = _bound(w, x)
+        sc = m.payload["output_scale"].double().reshape(1, O)
+        refs.append((ref * sc, err * sc.abs() * (1 + 2.0 ** -22) + (ref * sc).abs() * 2.0 ** -22))
+    half = lambda r, e: e * (1 + 2.0 ** -10) + r.abs() * 2.0 ** -11 + 2.0 ** -25
+    _assert_within(mods[0](x), refs[0][0], half(*refs[0]))
+    a, b = tm.run_compact3_gate_up_forward(mods[0], mods[1], x, fuse_silu_mul=False)
+    _assert_within(a, refs[0][0], half(*refs[0]))
+    _assert_within(b, refs[1][0], half(*refs[1]))
+    (ra, ea), (rb, eb) = refs
+    silu = ra * torch.sigmoid(ra)
+    err = 1.1 * ea * rb.abs() + silu.abs() * eb + 1.1 * ea * eb + (silu * rb).abs() * (2.0 ** -11 + 2.0 ** -19) + 2.0 ** -25
+    _assert_within(tm.run_compact3_gate_up_forward(mods[0], mods[1], x), silu * rb, err)
+
+
 @pytest.mark.parametrize("rows,cols,group,T", [
     (16, 32, 32, 1), (17, 40, 40, 8), (64, 64, 32, 9), (48, 96, 96, 17), (72, 128, 64, 33), (256, 264, 264, 65), (128, 2048, 128, 200),
 ])
