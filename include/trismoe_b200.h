@@ -463,6 +463,13 @@ int tris_grouped_hidden_layout(const TrisProjView* proj_a, const TrisProjView* p
                                int32_t num_segments, int32_t max_rows_per_segment);
 
 /*
+ * out = routed + sigmoid(x . gate_weight^T) * shared, all [T, H] fp16 but gate_weight [1, H]: how the shared
+ * expert joins the routed ones (modeling_qwen2_moe.py:815-818).  out may be routed.
+ */
+int tris_shared_expert_add(const void* x_f16, const void* gate_weight_f16, const void* routed_f16, const void* shared_f16,
+                           int32_t num_tokens, int32_t hidden_size, void* out_f16, void* stream);
+
+/*
  * final[T, H] fp16 = sum over slots of routing_weights[t, s] * down_out[row_of_flat[t*k+s]]
  * (the index_add_ of MO:1038-1043, as a deterministic gather in fp32).  A negative row index
  * contributes nothing.

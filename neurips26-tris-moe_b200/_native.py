@@ -117,6 +117,7 @@ SIGNATURES = {
     "tris_set_grouped_tc_min_rows": (C.c_int, [_i32]),
     "tris_set_grouped_row_split_max": (C.c_int, [_i32]),
     "tris_combine_routed": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp, _vp]),
+    "tris_shared_expert_add": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp]),
     "tris_page_experts": (C.c_int, [_vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp]),
     "tris_moe_layer_workspace_bytes": (C.c_size_t, [_P(TrisMoeLayerView), _i32]),
     "tris_moe_layer_last_status": (C.c_int, [_vp, _i32, _vp, _P(_i32)]),

@@ -554,6 +554,48 @@ int launch_router_route(const float* logits, int num_tokens, int num_experts, in
                                   segment_offsets, problem_offsets, counts, stream);
 }
 
+// out = routed + sigmoid(x . gate) * shared, one CTA per token; the dot product, the sigmoid and the product are rounded
+// to fp16 where separate operators round them.  Four small launches (matrix-vector product, sigmoid, product,
+// sum) cost 30 us of host time; the data is a few hundred KB.
+__global__ void __launch_bounds__(256) shared_expert_add_kernel(const __half* x, const __half* gate, const __half* routed, const __half* shared,
+                                                                int hidden, int vec, __half* out) {
+  __shared__ float parts[8];
+  pdl_wait();
+  pdl_launch_dependents();
+  const size_t row = static_cast<size_t>(blockIdx.x) * hidden;
+  float sum = 0.f;
+  if (vec) {
+    for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8) {
+      const uint4 a = *reinterpret_cast<const uint4*>(x + row + c), b = *reinterpret_cast<const uint4*>(gate + c);
+      const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 p = __half22float2(u32_as_h2(av[j])), q = __half22float2(u32_as_h2(bv[j]));
+        sum += p.x * q.x + p.y * q.y;
+      }
+    }
+  } else {
+    for (int c = threadIdx.x; c < hidden; c += 256) sum += __half2float(x[row + c]) * __half2float(gate[c]);
+  }
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+  if ((threadIdx.x & 31) == 0) parts[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sum += parts[i];
+  const float z = __half2float(__float2half_rn(sum));
+  const __half2 s = __half2half2(__float2half_rn(1.f / (1.f + expf(-z))));
+  if (vec) {
+    for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8) {
+      const uint4 a = *reinterpret_cast<const uint4*>(routed + row + c), b = *reinterpret_cast<const uint4*>(shared + row + c);
+      auto one = [&](uint32_t r, uint32_t v) { return h2_as_u32(__hadd2_rn(u32_as_h2(r), __hmul2_rn(s, u32_as_h2(v)))); };
+      *reinterpret_cast<uint4*>(out + row + c) = make_uint4(one(a.x, b.x), one(a.y, b.y), one(a.z, b.z), one(a.w, b.w));
+    }
+  } else {
+    for (int c = threadIdx.x; c < hidden; c += 256) out[row + c] = __hadd_rn(routed[row + c], __hmul_rn(__low2half(s), shared[row + c]));
+  }
+}
+
 // Owner rank of an expert under the contiguous partition (sizes differ by at most one).
 __device__ __forceinline__ int ep_owner(int e, int base, int extra) {
   const int big = extra * (base + 1);
@@ -721,4 +763,18 @@ extern "C" int tris_combine_routed(const void* down_out_f16, const int32_t* row_
                                    void* stream) {
   return combine_routed_impl(down_out_f16, row_of_flat, routing_weights, num_tokens, top_k, hidden_size, final_f16,
                              static_cast<cudaStream_t>(stream), programmatic_launch_default());
+}
+
+extern "C" int tris_shared_expert_add(const void* x_f16, const void* gate_weight_f16, const void* routed_f16, const void* shared_f16,
+                                      int32_t num_tokens, int32_t hidden_size, void* out_f16, void* stream) {
+  TRIS_REQUIRE(x_f16 && gate_weight_f16 && routed_f16 && shared_f16 && out_f16, TRIS_ERR_INVALID_ARG, "tris_shared_expert_add: null pointer");
+  TRIS_REQUIRE(num_tokens >= 0 && hidden_size > 0, TRIS_ERR_INVALID_ARG, "tris_shared_expert_add: bad sizes");
+  if (num_tokens == 0) return TRIS_OK;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(x_f16) | reinterpret_cast<uintptr_t>(gate_weight_f16) | reinterpret_cast<uintptr_t>(routed_f16) |
+                        reinterpret_cast<uintptr_t>(shared_f16) | reinterpret_cast<uintptr_t>(out_f16);
+  return check_cuda(launch_kernel(shared_expert_add_kernel, dim3(num_tokens), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                  programmatic_launch_default(), 1, static_cast<const __half*>(x_f16), static_cast<const __half*>(gate_weight_f16),
+                                  static_cast<const __half*>(routed_f16), static_cast<const __half*>(shared_f16), hidden_size,
+                                  hidden_size % 8 == 0 && (all & 15u) == 0 ? 1 : 0, static_cast<__half*>(out_f16)),
+                    "shared_expert_add_kernel launch");
 }

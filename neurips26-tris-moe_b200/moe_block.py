@@ -446,5 +446,13 @@ class TrisQwen2SparseMoeBlock(TrisSparseMoeBlock):
         shared = down_proj(mlp)
         if shared is None:
             raise RuntimeError("trismoe_b200: shared expert kernels returned no result")
-        scale = torch.sigmoid(torch.nn.functional.linear(hidden_states, self.shared_expert_gate.weight))
-        return routed + scale * shared, logits
+        w = self.shared_expert_gate.weight
+        if not (routed.dtype == shared.dtype == hidden_states.dtype == w.dtype == torch.float16 and routed.is_contiguous() and w.is_contiguous()):
+            return routed + torch.sigmoid(torch.nn.functional.linear(hidden_states, w)) * shared, logits
+        x, shared = hidden_states.contiguous(), shared.contiguous()
+        T = routed.numel() // self.hidden_size
+        with torch.cuda.device(routed.device):
+            _native.check(_native.load().tris_shared_expert_add(x.data_ptr(), w.data_ptr(), routed.data_ptr(), shared.data_ptr(), T, self.hidden_size,
+                                                                routed.data_ptr(), torch.cuda.current_stream(routed.device).cuda_stream),
+                          "shared_expert_add")
+        return routed, logits

@@ -129,6 +129,23 @@ def test_packed4_gemm_at_tile_edges(lib, rows, cols, group, T):
         _assert_within(lin(xi), ref, bound)
 
 
+@pytest.mark.parametrize("T,H", [(1, 64), (3, 100), (70, 2048), (2, 4104)])
+def test_shared_expert_add(lib, T, H):
+    import trismoe_b200 as tm
+
+    g = torch.Generator().manual_seed(H)
+    x, routed, shared = (torch.randn((T, H), generator=g).half().cuda() for _ in range(3))
+    w = (torch.randn((1, H), generator=g) * H ** -0.5).half().cuda()
+    out = torch.empty_like(x)
+    tm._native.check(lib.tris_shared_expert_add(x.data_ptr(), w.data_ptr(), routed.data_ptr(), shared.data_ptr(), T, H, out.data_ptr(),
+                                                torch.cuda.current_stream().cuda_stream))
+    z = (x.double() * w.double()).sum(1, keepdim=True)
+    gate = torch.sigmoid(z)
+    # the logit and the gate rounded to fp16 (|sigmoid'| <= 1/4), the product and the sum too
+    err = shared.double().abs() * (z.abs() * 2.0 ** -13 + 2.0 ** -20 + gate * 2.0 ** -10) + (routed.double() + gate * shared.double()).abs() * 2.0 ** -10 + 2.0 ** -24
+    _assert_within(out, routed.double() + gate * shared.double(), err)
+
+
 @pytest.mark.parametrize("T", [1, 37, 300])
 @pytest.mark.parametrize("pairs,scales", [("gate up down", ""), ("gate", "up"), ("up", "gate down"), ("down", "gate up down"), ("", "down")])
 def test_null_space_and_input_scales_in_one_sequence(lib, T, pairs, scales):
