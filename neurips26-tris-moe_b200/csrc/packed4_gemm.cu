@@ -18,10 +18,11 @@
 // per pass, in registers.  Lane (g, t) takes word row 4s + t of outputs g and g + 8 of a 32-column slice s:
 // 8 columns of each, A fragments of two K = 16 steps if step j's K positions are columns 8t + 4j .. + 3;
 // the lane's activations of the slice are then 16 contiguous bytes.  Nibbles and activations are read
-// straight from global memory (L2 / L1), up to four slices ahead, and nothing is staged.  Staging 32 KB of
-// nibbles and up to 128 KB of activation rows per CTA whatever the problem's size let one CTA fill an SM:
-// 64 segments of 5 rows, 2048 -> 64 and 64 -> 1024, took 42 us a launch and now take 12; gate and up
-// share a launch.
+// straight from global memory (L2 / L1) and nothing is staged; four CTAs on an SM hide the latency
+// better than loads four slices ahead in 125 registers (a whole block with null-space pairs, 37 tokens:
+// 128 against 148 us).  Staging 32 KB of nibbles and up to 128 KB of activation rows per CTA whatever the
+// problem's size let one CTA fill an SM: 64 segments of 5 rows, 2048 -> 64 and 64 -> 1024, took 42 us a
+// launch.  Gate and up share a launch.
 // The eight warps of a CTA split the columns as far as there are slices and take further groups of 16 outputs
 // otherwise; partial sums meet in shared memory.  What bounds it: latency of a handful of dependent
 // round trips; launches.
@@ -67,9 +68,8 @@ __device__ __forceinline__ uint32_t p4_dequant_pair(uint32_t word, int i, __half
 // kSilu: both problems belong to one CTA, the second one (up) first, and problem 0's output becomes
 // silu(gate) * up, each rounded to fp16 where separate operators would round it.
 template <int NT, bool kSilu>
-__global__ void __launch_bounds__(kP4Threads) packed4_gemm_kernel(const __grid_constant__ P4Args a) {
+__global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kernel(const __grid_constant__ P4Args a) {
   constexpr int kRows = 8 * NT;
-  constexpr int kAhead = NT <= 2 ? 4 : (NT == 4 ? 2 : 1);  // slices whose loads are in flight together
   extern __shared__ __align__(16) float red[];              // [warp][activation row][kP4RedStride]
 
   pdl_wait();  // activations (and a device-built route) come from the kernels before this one
@@ -124,52 +124,44 @@ __global__ void __launch_bounds__(kP4Threads) packed4_gemm_kernel(const __grid_c
     int grp = -1;
     __half2 zca = {}, zcb = {}, sca = {}, scb = {};
 #pragma unroll 1
-    for (int s = s_begin; s < s_end; s += kAhead) {
-      uint32_t wa[kAhead], wb[kAhead];
-      uint4 xv[kAhead][NT];
+    for (int s = s_begin; s < s_end; ++s) {
+      const int kw = 4 * s + t, k = 8 * kw;
+      const bool in = kw < kwords;
+      const uint32_t wa = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + na)) : 0u;
+      const uint32_t wb = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + nb)) : 0u;
+      uint4 xv[NT];
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int kw = 4 * (s + u) + t, k = 8 * kw;
-        const bool in = s + u < s_end && kw < kwords;
-        wa[u] = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + na)) : 0u;
-        wb[u] = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + nb)) : 0u;
+      for (int i = 0; i < NT; ++i) {
+        const __half* src = xr[i] + kP4SliceCols * s;
+        xv[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (in) {
+          if (pr.x_aligned && k + 8 <= K) {
+            xv[i] = *reinterpret_cast<const uint4*>(src);
+          } else {  // ragged end or unaligned rows; columns past K read as zeros
+            uint32_t h[8];
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          const __half* src = xr[i] + kP4SliceCols * (s + u);
-          xv[u][i] = make_uint4(0u, 0u, 0u, 0u);
-          if (in) {
-            if (pr.x_aligned && k + 8 <= K) {
-              xv[u][i] = *reinterpret_cast<const uint4*>(src);
-            } else {  // ragged end or unaligned rows; columns past K read as zeros
-              uint32_t h[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) h[j] = k + j < K ? __half_as_ushort(src[j]) : 0u;
-              xv[u][i] = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
-            }
+            for (int j = 0; j < 8; ++j) h[j] = k + j < K ? __half_as_ushort(src[j]) : 0u;
+            xv[i] = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
           }
         }
       }
+      const int gi = min(s * kP4SliceCols / gs, G - 1);
+      if (gi != grp) {
+        grp = gi;
+        const int32_t* z = qz + static_cast<size_t>(gi) * w.z_ld;
+        const uint32_t za = (static_cast<uint32_t>(__ldg(z + (na >> 3))) >> (4 * (na & 7))) & 0xFu;
+        const uint32_t zb = (static_cast<uint32_t>(__ldg(z + (nb >> 3))) >> (4 * (nb & 7))) & 0xFu;
+        zca = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + za + 1u)));
+        zcb = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + zb + 1u)));
+        sca = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + na));
+        scb = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + nb));
+      }
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        if (s + u >= s_end) break;
-        const int gi = min((s + u) * kP4SliceCols / gs, G - 1);
-        if (gi != grp) {
-          grp = gi;
-          const int32_t* z = qz + static_cast<size_t>(gi) * w.z_ld;
-          const uint32_t za = (static_cast<uint32_t>(__ldg(z + (na >> 3))) >> (4 * (na & 7))) & 0xFu;
-          const uint32_t zb = (static_cast<uint32_t>(__ldg(z + (nb >> 3))) >> (4 * (nb & 7))) & 0xFu;
-          zca = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + za + 1u)));
-          zcb = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + zb + 1u)));
-          sca = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + na));
-          scb = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + nb));
-        }
+      for (int j = 0; j < 2; ++j) {
+        const uint32_t a0 = p4_dequant_pair(wa, 2 * j, zca, sca), a1 = p4_dequant_pair(wb, 2 * j, zcb, scb);
+        const uint32_t a2 = p4_dequant_pair(wa, 2 * j + 1, zca, sca), a3 = p4_dequant_pair(wb, 2 * j + 1, zcb, scb);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t a0 = p4_dequant_pair(wa[u], 2 * j, zca, sca), a1 = p4_dequant_pair(wb[u], 2 * j, zcb, scb);
-          const uint32_t a2 = p4_dequant_pair(wa[u], 2 * j + 1, zca, sca), a3 = p4_dequant_pair(wb[u], 2 * j + 1, zcb, scb);
-#pragma unroll
-          for (int i = 0; i < NT; ++i) mma_m16n8k16(acc[i], a0, a1, a2, a3, j ? xv[u][i].z : xv[u][i].x, j ? xv[u][i].w : xv[u][i].y);
-        }
+        for (int i = 0; i < NT; ++i) mma_m16n8k16(acc[i], a0, a1, a2, a3, j ? xv[i].z : xv[i].x, j ? xv[i].w : xv[i].y);
       }
     }
     // add the partial sums of the warps that share 16 outputs
