@@ -93,16 +93,16 @@ typedef struct TrisProjView {
      expert_slot[e]: the layout tris_page_experts fills from pinned host memory. */
   const int32_t* expert_slot;
   /* Tile-major records built at load time by tris_tile_records_plan / _build (NULL when absent):
-     per (expert, 64 outputs, 256 columns) one contiguous piece holding everything a CTA needs
-     of that tile, so that it arrives with a single bulk copy, plus per (expert, 256 columns)
-     a record of finished column-scale tables.  When present, the grouped entry points and the
-     two dump entry points read the records instead of the tensors above. */
+     per (expert, 128 outputs, 128 columns) one piece with the grouping bits decoded, 2 bits per
+     weight in the order the unpack consumes them, plus per (expert, 128 columns) a record of
+     finished column-scale tables.  When present, the grouped entry points and the two dump entry
+     points read the records instead of the tensors above. */
   const void* tile_records;
-  const uint32_t* tile_desc;             /* [records + 1][2]: {offset / 16, bytes}                */
+  const uint32_t* tile_desc;             /* [records + 1][2]: {offset / 16, bytes}; the kernels do not need it */
   const void* col_records;               /* [E, chunks] x col_record_bytes                        */
   int32_t col_record_bytes;
-  int32_t max_record_bytes;              /* largest tile record of this projection                */
-  int32_t max_sal_words;                 /* salient words per column record                       */
+  int32_t max_record_bytes;              /* size of a tile record: all of a projection are alike  */
+  int32_t max_sal_words;                 /* salient steps (of 16 columns) a record has room for   */
   int32_t reserved0;
 } TrisProjView;
 
@@ -139,10 +139,10 @@ typedef struct TrisRouteView {
    of 32 columns, column j sits at position 2*(j%16) + j/16 (what tris_shared_hidden_forward
    writes with out_mode = TRIS_OUT_F16_PAIR_INTERLEAVED).  Needs rank % 32 == 0. */
 #define TRIS_ROUTE_HIDDEN_PAIR_INTERLEAVED 1
-/* Activation rows in "lane order", the order the tile-record kernels consume: inside every group
-   of 32 columns, column j sits at 8*(j%4) + 2*s + j/16 with s = 1, 3, 0, 2 for (j/4)%4 = 0..3
-   (what tris_shared_hidden_forward writes with out_mode = TRIS_OUT_F16_LANE_ORDER).  Needs
-   rank % 32 == 0 and a projection with tile records. */
+/* Activation rows in "lane order": inside every group of 32 columns, column j sits at
+   8*(j%4) + 2*s + j/16 with s = 1, 3, 0, 2 for (j/4)%4 = 0..3 (what tris_shared_hidden_forward
+   writes with out_mode = TRIS_OUT_F16_LANE_ORDER).  Needs rank % 32 == 0 and a projection with tile
+   records. */
 #define TRIS_ROUTE_HIDDEN_LANE_ORDER 2
 
 #define TRIS_OUT_F16 0
@@ -453,9 +453,9 @@ int tris_grouped_pair_forward(const TrisProjView* proj_a, const TrisProjView* pr
 /*
  * The activation layout (TRIS_OUT_F16, TRIS_OUT_F16_PAIR_INTERLEAVED or TRIS_OUT_F16_LANE_ORDER) the
  * grouped entry points read fastest for these projections (proj_b may be NULL) and a route of
- * num_rows rows in num_segments segments of at most max_rows_per_segment rows: lane order for
- * projections with tile records in the decode regime, pair-interleaved otherwise, row-major for
- * ranks that are not a multiple of 32.  Ask the backbone GEMM for that out_mode and set the
+ * num_rows rows in num_segments segments of at most max_rows_per_segment rows: row-major for
+ * projections with tile records and ranks that are not a multiple of 32, pair-interleaved
+ * otherwise.  Ask the backbone GEMM for that out_mode and set the
  * matching TRIS_ROUTE_HIDDEN_* flag.  No reference counterpart (the reference kernels read
  * row-major activations only).
  */
@@ -479,8 +479,8 @@ int tris_combine_routed(const void* down_out_f16, const int32_t* row_of_flat,
                         int32_t hidden_size, void* final_f16, void* stream);
 
 /*
- * Rows per expert segment (the launch's upper estimate) above which the grouped entry points use
- * their tcgen05/TMEM kernel instead of the register kernel; returns the previous value.  The
+ * Rows per expert segment (the launch's upper estimate) above which projections without tile
+ * records use their tcgen05/TMEM kernel instead of the register kernel; returns the previous value.  The
  * default (2048) lies above the range in which the register kernel measured faster on B200; the
  * tests lower it to exercise the tensor-core kernel.  Process-wide; no reference counterpart
  * (the reference decides per call in run_grouped_structured_expert_forward, QL:2187-2229).
@@ -488,9 +488,9 @@ int tris_combine_routed(const void* down_out_f16, const int32_t* row_of_flat,
 int tris_set_grouped_tc_min_rows(int32_t rows);
 
 /*
- * Upper limit on how many CTAs share the row passes of one (segment, output tile) unit in the
- * register-cached grouped kernel (segments of more than 64 rows); returns the previous value.  The
- * launcher splits only while there are fewer units than two CTAs per SM - few local experts with long
+ * Upper limit on how many CTAs share the row passes of one unit (segment, two output tiles) in the
+ * tiled kernel (typical segments of more than 32 rows); returns the previous value.  The
+ * launcher splits only while there are fewer units than SMs - few local experts with long
  * segments, as on an expert-parallel rank.  Default 4; 1 switches the split off.  Results do not depend
  * on it.  Process-wide; no reference counterpart.
  */

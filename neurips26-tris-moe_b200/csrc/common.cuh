@@ -200,9 +200,6 @@ __device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src, boo
 __device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_4(void* dst_smem, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -266,16 +263,6 @@ __device__ __forceinline__ uint32_t global_timer_lo() {
   uint32_t t;
   asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
   return t;
-}
-// The same in few instructions and registers (~1 s as well).
-__device__ __forceinline__ bool mbar_wait_lean(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t t0 = global_timer_lo();
-#pragma unroll 1
-  do {
-    if (mbar_try_wait(bar, parity)) return true;
-  } while (global_timer_lo() - t0 < 1000000000u);
-  return false;
 }
 // The same by a whole warp, with one answer for all lanes (collective instructions may follow).
 // kSleepNs > 0: naps between polls, for a role that waits long and must not take issue slots from the

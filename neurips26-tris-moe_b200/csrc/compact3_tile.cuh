@@ -718,12 +718,6 @@ __device__ __forceinline__ void unpack_fragments(const TileSmem<NPROJ, NT>& sm, 
   unpack_row(s1b, seb, rs[1], ct, any_salient, t, a[1]);
 }
 
-// B fragments of packed row p, local activation row `n`: 8 halves in pair order.
-template <int NPROJ, int NT>
-__device__ __forceinline__ uint4 load_b_fragments(const TileSmem<NPROJ, NT>& sm, int proj, int n, int p, int t) {
-  return *reinterpret_cast<const uint4*>(sm.hrows + (proj * NT * 8 + n) * kHiddenRowBytes + p * 64 + t * 16);
-}
-
 // ---- launch arguments shared by the grouped kernels ---------------------------------------
 struct GroupedArgs {
   TrisProjView proj[2];

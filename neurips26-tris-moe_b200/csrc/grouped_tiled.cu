@@ -701,7 +701,7 @@ static int row_split(long long units, int max_rows, int n) {
 // Column split of one ordinary matrix (no experts): its units of two output tiles and its row passes together are
 // too few for the SMs, and its columns many - parts of the columns go to CTAs of their own, whose fp32 sums
 // sum_parts_kernel adds in order.  4096 columns, 512 rows: 64 units for 4096 outputs (two parts), 32 for a pair of
-// 1024 (four): 92 -> SPLIT_Q and 88 -> SPLIT_KV us.  At least two chunks per part: the sums cost 128 KB of
+// 1024 (four): 108 -> 48 and 92 -> 35 us.  At least two chunks per part: the sums cost 128 KB of
 // traffic a part.
 static int col_split(const TiledArgs& args, int mode, long long units) {
   if (args.expert_ids || !args.partial || units <= 0) return 1;

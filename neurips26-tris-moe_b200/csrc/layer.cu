@@ -177,7 +177,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
   // Launch order.  With logits given, router + route run first, so that the grouped
   // gate/up kernel can stage its weights while the backbone GEMM is still running
   // (programmatic dependent launch); otherwise the logits come out of the backbone GEMM.
-  // Activation layout between the backbone GEMMs and the grouped kernels: lane order for the
+  // Activation layout between the backbone GEMMs and the grouped kernels: row-major for the
   // tile-record kernels, pair-interleaved for the plane-staging kernels, row-major for odd ranks.
   TrisRouteView route{};
   route.num_segments = std::min(layer->num_experts, R);
