@@ -48,7 +48,7 @@ FALLBACK_HBM_GBS = 6650.0
 LAUNCHES_PER_LAYER = 7  # backbone+router GEMM, top-k, route, gate/up, down backbone, down, combine
 
 
-KERNEL_SOURCES = ("grouped_tiled.cu", "tile_records.cuh", "tile_records.cu")  # what the dominant kernel is built from
+KERNEL_SOURCES = ("grouped_decode.cu", "grouped_tiled.cuh", "tile_records.cuh", "tile_records.cu")  # what the dominant kernel is built from
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "grouped_tiled_traffic.json")
 
 
@@ -219,13 +219,12 @@ def run_ours(args):
         route = tm.build_grouped_route(sel, 64)
         routes.append(route)
         tok = route["grouped_token_indices"]
-        # what the layer path feeds the grouped kernels: backbone outputs in lane order, read through the route's gather
-        hg = tm.compute_shared_hidden(x, blk.shared_gate, layout=tm.HIDDEN_LANE_ORDER)
-        hu = tm.compute_shared_hidden(x, blk.shared_up, layout=tm.HIDDEN_LANE_ORDER)
+        # what the layer path feeds the grouped kernels: row-major backbone outputs, read through the route's gather
+        hg = tm.compute_shared_hidden(x, blk.shared_gate)
+        hu = tm.compute_shared_hidden(x, blk.shared_up)
         hd = torch.randn((tok.numel(), 256), device=device).half()
         hid.append((hg, hu, hd))
-        route["_gather_route"] = dict(route, _row_gather=tok.to(torch.int32), _hidden_layout=tm.HIDDEN_LANE_ORDER)
-        route["_lane_route"] = dict(route, _hidden_layout=tm.HIDDEN_LANE_ORDER)
+        route["_gather_route"] = dict(route, _row_gather=tok.to(torch.int32))
         active = route["expert_ids"].tolist()
         per_proj, _ = layer_algorithmic_bytes(info, active, T)
         byts["pair"] += per_proj["gate"] + per_proj["up"]
@@ -238,7 +237,7 @@ def run_ours(args):
 
     def down_step():
         for blk, route, (hg, hu, hd) in zip(blocks, routes, hid):
-            tm.run_grouped_structured_expert_forward(blk._get_grouped_payload("down"), hd, None, route["_lane_route"])
+            tm.run_grouped_structured_expert_forward(blk._get_grouped_payload("down"), hd, None, route)
 
     for name, fn in (("pair", pair_step), ("down", down_step)):
         graph = capture(fn)
@@ -248,7 +247,7 @@ def run_ours(args):
         del graph
     dom = max(kern, key=lambda n: kern[n]["us_per_launch"])
     roofline = {
-        "bound": "hbm", "kernel": f"grouped_tiled_kernel ({'gate/up dual + SiLU*mul' if dom == 'pair' else 'down'})",
+        "bound": "hbm", "kernel": f"grouped_decode_kernel ({'gate/up dual + SiLU*mul' if dom == 'pair' else 'down'})",
         "achieved": round(kern[dom]["gbs"], 1), "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
         "frac": round(kern[dom]["gbs"] / peak, 4), "frac_of_nominal_8TBs": round(kern[dom]["gbs"] / NOMINAL_HBM_GBS, 4),
         # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this kernel on this workload, from the
