@@ -324,53 +324,61 @@ class TrisSparseMoeBlock(nn.Module):
         y = torch.empty_like(x)
         if T == 0:
             return y.reshape(shape), x.new_zeros((0, E), dtype=torch.float32)
-        stream = lambda: torch.cuda.current_stream(dev).cuda_stream
-        f16 = torch.float16
+        r_gu, r_d = self.backbone_rank("gate"), self.backbone_rank("down")
+        mode_gu, mode_d = (2 if r_gu % 32 == 0 else 0), (2 if r_d % 32 == 0 else 0)
+        plain = lambda name: name not in self.packed_backbones and name not in self.input_scales
         with torch.cuda.device(dev):
-            if router_logits is None:
-                logits = torch.empty((T, E), dtype=torch.float32, device=dev)
-                _native.check(lib.tris_shared_hidden_forward(x.data_ptr(), None, T, None, H, self.gate.weight.data_ptr(), E,
-                                                             logits.data_ptr(), 1, stream()), "router")
-            else:
+            stream = torch.cuda.current_stream(dev).cuda_stream
+            # one allocation for everything between the kernels; the host has 25 launches a layer to prepare
+            sizes = [4 * R] * 6 + [4 * E, 4 * (E + 1), 4 * (E + 1), 16, 2 * T * r_gu, 2 * T * r_gu, 2 * R * I, 2 * R * r_d, 2 * R * H]
+            offsets, total = [], 0
+            for n in sizes:
+                offsets.append(total)
+                total += (n + 255) & ~255
+            ws = torch.empty((total,), dtype=torch.uint8, device=dev)
+            base = ws.data_ptr()
+            sel, wts, perm, tok, slot, rof, ids, seg, prob, counts, hg, hu, mlp_ptr, hd, down = (base + o for o in offsets)
+            projected = router_logits is None and plain("gate") and plain("up") and self.backbone_rank("up") == r_gu
+            if router_logits is not None:
                 logits = router_logits.reshape(T, E).to(torch.float32).contiguous()
-            sel = torch.empty((T, k), dtype=torch.int32, device=dev)
-            wts = torch.empty((T, k), dtype=torch.float32, device=dev)
-            _native.check(lib.tris_router_topk(logits.data_ptr(), T, E, k, int(self.norm_topk_prob), sel.data_ptr(),
-                                               wts.data_ptr(), stream()), "router_topk")
-            buf = torch.empty((4 * R + 3 * E + 6,), dtype=torch.int32, device=dev)
-            perm, tok, slot, rof = (buf[i * R:(i + 1) * R] for i in range(4))
-            ids, seg = buf[4 * R: 4 * R + E], buf[4 * R + E: 4 * R + 2 * E + 1]
-            prob, counts = buf[4 * R + 2 * E + 1: 4 * R + 3 * E + 2], buf[4 * R + 3 * E + 2: 4 * R + 3 * E + 6]
-            _native.check(lib.tris_build_grouped_route(sel.data_ptr(), T, k, E, 4, perm.data_ptr(), tok.data_ptr(),
-                                                       slot.data_ptr(), rof.data_ptr(), ids.data_ptr(), seg.data_ptr(),
-                                                       prob.data_ptr(), counts.data_ptr(), stream()), "route")
-            route = {"expert_ids": ids, "segment_offsets": seg, "counts": counts, "experts": E, "rows": R}
-            paged = manager.page_layer(block_index, route)  # side stream, starts now
-
-            r_gu, r_d = self.backbone_rank("gate"), self.backbone_rank("down")
-            mode_gu, mode_d = (2 if r_gu % 32 == 0 else 0), (2 if r_d % 32 == 0 else 0)
-            hg = self.backbone_hidden("gate", x, mode_gu)
-            hu = self.backbone_hidden("up", x, mode_gu)
+            else:
+                logits = torch.empty((T, E), dtype=torch.float32, device=dev)
+                if projected:  # router and both input-side backbones in one launch
+                    _native.check(lib.tris_input_projections(x.data_ptr(), T, H, self.shared_gate.data_ptr(), self.shared_up.data_ptr(), r_gu,
+                                                             self.gate.weight.data_ptr(), E, hg, hu, mode_gu, logits.data_ptr(), stream),
+                                  "input_projections")
+                else:
+                    _native.check(lib.tris_shared_hidden_forward(x.data_ptr(), None, T, None, H, self.gate.weight.data_ptr(), E,
+                                                                 logits.data_ptr(), 1, stream), "router")
+            _native.check(lib.tris_router_topk(logits.data_ptr(), T, E, k, int(self.norm_topk_prob), sel, wts, stream), "router_topk")
+            _native.check(lib.tris_build_grouped_route(sel, T, k, E, 4, perm, tok, slot, rof, ids, seg, prob, counts, stream), "route")
+            paged = manager.page_layer(block_index, {"expert_ids": ids, "segment_offsets": seg, "counts": counts, "experts": E,
+                                                     "rows": R})  # side stream, starts now
+            keep = []
+            if not projected:
+                keep = [self.backbone_hidden("gate", x, mode_gu), self.backbone_hidden("up", x, mode_gu)]
+                hg, hu = keep[0].data_ptr(), keep[1].data_ptr()
             rv = _native.TrisRouteView()
-            rv.expert_ids, rv.segment_offsets, rv.num_segments_dev = ids.data_ptr(), seg.data_ptr(), counts.data_ptr()
+            rv.expert_ids, rv.segment_offsets, rv.num_segments_dev = ids, seg, counts
             rv.num_segments, rv.num_rows, rv.max_rows_per_segment = min(E, R), R, T
             if self._status_word is None or self._status_word.device != dev:
                 self._status_word = torch.zeros((1,), dtype=torch.int32, device=dev)
-            rv.row_gather, rv.status_dev, rv.flags = tok.data_ptr(), self._status_word.data_ptr(), (1 if mode_gu else 0)
+            rv.row_gather, rv.status_dev, rv.flags = tok, self._status_word.data_ptr(), (1 if mode_gu else 0)
             paged.wait("gate_up")  # down keeps paging under the gate/up kernel and the down backbone
-            mlp = torch.empty((R, I), dtype=f16, device=dev)
-            _native.check(lib.tris_grouped_pair_forward(C.byref(paged.views["gate"]), C.byref(paged.views["up"]), C.byref(rv),
-                                                        hg.data_ptr(), hu.data_ptr(), mlp.data_ptr(), None, 1, stream()),
-                          "grouped_pair_forward")
-            hd = self.backbone_hidden("down", mlp, mode_d)
+            _native.check(lib.tris_grouped_pair_forward(C.byref(paged.views["gate"]), C.byref(paged.views["up"]), C.byref(rv), hg, hu, mlp_ptr,
+                                                        None, 1, stream), "grouped_pair_forward")
+            if plain("down"):
+                _native.check(lib.tris_shared_hidden_forward(mlp_ptr, None, R, None, I, self.shared_down.data_ptr(), r_d, hd, mode_d, stream),
+                              "down backbone")
+            else:
+                mlp = ws[offsets[12]: offsets[12] + 2 * R * I].view(torch.float16).view(R, I)
+                keep.append(self.backbone_hidden("down", mlp, mode_d))
+                hd = keep[-1].data_ptr()
             rv.row_gather, rv.flags = None, (1 if mode_d else 0)
             paged.wait("all")
-            down = torch.empty((R, H), dtype=f16, device=dev)
-            _native.check(lib.tris_grouped_forward(C.byref(paged.views["down"]), C.byref(rv), hd.data_ptr(), down.data_ptr(),
-                                                   stream()), "grouped_forward")
+            _native.check(lib.tris_grouped_forward(C.byref(paged.views["down"]), C.byref(rv), hd, down, stream), "grouped_forward")
             paged.release()
-            _native.check(lib.tris_combine_routed(down.data_ptr(), rof.data_ptr(), wts.data_ptr(), T, k, H, y.data_ptr(),
-                                                  stream()), "combine")
+            _native.check(lib.tris_combine_routed(down, rof, wts, T, k, H, y.data_ptr(), stream), "combine")
         return y.reshape(shape), logits
 
     def forward_grouped_ops(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None):

@@ -99,6 +99,7 @@ class GroupedQGmapCPUStagingManager:
                                    # paged while the gate/up kernel is still reading the table of gate and up
         self._paged = []           # per ring slot: event "pager done" (all three projections)
         self._paged_gu = []        # per ring slot: event "gate and up paged" (down may still be in flight)
+        self._plans = {}           # (layer, ring slot) -> pager jobs and staged views: host and slot addresses are fixed
         self._consumed = []        # per ring slot: event "compute done with this slot"
         self._used = []
         self._copy_stream = None
@@ -191,36 +192,23 @@ class GroupedQGmapCPUStagingManager:
             copy.wait_event(self._consumed[ring])
             self.pipeline_stats["slot_reuses"] += 1
         nseg_bound = min(int(route["experts"]), int(route["rows"]), self.capacity)
-        tables = self.slot_tables[ring]
         timed = self.collect_timings
         start = end = None
         if timed:
             start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        views = {}
+        launches, views = self._plan(block_index, ring)
+        ids, counts, experts = route["expert_ids"], route["counts"], int(route["experts"])
+        ids, counts = (v if isinstance(v, int) else v.data_ptr() for v in (ids, counts))  # tensors or device addresses
         with torch.cuda.stream(copy):
             if timed:
                 start.record(copy)
             # gate and up go in one launch (they are needed together and share a slot table), down in a second one
             # that runs while the gate/up kernel computes
-            for group in (("gate", "up"), ("down",)):
-                pairs = [(proj, key) for proj in group for key in self.entries[(block_index, proj)].host]
-                table = tables[group[0]]
-                for lo in range(0, len(pairs), MAX_PAGE_JOBS):
-                    part = pairs[lo: lo + MAX_PAGE_JOBS]
-                    jobs = (TrisPageJob * len(part))()
-                    for j, (proj, key) in enumerate(part):
-                        entry = self.entries[(block_index, proj)]
-                        jobs[j].host_src = entry.host[key].data_ptr()
-                        jobs[j].dst = self.buffers[(ring, proj, key)].data_ptr()
-                        jobs[j].bytes_per_expert = entry.block_bytes[key]
-                        self.pipeline_stats["bytes"] += nseg_bound * entry.block_bytes[key]
-                    _native.check(lib.tris_page_experts(jobs, len(part), route["expert_ids"].data_ptr(),
-                                                        route["counts"].data_ptr(), nseg_bound, int(route["experts"]),
-                                                        table.data_ptr(), copy.cuda_stream), "page_experts")
-                    self.pipeline_stats["chunks"] += 1
-                for proj in group:
-                    views[proj] = self._staged_view(self.entries[(block_index, proj)], ring, proj, table)
-                if group[0] == "gate":  # the gate/up kernel may start while down is still paged
+            for jobs, count, per_segment, last_of_gate_up, table in launches:
+                self.pipeline_stats["bytes"] += nseg_bound * per_segment
+                _native.check(lib.tris_page_experts(jobs, count, ids, counts, nseg_bound, experts, table, copy.cuda_stream), "page_experts")
+                self.pipeline_stats["chunks"] += 1
+                if last_of_gate_up:  # the gate/up kernel may start while down is still paged
                     self._paged_gu[ring].record(copy)
             if timed:
                 end.record(copy)
@@ -228,6 +216,32 @@ class GroupedQGmapCPUStagingManager:
         self.pipeline_stats["calls"] += 1
         self._used[ring] = True
         return _PagedLayer(self, ring, views, start, end)
+
+    def _plan(self, block_index: int, ring: int):
+        """Pager launches ``(jobs, count, bytes per segment, ends gate/up, slot table)`` and staged views of a
+        layer in a ring slot, laid out on first use and again when a projection's own view was rebuilt."""
+        bases = tuple(id(proj_view(self.entries[(block_index, proj)].payload)) for proj in PROJECTIONS)
+        plan = self._plans.get((block_index, ring))
+        if plan is not None and plan[0] == bases:
+            return plan[1], plan[2]
+        launches, views = [], {}
+        for group in (("gate", "up"), ("down",)):
+            pairs = [(proj, key) for proj in group for key in self.entries[(block_index, proj)].host]
+            table = self.slot_tables[ring][group[0]]
+            for lo in range(0, len(pairs), MAX_PAGE_JOBS):
+                part = pairs[lo: lo + MAX_PAGE_JOBS]
+                jobs = (TrisPageJob * len(part))()
+                for j, (proj, key) in enumerate(part):
+                    entry = self.entries[(block_index, proj)]
+                    jobs[j].host_src = entry.host[key].data_ptr()
+                    jobs[j].dst = self.buffers[(ring, proj, key)].data_ptr()
+                    jobs[j].bytes_per_expert = entry.block_bytes[key]
+                per_segment = sum(self.entries[(block_index, proj)].block_bytes[key] for proj, key in part)
+                launches.append((jobs, len(part), per_segment, group[0] == "gate" and lo + MAX_PAGE_JOBS >= len(pairs), table.data_ptr()))
+            for proj in group:
+                views[proj] = self._staged_view(self.entries[(block_index, proj)], ring, proj, table)
+        self._plans[(block_index, ring)] = (bases, launches, views)
+        return launches, views
 
     def _staged_view(self, entry: _Entry, ring: int, proj: str, table: torch.Tensor):
         """Copy of the projection's ctypes view whose paged tensors point at the staging slots."""
