@@ -57,6 +57,7 @@ class TrisSparseMoeBlock(nn.Module):
         self._layer_view: Optional[TrisMoeLayerView] = None
         self._expanded_view: Optional[dict] = None  # expanded backbone names -> layer view
         self._workspace: Optional[torch.Tensor] = None
+        self._workspace_for = None
         self._status_word: Optional[torch.Tensor] = None  # status of the kernels forward_streaming launches
 
     # -- loading ---------------------------------------------------------------------------
@@ -213,11 +214,16 @@ class TrisSparseMoeBlock(nn.Module):
         return ex
 
     def workspace(self, num_tokens: int, device, extras: Optional[TrisMoeLayerExtras] = None) -> torch.Tensor:
+        view = self.layer_view()
+        sized = self._workspace_for  # (view, tokens) the buffer is known to hold: the size grows with the tokens
+        if (extras is None and sized is not None and sized[0] is view and num_tokens <= sized[1] and self._workspace is not None
+                and self._workspace.device == device):
+            return self._workspace
         lib = _native.load()
         if extras is None:
-            need = int(lib.tris_moe_layer_workspace_bytes(C.byref(self.layer_view()), int(num_tokens)))
+            need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), int(num_tokens)))
         else:
-            need = int(lib.tris_moe_layer_extras_workspace_bytes(C.byref(self.layer_view()), C.byref(extras), int(num_tokens)))
+            need = int(lib.tris_moe_layer_extras_workspace_bytes(C.byref(view), C.byref(extras), int(num_tokens)))
         if need == 0 and num_tokens > 0:
             raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
         if self._workspace is None or self._workspace.numel() < need or self._workspace.device != device:
@@ -225,6 +231,7 @@ class TrisSparseMoeBlock(nn.Module):
                 self.raise_on_kernel_status()  # do not lose a report with the old buffer
             self._workspace = torch.empty((need,), dtype=torch.uint8, device=device)
             self._workspace[:16].zero_()  # count words and the sticky status word
+        self._workspace_for = (view, int(num_tokens)) if extras is None else None
         return self._workspace
 
     def last_kernel_status(self, clear: bool = True) -> int:
@@ -288,7 +295,7 @@ class TrisSparseMoeBlock(nn.Module):
             logits_in, logits_out = None, logits.data_ptr()
         if T:
             ws = self.workspace(T, dev, extras)
-            view = self.layer_view()
+            view = self._layer_view  # which workspace() has just brought up to date
             if self.packed_backbones:  # gate and up see T rows, down T * top_k
                 big = [n for n in self.packed_backbones
                        if (T * self.top_k if n == "down" else T) > self.PACKED_BACKBONE_MAX_ROWS]
