@@ -264,6 +264,12 @@ class TrisSparseMoeBlock(nn.Module):
                                "(TRIS_ERR_TIMEOUT: a bounded wait on a copy ran out; TRIS_ERR_WORKSPACE: a streamed batch activated "
                                "more experts than the staging manager has slots for; output rows of that launch are stale)")
 
+    def _require_rows(self, x: torch.Tensor, what: str) -> None:
+        """The kernels take addresses: rows of another type or width would be misread or read out of range."""
+        if x.dtype != torch.float16 or x.shape[-1] != self.hidden_size:
+            raise RuntimeError(f"trismoe_b200 {what}: float16 hidden states of width {self.hidden_size} required, "
+                               f"got {x.dtype} of width {x.shape[-1]}")
+
     # -- forward ---------------------------------------------------------------------------
     def forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None):
         """Returns ``(final_hidden_states [B, S, H], router_logits [T, E])`` like
@@ -322,7 +328,6 @@ class TrisSparseMoeBlock(nn.Module):
         pager for gate/up/down starts on the side stream and overlaps the input-side backbone
         GEMM; the grouped kernels wait on its event.  Nothing synchronises with the host."""
         _native.require_cuda(hidden_states, "TrisSparseMoeBlock.forward_streaming")
-        lib = _native.load()
         shape = hidden_states.shape
         x = hidden_states.reshape(-1, shape[-1]).contiguous()
         T, dev = int(x.shape[0]), x.device
@@ -331,6 +336,8 @@ class TrisSparseMoeBlock(nn.Module):
         y = torch.empty_like(x)
         if T == 0:
             return y.reshape(shape), x.new_zeros((0, E), dtype=torch.float32)
+        self._require_rows(x, "forward_streaming")
+        lib = _native.load()
         r_gu, r_d = self.backbone_rank("gate"), self.backbone_rank("down")
         mode_gu, mode_d = (2 if r_gu % 32 == 0 else 0), (2 if r_d % 32 == 0 else 0)
         plain = lambda name: name not in self.packed_backbones and name not in self.input_scales
