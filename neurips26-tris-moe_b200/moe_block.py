@@ -199,18 +199,27 @@ class TrisSparseMoeBlock(nn.Module):
         return v
 
     def _layer_extras(self, dev) -> Optional[TrisMoeLayerExtras]:
-        """Input scales and null-space pairs as the native layer takes them; None where the layer has none."""
-        if not (self.input_scales or self.ns_payloads):
-            return None
+        """Input scales and null-space pairs as the native layer takes them; None where it cannot: a router wider
+        than its own, or scales and pairs of other sizes than the layer's, which the separate operators
+        broadcast, skip or refuse."""
         from .ns_compensation import prepare_ns_payload
 
+        H, I, E = self.hidden_size, self.intermediate_size, self.num_experts
+        if E > 256 or self.top_k > 32:
+            return None
         ex = TrisMoeLayerExtras()
-        for i, name in enumerate(("gate", "up", "down")):
-            if name in self.input_scales:
-                ex.input_scale[i] = self.input_scales[name].data_ptr()
+        for i, (name, width, out) in enumerate((("gate", H, I), ("up", H, I), ("down", I, H))):
+            scale = self.input_scales.get(name)
+            if scale is not None:
+                if scale.numel() != width or scale.device != dev:
+                    return None
+                ex.input_scale[i] = scale.data_ptr()
             if name in self.ns_payloads:
                 p = prepare_ns_payload(self.ns_payloads[name], dev)
-                ex.ns_c2[i], ex.ns_c1[i] = C.addressof(p["_tris_c2_view"]), C.addressof(p["_tris_c1_view"])
+                c2, c1 = p["_tris_c2_view"], p["_tris_c1_view"]
+                if (c2.k, c1.n, c2.num_experts) != (width, out, E):
+                    return None
+                ex.ns_c2[i], ex.ns_c1[i] = C.addressof(c2), C.addressof(c1)
         return ex
 
     def workspace(self, num_tokens: int, device, extras: Optional[TrisMoeLayerExtras] = None) -> torch.Tensor:
@@ -276,9 +285,10 @@ class TrisSparseMoeBlock(nn.Module):
         ``OlmoeSparseMoeBlock.forward`` (modeling_olmoe.py:1046-1105).  ``router_logits``
         (fp32 ``[T, E]``) may be passed in to skip the router linear."""
         _native.require_cuda(hidden_states, "TrisSparseMoeBlock.forward")
-        wide_router = self.num_experts > 256 or self.top_k > 32  # more than the native router takes
-        if not envflags.grouped_experts_enabled() or (wide_router and (self.input_scales or self.ns_payloads)):
-            # TRIS_GROUPED_EXPERTS=0: operator by operator
+        with_extras = bool(self.input_scales or self.ns_payloads)
+        extras = self._layer_extras(hidden_states.device) if with_extras else None
+        if not envflags.grouped_experts_enabled() or (with_extras and extras is None):
+            # TRIS_GROUPED_EXPERTS=0, or scales and pairs that the native sequence does not take: operator by operator
             return self.forward_grouped_ops(hidden_states, router_logits)
         if hidden_states.dtype != torch.float16:
             raise RuntimeError(f"trismoe_b200: grouped expert kernels require float16 hidden states, got {hidden_states.dtype}")
@@ -288,7 +298,6 @@ class TrisSparseMoeBlock(nn.Module):
         T = int(x.shape[0])
         dev = x.device
         y = torch.empty_like(x)
-        extras = self._layer_extras(dev)
         returned = router_logits
         if extras is not None and router_logits is None:
             # such blocks route by fp16 logits and return them
@@ -300,6 +309,7 @@ class TrisSparseMoeBlock(nn.Module):
             logits = torch.empty((T, self.num_experts), dtype=torch.float32, device=dev)
             logits_in, logits_out = None, logits.data_ptr()
         if T:
+            self._require_rows(x, "forward")
             ws = self.workspace(T, dev, extras)
             view = self._layer_view  # which workspace() has just brought up to date
             if self.packed_backbones:  # gate and up see T rows, down T * top_k
