@@ -52,3 +52,45 @@ def test_null_space_pairs_of_another_size_go_operator_by_operator(block, monkeyp
 def test_forward_refuses_narrow_rows(block):
     with pytest.raises(RuntimeError, match="float16 hidden states of width 64 required"):
         block(torch.zeros((1, 3, 56), dtype=torch.float16), torch.zeros((3, 4)))
+
+
+@pytest.mark.parametrize("gate,kernel", [(torch.zeros((1, 64)).half(), True), (torch.zeros((1, 56)).half(), False), (torch.zeros((1, 64)), False),
+                                         (torch.zeros((1, 64), dtype=torch.float16, device="meta"), False)])
+def test_shared_expert_gate_of_another_size_or_place(monkeypatch, gate, kernel):
+    """The routed and shared outputs are replaced by tensors on the CPU: a gate that the kernel cannot take must reach
+    torch's linear and its checks; one that it can take reaches the kernel (and fails for want of a GPU)."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import compact3_linear
+
+    blk = tm.TrisQwen2SparseMoeBlock(64, 32, 4, 2)
+    x = torch.zeros((1, 3, 64), dtype=torch.float16)
+    monkeypatch.setattr(tm.TrisSparseMoeBlock, "forward", lambda self, h, r=None: (torch.zeros_like(h), None))
+    monkeypatch.setattr(compact3_linear, "run_compact3_gate_up_forward", lambda *a, **k: x)
+    blk.shared_expert = (None, None, lambda m: torch.zeros_like(x))
+    blk.shared_expert_gate.weight = torch.nn.Parameter(gate, requires_grad=False)
+    linears = []
+    linear = torch.nn.functional.linear
+    monkeypatch.setattr(torch.nn.functional, "linear", lambda *a: linears.append(a) or linear(*a))
+    try:
+        blk(x)
+    except (RuntimeError, ValueError):
+        pass
+    assert len(linears) == (0 if kernel else 1)
+
+
+def test_shared_expert_gate_keeps_its_gradient(monkeypatch):
+    import trismoe_b200 as tm
+    from trismoe_b200 import compact3_linear
+
+    blk = tm.TrisQwen2SparseMoeBlock(64, 32, 4, 2)
+    g = torch.Generator().manual_seed(0)
+    x, shared = (torch.randn((1, 3, 64), generator=g).half() for _ in range(2))
+    monkeypatch.setattr(tm.TrisSparseMoeBlock, "forward", lambda self, h, r=None: (torch.zeros_like(h), None))
+    monkeypatch.setattr(compact3_linear, "run_compact3_gate_up_forward", lambda *a, **k: x)
+    blk.shared_expert = (None, None, lambda m: shared)
+    blk.shared_expert_gate.weight = torch.nn.Parameter(torch.randn((1, 64), generator=g).half())
+    y, _ = blk(x)
+    y.float().sum().backward()
+    z = torch.nn.functional.linear(x, blk.shared_expert_gate.weight.detach()).float()
+    want = (torch.sigmoid(z) * (1 - torch.sigmoid(z)) * shared.float().sum(-1, keepdim=True) * x.float()).sum((0, 1))
+    assert torch.allclose(blk.shared_expert_gate.weight.grad.float().view(-1), want, rtol=2e-2, atol=2e-2)
