@@ -7,7 +7,7 @@ qlinear_cuda.py:915-1022; dual gate/up of the shared expert, qlinear_cuda.py:102
 An ordinary linear is the grouped operator with one expert and one segment that holds every row,
 so it runs on the same tile-record kernels: ``y = x @ dequant(W).T`` with ``W`` the compact3
 matrix ``[out_features, in_features]`` (the columns are the layer's input features, several
-256-column chunks), optionally ``x`` scaled per input column and ``y`` per output row
+128-column chunks), optionally ``x`` scaled per input column and ``y`` per output row
 (``ns_mode == 1``: ``ns_vector_col`` / ``ns_vector_row``) and a bias.  Null-space matrices of rank
 > 0 are not supported.  There is no CPU path: tensors must live on a CUDA device.
 """
@@ -50,8 +50,9 @@ class Compact3Linear(nn.Module):
         self.out_features = out_features
         self.input_scale = None if ns_vector_col is None else ns_vector_col.reshape(self.in_features).to(dev, torch.float16).contiguous()
 
-    def _route(self, rows: int, device) -> dict:
-        if isinstance(self.payload.get("_tris_tile_records"), torch.Tensor):
+    def _route(self, rows: int, device, partner: Optional["Compact3Linear"] = None) -> dict:
+        """One segment with all rows, for this linear or a pair of them; without arrays where all have tile records."""
+        if all(isinstance(m.payload.get("_tris_tile_records"), torch.Tensor) for m in (self, partner) if m is not None):
             route = {"_one_segment": True, "_max_rows_per_segment": rows}
         else:
             zero = torch.zeros((1,), dtype=torch.int32, device=device)
@@ -89,7 +90,8 @@ def run_compact3_qkv_forward(q_proj: Compact3Linear, k_proj: Compact3Linear, v_p
     lead = hidden_states.shape[:-1]
     q = run_grouped_structured_expert_forward(q_proj.payload, x2, None, q_proj._route(rows, x2.device))
     if _same_shape(k_proj, v_proj):
-        k, v = run_grouped_structured_expert_pair_forward(k_proj.payload, v_proj.payload, x2, x2, None, k_proj._route(rows, x2.device))
+        k, v = run_grouped_structured_expert_pair_forward(k_proj.payload, v_proj.payload, x2, x2, None,
+                                                           k_proj._route(rows, x2.device, v_proj))
     else:
         k = run_grouped_structured_expert_forward(k_proj.payload, x2, None, k_proj._route(rows, x2.device))
         v = run_grouped_structured_expert_forward(v_proj.payload, x2, None, v_proj._route(rows, x2.device))
@@ -110,7 +112,7 @@ def run_compact3_gate_up_forward(gate_proj: Compact3Linear, up_proj: Compact3Lin
         return envflags.return_or_raise_none("run_compact3_gate_up_forward", "gate and up must share their shape and have no input scale")
     x2 = hidden_states.reshape(-1, gate_proj.in_features).contiguous()
     a, b = run_grouped_structured_expert_pair_forward(gate_proj.payload, up_proj.payload, x2, x2, None,
-                                                      gate_proj._route(int(x2.shape[0]), x2.device), fuse_silu_mul=fuse_silu_mul)
+                                                      gate_proj._route(int(x2.shape[0]), x2.device, up_proj), fuse_silu_mul=fuse_silu_mul)
     lead = hidden_states.shape[:-1]
     if a is None:
         return None

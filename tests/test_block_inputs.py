@@ -94,3 +94,26 @@ def test_shared_expert_gate_keeps_its_gradient(monkeypatch):
     z = torch.nn.functional.linear(x, blk.shared_expert_gate.weight.detach()).float()
     want = (torch.sigmoid(z) * (1 - torch.sigmoid(z)) * shared.float().sum(-1, keepdim=True) * x.float()).sum((0, 1))
     assert torch.allclose(blk.shared_expert_gate.weight.grad.float().view(-1), want, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("first,second,arrays", [(True, True, False), (True, False, True), (False, True, True), (False, False, True)])
+def test_pair_of_ordinary_linears_of_two_formats_gets_route_arrays(monkeypatch, first, second, arrays):
+    """Only the tile-record kernels take a route without arrays, and a pair runs on them only if both have records."""
+    from trismoe_b200 import compact3_linear as c3
+
+    def linear(records):
+        m = c3.Compact3Linear.__new__(c3.Compact3Linear)
+        torch.nn.Module.__init__(m)
+        m.payload = {"_tris_tile_records": torch.zeros(16, dtype=torch.uint8)} if records else {}
+        m.in_features, m.out_features, m.input_scale = 64, 32, None
+        return m
+
+    routes = []
+    monkeypatch.setattr(c3._native, "require_cuda", lambda tensor, what: None)
+    monkeypatch.setattr(c3, "run_grouped_structured_expert_forward", lambda p, x, _, route: x[:, :32])
+    monkeypatch.setattr(c3, "run_grouped_structured_expert_pair_forward",
+                        lambda a, b, x, y, _, route, **k: routes.append(route) or (x[:, :32], y[:, :32]))
+    x, a, b = torch.zeros((3, 64), dtype=torch.float16), linear(first), linear(second)
+    c3.run_compact3_qkv_forward(linear(True), a, b, x)
+    c3.run_compact3_gate_up_forward(a, b, x)
+    assert [("expert_ids" in r, r.get("_one_segment", False)) for r in routes] == [(arrays, not arrays)] * 2
