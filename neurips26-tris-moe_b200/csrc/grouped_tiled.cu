@@ -874,12 +874,17 @@ extern "C" int tris_set_grouped_row_split_max(int32_t ctas) {
   return tris::tr::g_row_split_max.exchange(ctas < 1 ? 1 : (ctas > 16 ? 16 : ctas), std::memory_order_relaxed);
 }
 
-// Bytes that let launch_grouped_tiled split the columns as far as it would: one part per SM-filling share.
+// Bytes that let launch_grouped_tiled split the columns as far as it would: one part per SM-filling share, within
+// 256 MB.  The sums grow with the rows while the gain does not (100 000 rows of a 1024-output pair would ask for 3 GB);
+// 4096 rows of a 4096 x 4096 matrix still get their two parts (134 MB).
+constexpr size_t kMostSplitBytes = size_t{256} << 20;
 size_t tris::grouped_split_bytes(const TrisProjView* proj, int projections, int num_rows) {
   using namespace tr;
   if (!proj_has_tile_records(*proj) || num_rows <= kDecodeMaxRows || num_chunks(proj->rank) < 4) return 0;
   const long long tiles = tiles_per_expert(proj->out_features), units = projections == 1 ? (tiles + 1) / 2 : tiles;
   const long long row_parts = std::max<long long>(1, std::min<long long>(sm_count() / units, (num_rows + 127) / 128));
-  const long long parts = std::min<long long>(num_chunks(proj->rank) / 2, sm_count() / (units * std::min<long long>(row_parts, g_row_split_max.load(std::memory_order_relaxed))));
-  return parts <= 1 ? 0 : sizeof(float) * static_cast<size_t>(parts) * projections * num_rows * proj->out_features;
+  const size_t part = sizeof(float) * static_cast<size_t>(projections) * num_rows * proj->out_features;
+  const long long parts = std::min<long long>({num_chunks(proj->rank) / 2, sm_count() / (units * std::min<long long>(row_parts, g_row_split_max.load(std::memory_order_relaxed))),
+                                               static_cast<long long>(kMostSplitBytes / part)});
+  return parts <= 1 ? 0 : part * static_cast<size_t>(parts);
 }

@@ -63,3 +63,24 @@ def test_cpu_tensors_are_rejected_loudly(lib):
         tm.compute_shared_hidden(torch.zeros(2, 8, dtype=torch.float16), torch.zeros(4, 8, dtype=torch.float16))
     with pytest.raises(RuntimeError, match="CUDA"):
         tm.build_grouped_route(torch.zeros(2, 2, dtype=torch.long), 4)
+
+
+def _record_view(out_features, rank):
+    """A projection with tile records as the host rules see it; the addresses are never followed."""
+    import trismoe_b200 as tm
+
+    v = tm._native.TrisProjView()
+    v.num_experts, v.out_features, v.rank, v.num_groups, v.use_block_gr = 1, out_features, rank, 1, 1
+    v.tile_records = v.col_records = 1 << 20
+    v.col_record_bytes, v.max_record_bytes, v.max_sal_words = 672, 4 * 1536, 1
+    return v
+
+
+def test_column_split_scratch_is_bounded(lib):
+    need = lambda o, rank, projections, rows: lib.tris_linear_workspace_bytes(C.byref(_record_view(o, rank)), projections, rows)
+    assert need(4096, 4096, 1, 512) == 2 * 4 * 512 * 4096 and need(1024, 4096, 2, 512) == 4 * 2 * 4 * 512 * 1024
+    assert need(4096, 4096, 1, 4096) == 2 * 4 * 4096 * 4096
+    for o, rank, projections in ((1024, 4096, 2), (256, 8192, 1), (72, 2048, 1), (4096, 4096, 1)):
+        for rows in (33, 1000, 16384, 100_000, 1 << 20, (1 << 31) - 1):
+            n = need(o, rank, projections, rows)
+            assert n <= 256 << 20 and n % (4 * projections * rows * o) == 0
