@@ -691,6 +691,7 @@ extern "C" size_t tris_linear_workspace_bytes(const TrisProjView* proj, int32_t 
 extern "C" int tris_linear_forward(const TrisProjView* proj_a, const TrisProjView* proj_b, const TrisRouteView* route, const void* hidden_a_f16,
                                    const void* hidden_b_f16, void* out_a_f16, void* out_b_f16, int32_t fuse_silu_mul, void* workspace,
                                    size_t workspace_bytes, void* stream) {
+  TRIS_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15u) == 0, TRIS_ERR_INVALID_ARG, "tris_linear_forward: the workspace must be 16-byte aligned");
   LaunchOpts opts;
   opts.pdl = programmatic_launch_default();
   opts.workspace = workspace;

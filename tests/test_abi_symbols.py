@@ -84,3 +84,15 @@ def test_column_split_scratch_is_bounded(lib):
         for rows in (33, 1000, 16384, 100_000, 1 << 20, (1 << 31) - 1):
             n = need(o, rank, projections, rows)
             assert n <= 256 << 20 and n % (4 * projections * rows * o) == 0
+
+
+def test_misaligned_workspace_of_an_ordinary_matrix_is_refused(lib):
+    """The sums of the column parts are read 16 bytes at a time.  Refused before any CUDA call, so no GPU is needed."""
+    import trismoe_b200 as tm
+
+    view, route = _record_view(256, 1024), tm._native.TrisRouteView()
+    route.num_segments, route.num_rows, route.max_rows_per_segment = 1, 64, 64
+    need = lib.tris_linear_workspace_bytes(C.byref(view), 1, 64)
+    assert need > 0
+    st = lib.tris_linear_forward(C.byref(view), None, C.byref(route), 4096, None, 8192, None, 0, 16388, need, None)
+    assert st == 1 and b"16-byte aligned" in lib.tris_last_error()
