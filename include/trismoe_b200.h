@@ -601,6 +601,13 @@ size_t tris_moe_layer_extras_workspace_bytes(const TrisMoeLayerView* layer, cons
 int tris_moe_layer_forward_extras(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
                                   const float* router_logits, int32_t num_tokens, void* y_f16,
                                   float* router_logits_out, void* workspace, size_t workspace_bytes, void* stream);
+/* The same with the status word outside the workspace, for callers that take a workspace per call (several threads or
+   streams in one layer): status_dev is a device word that the caller zeroed once; nothing in the workspace needs
+   zeroing then.  NULL: as above. */
+int tris_moe_layer_forward_extras_status(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
+                                         const float* router_logits, int32_t num_tokens, void* y_f16,
+                                         float* router_logits_out, void* workspace, size_t workspace_bytes,
+                                         int32_t* status_dev, void* stream);
 
 /*
  * Same computation as tris_moe_layer_forward for callers that cannot provide a workspace

@@ -124,6 +124,7 @@ SIGNATURES = {
     "tris_moe_layer_forward": (C.c_int, [_P(TrisMoeLayerView), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp]),
     "tris_moe_layer_extras_workspace_bytes": (C.c_size_t, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _i32]),
     "tris_moe_layer_forward_extras": (C.c_int, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp]),
+    "tris_moe_layer_forward_extras_status": (C.c_int, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp, _vp]),
     "tris_moe_layer_forward_static": (C.c_int, [_P(TrisMoeLayerView), _vp, _vp, _i32, _vp, _vp, _vp]),
 }
 STATIC_SCRATCH_BYTES = 8 << 20

@@ -154,7 +154,7 @@ extern "C" size_t tris_moe_layer_workspace_bytes(const TrisMoeLayerView* layer, 
 
 static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
                          const float* router_logits, int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace,
-                         size_t workspace_bytes, void* stream) {
+                         size_t workspace_bytes, int32_t* status, void* stream) {
   int st = validate_layer(layer);
   if (st == TRIS_OK && extras) st = validate_extras(layer, extras);
   if (st != TRIS_OK) return st;
@@ -253,7 +253,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
   route.expert_ids = w.expert_ids;
   route.segment_offsets = w.segment_offsets;
   route.num_segments_dev = w.counts;
-  route.status_dev = w.counts + 2;
+  route.status_dev = status ? status : w.counts + 2;
 
   // gate/up + SiLU*mul; rows read the per-token backbone outputs through tok[]
   route.row_gather = w.tok;
@@ -329,7 +329,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
 extern "C" int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void* x_f16, const float* router_logits,
                                       int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace,
                                       size_t workspace_bytes, void* stream) {
-  return layer_forward(layer, nullptr, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, stream);
+  return layer_forward(layer, nullptr, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, nullptr, stream);
 }
 
 extern "C" size_t tris_moe_layer_extras_workspace_bytes(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, int32_t num_tokens) {
@@ -341,7 +341,13 @@ extern "C" size_t tris_moe_layer_extras_workspace_bytes(const TrisMoeLayerView* 
 extern "C" int tris_moe_layer_forward_extras(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
                                              const float* router_logits, int32_t num_tokens, void* y_f16, float* router_logits_out,
                                              void* workspace, size_t workspace_bytes, void* stream) {
-  return layer_forward(layer, extras, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, stream);
+  return layer_forward(layer, extras, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, nullptr, stream);
+}
+
+extern "C" int tris_moe_layer_forward_extras_status(const TrisMoeLayerView* layer, const TrisMoeLayerExtras* extras, const void* x_f16,
+                                                    const float* router_logits, int32_t num_tokens, void* y_f16, float* router_logits_out,
+                                                    void* workspace, size_t workspace_bytes, int32_t* status_dev, void* stream) {
+  return layer_forward(layer, extras, x_f16, router_logits, num_tokens, y_f16, router_logits_out, workspace, workspace_bytes, status_dev, stream);
 }
 
 // ---- variant that allocates nothing ----------------------------------------------------------

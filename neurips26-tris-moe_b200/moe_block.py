@@ -58,7 +58,7 @@ class TrisSparseMoeBlock(nn.Module):
         self._expanded_view: Optional[dict] = None  # expanded backbone names -> layer view
         self._workspace: Optional[torch.Tensor] = None
         self._workspace_for = None
-        self._status_word: Optional[torch.Tensor] = None  # status of the kernels forward_streaming launches
+        self._status_word: Optional[torch.Tensor] = None  # see _status_of
 
     # -- loading ---------------------------------------------------------------------------
     # activation rows above which a 4-bit backbone is expanded to fp16 scratch and run on the dense GEMM
@@ -115,6 +115,8 @@ class TrisSparseMoeBlock(nn.Module):
         self.input_scales = {n: v.reshape(-1).to(dev, torch.float16).contiguous() for n, v in (input_scales or {}).items()}
         if set(self.input_scales) - set(given):
             raise ValueError("input_scales keys must be among 'gate', 'up', 'down'")
+        if self.input_scales:
+            self._status_of(dev)  # made here and not by the first of several threads
         self._layer_view = self._expanded_view = None
         return self
 
@@ -128,6 +130,8 @@ class TrisSparseMoeBlock(nn.Module):
 
         self.ns_payloads = {n: p for n, p in (("gate", gate_ns), ("up", up_ns), ("down", down_ns))
                             if p is not None and ns_payload_max_rank(p) > 0}
+        if self.ns_payloads and self.gate.weight.is_cuda:
+            self._status_of(self.gate.weight.device)
         return self
 
     def backbone_rank(self, name: str) -> int:
@@ -166,27 +170,32 @@ class TrisSparseMoeBlock(nn.Module):
             self._layer_view, self._expanded_view = v, None
         return self._layer_view
 
-    def _expanded_layer_view(self, dev, names) -> TrisMoeLayerView:
+    def _expanded_layer_view(self, dev, names, own: Optional[list] = None) -> TrisMoeLayerView:
         """The layer view with the 4-bit backbones in ``names`` expanded into fp16 scratch (enqueued on
         the current stream): what large batches use, where the dense GEMM beats re-expanding nibbles for
-        every pass over the rows.  The scratch is shared by all blocks of a model."""
+        every pass over the rows.  The scratch is shared by all blocks of a model, or with ``own`` the call's
+        own, kept in that list."""
         base = self.layer_view()
         if self._expanded_view is None:
             self._expanded_view = {}
         key = tuple(sorted(names))
-        v = self._expanded_view.get(key)
+        v = self._expanded_view.get(key) if own is None else None
         if v is None:
             v = TrisMoeLayerView()
             C.pointer(v)[0] = base
-            self._expanded_view[key] = v
+            if own is None:
+                self._expanded_view[key] = v
         lib = _native.load()
         for name in key:
             p = self.packed_backbones[name]
             skey = (str(dev), name, p.rows, p.cols)
-            scratch = TrisSparseMoeBlock._expand_scratch.get(skey)
+            scratch = TrisSparseMoeBlock._expand_scratch.get(skey) if own is None else None
             if scratch is None:
                 scratch = torch.empty((p.rows, p.cols), dtype=torch.float16, device=dev)
-                TrisSparseMoeBlock._expand_scratch[skey] = scratch
+                if own is None:
+                    TrisSparseMoeBlock._expand_scratch[skey] = scratch
+                else:
+                    own.append(scratch)
             if getattr(p, "_g_idx", None) is None:
                 g_idx = (torch.arange(p.cols, device=dev, dtype=torch.int32) // max(1, p.group_size)).clamp_(max=p.groups - 1)
                 p._g_idx = g_idx.to(torch.int32).contiguous()
@@ -222,17 +231,13 @@ class TrisSparseMoeBlock(nn.Module):
                 ex.ns_c2[i], ex.ns_c1[i] = C.addressof(c2), C.addressof(c1)
         return ex
 
-    def workspace(self, num_tokens: int, device, extras: Optional[TrisMoeLayerExtras] = None) -> torch.Tensor:
+    def workspace(self, num_tokens: int, device) -> torch.Tensor:
         view = self.layer_view()
         sized = self._workspace_for  # (view, tokens) the buffer is known to hold: the size grows with the tokens
-        if (extras is None and sized is not None and sized[0] is view and num_tokens <= sized[1] and self._workspace is not None
-                and self._workspace.device == device):
+        if sized is not None and sized[0] is view and num_tokens <= sized[1] and self._workspace is not None and self._workspace.device == device:
             return self._workspace
         lib = _native.load()
-        if extras is None:
-            need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), int(num_tokens)))
-        else:
-            need = int(lib.tris_moe_layer_extras_workspace_bytes(C.byref(view), C.byref(extras), int(num_tokens)))
+        need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), int(num_tokens)))
         if need == 0 and num_tokens > 0:
             raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
         if self._workspace is None or self._workspace.numel() < need or self._workspace.device != device:
@@ -240,8 +245,22 @@ class TrisSparseMoeBlock(nn.Module):
                 self.raise_on_kernel_status()  # do not lose a report with the old buffer
             self._workspace = torch.empty((need,), dtype=torch.uint8, device=device)
             self._workspace[:16].zero_()  # count words and the sticky status word
-        self._workspace_for = (view, int(num_tokens)) if extras is None else None
+        self._workspace_for = (view, int(num_tokens))
         return self._workspace
+
+    def _extras_workspace(self, num_tokens: int, device, extras: TrisMoeLayerExtras) -> torch.Tensor:
+        """Scratch of one call with input scales or null-space pairs: such blocks may be called from several threads and
+        streams at once, as the separate operators may, so no buffer outlives the call."""
+        need = int(_native.load().tris_moe_layer_extras_workspace_bytes(C.byref(self.layer_view()), C.byref(extras), int(num_tokens)))
+        if need == 0:
+            raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
+        return torch.empty((need,), dtype=torch.uint8, device=device)
+
+    def _status_of(self, device) -> torch.Tensor:
+        """Sticky status word of the kernels that do not report to a workspace of the block."""
+        if self._status_word is None or self._status_word.device != device:
+            self._status_word = torch.zeros((1,), dtype=torch.int32, device=device)
+        return self._status_word
 
     def last_kernel_status(self, clear: bool = True) -> int:
         """Status word of every kernel :meth:`forward` launched since the last clear: 0, or 6
@@ -310,23 +329,24 @@ class TrisSparseMoeBlock(nn.Module):
             logits_in, logits_out = None, logits.data_ptr()
         if T:
             self._require_rows(x, "forward")
-            ws = self.workspace(T, dev, extras)
-            view = self._layer_view  # which workspace() has just brought up to date
+            ws = self.workspace(T, dev) if extras is None else self._extras_workspace(T, dev, extras)
+            view = self._layer_view  # which the size query has just brought up to date
+            own = None if extras is None else []
             if self.packed_backbones:  # gate and up see T rows, down T * top_k
                 big = [n for n in self.packed_backbones
                        if (T * self.top_k if n == "down" else T) > self.PACKED_BACKBONE_MAX_ROWS]
                 if "gate" in big or "up" in big:
                     big = sorted(set(big) | ({"gate", "up"} & set(self.packed_backbones)))
                 if big:
-                    view = self._expanded_layer_view(dev, big)
+                    view = self._expanded_layer_view(dev, big, own)
             with torch.cuda.device(dev):
                 stream = torch.cuda.current_stream(dev).cuda_stream
                 if extras is None:
                     st = lib.tris_moe_layer_forward(C.byref(view), x.data_ptr(), logits_in, T, y.data_ptr(),
                                                     logits_out, ws.data_ptr(), ws.numel(), stream)
                 else:
-                    st = lib.tris_moe_layer_forward_extras(C.byref(view), C.byref(extras), x.data_ptr(), logits_in, T,
-                                                           y.data_ptr(), logits_out, ws.data_ptr(), ws.numel(), stream)
+                    st = lib.tris_moe_layer_forward_extras_status(C.byref(view), C.byref(extras), x.data_ptr(), logits_in, T, y.data_ptr(),
+                                                                  logits_out, ws.data_ptr(), ws.numel(), self._status_of(dev).data_ptr(), stream)
                 _native.check(st, "moe_layer_forward")
         return y.reshape(shape), logits if extras is None else returned
 
@@ -385,9 +405,7 @@ class TrisSparseMoeBlock(nn.Module):
             rv = _native.TrisRouteView()
             rv.expert_ids, rv.segment_offsets, rv.num_segments_dev = ids, seg, counts
             rv.num_segments, rv.num_rows, rv.max_rows_per_segment = min(E, R), R, T
-            if self._status_word is None or self._status_word.device != dev:
-                self._status_word = torch.zeros((1,), dtype=torch.int32, device=dev)
-            rv.row_gather, rv.status_dev, rv.flags = tok, self._status_word.data_ptr(), (1 if mode_gu else 0)
+            rv.row_gather, rv.status_dev, rv.flags = tok, self._status_of(dev).data_ptr(), (1 if mode_gu else 0)
             paged.wait("gate_up")  # down keeps paging under the gate/up kernel and the down backbone
             _native.check(lib.tris_grouped_pair_forward(C.byref(paged.views["gate"]), C.byref(paged.views["up"]), C.byref(rv), hg, hu, mlp_ptr,
                                                         None, 1, stream), "grouped_pair_forward")

@@ -117,3 +117,46 @@ def test_pair_of_ordinary_linears_of_two_formats_gets_route_arrays(monkeypatch, 
     c3.run_compact3_qkv_forward(linear(True), a, b, x)
     c3.run_compact3_gate_up_forward(a, b, x)
     assert [("expert_ids" in r, r.get("_one_segment", False)) for r in routes] == [(arrays, not arrays)] * 2
+
+
+@pytest.mark.parametrize("packed,tokens", [(False, 3), (True, 3), (True, 200)])
+def test_blocks_with_input_scales_share_no_scratch_between_calls(block, monkeypatch, packed, tokens):
+    """Two calls in flight at once (two threads, two streams), played by a second call from inside the first one's launch:
+    their workspaces and expanded backbones must not overlap.  The library is a recorder, so this needs no GPU."""
+    import contextlib
+    import ctypes as C
+    import types
+
+    import trismoe_b200 as tm
+
+    spans, depth = [], []
+
+    def forward(view, extras, x, logits, T, y, out, ws, size, *rest):
+        view = view._obj
+        mine = [(ws, ws + size)]
+        if packed and tokens > block.PACKED_BACKBONE_MAX_ROWS:
+            mine += [(getattr(view, "shared_" + n), getattr(view, "shared_" + n) + 64 * 32) for n in ("gate", "up", "down")]
+        depth.append(0)
+        if len(depth) == 1:
+            block(torch.zeros((1, tokens, 64), dtype=torch.float16), torch.zeros((tokens, 4)))
+        spans.append(mine)
+        return 0
+
+    lib = types.SimpleNamespace(tris_moe_layer_forward_extras=forward, tris_moe_layer_forward_extras_status=forward,
+                                tris_moe_layer_extras_workspace_bytes=lambda *a: 4096, tris_packed4_dequantize=lambda *a: 0)
+    monkeypatch.setattr(tm._native, "load", lambda: lib)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: types.SimpleNamespace(cuda_stream=0))
+    view = tm._native.TrisMoeLayerView()
+    block._layer_view = view
+    monkeypatch.setattr(block, "layer_view", lambda: view)
+    block.input_scales = {"gate": torch.ones((64,), dtype=torch.float16)}
+    if packed:
+        word = torch.zeros((1,), dtype=torch.int32)
+        for n, w in (("gate", 64), ("up", 64), ("down", 32)):
+            block.packed_backbones[n] = types.SimpleNamespace(rows=32, cols=w, groups=1, group_size=w, qweight=word, qzeros=word, scales=word)
+    block(torch.zeros((1, tokens, 64), dtype=torch.float16), torch.zeros((tokens, 4)))
+    assert len(spans) == 2
+    for a in spans[0]:
+        for b in spans[1]:
+            assert a[1] <= b[0] or b[1] <= a[0]
