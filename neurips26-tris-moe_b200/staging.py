@@ -219,8 +219,9 @@ class GroupedQGmapCPUStagingManager:
 
     def _plan(self, block_index: int, ring: int):
         """Pager launches ``(jobs, count, bytes per segment, ends gate/up, slot table)`` and staged views of a
-        layer in a ring slot, laid out on first use and again when a projection's own view was rebuilt."""
-        bases = tuple(id(proj_view(self.entries[(block_index, proj)].payload)) for proj in PROJECTIONS)
+        layer in a ring slot, laid out on first use and again when a projection's own view has other contents
+        (an object's identity would miss a view edited in place, and one built at a freed view's address)."""
+        bases = tuple(bytes(proj_view(self.entries[(block_index, proj)].payload)) for proj in PROJECTIONS)
         plan = self._plans.get((block_index, ring))
         if plan is not None and plan[0] == bases:
             return plan[1], plan[2]
