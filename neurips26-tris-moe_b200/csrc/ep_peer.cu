@@ -46,8 +46,8 @@ __device__ __forceinline__ void ep_signal_peers(int32_t* const* peer_flags, int 
 // costs one 4-byte store per slot and nothing else: (1) one thread per slot writes the id word and the
 // combine index; (2) thread groups copy the rows in use, one group per row.
 __global__ void __launch_bounds__(128) ep_dispatch_peer_kernel(
-    const __half* __restrict__ hidden_gate, const __half* __restrict__ hidden_up, int rank_gu,
-    const int32_t* __restrict__ selected, const int32_t* __restrict__ perm, const int32_t* __restrict__ tok,
+    const __half* hidden_gate, const __half* hidden_up, int rank_gu,
+    const int32_t* selected, const int32_t* perm, const int32_t* tok,  // not __restrict__: written by the kernels before this one
     int num_rows, int num_experts, int world, int my_rank, int capacity, __half* const* __restrict__ peer_recv,
     int row_stride, int32_t* __restrict__ combine_index, int32_t* __restrict__ overflow,
     int32_t* const* __restrict__ peer_flags) {
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(128) ep_dispatch_peer_kernel(
 // buffer.  Rows whose received id is negative (padding) are skipped: every thread looks at one slot
 // of a batch, the slots in use are listed in shared memory and the warps copy those, one row each.
 __global__ void __launch_bounds__(256) ep_return_peer_kernel(
-    const __half* __restrict__ results, const __half* __restrict__ recv_rows, int row_stride, int rank_gu,
+    const __half* results, const __half* recv_rows, int row_stride, int rank_gu,
     int hidden, int world, int my_rank, int capacity, __half* const* __restrict__ peer_back,
     int32_t* const* __restrict__ peer_flags) {
   __shared__ int32_t s_live[256];

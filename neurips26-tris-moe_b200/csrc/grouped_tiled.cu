@@ -498,8 +498,8 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
     const int tid = threadIdx.x - W::kLoad0 * 32;
     bool waited = !args.weights_before_wait;
     int next_src = 0, pass = 0;  // this thread's source row of the pass the walker has reached; that pass's parity
-    auto find_row = [&]() {
-      if (w.valid() && tid < w.rows()) next_src = args.row_gather ? __ldg(args.row_gather + w.r0 + tid) : w.r0 + tid;
+    auto find_row = [&]() {  // a plain load: a non-coherent one may be moved above the wait for the kernel that wrote the list
+      if (w.valid() && tid < w.rows()) next_src = args.row_gather ? args.row_gather[w.r0 + tid] : w.r0 + tid;
     };
     auto keep_row = [&]() { if (tid < N) src_rows[pass * N + tid] = next_src; };
     uint32_t rows_of = 0u;  // rows of the items in flight, oldest in the low byte
