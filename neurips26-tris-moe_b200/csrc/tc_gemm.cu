@@ -287,6 +287,11 @@ struct TcTmaMaps {
 constexpr int kTcRowBytes = kTcKChunk * 2;
 static_assert(kTcRowBytes == 128, "one swizzle row per operand row and chunk");
 
+// Parity of the last copy round of stage s when `issued` chunks went round-robin over the stages, -1: none.
+constexpr int last_round_parity(int issued, int s) { return issued > s ? ((issued - 1 - s) / kTcStages) & 1 : -1; }
+static_assert(last_round_parity(0, 0) == -1 && last_round_parity(3, 2) == 0 && last_round_parity(3, 3) == -1 && last_round_parity(4, 3) == 0, "first round");
+static_assert(last_round_parity(5, 0) == 1 && last_round_parity(5, 1) == 0 && last_round_parity(8, 3) == 1 && last_round_parity(9, 0) == 0, "later rounds");
+
 template <int NTILE>
 struct TcTmaSmem {  // at a 1024-byte boundary
   uint8_t a[kTcStages][kTcM * kTcRowBytes];
@@ -356,9 +361,10 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
   pdl_launch_dependents();
   const int n_live = args.n_dev ? min(args.n, *args.n_dev) : args.n;
 
+  int issued = 0;
   if (threadIdx.x == 0) {
     // producer: one tensor copy per operand per K chunk, kTcStages chunks in flight
-    for (int i = 0; i < nchunks; ++i) {
+    for (int i = 0; i < nchunks; ++i, ++issued) {
       const int s = i % kTcStages;
       if (i >= kTcStages && !mbar_wait_bounded(&sm.empty[s], ((i / kTcStages) - 1) & 1)) {
         sm.timed_out = 1;
@@ -396,7 +402,8 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
   __syncthreads();
   const bool failed = sm.timed_out != 0;
   if (failed && threadIdx.x == 0)  // copies in flight must not land in a buffer that is read as the partial tile
-    for (int i = 0; i < kTcStages; ++i) mbar_wait_bounded(&sm.full[i], 0);
+    for (int s = 0; s < kTcStages; ++s)
+      if (last_round_parity(issued, s) >= 0) mbar_wait_bounded(&sm.full[s], last_round_parity(issued, s));
   __syncthreads();
   tc_gemm_epilogue<NTILE>(args, pb, reinterpret_cast<float*>(base), tmem, failed, nchunks, m0, n0, n_live, cluster);
 }
