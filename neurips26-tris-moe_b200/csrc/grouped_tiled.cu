@@ -43,7 +43,8 @@ struct Roles {
 };
 constexpr int kMaxStages = 4;
 constexpr int kDBase = 4 * 2 * kACols;       // accumulators behind the four warpgroups' two slots
-constexpr int kBarBytes = 512;
+constexpr int kBarBytes = 512;               // barriers and the TMEM address
+static_assert((2 * kMaxStages + 8 + 8 + 4 + 4 + kMmaWarps) * sizeof(uint64_t) + sizeof(uint32_t) <= kBarBytes, "barriers");
 constexpr int kRowIdxBytes = 2 * 128 * 4;
 constexpr int kOutBytes = 2 * 2 * 16 * kTileOut * 2;         // per epilogue warpgroup two tiles of 16 rows, fp16
 constexpr int kHeadBytes = kBarBytes + kRowIdxBytes + kOutBytes + 1024;  // and the way to a 1024-byte boundary
@@ -232,7 +233,8 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
   uint64_t* a_empty = a_full + 8;                          // MMA (commit) -> unpack
   uint64_t* d_full = a_empty + 8;                          // MMA (commit) -> epilogue
   uint64_t* d_empty = d_full + 4;                          // epilogue warps -> MMA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 4);
+  uint64_t* mma_done = d_empty + 4;                        // [MMA warp] its last commit
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 2);
   int* src_rows = reinterpret_cast<int*>(sm + kBarBytes);  // [2][N] source rows of a pass, by pass parity
   uint8_t* stage_base = sm + ((smem_u32(sm) + kBarBytes + kRowIdxBytes + kOutBytes + 1023) & ~1023u) - smem_u32(sm);  // the swizzle counts from 1024-byte boundaries
 
@@ -250,6 +252,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       mbar_init(&d_full[i], 2);
       mbar_init(&d_empty[i], W::kEpiWarps);
     }
+    for (int i = 0; i < kMmaWarps; ++i) mbar_init(&mma_done[i], 1);
     fence_mbar_init();
   }
   if (warp == W::kMma0) tmem_alloc(tmem_slot, 512);  // before the dependents may start: they allocate too
@@ -637,6 +640,9 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
       if (!args.reuse) stage.advance(args.stages);
       else if (last && last_tile) stage = stage.at(pass_chunks, args.stages);
     }
+    // TMEM and shared memory go back below: not under an MMA that is still running, whichever role gave up
+    if (elect_one()) umma_commit(&mma_done[r]);
+    ok = mbar_wait_warp(&mma_done[r], 0u) && ok;
   }
   if (!ok && args.status) atomicExch(args.status, TRIS_ERR_TIMEOUT);
   __syncwarp();
