@@ -80,11 +80,15 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
   }
   const int seg = blockIdx.y;
   const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
-  if (seg >= nseg) return;
+  // A CTA without rows leaves at once, but the first one waits: if none did, the launch could end before its predecessor.
+  auto leave = [&]() {
+    if (args.weights_before_wait && blockIdx.x == 0 && blockIdx.y == 0) pdl_wait();
+  };
+  if (seg >= nseg) return leave();
   const int expert = args.expert_ids ? args.expert_ids[seg] : 0;  // no arrays: one segment of expert 0 with all rows
   const int row_begin = args.expert_ids ? args.segment_offsets[seg] : 0;
   const int row_end = args.expert_ids ? min(args.segment_offsets[seg + 1], args.num_rows) : args.num_rows;
-  if (expert < 0 || expert >= args.num_experts || row_end <= row_begin) return;
+  if (expert < 0 || expert >= args.num_experts || row_end <= row_begin) return leave();
 
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int p = DUAL ? warp & 1 : 0, og = (warp / P) % OG, ks = warp / (P * OG);

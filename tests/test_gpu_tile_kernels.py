@@ -219,3 +219,22 @@ def test_backbone_gemm_at_tile_edges(lib, n, k, m):
     w = (0.05 * torch.randn((m, k), generator=g)).half().cuda()
     ref, _, bound = _bound(w, x)
     _assert_within(tm.compute_shared_hidden(x, w), ref, bound)
+
+
+@pytest.mark.parametrize("T", [1, 16, 70])
+def test_batch_whose_logits_are_not_numbers(lib, T):
+    """No segment has rows: every launch of the sequence still waits for the one before, the outputs are not numbers
+    either and the next batch is computed as ever."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=5)
+    blk = tm.TrisSparseMoeBlock(256, 192, 8, 2, True)
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], layer["shared_gate"], layer["shared_up"], layer["shared_down"],
+                              layer["router_weight"], device="cuda")
+    x, logits = synth.synth_activations(T, 256, seed=T).cuda().view(1, T, 256), synth.synth_router_logits(T, 8, seed=T).cuda()
+    want = blk(x, logits)[0].clone()
+    for _ in range(3):
+        assert blk(x, torch.full_like(logits, float("nan")))[0].isnan().all()
+        assert torch.equal(blk(x, logits)[0], want)
