@@ -186,7 +186,7 @@ def _adopt_stored_derived(payload: dict, dev, E: int, pr: int, O: int, rank: int
     ok = all(isinstance(t, torch.Tensor) for t in (idx, grp, rec, desc, col)) and isinstance(meta, tuple) and len(meta) == 3
     ok = ok and tuple(idx.shape) == (E, nblk, 32) and tuple(grp.shape) == (E, pr) and tuple(desc.shape) == (count + 1, 2)
     ok = ok and col.numel() == E * chunks * int(meta[0]) and rec.dtype == torch.uint8 and col.dtype == torch.uint8
-    ok = ok and rec.numel() == count * int(meta[1])
+    ok = ok and rec.numel() == count * int(meta[1]) and _record_sizes_fit(rank, *meta)
     if ok:  # records of another layout version are rebuilt
         ok = int(col[:4].cpu().view(torch.int32).item()) == TILE_RECORD_MAGIC
     if not ok:
@@ -205,6 +205,15 @@ def _adopt_stored_derived(payload: dict, dev, E: int, pr: int, O: int, rank: int
 
 
 TILE_RECORD_MAGIC = 0x33305254  # layout version of the records, first word of every column record
+
+
+def _record_sizes_fit(rank: int, col_bytes: int, record_bytes: int, steps: int) -> bool:
+    """Whether the three sizes of a projection's records belong together: the kernels find every part of a record
+    from them.  Column record: header 64, scales 512, 96 a salient step.  Sub-record of 32 outputs: 512 a slice of
+    64 columns, 128 a step, 256 a row-scale slot (one to four)."""
+    sub, rest = divmod(record_bytes, 4)
+    slots, odd = divmod(sub - 512 * min(2, math.ceil(rank / 64)) - 128 * steps, 256)
+    return 0 <= steps <= 8 and col_bytes == 576 + 96 * steps and rest == odd == 0 and 1 <= slots <= 4
 
 
 def _col_record_bytes(view: TrisProjView, total: int) -> int:

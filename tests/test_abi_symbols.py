@@ -72,7 +72,7 @@ def _record_view(out_features, rank):
     v = tm._native.TrisProjView()
     v.num_experts, v.out_features, v.rank, v.num_groups, v.use_block_gr = 1, out_features, rank, 1, 1
     v.tile_records = v.col_records = 1 << 20
-    v.col_record_bytes, v.max_record_bytes, v.max_sal_words = 672, 4 * 1536, 1
+    v.col_record_bytes, v.max_record_bytes, v.max_sal_words = 672, 4 * 1408, 1
     return v
 
 

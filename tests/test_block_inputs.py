@@ -160,3 +160,20 @@ def test_blocks_with_input_scales_share_no_scratch_between_calls(block, monkeypa
     for a in spans[0]:
         for b in spans[1]:
             assert a[1] <= b[0] or b[1] <= a[0]
+
+
+@pytest.mark.parametrize("meta,adopted", [((672, 4 * 1408, 1), True), ((672, 4 * 2176, 1), True), ((576, 4 * 1280, 0), True), ((672, 4 * 1408, 2), False), ((768, 4 * 1408, 1), False),
+                                          ((672, 4 * 1408 + 2, 1), False), ((672, 4 * 1152, 1), False), ((672, 4 * 2432, 1), False), ((0, 4 * 1408, 1), False),
+                                          ((576 + 9 * 96, 4 * (1024 + 9 * 128 + 256), 9), False)])
+def test_stored_records_whose_sizes_disagree_are_rebuilt(meta, adopted):
+    """A checkpoint's stored tile records: the kernels compute every address from these three sizes."""
+    from trismoe_b200 import qlinear_grouped as qg
+
+    E, pr, O, rank, count = 2, 4, 100, 128, 2
+    col = torch.zeros((E * meta[0],), dtype=torch.uint8)
+    col[:4] = torch.tensor([qg.TILE_RECORD_MAGIC], dtype=torch.int32).view(torch.uint8)[: col.numel()]
+    payload = {"_tris_gr_index": torch.zeros((E, 4, 32), dtype=torch.int32), "_tris_packed_row_group": torch.zeros((E, pr), dtype=torch.int32),
+               "_tris_tile_records": torch.zeros((count * meta[1],), dtype=torch.uint8), "_tris_tile_desc": torch.zeros((count + 1, 2), dtype=torch.int32),
+               "_tris_col_records": col, "_tris_tile_meta": meta, "_tris_derived_from_checkpoint": True}
+    assert qg._adopt_stored_derived(payload, torch.device("cpu"), E, pr, O, rank, 1) is adopted
+    assert ("_tris_tile_records" in payload) is adopted
