@@ -853,8 +853,10 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   a.partial = static_cast<float*>(opts.workspace);
   a.partial_bytes = opts.workspace_bytes;
   a.col_scale = static_cast<const __half*>(route->hidden_col_scale);
-  a.hidden_vec = a.hidden_mode == TRIS_OUT_F16 && !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 &&
-                 ((reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1])) & 15u) == 0;
+  const bool in_pieces = !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 &&
+                         ((reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1])) & 15u) == 0;
+  a.hidden_vec = in_pieces && a.hidden_mode == TRIS_OUT_F16;
+  a.hidden_perm = in_pieces && a.hidden_mode != TRIS_OUT_F16;
   a.quad_store = proj_a->out_features % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 7u) == 0;
   a.vec_store = proj_a->out_features % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 15u) == 0;
   TRIS_REQUIRE(a.col_scale == nullptr || a.hidden_mode == TRIS_OUT_F16, TRIS_ERR_INVALID_ARG,

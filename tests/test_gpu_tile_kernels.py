@@ -238,3 +238,27 @@ def test_batch_whose_logits_are_not_numbers(lib, T):
     for _ in range(3):
         assert blk(x, torch.full_like(logits, float("nan")))[0].isnan().all()
         assert torch.equal(blk(x, logits)[0], want)
+
+
+@pytest.mark.parametrize("rank", [32, 96, 256, 320])
+@pytest.mark.parametrize("lengths", [[1, 5, 0, 16], [40, 3, 64, 33], [130, 70]])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_permuted_rows_give_the_same_bits(lib, rank, lengths, offset):
+    """Rows in the two permuted column orders, at 16-byte boundaries and off them, against the same rows row-major."""
+    import trismoe_b200 as tm
+
+    E, R, O = len(lengths), sum(lengths), 104
+    pa, pb = _payload(tm, E, O, rank, 32, rank), _payload(tm, E, O, rank, 32, rank + 1)
+    rows = (0.5 * torch.randn((R, rank), generator=torch.Generator().manual_seed(R))).half().cuda()
+    eye = torch.eye(rank, dtype=torch.float16, device="cuda")
+    route = dict(tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda"))
+    run = lambda h, r: (tm.run_grouped_structured_expert_forward(pa, h, None, r),
+                        *tm.run_grouped_structured_expert_pair_forward(pa, pb, h, h, None, r),
+                        tm.run_grouped_structured_expert_pair_forward(pa, pb, h, h, None, r, fuse_silu_mul=True)[0])
+    want = run(rows, route)
+    for layout in (tm.HIDDEN_PAIR_INTERLEAVED, tm.HIDDEN_LANE_ORDER):
+        buf = torch.empty((R * rank + 8,), dtype=torch.float16, device="cuda")
+        h = buf[offset: offset + R * rank].view(R, rank)
+        h.copy_(tm.compute_shared_hidden(rows, eye, layout=layout))  # single products: the rows themselves, permuted
+        for a, b in zip(run(h, {**route, "_hidden_layout": layout}), want):
+            assert torch.equal(a, b)
