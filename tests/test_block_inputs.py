@@ -97,7 +97,7 @@ def test_shared_expert_gate_keeps_its_gradient(monkeypatch):
 
 
 @pytest.mark.parametrize("first,second,arrays", [(True, True, False), (True, False, True), (False, True, True), (False, False, True)])
-def test_pair_of_ordinary_linears_of_two_formats_gets_route_arrays(monkeypatch, first, second, arrays):
+def test_pair_of_which_one_has_no_records_gets_route_arrays(monkeypatch, first, second, arrays):
     """Only the tile-record kernels take a route without arrays, and a pair runs on them only if both have records."""
     from trismoe_b200 import compact3_linear as c3
 

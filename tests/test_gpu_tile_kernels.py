@@ -262,3 +262,19 @@ def test_permuted_rows_give_the_same_bits(lib, rank, lengths, offset):
         h.copy_(tm.compute_shared_hidden(rows, eye, layout=layout))  # single products: the rows themselves, permuted
         for a, b in zip(run(h, {**route, "_hidden_layout": layout}), want):
             assert torch.equal(a, b)
+
+
+def test_pair_of_ordinary_linears_of_which_one_has_no_records(lib):
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(7)
+    mods = []
+    for records in (True, False):
+        p = synth.pack_projection(synth.raw_projection(rng, 1, 96, 512, group_size=128))
+        mods.append(tm.Compact3Linear(tm.prepare_grouped_payload(p, "cuda", tile_records=records)))
+    x = (0.5 * torch.randn((5, 512), generator=torch.Generator().manual_seed(5))).half().cuda()
+    for pair in (mods, mods[::-1]):
+        for y, m in zip(tm.run_compact3_gate_up_forward(*pair, x, fuse_silu_mul=False), pair):
+            ref, _, bound = _bound(tm.dequantize_grouped_payload(m.payload)[0], x)
+            _assert_within(y, ref, bound)
