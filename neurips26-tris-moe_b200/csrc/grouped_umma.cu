@@ -250,12 +250,13 @@ static std::atomic<int> g_tc_min_rows{2048};
 
 int grouped_tc_min_rows() { return g_tc_min_rows.load(std::memory_order_relaxed); }
 
-// Dense-contraction path: activations must be pair-interleaved, rank a multiple of 32 and at
-// most one 256-column chunk.
+// Dense-contraction path: activations must be pair-interleaved, their rows at 16-byte boundaries (cp.async of
+// 16 bytes), rank a multiple of 32 and at most one 256-column chunk.
 bool grouped_umma_applicable(const GroupedArgs& args, int rows_hint) {
   const TrisProjView& v = args.proj[0];
   return rows_hint > g_tc_min_rows.load(std::memory_order_relaxed) && args.hidden_interleaved &&
-         (v.rank % 32) == 0 && v.rank <= 256 && args.ksplit <= 1 && (args.hidden_stride % 8) == 0;
+         (v.rank % 32) == 0 && v.rank <= 256 && args.ksplit <= 1 && (args.hidden_stride % 8) == 0 &&
+         ((reinterpret_cast<uintptr_t>(args.hidden[0]) | reinterpret_cast<uintptr_t>(args.hidden[1])) & 15u) == 0;
 }
 
 int launch_grouped_umma(const GroupedArgs& args, int nproj, int epi, cudaStream_t stream, bool pdl) {

@@ -666,8 +666,9 @@ def test_streaming_qwen35_shape_vs_oracle(tm, mode, fmt, T):
 # ---------------------------------------------------------------------------------------
 @pytest.fixture
 def tensor_core_from_64_rows(tm):
-    """The launchers pick the tcgen05 kernel above a row count whose default lies beyond these
-    tests' sizes; lower it so that the tensor-core kernel is what runs, and put it back."""
+    """The launchers of the plane kernels pick the tcgen05 one above a row count whose default lies beyond
+    these tests' sizes; lower it, and put it back.  Projections with tile records do not look at it: they run
+    their own tcgen05 kernel from 33 rows a segment on."""
     lib = tm._native.load()
     previous = lib.tris_set_grouped_tc_min_rows(64)
     yield
@@ -676,8 +677,8 @@ def tensor_core_from_64_rows(tm):
 
 @pytest.mark.parametrize("rank,T", [(96, 200), (256, 150), (64, 700)])
 def test_layer_prefill_rows_take_the_tensor_core_path(tm, tensor_core_from_64_rows, rank, T):
-    """Few experts, many tokens: ~100+ rows per expert, rank a multiple of 32 -> the grouped
-    kernels run their tcgen05 variant (weights unpacked once per tile into shared memory)."""
+    """Few experts, many tokens: ~100+ rows per expert, so the tcgen05 kernel over tile records runs (weights
+    unpacked to tensor memory)."""
     from trismoe_b200 import synth
 
     shape = synth.LayerShape(256, 320, 4, 2, rank=rank, group_size=32)
@@ -697,7 +698,7 @@ def test_layer_prefill_rows_take_the_tensor_core_path(tm, tensor_core_from_64_ro
     max_abs, mean_rel = orc.error_metrics(y.view(T, -1).float().cpu().numpy(), ref)
     assert np.abs(ref).mean() > 1e-4
     assert max_abs <= MAX_ABS and mean_rel <= MEAN_REL, (max_abs, mean_rel)
-    # and agrees with the register (mma.sync) path, which the operator API takes for row-major input
+    # and agrees with the operators one by one
     y2, _ = blk.forward_grouped_ops(x.cuda().view(1, T, -1), router_logits=logits.cuda())
     max_abs, mean_rel = orc.error_metrics(y2.view(T, -1).float().cpu().numpy(), ref)
     assert max_abs <= MAX_ABS and mean_rel <= 2 * MEAN_REL, (max_abs, mean_rel)
@@ -705,7 +706,8 @@ def test_layer_prefill_rows_take_the_tensor_core_path(tm, tensor_core_from_64_ro
 
 @pytest.mark.parametrize("kernel", ["register", "tensor_core"])
 def test_layer_olmoe_shape_prefill_512(tm, olmoe_layer, kernel):
-    """Headline shape, 512-token prefill (64 rows per expert on average)."""
+    """Headline shape, 512-token prefill (64 rows per expert on average).  The payloads have tile records, so both
+    settings of the plane kernels' switch run the same kernel (test_layer_prefill_on_planes has both plane kernels)."""
     from trismoe_b200 import synth
 
     layer, blk = olmoe_layer
@@ -729,9 +731,57 @@ def test_layer_olmoe_shape_prefill_512(tm, olmoe_layer, kernel):
         assert torch.allclose(y_one.view(-1).float(), y.view(T, -1)[t].float(), atol=3e-3, rtol=3e-3)
 
 
+@pytest.mark.parametrize("min_rows", [64, 1 << 20])
+@pytest.mark.parametrize("rank,T", [(96, 200), (256, 150), (64, 700), (32, 600)])
+def test_layer_prefill_on_planes(tm, rank, T, min_rows):
+    """Payloads without tile records (what streaming and sparse payloads run on): ~75 to 350 rows per expert through
+    the tcgen05 plane kernel (switch at 64 rows) and through the mma.sync one, against the fp32 oracle; whole single
+    weights from one-hot rows, in rows at 16-byte boundaries and off them."""
+    from trismoe_b200 import synth
+
+    shape = synth.LayerShape(256, 320, 4, 2, rank=rank, group_size=32)
+    layer = synth.synth_layer(shape, seed=rank + T)
+    for name in ("gate", "up", "down"):
+        layer["shared_" + name] = (layer["shared_" + name].float() * 5.0).half()
+    weights = {n: [orc.dequantize_expert(to_numpy_payload(layer[n]), e) for e in range(4)] for n in ("gate", "up", "down")}
+    payloads = [tm.prepare_grouped_payload(layer[n], "cuda:0", tile_records=False) for n in ("gate", "up", "down")]
+    blk = tm.TrisSparseMoeBlock(256, 320, 4, 2, shape.norm_topk_prob)
+    blk.load_grouped_payloads(*payloads, layer["shared_gate"], layer["shared_up"], layer["shared_down"], layer["router_weight"], device="cuda:0")
+    assert blk._get_grouped_payload("gate").get("_tris_tile_records") is None
+    x = synth.synth_activations(T, shape.hidden_size, seed=T)
+    logits = synth.synth_router_logits(T, shape.num_experts, seed=T + 1)
+    shared = {n: layer["shared_" + n].numpy() for n in ("gate", "up", "down")}
+    lib = tm._native.load()
+    previous = lib.tris_set_grouped_tc_min_rows(min_rows)
+    try:
+        y, _ = blk(x.cuda().view(1, T, -1), router_logits=logits.cuda())
+        ref = orc.moe_layer_fp32(x.numpy(), logits.numpy(), weights, shared, shape.top_k, shape.norm_topk_prob)
+        max_abs, mean_rel = orc.error_metrics(y.view(T, -1).float().cpu().numpy(), ref)
+        assert np.abs(ref).mean() > 1e-4
+        assert max_abs <= MAX_ABS and mean_rel <= MEAN_REL, (max_abs, mean_rel)
+        # every weight of gate, up and down: one-hot rows, pair-interleaved as this path takes them
+        lengths = [70, 0, 150, 97]
+        expert = torch.repeat_interleave(torch.arange(4), torch.tensor(lengths)).cuda()
+        place = torch.cat([torch.arange(n) for n in lengths]).cuda()
+        route = {**tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda"), "_hidden_layout": tm.HIDDEN_PAIR_INTERLEAVED}
+        w = [tm.dequantize_grouped_payload(p) for p in payloads]
+        R, eye = int(expert.numel()), torch.eye(rank, dtype=torch.float16, device="cuda")
+        for c in range(0, rank, 70):
+            col = (place + c) % rank
+            for offset in (0, 2):  # halves
+                h = torch.empty((R * rank + 8,), dtype=torch.float16, device="cuda")[offset: offset + R * rank].view(R, rank)
+                h.copy_(tm.compute_shared_hidden(torch.nn.functional.one_hot(col, rank).half(), eye, layout=tm.HIDDEN_PAIR_INTERLEAVED))
+                assert torch.equal(tm.run_grouped_structured_expert_forward(payloads[2], h, None, route), w[2][expert, :, col])
+                a, b = tm.run_grouped_structured_expert_pair_forward(payloads[0], payloads[1], h, h, None, route)
+                assert torch.equal(a, w[0][expert, :, col]) and torch.equal(b, w[1][expert, :, col])
+    finally:
+        lib.tris_set_grouped_tc_min_rows(previous)
+    blk.raise_on_kernel_status()
+
+
 def test_row_split_of_long_segments_leaves_results_unchanged(tm):
-    """Few experts with long, uneven segments (an expert-parallel rank's shape): the register-cached kernel
-    shares a unit's 32-row passes among up to four CTAs.  With the split switched off the outputs are the same
+    """Few experts with long, uneven segments (an expert-parallel rank's shape): the tiled kernel shares a unit's
+    row passes among up to four CTAs.  With the split switched off the outputs are the same
     bits; segments of 1, 33, 70, 130 and 300 rows cover CTAs without a pass, a ragged last pass and CTAs with
     several passes; the result agrees with the fp32 oracle."""
     from trismoe_b200 import synth
