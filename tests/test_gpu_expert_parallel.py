@@ -53,8 +53,8 @@ def _worker(rank, world, port, out):
                 err = (got.float() - want.float()).abs()
                 ok = ok and bool(torch.isfinite(got.float()).all()) and \
                     float(err.max()) <= 2e-3 * max(1.0, float(want.float().abs().max()))
-        # prefill-sized batch: ~100 rows per local expert, so the tensor-core grouped kernels run
-        # on the received rows (strided activations in, scattered rows out)
+        # prefill-sized batch: ~100 rows per local expert, so the tcgen05 kernel over tile records runs on the
+        # received rows (strided activations in, scattered rows out); the switch is that of the plane kernels
         T = 200
         blk.set_capacity(T)
         previous_tc_rows = tm._native.load().tris_set_grouped_tc_min_rows(64)
@@ -66,7 +66,7 @@ def _worker(rank, world, port, out):
         err = (got.float() - want.float()).abs()
         ok = ok and float(err.max()) <= 2e-3 * max(1.0, float(want.float().abs().max()))
         ok = ok and not blk.exchange_overflowed()
-        # ... and with the register kernels on the same rows (several 64-row passes per expert)
+        # ... and once more with that switch off
         tm._native.load().tris_set_grouped_tc_min_rows(1 << 20)
         got_reg, _ = blk(x.view(1, T, -1), router_logits=logits)
         torch.cuda.synchronize()

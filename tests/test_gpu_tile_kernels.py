@@ -81,6 +81,26 @@ def test_grouped_kernels_at_tile_edges(lib, O, rank, group, lengths):
         _assert_within(mlp[rows], want, err)
 
 
+@pytest.mark.parametrize("O,rank,group,lengths", GROUPED)
+def test_grouped_kernels_give_every_single_weight(lib, O, rank, group, lengths):
+    """Rows that are one at one column and zero elsewhere: an output is a single weight, exactly, so one lost or misplaced
+    column or salient term shows whatever the size of a sum.  Every segment sees every column."""
+    import trismoe_b200 as tm
+
+    E = len(lengths)
+    pa, pb = _payload(tm, E, O, rank, group, O + rank), _payload(tm, E, O, rank, group, O + rank + 1)
+    wa, wb = tm.dequantize_grouped_payload(pa), tm.dequantize_grouped_payload(pb)
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(lengths)).cuda()
+    place = torch.cat([torch.arange(n) for n in lengths]).cuda()
+    route = tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda")
+    for c in range(0, rank, min(n for n in lengths if n)):
+        ca, cb = (place + c) % rank, (place + c + 7) % rank
+        ha, hb = (torch.nn.functional.one_hot(col, rank).half() for col in (ca, cb))
+        assert torch.equal(tm.run_grouped_structured_expert_forward(pa, ha, None, route), wa[expert, :, ca])
+        sa, sb = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, hb, None, route)
+        assert torch.equal(sa, wa[expert, :, ca]) and torch.equal(sb, wb[expert, :, cb])
+
+
 @pytest.mark.parametrize("O,K,T", [(136, 520, 33), (137, 1100, 64), (1024, 2048, 65), (256, 4096, 130), (72, 8192, 300), (4096, 512, 257)])
 def test_linear_columns_shared_among_ctas(lib, O, K, T):
     """An ordinary matrix of more than 32 rows: its columns in one to many parts, single and as a pair."""
@@ -110,6 +130,12 @@ def test_linear_columns_shared_among_ctas(lib, O, K, T):
     silu = ra * torch.sigmoid(ra)
     err = 1.1 * ea * rb.abs() + silu.abs() * eb + 1.1 * ea * eb + (silu * rb).abs() * (2.0 ** -11 + 2.0 ** -19) + 2.0 ** -25
     _assert_within(tm.run_compact3_gate_up_forward(mods[0], mods[1], x), silu * rb, err)
+    for c in range(0, K, T):  # one column of the matrix per row: exact but for the output scale's rounding
+        col = (torch.arange(T, device="cuda") + c) % K
+        hot = torch.nn.functional.one_hot(col, K).half()
+        want = [(tm.dequantize_grouped_payload(m.payload)[0][:, col].float() * m.payload["output_scale"].float().view(O, 1)).half().t() for m in mods]
+        a, b = tm.run_compact3_gate_up_forward(mods[0], mods[1], hot, fuse_silu_mul=False)
+        assert torch.equal(mods[0](hot), want[0]) and torch.equal(a, want[0]) and torch.equal(b, want[1])
 
 
 @pytest.mark.parametrize("rows,cols,group,T", [
@@ -117,11 +143,15 @@ def test_linear_columns_shared_among_ctas(lib, O, K, T):
 ])
 def test_packed4_gemm_at_tile_edges(lib, rows, cols, group, T):
     import trismoe_b200 as tm
+    import trismoe_oracle as orc
     from trismoe_b200 import synth
 
     m = synth.packed4_matrix(np.random.default_rng(rows + T), rows, cols, group_size=group, scale_std=0.02)
     lin = tm.Packed4Linear(m, "cuda")
-    w = lin(torch.eye(cols, dtype=torch.float16, device="cuda")).t()  # single products: the weights themselves
+    w = torch.from_numpy(orc.dequantize_packed4(*(m[k].numpy() for k in ("qweight", "qzeros", "scales", "g_idx")), rows, cols)).cuda()
+    eye = torch.eye(cols, dtype=torch.float16, device="cuda")
+    for c in range(0, cols, T):  # single products: the weights themselves, at this many rows
+        assert torch.equal(lin(eye[c: c + T]), w.t()[c: c + T])
     g = torch.Generator().manual_seed(T)
     x = torch.randn((T, cols + 8), generator=g).half().cuda()
     for xi in (x[:, :cols].contiguous(), x[:, 3:3 + cols]):  # aligned rows, rows read element by element
@@ -186,6 +216,47 @@ def test_null_space_and_input_scales_in_one_sequence(lib, T, pairs, scales):
     assert own.dtype == torch.float16 and own.shape == (T, E)
 
 
+@pytest.mark.parametrize("T", [3, 37, 100])
+@pytest.mark.parametrize("packed", ["gate up down", "gate up", "down"])
+@pytest.mark.parametrize("pairs,scales", [("gate up down", "gate up down"), ("", "gate"), ("up", "up"), ("down", "gate up"), ("gate", "down"), ("gate up", "")])
+def test_null_space_and_input_scales_with_4_bit_backbones(lib, T, packed, pairs, scales):
+    """The form checkpoints arrive in: backbones kept as nibbles (up to 64 rows; routed rows cross that earlier) or
+    expanded for the call, with scales and pairs on any of the projections."""
+    import trismoe_b200 as tm
+    import trismoe_oracle as orc
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(13)
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=4)
+    E, H, I = shape.num_experts, shape.hidden_size, shape.intermediate_size
+    width = {"gate": H, "up": H, "down": I}
+    backbone = {n: synth.packed4_matrix(rng, 96, width[n], 64, scale_std=0.02) if n in packed.split() else layer["shared_" + n] for n in width}
+    vec = {n: torch.from_numpy((1 + 0.2 * rng.standard_normal(width[n])).astype(np.float16)) for n in scales.split()}
+    blk = tm.TrisSparseMoeBlock(H, I, E, shape.top_k, shape.norm_topk_prob)
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], backbone["gate"], backbone["up"], backbone["down"],
+                              layer["router_weight"], device="cuda", input_scales=vec)
+    assert set(blk.packed_backbones) == set(packed.split())
+
+    def pair(n):
+        out = H if n == "down" else I
+        ex = [None if r == 0 else {"c2": synth.packed4_matrix(rng, r, width[n], 64, scale_std=0.02),
+                                   "c1": synth.packed4_matrix(rng, out, r, 64, scale_std=0.02)} for r in (16, 0, 24, 16, 8, 40, 0, 16)]
+        return tm.build_grouped_ns_compensation_payload(ex, "cuda", torch.float16, width[n], out)
+
+    blk.load_ns_compensation_payloads(*(pair(n) if n in pairs.split() else None for n in ("gate", "up", "down")))
+    x = synth.synth_activations(T, H, seed=T).cuda().view(1, T, -1)
+    logits = synth.synth_router_logits(T, E, seed=T).cuda()
+    want, _ = blk.forward_grouped_ops(x, router_logits=logits)
+    for _ in range(2):
+        got, _ = blk(x, router_logits=logits)
+        max_abs, mean_rel = orc.error_metrics(got.float().cpu().numpy(), want.float().cpu().numpy())
+        # the roundings that one side has alone, as in the test above
+        scale = want.float().abs().max().item()
+        assert want.abs().max() > 1e-3 and max_abs <= 8 * 2.0 ** -11 * scale and mean_rel <= 4 * 2.0 ** -11, (max_abs, mean_rel, scale)
+    blk.raise_on_kernel_status()
+
+
 @pytest.mark.parametrize("E,k", [(8, 2), (40, 8), (72, 3), (200, 8)])
 @pytest.mark.parametrize("T", [1, 31, 32, 33, 65, 2100])
 def test_router_and_route_of_the_layer(lib, E, k, T):
@@ -219,6 +290,9 @@ def test_backbone_gemm_at_tile_edges(lib, n, k, m):
     w = (0.05 * torch.randn((m, k), generator=g)).half().cuda()
     ref, _, bound = _bound(w, x)
     _assert_within(tm.compute_shared_hidden(x, w), ref, bound)
+    for c in range(0, k, n):
+        col = (torch.arange(n, device="cuda") + c) % k
+        assert torch.equal(tm.compute_shared_hidden(torch.nn.functional.one_hot(col, k).half(), w), w.t()[col])
 
 
 @pytest.mark.parametrize("T", [1, 16, 70])
