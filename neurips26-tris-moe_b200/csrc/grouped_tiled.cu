@@ -168,9 +168,9 @@ struct Ring {
 };
 
 // One chunk of a pass's activation rows; src[n] = source row of row n.  A warp covers 4 rows x 128
-// contiguous bytes.  Rows that can be copied as they are go by cp.async, anything else element by element;
+// contiguous bytes.  Rows that can be copied as they are (kVec) go by cp.async, anything else by read_piece;
 // columns past the matrix read as zeros up to a multiple of 16.
-template <int N>
+template <int N, bool kVec>
 __device__ __forceinline__ void stage_rows(const TiledArgs& args, uint8_t* dst, const __half* hidden, const int* src, int rows, int c0, int tid) {
   const int p = tid & 7, n0 = tid >> 3;
   const int cols = min(kChunkCols, args.rank - c0);
@@ -180,7 +180,7 @@ __device__ __forceinline__ void stage_rows(const TiledArgs& args, uint8_t* dst, 
     const int piece = 8 * s + p, left = cols - 8 * piece;  // columns of this piece that exist
     if (left <= -8 || (left <= 0 && !(cols & 15))) return;
     uint8_t* d = dst;
-    if (args.hidden_vec) {
+    if constexpr (kVec) {
       // the row numbers of four copies first: one shared-memory round trip for all of them
       const __half* from = hidden + (left > 0 ? c0 + 8 * piece : 0);
 #pragma unroll 1
@@ -218,8 +218,9 @@ __device__ __forceinline__ void gather_salient(uint8_t* dst, const uint8_t* rows
 }
 
 // N: activation rows per pass (the accumulators' TMEM columns).  A longer segment takes several
-// passes and unpacks its weights again for each.
-template <int N, int MODE>
+// passes and unpacks its weights again for each.  kVec: rows can be copied as they are; a variant of its own, because
+// the call that reads other rows costs the kernel registers it does not have (spills; qkv 512 91 -> 94 us).
+template <int N, int MODE, bool kVec>
 __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(const __grid_constant__ TiledArgs args) {
   using W = Roles<N>;
   constexpr bool DUAL = MODE != MODE_SINGLE;
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
         }
 #pragma unroll 1
         for (int s = 0; s < args.num_sets; ++s)
-          stage_rows<N>(args, base + s * L.rows_bytes, args.hidden[s], src_rows + pass * N, w.rows(), w.c * kChunkCols, tid);
+          stage_rows<N, kVec>(args, base + s * L.rows_bytes, args.hidden[s], src_rows + pass * N, w.rows(), w.c * kChunkCols, tid);
         rows_of |= static_cast<uint32_t>(w.rows()) << (8 * ahead);
         w.next_stage(args);
         if (w.c == w.c_begin) {
@@ -763,13 +764,17 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ 
   }
 }
 
-template <int N, int MODE>
-static int launch_main(const TiledArgs& args, int grid, size_t smem, cudaStream_t stream, bool pdl) {
-  auto kernel = grouped_tiled_kernel<N, MODE>;
+template <int N, int MODE, bool kVec>
+static int launch_rows(const TiledArgs& args, int grid, size_t smem, cudaStream_t stream, bool pdl) {
+  auto kernel = grouped_tiled_kernel<N, MODE, kVec>;
   static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
   const int st = configure_smem(kernel, smem, configured);
   if (st != TRIS_OK) return st;
   return check_cuda(launch_kernel(kernel, dim3(grid), dim3(Roles<N>::kThreads), smem, stream, pdl, 1, args), "grouped_tiled_kernel launch");
+}
+template <int N, int MODE>
+static int launch_main(const TiledArgs& args, int grid, size_t smem, cudaStream_t stream, bool pdl) {
+  return args.hidden_vec ? launch_rows<N, MODE, true>(args, grid, smem, stream, pdl) : launch_rows<N, MODE, false>(args, grid, smem, stream, pdl);
 }
 
 template <int N, int MODE>
@@ -853,10 +858,9 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   a.partial = static_cast<float*>(opts.workspace);
   a.partial_bytes = opts.workspace_bytes;
   a.col_scale = static_cast<const __half*>(route->hidden_col_scale);
-  const bool in_pieces = !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 &&
-                         ((reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1])) & 15u) == 0;
-  a.hidden_vec = in_pieces && a.hidden_mode == TRIS_OUT_F16;
-  a.hidden_perm = in_pieces && a.hidden_mode != TRIS_OUT_F16;
+  const uintptr_t rows_at = reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1]);
+  a.hidden_vec = a.hidden_mode == TRIS_OUT_F16 && !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 && (rows_at & 15u) == 0;
+  a.hidden_perm = a.hidden_mode != TRIS_OUT_F16 && a.hidden_stride % 2 == 0 && (rows_at & 3u) == 0;
   a.quad_store = proj_a->out_features % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 7u) == 0;
   a.vec_store = proj_a->out_features % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 15u) == 0;
   TRIS_REQUIRE(a.col_scale == nullptr || a.hidden_mode == TRIS_OUT_F16, TRIS_ERR_INVALID_ARG,

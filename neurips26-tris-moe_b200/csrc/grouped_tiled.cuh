@@ -35,7 +35,7 @@ struct TiledArgs {
   int32_t hidden_mode;          // column order of the activation rows (TRIS_OUT_F16 / _PAIR_INTERLEAVED / _LANE_ORDER)
   int32_t hidden_stride;        // halves between activation rows
   int32_t hidden_vec;           // rows can be copied in 16-byte pieces as they are
-  int32_t hidden_perm;          // rows in a permuted order that can be read in 16-byte pieces
+  int32_t hidden_perm;          // rows in a permuted order that can be read word by word
   int32_t num_sets;             // 2 when the two projections read different activation rows
   int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
   int32_t stages;               // ring depth, 2 .. kMaxStages
@@ -48,27 +48,20 @@ struct TiledArgs {
 };
 
 // Eight columns (8 * piece ..) of an activation row that cannot be copied as it is; `left`: how many of them exist.
-// Permuted rows come in groups of 32 columns = 64 bytes: a piece is the low or high halves of two of its 16-byte words
-// (pair-interleaved), or of two 32-bit words of each of the four (lane order).  Read half by half, a single
-// projection of 64 experts x 256 rows took 157 / 188 us (pair-interleaved / lane order); now 113 / 132; row-major rows 57.
+// Permuted rows come in groups of 32 columns = 16 words of two halves 16 columns apart: a piece is the low or high
+// halves of eight of them, read word by word.  Half by half a single projection of 64 experts x 256 rows took 157 / 188 us
+// (pair-interleaved / lane order), now 118 / 135; 16-byte loads were no faster (113 / 132) and ask for more alignment.
 static __device__ __noinline__ uint4 read_piece(const TiledArgs& args, const __half* chunk, int c0, int piece, int left) {
   if (args.hidden_perm) {
     if (left <= 0) return make_uint4(0u, 0u, 0u, 0u);  // rank % 32 == 0: a group exists as a whole
-    const uint4* grp = reinterpret_cast<const uint4*>(chunk + 32 * (piece >> 2));
-    const int odd = piece & 1;
+    const uint32_t* grp = reinterpret_cast<const uint32_t*>(chunk + 32 * (piece >> 2));
     const uint32_t sel = (piece & 2) ? 0x7632u : 0x5410u;
     if (args.hidden_mode == TRIS_OUT_F16_PAIR_INTERLEAVED) {
-      const uint4 a = grp[2 * odd], b = grp[2 * odd + 1];
-      return make_uint4(prmt(a.x, a.y, sel), prmt(a.z, a.w, sel), prmt(b.x, b.y, sel), prmt(b.z, b.w, sel));
+      grp += 8 * (piece & 1);
+      return make_uint4(prmt(grp[0], grp[1], sel), prmt(grp[2], grp[3], sel), prmt(grp[4], grp[5], sel), prmt(grp[6], grp[7], sel));
     }
-    uint32_t lo[4], hi[4];  // columns u and u + 4 of the piece sit in 16-byte word u
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint4 v = grp[u];
-      lo[u] = odd ? v.x : v.y;
-      hi[u] = odd ? v.z : v.w;
-    }
-    return make_uint4(prmt(lo[0], lo[1], sel), prmt(lo[2], lo[3], sel), prmt(hi[0], hi[1], sel), prmt(hi[2], hi[3], sel));
+    grp += (piece & 1) ? 0 : 1;
+    return make_uint4(prmt(grp[0], grp[4], sel), prmt(grp[8], grp[12], sel), prmt(grp[2], grp[6], sel), prmt(grp[10], grp[14], sel));
   }
   uint32_t w[4] = {0u, 0u, 0u, 0u};
   for (int v = 0; v < 8 && v < left; ++v) {
