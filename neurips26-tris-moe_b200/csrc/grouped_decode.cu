@@ -60,7 +60,7 @@ __device__ __forceinline__ void unpack_two(uint32_t w, int i, const uint4& c, co
 
 constexpr int dec_min_ctas(int nt, int warps) { return (nt <= 2 ? 28 : 20) / warps; }
 
-// grid (groups of 32 * dec_groups outputs, segments)
+// grid (groups of 32 * dec_groups outputs, segments, CTAs that share a segment's passes)
 template <int NT, int MODE, int KS>
 __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), dec_min_ctas(NT, dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS)))
     grouped_decode_kernel(const __grid_constant__ TiledArgs args) {
@@ -82,11 +82,11 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
   const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
   // A CTA without rows leaves at once, but the first one waits: if none did, the launch could end before its predecessor.
   auto leave = [&]() {
-    if (args.weights_before_wait && blockIdx.x == 0 && blockIdx.y == 0) pdl_wait();
+    if (args.weights_before_wait && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
   };
   if (seg >= nseg) return leave();
   const int expert = args.expert_ids ? args.expert_ids[seg] : 0;  // no arrays: one segment of expert 0 with all rows
-  const int row_begin = args.expert_ids ? args.segment_offsets[seg] : 0;
+  const int row_begin = (args.expert_ids ? args.segment_offsets[seg] : 0) + static_cast<int>(blockIdx.z) * 8 * NT;
   const int row_end = args.expert_ids ? min(args.segment_offsets[seg + 1], args.num_rows) : args.num_rows;
   if (expert < 0 || expert >= args.num_experts || row_end <= row_begin) return leave();
 
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
 
   int load = 0;  // column groups loaded so far
 #pragma unroll 1
-  for (int r0 = row_begin; r0 < row_end; r0 += 8 * NT) {
+  for (int r0 = row_begin; r0 < row_end; r0 += 8 * NT * gridDim.z) {
     const int rows = min(8 * NT, row_end - r0);
     float acc[2][NT][4];
 #pragma unroll
@@ -378,16 +378,17 @@ static int launch_decode(const TiledArgs& args, cudaStream_t stream, bool pdl) {
   static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
   int st = configure_smem(kernel, smem, configured);
   if (st != TRIS_OK) return st;
-  return check_cuda(launch_kernel(kernel, dim3(ceil_div(args.out_features, kDecOut * dec_groups(P, KS)), args.num_segments), dim3(32 * dec_warps(P, KS)),
+  return check_cuda(launch_kernel(kernel, dim3(ceil_div(args.out_features, kDecOut * dec_groups(P, KS)), args.num_segments, args.row_split), dim3(32 * dec_warps(P, KS)),
                                   smem, stream, pdl, 1, args),
                     "grouped_decode_kernel launch");
 }
 
 template <int NT, int MODE>
 static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) {
-  // Fewer than 14 warps per SM: split the columns, as far as there are columns to split
-  const long long warps = static_cast<long long>(ceil_div(args.out_features, kDecOut)) * args.num_segments * (MODE == MODE_SINGLE ? 1 : 2);
-  const int slices = ceil_div(args.rank, kSliceCols), want = 14 * sm_count();
+  // Fewer than 14 warps per SM: split the columns, as far as there are columns to split.  Shared passes have the widest
+  // tile, of which 20 warps fit an SM instead of 28: fewer than 10.
+  const long long warps = decode_warps(args, MODE) * args.row_split;
+  const int slices = ceil_div(args.rank, kSliceCols), want = (args.row_split > 1 ? 10 : 14) * sm_count();
   if (warps * 4 < want && slices >= 16) return launch_decode<NT, MODE, 8>(args, stream, pdl);
   if (warps * 2 < want && slices >= 4) return launch_decode<NT, MODE, 4>(args, stream, pdl);
   if (warps < want && slices >= 4) return launch_decode<NT, MODE, 2>(args, stream, pdl);

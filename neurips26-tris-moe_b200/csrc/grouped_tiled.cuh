@@ -98,7 +98,12 @@ int configure_smem(Kernel kernel, size_t smem, std::atomic<size_t> (&configured)
 
 constexpr size_t kMostSmem = 227 * 1024;
 
-// Segments of up to `max_rows` rows; MODE_SINGLE, MODE_DUAL_STORE or MODE_DUAL_SILU.
+// Warps of a decode launch that splits neither columns nor passes.
+inline long long decode_warps(const TiledArgs& args, int mode) {
+  return static_cast<long long>((args.out_features + 31) / 32) * args.num_segments * (mode == MODE_SINGLE ? 1 : 2);
+}
+// The tile of rows follows `typical_rows`; args.row_split CTAs share the passes of a segment.  MODE_SINGLE,
+// MODE_DUAL_STORE or MODE_DUAL_SILU.
 int launch_grouped_decode(const TiledArgs& args, int mode, int typical_rows, cudaStream_t stream, bool pdl);
 constexpr int kDecodeMaxRows = 32;
 

@@ -49,6 +49,10 @@ GROUPED = [
     (1040, 320, 128, [33 + i % 32 for i in range(40)]),  # several tiles per CTA on 3 and 4 staged chunks, several passes
     (1040, 512, 128, [70] + [33 + i % 32 for i in range(39)]),
     (1040, 300, 128, [70 + 9 * i for i in range(24)]),
+    (33, 264, 128, [128, 40]),  # decode kernel, several CTAs to a segment's passes: up to 128 rows, few experts
+    (1031, 72, 32, [97, 33, 64]),
+    (64, 1040, 64, [65, 0, 31]),
+    (2048, 256, 128, [100]),
 ]
 
 
