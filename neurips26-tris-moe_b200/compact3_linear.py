@@ -52,7 +52,7 @@ class Compact3Linear(nn.Module):
 
     def _route(self, rows: int, device, partner: Optional["Compact3Linear"] = None) -> dict:
         """One segment with all rows, for this linear or a pair of them; without arrays where all have tile records."""
-        if all(isinstance(m.payload.get("_tris_tile_records"), torch.Tensor) for m in (self, partner) if m is not None):
+        if self.payload.get("_tris_tile_records") is not None and (partner is None or partner.payload.get("_tris_tile_records") is not None):
             route = {"_one_segment": True, "_max_rows_per_segment": rows}
         else:
             zero = torch.zeros((1,), dtype=torch.int32, device=device)

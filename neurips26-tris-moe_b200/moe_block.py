@@ -497,8 +497,9 @@ class TrisQwen2SparseMoeBlock(TrisSparseMoeBlock):
         if shared is None:
             raise RuntimeError("trismoe_b200: shared expert kernels returned no result")
         w = self.shared_expert_gate.weight
-        native = (routed.dtype == shared.dtype == hidden_states.dtype == w.dtype == torch.float16 and routed.is_contiguous() and w.is_contiguous()
-                  and w.shape == (1, self.hidden_size) and w.device == hidden_states.device == routed.device == shared.device
+        dev, f16 = routed.device, torch.float16
+        native = (w.dtype == hidden_states.dtype == routed.dtype == shared.dtype == f16 and w.device == dev and hidden_states.device == dev
+                  and w.shape == (1, self.hidden_size) and routed.is_contiguous() and w.is_contiguous()
                   and not (torch.is_grad_enabled() and (w.requires_grad or hidden_states.requires_grad)))
         if not native:  # torch's own checks of the gate's size and place, and its gradients
             return routed + torch.sigmoid(torch.nn.functional.linear(hidden_states, w)) * shared, logits
