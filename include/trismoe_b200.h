@@ -455,7 +455,7 @@ int tris_grouped_pair_forward(const TrisProjView* proj_a, const TrisProjView* pr
  * grouped entry points read fastest for these projections (proj_b may be NULL) and a route of
  * num_rows rows in num_segments segments of at most max_rows_per_segment rows: row-major for
  * projections with tile records and ranks that are not a multiple of 32, pair-interleaved
- * otherwise.  Ask the backbone GEMM for that out_mode and set the
+ * otherwise (the sizes make no difference at present).  Ask the backbone GEMM for that out_mode and set the
  * matching TRIS_ROUTE_HIDDEN_* flag.  No reference counterpart (the reference kernels read
  * row-major activations only).
  */
@@ -489,7 +489,8 @@ int tris_set_grouped_tc_min_rows(int32_t rows);
 
 /*
  * Upper limit on how many CTAs share the row passes of one unit (segment, two output tiles) in the
- * tiled kernel (typical segments of more than 32 rows); returns the previous value.  The
+ * tiled kernel (typical segments of more than 32 rows; where all passes of 32 rows fit the GPU at once, the decode kernel
+ * takes them side by side whatever this value); returns the previous value.  The
  * launcher splits only while there are fewer units than SMs - few local experts with long
  * segments, as on an expert-parallel rank.  Default 4; 1 switches the split off.  Results do not depend
  * on it.  Process-wide; no reference counterpart.

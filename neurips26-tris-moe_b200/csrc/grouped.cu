@@ -460,7 +460,6 @@ static int launch_grouped(const GroupedArgs& args, cudaStream_t stream, bool pdl
 
 template <int NPROJ, int EPI>
 static int dispatch_grouped(const GroupedArgs& args, int max_rows, cudaStream_t stream, bool pdl) {
-  // one 256-column chunk and no K split: persistent CTAs that prefetch their next tile
   if (max_rows <= 8) return launch_grouped<NPROJ, 1, EPI>(args, stream, pdl);
   if (max_rows <= 16) return launch_grouped<NPROJ, 2, EPI>(args, stream, pdl);
   if (max_rows <= 32) return launch_grouped<NPROJ, 4, EPI>(args, stream, pdl);

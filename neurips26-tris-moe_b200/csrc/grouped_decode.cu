@@ -1,4 +1,5 @@
-// Grouped compact3 dequant-matmul over tile records for segments of few rows (decode), on mma.sync.
+// Grouped compact3 dequant-matmul over tile records for segments of few rows (decode), on mma.sync; also for a few
+// segments of up to 128 rows, whose passes CTAs share.
 //
 // A warp owns 32 outputs of one projection and multiplies them with up to 8 NT activation rows.  Lane
 // (g, t) takes code word t of output rows g, g + 8, g + 16, g + 24: 16 columns of each of a 64-column slice.
@@ -11,9 +12,11 @@
 // Everything a CTA reads - code words, scales, tables, activation rows - is asked for at its start by
 // cp.async and read from shared memory, so that the inner loop waits for nothing further away: with the
 // same loop on L1 / L2 loads half the stall cycles were theirs.  (Bulk copies issued by the
-// lanes of a warp take turns: gate/up and down of 64 experts 5.8 / 4.8 us at 1 token against 5.6 / 4.5, 14.0 / 13.4
-// at 32 against 14.0 / 12.7, but 21.4 / 20.5 at 128 against 23.4 / 20.1.)  What bounds it now: instruction
-// issue (3.4 lane-instructions per weight plus staging and epilogue).
+// lanes of a warp take turns: gate/up and down of 64 experts, both forms timed in one run, 5.8 / 4.8 us at 1 token against
+// 5.6 / 4.5, 14.0 / 13.4 at 32 against 14.0 / 12.7, but 21.4 / 20.5 at 128 against 23.4 / 20.1.)
+// What bounds it now (128 tokens of 64 experts, 20.9 / 17.9 us): latency at four warps per scheduler.  An instruction issues
+// in 55 / 57 % of the cycles; a warp waits 21 % of its time for fixed latencies, 17 % for the loads at a unit's start, 11 %
+// for the tensor pipe.  1024 CTAs over 740 slots are 1.4 waves.
 //
 // CTAs are small (four warps, five to seven CTAs per SM), so that the units of a decode batch are nearly
 // all resident at once and SMs are evenly loaded.  With few units the columns are split over KS warps

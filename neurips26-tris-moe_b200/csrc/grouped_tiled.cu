@@ -18,9 +18,10 @@
 //                        into TMEM accumulators [128 outputs][rows];
 //   epilogue (8 warps)   accumulators -> scale / bias or SiLU(gate) * up -> fp16 rows.
 //
-// No dequantised weight leaves the SM.  What bounds it: instruction issue, of which the unpack is the
-// larger part (3.9 lane-instructions per weight, against 16 for unpacking to mma.sync fragments
-// with the Golomb-Rice decode in the loop).
+// No dequantised weight leaves the SM.  What bounds it: the roles' dependent steps, each on few warps, of which the unpack
+// is the largest (3.9 lane-instructions per weight, against 16 for unpacking to mma.sync fragments with the
+// Golomb-Rice decode in the loop).  2048 tokens of 64 experts: issue slots 58 / 55 % busy (gate/up, down), tensor pipe
+// 16 / 17 %, the MMA warps a third of their time without a free accumulator.
 // Waits on mbarriers are bounded; a time-out is reported through the route's status word and the
 // CTA leaves.
 #include <math.h>
@@ -708,8 +709,8 @@ static int row_split(long long units, int max_rows, int n) {
 // Column split of one ordinary matrix (no experts): its units of two output tiles and its row passes together are
 // too few for the SMs, and its columns many - parts of the columns go to CTAs of their own, whose fp32 sums
 // sum_parts_kernel adds in order.  4096 columns, 512 rows: 64 units for 4096 outputs (two parts), 32 for a pair of
-// 1024 (four): 108 -> 48 and 92 -> 35 us.  At least two chunks per part: the sums cost 128 KB of
-// traffic a part.
+// 1024 (four): 108 -> 48 and 92 -> 35 us.  At least two chunks per part: a part's sums are written and read once,
+// 8 bytes per row and output (16 MB for 512 x 4096).
 static int col_split(const TiledArgs& args, int mode, long long units) {
   if (args.expert_ids || !args.partial || units <= 0) return 1;
   const size_t part = sizeof(float) * static_cast<size_t>(args.num_rows) * args.out_features * (mode == MODE_SINGLE ? 1 : 2);

@@ -240,12 +240,14 @@ static int launch_umma_grouped(const GroupedArgs& args, cudaStream_t stream, boo
   return check_cuda(launch_kernel(kernel, grid, dim3(kThreads), smem, stream, pdl, 1, args), "grouped_umma_kernel launch");
 }
 
-// Rows per segment above which the launchers pick this kernel.  Measured on B200 (OLMoE- and
-// Mixtral-shaped layers, 256 to 4096 prefill tokens, up to ~1000 rows per expert): the register
-// path (eight 8-row tiles per pass, two CTAs per SM, weights re-unpacked every pass) is faster
-// throughout - 220 vs 298 us per layer at 512 tokens, 616 vs 661 at 2048 (OLMoE), 1872 vs 1935 at
-// 4096 (Mixtral) - because this kernel holds a whole SM (192 KB of shared memory) while its
-// decode-and-unpack phase runs on eight warps.  So the default sits above the measured range.
+// Rows per segment above which the launchers of payloads without tile records pick this kernel.  Against the mma.sync
+// kernel on planes (eight 8-row tiles per pass, two CTAs per SM, weights unpacked again every pass), gate/up and down:
+//   64 experts, 1024 / 2048 outputs   64 rows 94 / 108 against 57 / 54 us, 256 rows 183 / 183 against 162 / 149,
+//                                     1024 rows 590 / 566 against 572 / 529, 2048 rows 1111 / 1067 against 1114 / 1030
+//   8 experts, 14336 / 4096 outputs   64 rows 163 / 33 against 98 / 16 us, 512 rows 539 / 84 against 521 / 77,
+//                                     1024 rows 963 / 152 against 998 / 147, 2048 rows 1847 / 303 against 1953 / 287
+// It holds a whole SM (192 KB of shared memory) while its decode-and-unpack phase runs on eight warps, which only pairs of
+// long segments pay back.
 static std::atomic<int> g_tc_min_rows{2048};
 
 int grouped_tc_min_rows() { return g_tc_min_rows.load(std::memory_order_relaxed); }

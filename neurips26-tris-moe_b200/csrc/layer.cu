@@ -187,8 +187,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
     return tris_grouped_hidden_layout(&a, &b, route.num_rows, route.num_segments, route.max_rows_per_segment);
   };
   auto route_flags = [](int mode) {
-    return mode == TRIS_OUT_F16_LANE_ORDER ? TRIS_ROUTE_HIDDEN_LANE_ORDER
-                                           : (mode == TRIS_OUT_F16_PAIR_INTERLEAVED ? TRIS_ROUTE_HIDDEN_PAIR_INTERLEAVED : 0);
+    return mode == TRIS_OUT_F16_PAIR_INTERLEAVED ? TRIS_ROUTE_HIDDEN_PAIR_INTERLEAVED : 0;
   };
   const int gu_mode = hidden_mode(layer->gate, layer->up);
   const int down_mode = hidden_mode(layer->down, layer->down);

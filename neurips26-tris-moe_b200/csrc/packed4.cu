@@ -1,4 +1,4 @@
-// 4-bit packed backbone -> fp16, once at load time.
+// 4-bit packed backbone -> fp16: once at load time, or into scratch in front of a product of many rows.
 //
 // Real TriS-MoE checkpoints store the shared input-side backbone as a GPTQ-style 4-bit matrix
 // (PackedQuantMatrix4bit, qlinear_cuda.py:2668-2784): qweight [ceil(cols/8), rows] int32 holds

@@ -61,9 +61,11 @@ class TrisSparseMoeBlock(nn.Module):
         self._status_word: Optional[torch.Tensor] = None  # see _status_of
 
     # -- loading ---------------------------------------------------------------------------
-    # activation rows above which a 4-bit backbone is expanded to fp16 scratch and run on the dense GEMM
-    # (measured on B200, 2048 x 2048: the 4-bit GEMM takes 7 / 8 / 16 / 23 us at 1 / 16 / 64 / 128 rows, the
-    # expansion 4 us plus 7 / 8 / 14 / 15 us of fp16 GEMM)
+    # Activation rows above which a 4-bit backbone is expanded to fp16 scratch and run on the dense GEMM.  One matrix on
+    # B200, 4-bit GEMM against expansion and GEMM in us: 256 x 2048 6.8 / 7.0 at 1 row, 8.1 / 9.3 at 32, 11.2 / 9.9 at
+    # 64, 13.2 / 12.4 at 1024; 256 x 1024 4.7 / 6.4 at 16, 7.5 / 9.0 at 128, 8.8 / 11.0 at 1024; 256 x 4096 13.3 / 9.9 at
+    # 16; 256 x 14336 38 / 18 at 1.  So 64 rows is right for 2048 columns; fewer columns would rather stay packed up to
+    # some 1000 rows (by 1.5 us), more columns rather be expanded from the first row on.
     PACKED_BACKBONE_MAX_ROWS = 64
     _expand_scratch: dict = {}  # (device, name, shape) -> fp16 scratch shared by every block of a model
 
@@ -81,8 +83,8 @@ class TrisSparseMoeBlock(nn.Module):
         ``input_scales`` (``{"gate" | "up" | "down": fp16 [in]}``): the vector null-space input scale of
         ``ns_mode == 1`` checkpoints (``expert_input_scale`` of expert 0, qlinear_cuda.py:3918-3923): the
         backbone of that projection sees ``x * scale`` rounded to fp16 (qlinear_cuda.py:4477-4480); the
-        matching output scale travels in the payload (``output_scale``).  With input scales the block
-        runs operator by operator (gate and up no longer share their input rows)."""
+        matching output scale travels in the payload (``output_scale``).  A scaled projection's
+        backbone is a launch of its own (gate and up no longer share their input rows)."""
         import os
 
         dev = torch.device(device) if device is not None else gate["qweight1"].device
@@ -125,7 +127,7 @@ class TrisSparseMoeBlock(nn.Module):
         """Attaches the grouped null-space compensation payloads of ``ns_mode == 2`` checkpoints (the
         ``gate_ns`` / ``up_ns`` / ``down_ns`` entries of the reference's payload cache,
         modeling_olmoe.py:950-975; built by ``build_grouped_ns_compensation_payload``).  With any of
-        them the block runs operator by operator and each grouped operator adds its compensation."""
+        them the layer's launch sequence gains the products of the pairs (``tris_moe_layer_forward_extras``)."""
         from .ns_compensation import ns_payload_max_rank
 
         self.ns_payloads = {n: p for n, p in (("gate", gate_ns), ("up", up_ns), ("down", down_ns))
