@@ -45,7 +45,7 @@ HEADLINE_TOKENS = 128
 SWEEP_TOKENS = (1, 8, 32, 128)
 NOMINAL_HBM_GBS = 8000.0
 FALLBACK_HBM_GBS = 6650.0
-LAUNCHES_PER_LAYER = 7  # backbone+router GEMM, top-k, route, gate/up, down backbone, down, combine
+LAUNCHES_PER_LAYER = 7  # backbone+router GEMM, router masks, route, gate/up, down backbone, down, combine
 
 
 KERNEL_SOURCES = ("grouped_decode.cu", "grouped_tiled.cuh", "tile_records.cuh", "tile_records.cu")  # what the dominant kernel is built from
