@@ -14,7 +14,7 @@
 // same loop on L1 / L2 loads half the stall cycles were theirs.  (Bulk copies issued by the
 // lanes of a warp take turns: gate/up and down of 64 experts, both forms timed in one run, 5.8 / 4.8 us at 1 token against
 // 5.6 / 4.5, 14.0 / 13.4 at 32 against 14.0 / 12.7, but 21.4 / 20.5 at 128 against 23.4 / 20.1.)
-// What bounds it now (128 tokens of 64 experts, 20.9 / 17.9 us): latency at four warps per scheduler.  An instruction issues
+// What bounds it now (128 tokens of 64 experts, 20.9 / 18.6 us): latency at four warps per scheduler.  An instruction issues
 // in 55 / 57 % of the cycles; a warp waits 21 % of its time for fixed latencies, 17 % for the loads at a unit's start, 11 %
 // for the tensor pipe.  1024 CTAs over 740 slots are 1.4 waves.
 //
