@@ -477,8 +477,8 @@ def streaming_records(blocks, manager, shape, device):
     from trismoe_b200 import staging, synth
 
     n_layers, H = len(blocks), shape.hidden_size
-    per_expert = [sum(manager.entries[(l, p)].block_bytes[k] for p in staging.PROJECTIONS
-                      for k in manager.entries[(l, p)].block_bytes) for l in range(n_layers)]
+    per_expert = [sum(manager.entries[(l, p)].link_bytes[k] for p in staging.PROJECTIONS
+                      for k in manager.entries[(l, p)].link_bytes) for l in range(n_layers)]
     recs = []
     for T in (1, 16):
         x = synth.synth_activations(T, H, seed=T).to(device)

@@ -525,6 +525,28 @@ int tris_page_experts(const TrisPageJob* jobs, int32_t num_jobs, const int32_t* 
                       const int32_t* num_segments_dev, int32_t num_segments, int32_t num_experts,
                       int32_t* slot_table, void* stream);
 
+/* One tensor to page that lies on the host in coded blocks (tris_page_code_blocks).  Expert e's block b starts at 16-byte
+   unit block_offsets[e * blocks + b] of host_src and ends where the next one starts; blocks = bytes_per_expert / 1024, rounded up. */
+typedef struct TrisCodedPageJob {
+  const void* host_src;           /* pinned, device-accessible host memory                        */
+  const int32_t* block_offsets;   /* device, [E * blocks + 1]                                     */
+  void* dst;                      /* device staging buffer, [slots, bytes_per_expert]             */
+  int64_t bytes_per_expert;       /* decoded, a multiple of 16                                    */
+} TrisCodedPageJob;
+#define TRIS_PAGE_BLOCK_BYTES 1024
+
+/*
+ * Codes an E-stacked device tensor of sparse bits, [E, bytes_per_expert], in blocks of 1024 bytes.  First call with
+ * block_offsets NULL: writes the size of every block in 16-byte units, 0 to 64, to units_out [E * blocks].  Second call with
+ * their exclusive sums ([E * blocks + 1]): writes the code to dst_dev.  bytes_per_expert is a multiple of 16.
+ */
+int tris_page_code_blocks(const void* src_dev, int64_t bytes_per_expert, int32_t num_experts, int32_t* units_out,
+                          const int32_t* block_offsets, void* dst_dev, void* stream);
+/* tris_page_experts for coded tensors: the blocks are decoded on their way into the staging buffer. */
+int tris_page_coded_experts(const TrisCodedPageJob* jobs, int32_t num_jobs, const int32_t* expert_ids,
+                            const int32_t* num_segments_dev, int32_t num_segments, int32_t num_experts,
+                            int32_t* slot_table, void* stream);
+
 /*
  * tris_grouped_forward (proj_b NULL) and tris_grouped_pair_forward with scratch, for an ordinary matrix (a route
  * without arrays) of more than a few rows: with it the columns of the matrix can be shared among CTAs too.  The

@@ -39,6 +39,10 @@ class TrisPageJob(C.Structure):
     _fields_ = [("host_src", _vp), ("dst", _vp), ("bytes_per_expert", C.c_int64)]
 
 
+class TrisCodedPageJob(C.Structure):
+    _fields_ = [("host_src", _vp), ("block_offsets", _vp), ("dst", _vp), ("bytes_per_expert", C.c_int64)]
+
+
 ABI_VERSION = 4  # TRIS_B200_ABI_VERSION of include/trismoe_b200.h
 
 
@@ -119,6 +123,8 @@ SIGNATURES = {
     "tris_combine_routed": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp, _vp]),
     "tris_shared_expert_add": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp]),
     "tris_page_experts": (C.c_int, [_vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp]),
+    "tris_page_code_blocks": (C.c_int, [_vp, C.c_int64, _i32, _vp, _vp, _vp, _vp]),
+    "tris_page_coded_experts": (C.c_int, [_vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp]),
     "tris_moe_layer_workspace_bytes": (C.c_size_t, [_P(TrisMoeLayerView), _i32]),
     "tris_moe_layer_last_status": (C.c_int, [_vp, _i32, _vp, _P(_i32)]),
     "tris_moe_layer_forward": (C.c_int, [_P(TrisMoeLayerView), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp]),

@@ -5,8 +5,8 @@ Role of ``GroupedQGmapCPUStagingManager`` (``grouped_payload_sidecar.py:764-1146
 TriS-MoE tree), with two modes:
 
 ``mode="bitmap"``   what the reference streams: only the sparse grouping bitmap
-                    ``q_gmap_sparse`` of every projection leaves the GPU (README:281-283);
-                    signs and scales stay resident.  Payloads must use the sparse bitmap
+                    ``q_gmap_sparse`` of every projection leaves the GPU (README:281-283), coded at
+                    half its size; signs and scales stay resident.  Payloads must use the sparse bitmap
                     format (``compact3_use_block_gr = False``).
 ``mode="payload"``  every bulky per-expert tensor (sign planes, bitmap or block-GR stream and
                     its index, scale packs) lives in pinned host memory; only the small
@@ -34,22 +34,27 @@ from typing import Optional
 import torch
 
 from . import _native
-from ._native import TrisPageJob
+from ._native import TrisCodedPageJob, TrisPageJob
 from .qlinear_grouped import proj_view
 
 BITMAP_KEYS = ("q_gmap_sparse",)
 PAYLOAD_KEYS = ("qweight1", "qweight2_sparse", "q_gmap_sparse", "q_gmap_gr_words", "_tris_gr_index", "col_pack3", "row_pack3")
 PROJECTIONS = ("gate", "up", "down")
 MAX_PAGE_JOBS = 16  # TRIS_MAX_PAGE_JOBS of the C header
+PAGE_BLOCK_BYTES = 1024  # TRIS_PAGE_BLOCK_BYTES
 
 
 class _Entry:
-    """One projection of one layer: pinned host tensors and their per-expert block sizes."""
+    """One projection of one layer: pinned host tensors and their per-expert block sizes.  A sparse bitmap lies on the
+    host in coded blocks (``tris_page_code_blocks``) where that makes it smaller."""
 
     def __init__(self, payload: dict, keys):
         self.payload = payload
         self.host = {}
-        self.block_bytes = {}
+        self.block_bytes = {}  # of an expert's block in a staging slot
+        self.link_bytes = {}   # the same on its way over the host link: of the largest expert
+        self.coded = {}        # key -> device offsets of the coded blocks
+        self.rows = {}         # key -> second dimension of the tensor
         E = int(payload["qweight1"].shape[0])
         for key in keys:
             t = payload.get(key)
@@ -59,17 +64,42 @@ class _Entry:
             if per == 0:
                 continue
             shape = list(t.shape)
+            self.rows[key] = int(shape[1])
             if per % 16:
                 # only a 2-D stream (block-GR words) can be ragged: pad each expert's row with zeros
                 if t.dim() != 2 or (16 % t.element_size()):
                     raise RuntimeError(f"trismoe_b200 staging: {key} has {per} bytes per expert, not a multiple of 16")
                 step = 16 // t.element_size()
-                shape[1] = (shape[1] + step - 1) // step * step
+                shape[1] = self.rows[key] = (shape[1] + step - 1) // step * step
                 per = shape[1] * t.element_size()
+            self.block_bytes[key] = self.link_bytes[key] = per
+            if key == "q_gmap_sparse" and t.is_cuda and self._code(key, t.contiguous(), E, per):
+                continue
             host = torch.zeros(shape, dtype=t.dtype, pin_memory=True)
             host[tuple(slice(0, d) for d in t.shape)].copy_(t)
             self.host[key] = host
-            self.block_bytes[key] = per
+
+    def _code(self, key: str, t: torch.Tensor, experts: int, per: int) -> bool:
+        """Codes a bitmap; False where the code would not be at least an eighth smaller."""
+        if t.data_ptr() % 16 or experts * -(-per // PAGE_BLOCK_BYTES) * 64 > 0x7FFFFFFF:
+            return False
+        lib, blocks = _native.load(), -(-per // PAGE_BLOCK_BYTES)
+        offsets = torch.zeros((experts * blocks + 1,), dtype=torch.int32, device=t.device)
+        with torch.cuda.device(t.device):
+            stream = torch.cuda.current_stream(t.device).cuda_stream
+            units = torch.empty((experts * blocks,), dtype=torch.int32, device=t.device)
+            _native.check(lib.tris_page_code_blocks(t.data_ptr(), per, experts, units.data_ptr(), None, None, stream), "page_code_blocks")
+            torch.cumsum(units, 0, dtype=torch.int32, out=offsets[1:])
+            ends = offsets[::blocks]
+            total, most = torch.stack([ends[-1], (ends[1:] - ends[:-1]).max()]).tolist()
+            if total * 16 * 8 > experts * per * 7:
+                return False
+            code = torch.empty((max(1, total) * 16,), dtype=torch.uint8, device=t.device)
+            _native.check(lib.tris_page_code_blocks(t.data_ptr(), per, experts, None, offsets.data_ptr(), code.data_ptr(), stream), "page_code_blocks")
+        host = torch.empty(code.shape, dtype=torch.uint8, pin_memory=True)
+        host.copy_(code)
+        self.host[key], self.coded[key], self.link_bytes[key] = host, offsets, most * 16
+        return True
 
 
 def staging_requested() -> bool:
@@ -204,9 +234,10 @@ class GroupedQGmapCPUStagingManager:
                 start.record(copy)
             # gate and up go in one launch (they are needed together and share a slot table), down in a second one
             # that runs while the gate/up kernel computes
-            for jobs, count, per_segment, last_of_gate_up, table in launches:
+            for coded, jobs, count, per_segment, last_of_gate_up, table in launches:
                 self.pipeline_stats["bytes"] += nseg_bound * per_segment
-                _native.check(lib.tris_page_experts(jobs, count, ids, counts, nseg_bound, experts, table, copy.cuda_stream), "page_experts")
+                page = lib.tris_page_coded_experts if coded else lib.tris_page_experts
+                _native.check(page(jobs, count, ids, counts, nseg_bound, experts, table, copy.cuda_stream), "page_experts")
                 self.pipeline_stats["chunks"] += 1
                 if last_of_gate_up:  # the gate/up kernel may start while down is still paged
                     self._paged_gu[ring].record(copy)
@@ -218,7 +249,7 @@ class GroupedQGmapCPUStagingManager:
         return _PagedLayer(self, ring, views, start, end)
 
     def _plan(self, block_index: int, ring: int):
-        """Pager launches ``(jobs, count, bytes per segment, ends gate/up, slot table)`` and staged views of a
+        """Pager launches ``(coded, jobs, count, bytes per segment, ends gate/up, slot table)`` and staged views of a
         layer in a ring slot, laid out on first use and again when a projection's own view has other contents
         (an object's identity would miss a view edited in place, and one built at a freed view's address)."""
         bases = tuple(bytes(proj_view(self.entries[(block_index, proj)].payload)) for proj in PROJECTIONS)
@@ -227,18 +258,20 @@ class GroupedQGmapCPUStagingManager:
             return plan[1], plan[2]
         launches, views = [], {}
         for group in (("gate", "up"), ("down",)):
-            pairs = [(proj, key) for proj in group for key in self.entries[(block_index, proj)].host]
-            table = self.slot_tables[ring][group[0]]
-            for lo in range(0, len(pairs), MAX_PAGE_JOBS):
-                part = pairs[lo: lo + MAX_PAGE_JOBS]
-                jobs = (TrisPageJob * len(part))()
+            table, entry_of, parts = self.slot_tables[ring][group[0]], lambda proj: self.entries[(block_index, proj)], []
+            for coded in (False, True):
+                pairs = [(proj, key) for proj in group for key in entry_of(proj).host if (key in getattr(entry_of(proj), "coded", ())) == coded]
+                parts += [(coded, pairs[lo: lo + MAX_PAGE_JOBS]) for lo in range(0, len(pairs), MAX_PAGE_JOBS)]
+            for i, (coded, part) in enumerate(parts):
+                jobs = ((TrisCodedPageJob if coded else TrisPageJob) * len(part))()
                 for j, (proj, key) in enumerate(part):
-                    entry = self.entries[(block_index, proj)]
-                    jobs[j].host_src = entry.host[key].data_ptr()
+                    jobs[j].host_src = entry_of(proj).host[key].data_ptr()
                     jobs[j].dst = self.buffers[(ring, proj, key)].data_ptr()
-                    jobs[j].bytes_per_expert = entry.block_bytes[key]
-                per_segment = sum(self.entries[(block_index, proj)].block_bytes[key] for proj, key in part)
-                launches.append((jobs, len(part), per_segment, group[0] == "gate" and lo + MAX_PAGE_JOBS >= len(pairs), table.data_ptr()))
+                    jobs[j].bytes_per_expert = entry_of(proj).block_bytes[key]
+                    if coded:
+                        jobs[j].block_offsets = entry_of(proj).coded[key].data_ptr()
+                per_segment = sum(getattr(entry_of(proj), "link_bytes", entry_of(proj).block_bytes)[key] for proj, key in part)
+                launches.append((coded, jobs, len(part), per_segment, group[0] == "gate" and i + 1 == len(parts), table.data_ptr()))
             for proj in group:
                 views[proj] = self._staged_view(self.entries[(block_index, proj)], ring, proj, table)
         self._plans[(block_index, ring)] = (bases, launches, views)
@@ -254,15 +287,16 @@ class GroupedQGmapCPUStagingManager:
                  "row_pack3": "row_pack3"}
         for key in entry.host:
             setattr(view, field[key], self.buffers[(ring, proj, key)].data_ptr())
+        rows = lambda key: entry.rows[key] if key in getattr(entry, "rows", ()) else int(entry.host[key].shape[1])
         if self.mode == "bitmap":
             view.gmap_slot = table.data_ptr()
-            view.gmap_sparse_rows = int(entry.host["q_gmap_sparse"].shape[1])
+            view.gmap_sparse_rows = rows("q_gmap_sparse")
         else:
             view.expert_slot = table.data_ptr()
             if "q_gmap_sparse" in entry.host:
-                view.gmap_sparse_rows = int(entry.host["q_gmap_sparse"].shape[1])
+                view.gmap_sparse_rows = rows("q_gmap_sparse")
             if "q_gmap_gr_words" in entry.host:
-                view.gr_max_words = int(entry.host["q_gmap_gr_words"].shape[1])
+                view.gr_max_words = rows("q_gmap_gr_words")
         return view
 
     # -- reporting -----------------------------------------------------------------------------

@@ -1,0 +1,61 @@
+"""Coded pages: every bit of a bitmap comes back, at block edges, at all densities and without code where that is larger."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _code(lib, bits, per):
+    E, blocks = bits.shape[0], -(-per // 1024)
+    units = torch.empty((E * blocks,), dtype=torch.int32, device="cuda")
+    assert lib.tris_page_code_blocks(bits.data_ptr(), per, E, units.data_ptr(), None, None, None) == 0
+    offsets = torch.nn.functional.pad(units.cumsum(0, dtype=torch.int32), (1, 0)).to(torch.int32).contiguous()
+    code = torch.empty((max(1, int(offsets[-1])) * 16,), dtype=torch.uint8, device="cuda")
+    assert lib.tris_page_code_blocks(bits.data_ptr(), per, E, None, offsets.data_ptr(), code.data_ptr(), None) == 0
+    host = torch.empty(code.shape, dtype=torch.uint8, pin_memory=True)
+    host.copy_(code)
+    return host, offsets, units.view(E, blocks)
+
+
+@pytest.mark.parametrize("per", [16, 1008, 1024, 1040, 9 * 1024 + 528])
+def test_every_bit_comes_back(lib, per):
+    import trismoe_b200 as tm
+
+    E, slots = 9, 5
+    g = torch.Generator(device="cuda").manual_seed(per)
+    density = torch.tensor([0.0, 1.0, 0.1, 0.02, 0.3, 0.5, 0.001, 0.1, 0.9], device="cuda")
+    dense = torch.rand((E, per, 8), generator=g, device="cuda") < density.view(E, 1, 1)
+    dense[7] = False
+    dense[7, 0, 0] = dense[7, -1, 7] = True  # the first and the last bit
+    bits = (dense.to(torch.int32) << torch.arange(8, device="cuda")).sum(2).to(torch.uint8)
+    host, offsets, units = _code(lib, bits, per)
+    assert (units[0] == 0).all() and (units[1, : per // 1024] == 64).all()  # nothing; left as it is
+    if per >= 1024:
+        assert 30 <= units[2].float()[: per // 1024].mean() <= 36  # half the size at one bit in ten
+    ids = torch.tensor([8, 2, -1, 0, 7, 1, 4, 3, 5, 6], dtype=torch.int32, device="cuda")  # more experts than slots
+    count = torch.tensor([ids.numel()], dtype=torch.int32, device="cuda")
+    dst = torch.full((slots, per), 0xAA, dtype=torch.uint8, device="cuda")
+    table = torch.zeros((E,), dtype=torch.int32, device="cuda")
+    jobs = (tm._native.TrisCodedPageJob * 1)()
+    jobs[0].host_src, jobs[0].block_offsets, jobs[0].dst, jobs[0].bytes_per_expert = host.data_ptr(), offsets.data_ptr(), dst.data_ptr(), per
+    assert lib.tris_page_coded_experts(jobs, 1, ids.data_ptr(), count.data_ptr(), slots, E, table.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    want_table = [-1] * E
+    for s, e in enumerate(ids.tolist()[:slots]):
+        if e >= 0:
+            want_table[e] = s
+            assert torch.equal(dst[s], bits[e]), (s, e)
+        else:
+            assert (dst[s] == 0xAA).all()
+    assert table.tolist() == want_table
+    # an expert in every slot in turn, so that each is decoded
+    for lo in range(0, E, slots):
+        part = torch.arange(lo, min(E, lo + slots), dtype=torch.int32, device="cuda")
+        assert lib.tris_page_coded_experts(jobs, 1, part.data_ptr(), None, part.numel(), E, table.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(dst[: part.numel()], bits[part.long()])
+    bad = (tm._native.TrisCodedPageJob * 1)()
+    assert lib.tris_page_coded_experts(bad, 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
+    assert lib.tris_page_coded_experts(C.cast(None, C.c_void_p), 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
