@@ -52,15 +52,6 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
   return d;
 }
 
-// Two half2 (columns 2i .. 2i + 3 of a code word) of one output; c = {d, nd} scale words of the two pairs.
-__device__ __forceinline__ void unpack_two(uint32_t w, int i, const uint4& c, const RowScales& rs, uint32_t& a, uint32_t& b) {
-  const uint32_t t0 = w << i, t1 = w << (i + 1);
-  const uint32_t d0 = h2_as_u32(__hmul2_rn(u32_as_h2(c.x), rs.rd)), n0 = h2_as_u32(__hmul2_rn(u32_as_h2(c.y), rs.rn));
-  const uint32_t d1 = h2_as_u32(__hmul2_rn(u32_as_h2(c.z), rs.rd)), n1 = h2_as_u32(__hmul2_rn(u32_as_h2(c.w), rs.rn));
-  a = flip_by_sign(lop3_select(d0, n0, prmt(t0, 0u, 0xAA88u)), t0);
-  b = flip_by_sign(lop3_select(d1, n1, prmt(t1, 0u, 0xAA88u)), t1);
-}
-
 constexpr int dec_min_ctas(int nt, int warps) { return (nt <= 2 ? 28 : 20) / warps; }
 
 // grid (groups of 32 * dec_groups outputs, segments, CTAs that share a segment's passes)
@@ -222,8 +213,8 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
 #pragma unroll
               for (int m = 0; m < 2; ++m) {
                 uint32_t a0, a1, a2, a3;
-                unpack_two(cur[2 * m], 4 * jj + 2 * j, cs, rs[2 * m], a0, a2);
-                unpack_two(cur[2 * m + 1], 4 * jj + 2 * j, cs, rs[2 * m + 1], a1, a3);
+                unpack_two(cur[2 * m] << (4 * jj + 2 * j), cur[2 * m] << (4 * jj + 2 * j + 1), cs, rs[2 * m], a0, a2);
+                unpack_two(cur[2 * m + 1] << (4 * jj + 2 * j), cur[2 * m + 1] << (4 * jj + 2 * j + 1), cs, rs[2 * m + 1], a1, a3);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt)
                   mma_m16n8k16(acc[m][nt], a0, a1, a2, a3, j ? bf[nt].z : bf[nt].x, j ? bf[nt].w : bf[nt].y);

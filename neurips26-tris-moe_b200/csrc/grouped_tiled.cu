@@ -800,6 +800,39 @@ static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool 
                     "sum_parts_kernel launch");
 }
 
+// Whether the weights-resident kernel is the faster one.  It pays about 5 us to start and its row tiles are 128 rows wide
+// whatever a segment has; the tiled kernel unpacks a segment's weights again for every pass, of 64 rows where that is typical.
+// us, tiled / wide, 64 experts, gate/up and down: 256 tokens (44 typical rows) 21.4 / 31.4, 21.6 / 26.3; 384 (62: tails of
+// 64-row passes) 35.3 / 32.2, 35.6 / 26.8; 509 (80) 28.2 / 32.4, 27.0 / 27.4; 700 (106) 46.1 / 36.7, 42.8 / 28.3; 2048 (288)
+// 93.5 / 56.7, 90.0 / 43.0.  One chunk of columns, 400 and 1000 tokens: 18.4 / 26.9, 17.6 / 20.4; 31.3 / 33.7, 34.1 / 24.6.  Three
+// chunks, 400 tokens: 46.4 / 37.4, 31.2 / 31.0.  As many segments as SMs are uneven whatever their mean: 256 experts, 256 and
+// 2048 tokens (43, 80) 56.4 / 48.6, 96.9 / 67.5; 69.7 / 56.8, 127 / 78.
+static bool wide_is_faster(const TiledArgs& args, int mode, int typical_rows) {
+  if (args.chunks == 1) return typical_rows > (mode == MODE_SINGLE ? 96 : 160);
+  if (typical_rows > 96 || args.num_segments >= sm_count()) return true;
+  if (typical_rows <= 56) return false;
+  // a few large experts are even, and their tails short: 8 experts, 192 tokens (62), the block 76 / 91
+  if (args.num_segments >= 32) return args.chunks > kWideChunks || typical_rows <= 64;
+  return args.chunks > kWideChunks && !args.expert_ids;  // 4096 columns, 100 rows: 21.1 / 18.8, a pair 24.2 / 22.5
+}
+template <int MODE>
+static int launch_wide(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {
+  const long long units = static_cast<long long>(args.units_x) * args.num_segments;
+  args.row_split = row_split(units, max_rows, args.chunks <= kWideChunks ? 128 : 256);
+  args.col_split = col_split(args, MODE, units * args.row_split);
+  args.resident = ceil_div(args.chunks, args.col_split) <= kWideChunks;
+  args.unit_cost = MODE == MODE_SINGLE ? 2 : 1;  // unpacking a unit against a row tile, whose SiLU is the longer epilogue (44.7 / 34.4 us, 45.9 / 37.6 us the other way round: 1024 tokens)
+  if (args.col_split == 1) args.partial = nullptr;
+  const int grid = static_cast<int>(std::min<long long>(units * args.row_split * args.col_split, sm_count()));
+  if (!args.partial) return launch_grouped_wide(args, MODE, grid, stream, pdl);
+  // parts of gate and up are stored apart; the sum kernel applies SiLU * up
+  const int st = launch_grouped_wide(args, MODE == MODE_DUAL_SILU ? MODE_DUAL_STORE : MODE, grid, stream, pdl);
+  if (st != TRIS_OK) return st;
+  const long long quads = static_cast<long long>(args.num_rows) * ceil_div(args.out_features, 4);
+  return check_cuda(launch_kernel(sum_parts_kernel<MODE>, dim3(static_cast<unsigned>((quads + 255) / 256)), dim3(256), 0, stream, /*pdl=*/true, 1, args),
+                    "sum_parts_kernel launch");
+}
+
 template <int MODE>
 static int dispatch_tiled(TiledArgs& args, int max_rows, int typical_rows, cudaStream_t stream, bool pdl) {
   args.units_x = MODE == MODE_SINGLE ? (args.tiles + 1) / 2 : args.tiles;
@@ -814,6 +847,7 @@ static int dispatch_tiled(TiledArgs& args, int max_rows, int typical_rows, cudaS
     args.row_split = passes;
     return launch_grouped_decode(args, MODE, kDecodeMaxRows, stream, pdl);
   }
+  if (wide_is_faster(args, MODE, typical_rows)) return launch_wide<MODE>(args, max_rows, stream, pdl);
   // two stages of the widest pass have to fit shared memory (many salient columns make a stage larger)
   if (typical_rows <= 64 || 2 * stage_bytes<MODE>(args, 128) + kHeadBytes > kMostSmem) return launch_tiled<64, MODE>(args, max_rows, stream, pdl);
   return launch_tiled<128, MODE>(args, max_rows, stream, pdl);

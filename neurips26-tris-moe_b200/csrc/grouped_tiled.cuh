@@ -1,6 +1,6 @@
-// What the two tile-record kernels share: launch arguments, result stores, host helpers.
+// What the tile-record kernels share: launch arguments, result stores, host helpers.
 // grouped_decode.cu: few rows per segment, many small CTAs; grouped_tiled.cu: wide passes, persistent
-// warp-specialised CTAs.
+// warp-specialised CTAs; grouped_wide.cu: the same with a segment's weights kept in shared memory.
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -40,6 +40,9 @@ struct TiledArgs {
   int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
   int32_t stages;               // ring depth, 2 .. kMaxStages
   int32_t reuse;                // the chunks of a pass fit the ring: staged once for all tiles of a run
+  int32_t rows_by_tensor;       // wide kernel: contiguous activation rows come by tensor copies
+  int32_t unit_cost;            // wide kernel: what a unit costs once, in row tiles
+  int32_t resident;             // wide kernel: the weights of a unit's columns fit shared memory together
   int32_t vec_store;            // 16-byte stores of eight outputs are aligned
   int32_t quad_store;           // 8-byte stores of four outputs are aligned
   float* partial;               // fp32 sums of the column parts, or null: no column split
@@ -106,6 +109,9 @@ inline long long decode_warps(const TiledArgs& args, int mode) {
 // MODE_DUAL_STORE or MODE_DUAL_SILU.
 int launch_grouped_decode(const TiledArgs& args, int mode, int typical_rows, cudaStream_t stream, bool pdl);
 constexpr int kDecodeMaxRows = 32;
+// args.units_x, row_split, col_split, unit_cost and resident are set.
+int launch_grouped_wide(const TiledArgs& args, int mode, int grid, cudaStream_t stream, bool pdl);
+constexpr int kWideChunks = 2;  // chunks of 128 columns whose weights it can keep in shared memory
 
 }  // namespace tr
 }  // namespace tris

@@ -14,7 +14,6 @@
 // Every mbarrier wait is bounded; a time-out frees the TMEM allocation and reports
 // TRIS_ERR_TIMEOUT through the status word.
 #include <cooperative_groups.h>
-#include <cuda.h>  // CUtensorMap and its enums; cuTensorMapEncodeTiled itself comes from the driver entry point
 
 #include <algorithm>
 #include <atomic>
@@ -303,13 +302,6 @@ struct TcTmaSmem {  // at a 1024-byte boundary
   int32_t timed_out;
 };
 
-__device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                   smem_u32(dst_smem)),
-               "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-               : "memory");
-}
-
 template <int NTILE>
 __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_constant__ TcGemmArgs args,
                                                                    const __grid_constant__ TcTmaMaps maps) {
@@ -443,13 +435,11 @@ static EncodeTiledFn encode_tiled_fn() {
   return reinterpret_cast<EncodeTiledFn>(cached.load(std::memory_order_acquire));
 }
 
-// Describes the row-major fp16 matrix [rows, k]; one copy = one 64-column chunk of box_rows rows,
-// 128-byte-swizzled.
-static bool encode_operand_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
+bool encode_rows_map(CUtensorMap* map, const void* base, int rows, int cols, int stride, int box_rows) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr || rows <= 0) return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};  // bytes, dimension 1
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(stride) * 2};  // bytes, dimension 1
   const cuuint32_t box[2] = {kTcKChunk, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
@@ -509,8 +499,8 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
   args.k_per_cta = ceil_div(ceil_div(k, ksplit), kTcKChunk) * kTcKChunk;
   if (row_gather == nullptr) {  // operands by tensor copies
     TcTmaMaps maps;
-    bool ok = encode_operand_map(&maps.x, x, n, k, ntile);
-    for (int i = 0; i < num_problems && ok; ++i) ok = encode_operand_map(&maps.a[i], probs[i].a, probs[i].m, k, kTcM);
+    bool ok = encode_rows_map(&maps.x, x, n, k, k, ntile);
+    for (int i = 0; i < num_problems && ok; ++i) ok = encode_rows_map(&maps.a[i], probs[i].a, probs[i].m, k, k, kTcM);
     if (ok) {
       if (ntile == 64) return launch_umma_tma<64>(args, maps, mtiles, ksplit, stream, pdl);
       return launch_umma_tma<128>(args, maps, mtiles, ksplit, stream, pdl);

@@ -158,6 +158,15 @@ __device__ __forceinline__ uint32_t flip_by_sign(uint32_t v, uint32_t t) {
   return d;
 }
 
+// Two half2 (columns 2i .. 2i + 3 of a code word w) of one output; t0 = w << i, t1 = w << (i + 1), c = {d, nd} scale words of
+// the two pairs.
+__device__ __forceinline__ void unpack_two(uint32_t t0, uint32_t t1, const uint4& c, const RowScales& rs, uint32_t& a, uint32_t& b) {
+  const uint32_t d0 = h2_as_u32(__hmul2_rn(u32_as_h2(c.x), rs.rd)), n0 = h2_as_u32(__hmul2_rn(u32_as_h2(c.y), rs.rn));
+  const uint32_t d1 = h2_as_u32(__hmul2_rn(u32_as_h2(c.z), rs.rd)), n1 = h2_as_u32(__hmul2_rn(u32_as_h2(c.w), rs.rn));
+  a = flip_by_sign(lop3_select(d0, n0, prmt(t0, 0u, 0xAA88u)), t0);
+  b = flip_by_sign(lop3_select(d1, n1, prmt(t1, 0u, 0xAA88u)), t1);
+}
+
 // 16 columns (code word i of a slice) -> 8 half2 in column order.  ct: the slice's scale table + i.
 __device__ __forceinline__ void unpack_word(uint32_t w, const uint4* ct, const RowScales& rs, uint32_t* a) {
 #pragma unroll

@@ -5,6 +5,8 @@
 // (k/8) * ROWS * 16 + row * 16 + (k%8) * 2; SBO = 128 B between 8-row groups, LBO = ROWS * 16 B
 // between 8-column K chunks).
 #pragma once
+#include <cuda.h>  // CUtensorMap and its enums; cuTensorMapEncodeTiled itself comes from the driver entry point
+
 #include "common.cuh"
 
 namespace tris {
@@ -56,16 +58,20 @@ __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fe
 
 // 32 lanes x 16 consecutive 32-bit columns of the accumulator: thread t of the warp gets lane
 // (taddr.lane + t), registers = columns.
+// The wait is part of the statement: nothing may touch the registers before it, not even a spill.
 __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+               : "r"(taddr)
+               : "memory");
+}
+// Two of them with one wait.
+__device__ __forceinline__ void tmem_ld_16_pair(uint32_t taddr_v, uint32_t taddr_w, float (&v)[16], float (&w)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]), "=f"(w[4]), "=f"(w[5]), "=f"(w[6]), "=f"(w[7]), "=f"(w[8]), "=f"(w[9]), "=f"(w[10]), "=f"(w[11]), "=f"(w[12]), "=f"(w[13]), "=f"(w[14]), "=f"(w[15])
+               : "r"(taddr_v), "r"(taddr_w)
+               : "memory");
 }
 
 template <int COUNT>
@@ -130,6 +136,14 @@ __device__ __forceinline__ void stage_operand_async(uint8_t* dst, const __half* 
   }
 }
 
+__device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                   smem_u32(dst_smem)),
+               "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+               : "memory");
+}
+// Describes row-major fp16 rows of `cols` columns, `stride` halves apart (multiples of 8, `base` at a 16-byte boundary);
+// one copy = one 64-column chunk of box_rows rows, 128-byte-swizzled, zeros past the matrix (tc_gemm.cu).
+bool encode_rows_map(CUtensorMap* map, const void* base, int rows, int cols, int stride, int box_rows);
 
 }  // namespace tris
-

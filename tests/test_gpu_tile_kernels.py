@@ -105,6 +105,52 @@ def test_grouped_kernels_give_every_single_weight(lib, O, rank, group, lengths):
         assert torch.equal(sa, wa[expert, :, ca]) and torch.equal(sb, wb[expert, :, cb])
 
 
+# Segments of many rows, unequal: one to six row tiles, more segments than a warp has lanes, columns that fit shared memory
+# together (one or two chunks, the last one full or not) and columns that stream through it, an odd number of output tiles.
+WIDE = [
+    (264, 256, [300, 0, 5, 129, 700, 128]),
+    (1040, 192, [130 + 61 * (i % 7) for i in range(40)]),
+    (136, 72, [129, 513, 1]),
+    (520, 328, [257, 640, 384, 3]),
+    (264, 1032, [400, 129]),
+]
+
+
+@pytest.mark.parametrize("O,rank,lengths", WIDE)
+def test_long_and_unequal_segments(lib, O, rank, lengths):
+    import trismoe_b200 as tm
+
+    E, R = len(lengths), sum(lengths)
+    pa, pb = _payload(tm, E, O, rank, 128, O + rank), _payload(tm, E, O, rank, 128, O + rank + 1)
+    wa, wb = tm.dequantize_grouped_payload(pa), tm.dequantize_grouped_payload(pb)
+    g = torch.Generator().manual_seed(R)
+    ha, hb = ((0.5 * torch.randn((R, rank), generator=g)).half().cuda() for _ in range(2))
+    route = tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda")
+    one = tm.run_grouped_structured_expert_forward(pa, ha, None, route)
+    sa, sb = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, hb, None, route)
+    ta, tb = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, ha, None, route)  # one set of rows
+    mlp, _ = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, hb, None, route, fuse_silu_mul=True)
+    row = 0
+    for e, n in enumerate(lengths):
+        if n == 0:
+            continue
+        rows = slice(row, row + n)
+        row += n
+        ra, ea, ba = _bound(wa[e], ha[rows])
+        rb, eb, bb = _bound(wb[e], hb[rows])
+        rc, _, bc = _bound(wb[e], ha[rows])
+        for got, ref, bound in ((one, ra, ba), (sa, ra, ba), (sb, rb, bb), (ta, ra, ba), (tb, rc, bc)):
+            _assert_within(got[rows], ref, bound)
+        silu = ra * torch.sigmoid(ra)
+        err = 1.1 * ea * rb.abs() + silu.abs() * eb + 1.1 * ea * eb + (silu * rb).abs() * (2.0 ** -11 + 2.0 ** -19) + 2.0 ** -25
+        _assert_within(mlp[rows], silu * rb, err)
+        for c in range(0, rank, n):  # one-hot rows: every weight exactly
+            hot = torch.zeros_like(ha)
+            hot[rows] = torch.nn.functional.one_hot((torch.arange(n, device="cuda") + c) % rank, rank).half()
+            col = (torch.arange(n, device="cuda") + c) % rank
+            assert torch.equal(tm.run_grouped_structured_expert_forward(pa, hot, None, route)[rows], wa[e][:, col].T)
+
+
 @pytest.mark.parametrize("O,K,T", [(136, 520, 33), (137, 1100, 64), (1024, 2048, 65), (256, 4096, 130), (72, 8192, 300), (4096, 512, 257)])
 def test_linear_columns_shared_among_ctas(lib, O, K, T):
     """An ordinary matrix of more than 32 rows: its columns in one to many parts, single and as a pair."""
