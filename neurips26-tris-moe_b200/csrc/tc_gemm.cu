@@ -87,11 +87,15 @@ __device__ __forceinline__ void tc_gemm_epilogue(const TcGemmArgs& args, const S
       parts[r] = reinterpret_cast<const float4*>(cluster.map_shared_rank(part, r < nblk ? r : 0));
     for (int i4 = rank * per + threadIdx.x; i4 < v_end; i4 += kTcThreads) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 v[8];
+      if (nblk == 1) {  // the columns are not split: no eight predicated remote reads of which one counts
+        acc = reinterpret_cast<const float4*>(part)[i4];
+      } else {
+        float4 v[8];
 #pragma unroll
-      for (unsigned r = 0; r < 8; ++r) v[r] = (r < nblk) ? parts[r][i4] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (unsigned r = 0; r < 8; ++r) v[r] = (r < nblk) ? parts[r][i4] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (unsigned r = 0; r < 8; ++r) { acc.x += v[r].x; acc.y += v[r].y; acc.z += v[r].z; acc.w += v[r].w; }
+        for (unsigned r = 0; r < 8; ++r) { acc.x += v[r].x; acc.y += v[r].y; acc.z += v[r].z; acc.w += v[r].w; }
+      }
       const int n = n0 + (4 * i4) / kTcM, mbase = m0 + (4 * i4) % kTcM;
       if (n >= n_live) continue;
       if ((pb.m & 3) == 0 && mbase < pb.m && (pb.out_mode == TRIS_OUT_F32 || pb.out_mode == TRIS_OUT_F16)) {
@@ -286,17 +290,24 @@ struct TcTmaMaps {
 constexpr int kTcRowBytes = kTcKChunk * 2;
 static_assert(kTcRowBytes == 128, "one swizzle row per operand row and chunk");
 
-// Parity of the last copy round of stage s when `issued` chunks went round-robin over the stages, -1: none.
-constexpr int last_round_parity(int issued, int s) { return issued > s ? ((issued - 1 - s) / kTcStages) & 1 : -1; }
-static_assert(last_round_parity(0, 0) == -1 && last_round_parity(3, 2) == 0 && last_round_parity(3, 3) == -1 && last_round_parity(4, 3) == 0, "first round");
-static_assert(last_round_parity(5, 0) == 1 && last_round_parity(5, 1) == 0 && last_round_parity(8, 3) == 1 && last_round_parity(9, 0) == 0, "later rounds");
+// Stages of 64 columns: as many as let two CTAs share an SM, so that one's start and epilogue run under the other's products.
+// With four stages of 128 rows there was one CTA to an SM, and the 256 CTAs of 16384 rows ran in two waves: 31.0 us at 1024 columns, now
+// 16.8 (with the reads of an unsplit tile below).
+constexpr int tma_stages(int ntile) { return ntile == 128 ? 3 : 4; }
+
+// Parity of the last copy round of stage s when `issued` chunks went round-robin over `stages`, -1: none.
+constexpr int last_round_parity(int issued, int s, int stages) { return issued > s ? ((issued - 1 - s) / stages) & 1 : -1; }
+static_assert(last_round_parity(0, 0, 4) == -1 && last_round_parity(3, 2, 4) == 0 && last_round_parity(3, 3, 4) == -1 && last_round_parity(4, 3, 4) == 0, "first round");
+static_assert(last_round_parity(5, 0, 4) == 1 && last_round_parity(5, 1, 4) == 0 && last_round_parity(8, 3, 4) == 1 && last_round_parity(9, 0, 4) == 0, "later rounds");
+static_assert(last_round_parity(4, 0, 3) == 1 && last_round_parity(4, 1, 3) == 0 && last_round_parity(7, 0, 3) == 0 && last_round_parity(2, 2, 3) == -1, "three stages");
 
 template <int NTILE>
 struct TcTmaSmem {  // at a 1024-byte boundary
-  uint8_t a[kTcStages][kTcM * kTcRowBytes];
-  uint8_t b[kTcStages][NTILE * kTcRowBytes];
-  uint64_t full[kTcStages];
-  uint64_t empty[kTcStages];
+  static constexpr int kStages = tma_stages(NTILE);
+  uint8_t a[kStages][kTcM * kTcRowBytes];
+  uint8_t b[kStages][NTILE * kTcRowBytes];
+  uint64_t full[kStages];
+  uint64_t empty[kStages];
   uint64_t done;
   uint32_t tmem_base;
   int32_t timed_out;
@@ -305,6 +316,7 @@ struct TcTmaSmem {  // at a 1024-byte boundary
 template <int NTILE>
 __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_constant__ TcGemmArgs args,
                                                                    const __grid_constant__ TcTmaMaps maps) {
+  constexpr int kStages = tma_stages(NTILE);
   extern __shared__ uint4 smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   auto& sm = *reinterpret_cast<TcTmaSmem<NTILE>*>(base);
@@ -326,7 +338,7 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
 
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int i = 0; i < kTcStages; ++i) {
+    for (int i = 0; i < kStages; ++i) {
       mbar_init(&sm.full[i], 1);
       mbar_init(&sm.empty[i], 1);
     }
@@ -341,11 +353,11 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
   const uint32_t tmem = warp_uniform(sm.tmem_base);
   constexpr uint32_t kBytes = (kTcM + NTILE) * kTcRowBytes;
   auto load_a = [&](int i) {
-    const int s = i % kTcStages;
+    const int s = i % kStages;
     mbar_arrive_expect_tx(&sm.full[s], kBytes);
     tma_load_2d(sm.a[s], &maps.a[pi], kbeg + i * kTcKChunk, m0, &sm.full[s]);
   };
-  const int ahead = args.a_before_wait ? min(nchunks, kTcStages) : 0;
+  const int ahead = args.a_before_wait ? min(nchunks, kStages) : 0;
   if (threadIdx.x == 0)
     for (int i = 0; i < ahead; ++i) load_a(i);
 
@@ -355,10 +367,10 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
 
   int issued = 0;
   if (threadIdx.x == 0) {
-    // producer: one tensor copy per operand per K chunk, kTcStages chunks in flight
+    // producer: one tensor copy per operand per K chunk, kStages chunks in flight
     for (int i = 0; i < nchunks; ++i, ++issued) {
-      const int s = i % kTcStages;
-      if (i >= kTcStages && !mbar_wait_bounded(&sm.empty[s], ((i / kTcStages) - 1) & 1)) {
+      const int s = i % kStages;
+      if (i >= kStages && !mbar_wait_bounded(&sm.empty[s], ((i / kStages) - 1) & 1)) {
         sm.timed_out = 1;
         break;
       }
@@ -372,8 +384,8 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
     const uint32_t idesc = umma_idesc_f16(kTcM, NTILE);
     bool ok = true;
     for (int i = 0; i < nchunks; ++i) {
-      const int s = i % kTcStages;
-      ok = mbar_wait_warp(&sm.full[s], (i / kTcStages) & 1);
+      const int s = i % kStages;
+      ok = mbar_wait_warp(&sm.full[s], (i / kStages) & 1);
       if (!ok) break;
       tcgen05_fence_after();
       const uint64_t da = umma_smem_desc_sw128(smem_u32(sm.a[s])), db = umma_smem_desc_sw128(smem_u32(sm.b[s]));
@@ -394,8 +406,8 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
   __syncthreads();
   const bool failed = sm.timed_out != 0;
   if (failed && threadIdx.x == 0)  // copies in flight must not land in a buffer that is read as the partial tile
-    for (int s = 0; s < kTcStages; ++s)
-      if (last_round_parity(issued, s) >= 0) mbar_wait_bounded(&sm.full[s], last_round_parity(issued, s));
+    for (int s = 0; s < kStages; ++s)
+      if (last_round_parity(issued, s, kStages) >= 0) mbar_wait_bounded(&sm.full[s], last_round_parity(issued, s, kStages));
   __syncthreads();
   tc_gemm_epilogue<NTILE>(args, pb, reinterpret_cast<float*>(base), tmem, failed, nchunks, m0, n0, n_live, cluster);
 }
@@ -489,7 +501,10 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
   args.k = k;
   args.a_before_wait = pdl && a_before_wait;
   // 128-row tiles re-read the matrices half as often; 64-row tiles give a small batch more CTAs
-  const int ntile = mtiles * ceil_div(n, 128) >= 148 ? 128 : 64;
+  // (and long rows, where the operands' way from L2 is what counts, if the split of the columns below fills the GPU all the same:
+  // 4096 x 14336 x 256 46.8 us with 64-row tiles, 39.7 with 128; 2048 rows 26.1, 23.9; at 4096 columns the other way round, 12.6, 14.4)
+  const int tiles128 = mtiles * ceil_div(n, 128);
+  const int ntile = tiles128 >= 148 || (k >= 8192 && tiles128 * 8 >= 148) ? 128 : 64;
   const int ntiles = ceil_div(n, ntile);
   int ksplit = 1;
   // split K over the cluster until the GPU is full or a CTA would get fewer than two 64-column chunks: a CTA's
