@@ -24,7 +24,7 @@
 //
 // 2048 tokens of 64 experts, gate/up and down: 56.5 / 43.6 us, against 93.5 / 90.0 on the tiled kernel, which unpacks for every
 // 128 rows and holds one accumulator buffer.  What bounds it: every role is a chain of dependent instructions, some 12
-// cycles each between the other warps' (30 warps, issue slots 55 % busy).  Taking work out, at a time when the two launches took 63.9 /
+// cycles each between the other warps' (30 warps, issue slots 43 % busy, tensor pipe 20 / 29 %).  Taking work out, at a time when the two launches took 63.9 /
 // 43.5: without the unpack 58 / 38, without the epilogue's work 46 / 32, without the products 57 / 38.  For segments of one row
 // tile the unpack of a unit is the longest chain (ALU pipe: byte permute, shift and two logic operations per two weights,
 // then 4 to 5 pairs of salient columns a slice), for longer ones the epilogue (SiLU: 8000 cycles a row tile) and the MMA
