@@ -470,18 +470,14 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
 #pragma unroll
           for (int k = 0; k < 16; k += 8) {
             float g[8], up[8];
-            tmem_ld<8>(d + n0 + k, g);
-            tmem_ld<8>(d + N + n0 + k, up);
-            tmem_wait_ld();
+            tmem_ld_8_pair(d + n0 + k, d + N + n0 + k, g, up);
             finish(0, g, 8);
             finish(1, up, 8);
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[k + j] = __fdividef(g[j], 1.f + __expf(-g[j])) * up[j];
           }
         } else {
-          tmem_ld<8>(d + half * N + n0, *reinterpret_cast<float(*)[8]>(&y[0]));
-          tmem_ld<8>(d + half * N + n0 + 8, *reinterpret_cast<float(*)[8]>(&y[8]));
-          tmem_wait_ld();
+          tmem_ld_16(d + half * N + n0, y);
           finish(half, y, 16);
         }
         if (i + 1 == steps) give_back();

@@ -74,20 +74,14 @@ __device__ __forceinline__ void tmem_ld_16_pair(uint32_t taddr_v, uint32_t taddr
                : "memory");
 }
 
-template <int COUNT>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[COUNT]) {  // as tmem_ld_16, 4 or 8 columns, no wait
-  static_assert(COUNT == 4 || COUNT == 8, "columns per load");
-  uint32_t r[COUNT];
-  if constexpr (COUNT == 8)
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-  else
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < COUNT; ++i) v[i] = __uint_as_float(r[i]);
+// Twice 8 columns with one wait.
+__device__ __forceinline__ void tmem_ld_8_pair(uint32_t taddr_v, uint32_t taddr_w, float (&v)[8], float (&w)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+               "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]), "=f"(w[4]), "=f"(w[5]), "=f"(w[6]), "=f"(w[7])
+               : "r"(taddr_v), "r"(taddr_w)
+               : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Registers -> TMEM: thread t of the warp writes COUNT consecutive 32-bit columns of lane (taddr.lane + t).
 // This is how a computed A operand gets to the tensor core without passing through shared memory: column

@@ -1,7 +1,8 @@
-"""CPU test of a rule of the kernel sources.  A kernel that is launched while its predecessor still runs
+"""CPU tests of two rules of the kernel sources.  A kernel that is launched while its predecessor still runs
 (``griddepcontrol.wait`` inside) must not read what the predecessor writes through loads that the compiler may move
 above the wait: parameters that are ``const ... __restrict__``, and the non-coherent ``__ldg`` / ``ld.global.nc``.
-Those are for weights."""
+Those are for weights.  And a load from TMEM has its wait in the same statement: the registers are not valid before it, and between
+two statements the compiler may place anything, a spill of them too."""
 import glob
 import os
 import re
@@ -36,3 +37,14 @@ def test_no_movable_load_of_a_predecessors_output(file, name, params, body):
         assert p in HOST_TABLES, (file, name, p)
     for load in re.findall(r"(?:__ldg|ldg_stream)\s*\(([^;]*)\)", body):
         assert not re.search(PRODUCED, load), (file, name, load)
+
+
+def test_a_tmem_load_and_its_wait_are_one_statement():
+    loads = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        for asm in re.findall(r"\basm\b[^;]*?\((\s*\"(?:[^\"\\]|\\.)*\".*?)\)\s*;", re.sub(r"//[^\n]*", "", open(path).read()), re.S):
+            text = "".join(re.findall(r"\"((?:[^\"\\]|\\.)*)\"", asm))
+            if "tcgen05.ld." in text:
+                loads += 1
+                assert "tcgen05.wait::ld" in text[text.rindex("tcgen05.ld."):], (os.path.basename(path), text[:90])
+    assert loads >= 3
