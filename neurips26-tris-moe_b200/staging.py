@@ -191,7 +191,7 @@ class GroupedQGmapCPUStagingManager:
         # drop the device copies: from here on the tensors exist only in pinned host memory
         for entry in self.entries.values():
             for key in entry.host:
-                entry.payload[key] = torch.empty((0,), dtype=entry.host[key].dtype, device=self.device)
+                entry.payload[key] = torch.empty((0,), dtype=entry.payload[key].dtype, device=self.device)
             if self.mode == "payload":
                 # the resident tile-major copy of the same planes would defeat the point of paging them
                 for key in ("_tris_tile_records", "_tris_tile_desc", "_tris_col_records", "_tris_tile_meta"):

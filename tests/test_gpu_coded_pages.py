@@ -59,3 +59,20 @@ def test_every_bit_comes_back(lib, per):
     bad = (tm._native.TrisCodedPageJob * 1)()
     assert lib.tris_page_coded_experts(bad, 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
     assert lib.tris_page_coded_experts(C.cast(None, C.c_void_p), 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
+
+
+def test_emptied_bitmap_of_a_payload_keeps_its_type(lib):
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging, synth
+
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=6, keep_sparse_gmap=True)
+    blk = tm.TrisSparseMoeBlock(256, 192, 8, 2, True)
+    for name in ("gate", "up", "down"):
+        layer[name]["compact3_use_block_gr"] = False
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], layer["shared_gate"], layer["shared_up"], layer["shared_down"],
+                              layer["router_weight"], device="cuda")
+    manager = staging.GroupedQGmapCPUStagingManager([blk])
+    assert manager.initialize()
+    for name in ("gate", "up", "down"):
+        assert manager.entries[(0, name)].coded and blk._get_grouped_payload(name)["q_gmap_sparse"].dtype == torch.int32
