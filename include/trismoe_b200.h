@@ -538,10 +538,11 @@ typedef struct TrisCodedPageJob {
 /*
  * Codes an E-stacked device tensor of sparse bits, [E, bytes_per_expert], in blocks of 1024 bytes.  First call with
  * block_offsets NULL: writes the size of every block in 16-byte units, 0 to 64, to units_out [E * blocks].  Second call with
- * their exclusive sums ([E * blocks + 1]): writes the code to dst_dev.  bytes_per_expert is a multiple of 16.
+ * their exclusive sums ([E * blocks + 1]): writes the code to dst, device memory or pinned host memory.  bytes_per_expert is a
+ * multiple of 16.
  */
 int tris_page_code_blocks(const void* src_dev, int64_t bytes_per_expert, int32_t num_experts, int32_t* units_out,
-                          const int32_t* block_offsets, void* dst_dev, void* stream);
+                          const int32_t* block_offsets, void* dst, void* stream);
 /* tris_page_experts for coded tensors: the blocks are decoded on their way into the staging buffer. */
 int tris_page_coded_experts(const TrisCodedPageJob* jobs, int32_t num_jobs, const int32_t* expert_ids,
                             const int32_t* num_segments_dev, int32_t num_segments, int32_t num_experts,

@@ -94,10 +94,10 @@ class _Entry:
             total, most = torch.stack([ends[-1], (ends[1:] - ends[:-1]).max()]).tolist()
             if total * 16 * 8 > experts * per * 7:
                 return False
-            code = torch.empty((max(1, total) * 16,), dtype=torch.uint8, device=t.device)
-            _native.check(lib.tris_page_code_blocks(t.data_ptr(), per, experts, None, offsets.data_ptr(), code.data_ptr(), stream), "page_code_blocks")
-        host = torch.empty(code.shape, dtype=torch.uint8, pin_memory=True)
-        host.copy_(code)
+            # straight into pinned memory: streaming is for GPUs that have no room for another copy
+            host = torch.empty((max(1, total) * 16,), dtype=torch.uint8, pin_memory=True)
+            _native.check(lib.tris_page_code_blocks(t.data_ptr(), per, experts, None, offsets.data_ptr(), host.data_ptr(), stream), "page_code_blocks")
+            torch.cuda.current_stream(t.device).synchronize()
         self.host[key], self.coded[key], self.link_bytes[key] = host, offsets, most * 16
         return True
 

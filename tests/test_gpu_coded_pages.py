@@ -61,6 +61,35 @@ def test_every_bit_comes_back(lib, per):
     assert lib.tris_page_coded_experts(C.cast(None, C.c_void_p), 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
 
 
+def test_entry_is_coded_without_a_device_copy(lib):
+    """Streaming is for GPUs whose memory is short: coding 16 MB asks for less than a thirty-second of it beside the bitmap."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging
+
+    E, rows, O = 32, 32, 4096
+    g = torch.Generator(device="cuda").manual_seed(3)
+    density = torch.linspace(0.0, 0.2, E, device="cuda").view(E, 1, 1)
+    bitmap = torch.zeros((E, rows, O), dtype=torch.int32, device="cuda")
+    for j in range(32):
+        bitmap |= (torch.rand((E, rows, O), generator=g, device="cuda") < density).to(torch.int32) << j
+    payload = {"qweight1": torch.zeros((E, 1, 1), dtype=torch.int32, device="cuda"), "q_gmap_sparse": bitmap}
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    entry = staging._Entry(payload, staging.BITMAP_KEYS)
+    assert torch.cuda.max_memory_allocated() - before <= bitmap.numel() * 4 // 32
+    per = rows * O * 4
+    assert entry.block_bytes["q_gmap_sparse"] == per and entry.rows["q_gmap_sparse"] == rows
+    dst, table = torch.empty_like(bitmap), torch.empty((E,), dtype=torch.int32, device="cuda")
+    jobs = (tm._native.TrisCodedPageJob * 1)()
+    jobs[0].host_src, jobs[0].block_offsets = entry.host["q_gmap_sparse"].data_ptr(), entry.coded["q_gmap_sparse"].data_ptr()
+    jobs[0].dst, jobs[0].bytes_per_expert = dst.data_ptr(), per
+    ids = torch.arange(E, dtype=torch.int32, device="cuda")
+    assert lib.tris_page_coded_experts(jobs, 1, ids.data_ptr(), None, E, E, table.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(dst, bitmap)
+
+
 def test_emptied_bitmap_of_a_payload_keeps_its_type(lib):
     import trismoe_b200 as tm
     from trismoe_b200 import staging, synth
