@@ -64,15 +64,16 @@ class _Entry:
             if per == 0:
                 continue
             shape = list(t.shape)
-            self.rows[key] = int(shape[1])
             if per % 16:
                 # only a 2-D stream (block-GR words) can be ragged: pad each expert's row with zeros
                 if t.dim() != 2 or (16 % t.element_size()):
                     raise RuntimeError(f"trismoe_b200 staging: {key} has {per} bytes per expert, not a multiple of 16")
                 step = 16 // t.element_size()
-                shape[1] = self.rows[key] = (shape[1] + step - 1) // step * step
+                shape[1] = (shape[1] + step - 1) // step * step
                 per = shape[1] * t.element_size()
             self.block_bytes[key] = self.link_bytes[key] = per
+            if t.dim() > 1:
+                self.rows[key] = int(shape[1])
             if key == "q_gmap_sparse" and t.is_cuda and self._code(key, t.contiguous(), E, per):
                 continue
             host = torch.zeros(shape, dtype=t.dtype, pin_memory=True)
@@ -135,6 +136,7 @@ class GroupedQGmapCPUStagingManager:
         self._copy_stream = None
         self._next = 0
         self._initialized = False
+        # bytes: at most, as if every slot of a launch were used and by the largest expert
         self.pipeline_stats = {"calls": 0, "chunks": 0, "bytes": 0, "slot_reuses": 0}
         self._timings = []         # (copy_start, copy_end, wait_start, wait_end) events
         self.collect_timings = True  # set False while capturing the forward into a CUDA graph
@@ -249,7 +251,7 @@ class GroupedQGmapCPUStagingManager:
         return _PagedLayer(self, ring, views, start, end)
 
     def _plan(self, block_index: int, ring: int):
-        """Pager launches ``(coded, jobs, count, bytes per segment, ends gate/up, slot table)`` and staged views of a
+        """Pager launches ``(coded, jobs, count, most bytes per segment, ends gate/up, slot table)`` and staged views of a
         layer in a ring slot, laid out on first use and again when a projection's own view has other contents
         (an object's identity would miss a view edited in place, and one built at a freed view's address)."""
         bases = tuple(bytes(proj_view(self.entries[(block_index, proj)].payload)) for proj in PROJECTIONS)
@@ -258,19 +260,20 @@ class GroupedQGmapCPUStagingManager:
             return plan[1], plan[2]
         launches, views = [], {}
         for group in (("gate", "up"), ("down",)):
-            table, entry_of, parts = self.slot_tables[ring][group[0]], lambda proj: self.entries[(block_index, proj)], []
+            table, parts = self.slot_tables[ring][group[0]], []
+            pages = [(proj, key, self.entries[(block_index, proj)]) for proj in group for key in self.entries[(block_index, proj)].host]
             for coded in (False, True):
-                pairs = [(proj, key) for proj in group for key in entry_of(proj).host if (key in getattr(entry_of(proj), "coded", ())) == coded]
-                parts += [(coded, pairs[lo: lo + MAX_PAGE_JOBS]) for lo in range(0, len(pairs), MAX_PAGE_JOBS)]
+                these = [page for page in pages if (page[1] in page[2].coded) == coded]
+                parts += [(coded, these[lo: lo + MAX_PAGE_JOBS]) for lo in range(0, len(these), MAX_PAGE_JOBS)]
             for i, (coded, part) in enumerate(parts):
                 jobs = ((TrisCodedPageJob if coded else TrisPageJob) * len(part))()
-                for j, (proj, key) in enumerate(part):
-                    jobs[j].host_src = entry_of(proj).host[key].data_ptr()
-                    jobs[j].dst = self.buffers[(ring, proj, key)].data_ptr()
-                    jobs[j].bytes_per_expert = entry_of(proj).block_bytes[key]
+                for job, (proj, key, entry) in zip(jobs, part):
+                    job.host_src = entry.host[key].data_ptr()
+                    job.dst = self.buffers[(ring, proj, key)].data_ptr()
+                    job.bytes_per_expert = entry.block_bytes[key]
                     if coded:
-                        jobs[j].block_offsets = entry_of(proj).coded[key].data_ptr()
-                per_segment = sum(getattr(entry_of(proj), "link_bytes", entry_of(proj).block_bytes)[key] for proj, key in part)
+                        job.block_offsets = entry.coded[key].data_ptr()
+                per_segment = sum(entry.link_bytes[key] for _, key, entry in part)
                 launches.append((coded, jobs, len(part), per_segment, group[0] == "gate" and i + 1 == len(parts), table.data_ptr()))
             for proj in group:
                 views[proj] = self._staged_view(self.entries[(block_index, proj)], ring, proj, table)
@@ -287,16 +290,15 @@ class GroupedQGmapCPUStagingManager:
                  "row_pack3": "row_pack3"}
         for key in entry.host:
             setattr(view, field[key], self.buffers[(ring, proj, key)].data_ptr())
-        rows = lambda key: entry.rows[key] if key in getattr(entry, "rows", ()) else int(entry.host[key].shape[1])
         if self.mode == "bitmap":
             view.gmap_slot = table.data_ptr()
-            view.gmap_sparse_rows = rows("q_gmap_sparse")
+            view.gmap_sparse_rows = entry.rows["q_gmap_sparse"]
         else:
             view.expert_slot = table.data_ptr()
             if "q_gmap_sparse" in entry.host:
-                view.gmap_sparse_rows = rows("q_gmap_sparse")
+                view.gmap_sparse_rows = entry.rows["q_gmap_sparse"]
             if "q_gmap_gr_words" in entry.host:
-                view.gr_max_words = rows("q_gmap_gr_words")
+                view.gr_max_words = entry.rows["q_gmap_gr_words"]
         return view
 
     # -- reporting -----------------------------------------------------------------------------

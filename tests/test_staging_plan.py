@@ -1,18 +1,22 @@
-"""CPU test: the cached pager plan of a layer follows the projections' own views."""
+"""CPU tests of the pager plan of a layer: what it launches, and that a cached one follows the projections' own views."""
+import ctypes as C
 import types
 
 import pytest
 import torch
 
 
-def _manager(tm, staging):
+def _manager(tm, staging, coded=()):
     man = staging.GroupedQGmapCPUStagingManager([], mode="bitmap")
     man.slot_tables = [{p: torch.zeros((4,), dtype=torch.int32) for p in ("gate", "down")}]
     for proj in staging.PROJECTIONS:
-        host = {"q_gmap_sparse": torch.zeros((4, 2, 8), dtype=torch.int32)}
+        host, key = torch.zeros((4, 2, 8), dtype=torch.int32), "q_gmap_sparse"
         view = tm._native.TrisProjView()
         view.out_features, view.output_scale = 8, 4096
-        man.entries[(0, proj)] = types.SimpleNamespace(payload={"_tris_prepared": True, "_tris_view": view}, host=host, block_bytes={"q_gmap_sparse": 64})
+        # all that an entry has but pinned memory, which needs a GPU
+        man.entries[(0, proj)] = types.SimpleNamespace(payload={"_tris_prepared": True, "_tris_view": view}, host={key: host}, block_bytes={key: 64},
+                                                       link_bytes={key: 32 if proj in coded else 64}, rows={key: 2},
+                                                       coded={key: torch.zeros((5,), dtype=torch.int32)} if proj in coded else {})
         man.buffers[(0, proj, "q_gmap_sparse")] = torch.zeros((64,), dtype=torch.uint8)
     return man
 
@@ -42,3 +46,28 @@ def test_plan_follows_a_view_that_is_rebuilt_or_edited(proj):
         seen.add(id(view))
     else:
         pytest.skip("no address was used twice")
+
+
+@pytest.mark.parametrize("coded", [(), ("gate",), ("up",), ("gate", "up"), ("down",), ("gate", "up", "down")])
+def test_raw_and_coded_tensors_go_in_launches_of_their_own(coded):
+    """One launch per kind and group, raw before coded; the last one of gate and up ends the group, none of down does."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging
+
+    man = _manager(tm, staging, coded)
+    launches, views = man._plan(0, 0)
+    want = [(kind, procs) for group in (("gate", "up"), ("down",)) for kind in (False, True)
+            for procs in [[p for p in group if (p in coded) == kind]] if procs]
+    assert [(kind, count) for kind, _, count, _, _, _ in launches] == [(kind, len(procs)) for kind, procs in want]
+    last_gate_up = max(i for i, (_, procs) in enumerate(want) if "down" not in procs)
+    for i, ((kind, jobs, count, most, ends, table), (_, procs)) in enumerate(zip(launches, want)):
+        assert isinstance(jobs, C.Array) and isinstance(jobs[0], tm._native.TrisCodedPageJob if kind else tm._native.TrisPageJob)
+        assert most == (32 if kind else 64) * count and ends == (i == last_gate_up)
+        assert table == man.slot_tables[0][procs[0] if procs[0] == "down" else "gate"].data_ptr()
+        for job, proj in zip(jobs, procs):
+            entry = man.entries[(0, proj)]
+            assert job.host_src == entry.host["q_gmap_sparse"].data_ptr() and job.bytes_per_expert == 64
+            assert job.dst == man.buffers[(0, proj, "q_gmap_sparse")].data_ptr()
+            assert not kind or job.block_offsets == entry.coded["q_gmap_sparse"].data_ptr()
+    for proj in staging.PROJECTIONS:
+        assert views[proj].q_gmap_sparse == man.buffers[(0, proj, "q_gmap_sparse")].data_ptr() and views[proj].gmap_sparse_rows == 2
