@@ -477,8 +477,8 @@ def streaming_records(blocks, manager, shape, device):
     from trismoe_b200 import staging, synth
 
     n_layers, H = len(blocks), shape.hidden_size
-    per_expert = [sum(manager.entries[(l, p)].link_bytes[k] for p in staging.PROJECTIONS
-                      for k in manager.entries[(l, p)].link_bytes) for l in range(n_layers)]
+    per_expert = [torch.tensor([sizes for p in staging.PROJECTIONS for sizes in manager.entries[(l, p)].link_bytes.values()]).sum(0)
+                  for l in range(n_layers)]
     recs = []
     for T in (1, 16):
         x = synth.synth_activations(T, H, seed=T).to(device)
@@ -488,9 +488,9 @@ def streaming_records(blocks, manager, shape, device):
                 blk.forward_streaming(x.view(1, T, H), manager, l)
 
         paged_bytes = 0
-        for l, blk in enumerate(blocks):  # bytes one pass pages: distinct routed experts x per-expert block sizes
+        for l, blk in enumerate(blocks):  # bytes one pass pages: those of the distinct routed experts
             _, logits = blk.forward_streaming(x.view(1, T, H), manager, l)
-            paged_bytes += torch.unique(torch.topk(logits, shape.top_k, dim=-1).indices).numel() * per_expert[l]
+            paged_bytes += int(per_expert[l][torch.unique(torch.topk(logits, shape.top_k, dim=-1).indices).cpu()].sum())
         for _ in range(3):
             step()
         torch.cuda.synchronize()

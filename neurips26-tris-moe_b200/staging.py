@@ -52,7 +52,7 @@ class _Entry:
         self.payload = payload
         self.host = {}
         self.block_bytes = {}  # of an expert's block in a staging slot
-        self.link_bytes = {}   # the same on its way over the host link: of the largest expert
+        self.link_bytes = {}   # key -> of every expert's block on its way over the host link
         self.coded = {}        # key -> device offsets of the coded blocks
         self.rows = {}         # key -> second dimension of the tensor
         E = int(payload["qweight1"].shape[0])
@@ -71,7 +71,7 @@ class _Entry:
                 step = 16 // t.element_size()
                 shape[1] = (shape[1] + step - 1) // step * step
                 per = shape[1] * t.element_size()
-            self.block_bytes[key] = self.link_bytes[key] = per
+            self.block_bytes[key], self.link_bytes[key] = per, [per] * E
             if t.dim() > 1:
                 self.rows[key] = int(shape[1])
             if key == "q_gmap_sparse" and t.is_cuda and self._code(key, t.contiguous(), E, per):
@@ -91,15 +91,15 @@ class _Entry:
             units = torch.empty((experts * blocks,), dtype=torch.int32, device=t.device)
             _native.check(lib.tris_page_code_blocks(t.data_ptr(), per, experts, units.data_ptr(), None, None, stream), "page_code_blocks")
             torch.cumsum(units, 0, dtype=torch.int32, out=offsets[1:])
-            ends = offsets[::blocks]
-            total, most = torch.stack([ends[-1], (ends[1:] - ends[:-1]).max()]).tolist()
-            if total * 16 * 8 > experts * per * 7:
+            ends = offsets[::blocks].tolist()  # waits
+            if ends[-1] * 16 * 8 > experts * per * 7:
                 return False
             # straight into pinned memory: streaming is for GPUs that have no room for another copy
-            host = torch.empty((max(1, total) * 16,), dtype=torch.uint8, pin_memory=True)
+            host = torch.empty((max(1, ends[-1]) * 16,), dtype=torch.uint8, pin_memory=True)
             _native.check(lib.tris_page_code_blocks(t.data_ptr(), per, experts, None, offsets.data_ptr(), host.data_ptr(), stream), "page_code_blocks")
             torch.cuda.current_stream(t.device).synchronize()
-        self.host[key], self.coded[key], self.link_bytes[key] = host, offsets, most * 16
+        self.host[key], self.coded[key] = host, offsets
+        self.link_bytes[key] = [16 * (hi - lo) for lo, hi in zip(ends, ends[1:])]
         return True
 
 
@@ -273,7 +273,7 @@ class GroupedQGmapCPUStagingManager:
                     job.bytes_per_expert = entry.block_bytes[key]
                     if coded:
                         job.block_offsets = entry.coded[key].data_ptr()
-                per_segment = sum(entry.link_bytes[key] for _, key, entry in part)
+                per_segment = sum(max(entry.link_bytes[key]) for _, key, entry in part)
                 launches.append((coded, jobs, len(part), per_segment, group[0] == "gate" and i + 1 == len(parts), table.data_ptr()))
             for proj in group:
                 views[proj] = self._staged_view(self.entries[(block_index, proj)], ring, proj, table)

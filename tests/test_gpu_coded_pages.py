@@ -62,7 +62,8 @@ def test_every_bit_comes_back(lib, per):
 
 
 def test_entry_is_coded_without_a_device_copy(lib):
-    """Streaming is for GPUs whose memory is short: coding 16 MB asks for less than a thirty-second of it beside the bitmap."""
+    """Streaming is for GPUs whose memory is short: coding 16 MB asks for less than a thirty-second of it beside the bitmap.  Link
+    bytes are those of the code, expert by expert."""
     import trismoe_b200 as tm
     from trismoe_b200 import staging
 
@@ -78,7 +79,9 @@ def test_entry_is_coded_without_a_device_copy(lib):
     before = torch.cuda.memory_allocated()
     entry = staging._Entry(payload, staging.BITMAP_KEYS)
     assert torch.cuda.max_memory_allocated() - before <= bitmap.numel() * 4 // 32
-    per = rows * O * 4
+    per, blocks = rows * O * 4, rows * O // 256
+    ends = entry.coded["q_gmap_sparse"][::blocks].tolist()
+    assert entry.link_bytes["q_gmap_sparse"] == [16 * (b - a) for a, b in zip(ends, ends[1:])] and entry.link_bytes["q_gmap_sparse"][0] == 0
     assert entry.block_bytes["q_gmap_sparse"] == per and entry.rows["q_gmap_sparse"] == rows
     dst, table = torch.empty_like(bitmap), torch.empty((E,), dtype=torch.int32, device="cuda")
     jobs = (tm._native.TrisCodedPageJob * 1)()

@@ -15,7 +15,7 @@ def _manager(tm, staging, coded=()):
         view.out_features, view.output_scale = 8, 4096
         # all that an entry has but pinned memory, which needs a GPU
         man.entries[(0, proj)] = types.SimpleNamespace(payload={"_tris_prepared": True, "_tris_view": view}, host={key: host}, block_bytes={key: 64},
-                                                       link_bytes={key: 32 if proj in coded else 64}, rows={key: 2},
+                                                       link_bytes={key: [16, 32, 0, 16] if proj in coded else [64] * 4}, rows={key: 2},
                                                        coded={key: torch.zeros((5,), dtype=torch.int32)} if proj in coded else {})
         man.buffers[(0, proj, "q_gmap_sparse")] = torch.zeros((64,), dtype=torch.uint8)
     return man
