@@ -701,16 +701,22 @@ static int row_split(long long units, int max_rows, int n) {
   if (limit <= 1 || units <= 0) return 1;
   return static_cast<int>(std::max<long long>(1, std::min<long long>({limit, sm_count() / units, (max_rows + n - 1) / n})));
 }
+// Rows of such a part on the weights-resident kernel.  Two row tiles would share an unpack where the columns do not fit shared
+// memory, but half as many CTAs unpack then: 4096 x 4096, 256 rows 30.0 us with parts of 256, 25.1 with 128; a pair of 512 x 2048
+// 22.6, 18.3; experts, 4096 x 320 x 2, a pair 17.7, 13.9.  (From 769 rows on there are four parts either way.)
+constexpr int kPartRows = 128;
 
 // Column split of one ordinary matrix (no experts): its units of two output tiles and its row passes together are
 // too few for the SMs, and its columns many - parts of the columns go to CTAs of their own, whose fp32 sums
-// sum_parts_kernel adds in order.  4096 columns, 512 rows: 64 units for 4096 outputs (two parts), 32 for a pair of
-// 1024 (four): 108 -> 48 and 92 -> 35 us.  At least two chunks per part: a part's sums are written and read once,
+// sum_parts_kernel adds in order.  4096 columns, 512 rows: 64 CTAs for 4096 outputs (two parts), 32 for a pair of
+// 1024 (four): 59 -> 39 and 61 -> 28 us.  At least two chunks per part: a part's sums are written and read once,
 // 8 bytes per row and output (16 MB for 512 x 4096).
+static size_t part_bytes(int num_rows, int out_features, int projections) { return sizeof(float) * static_cast<size_t>(projections) * num_rows * out_features; }
+static long long col_parts(int chunks, long long units) { return std::min<long long>(chunks / 2, sm_count() / units); }
 static int col_split(const TiledArgs& args, int mode, long long units) {
   if (args.expert_ids || !args.partial || units <= 0) return 1;
-  const size_t part = sizeof(float) * static_cast<size_t>(args.num_rows) * args.out_features * (mode == MODE_SINGLE ? 1 : 2);
-  return static_cast<int>(std::max<long long>(1, std::min<long long>({args.chunks / 2, sm_count() / units, static_cast<long long>(args.partial_bytes / part)})));
+  const size_t part = part_bytes(args.num_rows, args.out_features, mode == MODE_SINGLE ? 1 : 2);
+  return static_cast<int>(std::max<long long>(1, std::min<long long>(col_parts(args.chunks, units), static_cast<long long>(args.partial_bytes / part))));
 }
 
 // One thread per four outputs of a row: adds the parts, then scale, bias and SiLU * up as the epilogue would.
@@ -814,7 +820,7 @@ static bool wide_is_faster(const TiledArgs& args, int mode, int typical_rows) {
 template <int MODE>
 static int launch_wide(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {
   const long long units = static_cast<long long>(args.units_x) * args.num_segments;
-  args.row_split = row_split(units, max_rows, args.chunks <= kWideChunks ? 128 : 256);
+  args.row_split = row_split(units, max_rows, kPartRows);
   args.col_split = col_split(args, MODE, units * args.row_split);
   args.resident = ceil_div(args.chunks, args.col_split) <= kWideChunks;
   args.unit_cost = MODE == MODE_SINGLE ? 2 : 1;  // unpacking a unit against a row tile, whose SiLU is the longer epilogue (44.7 / 34.4 us, 45.9 / 37.6 us the other way round: 1024 tokens)
@@ -927,17 +933,17 @@ extern "C" int tris_set_grouped_row_split_max(int32_t ctas) {
   return tris::tr::g_row_split_max.exchange(ctas < 1 ? 1 : (ctas > 16 ? 16 : ctas), std::memory_order_relaxed);
 }
 
-// Bytes that let launch_grouped_tiled split the columns as far as it would: one part per SM-filling share, within
-// 256 MB.  The sums grow with the rows while the gain does not (100 000 rows of a 1024-output pair would ask for 3 GB);
-// 4096 rows of a 4096 x 4096 matrix still get their two parts (134 MB).
+// Bytes that let launch_grouped_tiled split the columns as far as it would: the parts of its launches (on the tiled kernel an
+// ordinary matrix has too few rows for a second part, of 64 or of 128), within 256 MB.  The sums grow with the rows while
+// the gain does not (100 000 rows of a 1024-output pair would ask for 3 GB); 4096 rows of a 4096 x 4096 matrix still get
+// their two parts (134 MB).
 constexpr size_t kMostSplitBytes = size_t{256} << 20;
 size_t tris::grouped_split_bytes(const TrisProjView* proj, int projections, int num_rows) {
-  using namespace tr;
+  using namespace tris::tr;
   if (!proj_has_tile_records(*proj) || num_rows <= kDecodeMaxRows || num_chunks(proj->rank) < 4) return 0;
   const long long tiles = tiles_per_expert(proj->out_features), units = projections == 1 ? (tiles + 1) / 2 : tiles;
-  const long long row_parts = std::max<long long>(1, std::min<long long>(sm_count() / units, (num_rows + 127) / 128));
-  const size_t part = sizeof(float) * static_cast<size_t>(projections) * num_rows * proj->out_features;
-  const long long parts = std::min<long long>({num_chunks(proj->rank) / 2, sm_count() / (units * std::min<long long>(row_parts, g_row_split_max.load(std::memory_order_relaxed))),
-                                               static_cast<long long>(kMostSplitBytes / part)});
+  const size_t part = part_bytes(num_rows, proj->out_features, projections);
+  const long long parts = std::min<long long>(col_parts(num_chunks(proj->rank), units * row_split(units, num_rows, kPartRows)),
+                                              static_cast<long long>(kMostSplitBytes / part));
   return parts <= 1 ? 0 : part * static_cast<size_t>(parts);
 }

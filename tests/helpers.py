@@ -1,5 +1,7 @@
 """Shared helpers for the tests: golden fixture loading and payload conversion."""
+import json
 import os
+import tempfile
 
 import numpy as np
 import torch
@@ -34,3 +36,14 @@ def golden_expert_payload(z, prefix):
 
 def to_numpy_payload(payload):
     return {k: (v.detach().cpu().numpy() if isinstance(v, torch.Tensor) else v) for k, v in payload.items()}
+
+
+def kernels_of(fn):
+    """Names and grids of the kernels that ``fn`` launches, in order of their start."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    with tempfile.NamedTemporaryFile(suffix=".json") as f:
+        prof.export_chrome_trace(f.name)
+        events = [e for e in json.load(open(f.name))["traceEvents"] if e.get("cat") == "kernel"]
+    return [(e["name"], e["args"]["grid"]) for e in sorted(events, key=lambda e: e["ts"])]

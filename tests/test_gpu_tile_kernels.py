@@ -5,6 +5,8 @@ import numpy as np
 import pytest
 import torch
 
+from helpers import kernels_of
+
 pytestmark = pytest.mark.gpu
 
 
@@ -186,6 +188,24 @@ def test_linear_columns_shared_among_ctas(lib, O, K, T):
         want = [(tm.dequantize_grouped_payload(m.payload)[0][:, col].float() * m.payload["output_scale"].float().view(O, 1)).half().t() for m in mods]
         a, b = tm.run_compact3_gate_up_forward(mods[0], mods[1], hot, fuse_silu_mul=False)
         assert torch.equal(mods[0](hot), want[0]) and torch.equal(a, want[0]) and torch.equal(b, want[1])
+
+
+@pytest.mark.parametrize("O,K,T,pair", [(1024, 2048, 256, False), (512, 2048, 512, True), (2048, 512, 300, False), (264, 1032, 129, True)])
+def test_linear_parts_fill_the_gpu(lib, O, K, T, pair):
+    """Rows in parts of 128, columns in as many parts as the SMs and two chunks a part allow."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(1)
+    mods = [tm.Compact3Linear(synth.pack_projection(synth.raw_projection(rng, 1, O, K, group_size=128)), device="cuda") for _ in range(2)]
+    x = torch.zeros((T, K), dtype=torch.float16, device="cuda")
+    run = (lambda: tm.run_compact3_gate_up_forward(*mods, x, fuse_silu_mul=False)) if pair else (lambda: mods[0](x))
+    sms, tiles, chunks = torch.cuda.get_device_properties(0).multi_processor_count, -(-O // 128), -(-K // 128)
+    units = tiles if pair else -(-tiles // 2)
+    rows = min(4, sms // units, -(-T // 128))
+    run()
+    grids = [grid for name, grid in kernels_of(run) if "grouped_wide_kernel" in name]
+    assert grids == [[units * rows * min(chunks // 2, sms // (units * rows)), 1, 1]]
 
 
 @pytest.mark.parametrize("rows,cols,group,T", [
