@@ -484,6 +484,37 @@ bool tc_gemm_applicable(int n, int k, const __half* x, const SkinnyProblem* prob
   return true;
 }
 
+constexpr int kTcSms = 148;
+// Split K over the cluster until the GPU is full or a CTA would get fewer than two 64-column chunks: a CTA's
+// time is its chain of chunk loads and MMAs, so shorter chains win (measured at 128 and 1024 rows: 85.7 us
+// per layer with a floor of two chunks, 86.8 with four; a cluster of 16 is slower again)
+static int column_split(int tiles, int k) {
+  int ksplit = 1;
+  while (ksplit < 8 && tiles * ksplit < kTcSms && k / (ksplit * 2) >= 2 * kTcKChunk) ksplit *= 2;
+  return ksplit;
+}
+// Clusters of 1, 2, 4 and 8 CTAs that a B200 holds at once where two of the CTAs share an SM and where one has it to itself: SMs come in
+// groups of 16 to 20, and a cluster does not span two (cudaOccupancyMaxActiveClusters for kernels of this footprint).
+static int clusters_at_once(bool alone, int ksplit) {
+  constexpr int kClusters[2][4] = {{296, 148, 71, 33}, {148, 74, 33, 15}};
+  return kClusters[alone][ksplit >= 8 ? 3 : ksplit >> 1];
+}
+// 128-row tiles re-read the matrices half as often; 64-row tiles give a small batch more CTAs.  For long rows, where the
+// operands' way from L2 is what counts, fewer 128-row tiles do too, if the split of the columns fills the GPU all the same: us,
+// 64-row / 128-row tiles of 256 outputs, 8192 columns, 40 tiles of 128 rows 22.4 / 21.8, 74: 43.2 / 35.0; 14336 columns, 24:
+// 23.7 / 21.7, 40: 38.5 / 31.7, 74: 74.9 / 56.3 (at 4096 columns 12.6 / 14.4).  Eighths of 8192 columns are too short for it (19 to
+// 32 tiles 0.92 to 1.06 of the time; of 10240, 0.92 to 1.02).  And if the clusters run at once: 72 of four CTAs, of which 71 fit,
+// 28.4 / 40.6, 34 of eight, of which 33 fit, 17.6 / 27.2.  Gathered 128-row tiles (128 KB) have an SM to themselves, and two turns of
+// them are no longer than one of 64-row tiles that share it (8192 columns, 30 tiles 66 / 56; 32 tiles, a third turn, 66 / 80).
+static int rows_per_tile(int mtiles, int n, int k, bool gathered) {
+  const int tiles128 = mtiles * ceil_div(n, 128), split128 = column_split(tiles128, k);
+  if (tiles128 >= kTcSms) return 128;
+  if (tiles128 * 8 < kTcSms || k < (split128 == 8 && !gathered ? 10240 : 8192)) return 64;
+  if (tiles128 <= (gathered ? 2 : 1) * clusters_at_once(gathered, split128)) return 128;
+  const int tiles64 = mtiles * ceil_div(n, 64);
+  return tiles64 <= clusters_at_once(false, column_split(tiles64, k)) ? 64 : 128;  // neither runs at once: 36 tiles, 0.9 to 1.0 of the time
+}
+
 int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x, const int32_t* row_gather, int n,
                    int k, cudaStream_t stream, bool pdl, const int32_t* n_dev, int32_t* status, bool a_before_wait) {
   TcGemmArgs args{};
@@ -500,17 +531,8 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
   args.n = n;
   args.k = k;
   args.a_before_wait = pdl && a_before_wait;
-  // 128-row tiles re-read the matrices half as often; 64-row tiles give a small batch more CTAs
-  // (and long rows, where the operands' way from L2 is what counts, if the split of the columns below fills the GPU all the same:
-  // 4096 x 14336 x 256 46.8 us with 64-row tiles, 39.7 with 128; 2048 rows 26.1, 23.9; at 4096 columns the other way round, 12.6, 14.4)
-  const int tiles128 = mtiles * ceil_div(n, 128);
-  const int ntile = tiles128 >= 148 || (k >= 8192 && tiles128 * 8 >= 148) ? 128 : 64;
-  const int ntiles = ceil_div(n, ntile);
-  int ksplit = 1;
-  // split K over the cluster until the GPU is full or a CTA would get fewer than two 64-column chunks: a CTA's
-  // time is its chain of chunk loads and MMAs, so shorter chains win (measured at 128 and 1024 rows: 85.7 us
-  // per layer with a floor of two chunks, 86.8 with four; a cluster of 16 is slower again)
-  while (ksplit < 8 && mtiles * ntiles * ksplit < 148 && k / (ksplit * 2) >= 2 * kTcKChunk) ksplit *= 2;
+  const int ntile = rows_per_tile(mtiles, n, k, row_gather != nullptr);
+  const int ntiles = ceil_div(n, ntile), ksplit = column_split(mtiles * ntiles, k);
   args.k_per_cta = ceil_div(ceil_div(k, ksplit), kTcKChunk) * kTcKChunk;
   if (row_gather == nullptr) {  // operands by tensor copies
     TcTmaMaps maps;

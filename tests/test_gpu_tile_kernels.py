@@ -350,9 +350,14 @@ def test_router_and_route_of_the_layer(lib, E, k, T):
     assert scale > 1e-3 and max_abs <= 10 * 2.0 ** -11 * scale and mean_rel <= 5 * 2.0 ** -11, (max_abs, mean_rel, scale)
 
 
-# 64- and 128-wide tiles of the backbone GEMM: ragged rows, outputs and columns, one to many row tiles
-@pytest.mark.parametrize("n,k,m", [(33, 64, 64), (127, 192, 72), (129, 1032, 256), (300, 2048, 136), (1025, 512, 264), (2048, 1024, 128)])
-def test_backbone_gemm_at_tile_edges(lib, n, k, m):
+# 64- and 128-row tiles of the backbone GEMM: ragged rows, outputs and columns, one to many row tiles.  128: as many tiles as SMs, two
+# to sixteen chunks of columns in a ring of three; long rows whose columns are split into fours and eights.  73 clusters
+# of four do not run at once, nor are eighths of 8192 columns long enough: 64.
+@pytest.mark.parametrize("n,k,m,tile", [
+    (33, 64, 64, None), (127, 192, 72, 64), (129, 1032, 256, None), (300, 2048, 136, 64), (1025, 512, 264, 64), (2048, 1024, 128, 64),
+    (9601, 128, 256, 128), (9601, 256, 250, 128), (9601, 1024, 256, 128), (2480, 8192, 256, 128), (1500, 10240, 200, 128), (1500, 8192, 256, 64), (9304, 8192, 128, 64),
+])
+def test_backbone_gemm_at_tile_edges(lib, n, k, m, tile):
     import trismoe_b200 as tm
 
     g = torch.Generator().manual_seed(n + m)
@@ -360,9 +365,27 @@ def test_backbone_gemm_at_tile_edges(lib, n, k, m):
     w = (0.05 * torch.randn((m, k), generator=g)).half().cuda()
     ref, _, bound = _bound(w, x)
     _assert_within(tm.compute_shared_hidden(x, w), ref, bound)
+    if tile is not None:
+        (name, _), = kernels_of(lambda: tm.compute_shared_hidden(x, w))
+        assert "umma_gemm_tma_kernel<%d>" % tile in name
     for c in range(0, k, n):
         col = (torch.arange(n, device="cuda") + c) % k
         assert torch.equal(tm.compute_shared_hidden(torch.nn.functional.one_hot(col, k).half(), w), w.t()[col])
+
+
+@pytest.mark.parametrize("n,k,m", [(2480, 8192, 256), (1880, 8192, 250), (4000, 8192, 128), (1200, 8192, 128)])
+def test_backbone_gemm_of_gathered_long_rows(lib, n, k, m):
+    import trismoe_b200 as tm
+
+    g = torch.Generator().manual_seed(n + m)
+    rows = torch.randn((300, k), generator=g).half().cuda()
+    w = (0.05 * torch.randn((m, k), generator=g)).half().cuda()
+    gather = torch.randint(0, 300, (n,), generator=g).to(torch.int32).cuda()
+    out = torch.empty((n, m), dtype=torch.float16, device="cuda")
+    tm._native.check(lib.tris_shared_hidden_forward(rows.data_ptr(), gather.data_ptr(), n, None, k, w.data_ptr(), m, out.data_ptr(), 0,
+                                                    torch.cuda.current_stream().cuda_stream))
+    ref, _, bound = _bound(w, rows)
+    _assert_within(out, ref[gather.long()], bound[gather.long()])
 
 
 @pytest.mark.parametrize("T", [1, 16, 70])
