@@ -804,18 +804,31 @@ static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool 
 
 // Whether the weights-resident kernel is the faster one.  It pays about 5 us to start and its row tiles are 128 rows wide
 // whatever a segment has; the tiled kernel unpacks a segment's weights again for every pass, of 64 rows where that is typical.
-// us, tiled / wide, 64 experts, gate/up and down: 256 tokens (44 typical rows) 21.4 / 31.4, 21.6 / 26.3; 384 (62: tails of
-// 64-row passes) 35.3 / 32.2, 35.6 / 26.8; 509 (80) 28.2 / 32.4, 27.0 / 27.4; 700 (106) 46.1 / 36.7, 42.8 / 28.3; 2048 (288)
-// 93.5 / 56.7, 90.0 / 43.0.  One chunk of columns, 400 and 1000 tokens: 18.4 / 26.9, 17.6 / 20.4; 31.3 / 33.7, 34.1 / 24.6.  Three
-// chunks, 400 tokens: 46.4 / 37.4, 31.2 / 31.0.  As many segments as SMs are uneven whatever their mean: 256 experts, 256 and
-// 2048 tokens (43, 80) 56.4 / 48.6, 96.9 / 67.5; 69.7 / 56.8, 127 / 78.
+// So what counts is how many segments need one pass more than is typical, and whether the SMs have several units each to even that
+// out: many experts.  us, tiled / wide, 64 experts, gate/up and down: 256 tokens (44 typical rows) 21.4 / 31.4, 21.6 / 26.3; 384
+// (62: tails of 64-row passes) 35.3 / 32.2, 35.6 / 26.8; 509 (80) 28.2 / 32.4, 27.0 / 27.4; 700 (106) 46.1 / 36.7, 42.8 / 28.3;
+// 2048 (288) 93.5 / 56.7, 90.0 / 43.0.  Whole blocks, tiled / wide: 64 experts, 57, 60 and 62 typical rows 95 / 87, 84 / 87, 100 /
+// 88; 32 experts, 58, 62 and 70 53 / 64, 71 / 68, 65 / 70, at 110 and 120 66 / 70, 86 / 77; 8 experts, 106, 120 and 129 85 / 90, 94 /
+// 97, 115 / 104.  One chunk of columns, 64 experts, gate/up and down: 400 and 1000 tokens 18.4 / 26.9, 17.6 / 20.4; 31.3 / 33.7, 34.1 /
+// 24.6; blocks of 8 and 16 experts with down on either, 100 to 112 typical rows 67 / 67, 49 / 49 and 54 / 54, at 180 94 / 92, 58 / 56;
+// with gate/up on either, at 180, 260 and 400 94 / 98, 110 / 113, 159 / 157 and 56 / 60, 69 / 74, 88 / 94.  Three chunks, 64 experts, 400
+// tokens: 46.4 / 37.4, 31.2 / 31.0; 32 experts, 58, 70, 90 78 / 76, 72 / 72, 76 / 74; 16 experts, 80 54 / 54.
 static bool wide_is_faster(const TiledArgs& args, int mode, int typical_rows) {
-  if (args.chunks == 1) return typical_rows > (mode == MODE_SINGLE ? 96 : 160);
-  if (typical_rows > 96 || args.num_segments >= sm_count()) return true;
+  const bool single = mode == MODE_SINGLE, many = args.num_segments >= 64;
+  const int line = many ? 96 : (args.num_segments >= 32 ? 112 : 120);
+  if (!args.expert_ids) {  // an ordinary matrix: 4096 columns, 100 rows 21.1 / 18.8, a pair 24.2 / 22.5
+    if (args.chunks > kWideChunks) return typical_rows > 56;
+    return typical_rows > (args.chunks == kWideChunks || single ? 96 : 160);
+  }
+  if (args.chunks == 1) return typical_rows > (single ? line : (many ? 160 : 400));
+  // As many segments as SMs are uneven whatever their mean, but for gate/up the tiled kernel is the safer one as long as hardly any has a
+  // second pass: 256 experts, blocks of 735 to 800 tokens (33 to 35) 143 to 210 us with tiled kernels, 143 to 173 with down on the wide
+  // one, 154 to 158 with both (160 experts of 320 columns, 40: 124 / 128 / 140); from 820 (36) on the two are the same, 950 (41) 180 / 158 /
+  // 158, 2048 (80) 273 / 211 / 196.
+  if (args.num_segments >= sm_count()) return single || typical_rows > 40;
+  if (typical_rows > (args.chunks > kWideChunks ? 96 : line)) return true;
   if (typical_rows <= 56) return false;
-  // a few large experts are even, and their tails short: 8 experts, 192 tokens (62), the block 76 / 91
-  if (args.num_segments >= 32) return args.chunks > kWideChunks || typical_rows <= 64;
-  return args.chunks > kWideChunks && !args.expert_ids;  // 4096 columns, 100 rows: 21.1 / 18.8, a pair 24.2 / 22.5
+  return args.chunks > kWideChunks ? args.num_segments >= 32 : many && typical_rows <= 64;
 }
 template <int MODE>
 static int launch_wide(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {

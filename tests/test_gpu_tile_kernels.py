@@ -32,6 +32,9 @@ def _payload(tm, E, O, rank, group, seed):
     return tm.prepare_grouped_payload(p, "cuda")
 
 
+# Few experts on the tiled kernel, in passes of 64 and of 128 rows: more units than the decode kernel's passes are taken for.
+SHORT, UNEVEN = [130] + [43] * 31, [150, 50, 60, 65, 80, 55, 70, 30] * 4
+
 # (outputs, rank, scale group, rows per expert): decode kernel with 8 / 4 / 2 / 1 warps per 32 outputs and 8 to 32
 # rows per pass, a segment of several passes, more columns than one stage holds; tiled kernel with 64- and
 # 128-row tiles, ragged last tile, one to five column chunks, one to several tiles per CTA.
@@ -105,6 +108,52 @@ def test_grouped_kernels_give_every_single_weight(lib, O, rank, group, lengths):
         assert torch.equal(tm.run_grouped_structured_expert_forward(pa, ha, None, route), wa[expert, :, ca])
         sa, sb = tm.run_grouped_structured_expert_pair_forward(pa, pb, ha, hb, None, route)
         assert torch.equal(sa, wa[expert, :, ca]) and torch.equal(sb, wb[expert, :, cb])
+
+
+# Which kernel a call reaches, single projection and gate/up pair with SiLU: the rules by columns, experts and typical rows (mean and
+# two standard deviations), either side of each line.
+DECODE, TILED64, TILED128, WIDE_KERNEL = "grouped_decode_kernel<", "grouped_tiled_kernel<64,", "grouped_tiled_kernel<128,", "grouped_wide_kernel<"
+REACHES = [
+    (136, 128, [20] * 40, DECODE, DECODE),
+    (264, 128, [130] + [35] * 39, DECODE, DECODE),     # 50 typical rows, all passes at once
+    (520, 72, SHORT, TILED64, TILED64),                # 60
+    (520, 192, SHORT, TILED64, TILED64),
+    (520, 320, SHORT, WIDE_KERNEL, WIDE_KERNEL),
+    (520, 320, SHORT[:-1], TILED64, TILED64),          # one expert less
+    (416, 128, UNEVEN, TILED128, TILED128),            # 89
+    (416, 192, UNEVEN, TILED128, TILED128),
+    (416, 320, UNEVEN[:-1], TILED128, TILED128),
+    (416, 520, UNEVEN[:-1], TILED128, TILED128),
+    (1500, 128, [170] + [80] * 7, TILED128, TILED128), # 111, few experts
+    (1500, 192, [170] + [80] * 7, TILED128, TILED128),
+    (136, 128, [170] + [100] * 7, WIDE_KERNEL, TILED128),     # 130
+    (136, 192, [170] + [100] * 7, WIDE_KERNEL, WIDE_KERNEL),
+    (520, 192, [130] + [95] * 31, WIDE_KERNEL, WIDE_KERNEL),  # 116, 32 experts
+    (520, 192, [130] + [95] * 30, TILED128, TILED128),
+    (136, 128, [500] + [330] * 7, WIDE_KERNEL, TILED128),     # 389
+    (136, 128, [500] + [400] * 7, WIDE_KERNEL, WIDE_KERNEL),  # 454
+    (264, 192, [130] + [45] * 63, WIDE_KERNEL, WIDE_KERNEL),  # 60, many experts
+    (264, 192, [130] + [56] * 63, TILED128, TILED128),        # 73
+    (264, 192, [130] + [80] * 63, WIDE_KERNEL, WIDE_KERNEL),  # 99
+    (264, 128, [140] + [80] * 63, WIDE_KERNEL, TILED128),     # 99
+    (136, 128, [200] + [140] * 63, WIDE_KERNEL, WIDE_KERNEL), # 165
+    (136, 192, [130] + [24] * 149, WIDE_KERNEL, TILED64),     # 35, as many experts as SMs
+    (136, 192, [130] + [29] * 149, WIDE_KERNEL, WIDE_KERNEL), # 41
+]
+
+
+@pytest.mark.parametrize("O,rank,lengths,single,pair", REACHES)
+def test_calls_reach_the_kernel_they_are_meant_for(lib, O, rank, lengths, single, pair):
+    import trismoe_b200 as tm
+
+    pa, pb = (_payload(tm, len(lengths), O, rank, 64, seed) for seed in (1, 2))
+    h = torch.zeros((sum(lengths), rank), dtype=torch.float16, device="cuda")
+    route = tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda")
+    for want, run in ((single, lambda: tm.run_grouped_structured_expert_forward(pa, h, None, route)),
+                      (pair, lambda: tm.run_grouped_structured_expert_pair_forward(pa, pb, h, h, None, route, fuse_silu_mul=True))):
+        run()
+        names = [name for name, _ in kernels_of(run) if "grouped_" in name]
+        assert len(names) == 1 and want in names[0], names
 
 
 # Segments of many rows, unequal: one to six row tiles, more segments than a warp has lanes, columns that fit shared memory
