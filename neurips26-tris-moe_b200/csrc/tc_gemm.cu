@@ -508,7 +508,9 @@ static int clusters_at_once(bool alone, int ksplit) {
 // them are no longer than one of 64-row tiles that share it (8192 columns, 30 tiles 66 / 56; 32 tiles, a third turn, 66 / 80).
 static int rows_per_tile(int mtiles, int n, int k, bool gathered) {
   const int tiles128 = mtiles * ceil_div(n, 128), split128 = column_split(tiles128, k);
-  if (tiles128 >= kTcSms) return 128;
+  // as many as SMs: twice as many of 64 rows run at once too, and two to an SM hide each other's start (us, 64 / 128: 9472 x 1024 x 256
+  // 13.4 / 14.7, 9472 x 8192 x 256 54.2 / 60.4; with one more tile 20.4 / 15.5)
+  if (tiles128 >= kTcSms) return tiles128 == kTcSms && !gathered ? 64 : 128;
   if (tiles128 * 8 < kTcSms || k < (split128 == 8 && !gathered ? 10240 : 8192)) return 64;
   if (tiles128 <= (gathered ? 2 : 1) * clusters_at_once(gathered, split128)) return 128;
   const int tiles64 = mtiles * ceil_div(n, 64);

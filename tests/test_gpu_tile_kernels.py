@@ -399,12 +399,12 @@ def test_router_and_route_of_the_layer(lib, E, k, T):
     assert scale > 1e-3 and max_abs <= 10 * 2.0 ** -11 * scale and mean_rel <= 5 * 2.0 ** -11, (max_abs, mean_rel, scale)
 
 
-# 64- and 128-row tiles of the backbone GEMM: ragged rows, outputs and columns, one to many row tiles.  128: as many tiles as SMs, two
-# to sixteen chunks of columns in a ring of three; long rows whose columns are split into fours and eights.  73 clusters
+# 64- and 128-row tiles of the backbone GEMM: ragged rows, outputs and columns, one to many row tiles.  128: more tiles than SMs, two
+# to sixteen chunks of columns in a ring of three (as many as SMs exactly: 64); long rows whose columns are split into fours and eights.  73 clusters
 # of four do not run at once, nor are eighths of 8192 columns long enough: 64.
 @pytest.mark.parametrize("n,k,m,tile", [
     (33, 64, 64, None), (127, 192, 72, 64), (129, 1032, 256, None), (300, 2048, 136, 64), (1025, 512, 264, 64), (2048, 1024, 128, 64),
-    (9601, 128, 256, 128), (9601, 256, 250, 128), (9601, 1024, 256, 128), (2480, 8192, 256, 128), (1500, 10240, 200, 128), (1500, 8192, 256, 64), (9304, 8192, 128, 64),
+    (9601, 128, 256, 128), (9601, 256, 250, 128), (9601, 1024, 256, 128), (9472, 512, 256, 64), (2480, 8192, 256, 128), (1500, 10240, 200, 128), (1500, 8192, 256, 64), (9304, 8192, 128, 64),
 ])
 def test_backbone_gemm_at_tile_edges(lib, n, k, m, tile):
     import trismoe_b200 as tm
