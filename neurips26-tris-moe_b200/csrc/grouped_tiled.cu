@@ -43,6 +43,7 @@ struct Roles {
   static constexpr int kThreads = (kMma0 + kMmaWarps) * 32;
 };
 constexpr int kMaxStages = 4;
+constexpr bool splits_columns(int n) { return n == 64; }  // whether an ordinary matrix with columns to split can come here
 constexpr int kDBase = 4 * 2 * kACols;       // accumulators behind the four warpgroups' two slots
 constexpr int kBarBytes = 512;               // barriers and the TMEM address
 static_assert((2 * kMaxStages + 8 + 8 + 4 + 4 + kMmaWarps) * sizeof(uint64_t) + sizeof(uint32_t) <= kBarBytes, "barriers");
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(Roles<N>::kThreads, 1) grouped_tiled_kernel(co
           finish(half, y, 16);
         }
         if (i + 1 == steps) give_back();
-        if (!SILU && args.partial) {  // a part of the columns: fp32 sums, [part][projection][row][output]
+        if (splits_columns(N) && !SILU && args.partial) {  // a part of the columns: fp32 sums, [part][projection][row][output]
           const int o = (DUAL ? x : 2 * x + half) * kTileOut + row;
           float* dst = args.partial + (static_cast<size_t>(w.part * NC + (DUAL ? half : 0)) * args.num_rows + w.r0 + n0) * args.out_features + o;
 #pragma unroll
@@ -780,6 +781,21 @@ static int launch_main(const TiledArgs& args, int grid, size_t smem, cudaStream_
   return args.hidden_vec ? launch_rows<N, MODE, true>(args, grid, smem, stream, pdl) : launch_rows<N, MODE, false>(args, grid, smem, stream, pdl);
 }
 
+// Launches with the columns whole or split as args.col_split says: parts of gate and up are stored apart, the sum kernel
+// applies SiLU * up.
+template <int MODE, typename Launch>
+static int launch_and_sum(TiledArgs& args, cudaStream_t stream, const Launch& launch) {
+  if (args.col_split == 1) {
+    args.partial = nullptr;
+    return launch(std::integral_constant<int, MODE>{});
+  }
+  const int st = launch(std::integral_constant<int, MODE == MODE_DUAL_SILU ? MODE_DUAL_STORE : MODE>{});
+  if (st != TRIS_OK) return st;
+  const long long quads = static_cast<long long>(args.num_rows) * ceil_div(args.out_features, 4);
+  return check_cuda(launch_kernel(sum_parts_kernel<MODE>, dim3(static_cast<unsigned>((quads + 255) / 256)), dim3(256), 0, stream, /*pdl=*/true, 1, args),
+                    "sum_parts_kernel launch");
+}
+
 template <int N, int MODE>
 static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool pdl) {
   const size_t stage = stage_bytes<MODE>(args, N);
@@ -788,18 +804,17 @@ static int launch_tiled(TiledArgs args, int max_rows, cudaStream_t stream, bool 
   const size_t smem = kHeadBytes + args.stages * stage;
   const long long units = static_cast<long long>(args.units_x) * args.num_segments;
   args.row_split = row_split(units, max_rows, N);
-  args.col_split = col_split(args, MODE, units * args.row_split);
+  // ordinary matrices of so many columns and more than 56 rows go to the weights-resident kernel
+  args.col_split = splits_columns(N) ? col_split(args, MODE, units * args.row_split) : 1;
   args.pass_chunks = ceil_div(args.chunks, args.col_split);
   args.reuse = args.pass_chunks <= args.stages;
-  if (args.col_split == 1) args.partial = nullptr;
   const int grid = static_cast<int>(std::min<long long>(units * args.row_split * args.col_split, sm_count()));
-  if (!args.partial) return launch_main<N, MODE>(args, grid, smem, stream, pdl);
-  // parts of gate and up are stored apart; the sum kernel applies SiLU * up
-  const int st = launch_main<N, MODE == MODE_DUAL_SILU ? MODE_DUAL_STORE : MODE>(args, grid, smem, stream, pdl);
-  if (st != TRIS_OK) return st;
-  const long long quads = static_cast<long long>(args.num_rows) * ceil_div(args.out_features, 4);
-  return check_cuda(launch_kernel(sum_parts_kernel<MODE>, dim3(static_cast<unsigned>((quads + 255) / 256)), dim3(256), 0, stream, /*pdl=*/true, 1, args),
-                    "sum_parts_kernel launch");
+  if constexpr (splits_columns(N)) {
+    return launch_and_sum<MODE>(args, stream, [&](auto mode) { return launch_main<N, decltype(mode)::value>(args, grid, smem, stream, pdl); });
+  } else {
+    args.partial = nullptr;
+    return launch_main<N, MODE>(args, grid, smem, stream, pdl);
+  }
 }
 
 // Whether the weights-resident kernel is the faster one.  It pays about 5 us to start and its row tiles are 128 rows wide
@@ -837,15 +852,8 @@ static int launch_wide(TiledArgs args, int max_rows, cudaStream_t stream, bool p
   args.col_split = col_split(args, MODE, units * args.row_split);
   args.resident = ceil_div(args.chunks, args.col_split) <= kWideChunks;
   args.unit_cost = MODE == MODE_SINGLE ? 2 : 1;  // unpacking a unit against a row tile, whose SiLU is the longer epilogue (44.7 / 34.4 us, 45.9 / 37.6 us the other way round: 1024 tokens)
-  if (args.col_split == 1) args.partial = nullptr;
   const int grid = static_cast<int>(std::min<long long>(units * args.row_split * args.col_split, sm_count()));
-  if (!args.partial) return launch_grouped_wide(args, MODE, grid, stream, pdl);
-  // parts of gate and up are stored apart; the sum kernel applies SiLU * up
-  const int st = launch_grouped_wide(args, MODE == MODE_DUAL_SILU ? MODE_DUAL_STORE : MODE, grid, stream, pdl);
-  if (st != TRIS_OK) return st;
-  const long long quads = static_cast<long long>(args.num_rows) * ceil_div(args.out_features, 4);
-  return check_cuda(launch_kernel(sum_parts_kernel<MODE>, dim3(static_cast<unsigned>((quads + 255) / 256)), dim3(256), 0, stream, /*pdl=*/true, 1, args),
-                    "sum_parts_kernel launch");
+  return launch_and_sum<MODE>(args, stream, [&](auto mode) { return launch_grouped_wide(args, decltype(mode)::value, grid, stream, pdl); });
 }
 
 template <int MODE>
