@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import kernels_of
+from helpers import kernels_of, to_numpy_payload
 
 pytestmark = pytest.mark.gpu
 
@@ -24,11 +24,11 @@ def _assert_within(got, ref, bound):
     assert worst <= 1.0, worst
 
 
-def _payload(tm, E, O, rank, group, seed):
+def _payload(tm, E, O, rank, group, seed, **more):
     from trismoe_b200 import synth
 
     rng = np.random.default_rng(seed)
-    p = synth.pack_projection(synth.raw_projection(rng, E, O, rank, group_size=group))
+    p = synth.pack_projection(synth.raw_projection(rng, E, O, rank, group_size=group, **more))
     return tm.prepare_grouped_payload(p, "cuda")
 
 
@@ -37,7 +37,8 @@ SHORT, UNEVEN = [130] + [43] * 31, [150, 50, 60, 65, 80, 55, 70, 30] * 4
 
 # (outputs, rank, scale group, rows per expert): decode kernel with 8 / 4 / 2 / 1 warps per 32 outputs and 8 to 32
 # rows per pass, a segment of several passes, more columns than one stage holds; tiled kernel with 64- and
-# 128-row tiles, ragged last tile, one to five column chunks, one to several tiles per CTA.
+# 128-row tiles (the last seven lines: one to five column chunks, two passes and more), ragged last tile; kernel for long
+# segments; one to several tiles per CTA.
 GROUPED = [
     (96, 256, 32, [1, 0, 8, 3]),
     (97, 264, 128, [16, 9, 16]),
@@ -58,6 +59,13 @@ GROUPED = [
     (1031, 72, 32, [97, 33, 64]),
     (64, 1040, 64, [65, 0, 31]),
     (2048, 256, 128, [100]),
+    (520, 72, 32, SHORT),
+    (520, 192, 64, SHORT),
+    (520, 320, 128, SHORT[:-1]),
+    (416, 128, 64, UNEVEN),
+    (416, 192, 32, UNEVEN),
+    (416, 320, 128, UNEVEN[:-1]),
+    (416, 520, 64, UNEVEN[:-1]),
 ]
 
 
@@ -157,23 +165,38 @@ def test_calls_reach_the_kernel_they_are_meant_for(lib, O, rank, lengths, single
 
 
 # Segments of many rows, unequal: one to six row tiles, more segments than a warp has lanes, columns that fit shared memory
-# together (one or two chunks, the last one full or not) and columns that stream through it, an odd number of output tiles.
+# together (one or two chunks, the last one full or not) and columns that stream through it, an odd number of output tiles, as many
+# segments as SMs; one to four row-scale slots a chunk, none to eight steps of salient columns, column scales.
 WIDE = [
-    (264, 256, [300, 0, 5, 129, 700, 128]),
-    (1040, 192, [130 + 61 * (i % 7) for i in range(40)]),
-    (136, 72, [129, 513, 1]),
-    (520, 328, [257, 640, 384, 3]),
-    (264, 1032, [400, 129]),
+    (264, 256, 128, None, [300, 0, 5, 129, 700, 128]),
+    (1040, 192, 128, None, [130 + 61 * (i % 7) for i in range(40)]),
+    (136, 72, 128, None, [129, 513, 1]),
+    (520, 328, 128, None, [257, 640, 384, 3]),
+    (264, 1032, 128, None, [400, 129]),
+    (136, 72, 128, None, [640, 513, 129]),
+    (136, 192, 64, 0.1, [38 + i % 9 for i in range(150)]),
+    (264, 256, 32, 0.0, [300, 131]),
+    (264, 256, 32, 0.5, [131, 300]),
+    (136, 328, 32, 0.97, [257, 140]),
+    (264, 256, 64, 0.97, [300, 131]),
+    (136, 328, 64, 0.5, [140, 257]),
+    (136, 200, 96, 0.9, [300, 131]),
 ]
 
 
-@pytest.mark.parametrize("O,rank,lengths", WIDE)
-def test_long_and_unequal_segments(lib, O, rank, lengths):
+@pytest.mark.parametrize("O,rank,group,salient,lengths", WIDE)
+def test_long_and_unequal_segments(lib, O, rank, group, salient, lengths):
     import trismoe_b200 as tm
+    import trismoe_oracle as orc
+    from trismoe_b200 import synth
 
     E, R = len(lengths), sum(lengths)
-    pa, pb = _payload(tm, E, O, rank, 128, O + rank), _payload(tm, E, O, rank, 128, O + rank + 1)
+    more = {} if salient is None else {"p_salient": salient, "col_scale_one": False}
+    pa, pb = _payload(tm, E, O, rank, group, O + rank, **more), _payload(tm, E, O, rank, group, O + rank + 1, **more)
     wa, wb = tm.dequantize_grouped_payload(pa), tm.dequantize_grouped_payload(pb)
+    if more:  # groups and densities that no other test compares with the oracle
+        p = synth.pack_projection(synth.raw_projection(np.random.default_rng(O + rank), E, O, rank, group_size=group, **more))
+        assert np.array_equal(wa[E - 1].cpu().numpy(), orc.dequantize_expert(to_numpy_payload(p), E - 1))
     g = torch.Generator().manual_seed(R)
     ha, hb = ((0.5 * torch.randn((R, rank), generator=g)).half().cuda() for _ in range(2))
     route = tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda")
@@ -200,6 +223,86 @@ def test_long_and_unequal_segments(lib, O, rank, lengths):
             hot[rows] = torch.nn.functional.one_hot((torch.arange(n, device="cuda") + c) % rank, rank).half()
             col = (torch.arange(n, device="cuda") + c) % rank
             assert torch.equal(tm.run_grouped_structured_expert_forward(pa, hot, None, route)[rows], wa[e][:, col].T)
+
+
+@pytest.mark.parametrize("rank", [192, 328])
+def test_long_segments_with_every_option(lib, rank):
+    """Output scales and biases that differ by expert, gathered rows, a scale of the columns, outputs scattered or dropped, and rows
+    further apart than they are long."""
+    import ctypes as C
+
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    lengths, O = [300, 129, 1, 200], 264
+    E, R = len(lengths), sum(lengths)
+    g = torch.Generator().manual_seed(rank)
+    plain, payloads = [], []
+    for seed in (5, 6):
+        raw = synth.raw_projection(np.random.default_rng(seed), E, O, rank, group_size=64, col_scale_one=False)
+        plain.append(tm.prepare_grouped_payload(synth.pack_projection(raw), "cuda"))
+        p = synth.pack_projection(raw)
+        p["output_scale"], p["has_output_scale"] = (1 + 0.2 * torch.randn((E, O), generator=g)).half(), True
+        p["bias"], p["has_bias"] = (0.3 * torch.randn((E, O), generator=g)).half(), True
+        payloads.append(tm.prepare_grouped_payload(p, "cuda"))
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(lengths)).cuda()
+    route = dict(tm.qlinear_grouped._coerce_grouped_route(lengths, "cuda"))
+    rows = (0.5 * torch.randn((57, rank), generator=g)).half().cuda()
+    gather = torch.randint(0, 57, (R,), generator=g).to(torch.int32).cuda()
+    scatter = torch.randperm(R, generator=g).to(torch.int32).cuda()
+    scatter[::11] = -1
+    col = (1 + 0.2 * torch.randn((rank,), generator=g)).half().cuda()
+    kept = scatter >= 0
+    h = rows[gather.long()]
+
+    def check(x, p, outs, at):
+        """One projection, both of a pair and SiLU * up of rows ``at`` against the dequantised matrices, output scale and bias."""
+        refs = []
+        for q in p:
+            w = tm.dequantize_grouped_payload(q)
+            ref, acc = torch.zeros((R, O), dtype=torch.float64, device="cuda"), torch.zeros((R, O), dtype=torch.float64, device="cuda")
+            for e in range(E):
+                ref[expert == e], acc[expert == e], _ = _bound(w[e], x[expert == e])
+            if q["has_output_scale"]:
+                sc, b = q["output_scale"].double()[expert], q["bias"].double()[expert]
+                acc = acc * sc.abs() * (1 + 2.0 ** -22) + (ref * sc).abs() * 2.0 ** -22 + (ref * sc + b).abs() * 2.0 ** -22
+                ref = ref * sc + b
+            refs.append((ref[at], acc[at]))
+        for got, (ref, acc) in zip(outs[:3], (refs[0], *refs)):
+            _assert_within(got, ref, acc * (1 + 2.0 ** -10) + ref.abs() * 2.0 ** -11 + 2.0 ** -25)
+        (ra, ea), (rb, eb) = refs
+        silu = ra * torch.sigmoid(ra)
+        err = 1.1 * ea * rb.abs() + silu.abs() * eb + 1.1 * ea * eb + (silu * rb).abs() * (2.0 ** -11 + 2.0 ** -19) + 2.0 ** -25
+        _assert_within(outs[3], silu * rb, err)
+
+    def run(p, x, r):
+        one = tm.run_grouped_structured_expert_forward(p[0], x, None, r)
+        return one, *tm.run_grouped_structured_expert_pair_forward(p[0], p[1], x, x, None, r), tm.run_grouped_structured_expert_pair_forward(p[0], p[1], x, x, None, r, fuse_silu_mul=True)[0]
+
+    everything = torch.ones((R,), dtype=torch.bool, device="cuda")
+    check(h, payloads, run(payloads, h, route), everything)
+    check(h, payloads, run(payloads, rows, {**route, "_row_gather": gather}), everything)
+    for p in (plain, payloads):
+        check(h, p, [t[scatter[kept].long()] for t in run(p, h, {**route, "_out_row_scatter": scatter})], kept)
+    scaled = (h.float() * col.float()).half()  # the product of two halves is rounded once
+    check(scaled, payloads, run(payloads, h, {**route, "_hidden_col_scale": col}), everything)
+    # rows 16 columns further apart, by tensor copies and (pair of two sets) without
+    wide_rows = torch.full((R, rank + 16), float("nan"), dtype=torch.float16, device="cuda")
+    wide_rows[:, :rank] = h
+    want = run(payloads, h, route)
+    keep, va, vb = [], tm.qlinear_grouped.proj_view(payloads[0]), tm.qlinear_grouped.proj_view(payloads[1])
+    rv = tm.qlinear_grouped._route_view(route, R, keep)
+    rv.hidden_row_stride = rank + 16
+    got = [torch.empty_like(y) for y in want]
+    stream = torch.cuda.current_stream().cuda_stream
+    tm._native.check(lib.tris_grouped_forward(C.byref(va), C.byref(rv), wide_rows.data_ptr(), got[0].data_ptr(), stream))
+    others = wide_rows.clone()
+    tm._native.check(lib.tris_grouped_pair_forward(C.byref(va), C.byref(vb), C.byref(rv), wide_rows.data_ptr(), others.data_ptr(),
+                                                   got[1].data_ptr(), got[2].data_ptr(), 0, stream))
+    tm._native.check(lib.tris_grouped_pair_forward(C.byref(va), C.byref(vb), C.byref(rv), wide_rows.data_ptr(), wide_rows.data_ptr(),
+                                                   got[3].data_ptr(), None, 1, stream))
+    for y, w in zip(got, want):
+        assert torch.equal(y, w)
 
 
 @pytest.mark.parametrize("O,K,T", [(136, 520, 33), (137, 1100, 64), (1024, 2048, 65), (256, 4096, 130), (72, 8192, 300), (4096, 512, 257)])
