@@ -52,8 +52,9 @@ struct TiledArgs {
 
 // Eight columns (8 * piece ..) of an activation row that cannot be copied as it is; `left`: how many of them exist.
 // Permuted rows come in groups of 32 columns = 16 words of two halves 16 columns apart: a piece is the low or high
-// halves of eight of them, read word by word.  Half by half a single projection of 64 experts x 256 rows took 157 / 188 us
-// (pair-interleaved / lane order), now 118 / 135; 16-byte loads were no faster (113 / 132) and ask for more alignment.
+// halves of eight of them, read word by word.  Half by half a single projection of 64 experts x 256 rows took the
+// tiled kernel 157 / 188 us (pair-interleaved / lane order), word by word 118 / 135; 16-byte loads were no faster (113 / 132) and ask
+// for more alignment.
 static __device__ __noinline__ uint4 read_piece(const TiledArgs& args, const __half* chunk, int c0, int piece, int left) {
   if (args.hidden_perm) {
     if (left <= 0) return make_uint4(0u, 0u, 0u, 0u);  // rank % 32 == 0: a group exists as a whole

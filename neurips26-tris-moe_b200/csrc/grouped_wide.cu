@@ -5,17 +5,18 @@
 // launch), or two neighbouring tiles of one projection.  The activation rows are the M side of the MMA (128 rows = the
 // TMEM lanes), the weights the N side.  One persistent CTA per SM, its warps specialised:
 //
-//   unpack (16 warps)    two groups of eight warps take alternate chunks of 128 columns, a thread one output of each: code
+//   unpack (16 warps)    two groups of eight warps, each one 64-column slice of every chunk, a thread one output of one tile: code
 //                        words from the record straight to fp16 in shared memory, in the 128-byte swizzle the MMA reads; the
-//                        salient columns are then written over the +-0 the main unpack leaves there.  Two slots of a chunk;
+//                        salient columns are then written over the +-0 the main unpack leaves there.  Four slots of a slice,
+//                        that is two chunks;
 //   tables (1 warp)      column scales and a list of the salient columns, per chunk, for the unpack;
-//   loader (4 warps)     activation rows, 128 rows x 64 columns a stage, a ring of four: contiguous rows by tensor copies,
-//                        gathered ones by cp.async;
+//   loader (4 warps)     activation rows, 128 rows x 64 columns a stage, a ring of four: contiguous rows by tensor copies (one
+//                        warp), gathered ones by cp.async;
 //   MMA (1 warp)         tcgen05.mma, both operands from shared memory, accumulators [128 rows][2 x 128 outputs] in TMEM;
 //   epilogue (8 warps)   accumulators -> scale / bias or SiLU(gate) * up -> fp16 rows.  A TMEM lane is a row, so eight
 //                        outputs of a thread are 16 contiguous bytes.
 //
-// Up to 256 columns (the usual rank) the two slots hold all of them: a unit is unpacked once however many rows its segment
+// Up to 256 columns (the usual rank) the slots hold all of them: a unit is unpacked once however many rows its segment
 // has, row tiles follow one another and two accumulator buffers let the epilogue of one run under the MMAs of the next.
 // More columns stream through the slots; two row tiles at a time share a walk over the columns, each with an accumulator.
 //
@@ -25,11 +26,12 @@
 // 2048 tokens of 64 experts, gate/up and down: 56.5 / 43.6 us, against 93.5 / 90.0 on the tiled kernel, which unpacks for every
 // 128 rows and holds one accumulator buffer.  What bounds it: every role is a chain of dependent instructions, some 12
 // cycles each between the other warps' (30 warps, issue slots 43 % busy, tensor pipe 20 / 29 %).  Taking work out, at a time when the two launches took 63.9 /
-// 43.5: without the unpack 58 / 38, without the epilogue's work 46 / 32, without the products 57 / 38.  For segments of one row
-// tile the unpack of a unit is the longest chain (ALU pipe: byte permute, shift and two logic operations per two weights,
-// then 4 to 5 pairs of salient columns a slice), for longer ones the epilogue (SiLU: 8000 cycles a row tile) and the MMA
-// warp's control.  Slower: shifting by multiplication on the other pipe (down 43.5 -> 47), listing the salient pairs twice to save
-// the wrap-around (43.0 -> 46.9).
+// 43.5: without the unpack 58 / 38, without the epilogue's work 46 / 32, without the products 57 / 38.  Without unpack and
+// epilogue both 42 / 27: two thirds stay, the rows' way through loader, barriers and MMA warp, which every unit takes anew (gate/up
+// of 2048 tokens: 160 row tiles x 8 units x 2 sets x 64 KB = 164 MB through two stages in flight per SM).  An SM is active for 77
+// to 82 % of the longest one's time: units are shared out whole.
+// Slower: shifting by multiplication on the other pipe (down 43.5 -> 47), listing the salient pairs
+// twice to save the wrap-around (43.0 -> 46.9).
 #include <cuda.h>
 
 #include "grouped_tiled.cuh"

@@ -677,8 +677,7 @@ def tensor_core_from_64_rows(tm):
 
 @pytest.mark.parametrize("rank,T", [(96, 200), (256, 150), (64, 700)])
 def test_layer_prefill_rows_take_the_tensor_core_path(tm, tensor_core_from_64_rows, rank, T):
-    """Few experts, many tokens: ~100+ rows per expert, so the tcgen05 kernel over tile records runs (weights
-    unpacked to tensor memory)."""
+    """Few experts, many tokens: 75 to 350 rows per expert: passes of the decode kernel, the tiled kernel and the one for long segments."""
     from trismoe_b200 import synth
 
     shape = synth.LayerShape(256, 320, 4, 2, rank=rank, group_size=32)
@@ -780,8 +779,8 @@ def test_layer_prefill_on_planes(tm, rank, T, min_rows):
 
 
 def test_row_split_of_long_segments_leaves_results_unchanged(tm):
-    """Few experts with long, uneven segments (an expert-parallel rank's shape): the tiled kernel shares a unit's
-    row passes among up to four CTAs.  With the split switched off the outputs are the same
+    """Few experts with long, uneven segments (an expert-parallel rank's shape): up to four CTAs share a unit's
+    row passes.  With the split switched off the outputs are the same
     bits; segments of 1, 33, 70, 130 and 300 rows cover CTAs without a pass, a ragged last pass and CTAs with
     several passes; the result agrees with the fp32 oracle."""
     from trismoe_b200 import synth
