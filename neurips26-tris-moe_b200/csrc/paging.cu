@@ -202,16 +202,22 @@ __global__ void __launch_bounds__(32 * kPageWarps) code_blocks_kernel(const char
 using namespace tris;
 
 extern "C" int tris_page_code_blocks(const void* src_dev, int64_t bytes_per_expert, int32_t num_experts, int32_t* units_out, const int32_t* block_offsets,
-                                     void* dst_dev, void* stream) {
-  TRIS_REQUIRE(src_dev && (block_offsets ? dst_dev != nullptr : units_out != nullptr), TRIS_ERR_INVALID_ARG, "tris_page_code_blocks: null pointer");
+                                     void* dst, void* stream) {
+  TRIS_REQUIRE(src_dev && (block_offsets ? dst != nullptr : units_out != nullptr), TRIS_ERR_INVALID_ARG, "tris_page_code_blocks: null pointer");
   TRIS_REQUIRE(bytes_per_expert > 0 && (bytes_per_expert & 15) == 0 && num_experts >= 0, TRIS_ERR_INVALID_ARG, "tris_page_code_blocks: bad sizes");
-  TRIS_REQUIRE(((reinterpret_cast<uintptr_t>(src_dev) | reinterpret_cast<uintptr_t>(dst_dev)) & 15) == 0, TRIS_ERR_INVALID_ARG,
+  TRIS_REQUIRE(((reinterpret_cast<uintptr_t>(src_dev) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0, TRIS_ERR_INVALID_ARG,
                "tris_page_code_blocks: buffers must be 16-byte aligned");
   const long long blocks = (bytes_per_expert + kPageBlock - 1) / kPageBlock, total = blocks * num_experts;
   TRIS_REQUIRE(total * kPageUnits <= 0x7FFFFFFFll, TRIS_ERR_UNSUPPORTED, "tris_page_code_blocks: more than 2^31 16-byte units");
   if (total == 0) return TRIS_OK;
+  if (block_offsets) {  // pinned host memory: by its address on the device
+    cudaPointerAttributes at{};
+    TRIS_CUDA(cudaPointerGetAttributes(&at, dst));
+    TRIS_REQUIRE(at.type != cudaMemoryTypeUnregistered, TRIS_ERR_INVALID_ARG, "tris_page_code_blocks: the code needs device memory or pinned host memory");
+    if (at.type == cudaMemoryTypeHost) dst = at.devicePointer;
+  }
   code_blocks_kernel<<<static_cast<unsigned>((total + kPageWarps - 1) / kPageWarps), 32 * kPageWarps, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const char*>(src_dev), bytes_per_expert, static_cast<int>(blocks), total, units_out, block_offsets, static_cast<uint4*>(dst_dev));
+      static_cast<const char*>(src_dev), bytes_per_expert, static_cast<int>(blocks), total, units_out, block_offsets, static_cast<uint4*>(dst));
   return check_cuda(cudaGetLastError(), "code_blocks_kernel launch");
 }
 

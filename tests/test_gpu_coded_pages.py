@@ -56,6 +56,8 @@ def test_every_bit_comes_back(lib, per):
         assert lib.tris_page_coded_experts(jobs, 1, part.data_ptr(), None, part.numel(), E, table.data_ptr(), None) == 0
         torch.cuda.synchronize()
         assert torch.equal(dst[: part.numel()], bits[part.long()])
+    pageable = torch.empty((bits.numel() + 64,), dtype=torch.uint8)
+    assert lib.tris_page_code_blocks(bits.data_ptr(), per, E, None, offsets.data_ptr(), pageable.data_ptr(), None) == 1
     bad = (tm._native.TrisCodedPageJob * 1)()
     assert lib.tris_page_coded_experts(bad, 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
     assert lib.tris_page_coded_experts(C.cast(None, C.c_void_p), 1, ids.data_ptr(), None, 1, E, table.data_ptr(), None) == 1
