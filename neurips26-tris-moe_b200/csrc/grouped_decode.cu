@@ -20,9 +20,14 @@
 //
 // CTAs are small (four warps, five to seven CTAs per SM), so that the units of a decode batch are nearly
 // all resident at once and SMs are evenly loaded.  With few units the columns are split over KS warps
-// (partial sums added through shared memory): whole 128-column chunks over KS = 2, 64-column halves over
-// KS = 4 and 8.
+// (partial sums added through shared memory): whole 128-column chunks over KS = 2, 64-column halves over KS = 4.
+// Matrices of many columns and few outputs: the CTAs of a cluster take column parts of the same outputs too, and each
+// finishes its share of the sums from the others' shared memory (no scratch, no atomics, always the same order).
+#include <cooperative_groups.h>
+
 #include "grouped_tiled.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tris {
 namespace tr {
@@ -30,8 +35,8 @@ namespace tr {
 constexpr int kDecOut = 32;                                                  // outputs of a warp
 constexpr int dec_warps(int proj, int ks) { return proj * ks > 4 ? proj * ks : 4; }
 constexpr int dec_groups(int proj, int ks) { return dec_warps(proj, ks) / (proj * ks); }
-constexpr int dec_stage_cols(int ks) { return ks == 8 ? 512 : 256; }        // columns staged at a time
-constexpr int dec_row_bytes(int ks) { return 2 * dec_stage_cols(ks) + 16; }  // odd multiple of 16: conflict-free
+constexpr int kDecCols = 256;                     // columns staged at a time
+constexpr int kDecRowBytes = 2 * kDecCols + 16;  // odd multiple of 16: conflict-free
 // One buffer: [projection][chunk]{sub-records of the CTA's outputs, column record}, then [set][8 NT rows]
 struct DecodeLayout {
   int col_off, chunk_bytes, acts_off, acts_bytes, total;
@@ -40,8 +45,8 @@ __host__ __device__ inline DecodeLayout decode_layout(int max_sub_bytes, int max
   DecodeLayout l;
   l.col_off = dec_groups(nproj, ks) * max_sub_bytes;
   l.chunk_bytes = l.col_off + col_record_bytes(max_steps);
-  l.acts_off = nproj * (dec_stage_cols(ks) / kChunkCols) * l.chunk_bytes;
-  l.acts_bytes = 8 * nt * dec_row_bytes(ks);
+  l.acts_off = nproj * (kDecCols / kChunkCols) * l.chunk_bytes;
+  l.acts_bytes = 8 * nt * kDecRowBytes;
   l.total = l.acts_off + nset * l.acts_bytes;
   return l;
 }
@@ -52,18 +57,19 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
   return d;
 }
 
-constexpr int dec_min_ctas(int nt, int warps) { return (nt <= 2 ? 28 : 20) / warps; }
+// Warps that an SM should hold; a launch with column parts has no more than 14 for it.
+constexpr int dec_min_ctas(int nt, int warps, bool parts) { return (parts ? 16 : (nt <= 2 ? 28 : 20)) / warps; }
 
-// grid (groups of 32 * dec_groups outputs, segments, CTAs that share a segment's passes)
-template <int NT, int MODE, int KS>
-__global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), dec_min_ctas(NT, dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS)))
+// grid (groups of 32 * dec_groups outputs, segments, CTAs that share a segment's passes or, as a cluster, its columns)
+template <int NT, int MODE, int KS, bool kParts>
+__global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), dec_min_ctas(NT, dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS), kParts))
     grouped_decode_kernel(const __grid_constant__ TiledArgs args) {
   constexpr bool DUAL = MODE != MODE_SINGLE;
   constexpr int P = DUAL ? 2 : 1;
   constexpr int NW = dec_warps(P, KS), OG = dec_groups(P, KS), kThreads = 32 * NW;
   constexpr bool HALF = KS >= 4;                         // a warp takes one half of a chunk
   constexpr int CS = HALF ? KS / 2 : KS;                 // chunks are dealt to CS warps
-  constexpr int kCols = dec_stage_cols(KS), kRow = dec_row_bytes(KS);
+  constexpr int kCols = kDecCols, kRow = kDecRowBytes;
   constexpr int kGroupChunks = kCols / kChunkCols;
   extern __shared__ uint4 smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>(smem_raw);
@@ -80,7 +86,9 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
   };
   if (seg >= nseg) return leave();
   const int expert = args.expert_ids ? args.expert_ids[seg] : 0;  // no arrays: one segment of expert 0 with all rows
-  const int row_begin = (args.expert_ids ? args.segment_offsets[seg] : 0) + static_cast<int>(blockIdx.z) * 8 * NT;
+  // kParts: args.col_split neighbours along z, a cluster, share the columns
+  const int part = kParts ? static_cast<int>(blockIdx.z) % args.col_split : 0, first_pass = kParts ? static_cast<int>(blockIdx.z) / args.col_split : blockIdx.z;
+  const int row_begin = (args.expert_ids ? args.segment_offsets[seg] : 0) + first_pass * 8 * NT;
   const int row_end = args.expert_ids ? min(args.segment_offsets[seg + 1], args.num_rows) : args.num_rows;
   if (expert < 0 || expert >= args.num_experts || row_end <= row_begin) return leave();
 
@@ -92,7 +100,13 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
   const TrisProjView& v = args.proj[p];
   const int sub_bytes = v.max_record_bytes / kSubs, sal_off = record_slices(args.rank) * kSliceBytes, rows_off = sal_off + v.max_sal_words * kStepBytes;
   const DecodeLayout L = decode_layout(args.max_sub_bytes, args.max_steps, P, args.num_sets, NT, KS);
-  const int groups = (args.rank + kCols - 1) / kCols;
+  int gr_begin = 0, gr_end = (args.rank + kCols - 1) / kCols;
+  if (kParts) {
+    const int all = gr_end;
+    gr_begin = part * all / args.col_split;
+    gr_end = (part + 1) * all / args.col_split;
+  }
+  const bool ring = args.stages > 1;  // two buffers
   auto buffer = [&](int b) { return sm + b * L.total; };
 
   // Records of column group gr: per projection and chunk one linear run each of the tile and column record.
@@ -140,15 +154,17 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
     cp_async_commit();
   };
 
-  stage_weights(0, 0);
+  stage_weights(gr_begin, 0);
   if (args.weights_before_wait) {
     pdl_wait();
     pdl_launch_dependents();
   }
 
+  // Whether this CTA of a cluster writes rows 8 nt .. of outputs 16 m ..
+  auto finishes = [&](int m, int nt) { return !kParts || (2 * nt + m) % args.col_split == part; };
   int load = 0;  // column groups loaded so far
 #pragma unroll 1
-  for (int r0 = row_begin; r0 < row_end; r0 += 8 * NT * gridDim.z) {
+  for (int r0 = row_begin; r0 < row_end; r0 += 8 * NT * args.row_split) {
     const int rows = min(8 * NT, row_end - r0);
     float acc[2][NT][4];
 #pragma unroll
@@ -158,19 +174,20 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[m][nt][c] = 0.f;
     {
-      const int b = groups > 1 ? load & 1 : 0;
-      if (r0 != row_begin) {
-        __syncthreads();  // the previous pass has read its buffers and partial sums
-        stage_weights(0, b);
+      const int b = ring ? load & 1 : 0;
+      if (r0 != row_begin) {  // the previous pass has read its buffers and partial sums
+        if constexpr (kParts) cg::this_cluster().sync();
+        else __syncthreads();
+        stage_weights(gr_begin, b);
       }
-      stage_acts(0, b, r0, rows);
+      stage_acts(gr_begin, b, r0, rows);
     }
 #pragma unroll 1
-    for (int gr = 0; gr < groups; ++gr, ++load) {
-      const int b = groups > 1 ? load & 1 : 0;
+    for (int gr = gr_begin; gr < gr_end; ++gr, ++load) {
+      const int b = ring ? load & 1 : 0;
       cp_async_wait<0>();
       __syncthreads();
-      if (gr + 1 < groups) {  // the other buffer was read before the barrier
+      if (gr + 1 < gr_end) {  // the other buffer was read before the barrier
         stage_weights(gr + 1, b ^ 1);
         stage_acts(gr + 1, b ^ 1, r0, rows);
       }
@@ -267,7 +284,7 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
       for (int i = 0; i < 4; ++i) {
         const size_t at = static_cast<size_t>(expert) * args.out_features + min(o0 + g + 8 * i, args.out_features - 1);
         const float scale = v.output_scale ? __half2float(static_cast<const __half*>(v.output_scale)[at]) : 1.f;
-        const float bias = v.bias && ks == 0 ? __half2float(static_cast<const __half*>(v.bias)[at]) : 0.f;
+        const float bias = v.bias && ks == 0 && part == 0 ? __half2float(static_cast<const __half*>(v.bias)[at]) : 0.f;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -278,17 +295,17 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
     // (m = 1) for SiLU(gate) * up, by each projection's own warp otherwise; always by the ks = 0 warp.
     float up[NT][4];
     if constexpr (KS > 1 || MODE == MODE_DUAL_SILU) {
-      float4* part = reinterpret_cast<float4*>(sm);
-      auto slot_of = [&](int pp, int kk, int m, int nt) { return part + (((((pp * KS + kk) * OG + og) * 2 + m) * NT + nt) * 32 + lane); };
+      float4* sums = reinterpret_cast<float4*>(sm);
+      auto slot_of = [&](int pp, int kk, int m, int nt) { return sums + (((((pp * KS + kk) * OG + og) * 2 + m) * NT + nt) * 32 + lane); };
       __syncthreads();  // every warp is done with the activation rows
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        if (ks == 0 && (MODE != MODE_DUAL_SILU || m == p)) continue;
+        if (ks == 0 && (MODE != MODE_DUAL_SILU || m == p || kParts)) continue;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) *slot_of(p, ks, m, nt) = make_float4(acc[m][nt][0], acc[m][nt][1], acc[m][nt][2], acc[m][nt][3]);
       }
       __syncthreads();
-      if (ks > 0) continue;
+      if (ks > 0 && !kParts) continue;
       auto add = [&](float (&x)[4], const float4* q) {
         const float4 y = *q;
         x[0] += y.x;
@@ -296,23 +313,58 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
         x[2] += y.z;
         x[3] += y.w;
       };
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        if constexpr (MODE == MODE_DUAL_SILU) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (p) acc[0][nt][e] = acc[1][nt][e];  // the finished half is m = p
-            up[nt][e] = 0.f;
-          }
-#pragma unroll
-          for (int k = 1; k < KS; ++k) add(acc[0][nt], slot_of(p, k, p, nt));
-#pragma unroll
-          for (int k = 0; k < KS; ++k) add(up[nt], slot_of(p ^ 1, k, p, nt));
-        } else {
+      if constexpr (kParts) {
+        // sums of this CTA's columns, then of the cluster's: a CTA finishes every col_split-th eight rows of 16 outputs
+        cg::cluster_group cluster = cg::this_cluster();
+        if (ks == 0) {
 #pragma unroll
           for (int m = 0; m < 2; ++m)
 #pragma unroll
-            for (int k = 1; k < KS; ++k) add(acc[m][nt], slot_of(p, k, m, nt));
+            for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+              for (int k = 1; k < KS; ++k) add(acc[m][nt], slot_of(p, k, m, nt));
+              *slot_of(p, 0, m, nt) = make_float4(acc[m][nt][0], acc[m][nt][1], acc[m][nt][2], acc[m][nt][3]);
+            }
+        }
+        cluster.sync();
+        if (ks > 0 || !mine) continue;
+        auto total = [&](float (&x)[4], int pp, int m, int nt) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = 0.f;
+#pragma unroll 4
+          for (int z = 0; z < args.col_split; ++z) add(x, cluster.map_shared_rank(slot_of(pp, 0, m, nt), z));
+        };
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          if constexpr (MODE == MODE_DUAL_SILU) {
+            if (!finishes(p, nt)) continue;
+            total(acc[0][nt], p, p, nt);
+            total(up[nt], p ^ 1, p, nt);
+          } else {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+              if (finishes(m, nt)) total(acc[m][nt], p, m, nt);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          if constexpr (MODE == MODE_DUAL_SILU) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (p) acc[0][nt][e] = acc[1][nt][e];  // the finished half is m = p
+              up[nt][e] = 0.f;
+            }
+#pragma unroll
+            for (int k = 1; k < KS; ++k) add(acc[0][nt], slot_of(p, k, p, nt));
+#pragma unroll
+            for (int k = 0; k < KS; ++k) add(up[nt], slot_of(p ^ 1, k, p, nt));
+          } else {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+              for (int k = 1; k < KS; ++k) add(acc[m][nt], slot_of(p, k, m, nt));
+          }
         }
       }
     }
@@ -324,7 +376,7 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
     for (int m = 0; m < kHalves; ++m) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        if (nt * 8 < rows) {
+        if (nt * 8 < rows && finishes(MODE == MODE_DUAL_SILU ? p : m, nt)) {
           float y[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -359,21 +411,23 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
       }
     }
   }
+  if constexpr (kParts) cg::this_cluster().sync();  // shared memory stays until the others have read their sums
 }
 
-template <int NT, int MODE, int KS>
-static int launch_decode(const TiledArgs& args, cudaStream_t stream, bool pdl) {
+template <int NT, int MODE, int KS, bool kParts = false>
+static int launch_decode(TiledArgs args, cudaStream_t stream, bool pdl, int col_split = 1) {
   constexpr int P = MODE == MODE_SINGLE ? 1 : 2;
-  const int bufs = args.rank > dec_stage_cols(KS) ? 2 : 1;
+  args.col_split = col_split;
+  args.stages = args.rank > kDecCols * col_split ? 2 : 1;  // col_split is no more than there are groups: every CTA has one
   const int part = (KS > 1 || MODE == MODE_DUAL_SILU) ? dec_warps(P, KS) * 2 * NT * 512 : 0;
-  const size_t smem = std::max(bufs * decode_layout(args.max_sub_bytes, args.max_steps, P, args.num_sets, NT, KS).total, part);
+  const size_t smem = std::max(args.stages * decode_layout(args.max_sub_bytes, args.max_steps, P, args.num_sets, NT, KS).total, part);
   TRIS_REQUIRE(smem <= kMostSmem, TRIS_ERR_UNSUPPORTED, "grouped_decode_kernel: %zu bytes of shared memory", smem);
-  auto kernel = grouped_decode_kernel<NT, MODE, KS>;
+  auto kernel = grouped_decode_kernel<NT, MODE, KS, kParts>;
   static std::atomic<size_t> configured[64] = {};  // per instantiation, per device: largest size set so far
   int st = configure_smem(kernel, smem, configured);
   if (st != TRIS_OK) return st;
-  return check_cuda(launch_kernel(kernel, dim3(ceil_div(args.out_features, kDecOut * dec_groups(P, KS)), args.num_segments, args.row_split), dim3(32 * dec_warps(P, KS)),
-                                  smem, stream, pdl, 1, args),
+  return check_cuda(launch_kernel(kernel, dim3(ceil_div(args.out_features, kDecOut * dec_groups(P, KS)), args.num_segments, args.row_split * col_split), dim3(32 * dec_warps(P, KS)),
+                                  smem, stream, pdl, col_split, args),
                     "grouped_decode_kernel launch");
 }
 
@@ -382,8 +436,16 @@ static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) 
   // Fewer than 14 warps per SM: split the columns, as far as there are columns to split.  Shared passes have the widest
   // tile, of which 20 warps fit an SM instead of 28: fewer than 10.
   const long long warps = decode_warps(args, MODE) * args.row_split;
-  const int slices = ceil_div(args.rank, kSliceCols), want = (args.row_split > 1 ? 10 : 14) * sm_count();
-  if (warps * 4 < want && slices >= 16) return launch_decode<NT, MODE, 8>(args, stream, pdl);
+  const int slices = ceil_div(args.rank, kSliceCols), groups = ceil_div(args.rank, kDecCols), want = (args.row_split > 1 ? 10 : 14) * sm_count();
+  // Many columns: over the CTAs of a cluster too, by 256 columns or more each, up to as many warps as above.  us at 8 rows, eight warps to
+  // 32 outputs in one CTA / this: 4096 x 4096 18.6 / 11.2, pair of 1024 x 4096 25.8 / 8.4, pair of 2048 x 2048 14.4 / 8.1, 512 x 1024 6.2 /
+  // 4.6, 256 x 8192 33.9 / 8.2 (clusters of 1, 2, 4 and 8 CTAs in an earlier form: 4096 x 4096 24.5, 15.7, 12.0, 13.8; pair of 2048 x 2048
+  // 18.1, 11.5, 8.6, 12.0).  With 512 columns two CTAs are no faster than one (2048 x 512, 8 and 24 rows 5.0 / 5.0, 6.6 / 7.5).
+  if (warps * 8 <= want && groups >= 4) {
+    int parts = 2;
+    while (parts < 8 && warps * 8 * parts <= want && groups >= 2 * parts) parts *= 2;
+    return launch_decode<NT, MODE, 4, true>(args, stream, pdl, parts);
+  }
   if (warps * 2 < want && slices >= 4) return launch_decode<NT, MODE, 4>(args, stream, pdl);
   if (warps < want && slices >= 4) return launch_decode<NT, MODE, 2>(args, stream, pdl);
   return launch_decode<NT, MODE, 1>(args, stream, pdl);

@@ -482,7 +482,7 @@ def _route_view(route: dict, num_rows: int, keep: list) -> TrisRouteView:
 
 def _linear_workspace(lib, view: TrisProjView, projections: int, rows: int, dev) -> Optional[torch.Tensor]:
     """Scratch of an ordinary matrix whose columns are shared among CTAs; None where they are not (32 rows
-    or fewer among others: the decode kernel shares them inside a CTA)."""
+    or fewer among others: the decode kernel shares them inside a CTA or a cluster)."""
     if rows <= 32:
         return None
     need = int(lib.tris_linear_workspace_bytes(C.byref(view), projections, rows))

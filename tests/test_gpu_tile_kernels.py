@@ -342,6 +342,25 @@ def test_linear_columns_shared_among_ctas(lib, O, K, T):
         assert torch.equal(mods[0](hot), want[0]) and torch.equal(a, want[0]) and torch.equal(b, want[1])
 
 
+@pytest.mark.parametrize("O,K,T", [(40, 1024, 1), (33, 1040, 7), (136, 2300, 17), (72, 8192, 32), (1000, 1536, 24), (4096, 1100, 16), (96, 1288, 9)])
+def test_linear_columns_shared_by_a_cluster(lib, O, K, T):
+    """An ordinary matrix of up to 32 rows: its columns over two, four and eight CTAs, in equal and unequal parts; the bias once."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    test_linear_columns_shared_among_ctas(lib, O, K, T)
+    rng = np.random.default_rng(O)
+    p = synth.pack_projection(synth.raw_projection(rng, 1, O, K, group_size=128))
+    bias = torch.from_numpy(rng.standard_normal(O).astype(np.float16))
+    lin = tm.Compact3Linear(p, bias=bias, device="cuda")
+    x = (0.5 * torch.randn((T, K), generator=torch.Generator().manual_seed(T))).half().cuda()
+    y = lin(x)
+    ref, err, _ = _bound(tm.dequantize_grouped_payload(lin.payload)[0], x)
+    ref = ref + bias.cuda().double()
+    _assert_within(y, ref, err * (1 + 2.0 ** -10) + ref.abs() * (2.0 ** -11 + 2.0 ** -22) + 2.0 ** -25)
+    assert all(torch.equal(lin(x), y) for _ in range(3))
+
+
 @pytest.mark.parametrize("O,K,T,pair", [(1024, 2048, 256, False), (512, 2048, 512, True), (2048, 512, 300, False), (264, 1032, 129, True)])
 def test_linear_parts_fill_the_gpu(lib, O, K, T, pair):
     """Rows in parts of 128, columns in as many parts as the SMs and two chunks a part allow."""
