@@ -634,6 +634,27 @@ int tris_moe_layer_forward_extras_status(const TrisMoeLayerView* layer, const Tr
                                          int32_t* status_dev, void* stream);
 
 /*
+ * The same launch sequence with one always-on shared expert, the dense MLP of Qwen2-MoE blocks: gate and up [I_s, H] and down
+ * [H, I_s] are ordinary compact3 matrices with tile records, joined as tris_shared_expert_add does it
+ * (modeling_qwen2_moe.py:815-818).  The workspace holds the expert's rows too
+ * (tris_moe_layer_shared_workspace_bytes); scratch: as for tris_linear_forward, as many bytes as
+ * tris_linear_workspace_bytes names for either launch, or NULL; not used after the call's last kernel.
+ */
+typedef struct TrisSharedExpert {
+  const TrisProjView* gate;
+  const TrisProjView* up;
+  const TrisProjView* down;
+  const void* gate_weight; /* fp16 [H] */
+} TrisSharedExpert;
+
+size_t tris_moe_layer_shared_workspace_bytes(const TrisMoeLayerView* layer, const TrisSharedExpert* shared,
+                                             int32_t num_tokens);
+int tris_moe_layer_forward_shared(const TrisMoeLayerView* layer, const TrisSharedExpert* shared, const void* x_f16,
+                                  const float* router_logits, int32_t num_tokens, void* y_f16,
+                                  float* router_logits_out, void* workspace, size_t workspace_bytes, void* scratch,
+                                  size_t scratch_bytes, void* stream);
+
+/*
  * Same computation as tris_moe_layer_forward for callers that cannot provide a workspace
  * because they are not allowed to allocate device memory: for example a serving process
  * whose memory pool claimed the whole GPU at start-up (a later cudaMalloc fails or

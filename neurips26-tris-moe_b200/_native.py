@@ -79,6 +79,10 @@ class TrisMoeLayerExtras(C.Structure):
     _fields_ = [("input_scale", _vp * 3), ("ns_c2", _vp * 3), ("ns_c1", _vp * 3)]
 
 
+class TrisSharedExpert(C.Structure):
+    _fields_ = [("gate", _vp), ("up", _vp), ("down", _vp), ("gate_weight", _vp)]
+
+
 # name -> (restype, argtypes); also the list of symbols include/trismoe_b200.h declares.
 _P = C.POINTER
 SIGNATURES = {
@@ -131,6 +135,8 @@ SIGNATURES = {
     "tris_moe_layer_extras_workspace_bytes": (C.c_size_t, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _i32]),
     "tris_moe_layer_forward_extras": (C.c_int, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp]),
     "tris_moe_layer_forward_extras_status": (C.c_int, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp, _vp]),
+    "tris_moe_layer_shared_workspace_bytes": (C.c_size_t, [_P(TrisMoeLayerView), _P(TrisSharedExpert), _i32]),
+    "tris_moe_layer_forward_shared": (C.c_int, [_P(TrisMoeLayerView), _P(TrisSharedExpert), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp, C.c_size_t, _vp]),
     "tris_moe_layer_forward_static": (C.c_int, [_P(TrisMoeLayerView), _vp, _vp, _i32, _vp, _vp, _vp]),
 }
 STATIC_SCRATCH_BYTES = 8 << 20

@@ -113,6 +113,7 @@ int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRou
 struct LaunchOpts {
   bool pdl = false;                  // programmatic dependent launch
   bool weights_before_wait = false;  // the route was complete before the predecessor kernel started
+  bool rows_ready = false;           // and so were the activation rows: only the stores have to wait (a hint; needs weights_before_wait)
   void* workspace = nullptr;         // scratch of the column split (grouped_split_bytes), optional
   size_t workspace_bytes = 0;
 };
@@ -135,6 +136,10 @@ int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t 
 int combine_routed_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,
                         int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream, bool pdl,
                         bool indices_ready = false);
+// The same joined with a shared expert's rows: out = combined + sigmoid(x . gate_weight) * shared.
+int combine_shared_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights, int num_tokens, int top_k,
+                        int hidden_size, const void* x_f16, const void* gate_weight_f16, const void* shared_f16, void* final_f16,
+                        cudaStream_t stream);
 int launch_router_route(const float* logits, int num_tokens, int num_experts, int top_k, int norm, int m_tile,
                         int32_t* selected, float* weights, int32_t* perm, int32_t* tok, int32_t* slot,
                         int32_t* row_of_flat, int32_t* expert_ids, int32_t* segment_offsets, int32_t* problem_offsets,

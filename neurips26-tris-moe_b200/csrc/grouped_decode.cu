@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
 
   stage_weights(gr_begin, 0);
   if (args.weights_before_wait) {
-    pdl_wait();
+    if (!kParts || !args.rows_ready) pdl_wait();
     pdl_launch_dependents();
   }
 
@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
     }
     if (!mine) continue;
 
+    if (kParts && args.rows_ready) pdl_wait();
     // epilogue: a 16-output half holds {(output g, row 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1)}
     constexpr int kHalves = MODE == MODE_DUAL_SILU ? 1 : 2;
 #pragma unroll
@@ -441,9 +442,10 @@ static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) 
   // 32 outputs in one CTA / this: 4096 x 4096 18.6 / 11.2, pair of 1024 x 4096 25.8 / 8.4, pair of 2048 x 2048 14.4 / 8.1, 512 x 1024 6.2 /
   // 4.6, 256 x 8192 33.9 / 8.2 (clusters of 1, 2, 4 and 8 CTAs in an earlier form: 4096 x 4096 24.5, 15.7, 12.0, 13.8; pair of 2048 x 2048
   // 18.1, 11.5, 8.6, 12.0).  With 512 columns two CTAs are no faster than one (2048 x 512, 8 and 24 rows 5.0 / 5.0, 6.6 / 7.5).
-  if (warps * 8 <= want && groups >= 4) {
-    int parts = 2;
-    while (parts < 8 && warps * 8 * parts <= want && groups >= 2 * parts) parts *= 2;
+  // Rows that are ready before the kernel ahead has ended: that variant too, as a cluster of one at least, so that the others need not look.
+  if (warps * 8 <= want && (groups >= 4 || args.rows_ready)) {
+    int parts = 1;
+    while (parts < 8 && warps * 8 * parts <= want && groups >= 2 * parts && groups >= 4) parts *= 2;
     return launch_decode<NT, MODE, 4, true>(args, stream, pdl, parts);
   }
   if (warps * 2 < want && slices >= 4) return launch_decode<NT, MODE, 4>(args, stream, pdl);

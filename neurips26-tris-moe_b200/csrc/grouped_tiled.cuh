@@ -38,6 +38,7 @@ struct TiledArgs {
   int32_t hidden_perm;          // rows in a permuted order that can be read word by word
   int32_t num_sets;             // 2 when the two projections read different activation rows
   int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
+  int32_t rows_ready;           // decode kernel with column parts: activation rows too, only the stores wait
   int32_t stages;               // ring depth, 2 .. kMaxStages
   int32_t reuse;                // the chunks of a pass fit the ring: staged once for all tiles of a run
   int32_t rows_by_tensor;       // wide kernel: contiguous activation rows come by tensor copies

@@ -554,19 +554,14 @@ int launch_router_route(const float* logits, int num_tokens, int num_experts, in
                                   segment_offsets, problem_offsets, counts, stream);
 }
 
-// out = routed + sigmoid(x . gate) * shared, one CTA per token; the dot product, the sigmoid and the product are rounded
-// to fp16 where separate operators round them.  Four small launches (matrix-vector product, sigmoid, product,
-// sum) cost 30 us of host time; the data is a few hundred KB.
-__global__ void __launch_bounds__(256) shared_expert_add_kernel(const __half* x, const __half* gate, const __half* routed, const __half* shared,
-                                                                int hidden, int vec, __half* out) {
+// sigmoid(x . gate) of one row by a CTA of 256 threads, in both halves; dot product and sigmoid are rounded to fp16 where separate
+// operators round them.
+__device__ __forceinline__ __half2 shared_gate_of(const __half* x, const __half* gate, int hidden, bool vec) {
   __shared__ float parts[8];
-  pdl_wait();
-  pdl_launch_dependents();
-  const size_t row = static_cast<size_t>(blockIdx.x) * hidden;
   float sum = 0.f;
   if (vec) {
     for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8) {
-      const uint4 a = *reinterpret_cast<const uint4*>(x + row + c), b = *reinterpret_cast<const uint4*>(gate + c);
+      const uint4 a = *reinterpret_cast<const uint4*>(x + c), b = *reinterpret_cast<const uint4*>(gate + c);
       const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -575,7 +570,7 @@ __global__ void __launch_bounds__(256) shared_expert_add_kernel(const __half* x,
       }
     }
   } else {
-    for (int c = threadIdx.x; c < hidden; c += 256) sum += __half2float(x[row + c]) * __half2float(gate[c]);
+    for (int c = threadIdx.x; c < hidden; c += 256) sum += __half2float(x[c]) * __half2float(gate[c]);
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
   if ((threadIdx.x & 31) == 0) parts[threadIdx.x >> 5] = sum;
@@ -584,15 +579,78 @@ __global__ void __launch_bounds__(256) shared_expert_add_kernel(const __half* x,
 #pragma unroll
   for (int i = 0; i < 8; ++i) sum += parts[i];
   const float z = __half2float(__float2half_rn(sum));
-  const __half2 s = __half2half2(__float2half_rn(1.f / (1.f + expf(-z))));
+  return __half2half2(__float2half_rn(1.f / (1.f + expf(-z))));
+}
+__device__ __forceinline__ uint4 add_scaled(const uint4& a, __half2 s, const uint4& b) {
+  auto one = [&](uint32_t r, uint32_t v) { return h2_as_u32(__hadd2_rn(u32_as_h2(r), __hmul2_rn(s, u32_as_h2(v)))); };
+  return make_uint4(one(a.x, b.x), one(a.y, b.y), one(a.z, b.z), one(a.w, b.w));
+}
+
+// out = routed + sigmoid(x . gate) * shared, one CTA per token; the product is rounded to fp16 too.
+// Four small launches (matrix-vector product, sigmoid, product, sum) cost 30 us of host time; the data is a few hundred KB.
+__global__ void __launch_bounds__(256) shared_expert_add_kernel(const __half* x, const __half* gate, const __half* routed, const __half* shared,
+                                                                int hidden, int vec, __half* out) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const size_t row = static_cast<size_t>(blockIdx.x) * hidden;
+  const __half2 s = shared_gate_of(x + row, gate, hidden, vec);
   if (vec) {
-    for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8) {
-      const uint4 a = *reinterpret_cast<const uint4*>(routed + row + c), b = *reinterpret_cast<const uint4*>(shared + row + c);
-      auto one = [&](uint32_t r, uint32_t v) { return h2_as_u32(__hadd2_rn(u32_as_h2(r), __hmul2_rn(s, u32_as_h2(v)))); };
-      *reinterpret_cast<uint4*>(out + row + c) = make_uint4(one(a.x, b.x), one(a.y, b.y), one(a.z, b.z), one(a.w, b.w));
-    }
+    for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8)
+      *reinterpret_cast<uint4*>(out + row + c) =
+          add_scaled(*reinterpret_cast<const uint4*>(routed + row + c), s, *reinterpret_cast<const uint4*>(shared + row + c));
   } else {
     for (int c = threadIdx.x; c < hidden; c += 256) out[row + c] = __hadd_rn(routed[row + c], __hmul_rn(__low2half(s), shared[row + c]));
+  }
+}
+
+// The combine and that sum in one launch of the layer sequence, where x, the gate and the route are older than the kernel before:
+// one CTA per token, whose gate is there when the rows are.
+__global__ void __launch_bounds__(256) combine_shared_kernel(const __half* rows, const int32_t* row_of_flat, const float* weights, int top_k,
+                                                             int hidden, const __half* x, const __half* gate, int vec, const __half* shared,
+                                                             __half* out) {
+  const int t = blockIdx.x;
+  const size_t row = static_cast<size_t>(t) * hidden;
+  const __half2 s = shared_gate_of(x + row, gate, hidden, vec);
+  int r[8];
+  float w[8];
+  auto slots = [&](int s0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const bool in = s0 + j < top_k;
+      r[j] = in ? row_of_flat[t * top_k + s0 + j] : -1;
+      w[j] = in ? weights[t * top_k + s0 + j] : 0.f;
+    }
+  };
+  slots(0);
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8) {
+    const uint4 b = *reinterpret_cast<const uint4*>(shared + row + c);
+    float acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc[u] = 0.f;
+    for (int s0 = 0; s0 < top_k; s0 += 8) {
+      if (top_k > 8) slots(s0);
+      uint4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = r[j] >= 0 ? *reinterpret_cast<const uint4*>(rows + static_cast<size_t>(r[j]) * hidden + c) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const __half2* h2 = reinterpret_cast<const __half2*>(&v[j]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float2 f = __half22float2(h2[u]);
+          acc[2 * u] += w[j] * f.x;
+          acc[2 * u + 1] += w[j] * f.y;
+        }
+      }
+    }
+    uint4 o;
+    __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) oh[u] = __floats2half2_rn(acc[2 * u], acc[2 * u + 1]);
+    *reinterpret_cast<uint4*>(out + row + c) = add_scaled(o, s, b);
   }
 }
 
@@ -756,6 +814,18 @@ int tris::combine_routed_impl(const void* down_out_f16, const int32_t* row_of_fl
                                   row_of_flat, routing_weights, num_tokens, top_k, hidden_size,
                                   static_cast<__half*>(final_f16)),
                     "combine_routed_kernel launch");
+}
+
+int tris::combine_shared_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights, int num_tokens, int top_k,
+                              int hidden_size, const void* x_f16, const void* gate_weight_f16, const void* shared_f16, void* final_f16,
+                              cudaStream_t stream) {
+  TRIS_REQUIRE((hidden_size & 7) == 0, TRIS_ERR_UNSUPPORTED, "moe layer with a shared expert: hidden_size must be a multiple of 8");
+  const int vec = ((reinterpret_cast<uintptr_t>(x_f16) | reinterpret_cast<uintptr_t>(gate_weight_f16)) & 15u) == 0;
+  return check_cuda(launch_kernel(combine_shared_kernel, dim3(num_tokens), dim3(256), 0, stream, /*pdl=*/true, 1,
+                                  static_cast<const __half*>(down_out_f16), row_of_flat, routing_weights, top_k, hidden_size,
+                                  static_cast<const __half*>(x_f16), static_cast<const __half*>(gate_weight_f16), vec,
+                                  static_cast<const __half*>(shared_f16), static_cast<__half*>(final_f16)),
+                    "combine_shared_kernel launch");
 }
 
 extern "C" int tris_combine_routed(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,

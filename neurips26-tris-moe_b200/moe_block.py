@@ -17,7 +17,7 @@ import torch
 from torch import nn
 
 from . import _native, envflags
-from ._native import TrisMoeLayerExtras, TrisMoeLayerView
+from ._native import TrisMoeLayerExtras, TrisMoeLayerView, TrisSharedExpert
 from .ns_compensation import Packed4Linear
 from .qlinear_grouped import (
     build_grouped_route,
@@ -233,13 +233,17 @@ class TrisSparseMoeBlock(nn.Module):
                 ex.ns_c2[i], ex.ns_c1[i] = C.addressof(c2), C.addressof(c1)
         return ex
 
-    def workspace(self, num_tokens: int, device) -> torch.Tensor:
+    def workspace(self, num_tokens: int, device, shared: Optional[TrisSharedExpert] = None) -> torch.Tensor:
         view = self.layer_view()
-        sized = self._workspace_for  # (view, tokens) the buffer is known to hold: the size grows with the tokens
-        if sized is not None and sized[0] is view and num_tokens <= sized[1] and self._workspace is not None and self._workspace.device == device:
+        width = 0 if shared is None else C.cast(shared.gate, C.POINTER(_native.TrisProjView))[0].out_features
+        sized = self._workspace_for  # (view, shared expert's width, tokens) the buffer is known to hold: the size grows with the tokens
+        if sized is not None and sized[0] is view and sized[1] == width and num_tokens <= sized[2] and self._workspace is not None and self._workspace.device == device:
             return self._workspace
         lib = _native.load()
-        need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), int(num_tokens)))
+        if shared is None:
+            need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), int(num_tokens)))
+        else:
+            need = int(lib.tris_moe_layer_shared_workspace_bytes(C.byref(view), C.byref(shared), int(num_tokens)))
         if need == 0 and num_tokens > 0:
             raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
         if self._workspace is None or self._workspace.numel() < need or self._workspace.device != device:
@@ -247,7 +251,7 @@ class TrisSparseMoeBlock(nn.Module):
                 self.raise_on_kernel_status()  # do not lose a report with the old buffer
             self._workspace = torch.empty((need,), dtype=torch.uint8, device=device)
             self._workspace[:16].zero_()  # count words and the sticky status word
-        self._workspace_for = (view, int(num_tokens))
+        self._workspace_for = (view, width, int(num_tokens))
         return self._workspace
 
     def _extras_workspace(self, num_tokens: int, device, extras: TrisMoeLayerExtras) -> torch.Tensor:
@@ -305,6 +309,10 @@ class TrisSparseMoeBlock(nn.Module):
         """Returns ``(final_hidden_states [B, S, H], router_logits [T, E])`` like
         ``OlmoeSparseMoeBlock.forward`` (modeling_olmoe.py:1046-1105).  ``router_logits``
         (fp32 ``[T, E]``) may be passed in to skip the router linear."""
+        return self._forward(hidden_states, router_logits)
+
+    def _forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor], shared: Optional[TrisSharedExpert] = None):
+        """``shared``: a shared expert that joins the launch sequence (blocks without scales and pairs only)."""
         _native.require_cuda(hidden_states, "TrisSparseMoeBlock.forward")
         with_extras = bool(self.input_scales or self.ns_payloads)
         extras = self._layer_extras(hidden_states.device) if with_extras else None
@@ -331,7 +339,7 @@ class TrisSparseMoeBlock(nn.Module):
             logits_in, logits_out = None, logits.data_ptr()
         if T:
             self._require_rows(x, "forward")
-            ws = self.workspace(T, dev) if extras is None else self._extras_workspace(T, dev, extras)
+            ws = self.workspace(T, dev, shared) if extras is None else self._extras_workspace(T, dev, extras)
             view = self._layer_view  # which the size query has just brought up to date
             own = None if extras is None else []
             if self.packed_backbones:  # gate and up see T rows, down T * top_k
@@ -343,7 +351,12 @@ class TrisSparseMoeBlock(nn.Module):
                     view = self._expanded_layer_view(dev, big, own)
             with torch.cuda.device(dev):
                 stream = torch.cuda.current_stream(dev).cuda_stream
-                if extras is None:
+                if shared is not None:
+                    scratch = self._shared_scratch(lib, shared, T, dev)
+                    st = lib.tris_moe_layer_forward_shared(C.byref(view), C.byref(shared), x.data_ptr(), logits_in, T, y.data_ptr(), logits_out,
+                                                           ws.data_ptr(), ws.numel(), None if scratch is None else scratch.data_ptr(),
+                                                           0 if scratch is None else scratch.numel(), stream)
+                elif extras is None:
                     st = lib.tris_moe_layer_forward(C.byref(view), x.data_ptr(), logits_in, T, y.data_ptr(),
                                                     logits_out, ws.data_ptr(), ws.numel(), stream)
                 else:
@@ -487,11 +500,45 @@ class TrisQwen2SparseMoeBlock(TrisSparseMoeBlock):
                                                       requires_grad=False)
         return self
 
+    def _shared_view(self, hidden_states: torch.Tensor) -> Optional[TrisSharedExpert]:
+        """The shared expert as the native layer takes it; None where the separate operators have to run: planes without tile records,
+        scales, other sizes, types or places, gradients, hooks on the down projection."""
+        from .compact3_linear import Compact3Linear
+
+        mods, w, H = self.shared_expert, self.shared_expert_gate.weight, self.hidden_size
+        if self.input_scales or self.ns_payloads or not envflags.grouped_experts_enabled() or not all(type(m) is Compact3Linear for m in mods):
+            return None
+        gate, up, down = mods
+        hooks = torch.nn.modules.module._has_any_global_hook() or down._forward_hooks or down._forward_pre_hooks
+        if (hooks or any(m.input_scale is not None or m.payload.get("_tris_tile_records") is None for m in mods)
+                or (gate.in_features, up.in_features, up.out_features, down.in_features, down.out_features)
+                != (H, H, gate.out_features, gate.out_features, H)):
+            return None
+        dev = hidden_states.device
+        if (hidden_states.dtype != torch.float16 or w.dtype != torch.float16 or w.shape != (1, H) or not w.is_contiguous() or H % 8
+                or hidden_states.shape[-1] != H or dev.type != "cuda" or w.device != dev
+                or any(m.payload["qweight1"].device != dev for m in mods)
+                or (torch.is_grad_enabled() and (w.requires_grad or hidden_states.requires_grad))):
+            return None
+        return TrisSharedExpert(*(C.addressof(proj_view(m.payload)) for m in mods), w.data_ptr())
+
+    @staticmethod
+    def _shared_scratch(lib, shared: TrisSharedExpert, rows: int, device) -> Optional[torch.Tensor]:
+        """Scratch of one call for the shared expert's two launches, as the separate operators take it (a block's own buffer would hold on to
+        up to 256 MB of it)."""
+        if rows <= 32:
+            return None
+        need = max(int(lib.tris_linear_workspace_bytes(C.cast(p, C.POINTER(_native.TrisProjView)), n, rows)) for p, n in ((shared.gate, 2), (shared.down, 1)))
+        return torch.empty((need,), dtype=torch.uint8, device=device) if need else None
+
     def forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None):
         from .compact3_linear import run_compact3_gate_up_forward
 
         if self.shared_expert is None:
             raise RuntimeError("trismoe_b200: the shared expert was not loaded (load_shared_expert)")
+        view = self._shared_view(hidden_states)
+        if view is not None:
+            return self._forward(hidden_states, router_logits, view)
         routed, logits = super().forward(hidden_states, router_logits)
         gate_proj, up_proj, down_proj = self.shared_expert
         mlp = run_compact3_gate_up_forward(gate_proj, up_proj, hidden_states, fuse_silu_mul=True)

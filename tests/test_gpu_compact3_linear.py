@@ -121,3 +121,40 @@ def test_qwen2_block_with_shared_expert(lib):
     shared_out = mlp @ d_w.astype(np.float32).T
     ref = ref + 1.0 / (1.0 + np.exp(-(xf @ gate_w.astype(np.float32).T))) * shared_out
     _check(y.view(T, -1), ref)
+
+
+@pytest.mark.parametrize("T,given", [(1, False), (5, True), (16, False), (32, False), (33, True), (70, False), (300, False)])
+def test_shared_expert_in_the_layer_sequence(lib, T, given):
+    """The shared expert's launches between those of the routed experts, where they read rows before the kernel ahead of them has ended:
+    the same bits as the separate operators, call after call in one workspace and in a captured graph."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    shape = synth.LayerShape(1032, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=7)
+    rng = np.random.default_rng(7)
+    blk = tm.TrisQwen2SparseMoeBlock(shape.hidden_size, shape.intermediate_size, shape.num_experts, shape.top_k, True)
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], layer["shared_gate"], layer["shared_up"],
+                              layer["shared_down"], layer["router_weight"], device="cuda")
+    gate_w = (rng.standard_normal((1, 1032)) / 32).astype(np.float16)
+    blk.load_shared_expert(_single(rng, 328, 1032)[0], _single(rng, 328, 1032)[0], _single(rng, 1032, 328)[0], torch.from_numpy(gate_w))
+    rows = [(synth.synth_activations(T, 1032, seed=s).float() * 0.25).half().cuda().view(1, T, -1) for s in range(4)]
+    logits = [synth.synth_router_logits(T, shape.num_experts, seed=s).cuda() if given else None for s in range(4)]
+    with torch.no_grad():
+        view, blk._shared_view = blk._shared_view, lambda h: None
+        want = [blk(x, router_logits=l) for x, l in zip(rows, logits)]
+        blk._shared_view = view
+        assert blk._shared_view(rows[0]) is not None
+        got = [blk(x, router_logits=l) for x, l in zip(rows, logits)]
+        for (y, l), (wy, wl) in zip(got, want):
+            assert torch.equal(y, wy) and torch.equal(l, wl)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [blk(x, router_logits=l)[0] for x, l in zip(rows, logits)]
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for y, (w, _) in zip(outs, want))
+    assert blk.last_kernel_status() == 0
+    blk.shared_expert[2].register_forward_hook(lambda *a: None)  # a hook on the down projection is called as before
+    assert blk._shared_view(rows[0]) is None
