@@ -655,6 +655,44 @@ int tris_moe_layer_forward_shared(const TrisMoeLayerView* layer, const TrisShare
                                   size_t scratch_bytes, void* stream);
 
 /*
+ * One layer in streaming mode: router, route, pager launches on a second stream, backbones, grouped kernels, combine, ordered by
+ * events and without a host round trip.  pages: the pager launches of gate and up ([0]) and of down ([1]); gate and up are
+ * computed while down is paged.  staged: the projections with their paged tensors in staging slots.  records: the same as
+ * tile records in buffers that the call fills from the staged tensors, segment s at place s (num_experts = capacity, no
+ * output scale or bias), so that the record kernels compute them; tile_records NULL in them: the plane kernels read the
+ * staged tensors.  slot_ids: device array, i below capacity and -1 up to num_experts (with records).  Events are
+ * cudaEvent_t that exist already: route, paged (one each for pages[0] and pages[1]), consumed; the pager waits for
+ * `consumed` first where wait_consumed is set.  timing: NULL, or around the pages and around the two waits of the compute stream.
+ * TRIS_ERR_WORKSPACE in status_dev: more experts than slots; their rows are stale.
+ */
+typedef struct TrisPageLaunch {
+  const void* jobs; /* TrisPageJob or TrisCodedPageJob */
+  int32_t* slot_table;
+  int32_t num_jobs;
+  int32_t coded;
+} TrisPageLaunch;
+
+typedef struct TrisPagedLayer {
+  const TrisPageLaunch* pages[2];
+  int32_t num_pages[2];
+  TrisProjView staged[3];  /* gate, up, down */
+  TrisProjView records[3];
+  const int32_t* slot_ids;
+  int32_t capacity;
+  int32_t wait_consumed;
+  void* copy_stream;
+  void* event_route;
+  void* event_paged[2];
+  void* event_consumed;
+  void* timing[6];
+} TrisPagedLayer;
+
+int tris_paged_records_plan(const TrisProjView* proj, int64_t* info_out, void* stream); /* info (device): {bytes of an expert's records, bytes of one, steps, slots} */
+int tris_moe_layer_forward_paged(const TrisMoeLayerView* layer, const TrisPagedLayer* paged, const void* x_f16, const float* router_logits,
+                                 int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace, size_t workspace_bytes,
+                                 int32_t* status_dev, void* stream);
+
+/*
  * Same computation as tris_moe_layer_forward for callers that cannot provide a workspace
  * because they are not allowed to allocate device memory: for example a serving process
  * whose memory pool claimed the whole GPU at start-up (a later cudaMalloc fails or

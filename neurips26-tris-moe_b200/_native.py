@@ -79,6 +79,18 @@ class TrisMoeLayerExtras(C.Structure):
     _fields_ = [("input_scale", _vp * 3), ("ns_c2", _vp * 3), ("ns_c1", _vp * 3)]
 
 
+class TrisPageLaunch(C.Structure):
+    _fields_ = [("jobs", _vp), ("slot_table", _vp), ("num_jobs", _i32), ("coded", _i32)]
+
+
+class TrisPagedLayer(C.Structure):
+    _fields_ = [
+        ("pages", _vp * 2), ("num_pages", _i32 * 2), ("staged", TrisProjView * 3), ("records", TrisProjView * 3),
+        ("slot_ids", _vp), ("capacity", _i32), ("wait_consumed", _i32), ("copy_stream", _vp),
+        ("event_route", _vp), ("event_paged", _vp * 2), ("event_consumed", _vp), ("timing", _vp * 6),
+    ]
+
+
 class TrisSharedExpert(C.Structure):
     _fields_ = [("gate", _vp), ("up", _vp), ("down", _vp), ("gate_weight", _vp)]
 
@@ -137,6 +149,8 @@ SIGNATURES = {
     "tris_moe_layer_forward_extras_status": (C.c_int, [_P(TrisMoeLayerView), _P(TrisMoeLayerExtras), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp, _vp]),
     "tris_moe_layer_shared_workspace_bytes": (C.c_size_t, [_P(TrisMoeLayerView), _P(TrisSharedExpert), _i32]),
     "tris_moe_layer_forward_shared": (C.c_int, [_P(TrisMoeLayerView), _P(TrisSharedExpert), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp, C.c_size_t, _vp]),
+    "tris_paged_records_plan": (C.c_int, [_P(TrisProjView), _vp, _vp]),
+    "tris_moe_layer_forward_paged": (C.c_int, [_P(TrisMoeLayerView), _P(TrisPagedLayer), _vp, _vp, _i32, _vp, _vp, _vp, C.c_size_t, _vp, _vp]),
     "tris_moe_layer_forward_static": (C.c_int, [_P(TrisMoeLayerView), _vp, _vp, _i32, _vp, _vp, _vp]),
 }
 STATIC_SCRATCH_BYTES = 8 << 20

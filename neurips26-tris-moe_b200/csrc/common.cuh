@@ -132,6 +132,16 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
 int grouped_tc_min_rows();
 int route_rows_hint(const TrisRouteView* route);
 size_t grouped_split_bytes(const TrisProjView* proj, int projections, int num_rows);
+// Streaming: tile records of the experts that were paged in, one per segment; staged / records: views of the paged tensors and of the
+// record buffers (num_experts = capacity) of one or two projections (tile_records.cu).  Called once before the pages have arrived, when it
+// builds what does not depend on them, and once after.
+int build_paged_records(const TrisProjView* staged, const TrisProjView* records, int projections, const TrisRouteView* route, int capacity,
+                        bool paged, cudaStream_t stream);
+// One pager launch (paging.cu).  reset: experts that are not paged read -1 in the slot table afterwards.
+int page_experts_impl(const TrisPageJob* jobs, int num_jobs, const int32_t* expert_ids, const int32_t* num_segments_dev, int num_segments,
+                      int num_experts, int32_t* slot_table, bool reset, cudaStream_t stream);
+int page_coded_experts_impl(const TrisCodedPageJob* jobs, int num_jobs, const int32_t* expert_ids, const int32_t* num_segments_dev,
+                            int num_segments, int num_experts, int32_t* slot_table, bool reset, cudaStream_t stream);
 int launch_tiled_dump(const TrisProjView* proj, void* weights_out, cudaStream_t stream);
 int combine_routed_impl(const void* down_out_f16, const int32_t* row_of_flat, const float* routing_weights,
                         int num_tokens, int top_k, int hidden_size, void* final_f16, cudaStream_t stream, bool pdl,

@@ -416,6 +416,121 @@ extern "C" int tris_moe_layer_forward_shared(const TrisMoeLayerView* layer, cons
                        {shared, scratch, scratch_bytes});
 }
 
+// ---- streaming mode ----------------------------------------------------------------------------
+// Two streams: the pages cross the host link on one while the other computes what it has.  The router runs before the backbones, since the
+// pages wait for its route; the backbones run beside them.  Paged experts become tile records, all but the paged bits of them while the
+// pages are on their way: with those bits put in, 8 and 12 us, and the kernels for records, 11 and 15, gate/up and down of 102 experts of 512 x 256
+// (twice) and 2048 x 256 take half of what the kernels for planes did (45 each, 78 beside a pager).  Two such layers, 16 tokens:
+// 416 us with planes and seven calls a layer from Python, 360 here; 1 token 271 / 171.
+extern "C" int tris_moe_layer_forward_paged(const TrisMoeLayerView* layer, const TrisPagedLayer* paged, const void* x_f16, const float* router_logits,
+                                            int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace, size_t workspace_bytes,
+                                            int32_t* status_dev, void* stream) {
+  int st = validate_layer(layer);
+  if (st != TRIS_OK) return st;
+  TRIS_REQUIRE(paged && x_f16 && y_f16 && status_dev, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: null pointer");
+  TRIS_REQUIRE(num_tokens >= 0, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: negative token count");
+  TRIS_REQUIRE(router_logits || layer->router_weight, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: need router_logits or a router weight");
+  TRIS_REQUIRE(!layer->packed_gate && !layer->packed_up && !layer->packed_down, TRIS_ERR_UNSUPPORTED, "tris_moe_layer_forward_paged: fp16 backbones only");
+  TRIS_REQUIRE(paged->copy_stream && paged->event_route && paged->event_paged[0] && paged->event_paged[1] && paged->event_consumed && paged->capacity > 0,
+               TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: streams, events and slots are needed");
+  const bool records = paged->records[0].tile_records != nullptr;
+  TRIS_REQUIRE(!records || paged->slot_ids, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: records need slot_ids");
+  if (num_tokens == 0) return TRIS_OK;
+  const int T = num_tokens, E = layer->num_experts, R = T * layer->top_k;
+  LayerWorkspace w = carve(layer, T, static_cast<char*>(workspace));
+  TRIS_REQUIRE(workspace != nullptr && workspace_bytes >= w.bytes, TRIS_ERR_WORKSPACE, "tris_moe_layer_forward_paged: workspace %zu < %zu bytes",
+               workspace_bytes, w.bytes);
+  cudaStream_t s = static_cast<cudaStream_t>(stream), copy = static_cast<cudaStream_t>(paged->copy_stream);
+  const __half* x = static_cast<const __half*>(x_f16);
+  auto event = [&](void* e) { return static_cast<cudaEvent_t>(e); };
+  auto time = [&](int i, cudaStream_t on) { return paged->timing[i] ? cudaEventRecord(event(paged->timing[i]), on) : cudaSuccess; };
+
+  const float* logits = router_logits;
+  if (logits == nullptr) {
+    float* dst = router_logits_out ? router_logits_out : w.logits;
+    const SkinnyProblem router{static_cast<const __half*>(layer->router_weight), dst, E, TRIS_OUT_F32};
+    st = launch_shared_hidden(&router, 1, x, nullptr, T, layer->hidden_size, s, /*pdl=*/true);
+    if (st != TRIS_OK) return st;
+    logits = dst;
+  } else if (router_logits_out && router_logits_out != router_logits) {
+    TRIS_CUDA(cudaMemcpyAsync(router_logits_out, router_logits, sizeof(float) * T * E, cudaMemcpyDeviceToDevice, s));
+  }
+  st = launch_router_route(logits, T, E, layer->top_k, layer->norm_topk_prob, 4, w.selected, w.weights, w.perm, w.tok, w.slot, w.row_of_flat,
+                           w.expert_ids, w.segment_offsets, w.problem_offsets, w.counts, s, reinterpret_cast<int32_t*>(w.down_out),
+                           2 * static_cast<size_t>(R) * layer->hidden_size);
+  if (st != TRIS_OK) return st;
+
+  TRIS_CUDA(cudaEventRecord(event(paged->event_route), s));
+  TRIS_CUDA(cudaStreamWaitEvent(copy, event(paged->event_route), 0));
+  if (paged->wait_consumed) TRIS_CUDA(cudaStreamWaitEvent(copy, event(paged->event_consumed), 0));
+  TRIS_CUDA(time(0, copy));
+  const int segments = std::min(E, R), slots = std::min(segments, paged->capacity);
+  for (int g = 0; g < 2; ++g) {
+    for (int i = 0; i < paged->num_pages[g]; ++i) {
+      const TrisPageLaunch& p = paged->pages[g][i];
+      st = p.coded ? page_coded_experts_impl(static_cast<const TrisCodedPageJob*>(p.jobs), p.num_jobs, w.expert_ids, w.counts, slots, E, p.slot_table, !records, copy)
+                   : page_experts_impl(static_cast<const TrisPageJob*>(p.jobs), p.num_jobs, w.expert_ids, w.counts, slots, E, p.slot_table, !records, copy);
+      if (st != TRIS_OK) return st;
+    }
+    if (g == 1) TRIS_CUDA(time(1, copy));
+    TRIS_CUDA(cudaEventRecord(event(paged->event_paged[g]), copy));
+  }
+
+  TrisRouteView route{};
+  route.expert_ids = w.expert_ids;
+  route.segment_offsets = w.segment_offsets;
+  route.num_segments_dev = w.counts;
+  route.num_segments = segments;
+  route.num_rows = R;
+  route.max_rows_per_segment = T;
+  route.status_dev = status_dev;
+  const TrisProjView* views = records ? paged->records : paged->staged;
+  const int gu_mode = tris_grouped_hidden_layout(views, views + 1, R, segments, T), down_mode = tris_grouped_hidden_layout(views + 2, nullptr, R, segments, T);
+  const SkinnyProblem gu[2] = {{static_cast<const __half*>(layer->shared_gate), w.hidden_gate, layer->gate.rank, gu_mode},
+                               {static_cast<const __half*>(layer->shared_up), w.hidden_up, layer->up.rank, gu_mode}};
+  st = launch_shared_hidden(gu, 2, x, nullptr, T, layer->hidden_size, s, /*pdl=*/true, nullptr, /*matrices_before_wait=*/true);
+  if (st != TRIS_OK) return st;
+  // Records are those of the segments, in their order: place s holds segment s.
+  auto paged_route = [&](int g) {
+    TrisRouteView r = route;
+    if (records) r.expert_ids = paged->slot_ids;
+    r.row_gather = g == 0 ? w.tok : nullptr;
+    r.flags = (g == 0 ? gu_mode : down_mode) == TRIS_OUT_F16_PAIR_INTERLEAVED ? TRIS_ROUTE_HIDDEN_PAIR_INTERLEAVED : 0;
+    return r;
+  };
+  LaunchOpts opts;
+  opts.pdl = records;  // after the builder; a launch that follows a wait for an event is an ordinary one
+  auto arrived = [&](int g) -> int {
+    TRIS_CUDA(time(2 + 2 * g, s));
+    TRIS_CUDA(cudaStreamWaitEvent(s, event(paged->event_paged[g]), 0));
+    TRIS_CUDA(time(3 + 2 * g, s));
+    return records ? build_paged_records(paged->staged + 2 * g, paged->records + 2 * g, g == 0 ? 2 : 1, &route, paged->capacity, true, s) : static_cast<int>(TRIS_OK);
+  };
+  auto ahead = [&](int g) -> int {  // records as far as they do not depend on the pages
+    return records ? build_paged_records(paged->staged + 2 * g, paged->records + 2 * g, g == 0 ? 2 : 1, &route, paged->capacity, false, s) : static_cast<int>(TRIS_OK);
+  };
+  st = ahead(0);
+  if (st == TRIS_OK) st = arrived(0);
+  if (st != TRIS_OK) return st;
+  const TrisRouteView gu_route = paged_route(0), down_route = paged_route(1);
+  st = records ? launch_grouped_tiled(views, views + 1, &gu_route, w.hidden_gate, w.hidden_up, w.mlp, nullptr, 2, route_rows_hint(&gu_route), s, opts)
+               : grouped_pair_forward_impl(views, views + 1, &gu_route, w.hidden_gate, w.hidden_up, w.mlp, nullptr, 1, s, opts);
+  if (st != TRIS_OK) return st;
+  const SkinnyProblem down{static_cast<const __half*>(layer->shared_down), w.hidden_down, layer->down.rank, down_mode};
+  st = launch_shared_hidden(&down, 1, w.mlp, nullptr, R, layer->intermediate_size, s, /*pdl=*/true, nullptr, true);
+  if (st != TRIS_OK) return st;
+  st = ahead(1);
+  if (st == TRIS_OK) st = arrived(1);
+  if (st != TRIS_OK) return st;
+  st = records ? launch_grouped_tiled(views + 2, nullptr, &down_route, w.hidden_down, nullptr, w.down_out, nullptr, 0, route_rows_hint(&down_route), s, opts)
+               : grouped_forward_impl(views + 2, &down_route, w.hidden_down, w.down_out, s, opts);
+  if (st != TRIS_OK) return st;
+  st = combine_routed_impl(w.down_out, w.row_of_flat, w.weights, T, layer->top_k, layer->hidden_size, y_f16, s, true, /*indices_ready=*/true);
+  if (st != TRIS_OK) return st;
+  TRIS_CUDA(cudaEventRecord(event(paged->event_consumed), s));
+  return TRIS_OK;
+}
+
 // ---- variant that allocates nothing ----------------------------------------------------------
 // Scratch for tris_moe_layer_forward_static.  Lives in every process image that loads the
 // library, once per GPU that touches it, until the process exits.

@@ -18,30 +18,43 @@ struct PageArgs {
   int32_t* slot_table;
 };
 
-// grid (chunks, segment bound, jobs); 256 threads, 16 bytes per thread per step
-__global__ void __launch_bounds__(256) page_experts_kernel(const __grid_constant__ PageArgs args) {
-  const int seg = blockIdx.y;
+// CTAs of a pager and their warps.  The reads in flight have to cover the host link's latency, and the warps of coded pages keep up with it
+// while they decode, on SMs that are not all as near to the link and of which a pager that starts beside another kernel gets
+// fewer than there are; but no more of them: what is queued beyond that delays every other read of the memory system and every
+// launch, and the kernels that work on what is there already run beside the pager.  With all warps of a page resident at once they took
+// three times as long.  us, two streamed layers of 102 experts, nine states, 64 / 96 / 148 / 222 CTAs of coded pages: 538-600, 425-457,
+// 354-369, 373-397; uncoded ones, whose threads have eight reads in flight, one layer, 20 / 28 / 64 / 148 CTAs: 590, 583, 583, 584, and 4
+// tokens of 64 experts 205, 206, 209, 213.
+constexpr int kPageWarps = 4, kPageThreads = 32 * kPageWarps, kPagerCtas = 32, kCodedPagerCtas = 148;
+
+// Pieces of 16 KB (eight 16-byte reads a thread) of the active experts' blocks, dealt to the CTAs in turn.
+__global__ void __launch_bounds__(kPageThreads) page_experts_kernel(const __grid_constant__ PageArgs args) {
+  constexpr int kPiece = 8 * kPageThreads;  // 16-byte words
   const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
-  if (seg >= nseg) return;
-  const int e = args.expert_ids[seg];
-  if (e < 0 || e >= args.num_experts) return;
-  if (blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0) args.slot_table[e] = seg;
-  const TrisPageJob& job = args.jobs[blockIdx.z];
-  const long long vecs = job.bytes_per_expert >> 4;
-  const uint4* src = reinterpret_cast<const uint4*>(static_cast<const char*>(job.host_src) + e * job.bytes_per_expert);
-  uint4* dst = reinterpret_cast<uint4*>(static_cast<char*>(job.dst) + seg * job.bytes_per_expert);
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  // eight independent 16-byte reads in flight per thread: host reads cross PCIe/C2C, whose latency
-  // (microseconds) has to be covered by bytes in flight
-  for (; i + 7 * stride < vecs; i += 8 * stride) {
+  int per_segment = 0;
+  for (int j = 0; j < args.num_jobs; ++j) per_segment += static_cast<int>(((args.jobs[j].bytes_per_expert >> 4) + kPiece - 1) / kPiece);
+  for (int i = blockIdx.x; i < nseg * per_segment; i += gridDim.x) {
+    const int seg = i / per_segment, e = args.expert_ids[seg];
+    if (e < 0 || e >= args.num_experts) continue;
+    int piece = i - seg * per_segment, j = 0;
+    if (piece == 0 && threadIdx.x == 0) args.slot_table[e] = seg;
+    for (;; ++j) {
+      const int pieces = static_cast<int>(((args.jobs[j].bytes_per_expert >> 4) + kPiece - 1) / kPiece);
+      if (piece < pieces) break;
+      piece -= pieces;
+    }
+    const TrisPageJob& job = args.jobs[j];
+    const long long vecs = job.bytes_per_expert >> 4, at = static_cast<long long>(piece) * kPiece + threadIdx.x;
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const char*>(job.host_src) + e * job.bytes_per_expert) + at;
+    uint4* dst = reinterpret_cast<uint4*>(static_cast<char*>(job.dst) + seg * job.bytes_per_expert) + at;
     uint4 v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldcs(src + i + j * stride);
+    for (int k = 0; k < 8; ++k)
+      if (at + k * kPageThreads < vecs) v[k] = __ldcs(src + k * kPageThreads);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dst[i + j * stride] = v[j];
+    for (int k = 0; k < 8; ++k)
+      if (at + k * kPageThreads < vecs) dst[k * kPageThreads] = v[k];
   }
-  for (; i < vecs; i += stride) dst[i] = __ldcs(src + i);
 }
 
 // ---- coded pages -------------------------------------------------------------------------------------
@@ -52,11 +65,11 @@ __global__ void __launch_bounds__(256) page_experts_kernel(const __grid_constant
 // resident format (0.48 and a 0.25-bit index of sub-streams), any 16 bytes of it can be read without the ones before: a lane adds
 // up what its symbols advance by, a warp scan gives it its place.  A block that would not get smaller stays as it is.
 constexpr int kPageBlock = TRIS_PAGE_BLOCK_BYTES, kPageWords = kPageBlock / 4, kPageUnits = kPageBlock / 16;
-constexpr int kPageWarps = 8;
 static_assert(kPageUnits == 64 && kPageWords == 8 * 32, "two 16-byte words and eight 4-byte words a lane");
 
 struct CodedPageArgs {
   TrisCodedPageJob jobs[TRIS_MAX_PAGE_JOBS];
+  int32_t num_jobs;
   const int32_t* expert_ids;
   const int32_t* num_segments_dev;
   int32_t num_segments;
@@ -69,61 +82,96 @@ __device__ __forceinline__ int symbols_advance(uint32_t w) {  // sum over eight 
   return static_cast<int>(__dp4a(bytes, 0x01010101u, 0u)) + 8 - __popc(skips);
 }
 
-// grid (blocks of an expert / 8, segment bound, jobs); a warp decodes one block.  All warps of a page are resident at once, so
-// that their reads cover the link's latency.  Two streamed layers of 102 active experts, 16 tokens: 593 us with raw pages, 420 coded.
-__global__ void __launch_bounds__(32 * kPageWarps) page_coded_kernel(const __grid_constant__ CodedPageArgs args) {
-  __shared__ __align__(16) uint32_t bits[kPageWarps][kPageWords];
-  const int seg = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// A load that stays where it is written: the next block is asked for before the last one is decoded.
+__device__ __forceinline__ uint4 load_now(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.cs.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+// A warp decodes blocks dealt to it in turn, and asks for the next one before it decodes the last.
+__global__ void __launch_bounds__(kPageThreads) page_coded_kernel(const __grid_constant__ CodedPageArgs args) {
+  // the lanes' places in a block are some eight words apart: a pad word after every 32 keeps them out of one another's banks
+  __shared__ uint32_t bits[kPageWarps][kPageWords + kPageWords / 32];
+  __shared__ __align__(16) uint32_t code[kPageWarps][kPageWords];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nseg = args.num_segments_dev ? min(*args.num_segments_dev, args.num_segments) : args.num_segments;
-  if (seg >= nseg) return;
-  const int e = args.expert_ids[seg];
-  if (e < 0 || e >= args.num_experts) return;
-  if (blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0) args.slot_table[e] = seg;
-  const TrisCodedPageJob& job = args.jobs[blockIdx.z];
-  const int blocks = static_cast<int>((job.bytes_per_expert + kPageBlock - 1) / kPageBlock), block = blockIdx.x * kPageWarps + warp;
-  if (block >= blocks) return;
-  const int32_t* offset = job.block_offsets + static_cast<size_t>(e) * blocks + block;
-  const int first = offset[0], units = min(offset[1] - first, kPageUnits);
-  const uint4* src = static_cast<const uint4*>(job.host_src) + first;
+  auto blocks_of = [&](int j) { return static_cast<int>((args.jobs[j].bytes_per_expert + kPageBlock - 1) / kPageBlock); };
+  int per_segment = 0;
+  for (int j = 0; j < args.num_jobs; ++j) per_segment += blocks_of(j);
+  const int total = nseg * per_segment, step = gridDim.x * kPageWarps;
   const uint4 skip = make_uint4(~0u, ~0u, ~0u, ~0u);
-  const uint4 a = lane < units ? __ldcs(src + lane) : skip, b = lane + 32 < units ? __ldcs(src + lane + 32) : skip;
-  const int left = static_cast<int>(min(static_cast<long long>(kPageBlock), job.bytes_per_expert - static_cast<long long>(block) * kPageBlock)) >> 4;
-  uint4* dst = reinterpret_cast<uint4*>(static_cast<char*>(job.dst) + static_cast<size_t>(seg) * job.bytes_per_expert + static_cast<size_t>(block) * kPageBlock);
-  if (units == kPageUnits) {
-    if (lane < left) dst[lane] = a;
-    if (lane + 32 < left) dst[lane + 32] = b;
-    return;
-  }
-  uint4* out = reinterpret_cast<uint4*>(bits[warp]);
-  out[lane] = out[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
-  __syncwarp();
-  int at = 0;
+  struct Block {
+    uint4 a, b;
+    uint4* dst;
+    int units, left;  // 16-byte words of the code and of the block; -1: nothing to do
+  };
+  auto fetch = [&](int i) {
+    Block f;
+    f.left = -1;
+    if (i >= total) return f;
+    const int seg = i / per_segment, e = args.expert_ids[seg];
+    if (e < 0 || e >= args.num_experts) return f;
+    int block = i - seg * per_segment, j = 0;
+    if (block == 0 && lane == 0) args.slot_table[e] = seg;
+    for (; block >= blocks_of(j); ++j) block -= blocks_of(j);
+    const TrisCodedPageJob& job = args.jobs[j];
+    const int32_t* offset = job.block_offsets + static_cast<size_t>(e) * blocks_of(j) + block;
+    const int first = offset[0];
+    f.units = min(offset[1] - first, kPageUnits);
+    const uint4* src = static_cast<const uint4*>(job.host_src) + first;
+    f.a = f.b = skip;
+    if (lane < f.units) f.a = load_now(src + lane);
+    if (lane + 32 < f.units) f.b = load_now(src + lane + 32);
+    f.left = static_cast<int>(min(static_cast<long long>(kPageBlock), job.bytes_per_expert - static_cast<long long>(block) * kPageBlock)) >> 4;
+    f.dst = reinterpret_cast<uint4*>(static_cast<char*>(job.dst) + static_cast<size_t>(seg) * job.bytes_per_expert + static_cast<size_t>(block) * kPageBlock);
+    return f;
+  };
+  int i = blockIdx.x * kPageWarps + warp;
+  Block next = fetch(i);
 #pragma unroll 1
-  for (int half = 0; half * 32 < units; ++half) {
-    uint4 v = half ? b : a;
-    const int mine = symbols_advance(v.x) + symbols_advance(v.y) + symbols_advance(v.z) + symbols_advance(v.w);
+  for (; i < total; i += step) {
+    const Block f = next;
+    next = fetch(i + step);
+    if (f.left < 0) continue;
+    if (f.units == kPageUnits) {
+      if (lane < f.left) f.dst[lane] = f.a;
+      if (lane + 32 < f.left) f.dst[lane + 32] = f.b;
+      continue;
+    }
+    // The code's words are dealt to the lanes in runs of equal length, so that every lane has its share of the symbols.
+    uint32_t* out = bits[warp];
+    for (int q = lane; q < kPageWords + kPageWords / 32; q += 32) out[q] = 0u;
+    uint4* in = reinterpret_cast<uint4*>(code[warp]);
+    in[lane] = f.a;
+    in[lane + 32] = f.b;
+    __syncwarp();
+    const int run = (4 * f.units + 31) >> 5, begin = lane * run, end = min(begin + run, 4 * f.units);
+    int mine = 0;
+    for (int q = begin; q < end; ++q) mine += symbols_advance(code[warp][q]);
     int upto = mine;
     for (int o = 1; o < 32; o <<= 1) {
       const int n = __shfl_up_sync(0xFFFFFFFFu, upto, o);
       if (lane >= o) upto += n;
     }
-    int pos = at + upto - mine;
-    at += __shfl_sync(0xFFFFFFFFu, upto, 31);
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-      uint32_t w = v.x;
+    int pos = upto - mine;
+    for (int q = begin; q < end; ++q) {
+      uint32_t w = code[warp][q];
 #pragma unroll
-      for (int j = 0; j < 8; ++j, w >>= 4) {
+      for (int k = 0; k < 8; ++k, w >>= 4) {
         const int gap = static_cast<int>(w & 15u), bit = pos + gap;
-        if (gap != 15 && bit < 8 * kPageBlock) atomicOr(&bits[warp][bit >> 5], 1u << (bit & 31));
+        if (gap != 15 && bit < 8 * kPageBlock) atomicOr(&out[(bit >> 5) + (bit >> 10)], 1u << (bit & 31));
         pos = bit + (gap != 15);
       }
-      v.x = v.y, v.y = v.z, v.z = v.w;
     }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int q = lane + 32 * h;
+      const uint32_t* w = out + 4 * q + (q >> 3);
+      if (q < f.left) f.dst[q] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    __syncwarp();  // before the next block's zeros
   }
-  __syncwarp();
-  if (lane < left) dst[lane] = out[lane];
-  if (lane + 32 < left) dst[lane + 32] = out[lane + 32];
 }
 
 // One warp per block: its size in 16-byte units (offsets null) or its code.
@@ -221,15 +269,14 @@ extern "C" int tris_page_code_blocks(const void* src_dev, int64_t bytes_per_expe
   return check_cuda(cudaGetLastError(), "code_blocks_kernel launch");
 }
 
-extern "C" int tris_page_coded_experts(const TrisCodedPageJob* jobs, int32_t num_jobs, const int32_t* expert_ids, const int32_t* num_segments_dev,
-                                       int32_t num_segments, int32_t num_experts, int32_t* slot_table, void* stream) {
+int tris::page_coded_experts_impl(const TrisCodedPageJob* jobs, int num_jobs, const int32_t* expert_ids, const int32_t* num_segments_dev,
+                                  int num_segments, int num_experts, int32_t* slot_table, bool reset, cudaStream_t stream) {
   TRIS_REQUIRE(jobs && expert_ids && slot_table, TRIS_ERR_INVALID_ARG, "tris_page_coded_experts: null pointer");
   TRIS_REQUIRE(num_jobs >= 1 && num_jobs <= TRIS_MAX_PAGE_JOBS, TRIS_ERR_INVALID_ARG,
                "tris_page_coded_experts: %d jobs (1..%d supported)", num_jobs, TRIS_MAX_PAGE_JOBS);
   TRIS_REQUIRE(num_segments >= 0 && num_experts > 0, TRIS_ERR_INVALID_ARG, "tris_page_coded_experts: bad sizes");
   if (num_segments == 0) return TRIS_OK;
   CodedPageArgs args{};
-  long long most = 0;
   for (int j = 0; j < num_jobs; ++j) {
     TRIS_REQUIRE(jobs[j].host_src && jobs[j].block_offsets && jobs[j].dst && jobs[j].bytes_per_expert > 0 && (jobs[j].bytes_per_expert & 15) == 0,
                  TRIS_ERR_INVALID_ARG, "tris_page_coded_experts: job %d needs pointers and a block size that is a multiple of 16", j);
@@ -239,28 +286,30 @@ extern "C" int tris_page_coded_experts(const TrisCodedPageJob* jobs, int32_t num
     void* dev_alias = nullptr;  // as for uncoded pages
     TRIS_CUDA(cudaHostGetDevicePointer(&dev_alias, const_cast<void*>(jobs[j].host_src), 0));
     args.jobs[j].host_src = dev_alias;
-    most = std::max<long long>(most, (jobs[j].bytes_per_expert + kPageBlock - 1) / kPageBlock);
   }
+  args.num_jobs = num_jobs;
   args.expert_ids = expert_ids;
   args.num_segments_dev = num_segments_dev;
   args.num_segments = num_segments;
   args.num_experts = num_experts;
   args.slot_table = slot_table;
-  TRIS_CUDA(cudaMemsetAsync(slot_table, 0xFF, sizeof(int32_t) * static_cast<size_t>(num_experts), static_cast<cudaStream_t>(stream)));
-  page_coded_kernel<<<dim3(static_cast<unsigned>((most + kPageWarps - 1) / kPageWarps), num_segments, num_jobs), 32 * kPageWarps, 0, static_cast<cudaStream_t>(stream)>>>(args);
+  if (reset) TRIS_CUDA(cudaMemsetAsync(slot_table, 0xFF, sizeof(int32_t) * static_cast<size_t>(num_experts), stream));
+  page_coded_kernel<<<kCodedPagerCtas, kPageThreads, 0, stream>>>(args);
   return check_cuda(cudaGetLastError(), "page_coded_kernel launch");
 }
+extern "C" int tris_page_coded_experts(const TrisCodedPageJob* jobs, int32_t num_jobs, const int32_t* expert_ids, const int32_t* num_segments_dev,
+                                       int32_t num_segments, int32_t num_experts, int32_t* slot_table, void* stream) {
+  return page_coded_experts_impl(jobs, num_jobs, expert_ids, num_segments_dev, num_segments, num_experts, slot_table, true, static_cast<cudaStream_t>(stream));
+}
 
-extern "C" int tris_page_experts(const TrisPageJob* jobs, int32_t num_jobs, const int32_t* expert_ids,
-                                 const int32_t* num_segments_dev, int32_t num_segments, int32_t num_experts,
-                                 int32_t* slot_table, void* stream) {
+int tris::page_experts_impl(const TrisPageJob* jobs, int num_jobs, const int32_t* expert_ids, const int32_t* num_segments_dev, int num_segments,
+                            int num_experts, int32_t* slot_table, bool reset, cudaStream_t stream) {
   TRIS_REQUIRE(jobs && expert_ids && slot_table, TRIS_ERR_INVALID_ARG, "tris_page_experts: null pointer");
   TRIS_REQUIRE(num_jobs >= 1 && num_jobs <= TRIS_MAX_PAGE_JOBS, TRIS_ERR_INVALID_ARG,
                "tris_page_experts: %d jobs (1..%d supported)", num_jobs, TRIS_MAX_PAGE_JOBS);
   TRIS_REQUIRE(num_segments >= 0 && num_experts > 0, TRIS_ERR_INVALID_ARG, "tris_page_experts: bad sizes");
   if (num_segments == 0) return TRIS_OK;
   PageArgs args{};
-  long long max_bytes = 0;
   for (int j = 0; j < num_jobs; ++j) {
     TRIS_REQUIRE(jobs[j].host_src && jobs[j].dst && jobs[j].bytes_per_expert > 0 && (jobs[j].bytes_per_expert & 15) == 0,
                  TRIS_ERR_INVALID_ARG, "tris_page_experts: job %d needs pointers and a block size that is a multiple of 16", j);
@@ -271,7 +320,6 @@ extern "C" int tris_page_experts(const TrisPageJob* jobs, int32_t num_jobs, cons
     void* dev_alias = nullptr;
     TRIS_CUDA(cudaHostGetDevicePointer(&dev_alias, const_cast<void*>(jobs[j].host_src), 0));
     args.jobs[j].host_src = dev_alias;
-    max_bytes = std::max<long long>(max_bytes, jobs[j].bytes_per_expert);
   }
   args.num_jobs = num_jobs;
   args.expert_ids = expert_ids;
@@ -281,8 +329,12 @@ extern "C" int tris_page_experts(const TrisPageJob* jobs, int32_t num_jobs, cons
   args.slot_table = slot_table;
   // Experts that get no slot (more live segments than num_segments) must not keep a stale entry:
   // the grouped kernels treat -1 as "not paged in", store nothing and report TRIS_ERR_WORKSPACE.
-  TRIS_CUDA(cudaMemsetAsync(slot_table, 0xFF, sizeof(int32_t) * static_cast<size_t>(num_experts), static_cast<cudaStream_t>(stream)));
-  const int chunks = static_cast<int>(std::min<long long>(16, std::max<long long>(1, max_bytes / (256 * 16 * 8))));
-  page_experts_kernel<<<dim3(chunks, num_segments, num_jobs), 256, 0, static_cast<cudaStream_t>(stream)>>>(args);
+  if (reset) TRIS_CUDA(cudaMemsetAsync(slot_table, 0xFF, sizeof(int32_t) * static_cast<size_t>(num_experts), stream));
+  page_experts_kernel<<<kPagerCtas, kPageThreads, 0, stream>>>(args);
   return check_cuda(cudaGetLastError(), "page_experts_kernel launch");
+}
+extern "C" int tris_page_experts(const TrisPageJob* jobs, int32_t num_jobs, const int32_t* expert_ids,
+                                 const int32_t* num_segments_dev, int32_t num_segments, int32_t num_experts,
+                                 int32_t* slot_table, void* stream) {
+  return page_experts_impl(jobs, num_jobs, expert_ids, num_segments_dev, num_segments, num_experts, slot_table, true, static_cast<cudaStream_t>(stream));
 }

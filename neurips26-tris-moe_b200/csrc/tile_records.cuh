@@ -81,54 +81,27 @@ __host__ __device__ inline int record_bytes(int rank, int max_steps, int max_slo
 }
 
 // ---- salient step assignment ------------------------------------------------------------------
-// One thread walks the chunk's packed rows.  slot_of_row[p] = index of the run of equal group ids
-// that packed row p belongs to.  Salient columns of a run fill steps of 16; a new run starts a new
-// step.  col_of_slot gets the chunk-relative column of every step position or 0xFFFF.
+// One thread walks the chunk's packed rows.  A run of equal group ids is a row-scale slot.  Salient columns of a run
+// fill steps of 16; a new run starts a new step.
 struct ChunkPlan {
-  uint8_t slot_of_row[kChunkRows];
-  uint8_t step_slot[kMaxSteps];
-  int num_slots, num_steps, num_salient;
+  int num_slots, num_steps;
 };
-__device__ inline void plan_chunk(const int32_t* c_map_e, const int32_t* row_group_e, int pr, int p0, int rank,
-                                  ChunkPlan& plan, uint16_t* col_of_slot /* [kMaxSteps * 16] or null */) {
-  plan.num_slots = 0;
-  plan.num_steps = 0;
-  plan.num_salient = 0;
-  if (col_of_slot)
-    for (int i = 0; i < kMaxSteps * 16; ++i) col_of_slot[i] = 0xFFFFu;
-  for (int i = 0; i < kMaxSteps; ++i) plan.step_slot[i] = 0;
-  int prev_group = -0x7fffffff, fill = 16;
-  for (int p = 0; p < kChunkRows; ++p) {
-    const int pg = p0 + p;
-    if (pg >= pr) {
-      plan.slot_of_row[p] = static_cast<uint8_t>(plan.num_slots > 0 ? plan.num_slots - 1 : 0);
-      continue;
-    }
-    const int grp = row_group_e ? row_group_e[pg] : 0;
+__device__ inline ChunkPlan plan_chunk(const int32_t* c_map_e, const int32_t* row_group_e, int pr, int p0, int rank) {
+  ChunkPlan plan{0, 0};
+  int prev_group = -0x7fffffff, fill = 0;  // fill: salient columns of the run so far
+  for (int p = p0; p < min(pr, p0 + kChunkRows); ++p) {
+    const int grp = row_group_e ? row_group_e[p] : 0, ncols = rank - 32 * p;
     if (grp != prev_group) {
       prev_group = grp;
       ++plan.num_slots;
-      fill = 16;  // the next salient column opens a new step
+      fill = 0;
     }
-    const int slot = plan.num_slots - 1;
-    plan.slot_of_row[p] = static_cast<uint8_t>(slot);
-    uint32_t cw = static_cast<uint32_t>(c_map_e[pg]);
-    const int ncols = rank - 32 * pg;
-    if (ncols < 32) cw &= (ncols <= 0) ? 0u : ((1u << ncols) - 1u);
-    while (cw) {
-      const int j = __ffs(cw) - 1;
-      cw &= cw - 1;
-      if (fill == 16) {
-        fill = 0;
-        plan.step_slot[plan.num_steps] = static_cast<uint8_t>(slot);
-        ++plan.num_steps;
-      }
-      if (col_of_slot) col_of_slot[(plan.num_steps - 1) * 16 + fill] = static_cast<uint16_t>(32 * p + j);
-      ++fill;
-      ++plan.num_salient;
-    }
+    const int n = __popc(static_cast<uint32_t>(c_map_e[p]) & (ncols >= 32 ? ~0u : (ncols <= 0 ? 0u : (1u << ncols) - 1u)));
+    plan.num_steps += (fill + n + 15) / 16 - (fill + 15) / 16;
+    fill += n;
   }
   if (plan.num_slots == 0) plan.num_slots = 1;
+  return plan;
 }
 
 // ---- register unpack ----------------------------------------------------------------------------

@@ -386,6 +386,9 @@ class TrisSparseMoeBlock(nn.Module):
         r_gu, r_d = self.backbone_rank("gate"), self.backbone_rank("down")
         mode_gu, mode_d = (2 if r_gu % 32 == 0 else 0), (2 if r_d % 32 == 0 else 0)
         plain = lambda name: name not in self.packed_backbones and name not in self.input_scales
+        if all(plain(name) for name in ("gate", "up", "down")):
+            y, logits = self._forward_streaming_native(lib, x, y, manager, block_index, router_logits)
+            return y.reshape(shape), logits
         with torch.cuda.device(dev):
             stream = torch.cuda.current_stream(dev).cuda_stream
             # one allocation for everything between the kernels; the host has 25 launches a layer to prepare
@@ -437,6 +440,28 @@ class TrisSparseMoeBlock(nn.Module):
             paged.release()
             _native.check(lib.tris_combine_routed(down, rof, wts, T, k, H, y.data_ptr(), stream), "combine")
         return y.reshape(shape), logits
+
+    def _forward_streaming_native(self, lib, x, y, manager, block_index, router_logits):
+        """The same as one native call over both streams (``tris_moe_layer_forward_paged``)."""
+        T, E, dev = int(x.shape[0]), self.num_experts, x.device
+        view = self.layer_view()
+        if router_logits is not None:
+            logits = router_logits.reshape(T, E).to(torch.float32).contiguous()
+            logits_in, logits_out = logits.data_ptr(), None
+        else:
+            logits = torch.empty((T, E), dtype=torch.float32, device=dev)
+            logits_in, logits_out = None, logits.data_ptr()
+        with torch.cuda.device(dev):
+            need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), T))
+            if need == 0:
+                raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
+            ws = torch.empty((need,), dtype=torch.uint8, device=dev)
+            paged = manager.native_layer(block_index, T * self.top_k, E)
+            _native.check(lib.tris_moe_layer_forward_paged(C.byref(view), C.byref(paged), x.data_ptr(), logits_in, T, y.data_ptr(), logits_out,
+                                                           ws.data_ptr(), need, self._status_of(dev).data_ptr(),
+                                                           torch.cuda.current_stream(dev).cuda_stream), "moe_layer_forward_paged")
+            manager.end_layer()
+        return y, logits
 
     def forward_grouped_ops(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None):
         """Same result as :meth:`forward`, composed from the reference-named operators in

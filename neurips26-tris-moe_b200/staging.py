@@ -34,7 +34,7 @@ from typing import Optional
 import torch
 
 from . import _native
-from ._native import TrisCodedPageJob, TrisPageJob
+from ._native import TrisCodedPageJob, TrisPagedLayer, TrisPageJob, TrisPageLaunch, TrisProjView
 from .qlinear_grouped import proj_view
 
 BITMAP_KEYS = ("q_gmap_sparse",)
@@ -148,6 +148,10 @@ class GroupedQGmapCPUStagingManager:
         self._epoch = 0
         self._capturing = False
         self._consumed_epoch = []
+        self._route_done = None
+        self._record_info = {}     # (block index, projection) -> sizes of the tile records of its paged experts
+        self._slot_ids = None
+        self._layers = {}          # (layer, ring slot) -> what the native layer call takes: TrisPagedLayer and what it points at
 
     @property
     def buffer_nbytes(self) -> int:
@@ -190,6 +194,10 @@ class GroupedQGmapCPUStagingManager:
             self._consumed_epoch.append(-1)
         self._copy_stream = torch.cuda.Stream(device=self.device)
         self.capacity = cap
+        self._route_done = torch.cuda.Event()
+        for event in (*self._paged, *self._paged_gu, *self._consumed, self._route_done):
+            event.record(self._copy_stream)  # an event has its handle from then on
+        self._plan_records(E, cap)
         # drop the device copies: from here on the tensors exist only in pinned host memory
         for entry in self.entries.values():
             for key in entry.host:
@@ -204,22 +212,118 @@ class GroupedQGmapCPUStagingManager:
         self._initialized = True
         return True
 
+    def _plan_records(self, experts: int, cap: int) -> None:
+        """Buffers for the tile records of the experts of one layer, gate and up or down, per ring slot: the grouped kernels for records
+        are about twice as fast as those that read the planes, and building records from paged planes takes a fraction of that."""
+        lib, most = _native.load(), 0
+        with torch.cuda.device(self.device):
+            stream = torch.cuda.current_stream(self.device).cuda_stream
+            for bi in range(len(self.blocks)):
+                views = [proj_view(self.entries[(bi, proj)].payload) for proj in PROJECTIONS]
+                # a record's place is that of its segment, which output scales and biases are not indexed by
+                if any(v.output_scale or v.bias or (v.use_block_gr and v.gr_substreams != 32) for v in views):
+                    continue
+                info = torch.zeros((3, 4), dtype=torch.int64, device=self.device)
+                for i, v in enumerate(views):
+                    _native.check(lib.tris_paged_records_plan(C.byref(v), info[i].data_ptr(), stream), "paged_records_plan")
+                for proj, v, (per, size, steps, _) in zip(PROJECTIONS, views, info.tolist()):
+                    one = TrisProjView()
+                    C.pointer(one)[0] = v
+                    one.num_experts = 1
+                    columns = int(lib.tris_col_record_bytes(C.byref(one), steps))
+                    self._record_info[(bi, proj)] = (per, size, steps, columns)
+                gate, up, down = (sum(self._record_info[(bi, proj)][i] for i in (0, 3)) for proj in PROJECTIONS)
+                most = max(most, gate + up, down)
+            if most:
+                for ring in range(self.ring):
+                    self.buffers[(ring, "all", "tile_records")] = torch.empty((cap * most,), dtype=torch.uint8, device=self.device)
+                ids = torch.arange(max(experts, cap), dtype=torch.int32, device=self.device)
+                self._slot_ids = torch.where(ids < cap, ids, torch.full_like(ids, -1))
+
     # -- one layer ---------------------------------------------------------------------------
+    def native_layer(self, block_index: int, rows: int, experts: int) -> TrisPagedLayer:
+        """The argument of ``tris_moe_layer_forward_paged`` for a layer that routes ``rows`` rows: takes a ring slot as
+        :meth:`page_layer` does.  Call :meth:`end_layer` after the launch."""
+        self.initialize()
+        ring = self._take_slot()
+        launches, views = self._plan(block_index, ring)
+        layer = self._layers.get((block_index, ring))
+        if layer is None or layer[0] is not launches:
+            layer = self._layers[(block_index, ring)] = (launches, *self._paged_layer(block_index, ring, launches, views))
+        arg = layer[1]
+        arg.wait_consumed = int(self._used[ring] and self._consumed_epoch[ring] == self._epoch)
+        self.pipeline_stats["slot_reuses"] += arg.wait_consumed
+        nseg_bound = min(experts, rows, self.capacity)
+        self.pipeline_stats["bytes"] += nseg_bound * sum(launch[3] for launch in launches)
+        self.pipeline_stats["chunks"] += len(launches)
+        self.pipeline_stats["calls"] += 1
+        if self.collect_timings:
+            compute = torch.cuda.current_stream(self.device)
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
+            for event in events:
+                event.record(compute)  # an event has its handle from then on; recorded again by the call
+            arg.timing[:] = [event.cuda_event for event in events]
+            begin, end, w0, w1, w2, w3 = events
+            self._timings += [(begin, end, w0, w1), (w2, w2, w2, w3)]
+        else:
+            arg.timing[:] = [None] * 6
+        return arg
+
+    def end_layer(self) -> None:
+        """The slot of the last :meth:`native_layer` is in use until its "consumed" event, which the call has recorded."""
+        ring = (self._next - 1) % self.ring
+        self._used[ring] = True
+        self._consumed_epoch[ring] = self._epoch
+
+    def _paged_layer(self, block_index: int, ring: int, launches, views):
+        arg, keep = TrisPagedLayer(), []
+        groups, group = ([], []), 0
+        for coded, jobs, count, _, last_of_gate_up, table in launches:
+            groups[group].append(TrisPageLaunch(C.addressof(jobs), table, count, int(coded)))
+            group += int(last_of_gate_up)
+        for g, group in enumerate(groups):
+            pages = (TrisPageLaunch * max(1, len(group)))(*group)
+            keep.append(pages)
+            arg.pages[g], arg.num_pages[g] = C.addressof(pages), len(group)
+        records = self.buffers.get((ring, "all", "tile_records")) if (block_index, "gate") in self._record_info else None
+        at = 0
+        for i, proj in enumerate(PROJECTIONS):
+            arg.staged[i] = views[proj]
+            if records is None:
+                continue
+            arg.records[i] = proj_view(self.entries[(block_index, proj)].payload)
+            per, size, steps, columns = self._record_info[(block_index, proj)]
+            rec, at = arg.records[i], at if proj != "down" else 0  # down's take the place of gate's and up's, which are done with
+            rec.num_experts, rec.use_block_gr, rec.gmap_slot, rec.expert_slot = self.capacity, 1, None, None
+            rec.max_record_bytes, rec.max_sal_words = size, steps
+            rec.col_record_bytes = columns // max(1, per // (size * -(-rec.out_features // 128)))
+            rec.tile_records, rec.col_records = records.data_ptr() + at, records.data_ptr() + at + self.capacity * per
+            at += self.capacity * (per + columns)
+        arg.slot_ids, arg.capacity = None if self._slot_ids is None else self._slot_ids.data_ptr(), self.capacity
+        arg.copy_stream, arg.event_route = self._copy_stream.cuda_stream, self._route_done.cuda_event
+        arg.event_paged[:] = [self._paged_gu[ring].cuda_event, self._paged[ring].cuda_event]
+        arg.event_consumed = self._consumed[ring].cuda_event
+        return arg, keep
+
+    def _take_slot(self) -> int:
+        ring = self._next
+        self._next = (self._next + 1) % self.ring
+        capturing = bool(torch.cuda.is_current_stream_capturing())
+        if capturing != self._capturing:
+            self._capturing = capturing
+            self._epoch += 1
+        return ring
+
     def page_layer(self, block_index: int, route: dict):
         """Enqueues, on the side stream, the paging of gate/up/down of one layer for the
         experts of ``route`` (device arrays from ``tris_build_grouped_route``), and returns a
         handle whose views the grouped kernels of this layer must use."""
         self.initialize()
         lib = _native.load()
-        ring = self._next
-        self._next = (self._next + 1) % self.ring
         compute = torch.cuda.current_stream(self.device)
         copy = self._copy_stream
         copy.wait_stream(compute)  # the route must be final before the pager reads it
-        capturing = bool(torch.cuda.is_current_stream_capturing())
-        if capturing != self._capturing:
-            self._capturing = capturing
-            self._epoch += 1
+        ring = self._take_slot()
         if self._used[ring] and self._consumed_epoch[ring] == self._epoch:
             copy.wait_event(self._consumed[ring])
             self.pipeline_stats["slot_reuses"] += 1

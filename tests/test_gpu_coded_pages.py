@@ -110,3 +110,75 @@ def test_emptied_bitmap_of_a_payload_keeps_its_type(lib):
     assert manager.initialize()
     for name in ("gate", "up", "down"):
         assert manager.entries[(0, name)].coded and blk._get_grouped_payload(name)["q_gmap_sparse"].dtype == torch.int32
+
+
+RECORD_SHAPES = [(256, 192, 8, 2, 96, 32, 0.1), (264, 136, 12, 3, 300, 128, 0.1), (520, 200, 6, 2, 256, 64, 0.5), (128, 72, 5, 2, 44, 32, 0.97),
+                 (128, 136, 4, 2, 136, 32, 0.0)]
+
+
+@pytest.mark.parametrize("H,I,E,k,rank,group,salient", RECORD_SHAPES)
+@pytest.mark.parametrize("mode,sparse", [("bitmap", True), ("payload", True), ("payload", False)])
+def test_paged_experts_become_the_resident_records(lib, H, I, E, k, rank, group, salient, mode, sparse):
+    """Tile records built from paged planes are those of the resident block byte for byte, so that the kernels that read them give the same
+    bits; salient columns from none to nearly all, one to four row-scale slots a chunk, ragged outputs and columns, one to many row tiles."""
+    import numpy as np
+
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging, synth
+
+    rng = np.random.default_rng(H + rank)
+    raws = {n: synth.raw_projection(rng, E, O, rank, group_size=group, p_salient=salient, col_scale_one=False)
+            for n, O in (("gate", I), ("up", I), ("down", H))}
+    backbones = [torch.from_numpy(rng.normal(0, 0.1, (rank, w)).astype(np.float16)) for w in (H, H, I)]
+    router = torch.from_numpy(rng.standard_normal((E, H)).astype(np.float16))
+
+    def block(sparse):
+        blk = tm.TrisSparseMoeBlock(H, I, E, k, True)
+        payloads = [synth.pack_projection(raws[n], "cpu", True, True) for n in ("gate", "up", "down")]
+        for p in payloads:
+            p["compact3_use_block_gr"] = not sparse
+        return blk.load_grouped_payloads(*payloads, *backbones, router, device="cuda")
+
+    resident, streamed = block(False), block(sparse)
+    down = resident._get_grouped_payload("down")
+    records, cols = down["_tris_tile_records"].view(E, -1).clone(), down["_tris_col_records"].view(E, -1).clone()
+    manager = staging.GroupedQGmapCPUStagingManager([streamed], mode=mode)
+    manager.initialize()
+    for i, T in enumerate((1, 9, 40, 300)):
+        x = synth.synth_activations(T, H, seed=T).cuda().view(1, T, H)
+        logits = synth.synth_router_logits(T, E, seed=T).cuda()
+        want, _ = resident(x, router_logits=logits)
+        manager.collect_timings = bool(i % 2)
+        got, _ = streamed.forward_streaming(x, manager, 0, router_logits=logits)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want), T
+        assert streamed.last_kernel_status() == 0
+        active = sorted(set(torch.topk(torch.softmax(logits, 1), k, -1)[1].reshape(-1).tolist()))
+        per, size, steps, columns = manager._record_info[(0, "down")]
+        assert (per, columns) == (records.shape[1], cols.shape[1])
+        buffer = manager.buffers[((manager._next - 1) % manager.ring, "all", "tile_records")]
+        assert torch.equal(buffer[: len(active) * per].view(-1, per), records[active])
+        assert torch.equal(buffer[E * per: E * per + len(active) * columns].view(-1, columns), cols[active])
+    y, logits = streamed.forward_streaming(x, manager, 0)  # its own router
+    assert (y.float() - resident(x, router_logits=logits)[0].float()).abs().max() <= 2e-2
+
+
+def test_layers_with_output_scales_are_streamed_as_planes(lib):
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging, synth
+
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=6, keep_sparse_gmap=True)
+    outs = []
+    for scaled in (False, True):
+        blk = tm.TrisSparseMoeBlock(256, 192, 8, 2, True)
+        payloads = [dict(layer[n], compact3_use_block_gr=False) for n in ("gate", "up", "down")]
+        if scaled:
+            payloads[2].update(output_scale=torch.full((8, 256), 2.0, dtype=torch.float16), has_output_scale=True)
+        blk.load_grouped_payloads(*payloads, layer["shared_gate"], layer["shared_up"], layer["shared_down"], layer["router_weight"], device="cuda")
+        manager = staging.GroupedQGmapCPUStagingManager([blk])
+        manager.initialize()
+        assert ((0, "down") in manager._record_info) == (not scaled)
+        x = synth.synth_activations(7, 256, seed=1).cuda().view(1, 7, 256)
+        outs.append(blk.forward_streaming(x, manager, 0, router_logits=synth.synth_router_logits(7, 8, seed=2).cuda())[0].float())
+    assert (outs[1] - 2 * outs[0]).abs().max() <= 2e-2 * outs[0].abs().max()
