@@ -105,10 +105,11 @@ struct P4Problem {
   __half* out;
   int x_ld, out_ld;
   int x_aligned;  // set by packed4_gemm_impl: rows of x start on 16-byte boundaries
+  int out_quads;  // and four outputs of a row on 8-byte ones
 };
 int validate_packed4(const TrisPacked4View* w);
 int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRouteView* route, int num_rows, int out_mode,
-                      bool accumulate, bool silu, cudaStream_t stream);
+                      bool accumulate, bool silu, cudaStream_t stream, bool pdl);
 
 struct LaunchOpts {
   bool pdl = false;                  // programmatic dependent launch
@@ -173,6 +174,20 @@ __device__ __forceinline__ void mma_m16n8k16(float (&c)[4], uint32_t a0, uint32_
       "{%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
+  return d;
+}
+// Results of an m16n8 tile, rounded: lo = outputs g of rows 2t, 2t + 1, hi = outputs g + 8.  Afterwards the lane has row g, outputs
+// 8 (t & 1) + 2 (t & 2) .. + 3.  By a whole warp.
+__device__ __forceinline__ uint2 outputs_of_row(uint32_t lo, uint32_t hi, int t) {
+  lo = transpose_8x8(lo);  // row g, outputs 2t, 2t + 1
+  hi = transpose_8x8(hi);  // 8 + 2t, 9 + 2t; neighbours swap one
+  const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, (t & 1) ? lo : hi, 1);
+  return (t & 1) ? make_uint2(other, hi) : make_uint2(lo, other);
 }
 
 // One lane's value for the whole warp, in a form the compiler knows to be uniform.  The operands of a

@@ -51,12 +51,6 @@ __host__ __device__ inline DecodeLayout decode_layout(int max_sub_bytes, int max
   return l;
 }
 
-__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
-  uint32_t d;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
-  return d;
-}
-
 // Warps that an SM should hold; a launch with column parts has no more than 14 for it.
 constexpr int dec_min_ctas(int nt, int warps, bool parts) { return (parts ? 16 : (nt <= 2 ? 28 : 20)) / warps; }
 
@@ -389,10 +383,7 @@ __global__ void __launch_bounds__(32 * dec_warps(MODE == MODE_SINGLE ? 1 : 2, KS
           }
           // transposed: this lane holds row g, outputs 2t, 2t + 1 (lo) and 8 + 2t, 9 + 2t (hi); neighbours swap one
           // so that each stores four outputs
-          const uint32_t lo = transpose_8x8(h2_as_u32(__floats2half2_rn(y[0], y[1])));
-          const uint32_t hi = transpose_8x8(h2_as_u32(__floats2half2_rn(y[2], y[3])));
-          const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, (t & 1) ? lo : hi, 1);
-          const uint2 w = (t & 1) ? make_uint2(other, hi) : make_uint2(lo, other);
+          const uint2 w = outputs_of_row(h2_as_u32(__floats2half2_rn(y[0], y[1])), h2_as_u32(__floats2half2_rn(y[2], y[3])), t);
           const int n = nt * 8 + g;
           const int orow = n >= rows ? -1 : (args.out_scatter ? args.out_scatter[r0 + n] : r0 + n);
           if (orow >= 0) {

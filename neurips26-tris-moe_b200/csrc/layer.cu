@@ -163,7 +163,7 @@ static int launch_packed(const TrisPacked4View* const* w, int count, const __hal
     if (st != TRIS_OK) return st;
     p[i] = {*w[i], x, i ? out1 : out0, cols, w[i]->n, 0};
   }
-  return packed4_gemm_impl(p, count, nullptr, rows, out_mode, false, false, s);
+  return packed4_gemm_impl(p, count, nullptr, rows, out_mode, false, false, s, /*pdl=*/true);
 }
 }  // namespace tris
 
@@ -317,7 +317,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
       c2[n2++] = {*extras->ns_c2[i], x, w.ns_hidden[i], layer->hidden_size, ld, 0};
       c1[i] = {*extras->ns_c1[i], w.ns_hidden[i], c1[i].out, ld, layer->intermediate_size, 0};
     }
-    st = packed4_gemm_impl(c2, n2, &route, R, TRIS_OUT_F16, false, false, s);
+    st = packed4_gemm_impl(c2, n2, &route, R, TRIS_OUT_F16, false, false, s, true);
     if (st != TRIS_OK) return st;
     opts.weights_before_wait = true;  // the route is older than that launch
   }
@@ -327,7 +327,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
   if (ns_gu) {
     TrisRouteView rows = route;
     rows.row_gather = nullptr;
-    st = packed4_gemm_impl(c1, 2, &rows, R, TRIS_OUT_F16, true, /*silu=*/true, s);
+    st = packed4_gemm_impl(c1, 2, &rows, R, TRIS_OUT_F16, true, /*silu=*/true, s, true);
     if (st != TRIS_OK) return st;
   }
 
@@ -360,13 +360,13 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
     const int ld = ns_hidden_ld(extras->ns_c2[2]);
     const P4Problem dc2{*extras->ns_c2[2], w.mlp, w.ns_hidden[0], layer->intermediate_size, ld, 0};
     dc1 = {*extras->ns_c1[2], w.ns_hidden[0], w.down_out, ld, layer->hidden_size, 0};
-    st = packed4_gemm_impl(&dc2, 1, &route, R, TRIS_OUT_F16, false, false, s);
+    st = packed4_gemm_impl(&dc2, 1, &route, R, TRIS_OUT_F16, false, false, s, true);
     if (st != TRIS_OK) return st;
   }
   st = grouped_forward_impl(&layer->down, &route, w.hidden_down, w.down_out, s, opts);
   if (st != TRIS_OK) return st;
   if (dc1.x != nullptr) {
-    st = packed4_gemm_impl(&dc1, 1, &route, R, TRIS_OUT_F16, true, false, s);
+    st = packed4_gemm_impl(&dc1, 1, &route, R, TRIS_OUT_F16, true, false, s, true);
     if (st != TRIS_OK) return st;
   }
 

@@ -19,7 +19,7 @@
 // 8 columns of each, A fragments of two K = 16 steps if step j's K positions are columns 8t + 4j .. + 3;
 // the lane's activations of the slice are then 16 contiguous bytes.  Nibbles and activations are read
 // straight from global memory (L2 / L1) and nothing is staged; four CTAs on an SM hide the latency
-// better than loads four slices ahead in 125 registers (a whole block with null-space pairs, 37 tokens:
+// better than loads four slices ahead in 125 registers (a whole block with null-space pairs, 37 tokens, when C1 took this kernel too:
 // 128 against 148 us).  Staging 32 KB of nibbles and up to 128 KB of activation rows per CTA whatever the
 // problem's size let one CTA fill an SM: 64 segments of 5 rows, 2048 -> 64 and 64 -> 1024, took 42 us a
 // launch.  Gate and up share a launch.
@@ -64,10 +64,28 @@ __device__ __forceinline__ uint32_t p4_dequant_pair(uint32_t word, int i, __half
   return h2_as_u32(__hmul2(__hsub2(u32_as_h2(v), zc), sc));
 }
 
+// A lane's view of 16 outputs of one matrix: the quantisation of a group of columns.
+struct P4Group {
+  __half2 za, zb, sa, sb;  // 1024 + zero and scale of outputs a and b
+};
+__device__ __forceinline__ P4Group p4_group(const int32_t* z, const __half* s, int na, int nb) {
+  const uint32_t za = (static_cast<uint32_t>(__ldg(z + (na >> 3))) >> (4 * (na & 7))) & 0xFu;
+  const uint32_t zb = (static_cast<uint32_t>(__ldg(z + (nb >> 3))) >> (4 * (nb & 7))) & 0xFu;
+  return {__half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + za + 1u))),
+          __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + zb + 1u))), __half2half2(__ldg(s + na)), __half2half2(__ldg(s + nb))};
+}
+// Eight columns k .. k + 7 of a row of K; columns past K read as zeros.
+__device__ __forceinline__ uint4 p4_row_piece(const __half* src, int k, int K, bool aligned) {
+  if (k >= K) return make_uint4(0u, 0u, 0u, 0u);
+  if (aligned && k + 8 <= K) return *reinterpret_cast<const uint4*>(src);
+  uint32_t h[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = k + j < K ? __half_as_ushort(src[j]) : 0u;
+  return make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+}
+
 // grid (groups of 16 * 8 / ksplit outputs, segments or 1, problems * CTAs that share a segment's rows)
-// kSilu: both problems belong to one CTA, the second one (up) first, and problem 0's output becomes
-// silu(gate) * up, each rounded to fp16 where separate operators would round it.
-template <int NT, bool kSilu>
+template <int NT>
 __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kernel(const __grid_constant__ P4Args a) {
   constexpr int kRows = 8 * NT;
   extern __shared__ __align__(16) float red[];              // [warp][activation row][kP4RedStride]
@@ -89,19 +107,14 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
   const int outs = (kP4Warps / a.ksplit) * kP4TileN;
   const int cta_n = blockIdx.x * outs, n0 = cta_n + og * kP4TileN;
   if (rows <= 0 || row0 < 0) return;
-  const int np = kSilu ? 1 : a.num_problems;  // problems that CTAs of their own take
-  const int first = kSilu ? a.num_problems - 1 : static_cast<int>(blockIdx.z) % np;
-
+  const int np = a.num_problems;  // CTAs of their own for each
+  const P4Problem& pr = a.p[blockIdx.z % np];
+  const TrisPacked4View& w = pr.w;
   for (int r0 = (blockIdx.z / np) * kRows; r0 < rows; r0 += kRows * (gridDim.z / np)) {
-#pragma unroll 1
-  for (int pi = first; pi >= (kSilu ? 0 : first); --pi) {
-    const P4Problem& pr = a.p[pi];
-    const TrisPacked4View& w = pr.w;
-    const bool present = w.num_experts > 0;
     const int N = w.n_count ? w.n_count[e] : w.n;
-    const int K = !present ? 0 : (w.k_count ? w.k_count[e] : w.k);
+    const int K = w.k_count ? w.k_count[e] : w.k;
     const int G = max(1, w.g_count ? w.g_count[e] : w.num_groups);
-    if (cta_n >= N) continue;
+    if (cta_n >= N) return;
     const int n_off = w.n_off ? w.n_off[e] : 0;
     const int g_off = w.g_off ? w.g_off[e] : 0;
     // outputs past N repeat the last one
@@ -122,7 +135,7 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
       xr[i] = pr.x + static_cast<size_t>(a.row_gather ? a.row_gather[r] : r) * pr.x_ld + 8 * t;
     }
     int grp = -1;
-    __half2 zca = {}, zcb = {}, sca = {}, scb = {};
+    P4Group q = {};
 #pragma unroll 1
     for (int s = s_begin; s < s_end; ++s) {
       const int kw = 4 * s + t, k = 8 * kw;
@@ -131,35 +144,16 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
       const uint32_t wb = in ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + nb)) : 0u;
       uint4 xv[NT];
 #pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const __half* src = xr[i] + kP4SliceCols * s;
-        xv[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (in) {
-          if (pr.x_aligned && k + 8 <= K) {
-            xv[i] = *reinterpret_cast<const uint4*>(src);
-          } else {  // ragged end or unaligned rows; columns past K read as zeros
-            uint32_t h[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) h[j] = k + j < K ? __half_as_ushort(src[j]) : 0u;
-            xv[i] = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
-          }
-        }
-      }
+      for (int i = 0; i < NT; ++i) xv[i] = p4_row_piece(xr[i] + kP4SliceCols * s, k, K, pr.x_aligned);
       const int gi = min(s * kP4SliceCols / gs, G - 1);
       if (gi != grp) {
         grp = gi;
-        const int32_t* z = qz + static_cast<size_t>(gi) * w.z_ld;
-        const uint32_t za = (static_cast<uint32_t>(__ldg(z + (na >> 3))) >> (4 * (na & 7))) & 0xFu;
-        const uint32_t zb = (static_cast<uint32_t>(__ldg(z + (nb >> 3))) >> (4 * (nb & 7))) & 0xFu;
-        zca = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + za + 1u)));
-        zcb = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u + zb + 1u)));
-        sca = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + na));
-        scb = __half2half2(__ldg(sc + static_cast<size_t>(gi) * w.s_ld + nb));
+        q = p4_group(qz + static_cast<size_t>(gi) * w.z_ld, sc + static_cast<size_t>(gi) * w.s_ld, na, nb);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const uint32_t a0 = p4_dequant_pair(wa, 2 * j, zca, sca), a1 = p4_dequant_pair(wb, 2 * j, zcb, scb);
-        const uint32_t a2 = p4_dequant_pair(wa, 2 * j + 1, zca, sca), a3 = p4_dequant_pair(wb, 2 * j + 1, zcb, scb);
+        const uint32_t a0 = p4_dequant_pair(wa, 2 * j, q.za, q.sa), a1 = p4_dequant_pair(wb, 2 * j, q.zb, q.sb);
+        const uint32_t a2 = p4_dequant_pair(wa, 2 * j + 1, q.za, q.sa), a3 = p4_dequant_pair(wb, 2 * j + 1, q.zb, q.sb);
 #pragma unroll
         for (int i = 0; i < NT; ++i) mma_m16n8k16(acc[i], a0, a1, a2, a3, j ? xv[i].z : xv[i].x, j ? xv[i].w : xv[i].y);
       }
@@ -184,33 +178,175 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
       const int col = out_mode_pos(n, a.out_mode);
       __half* dst = pr.out + row * pr.out_ld + col;
       __half v = __float2half_rn(sum);
-      if (a.accumulate) v = present ? __hadd(*dst, v) : *dst;  // what out.add_(compensation) does in fp16
-      if constexpr (kSilu) {
-        if (pi == 0) {  // this thread wrote the other problem's element too
-          const float f = __half2float(v);
-          v = __hmul(__float2half_rn(f / (1.f + expf(-f))), a.p[1].out[row * a.p[1].out_ld + col]);
-        }
-      }
+      if (a.accumulate) v = __hadd(*dst, v);  // what out.add_(compensation) does in fp16
       *dst = v;
     }
     __syncthreads();
   }
+}
+
+// Products of few columns, as a rule added to what lies in the output: C1 of the null-space pairs.  A warp takes 32 outputs of one segment and
+// all their columns, so nothing is exchanged between warps, and asks for weights, rows and old outputs at once: a launch is
+// one round trip after the tables of the segment.  kSilu: both problems (gate, up) belong to a warp, and problem 0's output becomes silu(gate) *
+// up, each rounded to fp16 where separate operators would round it; up's own output is not stored.
+// grid (groups of 128 outputs, segments, 1 or problems), four warps.
+constexpr int kP4AddWarps = 4, kP4AddN = 32;
+template <int NT, bool kSilu>
+__global__ void __launch_bounds__(32 * kP4AddWarps) packed4_add_kernel(const __grid_constant__ P4Args a) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int seg = blockIdx.y;
+  const int nseg = a.num_segments_dev ? min(*a.num_segments_dev, a.num_segments) : a.num_segments;
+  if (seg >= nseg) return;
+  const int e = a.expert_ids[seg];
+  if (e < 0 || e >= a.num_experts) return;
+  const int row0 = a.segment_offsets[seg], rows = min(a.segment_offsets[seg + 1], a.num_rows) - row0;
+  if (rows <= 0 || row0 < 0) return;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = (blockIdx.x * kP4AddWarps + warp) * kP4AddN;
+
+  // sum of x . W^T for rows r0 .. of 32 outputs
+  auto product = [&](const P4Problem& pr, int N, int r0, float (&acc)[2][NT][4]) {
+    const TrisPacked4View& w = pr.w;
+    const int K = w.k_count ? w.k_count[e] : w.k, G = max(1, w.g_count ? w.g_count[e] : w.num_groups);
+    const int n_off = w.n_off ? w.n_off[e] : 0, g_off = w.g_off ? w.g_off[e] : 0;
+    const int32_t* qw = w.qweight + static_cast<size_t>(w.kw_off ? w.kw_off[e] : 0) * w.q_ld + n_off;
+    const int32_t* qz = w.qzeros + static_cast<size_t>(g_off) * w.z_ld + (w.z_off ? w.z_off[e] : 0);
+    const __half* sc = static_cast<const __half*>(w.scales) + static_cast<size_t>(g_off) * w.s_ld + n_off;
+    const int kwords = (K + 7) >> 3, slices = (K + kP4SliceCols - 1) / kP4SliceCols;
+    const int gs = w.group_size > 0 ? w.group_size : (K + kP4SliceCols);
+    const __half* xr[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      const int r = row0 + min(r0 + 8 * i + g, rows - 1);
+      xr[i] = pr.x + static_cast<size_t>(a.row_gather ? a.row_gather[r] : r) * pr.x_ld + 8 * t;
+    }
+    int grp = -1;
+    P4Group q[2] = {};
+#pragma unroll 1
+    for (int s0 = 0; s0 < slices; s0 += 2) {  // two slices in flight
+      uint32_t wv[2][4];
+      uint4 xv[2][NT];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int kw = 4 * (s0 + u) + t;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          wv[u][h] = kw < kwords ? static_cast<uint32_t>(__ldg(qw + static_cast<size_t>(kw) * w.q_ld + min(n0 + 8 * h + g, N - 1))) : 0u;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) xv[u][i] = p4_row_piece(xr[i] + kP4SliceCols * (s0 + u), 8 * kw, K, pr.x_aligned);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int gi = min((s0 + u) * kP4SliceCols / gs, G - 1);
+        if (gi != grp) {
+          grp = gi;
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+            q[m] = p4_group(qz + static_cast<size_t>(gi) * w.z_ld, sc + static_cast<size_t>(gi) * w.s_ld, min(n0 + 16 * m + g, N - 1), min(n0 + 16 * m + 8 + g, N - 1));
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t a0 = p4_dequant_pair(wv[u][2 * m], 2 * j, q[m].za, q[m].sa), a1 = p4_dequant_pair(wv[u][2 * m + 1], 2 * j, q[m].zb, q[m].sb);
+            const uint32_t a2 = p4_dequant_pair(wv[u][2 * m], 2 * j + 1, q[m].za, q[m].sa), a3 = p4_dequant_pair(wv[u][2 * m + 1], 2 * j + 1, q[m].zb, q[m].sb);
+#pragma unroll
+            for (int i = 0; i < NT; ++i) mma_m16n8k16(acc[m][i], a0, a1, a2, a3, j ? xv[u][i].z : xv[u][i].x, j ? xv[u][i].w : xv[u][i].y);
+          }
+      }
+    }
+  };
+  // four outputs of a row, 8 bytes where they are aligned
+  auto at = [&](const P4Problem& pr, int r, int n) { return pr.out + static_cast<size_t>(row0 + r) * pr.out_ld + n; };
+  auto load4 = [&](const P4Problem& pr, int N, int r, int n) {
+    uint2 v = make_uint2(0u, 0u);
+    if (!a.accumulate || r >= rows || n >= N) return v;
+    const __half* p = at(pr, r, n);
+    if (pr.out_quads && n + 4 <= N) return *reinterpret_cast<const uint2*>(p);
+    uint32_t h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = n + j < N ? __half_as_ushort(p[j]) : 0u;
+    return make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+  };
+  const P4Problem& first = a.p[kSilu ? 0 : blockIdx.z];
+  const int N0 = first.w.n_count ? first.w.n_count[e] : first.w.n, N1 = kSilu ? (a.p[1].w.n_count ? a.p[1].w.n_count[e] : a.p[1].w.n) : 0;
+  if (n0 >= max(N0, N1)) return;
+  auto pass = [&](const P4Problem& pr, int N, int r0, uint2 (&sum)[2][NT]) {  // old outputs and the product, each four outputs of a row
+    uint2 old[2][NT];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int i = 0; i < NT; ++i) old[m][i] = load4(pr, N, r0 + 8 * i + g, n0 + 16 * m + 8 * (t & 1) + 2 * (t & 2));
+    const bool present = pr.w.num_experts > 0 && n0 < N;
+    float acc[2][NT][4] = {};
+    if (present) product(pr, N, r0, acc);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        const uint2 v = outputs_of_row(h2_as_u32(__floats2half2_rn(acc[m][i][0], acc[m][i][1])), h2_as_u32(__floats2half2_rn(acc[m][i][2], acc[m][i][3])), t);
+        if (!a.accumulate) sum[m][i] = v;
+        else sum[m][i] = !present ? old[m][i] : make_uint2(h2_as_u32(__hadd2_rn(u32_as_h2(old[m][i].x), u32_as_h2(v.x))), h2_as_u32(__hadd2_rn(u32_as_h2(old[m][i].y), u32_as_h2(v.y))));
+      }
+  };
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += 8 * NT) {
+    uint2 y[2][NT];
+    pass(first, N0, r0, y);
+    if constexpr (kSilu) {
+      uint2 up[2][NT];
+      pass(a.p[1], N1, r0, up);
+      auto silu = [](uint32_t f, uint32_t u) {
+        const float2 v = __half22float2(u32_as_h2(f));
+        return h2_as_u32(__hmul2_rn(__floats2half2_rn(v.x / (1.f + expf(-v.x)), v.y / (1.f + expf(-v.y))), u32_as_h2(u)));
+      };
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int i = 0; i < NT; ++i) y[m][i] = make_uint2(silu(y[m][i].x, up[m][i].x), silu(y[m][i].y, up[m][i].y));
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        const int r = r0 + 8 * i + g, n = n0 + 16 * m + 8 * (t & 1) + 2 * (t & 2);
+        if (r >= rows) continue;
+        __half* p = at(first, r, n);
+        if (first.out_quads && n + 4 <= N0) {
+          *reinterpret_cast<uint2*>(p) = y[m][i];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (n + j < N0) p[j] = __ushort_as_half(static_cast<unsigned short>((j & 2 ? y[m][i].y : y[m][i].x) >> (16 * (j & 1))));
+        }
+      }
   }
 }
 
-template <int NT>
-static int launch_p4(const P4Args& args, bool silu, dim3 grid, cudaStream_t stream, bool pdl) {
-  constexpr size_t smem = static_cast<size_t>(kP4Warps) * 8 * NT * kP4RedStride * sizeof(float);
-  static_assert(smem <= 48 * 1024, "reduction buffer");
-  return check_cuda(silu ? launch_kernel(packed4_gemm_kernel<NT, true>, grid, dim3(kP4Threads), smem, stream, pdl, 1, args)
-                         : launch_kernel(packed4_gemm_kernel<NT, false>, grid, dim3(kP4Threads), smem, stream, pdl, 1, args),
-                    "packed4_gemm_kernel launch");
+template <int NT, bool kSilu>
+static int launch_add(const P4Args& args, cudaStream_t stream, bool pdl) {
+  const dim3 grid(ceil_div(args.n, kP4AddN * kP4AddWarps), args.num_segments, kSilu ? 1 : args.num_problems);
+  return check_cuda(launch_kernel(packed4_add_kernel<NT, kSilu>, grid, dim3(32 * kP4AddWarps), 0, stream, pdl, 1, args), "packed4_add_kernel launch");
+}
+template <bool kSilu>
+static int dispatch_add(const P4Args& args, int hint, cudaStream_t stream, bool pdl) {
+  if (hint <= 8) return launch_add<1, kSilu>(args, stream, pdl);
+  if (hint <= 16) return launch_add<2, kSilu>(args, stream, pdl);
+  return launch_add<4, kSilu>(args, stream, pdl);
 }
 
-// One launch for one or two problems on the same rows (gate and up).  `silu`: see the kernel; needs
+template <int NT>
+static int launch_p4(const P4Args& args, dim3 grid, cudaStream_t stream, bool pdl) {
+  constexpr size_t smem = static_cast<size_t>(kP4Warps) * 8 * NT * kP4RedStride * sizeof(float);
+  static_assert(smem <= 48 * 1024, "reduction buffer");
+  return check_cuda(launch_kernel(packed4_gemm_kernel<NT>, grid, dim3(kP4Threads), smem, stream, pdl, 1, args), "packed4_gemm_kernel launch");
+}
+
+// One launch for one or two problems on the same rows (gate and up).  `silu`: see packed4_add_kernel; needs a route and
 // two problems with `accumulate`, of which one may be absent (num_experts = 0; its `w.n` is still read).
 int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRouteView* route, int num_rows, int out_mode,
-                      bool accumulate, bool silu, cudaStream_t stream) {
+                      bool accumulate, bool silu, cudaStream_t stream, bool pdl) {
   if (num_rows == 0) return TRIS_OK;
   P4Args args{};
   args.num_problems = num_problems;
@@ -219,6 +355,7 @@ int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRou
     const TrisPacked4View& w = problems[i].w;
     args.p[i] = problems[i];
     args.p[i].x_aligned = ((reinterpret_cast<uintptr_t>(problems[i].x) & 15u) == 0 && problems[i].x_ld % 8 == 0) ? 1 : 0;
+    args.p[i].out_quads = (reinterpret_cast<uintptr_t>(problems[i].out) & 7u) == 0 && problems[i].out_ld % 4 == 0;
     args.n = std::max(args.n, w.n);
     args.num_experts = std::max(args.num_experts, w.num_experts);
     k = std::max(k, w.num_experts > 0 ? w.k : 0);
@@ -240,19 +377,22 @@ int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRou
   args.num_rows = num_rows;
   args.out_mode = out_mode;
   args.accumulate = accumulate ? 1 : 0;
-  // eight warps share 16 outputs where there are columns for all of them, else they take more outputs
   const int slices = ceil_div(k, kP4SliceCols);
+  // Few columns of many segments (C1 of null-space pairs): a warp per 32 outputs.  64 segments, 37 tokens, pairs of rank 32 and 64, a block
+  // with them on the kernel below / on this one 107 / 87 us, 512 tokens 350 / 208, 1 token 45.9 / 46.4.
+  TRIS_REQUIRE(args.num_segments <= 65535, TRIS_ERR_UNSUPPORTED, "tris_packed4_grouped_forward: more than 65535 segments");
+  if (silu) return dispatch_add<true>(args, hint, stream, pdl);
+  if (route && out_mode == TRIS_OUT_F16 && slices <= 4) return dispatch_add<false>(args, hint, stream, pdl);
+  // eight warps share 16 outputs where there are columns for all of them, else they take more outputs
   args.ksplit = slices >= 8 ? 8 : (slices >= 4 ? 4 : (slices >= 2 ? 2 : 1));
   dim3 grid(ceil_div(args.n, kP4TileN * kP4Warps / args.ksplit), route ? route->num_segments : 1);
-  TRIS_REQUIRE(grid.y <= 65535u, TRIS_ERR_UNSUPPORTED, "tris_packed4_grouped_forward: more than 65535 segments");
   // passes of 64 rows go to CTAs of their own while that leaves four per SM
-  const unsigned np = silu ? 1u : static_cast<unsigned>(num_problems);
+  const unsigned np = static_cast<unsigned>(num_problems);
   grid.z = np * std::max(1u, std::min(static_cast<unsigned>(ceil_div(hint, 64)), 592u / std::max(1u, grid.x * grid.y * np)));
-  const bool pdl = programmatic_launch_default();
-  if (hint <= 8) return launch_p4<1>(args, silu, grid, stream, pdl);
-  if (hint <= 16) return launch_p4<2>(args, silu, grid, stream, pdl);
-  if (hint <= 32) return launch_p4<4>(args, silu, grid, stream, pdl);
-  return launch_p4<8>(args, silu, grid, stream, pdl);
+  if (hint <= 8) return launch_p4<1>(args, grid, stream, pdl);
+  if (hint <= 16) return launch_p4<2>(args, grid, stream, pdl);
+  if (hint <= 32) return launch_p4<4>(args, grid, stream, pdl);
+  return launch_p4<8>(args, grid, stream, pdl);
 }
 
 int validate_packed4(const TrisPacked4View* w) {
@@ -279,6 +419,7 @@ extern "C" int tris_packed4_grouped_forward(const TrisPacked4View* w, const Tris
                "tris_packed4_grouped_forward: permuted output layouts need n %% 32 == 0");
   TRIS_REQUIRE(x_ld >= w->k && out_ld >= w->n && num_rows >= 0, TRIS_ERR_INVALID_ARG,
                "tris_packed4_grouped_forward: row strides x_ld=%d out_ld=%d", x_ld, out_ld);
-  const P4Problem problem{*w, static_cast<const __half*>(x_f16), static_cast<__half*>(out_f16), x_ld, out_ld, 0};
-  return packed4_gemm_impl(&problem, 1, route, num_rows, out_mode, accumulate != 0, false, static_cast<cudaStream_t>(stream));
+  const P4Problem problem{*w, static_cast<const __half*>(x_f16), static_cast<__half*>(out_f16), x_ld, out_ld, 0, 0};
+  return packed4_gemm_impl(&problem, 1, route, num_rows, out_mode, accumulate != 0, false, static_cast<cudaStream_t>(stream),
+                           programmatic_launch_default());
 }

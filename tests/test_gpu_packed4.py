@@ -286,3 +286,47 @@ def test_moe_block_with_vector_and_matrix_null_space(lib):
             mlp = gate_o / (1.0 + np.exp(-gate_o)) * up_o
             ref[t] += wts[t, s] * linear("down", e, mlp)[0]
     _check(y.view(T, -1), ref, floor=1e-4)
+
+
+@pytest.mark.parametrize("N,ranks,lengths,ld", [(33, [8, 0, 40, 16], [1, 9, 16, 3], 33), (130, [64, 128, 24, 96], [40, 1, 0, 17], 132), (1000, [16, 32, 64, 104], [8, 33, 70, 2], 1001),
+                                                (256, [128, 8, 72, 48], [5, 5, 24, 1], 256)])
+def test_grouped_product_of_few_columns(lib, N, ranks, lengths, ld):
+    """One to four slices of columns per segment, ragged outputs and rows, none to several passes, rows of the output on 2-, 4- and 8-byte
+    boundaries: plain and added, against the dequantised matrices."""
+    import ctypes as C
+
+    import trismoe_b200 as tm
+
+    rng = np.random.default_rng(N)
+    E, R, K = len(ranks), sum(lengths), max(ranks)
+    payload = _ns_layer(rng, E, 64, N, ranks)
+    np_payload = {k: (v.numpy() if isinstance(v, torch.Tensor) else v) for k, v in payload.items()}
+    from trismoe_b200.ns_compensation import prepare_ns_payload
+
+    view = prepare_ns_payload(payload, torch.device("cuda"))["_tris_c1_view"]
+    seg = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    ids = torch.arange(E, dtype=torch.int32, device="cuda")
+    offsets = torch.from_numpy(seg).cuda()
+    rv = tm._native.TrisRouteView()
+    rv.expert_ids, rv.segment_offsets, rv.num_segments, rv.num_rows, rv.max_rows_per_segment = ids.data_ptr(), offsets.data_ptr(), E, R, max(lengths)
+    for x_ld in (K, K + 3):  # rows on 16-byte boundaries and not
+        x = torch.full((R, x_ld), float("nan"), dtype=torch.float16, device="cuda")
+        x[:, :K] = torch.from_numpy(rng.standard_normal((R, K)).astype(np.float16))
+        for e in range(E):
+            x[seg[e]:seg[e + 1], ranks[e]:K] = float("nan")  # columns past a segment's own are not read
+        old = torch.from_numpy(rng.standard_normal((R, ld)).astype(np.float16)).cuda()
+        plain, added = torch.full_like(old, 7.0), old.clone()
+        stream = torch.cuda.current_stream().cuda_stream
+        for out, accumulate in ((plain, 0), (added, 1)):
+            tm._native.check(lib.tris_packed4_grouped_forward(C.byref(view), C.byref(rv), x.data_ptr(), x_ld, R, out.data_ptr(), ld, 0, accumulate, stream))
+        for e in range(E):
+            rows = slice(int(seg[e]), int(seg[e + 1]))
+            c1, _ = orc.ns_expert_matrices(np_payload, e)
+            if c1 is None or lengths[e] == 0:
+                continue
+            w, h = torch.from_numpy(c1).cuda().double(), x[rows, : ranks[e]].double()
+            ref = h @ w.T
+            bound = ranks[e] * 2.0 ** -22 * (h.abs() @ w.abs().T) * (1 + 2.0 ** -10) + ref.abs() * 2.0 ** -11 + 2.0 ** -25  # fp32 sums, rounded once
+            assert ((plain[rows, :N].double() - ref).abs() <= bound).all(), e
+            assert torch.equal(added[rows, :N], old[rows, :N] + plain[rows, :N])
+        assert (plain[:, N:] == 7.0).all() and torch.equal(added[:, N:], old[:, N:])
