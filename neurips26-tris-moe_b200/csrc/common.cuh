@@ -109,7 +109,7 @@ struct P4Problem {
 };
 int validate_packed4(const TrisPacked4View* w);
 int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRouteView* route, int num_rows, int out_mode,
-                      bool accumulate, bool silu, cudaStream_t stream, bool pdl);
+                      bool accumulate, bool silu, cudaStream_t stream, bool pdl, bool rows_ready = false);
 
 struct LaunchOpts {
   bool pdl = false;                  // programmatic dependent launch

@@ -54,6 +54,7 @@ struct P4Args {
   int accumulate;
   int n;       // outputs of either problem, at most
   int ksplit;  // warps that share 16 outputs: 1, 2, 4 or 8
+  int rows_ready;  // route and rows are older than the kernel before: only the stores wait for it
 };
 
 // byte i of `word` holds the nibbles of input columns 2i (low) and 2i+1 (high): returns
@@ -90,15 +91,19 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
   constexpr int kRows = 8 * NT;
   extern __shared__ __align__(16) float red[];              // [warp][activation row][kP4RedStride]
 
-  pdl_wait();  // activations (and a device-built route) come from the kernels before this one
+  if (!a.rows_ready) pdl_wait();  // activations (and a device-built route) come from the kernels before this one
   pdl_launch_dependents();
+  // A CTA without work leaves at once, but the first one waits: if none did, the launch could end before its predecessor.
+  auto leave = [&] {
+    if (a.rows_ready && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
+  };
   int e = 0, row0 = 0, rows = a.num_rows;
   if (a.num_segments > 0) {
     const int seg = blockIdx.y;
     const int nseg = a.num_segments_dev ? min(*a.num_segments_dev, a.num_segments) : a.num_segments;
-    if (seg >= nseg) return;
+    if (seg >= nseg) return leave();
     e = a.expert_ids[seg];
-    if (e < 0 || e >= a.num_experts) return;
+    if (e < 0 || e >= a.num_experts) return leave();
     row0 = a.segment_offsets[seg];
     rows = min(a.segment_offsets[seg + 1], a.num_rows) - row0;
   }
@@ -106,7 +111,7 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
   const int og = warp / a.ksplit, ks = warp % a.ksplit;
   const int outs = (kP4Warps / a.ksplit) * kP4TileN;
   const int cta_n = blockIdx.x * outs, n0 = cta_n + og * kP4TileN;
-  if (rows <= 0 || row0 < 0) return;
+  if (rows <= 0 || row0 < 0) return leave();
   const int np = a.num_problems;  // CTAs of their own for each
   const P4Problem& pr = a.p[blockIdx.z % np];
   const TrisPacked4View& w = pr.w;
@@ -114,7 +119,7 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
     const int N = w.n_count ? w.n_count[e] : w.n;
     const int K = w.k_count ? w.k_count[e] : w.k;
     const int G = max(1, w.g_count ? w.g_count[e] : w.num_groups);
-    if (cta_n >= N) return;
+    if (cta_n >= N) return leave();
     const int n_off = w.n_off ? w.n_off[e] : 0;
     const int g_off = w.g_off ? w.g_off[e] : 0;
     // outputs past N repeat the last one
@@ -167,6 +172,7 @@ __global__ void __launch_bounds__(kP4Threads, NT <= 2 ? 4 : 2) packed4_gemm_kern
       base[g + 8] = acc[i][2];
       base[kP4RedStride + g + 8] = acc[i][3];
     }
+    if (a.rows_ready) pdl_wait();
     __syncthreads();
     for (int i = tid; i < min(kRows, rows - r0) * outs; i += kP4Threads) {
       const int r = i / outs, j = i - r * outs, n = cta_n + j;
@@ -346,7 +352,7 @@ static int launch_p4(const P4Args& args, dim3 grid, cudaStream_t stream, bool pd
 // One launch for one or two problems on the same rows (gate and up).  `silu`: see packed4_add_kernel; needs a route and
 // two problems with `accumulate`, of which one may be absent (num_experts = 0; its `w.n` is still read).
 int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRouteView* route, int num_rows, int out_mode,
-                      bool accumulate, bool silu, cudaStream_t stream, bool pdl) {
+                      bool accumulate, bool silu, cudaStream_t stream, bool pdl, bool rows_ready) {
   if (num_rows == 0) return TRIS_OK;
   P4Args args{};
   args.num_problems = num_problems;
@@ -377,6 +383,7 @@ int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRou
   args.num_rows = num_rows;
   args.out_mode = out_mode;
   args.accumulate = accumulate ? 1 : 0;
+  args.rows_ready = pdl && rows_ready;
   const int slices = ceil_div(k, kP4SliceCols);
   // Few columns of many segments (C1 of null-space pairs): a warp per 32 outputs.  64 segments, 37 tokens, pairs of rank 32 and 64, a block
   // with them on the kernel below / on this one 107 / 87 us, 512 tokens 350 / 208, 1 token 45.9 / 46.4.
