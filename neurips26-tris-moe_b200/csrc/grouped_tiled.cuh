@@ -38,7 +38,6 @@ struct TiledArgs {
   int32_t hidden_perm;          // rows in a permuted order that can be read word by word
   int32_t num_sets;             // 2 when the two projections read different activation rows
   int32_t weights_before_wait;  // route arrays were final before the predecessor kernel started
-  int32_t rows_ready;           // decode kernel with column parts: activation rows too, only the stores wait
   int32_t stages;               // ring depth, 2 .. kMaxStages
   int32_t reuse;                // the chunks of a pass fit the ring: staged once for all tiles of a run
   int32_t rows_by_tensor;       // wide kernel: contiguous activation rows come by tensor copies
@@ -49,6 +48,7 @@ struct TiledArgs {
   float* partial;               // fp32 sums of the column parts, or null: no column split
   size_t partial_bytes;
   const __half* col_scale;      // optional [rank]: activation rows are multiplied by it while staged
+  int32_t rows_ready;           // decode kernel with column parts: route and activation rows were final then, only the stores wait
 };
 
 // Eight columns (8 * piece ..) of an activation row that cannot be copied as it is; `left`: how many of them exist.

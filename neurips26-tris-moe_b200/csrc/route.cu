@@ -2,9 +2,13 @@
 //
 // The route is built entirely on the device and written into arrays padded to the number
 // of experts, so the launch sequence of a layer never waits on the host.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tris {
 
@@ -83,6 +87,8 @@ __global__ void router_topk_kernel(const float* logits, int num_tokens, int num_
 // kernel<experts per lane> for the expert count
 #define TRIS_BY_EXPERTS(num_experts, kernel) \
   ((num_experts) <= 32 ? kernel<1> : (num_experts) <= 64 ? kernel<2> : (num_experts) <= 128 ? kernel<4> : kernel<8>)
+#define TRIS_BY_EXPERTS_2(num_experts, kernel, flag) \
+  ((num_experts) <= 32 ? kernel<1, flag> : (num_experts) <= 64 ? kernel<2, flag> : (num_experts) <= 128 ? kernel<4, flag> : kernel<8, flag>)
 
 // The flat (token, slot) list of expert ids: entry f is base[f * stride] - offset (stride 1, offset 0 for
 // a plain [T, k] array; an exchange buffer keeps the id of slot f behind that slot's activation row and
@@ -354,9 +360,9 @@ static int launch_route_parallel(const SelectedIds selected, int num_tokens, int
 
 // Router head and route together.  The experts of a token are distinct, so 32 tokens are one 32-bit mask per
 // expert, a row's place among its expert's rows of the group is the number of set bits below its token's,
-// and nothing is sorted.  Up to 32 tokens: one CTA, one warp per token, picks stay in registers.  More:
-// one CTA per 32 tokens writes picks and masks, and a second launch in which every CTA adds up the masks
-// for itself (they are a few KB) places them.  512 tokens of 64 experts: 17 us for top-k, then a
+// and nothing is sorted.  Up to 256 tokens: one launch, a CTA per 32 tokens with one warp per token, whose picks stay in registers;
+// several CTAs are a cluster and read one another's masks.  More: one CTA per 32 tokens writes picks and masks, and a second launch in
+// which every CTA adds up the masks for itself (they are a few KB) places them.  512 tokens of 64 experts: 17 us for top-k, then a
 // single-CTA counting sort of the flat list; now 6.
 struct RouteArgs {
   const float* logits;
@@ -380,16 +386,15 @@ __device__ __forceinline__ void route_place(const RouteArgs& a, int token, int s
   a.row_of_flat[f] = pos;
 }
 
-// kPlace: the whole route (one CTA, up to 32 tokens); otherwise the picks and masks of 32 tokens
-template <int NE, bool kPlace>
-__device__ __forceinline__ void router_group(const RouteArgs& a, uint32_t* sh) {
-  uint32_t* mask = sh;  // [E]
+// Picks of one group of 32 tokens, and their masks to shared memory.  The caller synchronises.
+template <int NE>
+__device__ __forceinline__ Pick router_picks(const RouteArgs& a, int group, uint32_t* mask) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = a.num_experts;
   for (int e = tid; e < E; e += blockDim.x) mask[e] = 0u;
   __syncthreads();
   pdl_wait();
   pdl_launch_dependents();
-  const int token = blockIdx.x * 32 + warp;
+  const int token = group * 32 + warp;
   Pick pick{0x7FFFFFFF, 0.f};
   if (token < a.num_tokens) {
     pick = topk_one_token<NE>(a.logits + static_cast<size_t>(token) * E, E, a.top_k, a.norm, lane);
@@ -399,30 +404,93 @@ __device__ __forceinline__ void router_group(const RouteArgs& a, uint32_t* sh) {
       a.weights[static_cast<size_t>(token) * a.top_k + lane] = pick.weight;
     }
   }
-  __syncthreads();
-  if constexpr (!kPlace) {
-    for (int e = tid; e < E; e += blockDim.x) a.masks[static_cast<size_t>(blockIdx.x) * E + e] = mask[e];
-  } else {
-    int32_t* count = reinterpret_cast<int32_t*>(sh) + E;
-    int32_t* start = count + E;
-    if (warp == 0) {
-      for (int e = lane; e < E; e += 32) count[e] = __popc(mask[e]);
-      __syncwarp();
-      route_scan_segments(count, start, E, a.m_tile, a.expert_ids, a.segment_offsets, a.problem_offsets, a.counts, lane);
-    }
-    __syncthreads();
-    if (token < a.num_tokens && lane < a.top_k) route_place(a, token, lane, pick.expert, start, pick.expert < E ? mask[pick.expert] : 0u);
-  }
+  return pick;
 }
-template <int NE>
+
+// The whole route; grid (1, 1, groups of 32 tokens), kCluster: a cluster of them.  At least as many threads as experts: thread e scans for expert e
+// (before: a single warp with E / 32 experts to a lane and three sums to scan, and from 33 tokens on two launches).  us for a block, before / now: 256
+// experts, 1, 32, 64, 256 tokens 22.1 / 20.0, 58.3 / 56.5, 73.1 / 70.4, 103.7 / 101.5; 64 experts, 1, 32, 128, 256 tokens 21.3 / 20.8, 45.8 /
+// 45.4, 60.7 / 60.2, 68.5 / 67.2.
+template <int NE, bool kCluster>
 __global__ void __launch_bounds__(kRouteThreads) router_route_kernel(const __grid_constant__ RouteArgs a) {
-  extern __shared__ int32_t sh[];
-  router_group<NE, true>(a, reinterpret_cast<uint32_t*>(sh));
+  __shared__ uint32_t mask[32 * kMaxExpertsPerLane];
+  __shared__ int32_t start[32 * kMaxExpertsPerLane];
+  __shared__ uint32_t warp_sums[kMaxExpertsPerLane];  // of 32 experts: rows | tiles << 16
+  __shared__ int32_t warp_segments[kMaxExpertsPerLane];
+  const int group = kCluster ? blockIdx.z : 0, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = a.num_experts;
+  const Pick pick = router_picks<NE>(a, group, mask);
+  if constexpr (kCluster) cg::this_cluster().sync();
+  else __syncthreads();
+  int rows = 0, before = 0, segment = 0;
+  uint32_t upto = 0u;  // rows | tiles << 16 of the experts up to this one
+  bool active = false;
+  if (warp * 32 < E) {
+    if (tid < E) {
+      if constexpr (kCluster) {
+        for (int g = 0; g < static_cast<int>(gridDim.z); ++g) {
+          const int n = __popc(*cg::this_cluster().map_shared_rank(&mask[tid], g));
+          rows += n;
+          if (g < group) before += n;
+        }
+      } else {
+        rows = __popc(mask[tid]);
+      }
+    }
+    active = rows > 0;
+    upto = static_cast<uint32_t>(rows) | static_cast<uint32_t>((rows + a.m_tile - 1) / a.m_tile) << 16;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t n = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+      if (lane >= o) upto += n;
+    }
+    const uint32_t any = __ballot_sync(0xFFFFFFFFu, active);
+    segment = __popc(any & ((1u << lane) - 1u));
+    if (lane == 31) {
+      warp_sums[warp] = upto;
+      warp_segments[warp] = __popc(any);
+    }
+  }
+  __syncthreads();
+  uint32_t total = 0u, first = 0u;
+  int segments = 0, first_segment = 0;
+  for (int w = 0; w * 32 < E; ++w) {
+    if (w < warp) first += warp_sums[w], first_segment += warp_segments[w];
+    total += warp_sums[w];
+    segments += warp_segments[w];
+  }
+  if (tid < E) {
+    const int tiles = (rows + a.m_tile - 1) / a.m_tile, row = static_cast<int>((first + upto) & 0xFFFFu) - rows, tile = static_cast<int>((first + upto) >> 16) - tiles;
+    start[tid] = row + before;
+    if (active && group == 0) {
+      const int s = first_segment + segment;
+      a.expert_ids[s] = tid;
+      a.segment_offsets[s] = row;
+      a.problem_offsets[s] = tile;
+    }
+  }
+  if (group == 0) {
+    for (int q = segments + tid; q <= E; q += blockDim.x) {
+      a.segment_offsets[q] = static_cast<int>(total & 0xFFFFu);
+      a.problem_offsets[q] = static_cast<int>(total >> 16);
+      if (q < E) a.expert_ids[q] = -1;
+    }
+    if (tid == 0) {
+      a.counts[0] = segments;
+      a.counts[1] = static_cast<int>(total >> 16);
+    }
+  }
+  __syncthreads();
+  const int token = group * 32 + warp;
+  if (token < a.num_tokens && lane < a.top_k) route_place(a, token, lane, pick.expert, start, pick.expert < E ? mask[pick.expert] : 0u);
+  if constexpr (kCluster) cg::this_cluster().sync();  // the masks stay until every CTA has read them
 }
+// Picks and masks of 32 tokens
 template <int NE>
 __global__ void __launch_bounds__(kRouteThreads) router_masks_kernel(const __grid_constant__ RouteArgs a) {
   extern __shared__ int32_t sh[];
-  router_group<NE, false>(a, reinterpret_cast<uint32_t*>(sh));
+  uint32_t* mask = reinterpret_cast<uint32_t*>(sh);
+  router_picks<NE>(a, blockIdx.x, mask);
+  __syncthreads();
+  for (int e = threadIdx.x; e < a.num_experts; e += blockDim.x) a.masks[static_cast<size_t>(blockIdx.x) * a.num_experts + e] = mask[e];
 }
 
 // grid: CTAs that share the groups of 32 tokens in runs
@@ -524,7 +592,7 @@ __global__ void combine_routed_kernel(const __half* rows, const int32_t* row_of_
 
 static int route_smem_bytes(int num_experts) { return static_cast<int>((2 + kRouteThreads / 32) * num_experts * sizeof(int32_t)); }
 
-// Router head + route for the fused layer path: one launch for up to 32 tokens, two for more, or top-k and the
+// Router head + route for the fused layer path: one launch for up to 256 tokens, two for more, or top-k and the
 // general route where `scratch` does not hold the masks.
 int launch_router_route(const float* logits, int num_tokens, int num_experts, int top_k, int norm, int m_tile,
                         int32_t* selected, float* weights, int32_t* perm, int32_t* tok, int32_t* slot,
@@ -534,11 +602,14 @@ int launch_router_route(const float* logits, int num_tokens, int num_experts, in
                "router: supports up to %d experts and top-32", 32 * kMaxExpertsPerLane);
   const RouteArgs args{logits, num_tokens, top_k, num_experts, norm, m_tile, selected, weights, perm, tok, slot, row_of_flat,
                        expert_ids, segment_offsets, problem_offsets, counts, reinterpret_cast<uint32_t*>(scratch)};
-  if (num_tokens <= 32)
-    return check_cuda(launch_kernel(TRIS_BY_EXPERTS(num_experts, router_route_kernel), dim3(1), dim3(32 * num_tokens),
-                                    3 * sizeof(int32_t) * num_experts, stream, /*pdl=*/true, 1, args),
-                      "router_route_kernel launch");
   const int groups = ceil_div(num_tokens, 32);
+  if (groups == 1)
+    return check_cuda(launch_kernel(TRIS_BY_EXPERTS_2(num_experts, router_route_kernel, false), dim3(1), dim3(std::max(32 * num_tokens, ceil_div(num_experts, 32) * 32)), 0,
+                                    stream, /*pdl=*/true, 1, args),
+                      "router_route_kernel launch");
+  if (groups <= 8)  // a portable cluster
+    return check_cuda(launch_kernel(TRIS_BY_EXPERTS_2(num_experts, router_route_kernel, true), dim3(1, 1, groups), dim3(kRouteThreads), 0, stream, /*pdl=*/true, groups, args),
+                      "router_route_kernel launch");
   if (scratch && scratch_bytes >= sizeof(int32_t) * static_cast<size_t>(groups) * num_experts) {
     const int st = check_cuda(launch_kernel(TRIS_BY_EXPERTS(num_experts, router_masks_kernel), dim3(groups), dim3(kRouteThreads),
                                             sizeof(int32_t) * num_experts, stream, /*pdl=*/true, 1, args),

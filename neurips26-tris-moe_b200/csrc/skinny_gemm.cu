@@ -137,8 +137,10 @@ int launch_shared_hidden(const SkinnyProblem* probs, int num_problems, const __h
   if (n == 0) return TRIS_OK;
   for (int i = 0; i < num_problems; ++i)
     TRIS_REQUIRE(probs[i].a && probs[i].out && probs[i].m > 0, TRIS_ERR_INVALID_ARG, "shared hidden: bad problem %d", i);
-  // enough rows for a dense contraction: tcgen05 / TMEM tiles
-  if (tc_gemm_applicable(n, k, x, probs, num_problems))
+  // Enough rows for a dense contraction: tcgen05 / TMEM tiles.  us, here / there, 256 outputs: 36 and 63 rows of 2048 columns (two matrices and
+  // a router of 64) 9.2 / 7.4, 10.1 / 7.4, of 1024 8.2 / 6.7, of 512 6.7 / 6.9, of 14336 15.1 / 12.0; 32 rows 6.8 / 7.4, 5.8 / 6.7,
+  // 4.8 / 6.9, 12.5 / 12.0.  Gathered rows from 64 on.
+  if ((row_gather == nullptr || n >= 64) && tc_gemm_applicable(n, k, x, probs, num_problems))
     return launch_tc_gemm(probs, num_problems, x, row_gather, n, k, stream, pdl, n_dev, nullptr, matrices_before_wait);
   SkinnyArgs args{};
   int mtiles = 0;

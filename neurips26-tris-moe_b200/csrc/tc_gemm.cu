@@ -475,10 +475,10 @@ static int launch_umma_tma(const TcGemmArgs& args, const TcTmaMaps& maps, int mt
                     "umma_gemm_tma_kernel launch");
 }
 
-// True when the tensor-core path applies: enough rows for a dense contraction, K a multiple
+// True when the tensor-core path applies: more rows than the skinny GEMM takes better for a dense contraction, K a multiple
 // of the 64-column chunk, 16-byte aligned rows.
 bool tc_gemm_applicable(int n, int k, const __half* x, const SkinnyProblem* probs, int num_problems) {
-  if (n < 64 || (k % kTcKChunk) != 0 || (reinterpret_cast<uintptr_t>(x) & 15u)) return false;
+  if (n <= 32 || (k % kTcKChunk) != 0 || (reinterpret_cast<uintptr_t>(x) & 15u)) return false;
   for (int i = 0; i < num_problems; ++i)
     if (reinterpret_cast<uintptr_t>(probs[i].a) & 15u) return false;
   return true;
