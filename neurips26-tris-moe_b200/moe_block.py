@@ -190,7 +190,7 @@ class TrisSparseMoeBlock(nn.Module):
         lib = _native.load()
         for name in key:
             p = self.packed_backbones[name]
-            skey = (str(dev), name, p.rows, p.cols)
+            skey = (dev, name, p.rows, p.cols)
             scratch = TrisSparseMoeBlock._expand_scratch.get(skey) if own is None else None
             if scratch is None:
                 scratch = torch.empty((p.rows, p.cols), dtype=torch.float16, device=dev)
@@ -201,10 +201,10 @@ class TrisSparseMoeBlock(nn.Module):
             if getattr(p, "_g_idx", None) is None:
                 g_idx = (torch.arange(p.cols, device=dev, dtype=torch.int32) // max(1, p.group_size)).clamp_(max=p.groups - 1)
                 p._g_idx = g_idx.to(torch.int32).contiguous()
-            with torch.cuda.device(dev):
+            with _native.on_device(dev):
                 _native.check(lib.tris_packed4_dequantize(p.qweight.data_ptr(), p.qzeros.data_ptr(), p.scales.data_ptr(),
                                                           p._g_idx.data_ptr(), p.rows, p.cols, p.groups, scratch.data_ptr(),
-                                                          torch.cuda.current_stream(dev).cuda_stream), "packed4_dequantize")
+                                                          _native.stream_of(dev)), "packed4_dequantize")
             setattr(v, "shared_" + name, scratch.data_ptr())
             setattr(v, "packed_" + name, None)
         return v
@@ -283,9 +283,9 @@ class TrisSparseMoeBlock(nn.Module):
         lib = _native.load()
         dev = self._workspace.device
         word = C.c_int32(0)
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             _native.check(lib.tris_moe_layer_last_status(self._workspace.data_ptr(), int(bool(clear)),
-                                                         torch.cuda.current_stream(dev).cuda_stream, C.byref(word)),
+                                                         _native.stream_of(dev), C.byref(word)),
                           "moe_layer_last_status")
         return int(word.value) or streamed
 
@@ -323,8 +323,11 @@ class TrisSparseMoeBlock(nn.Module):
             raise RuntimeError(f"trismoe_b200: grouped expert kernels require float16 hidden states, got {hidden_states.dtype}")
         lib = _native.load()
         shape = hidden_states.shape
-        x = hidden_states.reshape(-1, shape[-1]).contiguous()
-        T = int(x.shape[0])
+        if extras is None and hidden_states.is_contiguous() and shape[-1] == self.hidden_size:
+            x, T = hidden_states, hidden_states.numel() // self.hidden_size  # as it is: the kernels take addresses
+        else:
+            x = hidden_states.reshape(-1, shape[-1]).contiguous()
+            T = int(x.shape[0])
         dev = x.device
         y = torch.empty_like(x)
         returned = router_logits
@@ -349,8 +352,8 @@ class TrisSparseMoeBlock(nn.Module):
                     big = sorted(set(big) | ({"gate", "up"} & set(self.packed_backbones)))
                 if big:
                     view = self._expanded_layer_view(dev, big, own)
-            with torch.cuda.device(dev):
-                stream = torch.cuda.current_stream(dev).cuda_stream
+            with _native.on_device(dev):
+                stream = _native.stream_of(dev)
                 if shared is not None:
                     scratch = self._shared_scratch(lib, shared, T, dev)
                     st = lib.tris_moe_layer_forward_shared(C.byref(view), C.byref(shared), x.data_ptr(), logits_in, T, y.data_ptr(), logits_out,
@@ -363,7 +366,7 @@ class TrisSparseMoeBlock(nn.Module):
                     st = lib.tris_moe_layer_forward_extras_status(C.byref(view), C.byref(extras), x.data_ptr(), logits_in, T, y.data_ptr(),
                                                                   logits_out, ws.data_ptr(), ws.numel(), self._status_of(dev).data_ptr(), stream)
                 _native.check(st, "moe_layer_forward")
-        return y.reshape(shape), logits if extras is None else returned
+        return y if x is hidden_states else y.reshape(shape), logits if extras is None else returned
 
     def forward_streaming(self, hidden_states: torch.Tensor, manager, block_index: int,
                           router_logits: Optional[torch.Tensor] = None):
@@ -389,8 +392,8 @@ class TrisSparseMoeBlock(nn.Module):
         if all(plain(name) for name in ("gate", "up", "down")):
             y, logits = self._forward_streaming_native(lib, x, y, manager, block_index, router_logits)
             return y.reshape(shape), logits
-        with torch.cuda.device(dev):
-            stream = torch.cuda.current_stream(dev).cuda_stream
+        with _native.on_device(dev):
+            stream = _native.stream_of(dev)
             # one allocation for everything between the kernels; the host has 25 launches a layer to prepare
             sizes = [4 * R] * 6 + [4 * E, 4 * (E + 1), 4 * (E + 1), 16, 2 * T * r_gu, 2 * T * r_gu, 2 * R * I, 2 * R * r_d, 2 * R * H]
             offsets, total = [], 0
@@ -451,7 +454,7 @@ class TrisSparseMoeBlock(nn.Module):
         else:
             logits = torch.empty((T, E), dtype=torch.float32, device=dev)
             logits_in, logits_out = None, logits.data_ptr()
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             need = int(lib.tris_moe_layer_workspace_bytes(C.byref(view), T))
             if need == 0:
                 raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
@@ -459,7 +462,7 @@ class TrisSparseMoeBlock(nn.Module):
             paged = manager.native_layer(block_index, T * self.top_k, E)
             _native.check(lib.tris_moe_layer_forward_paged(C.byref(view), C.byref(paged), x.data_ptr(), logits_in, T, y.data_ptr(), logits_out,
                                                            ws.data_ptr(), need, self._status_of(dev).data_ptr(),
-                                                           torch.cuda.current_stream(dev).cuda_stream), "moe_layer_forward_paged")
+                                                           _native.stream_of(dev)), "moe_layer_forward_paged")
             manager.end_layer()
         return y, logits
 
@@ -579,8 +582,8 @@ class TrisQwen2SparseMoeBlock(TrisSparseMoeBlock):
             return routed + torch.sigmoid(torch.nn.functional.linear(hidden_states, w)) * shared, logits
         x, shared = hidden_states.contiguous(), shared.contiguous()
         T = routed.numel() // self.hidden_size
-        with torch.cuda.device(routed.device):
+        with _native.on_device(routed.device):
             _native.check(_native.load().tris_shared_expert_add(x.data_ptr(), w.data_ptr(), routed.data_ptr(), shared.data_ptr(), T, self.hidden_size,
-                                                                routed.data_ptr(), torch.cuda.current_stream(routed.device).cuda_stream),
+                                                                routed.data_ptr(), _native.stream_of(routed.device)),
                           "shared_expert_add")
         return routed, logits

@@ -199,7 +199,7 @@ def _launch(view, route, x, x_ld, rows, out, out_ld, accumulate, gather: bool):
     if not gather:
         rv.row_gather = None
     lib = _native.load()
-    with torch.cuda.device(x.device):
+    with _native.on_device(x.device):
         _native.check(lib.tris_packed4_grouped_forward(C.byref(view), C.byref(rv), x.data_ptr(), int(x_ld), int(rows), out.data_ptr(),
                                                        int(out_ld), 0, int(bool(accumulate)), _stream_ptr(x.device)),
                       "packed4_grouped_forward")
@@ -310,7 +310,7 @@ class Packed4Linear(torch.nn.Module):
         out = torch.empty((x2.shape[0], self.rows), dtype=torch.float16, device=x.device)
         if x2.shape[0]:
             lib = _native.load()
-            with torch.cuda.device(x.device):
+            with _native.on_device(x.device):
                 _native.check(lib.tris_packed4_grouped_forward(C.byref(self._view), None, x2.data_ptr(), int(x2.stride(0)),
                                                                int(x2.shape[0]), out.data_ptr(), self.rows, int(layout), 0,
                                                                _stream_ptr(x.device)), "packed4_grouped_forward")

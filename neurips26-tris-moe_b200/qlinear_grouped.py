@@ -32,7 +32,7 @@ HIDDEN_ROW_MAJOR, HIDDEN_PAIR_INTERLEAVED, HIDDEN_LANE_ORDER = 0, 2, 3
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return _native.stream_of(device)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -135,7 +135,7 @@ def prepare_grouped_payload(payload: dict, device=None, gr_substreams: int = DEF
         return payload
     status = torch.zeros((2,), dtype=i32, device=dev)
     stream = _stream_ptr(dev)
-    with torch.cuda.device(dev):
+    with _native.on_device(dev):
         groups = torch.empty((E, pr), dtype=i32, device=dev)
         _native.check(
             lib.tris_build_row_groups(payload["g_idx"].data_ptr(), E, rank, G, groups.data_ptr(), status[0:].data_ptr(), stream),
@@ -225,7 +225,7 @@ def _build_tile_records(payload: dict, lib, dev) -> None:
     ``tris_tile_records_build``) into tensors kept in the payload dict."""
     view = _build_view(payload, need_index=True)
     stream = _stream_ptr(dev)
-    with torch.cuda.device(dev):
+    with _native.on_device(dev):
         count = int(lib.tris_tile_record_count(C.byref(view)))
         desc = torch.empty((count + 1, 2), dtype=torch.int32, device=dev)
         info = torch.zeros((4,), dtype=torch.int64, device=dev)
@@ -327,7 +327,7 @@ def decode_block_gr_gmap(payload: dict) -> torch.Tensor:
     dev = payload["qweight1"].device
     E, O, rank, _ = payload["_tris_dims"]
     out = torch.empty((E, math.ceil(rank / 32), O), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _native.on_device(dev):
         _native.check(lib.tris_block_gr_decode(C.byref(view), out.data_ptr(), _stream_ptr(dev)), "block_gr_decode")
     return out
 
@@ -340,7 +340,7 @@ def dequantize_grouped_payload(payload: dict) -> torch.Tensor:
     dev = payload["qweight1"].device
     E, O, rank, _ = payload["_tris_dims"]
     out = torch.empty((E, O, rank), dtype=torch.float16, device=dev)
-    with torch.cuda.device(dev):
+    with _native.on_device(dev):
         _native.check(lib.tris_compact3_dequantize(C.byref(view), out.data_ptr(), _stream_ptr(dev)), "compact3_dequantize")
     return out
 
@@ -385,7 +385,7 @@ def build_grouped_route(selected_experts: torch.Tensor, num_experts: int, m_tile
     seg = buf[base + E: base + 2 * E + 1]
     prob = buf[base + 2 * E + 1: base + 3 * E + 2]
     counts = buf[base + 3 * E + 2: base + 3 * E + 4]
-    with torch.cuda.device(device):
+    with _native.on_device(device):
         _native.check(
             lib.tris_build_grouped_route_ex(sel.data_ptr(), 1, 0, T, k, E, int(m_tile), perm.data_ptr(), tok.data_ptr(),
                                             slot.data_ptr(), rof.data_ptr(), expert_ids.data_ptr(), seg.data_ptr(),
@@ -553,7 +553,7 @@ def run_grouped_structured_expert_forward(
         return out
     keep: list = []
     rv = _route_view(route, R, keep)
-    with torch.cuda.device(hidden.device):
+    with _native.on_device(hidden.device):
         ws = _linear_workspace(lib, view, 1, R, hidden.device) if route.get("_one_segment") else None
         if ws is not None:
             st = lib.tris_linear_forward(C.byref(view), None, C.byref(rv), hidden.data_ptr(), None, out.data_ptr(), None, 0, ws.data_ptr(),
@@ -619,7 +619,7 @@ def run_grouped_structured_expert_pair_forward(
         return out_a, out_b
     keep: list = []
     rv = _route_view(route, R, keep)
-    with torch.cuda.device(dev):
+    with _native.on_device(dev):
         b_ptr = None if out_b is None else out_b.data_ptr()
         ws = _linear_workspace(lib, va, 2, R, dev) if route.get("_one_segment") else None
         if ws is not None:
@@ -661,7 +661,7 @@ def compute_shared_hidden(x: torch.Tensor, shared_sv: torch.Tensor, layout: int 
         raise RuntimeError("trismoe_b200 compute_shared_hidden: x and shared_sv disagree on in_features")
     out = torch.empty((x2.shape[0], rank), dtype=torch.float16, device=x.device)
     if x2.shape[0]:
-        with torch.cuda.device(x.device):
+        with _native.on_device(x.device):
             _native.check(
                 lib.tris_shared_hidden_forward(x2.data_ptr(), None, int(x2.shape[0]), None, in_features, sv.data_ptr(), rank,
                                                out.data_ptr(), int(layout), _stream_ptr(x.device)),
@@ -692,10 +692,10 @@ def dequantize_packed_4bit(payload: dict, device) -> torch.Tensor:
         raise RuntimeError(f"trismoe_b200: inconsistent 4-bit matrix payload: qweight {tuple(qweight.shape)}, qzeros "
                            f"{tuple(qzeros.shape)}, scales {tuple(scales.shape)}, g_idx {g_idx.numel()}, rows {rows}, cols {cols}")
     out = torch.empty((rows, cols), dtype=torch.float16, device=dev)
-    with torch.cuda.device(dev):
+    with _native.on_device(dev):
         _native.check(lib.tris_packed4_dequantize(qweight.data_ptr(), qzeros.data_ptr(), scales.data_ptr(), g_idx.data_ptr(),
                                                   rows, cols, groups, out.data_ptr(),
-                                                  torch.cuda.current_stream(dev).cuda_stream), "packed4_dequantize")
+                                                  _native.stream_of(dev)), "packed4_dequantize")
     return out
 
 
