@@ -425,11 +425,12 @@ static int launch_decode(TiledArgs args, cudaStream_t stream, bool pdl, int col_
 
 template <int NT, int MODE>
 static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) {
-  // Fewer than 14 warps per SM: split the columns, as far as there are columns to split.  Shared passes have the widest
-  // tile, of which 20 warps fit an SM instead of 28: fewer than 10.
-  const long long warps = decode_warps(args, MODE) * args.row_split;
+  // Fewer than 13 warps per SM: split the columns, as far as there are columns to split.  Of the wider tiles 20 warps fit an SM instead of 28:
+  // fewer than 10 (1024 warps of 8 experts x 4096 x 256 in halves and not in quarters: blocks of 24, 40, 64 and 80 tokens 50.4 / 49.3, 59.5 / 56.1,
+  // 61.4 / 58.1, 68.0 / 63.7 us).
+  const long long warps = decode_warps(args, MODE) * args.row_split, split = (NT >= 3 ? 10 : 13) * sm_count();
   const int slices = ceil_div(args.rank, kSliceCols), groups = ceil_div(args.rank, kDecCols), want = (args.row_split > 1 ? 10 : 14) * sm_count();
-  // Many columns: over the CTAs of a cluster too, by 256 columns or more each, up to as many warps as above.  us at 8 rows, eight warps to
+  // Many columns: over the CTAs of a cluster too, by 256 columns or more each, up to 14 warps per SM (10 with shared passes).  us at 8 rows, eight warps to
   // 32 outputs in one CTA / this: 4096 x 4096 18.6 / 11.2, pair of 1024 x 4096 25.8 / 8.4, pair of 2048 x 2048 14.4 / 8.1, 512 x 1024 6.2 /
   // 4.6, 256 x 8192 33.9 / 8.2 (clusters of 1, 2, 4 and 8 CTAs in an earlier form: 4096 x 4096 24.5, 15.7, 12.0, 13.8; pair of 2048 x 2048
   // 18.1, 11.5, 8.6, 12.0).  With 512 columns two CTAs are no faster than one (2048 x 512, 8 and 24 rows 5.0 / 5.0, 6.6 / 7.5).
@@ -439,23 +440,23 @@ static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) 
     while (parts < 8 && warps * 8 * parts <= want && groups >= 2 * parts && groups >= 4) parts *= 2;
     return launch_decode<NT, MODE, 4, true>(args, stream, pdl, parts);
   }
-  if (warps * 2 < want && slices >= 4) return launch_decode<NT, MODE, 4>(args, stream, pdl);
-  if (warps < want && slices >= 4) return launch_decode<NT, MODE, 2>(args, stream, pdl);
+  if (warps * 2 < split && slices >= 4) return launch_decode<NT, MODE, 4>(args, stream, pdl);
+  if (warps < split && slices >= 4) return launch_decode<NT, MODE, 2>(args, stream, pdl);
   return launch_decode<NT, MODE, 1>(args, stream, pdl);
 }
 
 template <int MODE>
-static int dispatch_decode(const TiledArgs& args, int typical_rows, cudaStream_t stream, bool pdl) {
-  if (typical_rows <= 8) return dispatch_split<1, MODE>(args, stream, pdl);
-  if (typical_rows <= 16) return dispatch_split<2, MODE>(args, stream, pdl);
-  if (typical_rows <= 24) return dispatch_split<3, MODE>(args, stream, pdl);
+static int dispatch_decode(const TiledArgs& args, int rows, cudaStream_t stream, bool pdl) {
+  if (rows <= 8) return dispatch_split<1, MODE>(args, stream, pdl);
+  if (rows <= 16) return dispatch_split<2, MODE>(args, stream, pdl);
+  if (rows <= 24) return dispatch_split<3, MODE>(args, stream, pdl);
   return dispatch_split<4, MODE>(args, stream, pdl);
 }
 
-int launch_grouped_decode(const TiledArgs& args, int mode, int typical_rows, cudaStream_t stream, bool pdl) {
-  if (mode == MODE_SINGLE) return dispatch_decode<MODE_SINGLE>(args, typical_rows, stream, pdl);
-  if (mode == MODE_DUAL_SILU) return dispatch_decode<MODE_DUAL_SILU>(args, typical_rows, stream, pdl);
-  return dispatch_decode<MODE_DUAL_STORE>(args, typical_rows, stream, pdl);
+int launch_grouped_decode(const TiledArgs& args, int mode, int rows, cudaStream_t stream, bool pdl) {
+  if (mode == MODE_SINGLE) return dispatch_decode<MODE_SINGLE>(args, rows, stream, pdl);
+  if (mode == MODE_DUAL_SILU) return dispatch_decode<MODE_DUAL_SILU>(args, rows, stream, pdl);
+  return dispatch_decode<MODE_DUAL_STORE>(args, rows, stream, pdl);
 }
 
 }  // namespace tr

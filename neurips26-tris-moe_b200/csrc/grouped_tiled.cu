@@ -855,11 +855,23 @@ static int launch_wide(TiledArgs args, int max_rows, cudaStream_t stream, bool p
   return launch_and_sum<MODE>(args, stream, [&](auto mode) { return launch_grouped_wide(args, decltype(mode)::value, grid, stream, pdl); });
 }
 
+// Rows a decode pass should hold: a segment with more takes a second pass, and a launch as long as its longest segment, so it is the larger
+// ones among all segments that count, the more of them the more; a wider pass makes the others slower.  Blocks in us, passes of 8 / 16 rows: 64
+// experts, mean 3, 3.5 and 4 rows 38.5 / 41.1, 45.7 / 42.2, 47.3 / 43.4; 256 experts, 3 and 4 78.4 / 80.8, 86.9 / 82.9; 8 experts, 5 and 6 46.1 / 48.7,
+// 51.7 / 49.3.  16 / 24 rows: 64 experts, 8 and 9 46.1 / 51.1, 54.9 / 51.8; 8 experts, 12 and 13 52.8 / 56.3, 60.4 / 56.8.  24 / 32 rows: 64
+// experts, 15 and 16 59.2 / 57.7, 61.9 / 58.3 with one set of weights and 57.1 / 60.4 with another; 8 experts, 20 and 22 59.2 / 63.7, 69.1 / 66.2.
+static int decode_rows(const TiledArgs& args, int max_rows) {
+  const double mean = static_cast<double>(args.num_rows) / args.num_segments, sigma = sqrt(mean);
+  const bool few = args.num_segments <= 16, many = args.num_segments >= 64;
+  const int rows = static_cast<int>(ceil(mean + (few ? 0.85 : many ? 2.5 : 2.0) * sigma));
+  return std::max(1, std::min(max_rows, rows > 16 && many ? std::max(17, static_cast<int>(ceil(mean + 2.0 * sigma))) : rows));
+}
+
 template <int MODE>
 static int dispatch_tiled(TiledArgs& args, int max_rows, int typical_rows, cudaStream_t stream, bool pdl) {
   args.units_x = MODE == MODE_SINGLE ? (args.tiles + 1) / 2 : args.tiles;
   args.row_split = 1;
-  if (typical_rows <= kDecodeMaxRows) return launch_grouped_decode(args, MODE, typical_rows, stream, pdl);
+  if (typical_rows <= kDecodeMaxRows) return launch_grouped_decode(args, MODE, decode_rows(args, max_rows), stream, pdl);
   // A few experts of up to 128 rows: passes of 32 rows, each in CTAs of its own, while all of them fit the SMs at once (20 warps
   // each with this tile, half of them the line because their columns are split too).  One expert with 128 rows, 4096 x 256:
   // 7.4 us against 12.1 on the tiled kernel, whose units are then fewer than the SMs.  At 14 warps the line would take

@@ -107,9 +107,9 @@ constexpr size_t kMostSmem = 227 * 1024;
 inline long long decode_warps(const TiledArgs& args, int mode) {
   return static_cast<long long>((args.out_features + 31) / 32) * args.num_segments * (mode == MODE_SINGLE ? 1 : 2);
 }
-// The tile of rows follows `typical_rows`; args.row_split CTAs share the passes of a segment.  MODE_SINGLE,
+// A pass holds `rows` rows or more, 32 at most; args.row_split CTAs share the passes of a segment.  MODE_SINGLE,
 // MODE_DUAL_STORE or MODE_DUAL_SILU.
-int launch_grouped_decode(const TiledArgs& args, int mode, int typical_rows, cudaStream_t stream, bool pdl);
+int launch_grouped_decode(const TiledArgs& args, int mode, int rows, cudaStream_t stream, bool pdl);
 constexpr int kDecodeMaxRows = 32;
 // args.units_x, row_split, col_split, unit_cost and resident are set.
 int launch_grouped_wide(const TiledArgs& args, int mode, int grid, cudaStream_t stream, bool pdl);
