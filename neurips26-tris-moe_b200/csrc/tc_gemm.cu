@@ -412,6 +412,188 @@ __global__ void __launch_bounds__(kTcThreads) umma_gemm_tma_kernel(const __grid_
   tc_gemm_epilogue<NTILE>(args, pb, reinterpret_cast<float*>(base), tmem, failed, nchunks, m0, n0, n_live, cluster);
 }
 
+// ---- tiles of 128 rows x 256 outputs ----------------------------------------------------------------
+// With many rows the operands' way from L2 is what counts, and a tile of 128 outputs x 64 (128) rows asks for 24 (32) KB to do what this one
+// does with 12 (24).  The rows are the M side, a whole matrix of the usual rank the N side; one CTA to an SM, four stages of 48 KB.  A lane
+// of the accumulator is a row; the tile goes through shared memory (padded lines) to rows of 16-byte stores, or to the cluster's sums.
+constexpr int kBigRows = 128, kBigOuts = 256, kBigThreads = 256, kBigStages = 4, kBigLine = kBigOuts + 4;  // floats of a line
+struct TcBigMaps {
+  CUtensorMap a[3];
+  CUtensorMap x;
+  int32_t outs[3];  // outputs of a tile: a multiple of 16, 256 at most
+};
+struct TcBigSmem {  // at a 1024-byte boundary
+  uint8_t a[kBigStages][kBigOuts * kTcRowBytes];
+  uint8_t x[kBigStages][kBigRows * kTcRowBytes];
+  uint64_t full[kBigStages];
+  uint64_t empty[kBigStages];
+  uint64_t done;
+  uint32_t tmem_base;
+  int32_t timed_out;
+};
+static_assert(kBigRows * kBigLine * sizeof(float) <= sizeof(TcBigSmem::a) + sizeof(TcBigSmem::x), "the tile lies where the stages were");
+
+// grid (tiles of outputs over all problems, row tiles, ksplit); cluster (1, 1, ksplit)
+__global__ void __launch_bounds__(kBigThreads) umma_gemm_big_kernel(const __grid_constant__ TcGemmArgs args, const __grid_constant__ TcBigMaps maps) {
+  extern __shared__ uint4 smem_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  auto& sm = *reinterpret_cast<TcBigSmem*>(base);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  int tile = blockIdx.x, pi = 0;
+  while (pi + 1 < args.num_problems && tile >= (args.prob[pi].m + kBigOuts - 1) / kBigOuts) {
+    tile -= (args.prob[pi].m + kBigOuts - 1) / kBigOuts;
+    ++pi;
+  }
+  const SkinnyProblem& pb = args.prob[pi];
+  const int outs = maps.outs[pi], m0 = tile * kBigOuts, n0 = blockIdx.y * kBigRows;
+  const int kbeg = blockIdx.z * args.k_per_cta, kend = min(args.k, kbeg + args.k_per_cta);
+  const int nchunks = max(0, (kend - kbeg + kTcKChunk - 1) / kTcKChunk);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kBigStages; ++i) {
+      mbar_init(&sm.full[i], 1);
+      mbar_init(&sm.empty[i], 1);
+    }
+    mbar_init(&sm.done, 1);
+    fence_mbar_init();
+    sm.timed_out = 0;
+  }
+  if (warp == 0) tmem_alloc(&sm.tmem_base, kBigOuts);
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = warp_uniform(sm.tmem_base);
+  auto load_a = [&](int i) {
+    const int s = i % kBigStages;
+    mbar_arrive_expect_tx(&sm.full[s], (kBigRows + outs) * kTcRowBytes);
+    tma_load_2d(sm.a[s], &maps.a[pi], kbeg + i * kTcKChunk, m0, &sm.full[s]);
+  };
+  const int ahead = args.a_before_wait ? min(nchunks, kBigStages) : 0;
+  if (threadIdx.x == 0)
+    for (int i = 0; i < ahead; ++i) load_a(i);
+
+  pdl_wait();  // x and n_dev come from earlier kernels
+  pdl_launch_dependents();
+  const int n_live = args.n_dev ? min(args.n, *args.n_dev) : args.n;
+
+  int issued = 0;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < nchunks; ++i, ++issued) {
+      const int s = i % kBigStages;
+      if (i >= kBigStages && !mbar_wait_bounded(&sm.empty[s], ((i / kBigStages) - 1) & 1)) {
+        sm.timed_out = 1;
+        break;
+      }
+      if (i >= ahead) load_a(i);
+      tma_load_2d(sm.x[s], &maps.x, kbeg + i * kTcKChunk, n0, &sm.full[s]);
+    }
+  }
+  __syncwarp();
+  if (warp == 1) {
+    const uint32_t idesc = umma_idesc_f16(kBigRows, outs);
+    bool ok = true;
+    for (int i = 0; i < nchunks; ++i) {
+      const int s = i % kBigStages;
+      ok = mbar_wait_warp(&sm.full[s], (i / kBigStages) & 1);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint64_t dx = umma_smem_desc_sw128(smem_u32(sm.x[s])), da = umma_smem_desc_sw128(smem_u32(sm.a[s]));
+      if (elect_one()) {
+#pragma unroll
+        for (int j = 0; j < kTcKChunk / 16; ++j) umma_f16_ss(tmem, dx + 2 * j, da + 2 * j, idesc, (i > 0 || j > 0) ? 1u : 0u);
+        umma_commit(&sm.empty[s]);
+      }
+    }
+    if (elect_one()) {
+      if (!ok) sm.timed_out = 1;
+      umma_commit(&sm.done);  // arrives once every MMA issued so far has completed
+    }
+    __syncwarp();
+  }
+  if (!mbar_wait_bounded(&sm.done, 0)) sm.timed_out = 1;
+  tcgen05_fence_after();
+  __syncthreads();
+  const bool failed = sm.timed_out != 0;
+  if (failed && threadIdx.x == 0)  // copies in flight must not land in a buffer that is read as the tile
+    for (int s = 0; s < kBigStages; ++s)
+      if (last_round_parity(issued, s, kBigStages) >= 0) mbar_wait_bounded(&sm.full[s], last_round_parity(issued, s, kBigStages));
+  __syncthreads();
+
+  // accumulator -> lines of shared memory: warp w rows 32 (w % 4) .. + 31, half w / 4 of the outputs
+  float* part = reinterpret_cast<float*>(base);
+  float* line = part + (32 * (warp & 3) + lane) * kBigLine;
+  const int half = kBigOuts / 2 * (warp >> 2);
+  if (!failed && nchunks > 0) {
+    const uint32_t at = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll 1
+    for (int c0 = half; c0 < min(outs, half + kBigOuts / 2); c0 += 16) {
+      float v[16];
+      tmem_ld_16(at + c0, v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(line + c0 + 4 * j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+  } else {
+    for (int c = half; c < half + kBigOuts / 2; ++c) line[c] = 0.f;
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, kBigOuts);
+  if (failed && threadIdx.x == 0 && args.status) atomicExch(args.status, TRIS_ERR_TIMEOUT);
+  cluster.sync();
+  // every CTA of the cluster adds up and stores its own rows, a warp eight outputs a lane of one row at a time
+  const int nblk = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+  const int per = (kBigRows + nblk - 1) / nblk, r_end = min(kBigRows, (rank + 1) * per), m = m0 + 8 * lane;
+  const bool lives = 8 * lane < outs && m < pb.m;
+  const bool whole = m + 8 <= pb.m && pb.m % 8 == 0 && (reinterpret_cast<uintptr_t>(pb.out) & 15u) == 0;
+  const float* parts[8];
+#pragma unroll
+  for (int b = 0; b < 8; ++b) parts[b] = cluster.map_shared_rank(part, b < nblk ? b : 0) + 8 * lane;
+#pragma unroll 2
+  for (int r = rank * per + warp; r < r_end; r += kBigThreads / 32) {
+    const int n = n0 + r;
+    if (n >= n_live || !lives) continue;
+    float v[8] = {};
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      if (b >= nblk) break;
+      const float4 lo = *reinterpret_cast<const float4*>(parts[b] + r * kBigLine), hi = *reinterpret_cast<const float4*>(parts[b] + r * kBigLine + 4);
+      v[0] += lo.x, v[1] += lo.y, v[2] += lo.z, v[3] += lo.w, v[4] += hi.x, v[5] += hi.y, v[6] += hi.z, v[7] += hi.w;
+    }
+    const size_t at = static_cast<size_t>(n) * pb.m + m;
+    if (whole && pb.out_mode == TRIS_OUT_F32) {
+      float4* dst = reinterpret_cast<float4*>(static_cast<float*>(pb.out) + at);
+      dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+      dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else if (whole && pb.out_mode == TRIS_OUT_F16) {
+      *reinterpret_cast<uint4*>(static_cast<__half*>(pb.out) + at) =
+          make_uint4(h2_as_u32(__floats2half2_rn(v[0], v[1])), h2_as_u32(__floats2half2_rn(v[2], v[3])), h2_as_u32(__floats2half2_rn(v[4], v[5])), h2_as_u32(__floats2half2_rn(v[6], v[7])));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (m + j >= pb.m) continue;
+        if (pb.out_mode == TRIS_OUT_F32) static_cast<float*>(pb.out)[at + j] = v[j];
+        else static_cast<__half*>(pb.out)[static_cast<size_t>(n) * pb.m + out_mode_pos(m + j, pb.out_mode)] = __float2half_rn(v[j]);
+      }
+    }
+  }
+  cluster.sync();  // keep every CTA's shared memory alive until its peers have read it
+}
+
+static int launch_umma_big(const TcGemmArgs& args, const TcBigMaps& maps, int tiles, int ksplit, cudaStream_t stream, bool pdl) {
+  constexpr size_t smem = sizeof(TcBigSmem) + 1024;
+  static_assert(smem <= 227 * 1024, "shared memory");
+  static bool configured[64] = {};
+  int dev = 0;
+  TRIS_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    TRIS_CUDA(cudaFuncSetAttribute(umma_gemm_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  return check_cuda(launch_kernel(umma_gemm_big_kernel, dim3(tiles, ceil_div(args.n, kBigRows), ksplit), dim3(kBigThreads), smem, stream, pdl, ksplit, args, maps),
+                    "umma_gemm_big_kernel launch");
+}
+
 template <int NTILE>
 static int launch_umma(const TcGemmArgs& args, int mtiles, int ksplit, cudaStream_t stream, bool pdl) {
   const size_t smem = std::max(sizeof(TcSmem<NTILE>), static_cast<size_t>(NTILE) * kTcM * 4 + 128);
@@ -517,6 +699,29 @@ static int rows_per_tile(int mtiles, int n, int k, bool gathered) {
   return tiles64 <= clusters_at_once(false, column_split(tiles64, k)) ? 64 : 128;  // neither runs at once: 36 tiles, 0.9 to 1.0 of the time
 }
 
+// Split of the columns for tiles of 128 rows x 256 outputs, 0: smaller tiles are better.  A CTA fills 192 KB of stages before its first product and a
+// 133 KB tile goes through shared memory after its last one, which takes many rows to pay; in a layer's sequence half of that start runs under the
+// kernel before, which is where they are used.  us, smaller tiles / these, launch by launch: two matrices of 256 x 2048 and a router of 64, 1700 rows
+// 13.7 / 14.6, 2048 18.2 / 14.4 (halves of the columns), of 256 x 4096 and a router of 8, 1300, 1700 and 2048 rows 20.9 / 18.5, 22.6 / 19.0,
+// 30.4 / 19.2; 256 x 1024, 4072, 6144, 12000 and 16384 rows 10.3 / 11.8, 13.0 / 11.8, 16.5 / 12.2, 17.2 / 12.6; 320 x 1024, 8192, 12000 (188 tiles, two
+// turns) and 16384 rows (256) 20.2 / 12.4, 20.6 / 22.4, 32.9 / 23.0; 128 x 1024, 8192 and 12000 10.2 / 10.3, 12.8 / 10.5; 256 x 14336, 2048, 3000 and
+// 4072 rows 24.7 / 28.5, 35.0 / 33.6, 39.4 / 38.6.  Parts of fewer than 1024 columns are not worth the sum (1024 columns, 6144 rows 12.0),
+// nor are eighths (blocks whose down backbone has 1280 and 1600 rows of 14336 columns 127 / 132, 131 / 136).
+static int big_tile_split(const SkinnyProblem* probs, int num_problems, int n, int k) {
+  const int row_tiles = ceil_div(n, kBigRows);
+  int tiles = 0, outs = 0;
+  for (int i = 0; i < num_problems; ++i) {
+    tiles += ceil_div(probs[i].m, kBigOuts) * row_tiles;
+    outs += probs[i].m;
+  }
+  int ksplit = 1;
+  while (ksplit < 4 && tiles <= clusters_at_once(true, 2 * ksplit) && k / (ksplit * 2) >= 1024) ksplit *= 2;
+  const int ctas = tiles * ksplit, filled = static_cast<int>(static_cast<long long>(outs) * row_tiles * ksplit / kBigOuts);  // tiles' worth of outputs
+  if (ctas > kTcSms && ctas * 5 < ceil_div(ctas, kTcSms) * kTcSms * 4) return 0;
+  if (ksplit == 1) return filled >= 40 ? 1 : 0;
+  return ctas >= 80 && filled >= (k / ksplit >= 2048 ? 55 : 70) ? ksplit : 0;
+}
+
 int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x, const int32_t* row_gather, int n,
                    int k, cudaStream_t stream, bool pdl, const int32_t* n_dev, int32_t* status, bool a_before_wait) {
   TcGemmArgs args{};
@@ -533,6 +738,19 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
   args.n = n;
   args.k = k;
   args.a_before_wait = pdl && a_before_wait;
+  const int big = pdl && row_gather == nullptr ? big_tile_split(probs, num_problems, n, k) : 0;
+  if (big > 0) {
+    TcBigMaps maps;
+    int tiles = 0;
+    bool ok = encode_rows_map(&maps.x, x, n, k, k, kBigRows);
+    for (int i = 0; i < num_problems && ok; ++i) {
+      maps.outs[i] = std::min(kBigOuts, ceil_div(probs[i].m, 16) * 16);
+      tiles += ceil_div(probs[i].m, kBigOuts);
+      ok = encode_rows_map(&maps.a[i], probs[i].a, probs[i].m, k, k, maps.outs[i]);
+    }
+    args.k_per_cta = ceil_div(ceil_div(k, big), kTcKChunk) * kTcKChunk;
+    if (ok) return launch_umma_big(args, maps, tiles, big, stream, pdl);
+  }
   const int ntile = rows_per_tile(mtiles, n, k, row_gather != nullptr);
   const int ntiles = ceil_div(n, ntile), ksplit = column_split(mtiles * ntiles, k);
   args.k_per_cta = ceil_div(ceil_div(k, ksplit), kTcKChunk) * kTcKChunk;

@@ -544,6 +544,51 @@ def test_backbone_gemm_at_tile_edges(lib, n, k, m, tile):
         assert torch.equal(tm.compute_shared_hidden(torch.nn.functional.one_hot(col, k).half(), w), w.t()[col])
 
 
+# Tiles of 128 rows x 256 outputs, taken by launches that overlap their predecessor: ragged rows, one to several tiles of outputs (the last one
+# narrow), two to many chunks of columns in a ring of four, columns in halves and quarters, two turns of tiles.
+@pytest.mark.parametrize("n,k,ms", [(5100, 128, [256]), (6145, 192, [250]), (5200, 1024, [300]), (17000, 64, [320]), (10400, 320, [128]), (2048, 2048, [256, 256, 64]),
+                                    (1793, 4096, [256, 256, 8]), (3000, 8192, [256]), (2100, 2112, [264, 264, 250])])
+def test_backbone_gemm_in_big_tiles(lib, n, k, ms):
+    import trismoe_b200 as tm
+
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn((n, k), generator=g).half().cuda()
+    ws = [(0.05 * torch.randn((m, k), generator=g)).half().cuda() for m in ms]
+
+    def run(x):
+        if len(ws) == 1:
+            return [tm.compute_shared_hidden(x, ws[0])]
+        # two matrices and a router of one launch
+        outs = [torch.empty((n, m), dtype=torch.float16 if i < 2 else torch.float32, device="cuda") for i, m in enumerate(ms)]
+        tm._native.check(lib.tris_input_projections(x.data_ptr(), n, k, ws[0].data_ptr(), ws[1].data_ptr(), ms[0], ws[2].data_ptr(), ms[2], outs[0].data_ptr(),
+                                                    outs[1].data_ptr(), 0, outs[2].data_ptr(), torch.cuda.current_stream().cuda_stream))
+        return outs
+
+    previous = lib.tris_set_programmatic_launch(1)
+    try:
+        outs = run(x)
+        names = [name for name, _ in kernels_of(lambda: run(x))]
+        hots = []
+        for c in range(0, k, n):
+            col = (torch.arange(n, device="cuda") + c) % k
+            hots.append((col, run(torch.nn.functional.one_hot(col, k).half())))
+        if ms[0] % 32 == 0 and len(ws) == 1:
+            plain, permuted = outs[0], tm.compute_shared_hidden(x, ws[0], layout=2)
+    finally:
+        lib.tris_set_programmatic_launch(previous)
+    assert any("umma_gemm_big_kernel" in name for name in names), names
+    for got, w in zip(outs, ws):
+        ref, acc, bound = _bound(w, x)
+        _assert_within(got, ref, bound if got.dtype == torch.float16 else acc + 2.0 ** -25)
+    for col, outs in hots:
+        for got, w in zip(outs, ws):
+            assert torch.equal(got, w.t()[col].to(got.dtype))
+    if ms[0] % 32 == 0 and len(ws) == 1:
+        at = torch.arange(ms[0])
+        place = (at & ~31) | ((at & 15) << 1) | ((at >> 4) & 1)
+        assert torch.equal(permuted[:, place.cuda()], plain)
+
+
 @pytest.mark.parametrize("n,k,m", [(2480, 8192, 256), (1880, 8192, 250), (4000, 8192, 128), (1200, 8192, 128)])
 def test_backbone_gemm_of_gathered_long_rows(lib, n, k, m):
     import trismoe_b200 as tm
