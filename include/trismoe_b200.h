@@ -485,6 +485,14 @@ int tris_combine_routed(const void* down_out_f16, const int32_t* row_of_flat,
  * tests lower it to exercise the tensor-core kernel.  Process-wide; no reference counterpart
  * (the reference decides per call in run_grouped_structured_expert_forward, QL:2187-2229).
  */
+/*
+ * The three projections of an attention block on the same rows x [num_rows, in], each an ordinary matrix with tile records: q, and
+ * k with v (one launch where their shapes agree), as tris_linear_forward computes them.  k and v do not wait for q's
+ * results: their launches start as q's ends.  workspace: as many bytes as tris_linear_workspace_bytes names for (q, 1) or (k, 2), or NULL.
+ */
+int tris_qkv_forward(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, const void* x_f16, int32_t num_rows,
+                     void* q_out_f16, void* k_out_f16, void* v_out_f16, void* workspace, size_t workspace_bytes, void* stream);
+
 int tris_set_grouped_tc_min_rows(int32_t rows);
 
 /*

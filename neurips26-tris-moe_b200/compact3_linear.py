@@ -13,6 +13,7 @@ matrix ``[out_features, in_features]`` (the columns are the layer's input featur
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional
 
 import torch
@@ -22,6 +23,7 @@ from . import _native, envflags
 from .formats import stack_expert_payloads
 from .qlinear_grouped import (
     prepare_grouped_payload,
+    proj_view,
     run_grouped_structured_expert_forward,
     run_grouped_structured_expert_pair_forward,
 )
@@ -79,7 +81,8 @@ def run_compact3_qkv_forward(q_proj: Compact3Linear, k_proj: Compact3Linear, v_p
     """``(q, k, v)`` of one attention block (``run_compact3_qkv_block_gr_forward``,
     qlinear_cuda.py:915-1022).  k and v share the activation staging of one launch when they
     have the same shape (the gate/up dual kernel, two projections per CTA); q runs in its own
-    launch (with grouped-query attention its width differs from k/v's)."""
+    launch (with grouped-query attention its width differs from k/v's).  Where all three have tile
+    records that is one native call whose launches overlap (``tris_qkv_forward``)."""
     _native.require_cuda(hidden_states, "run_compact3_qkv_forward")
     if any(m.input_scale is not None for m in (q_proj, k_proj, v_proj)):
         return envflags.return_or_raise_none("run_compact3_qkv_forward", "input scales are not supported by the fused form")
@@ -88,6 +91,21 @@ def run_compact3_qkv_forward(q_proj: Compact3Linear, k_proj: Compact3Linear, v_p
     x2 = hidden_states.reshape(-1, q_proj.in_features).contiguous()
     rows = int(x2.shape[0])
     lead = hidden_states.shape[:-1]
+    mods, dev = (q_proj, k_proj, v_proj), x2.device
+    if all(m.payload.get("_tris_tile_records") is not None and m.in_features == q_proj.in_features
+           and getattr(m.payload.get("qweight1"), "device", None) == dev for m in mods):
+        lib = _native.load()
+        views = [proj_view(m.payload) for m in mods]
+        # the leading dimensions at once; no reshape afterwards
+        outs = [torch.empty(lead + (m.out_features,), dtype=torch.float16, device=dev) for m in mods]
+        if rows:
+            pair = 2 if _same_shape(k_proj, v_proj) else 1
+            need = 0 if rows <= 32 else max(int(lib.tris_linear_workspace_bytes(C.byref(v), n, rows)) for v, n in zip(views, (1, pair, pair)))
+            with _native.on_device(dev):
+                ws = torch.empty((need,), dtype=torch.uint8, device=dev) if need else None
+                _native.check(lib.tris_qkv_forward(*(C.byref(v) for v in views), x2.data_ptr(), rows, *(o.data_ptr() for o in outs),
+                                                   None if ws is None else ws.data_ptr(), need, _native.stream_of(dev)), "qkv_forward")
+        return tuple(outs)
     q = run_grouped_structured_expert_forward(q_proj.payload, x2, None, q_proj._route(rows, x2.device))
     if _same_shape(k_proj, v_proj):
         k, v = run_grouped_structured_expert_pair_forward(k_proj.payload, v_proj.payload, x2, x2, None,

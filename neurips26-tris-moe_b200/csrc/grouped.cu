@@ -699,3 +699,31 @@ extern "C" int tris_linear_forward(const TrisProjView* proj_a, const TrisProjVie
   if (proj_b == nullptr) return grouped_forward_impl(proj_a, route, hidden_a_f16, out_a_f16, s, opts);
   return grouped_pair_forward_impl(proj_a, proj_b, route, hidden_a_f16, hidden_b_f16, out_a_f16, out_b_f16, fuse_silu_mul, s, opts);
 }
+
+extern "C" int tris_qkv_forward(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, const void* x_f16, int32_t num_rows,
+                                void* q_out_f16, void* k_out_f16, void* v_out_f16, void* workspace, size_t workspace_bytes, void* stream) {
+  TRIS_REQUIRE(q && k && v && x_f16 && q_out_f16 && k_out_f16 && v_out_f16, TRIS_ERR_INVALID_ARG, "tris_qkv_forward: null pointer");
+  TRIS_REQUIRE(num_rows >= 0 && q->rank == k->rank && q->rank == v->rank && q->num_experts == 1 && k->num_experts == 1 && v->num_experts == 1,
+               TRIS_ERR_INVALID_ARG, "tris_qkv_forward: the projections do not read the same rows");
+  TRIS_REQUIRE(proj_has_tile_records(*q) && proj_has_tile_records(*k) && proj_has_tile_records(*v), TRIS_ERR_UNSUPPORTED,
+               "tris_qkv_forward: the projections need tile records");
+  TRIS_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15u) == 0, TRIS_ERR_INVALID_ARG, "tris_qkv_forward: the workspace must be 16-byte aligned");
+  if (num_rows == 0) return TRIS_OK;
+  TrisRouteView rows{};
+  rows.num_segments = 1;
+  rows.num_rows = rows.max_rows_per_segment = num_rows;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  LaunchOpts opts;
+  opts.pdl = programmatic_launch_default();
+  opts.workspace = workspace;
+  opts.workspace_bytes = workspace ? workspace_bytes : 0;
+  int st = grouped_forward_impl(q, &rows, x_f16, q_out_f16, s, opts);
+  if (st != TRIS_OK) return st;
+  // Every CTA of q's launch waits before it lets the next one start, so the rows are final for k and v.  Their stores, the sums of column
+  // parts in the scratch that q used too among them, come after their wait.
+  opts.pdl = opts.weights_before_wait = opts.rows_ready = true;
+  if (k->out_features == v->out_features)
+    return grouped_pair_forward_impl(k, v, &rows, x_f16, x_f16, k_out_f16, v_out_f16, 0, s, opts);
+  st = grouped_forward_impl(k, &rows, x_f16, k_out_f16, s, opts);
+  return st == TRIS_OK ? grouped_forward_impl(v, &rows, x_f16, v_out_f16, s, opts) : st;
+}

@@ -91,6 +91,29 @@ def test_fused_qkv_and_dual_gate_up(lib):
     _check(b, u32)
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 32, 33, 63, 64, 65, 129, 200])
+@pytest.mark.parametrize("widths,K", [((512, 128, 128), 512), ((256, 256, 256), 1024), ((192, 128, 64), 2048)])
+def test_qkv_in_one_call(lib, widths, K, rows):
+    """The launches of k and v start while q's ends: passes of 8 to 32 rows, row tiles and parts of the columns, k and v in one launch
+    and in two, against the fp32 product; then calls back to back on new rows in the same memory, which must give what each linear alone gives."""
+    import trismoe_b200 as tm
+
+    rng = np.random.default_rng(K + rows)
+    made = [_single(rng, o, K) for o in widths]
+    mods = [tm.Compact3Linear(p, device="cuda") for p, _ in made]
+    xs = [torch.from_numpy(rng.standard_normal((1, rows, K)).astype(np.float16)).cuda() for _ in range(4)]
+    for y, (_, w) in zip(tm.run_compact3_qkv_forward(*mods, xs[0]), made):
+        assert y.shape == (1, rows, w.shape[0])
+        _check(y.view(rows, -1), xs[0].view(rows, K).float().cpu().numpy() @ w.astype(np.float32).T)
+    want = [[m(x).float() for m in mods] for x in xs]
+    got = [[y.float() for y in tm.run_compact3_qkv_forward(*mods, xs[i % 4].clone())] for i in range(12)]
+    for i, ys in enumerate(got):
+        for y, ref in zip(ys, want[i % 4]):
+            # fp32 sums of the same products in another order, each rounded to fp16 once: one unit in the last place at most, and where
+            # the terms cancel K roundings of 2^-24 of the sum of their sizes, which the largest output bounds to a few
+            assert (y - ref).abs().max() <= 2.0**-10 * ref.abs().max()
+
+
 def test_qwen2_block_with_shared_expert(lib):
     """Qwen2-MoE style block: routed experts + an always-on shared expert (compact3 gate/up/down) scaled
     by sigmoid(shared_expert_gate(x)), against the fp32 oracle."""
