@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kBigThreads) umma_gemm_big_kernel(const __grid
     ++pi;
   }
   const SkinnyProblem& pb = args.prob[pi];
-  const int outs = maps.outs[pi], m0 = tile * kBigOuts, n0 = blockIdx.y * kBigRows;
+  const int outs = maps.outs[pi], m0 = tile * outs, n0 = blockIdx.y * kBigRows;
   const int kbeg = blockIdx.z * args.k_per_cta, kend = min(args.k, kbeg + args.k_per_cta);
   const int nchunks = max(0, (kend - kbeg + kTcKChunk - 1) / kTcKChunk);
 
@@ -703,23 +703,30 @@ static int rows_per_tile(int mtiles, int n, int k, bool gathered) {
 // 133 KB tile goes through shared memory after its last one, which takes many rows to pay; in a layer's sequence half of that start runs under the
 // kernel before, which is where they are used.  us, smaller tiles / these, launch by launch: two matrices of 256 x 2048 and a router of 64, 1700 rows
 // 13.7 / 14.6, 2048 18.2 / 14.4 (halves of the columns), of 256 x 4096 and a router of 8, 1300, 1700 and 2048 rows 20.9 / 18.5, 22.6 / 19.0,
-// 30.4 / 19.2; 256 x 1024, 4072, 6144, 12000 and 16384 rows 10.3 / 11.8, 13.0 / 11.8, 16.5 / 12.2, 17.2 / 12.6; 320 x 1024, 8192, 12000 (188 tiles, two
-// turns) and 16384 rows (256) 20.2 / 12.4, 20.6 / 22.4, 32.9 / 23.0; 128 x 1024, 8192 and 12000 10.2 / 10.3, 12.8 / 10.5; 256 x 14336, 2048, 3000 and
-// 4072 rows 24.7 / 28.5, 35.0 / 33.6, 39.4 / 38.6.  Parts of fewer than 1024 columns are not worth the sum (1024 columns, 6144 rows 12.0),
-// nor are eighths (blocks whose down backbone has 1280 and 1600 rows of 14336 columns 127 / 132, 131 / 136).
+// 30.4 / 19.2; 256 x 1024, 4072, 6144, 12000 and 16384 rows 10.3 / 11.8, 13.0 / 11.8, 16.5 / 12.2, 17.2 / 12.6; 320 x 1024 in tiles of 160 outputs,
+// 3600, 4072, 8192 and 16384 rows 13.4 / 13.6, 13.5 / 9.8, 19.2 / 10.1, 33.2 / 19.5 (in tiles of 256 and 64 8192 rows 12.4, 16384 23.0); 128 x 1024,
+// 8192 and 12000 10.2 / 10.3, 12.8 / 10.5; 256 x 14336, 2048, 3000 and 4072 rows 24.7 / 28.5, 35.0 / 33.6, 39.4 / 38.6.  Parts of fewer than
+// 1024 columns are not worth the sum (1024 columns, 6144 rows 12.0), nor are eighths (blocks whose down backbone has 1280 and 1600 rows of 14336
+// columns 127 / 132, 131 / 136).  Where the lines for split columns lie: 320 x 14336, 2758 rows (55) 36.5 / 43.6, 3600 rows 58.3 / 45.7; blocks with
+// it, 1340, 1400 and 1460 tokens (gate and up in these tiles in all three; 52, 55 and 57 of down's) 1.015, 1.005 and 1.04; blocks with
+// 128 x 14336, 1862, 1906 and 1950 tokens (58, 60, 62) 0.98, 0.99, 1.02.  Quarters of 1024 columns: two matrices of 256 x 4096, 1100 rows
+// (73) 0.99 of a block, 1379 (89) 1.02.
 static int big_tile_split(const SkinnyProblem* probs, int num_problems, int n, int k) {
   const int row_tiles = ceil_div(n, kBigRows);
-  int tiles = 0, outs = 0;
+  int tiles = 0, outs = 0, widest = 0;
   for (int i = 0; i < num_problems; ++i) {
     tiles += ceil_div(probs[i].m, kBigOuts) * row_tiles;
     outs += probs[i].m;
+    widest = std::max(widest, probs[i].m);
   }
   int ksplit = 1;
   while (ksplit < 4 && tiles <= clusters_at_once(true, 2 * ksplit) && k / (ksplit * 2) >= 1024) ksplit *= 2;
   const int ctas = tiles * ksplit, filled = static_cast<int>(static_cast<long long>(outs) * row_tiles * ksplit / kBigOuts);  // tiles' worth of outputs
   if (ctas > kTcSms && ctas * 5 < ceil_div(ctas, kTcSms) * kTcSms * 4) return 0;
   if (ksplit == 1) return filled >= 40 ? 1 : 0;
-  return ctas >= 80 && filled >= (k / ksplit >= 2048 ? 55 : 70) ? ksplit : 0;
+  const int part = k / ksplit;
+  const int least = part >= 3072 ? (widest <= 128 ? 62 : 57) : part >= 2048 ? 55 : (ksplit == 4 ? 85 : 70);
+  return ctas >= 80 && filled >= least ? ksplit : 0;
 }
 
 int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x, const int32_t* row_gather, int n,
@@ -744,8 +751,9 @@ int launch_tc_gemm(const SkinnyProblem* probs, int num_problems, const __half* x
     int tiles = 0;
     bool ok = encode_rows_map(&maps.x, x, n, k, k, kBigRows);
     for (int i = 0; i < num_problems && ok; ++i) {
-      maps.outs[i] = std::min(kBigOuts, ceil_div(probs[i].m, 16) * 16);
-      tiles += ceil_div(probs[i].m, kBigOuts);
+      const int parts = ceil_div(probs[i].m, kBigOuts);
+      maps.outs[i] = ceil_div(ceil_div(probs[i].m, parts), 16) * 16;  // equal tiles: 320 outputs are two of 160
+      tiles += parts;
       ok = encode_rows_map(&maps.a[i], probs[i].a, probs[i].m, k, k, maps.outs[i]);
     }
     args.k_per_cta = ceil_div(ceil_div(k, big), kTcKChunk) * kTcKChunk;
