@@ -427,8 +427,8 @@ template <int NT, int MODE>
 static int dispatch_split(const TiledArgs& args, cudaStream_t stream, bool pdl) {
   // Fewer than 13 warps per SM: split the columns, as far as there are columns to split.  Of the wider tiles 20 warps fit an SM instead of 28:
   // fewer than 10 (1024 warps of 8 experts x 4096 x 256 in halves and not in quarters: blocks of 24, 40, 64 and 80 tokens 50.4 / 49.3, 59.5 / 56.1,
-  // 61.4 / 58.1, 68.0 / 63.7 us).
-  const long long warps = decode_warps(args, MODE) * args.row_split, split = (NT >= 3 ? 10 : 13) * sm_count();
+  // 61.4 / 58.1, 68.0 / 63.7 us).  With more than 256 columns, 14: 32 segments of 64 experts x 320 34.2 / 35.4 us.
+  const long long warps = decode_warps(args, MODE) * args.row_split, split = (args.rank > 256 ? 14 : NT >= 3 ? 10 : 13) * sm_count();
   const int slices = ceil_div(args.rank, kSliceCols), groups = ceil_div(args.rank, kDecCols), want = (args.row_split > 1 ? 10 : 14) * sm_count();
   // Many columns: over the CTAs of a cluster too, by 256 columns or more each, up to 14 warps per SM (10 with shared passes).  us at 8 rows, eight warps to
   // 32 outputs in one CTA / this: 4096 x 4096 18.6 / 11.2, pair of 1024 x 4096 25.8 / 8.4, pair of 2048 x 2048 14.4 / 8.1, 512 x 1024 6.2 /

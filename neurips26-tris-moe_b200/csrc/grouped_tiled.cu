@@ -860,11 +860,16 @@ static int launch_wide(TiledArgs args, int max_rows, cudaStream_t stream, bool p
 // experts, mean 3, 3.5 and 4 rows 38.5 / 41.1, 45.7 / 42.2, 47.3 / 43.4; 256 experts, 3 and 4 78.4 / 80.8, 86.9 / 82.9; 8 experts, 5 and 6 46.1 / 48.7,
 // 51.7 / 49.3.  16 / 24 rows: 64 experts, 8 and 9 46.1 / 51.1, 54.9 / 51.8; 8 experts, 12 and 13 52.8 / 56.3, 60.4 / 56.8.  24 / 32 rows: 64
 // experts, 15 and 16 59.2 / 57.7, 61.9 / 58.3 with one set of weights and 57.1 / 60.4 with another; 8 experts, 20 and 22 59.2 / 63.7, 69.1 / 66.2.
+// Of other widths than two chunks of columns the wider pass costs more: 256 experts x 320 columns, 3.5 and 3.8 rows, 8 / 16 112.3 / 119.1,
+// 109.4 / 116.0; 64 experts x 320, 3.5, 4 and 9 rows 57.0 / 60.9, 54.2 / 61.0, 70.5 / 73.0; 64 x 128, 9 rows, 16 / 24 39.4 / 41.6; 8 x 128,
+// 20 rows, 24 / 32 56.4 / 54.7.
 static int decode_rows(const TiledArgs& args, int max_rows) {
   const double mean = static_cast<double>(args.num_rows) / args.num_segments, sigma = sqrt(mean);
-  const bool few = args.num_segments <= 16, many = args.num_segments >= 64;
-  const int rows = static_cast<int>(ceil(mean + (few ? 0.85 : many ? 2.5 : 2.0) * sigma));
-  return std::max(1, std::min(max_rows, rows > 16 && many ? std::max(17, static_cast<int>(ceil(mean + 2.0 * sigma))) : rows));
+  const bool few = args.num_segments <= 16, many = args.num_segments >= 64 && args.chunks <= 2;
+  const int plain = static_cast<int>(ceil(mean + 2.0 * sigma));
+  int rows = few ? static_cast<int>(ceil(mean + (args.chunks == 1 ? 1.0 : 0.85) * sigma)) : many ? static_cast<int>(ceil(mean + 2.5 * sigma)) : plain;
+  if (many && rows > 16) rows = args.chunks == 2 ? std::max(17, plain) : plain;
+  return std::max(1, std::min(max_rows, rows));
 }
 
 template <int MODE>
