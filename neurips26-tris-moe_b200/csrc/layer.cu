@@ -5,8 +5,8 @@
 //   down backbone on the routed rows
 //   grouped down
 //   weighted combine back to token order
-// Input scales and null-space pairs (TrisMoeLayerExtras) join the same sequence: three 4-bit launches and,
-// where gate or up has a pair, SiLU*mul in the epilogue of the second one.
+// Input scales and null-space pairs (TrisMoeLayerExtras) join the same sequence: each matrix C2 in the wake of the grouped launch whose
+// outputs its pair corrects, each C1 after it; of gate and up in one launch each, SiLU*mul in the epilogue of the second.
 // A shared expert's (TrisSharedExpert) gate/up launch follows the route and its down launch the down backbone.  Both read rows that are older
 // than the kernel before them and, at a few rows, wait only before they store: they run beside the route's one CTA and the down
 // backbone's few.  256 experts of 512, 16 tokens, a call of the whole layer: 121 us with the two linears and the sum as operators of their
@@ -163,7 +163,9 @@ static int launch_packed(const TrisPacked4View* const* w, int count, const __hal
     if (st != TRIS_OK) return st;
     p[i] = {*w[i], x, i ? out1 : out0, cols, w[i]->n, 0};
   }
-  return packed4_gemm_impl(p, count, nullptr, rows, out_mode, false, false, s, /*pdl=*/true);
+  // Overlapped where the columns are few: with 4096 and 14336 columns and 8 experts a block of 1 and 32 tokens took 74.5 and 120.6 us so, and
+  // 52.7 and 113.9 with launches that wait for the one before.
+  return packed4_gemm_impl(p, count, nullptr, rows, out_mode, false, false, s, /*pdl=*/cols <= 2048);
 }
 }  // namespace tris
 
