@@ -18,7 +18,10 @@ one kernel per chunk.  Here the copy is itself a kernel (``tris_page_experts``) 
 pinned buffers through their device mapping and is driven by the device-side route: it is
 enqueued on a side stream right after the route kernel, copies exactly the active experts'
 blocks into staging slot ``s`` = segment index, and writes the expert -> slot table the
-grouped kernels index with.  Nothing is read back to the host.  Ordering is by events:
+grouped kernels index with.  Nothing is read back to the host.  Payloads without output scales
+and biases are then built into tile records from the slots (``tris_moe_layer_forward_paged``: route,
+pagers, builders and the rest of the layer in one native call), which the kernels of resident layers
+read; the others are computed from the slots' planes.  Ordering is by events:
 compute waits on "paged", the pager of the next use of a slot waits on "consumed".
 
 Statistics: ``pipeline_stats`` counts calls and bytes as the reference's does (exact bytes
