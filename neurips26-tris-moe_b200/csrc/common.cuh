@@ -123,6 +123,8 @@ int grouped_forward_impl(const TrisProjView* proj, const TrisRouteView* route, c
 int grouped_pair_forward_impl(const TrisProjView* proj_a, const TrisProjView* proj_b, const TrisRouteView* route,
                               const void* hidden_a_f16, const void* hidden_b_f16, void* out_a_f16, void* out_b_f16,
                               int fuse_silu_mul, cudaStream_t stream, LaunchOpts opts);
+int validate_grouped_view(const TrisProjView* v, const char* name);        // what every grouped launch asks of a view
+int validate_pair(const TrisProjView& a, const TrisProjView& b);           // and of two that share a launch
 // Tile-record path (grouped_tiled.cu).  mode: 0 single projection, 1 gate/up pair, 2 pair with SiLU * mul.
 bool proj_has_tile_records(const TrisProjView& v);
 int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b, const TrisRouteView* route,

@@ -622,6 +622,15 @@ extern "C" int tris_grouped_forward(const TrisProjView* proj, const TrisRouteVie
   return grouped_forward_impl(proj, route, hidden_f16, out_f16, static_cast<cudaStream_t>(stream), opts);
 }
 
+int tris::validate_grouped_view(const TrisProjView* v, const char* name) { return validate_proj(v, name, true); }
+int tris::validate_pair(const TrisProjView& a, const TrisProjView& b) {
+  TRIS_REQUIRE(a.num_experts == b.num_experts && a.out_features == b.out_features && a.rank == b.rank && a.num_groups == b.num_groups,
+               TRIS_ERR_UNSUPPORTED, "tris_grouped_pair_forward: the two projections must share E, O, r and G");
+  TRIS_REQUIRE((a.use_block_gr != 0) == (b.use_block_gr != 0) && (!a.use_block_gr || a.gr_substreams == b.gr_substreams),
+               TRIS_ERR_UNSUPPORTED, "tris_grouped_pair_forward: the two projections must share the g_map format");
+  return TRIS_OK;
+}
+
 int tris::grouped_pair_forward_impl(const TrisProjView* proj_a, const TrisProjView* proj_b,
                                     const TrisRouteView* route, const void* hidden_a_f16, const void* hidden_b_f16,
                                     void* out_a_f16, void* out_b_f16, int fuse_silu_mul, cudaStream_t stream,
@@ -630,12 +639,8 @@ int tris::grouped_pair_forward_impl(const TrisProjView* proj_a, const TrisProjVi
   if (st != TRIS_OK) return st;
   st = validate_proj(proj_b, "tris_grouped_pair_forward(b)", true);
   if (st != TRIS_OK) return st;
-  TRIS_REQUIRE(proj_a->num_experts == proj_b->num_experts && proj_a->out_features == proj_b->out_features &&
-                   proj_a->rank == proj_b->rank && proj_a->num_groups == proj_b->num_groups,
-               TRIS_ERR_UNSUPPORTED, "tris_grouped_pair_forward: the two projections must share E, O, r and G");
-  TRIS_REQUIRE((proj_a->use_block_gr != 0) == (proj_b->use_block_gr != 0) &&
-                   (!proj_a->use_block_gr || proj_a->gr_substreams == proj_b->gr_substreams),
-               TRIS_ERR_UNSUPPORTED, "tris_grouped_pair_forward: the two projections must share the g_map format");
+  st = validate_pair(*proj_a, *proj_b);
+  if (st != TRIS_OK) return st;
   TRIS_REQUIRE(hidden_a_f16 && hidden_b_f16 && out_a_f16 && (fuse_silu_mul || out_b_f16), TRIS_ERR_INVALID_ARG,
                "tris_grouped_pair_forward: null hidden/out");
   GroupedArgs a{};

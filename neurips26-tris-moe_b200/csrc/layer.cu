@@ -154,6 +154,22 @@ static int validate_shared(const TrisMoeLayerView* L, const TrisSharedExpert* S)
   return TRIS_OK;
 }
 
+// The staged projections of a streamed layer: what the grouped entry points ask of them, here before anything is launched, since the record
+// kernels are launched without those entry points.
+static int validate_paged(const TrisMoeLayerView* L, const TrisPagedLayer* P) {
+  const TrisProjView* own[3] = {&L->gate, &L->up, &L->down};
+  for (int i = 0; i < 3; ++i) {
+    const int st = validate_grouped_view(P->staged + i, "tris_moe_layer_forward_paged");
+    if (st != TRIS_OK) return st;
+  }
+  const int st = validate_pair(P->staged[0], P->staged[1]);
+  if (st != TRIS_OK) return st;
+  for (int i = 0; i < 3; ++i)
+    TRIS_REQUIRE(P->staged[i].num_experts == own[i]->num_experts && P->staged[i].out_features == own[i]->out_features && P->staged[i].rank == own[i]->rank,
+                 TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: staged projection %d is not the layer's", i);
+  return TRIS_OK;
+}
+
 // One or two 4-bit backbones on the same dense rows.
 static int launch_packed(const TrisPacked4View* const* w, int count, const __half* x, int rows, int cols, __half* out0, __half* out1,
                          int out_mode, cudaStream_t s) {
@@ -436,6 +452,8 @@ extern "C" int tris_moe_layer_forward_paged(const TrisMoeLayerView* layer, const
   const bool records = paged->records[0].tile_records != nullptr;
   TRIS_REQUIRE(!records || paged->slot_ids, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: records need slot_ids");
   if (num_tokens == 0) return TRIS_OK;
+  st = validate_paged(layer, paged);
+  if (st != TRIS_OK) return st;
   const int T = num_tokens, E = layer->num_experts, R = T * layer->top_k;
   LayerWorkspace w = carve(layer, T, static_cast<char*>(workspace));
   TRIS_REQUIRE(workspace != nullptr && workspace_bytes >= w.bytes, TRIS_ERR_WORKSPACE, "tris_moe_layer_forward_paged: workspace %zu < %zu bytes",
