@@ -71,9 +71,10 @@ struct BuildArgs {
 };
 
 // Column record of a chunk by a warp; cw, grp: the salient columns and the groups of its packed rows, cp: scales of its first column.  Salient
-// columns take places in order, and a new group starts at a multiple of 16 of them (as plan_chunk deals them).
-__device__ __forceinline__ void build_col_record(const TrisProjView& v, int p0, int rows, const uint32_t (&cw)[kChunkRows], const int (&grp)[kChunkRows],
-                                                 const unsigned long long* cp, int max_steps, int lane, uint16_t* col_of, uint8_t* rec) {
+// columns take places in order, and a new group starts at a multiple of 16 of them (as plan_chunk deals them).  Steps and slots that the plan
+// did not count are left out, so that the record's readers stay inside it.  Returns whether there were any.
+__device__ __forceinline__ bool build_col_record(const TrisProjView& v, int p0, int rows, const uint32_t (&cw)[kChunkRows], const int (&grp)[kChunkRows],
+                                                 const unsigned long long* cp, int max_steps, int max_slots, int lane, uint16_t* col_of, uint8_t* rec) {
   ColHeader h = {};
   h.magic = kColMagic;
   for (int i = lane; i < kMaxSteps * 16; i += 32) col_of[i] = 0xFFFFu;
@@ -85,17 +86,18 @@ __device__ __forceinline__ void build_col_record(const TrisProjView& v, int p0, 
       ++slots;
       at = (at + 15) & ~15;
     }
-    h.slot_of_row[p] = static_cast<uint8_t>(slots - 1);
+    h.slot_of_row[p] = static_cast<uint8_t>(min(slots, max_slots) - 1);
     const int n = __popc(cw[p]), end = at + n;
     if ((cw[p] >> lane) & 1u) col_of[at + __popc(cw[p] & ((1u << lane) - 1u))] = static_cast<uint16_t>(32 * p + lane);
 #pragma unroll
     for (int s = 0; s < kMaxSteps; ++s)
-      if (n > 0 && 16 * s < end && 16 * s + 16 > at) h.step_slot[s] = static_cast<uint8_t>(slots - 1);
+      if (n > 0 && 16 * s < end && 16 * s + 16 > at) h.step_slot[s] = static_cast<uint8_t>(min(slots, max_slots) - 1);
     at = end;
     salient += n;
   }
-  h.num_slots = static_cast<uint8_t>(slots);
-  h.num_steps = static_cast<uint8_t>((at + 15) >> 4);
+  const int steps = (at + 15) >> 4;
+  h.num_slots = static_cast<uint8_t>(min(slots, max_slots));
+  h.num_steps = static_cast<uint8_t>(min(steps, max_steps));
   h.num_salient = static_cast<uint16_t>(salient);
   if (lane == 0) *reinterpret_cast<ColHeader*>(rec) = h;
   __syncwarp();
@@ -131,6 +133,7 @@ __device__ __forceinline__ void build_col_record(const TrisProjView& v, int p0, 
     }
     reinterpret_cast<uint2*>(ent)[pair] = c;
   }
+  return steps > max_steps || slots > max_slots;
 }
 
 // Bytes 3, 2 of the result: bits 0, 2 .. 14 and 1, 3 .. 15 of v, the first one on top; bytes 1, 0: those of the upper half.
@@ -215,8 +218,9 @@ __global__ void __launch_bounds__(32 * kBuildWarps, 7) build_tile_records_kernel
   if (columns) {
     const uint32_t cw[kChunkRows] = {salient[0], salient[1], salient[2], salient[3]};
     const int gr[kChunkRows] = {grp[0], grp[1], grp[2], grp[3]};
-    build_col_record(v, p0, min(kChunkRows, rows), cw, gr, reinterpret_cast<const unsigned long long*>(v.col_pack3) + static_cast<size_t>(at) * v.rank + 32 * p0,
-                     max_steps, lane, col_of[warp], args.cols[blockIdx.z] + static_cast<size_t>(place * d.chunks + c0) * col_record_bytes(max_steps));
+    const bool more = build_col_record(v, p0, min(kChunkRows, rows), cw, gr, reinterpret_cast<const unsigned long long*>(v.col_pack3) + static_cast<size_t>(at) * v.rank + 32 * p0,
+                                       max_steps, max_slots, lane, col_of[warp], args.cols[blockIdx.z] + static_cast<size_t>(place * d.chunks + c0) * col_record_bytes(max_steps));
+    if (more && lane == 0 && args.status) *args.status = TRIS_ERR_CORRUPT;  // the payload is not the one that was planned
     return;
   }
 
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps, 7) build_tile_records_kernel
       const int ahead = begin2 - first2;
       uint32_t w2 = run2[c] >> (ahead & 31);
       if (ahead > 16 && live && second && begin2 >= 0) w2 = stream_bits(signs2, v.sign2_rows, O, begin2);
-      step_at[(steps - 1) * kSubOut] = code_words(w1, ~(w2 & ((1u << fill) - 1u))).x;  // both bits as "negative"
+      if (steps <= max_steps) step_at[(steps - 1) * kSubOut] = code_words(w1, ~(w2 & ((1u << fill) - 1u))).x;  // both bits as "negative"
       w1 = 0u;
     };
 #pragma unroll
@@ -331,7 +335,8 @@ __global__ void __launch_bounds__(32 * kBuildWarps, 7) build_tile_records_kernel
       if (opens(p)) {
         if (fill < 16) close();
         fill = 16;
-        slot_at[slots++ * kSubOut] = make_uint2(static_cast<uint32_t>(scales[p]), static_cast<uint32_t>(scales[p] >> 32));
+        if (slots < max_slots) slot_at[slots * kSubOut] = make_uint2(static_cast<uint32_t>(scales[p]), static_cast<uint32_t>(scales[p] >> 32));
+        ++slots;
       }
       int at2 = rank2[p];
 #pragma unroll 1

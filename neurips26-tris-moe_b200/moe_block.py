@@ -296,7 +296,8 @@ class TrisSparseMoeBlock(nn.Module):
         if status != 0:
             raise RuntimeError(f"trismoe_b200: a grouped kernel reported {_native.STATUS_NAMES.get(status, status)} "
                                "(TRIS_ERR_TIMEOUT: a bounded wait on a copy ran out; TRIS_ERR_WORKSPACE: a streamed batch activated "
-                               "more experts than the staging manager has slots for; output rows of that launch are stale)")
+                               "more experts than the staging manager has slots for; TRIS_ERR_CORRUPT: a streamed payload's column maps were changed "
+                               "after its records were planned; output rows of that launch are stale)")
 
     def _require_rows(self, x: torch.Tensor, what: str) -> None:
         """The kernels take addresses: rows of another type or width would be misread or read out of range."""

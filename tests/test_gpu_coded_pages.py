@@ -1,6 +1,7 @@
 """Coded pages: every bit of a bitmap comes back, at block edges, at all densities and without code where that is larger."""
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
 
@@ -182,3 +183,53 @@ def test_layers_with_output_scales_are_streamed_as_planes(lib):
         x = synth.synth_activations(7, 256, seed=1).cuda().view(1, 7, 256)
         outs.append(blk.forward_streaming(x, manager, 0, router_logits=synth.synth_router_logits(7, 8, seed=2).cuda())[0].float())
     assert (outs[1] - 2 * outs[0]).abs().max() <= 2e-2 * outs[0].abs().max()
+
+
+@pytest.mark.parametrize("rank,group", [(96, 32), (256, 128), (300, 64)])
+def test_records_stay_inside_their_plan(lib, rank, group):
+    """Built for one salient step and one row-scale slot fewer than the payload has: what is beyond that is left out, and nothing behind the
+    buffers is written."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+    from trismoe_b200.qlinear_grouped import proj_view
+
+    rng = np.random.default_rng(rank)
+    raws = synth.raw_projection(rng, 3, 200, rank, group_size=group, p_salient=0.5)
+    payload = tm.prepare_grouped_payload(synth.pack_projection(raws, "cpu", True, True), "cuda")
+    view = tm._native.TrisProjView.from_buffer_copy(proj_view(payload))
+    count, steps = int(lib.tris_tile_record_count(C.byref(view))), view.max_sal_words
+    slots = min(4, -(-min(rank, 128) // group))
+    assert steps >= 2
+    for fewer_steps, fewer_slots in ((1, 0), (steps, 0), (0, min(1, slots - 1)), (steps, slots - 1)):
+        n, size = steps - fewer_steps, proj_view(payload).max_record_bytes - 4 * (128 * fewer_steps + 256 * fewer_slots)
+        columns = int(lib.tris_col_record_bytes(C.byref(view), n))
+        records, cols = (torch.full((b + 8192,), 0xA5, dtype=torch.uint8, device="cuda") for b in (count * size, columns))
+        view.max_record_bytes = size
+        tm._native.check(lib.tris_tile_records_build(C.byref(view), payload["_tris_tile_desc"].data_ptr(), records.data_ptr(), cols.data_ptr(), n,
+                                                     torch.cuda.current_stream().cuda_stream), "tile_records_build")
+        assert bool((records[count * size:] == 0xA5).all()) and bool((cols[columns:] == 0xA5).all())
+        # what does fit: the code words of every record are those of the whole plan
+        if fewer_slots == 0:
+            whole = payload["_tris_tile_records"][: count * (size + 512 * fewer_steps)].view(count, 4, -1)
+            assert torch.equal(records[: count * size].view(count, 4, -1)[:, :, : size // 4 - 256 * slots], whole[:, :, : size // 4 - 256 * slots])
+
+
+def test_paged_records_that_outgrow_their_plan_are_reported(lib):
+    """Column maps edited in place after the buffers were laid out: more salient columns than the records have room for."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging, synth
+
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=6, keep_sparse_gmap=True)
+    blk = tm.TrisSparseMoeBlock(256, 192, 8, 2, True)
+    blk.load_grouped_payloads(*(dict(layer[n], compact3_use_block_gr=False) for n in ("gate", "up", "down")), layer["shared_gate"], layer["shared_up"],
+                              layer["shared_down"], layer["router_weight"], device="cuda")
+    manager = staging.GroupedQGmapCPUStagingManager([blk])
+    manager.initialize()
+    x = synth.synth_activations(7, 256, seed=1).cuda().view(1, 7, 256)
+    blk.forward_streaming(x, manager, 0)
+    assert blk.last_kernel_status() == 0
+    blk._get_grouped_payload("down")["c_map"].fill_(-1)
+    blk.forward_streaming(x, manager, 0)
+    torch.cuda.synchronize()
+    assert blk.last_kernel_status() == 4  # TRIS_ERR_CORRUPT
