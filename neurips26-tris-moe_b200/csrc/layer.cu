@@ -167,6 +167,10 @@ static int validate_paged(const TrisMoeLayerView* L, const TrisPagedLayer* P) {
   for (int i = 0; i < 3; ++i)
     TRIS_REQUIRE(P->staged[i].num_experts == own[i]->num_experts && P->staged[i].out_features == own[i]->out_features && P->staged[i].rank == own[i]->rank,
                  TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: staged projection %d is not the layer's", i);
+  // a record's number is that of its segment, by which scales and biases are not indexed
+  for (int i = 0; i < 3 && P->records[0].tile_records; ++i)
+    TRIS_REQUIRE(!P->staged[i].output_scale && !P->staged[i].bias && !P->records[i].output_scale && !P->records[i].bias, TRIS_ERR_INVALID_ARG,
+                 "tris_moe_layer_forward_paged: projection %d has an output scale or a bias, which records cannot have", i);
   return TRIS_OK;
 }
 

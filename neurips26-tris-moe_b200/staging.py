@@ -153,6 +153,8 @@ class GroupedQGmapCPUStagingManager:
         self._consumed_epoch = []
         self._route_done = None
         self._record_info = {}     # (block index, projection) -> sizes of the tile records of its paged experts
+        self._record_keys = {}     # block index -> what they were planned for
+        self._record_bytes = 0     # of an expert, at most
         self._slot_ids = None
         self._layers = {}          # (layer, ring slot) -> what the native layer call takes: TrisPagedLayer and what it points at
 
@@ -215,33 +217,58 @@ class GroupedQGmapCPUStagingManager:
         self._initialized = True
         return True
 
+    @staticmethod
+    def _record_key(views):
+        """What the sizes of a layer's records, and whether it may have any, follow from."""
+        return tuple((v.num_experts, v.out_features, v.rank, v.num_groups, v.use_block_gr, v.gr_substreams, v.c_map, v.packed_row_group, v.output_scale,
+                      v.bias) for v in views)
+
+    def _plan_block(self, block_index: int) -> int:
+        """Sizes of the tile records of one expert of a layer; returns the bytes of them, gate and up or down.  0: none, the layer is
+        computed from the planes.  Waits for the GPU."""
+        lib = _native.load()
+        views = [proj_view(self.entries[(block_index, proj)].payload) for proj in PROJECTIONS]
+        self._record_keys[block_index] = self._record_key(views)
+        for proj in PROJECTIONS:
+            self._record_info.pop((block_index, proj), None)
+        # a record's place is that of its segment, which output scales and biases are not indexed by
+        if any(v.output_scale or v.bias or (v.use_block_gr and v.gr_substreams != 32) for v in views):
+            return 0
+        with torch.cuda.device(self.device):
+            stream = torch.cuda.current_stream(self.device).cuda_stream
+            info = torch.zeros((3, 4), dtype=torch.int64, device=self.device)
+            for i, v in enumerate(views):
+                _native.check(lib.tris_paged_records_plan(C.byref(v), info[i].data_ptr(), stream), "paged_records_plan")
+            for proj, v, (per, size, steps, _) in zip(PROJECTIONS, views, info.tolist()):
+                one = TrisProjView()
+                C.pointer(one)[0] = v
+                one.num_experts = 1
+                columns = int(lib.tris_col_record_bytes(C.byref(one), steps))
+                self._record_info[(block_index, proj)] = (per, size, steps, columns)
+        gate, up, down = (sum(self._record_info[(block_index, proj)][i] for i in (0, 3)) for proj in PROJECTIONS)
+        return max(gate + up, down)
+
     def _plan_records(self, experts: int, cap: int) -> None:
         """Buffers for the tile records of the experts of one layer, gate and up or down, per ring slot: the grouped kernels for records
         are about twice as fast as those that read the planes, and building records from paged planes takes a fraction of that."""
-        lib, most = _native.load(), 0
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream(self.device).cuda_stream
-            for bi in range(len(self.blocks)):
-                views = [proj_view(self.entries[(bi, proj)].payload) for proj in PROJECTIONS]
-                # a record's place is that of its segment, which output scales and biases are not indexed by
-                if any(v.output_scale or v.bias or (v.use_block_gr and v.gr_substreams != 32) for v in views):
-                    continue
-                info = torch.zeros((3, 4), dtype=torch.int64, device=self.device)
-                for i, v in enumerate(views):
-                    _native.check(lib.tris_paged_records_plan(C.byref(v), info[i].data_ptr(), stream), "paged_records_plan")
-                for proj, v, (per, size, steps, _) in zip(PROJECTIONS, views, info.tolist()):
-                    one = TrisProjView()
-                    C.pointer(one)[0] = v
-                    one.num_experts = 1
-                    columns = int(lib.tris_col_record_bytes(C.byref(one), steps))
-                    self._record_info[(bi, proj)] = (per, size, steps, columns)
-                gate, up, down = (sum(self._record_info[(bi, proj)][i] for i in (0, 3)) for proj in PROJECTIONS)
-                most = max(most, gate + up, down)
-            if most:
-                for ring in range(self.ring):
-                    self.buffers[(ring, "all", "tile_records")] = torch.empty((cap * most,), dtype=torch.uint8, device=self.device)
-                ids = torch.arange(max(experts, cap), dtype=torch.int32, device=self.device)
-                self._slot_ids = torch.where(ids < cap, ids, torch.full_like(ids, -1))
+        self._record_bytes = max(self._plan_block(bi) for bi in range(len(self.blocks)))
+        if self._record_bytes:
+            for ring in range(self.ring):
+                self.buffers[(ring, "all", "tile_records")] = torch.empty((cap * self._record_bytes,), dtype=torch.uint8, device=self.device)
+            ids = torch.arange(max(experts, cap), dtype=torch.int32, device=self.device)
+            self._slot_ids = torch.where(ids < cap, ids, torch.full_like(ids, -1))
+
+    def _has_records(self, block_index: int) -> bool:
+        """Whether a layer's experts become tile records: not with output scales or biases, which a view may have been given after the
+        buffers were laid out, and not where the records of the view's present tables would not fit the buffers."""
+        views = [proj_view(self.entries[(block_index, proj)].payload) for proj in PROJECTIONS]
+        if self._record_keys.get(block_index) != self._record_key(views):
+            if torch.cuda.is_current_stream_capturing():
+                return False  # planning waits for the GPU
+            if self._plan_block(block_index) > self._record_bytes:
+                for proj in PROJECTIONS:
+                    del self._record_info[(block_index, proj)]
+        return (block_index, "gate") in self._record_info
 
     # -- one layer ---------------------------------------------------------------------------
     def native_layer(self, block_index: int, rows: int, experts: int) -> TrisPagedLayer:
@@ -288,7 +315,7 @@ class GroupedQGmapCPUStagingManager:
             pages = (TrisPageLaunch * max(1, len(group)))(*group)
             keep.append(pages)
             arg.pages[g], arg.num_pages[g] = C.addressof(pages), len(group)
-        records = self.buffers.get((ring, "all", "tile_records")) if (block_index, "gate") in self._record_info else None
+        records = self.buffers.get((ring, "all", "tile_records")) if self._has_records(block_index) else None
         at = 0
         for i, proj in enumerate(PROJECTIONS):
             arg.staged[i] = views[proj]

@@ -233,3 +233,41 @@ def test_paged_records_that_outgrow_their_plan_are_reported(lib):
     blk.forward_streaming(x, manager, 0)
     torch.cuda.synchronize()
     assert blk.last_kernel_status() == 4  # TRIS_ERR_CORRUPT
+
+
+@pytest.mark.parametrize("name", ["output_scale", "bias"])
+@pytest.mark.parametrize("mode,sparse", [("bitmap", True), ("payload", False)])
+def test_a_scale_or_bias_given_after_initialisation_is_applied(lib, name, mode, sparse):
+    """The same bits as a block that had it from the start, whose slots are read as planes, and those of before once it is taken away."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging, synth
+    from trismoe_b200.qlinear_grouped import proj_view
+
+    layer = synth.synth_layer(synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32), seed=6, keep_sparse_gmap=True)
+    value = torch.linspace(0.5, 2.0, 8 * 256).view(8, 256).half()
+    x, logits = synth.synth_activations(7, 256, seed=1).cuda().view(1, 7, 256), synth.synth_router_logits(7, 8, seed=2).cuda()
+
+    def block(given):
+        blk = tm.TrisSparseMoeBlock(256, 192, 8, 2, True)
+        payloads = [{k: v.clone() if isinstance(v, torch.Tensor) else v for k, v in layer[n].items()} for n in ("gate", "up", "down")]
+        for p in payloads:
+            p["compact3_use_block_gr"] = not sparse
+        if given:
+            payloads[2].update({name: value.clone(), "has_" + name: True})
+        blk.load_grouped_payloads(*payloads, layer["shared_gate"], layer["shared_up"], layer["shared_down"], layer["router_weight"], device="cuda")
+        manager = staging.GroupedQGmapCPUStagingManager([blk], mode=mode)
+        manager.initialize()
+        return blk, manager, lambda: blk.forward_streaming(x, manager, 0, router_logits=logits)[0].clone()
+
+    want = block(True)[2]()
+    blk, manager, run = block(False)
+    plain = run()
+    dev_value = value.cuda()
+    view = proj_view(blk._get_grouped_payload("down"))
+    for _ in range(3):  # both ring places
+        setattr(view, name, dev_value.data_ptr())
+        assert torch.equal(run(), want)
+    for _ in range(3):
+        setattr(view, name, None)
+        assert torch.equal(run(), plain)
+    assert blk.last_kernel_status() == 0

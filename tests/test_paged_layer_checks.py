@@ -83,3 +83,16 @@ def test_staged_projections_with_missing_tensors_are_refused(lib, name):
     layer, paged = _layer(tm)
     setattr(paged.staged[2], name, None)
     assert _call(lib, layer, _with_records(paged)) == INVALID
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("name", ["output_scale", "bias"])
+@pytest.mark.parametrize("where", ["staged", "records"])
+def test_records_with_a_scale_or_a_bias_are_refused(lib, which, name, where):
+    """They would be read at a segment's number in place of its expert's."""
+    import trismoe_b200 as tm
+
+    layer, paged = _layer(tm)
+    _with_records(paged)
+    setattr(getattr(paged, where)[which], name, ADDRESS)
+    assert _call(lib, layer, paged) == INVALID and b"output scale or a bias" in lib.tris_last_error()
