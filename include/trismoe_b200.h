@@ -669,8 +669,8 @@ int tris_moe_layer_forward_shared(const TrisMoeLayerView* layer, const TrisShare
  * tile records in buffers that the call fills from the staged tensors, segment s at place s (num_experts = capacity, no
  * output scale or bias), so that the record kernels compute them; tile_records NULL in them: the plane kernels read the
  * staged tensors.  slot_ids: device array, i below capacity and -1 up to num_experts (with records).  Events are
- * cudaEvent_t that exist already: route, paged (one each for pages[0] and pages[1]), consumed; the pager waits for
- * `consumed` first where wait_consumed is set.  timing: NULL, or around the pages and around the two waits of the compute stream.
+ * cudaEvent_t that exist already: route, paged (one each for pages[0] and pages[1]), consumed; where wait_consumed is
+ * set, the pager and the builder of records wait for `consumed` first, whatever stream recorded it.  timing: NULL, or around the pages and around the two waits of the compute stream.
  * TRIS_ERR_WORKSPACE in status_dev: more experts than slots; their rows are stale.
  */
 typedef struct TrisPageLaunch {

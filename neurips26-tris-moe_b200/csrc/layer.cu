@@ -531,6 +531,8 @@ extern "C" int tris_moe_layer_forward_paged(const TrisMoeLayerView* layer, const
   auto ahead = [&](int g) -> int {  // records as far as they do not depend on the pages
     return records ? build_paged_records(paged->staged + 2 * g, paged->records + 2 * g, g == 0 ? 2 : 1, &route, paged->capacity, false, s) : static_cast<int>(TRIS_OK);
   };
+  // The builder writes the records of the ring's place, which a layer on another stream may still read.
+  if (records && paged->wait_consumed) TRIS_CUDA(cudaStreamWaitEvent(s, event(paged->event_consumed), 0));
   st = ahead(0);
   if (st == TRIS_OK) st = arrived(0);
   if (st != TRIS_OK) return st;

@@ -271,3 +271,34 @@ def test_a_scale_or_bias_given_after_initialisation_is_applied(lib, name, mode, 
         setattr(view, name, None)
         assert torch.equal(run(), plain)
     assert blk.last_kernel_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["bitmap", "payload"])
+def test_layers_on_different_streams_share_a_manager(lib, mode):
+    """Layers enqueued in turn on three streams with nothing but the manager's events between them: a place of the ring is written again
+    while its last reader, on another stream, may still run.  The same bits as one after the other on one stream."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging, synth
+
+    H, I, E, k = 512, 384, 32, 4
+    layer = synth.synth_layer(synth.LayerShape(H, I, E, k, rank=256, group_size=128), seed=9, keep_sparse_gmap=True)
+    blk = tm.TrisSparseMoeBlock(H, I, E, k, True)
+    payloads = [dict(layer[n], compact3_use_block_gr=mode == "payload") for n in ("gate", "up", "down")]
+    blk.load_grouped_payloads(*payloads, layer["shared_gate"], layer["shared_up"], layer["shared_down"], layer["router_weight"], device="cuda")
+    manager = staging.GroupedQGmapCPUStagingManager([blk], mode=mode)
+    manager.collect_timings = False
+    manager.initialize()
+    xs = [synth.synth_activations(T, H, seed=i).cuda().view(1, T, H) for i, T in enumerate((40, 3, 64, 1, 24, 17))]
+    logits = [synth.synth_router_logits(x.shape[1], E, seed=i).cuda() for i, x in enumerate(xs)]
+    want = []
+    for x, l in zip(xs, logits):
+        want.append(blk.forward_streaming(x, manager, 0, router_logits=l)[0].clone())
+        torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in range(3)], []
+    for i in range(60):
+        with torch.cuda.stream(streams[i % 3]):
+            got.append(blk.forward_streaming(xs[i % 6], manager, 0, router_logits=logits[i % 6])[0])
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 6]), i
+    assert blk.last_kernel_status() == 0

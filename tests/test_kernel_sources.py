@@ -48,3 +48,11 @@ def test_a_tmem_load_and_its_wait_are_one_statement():
                 loads += 1
                 assert "tcgen05.wait::ld" in text[text.rindex("tcgen05.ld."):], (os.path.basename(path), text[:90])
     assert loads >= 3
+
+
+def test_the_record_builder_of_a_streamed_layer_waits_for_the_last_use_of_its_place():
+    """The layer before may run on another stream, which only the event orders."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "layer.cu")).read())
+    body = text[text.index("int tris_moe_layer_forward_paged("):]
+    wait = re.search(r"cudaStreamWaitEvent\(s, event\(paged->event_consumed\)", body)
+    assert wait and wait.start() < body.index("ahead(0);"), "records are written before their last reader is done"
