@@ -460,11 +460,10 @@ class TrisSparseMoeBlock(nn.Module):
             if need == 0:
                 raise RuntimeError("trismoe_b200: invalid layer view (workspace size query failed)")
             ws = torch.empty((need,), dtype=torch.uint8, device=dev)
-            paged = manager.native_layer(block_index, T * self.top_k, E)
-            _native.check(lib.tris_moe_layer_forward_paged(C.byref(view), C.byref(paged), x.data_ptr(), logits_in, T, y.data_ptr(), logits_out,
-                                                           ws.data_ptr(), need, self._status_of(dev).data_ptr(),
-                                                           _native.stream_of(dev)), "moe_layer_forward_paged")
-            manager.end_layer()
+            status = self._status_of(dev).data_ptr()
+            with manager.native_layer(block_index, T * self.top_k, E) as paged:
+                _native.check(lib.tris_moe_layer_forward_paged(C.byref(view), C.byref(paged), x.data_ptr(), logits_in, T, y.data_ptr(), logits_out,
+                                                               ws.data_ptr(), need, status, _native.stream_of(dev)), "moe_layer_forward_paged")
         return y, logits
 
     def forward_grouped_ops(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None):

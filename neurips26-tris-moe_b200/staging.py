@@ -31,7 +31,9 @@ fraction ``1 - stall / copy``.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import threading
 from typing import Optional
 
 import torch
@@ -138,6 +140,7 @@ class GroupedQGmapCPUStagingManager:
         self._used = []
         self._copy_stream = None
         self._next = 0
+        self._lock = threading.RLock()
         self._initialized = False
         # bytes: at most, as if every slot of a launch were used and by the largest expert
         self.pipeline_stats = {"calls": 0, "chunks": 0, "bytes": 0, "slot_reuses": 0}
@@ -163,8 +166,10 @@ class GroupedQGmapCPUStagingManager:
         return sum(t.numel() * t.element_size() for t in self.buffers.values())
 
     def initialize(self) -> bool:
-        if self._initialized:
-            return True
+        with self._lock:  # of several threads' first calls one lays the buffers out
+            return self._initialized or self._initialize()
+
+    def _initialize(self) -> bool:
         if not self.blocks:
             return False
         keys = BITMAP_KEYS if self.mode == "bitmap" else PAYLOAD_KEYS
@@ -271,39 +276,38 @@ class GroupedQGmapCPUStagingManager:
         return (block_index, "gate") in self._record_info
 
     # -- one layer ---------------------------------------------------------------------------
-    def native_layer(self, block_index: int, rows: int, experts: int) -> TrisPagedLayer:
-        """The argument of ``tris_moe_layer_forward_paged`` for a layer that routes ``rows`` rows: takes a ring slot as
-        :meth:`page_layer` does.  Call :meth:`end_layer` after the launch."""
-        self.initialize()
-        ring = self._take_slot()
-        launches, views = self._plan(block_index, ring)
-        layer = self._layers.get((block_index, ring))
-        if layer is None or layer[0] is not launches:
-            layer = self._layers[(block_index, ring)] = (launches, *self._paged_layer(block_index, ring, launches, views))
-        arg = layer[1]
-        arg.wait_consumed = int(self._used[ring] and self._consumed_epoch[ring] == self._epoch)
-        self.pipeline_stats["slot_reuses"] += arg.wait_consumed
-        nseg_bound = min(experts, rows, self.capacity)
-        self.pipeline_stats["bytes"] += nseg_bound * sum(launch[3] for launch in launches)
-        self.pipeline_stats["chunks"] += len(launches)
-        self.pipeline_stats["calls"] += 1
-        if self.collect_timings:
-            compute = torch.cuda.current_stream(self.device)
-            events = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
-            for event in events:
-                event.record(compute)  # an event has its handle from then on; recorded again by the call
-            arg.timing[:] = [event.cuda_event for event in events]
-            begin, end, w0, w1, w2, w3 = events
-            self._timings += [(begin, end, w0, w1), (w2, w2, w2, w3)]
-        else:
-            arg.timing[:] = [None] * 6
-        return arg
-
-    def end_layer(self) -> None:
-        """The slot of the last :meth:`native_layer` is in use until its "consumed" event, which the call has recorded."""
-        ring = (self._next - 1) % self.ring
-        self._used[ring] = True
-        self._consumed_epoch[ring] = self._epoch
+    @contextlib.contextmanager
+    def native_layer(self, block_index: int, rows: int, experts: int):
+        """The argument of ``tris_moe_layer_forward_paged`` for a layer that routes ``rows`` rows, for the length of that call: takes a
+        ring slot as :meth:`page_layer` does, which is in use afterwards until its "consumed" event, recorded by the call.  Other
+        threads wait meanwhile: the argument, the events and the order of the copy stream are the manager's."""
+        with self._lock:
+            self.initialize()
+            ring = self._take_slot()
+            launches, views = self._plan(block_index, ring)
+            layer = self._layers.get((block_index, ring))
+            if layer is None or layer[0] is not launches:
+                layer = self._layers[(block_index, ring)] = (launches, *self._paged_layer(block_index, ring, launches, views))
+            arg = layer[1]
+            arg.wait_consumed = int(self._used[ring] and self._consumed_epoch[ring] == self._epoch)
+            self.pipeline_stats["slot_reuses"] += arg.wait_consumed
+            nseg_bound = min(experts, rows, self.capacity)
+            self.pipeline_stats["bytes"] += nseg_bound * sum(launch[3] for launch in launches)
+            self.pipeline_stats["chunks"] += len(launches)
+            self.pipeline_stats["calls"] += 1
+            if self.collect_timings:
+                compute = torch.cuda.current_stream(self.device)
+                events = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
+                for event in events:
+                    event.record(compute)  # an event has its handle from then on; recorded again by the call
+                arg.timing[:] = [event.cuda_event for event in events]
+                begin, end, w0, w1, w2, w3 = events
+                self._timings += [(begin, end, w0, w1), (w2, w2, w2, w3)]
+            else:
+                arg.timing[:] = [None] * 6
+            yield arg
+            self._used[ring] = True
+            self._consumed_epoch[ring] = self._epoch
 
     def _paged_layer(self, block_index: int, ring: int, launches, views):
         arg, keep = TrisPagedLayer(), []
@@ -336,13 +340,14 @@ class GroupedQGmapCPUStagingManager:
         return arg, keep
 
     def _take_slot(self) -> int:
-        ring = self._next
-        self._next = (self._next + 1) % self.ring
-        capturing = bool(torch.cuda.is_current_stream_capturing())
-        if capturing != self._capturing:
-            self._capturing = capturing
-            self._epoch += 1
-        return ring
+        with self._lock:
+            ring = self._next
+            self._next = (self._next + 1) % self.ring
+            capturing = bool(torch.cuda.is_current_stream_capturing())
+            if capturing != self._capturing:
+                self._capturing = capturing
+                self._epoch += 1
+            return ring
 
     def page_layer(self, block_index: int, route: dict):
         """Enqueues, on the side stream, the paging of gate/up/down of one layer for the

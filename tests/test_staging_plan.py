@@ -1,5 +1,7 @@
 """CPU tests of the pager plan of a layer: what it launches, and that a cached one follows the projections' own views."""
+import contextlib
 import ctypes as C
+import threading
 import types
 
 import pytest
@@ -71,3 +73,45 @@ def test_raw_and_coded_tensors_go_in_launches_of_their_own(coded):
             assert not kind or job.block_offsets == entry.coded["q_gmap_sparse"].data_ptr()
     for proj in staging.PROJECTIONS:
         assert views[proj].q_gmap_sparse == man.buffers[(0, proj, "q_gmap_sparse")].data_ptr() and views[proj].gmap_sparse_rows == 2
+
+
+def test_threads_that_stream_at_once_take_places_of_their_own(monkeypatch):
+    """The native call gives up the interpreter lock: a layer of another thread that comes in meanwhile changes nothing of the argument, and
+    each marks its own place of the ring as used."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import staging
+
+    man = _manager(tm, staging)
+    man._initialized, man.device, man.capacity, man.ring, man.collect_timings = True, torch.device("cpu"), 4, 2, False
+    man.slot_tables = man.slot_tables * 2
+    man.buffers.update({(1, proj, key): t for (_, proj, key), t in list(man.buffers.items())})
+    man._used, man._consumed_epoch = [False, False], [-1, -1]
+    man._paged_layer = lambda bi, ring, launches, views: (types.SimpleNamespace(ring=ring, wait_consumed=0, timing=[None] * 6), [])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(tm._native, "on_device", lambda dev: contextlib.nullcontext())
+    monkeypatch.setattr(tm._native, "stream_of", lambda dev: 0)
+    monkeypatch.setattr(C, "byref", lambda v: v)
+    calls, others, inside = [], [], threading.Event()
+
+    def forward_paged(view, paged, *rest):
+        seen = (paged.ring, paged.wait_consumed)
+        if not others:  # the first call: another thread's layer comes in before this one returns
+            others.append(threading.Thread(target=forward))
+            others[0].start()
+            inside.wait(0.5)  # runs out where the other one has to wait
+        else:
+            inside.set()
+        calls.append((seen, (paged.ring, paged.wait_consumed)))
+        return 0
+
+    lib = types.SimpleNamespace(tris_moe_layer_workspace_bytes=lambda view, tokens: 64, tris_moe_layer_forward_paged=forward_paged)
+    status = torch.zeros((1,), dtype=torch.int32)
+    blk = types.SimpleNamespace(num_experts=4, top_k=2, layer_view=lambda: None, _status_of=lambda dev: status)
+    x = torch.zeros((3, 8), dtype=torch.float16)
+    forward = lambda: tm.TrisSparseMoeBlock._forward_streaming_native(blk, lib, x, x.clone(), man, 0, torch.zeros((3, 4)))
+    forward()
+    others[0].join()
+    assert all(before == after for before, after in calls) and sorted(ring for (ring, _), _ in calls) == [0, 1]
+    assert man._used == [True, True] and man._consumed_epoch == [man._epoch] * 2
+    forward()
+    assert calls[-1][0] == (0, 1)  # waits for the last use of its place
