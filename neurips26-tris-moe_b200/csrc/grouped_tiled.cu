@@ -945,7 +945,7 @@ int launch_grouped_tiled(const TrisProjView* proj_a, const TrisProjView* proj_b,
   const uintptr_t rows_at = reinterpret_cast<uintptr_t>(a.hidden[0]) | reinterpret_cast<uintptr_t>(a.hidden[1]);
   a.hidden_vec = a.hidden_mode == TRIS_OUT_F16 && !a.col_scale && proj_a->rank % 8 == 0 && a.hidden_stride % 8 == 0 && (rows_at & 15u) == 0;
   a.hidden_perm = a.hidden_mode != TRIS_OUT_F16 && a.hidden_stride % 2 == 0 && (rows_at & 3u) == 0;
-  a.rows_ready = a.weights_before_wait && opts.rows_ready && a.hidden_vec;  // copies through L2; other rows may be in L1
+  a.rows_ready = a.weights_before_wait && opts.rows_ready;
   a.quad_store = proj_a->out_features % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 7u) == 0;
   a.vec_store = proj_a->out_features % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.out[0]) | reinterpret_cast<uintptr_t>(a.out[1])) & 15u) == 0;
   TRIS_REQUIRE(a.col_scale == nullptr || a.hidden_mode == TRIS_OUT_F16, TRIS_ERR_INVALID_ARG,

@@ -114,6 +114,35 @@ def test_qkv_in_one_call(lib, widths, K, rows):
             assert (y - ref).abs().max() <= 2.0**-10 * ref.abs().max()
 
 
+@pytest.mark.parametrize("rows", [1, 7, 32])
+@pytest.mark.parametrize("K,offset", [(1100, 0), (1096, 4), (1032, 1)])
+def test_qkv_of_rows_that_are_read_piece_by_piece(lib, K, offset, rows):
+    """Rows of a width or an address that 16-byte copies do not take are read ahead of the wait too: in calls with other rows in the same
+    memory, nothing between them, every result is that of the same call by itself."""
+    import trismoe_b200 as tm
+
+    rng = np.random.default_rng(K + rows)
+    made = [_single(rng, o, K) for o in (192, 128, 128)]
+    mods = [tm.Compact3Linear(p, device="cuda") for p, _ in made]
+    xs = [torch.from_numpy(rng.standard_normal((rows, K)).astype(np.float16)).cuda() for _ in range(4)]
+    memory = torch.zeros((rows * K + 8,), dtype=torch.float16, device="cuda")
+    x = memory[offset: offset + rows * K].view(rows, K)
+
+    def call(i):
+        x.copy_(xs[i])
+        return tm.run_compact3_qkv_forward(*mods, x)
+
+    want = []
+    for i in range(4):
+        want.append([y.clone() for y in call(i)])
+        torch.cuda.synchronize()
+        for y, (_, w) in zip(want[-1], made):
+            _check(y, xs[i].float().cpu().numpy() @ w.astype(np.float32).T)
+    got = [call(i % 4) for i in range(40)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, w) for i, ys in enumerate(got) for y, w in zip(ys, want[i % 4]))
+
+
 def test_qwen2_block_with_shared_expert(lib):
     """Qwen2-MoE style block: routed experts + an always-on shared expert (compact3 gate/up/down) scaled
     by sigmoid(shared_expert_gate(x)), against the fp32 oracle."""
