@@ -457,6 +457,50 @@ def test_null_space_and_input_scales_in_one_sequence(lib, T, pairs, scales):
     assert own.dtype == torch.float16 and own.shape == (T, E)
 
 
+@pytest.mark.parametrize("T", [1, 8, 32, 70, 300])
+@pytest.mark.parametrize("pairs,given", [("gate up down", True), ("gate up down", False), ("down", True), ("up", False)])
+def test_null_space_layers_back_to_back(lib, T, pairs, given):
+    """Products that start beside the launch ahead of them read rows, route and intermediate results before their wait: in calls with other
+    rows each, nothing between them, eager and replayed, every result is that of the same call by itself."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    rng = np.random.default_rng(17)
+    E, H, I = 16, 512, 256
+    layer = synth.synth_layer(synth.LayerShape(H, I, E, 4, rank=96, group_size=32), seed=5)
+    blk = tm.TrisSparseMoeBlock(H, I, E, 4, True)
+    blk.load_grouped_payloads(layer["gate"], layer["up"], layer["down"], layer["shared_gate"], layer["shared_up"], layer["shared_down"],
+                              layer["router_weight"], device="cuda")
+
+    def pair(n):
+        width, out = (I, H) if n == "down" else (H, I)
+        ex = [{"c2": synth.packed4_matrix(rng, r, width, 64, scale_std=0.02), "c1": synth.packed4_matrix(rng, out, r, 64, scale_std=0.02)}
+              for r in rng.choice([16, 32, 64], E)]
+        return tm.build_grouped_ns_compensation_payload(ex, "cuda", torch.float16, width, out)
+
+    blk.load_ns_compensation_payloads(*(pair(n) if n in pairs.split() else None for n in ("gate", "up", "down")))
+    xs = [synth.synth_activations(T, H, seed=10 * T + i).cuda().view(1, T, H) for i in range(4)]
+    logits = [synth.synth_router_logits(T, E, seed=20 * T + i).cuda() if given else None for i in range(4)]
+    want = []
+    for x, l in zip(xs, logits):
+        torch.cuda.synchronize()
+        want.append(blk(x, router_logits=l)[0].clone())
+        torch.cuda.synchronize()
+    assert not any(torch.equal(want[0], w) for w in want[1:])
+    got = [blk(x, router_logits=l)[0] for _ in range(8) for x, l in zip(xs, logits)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i % 4]) for i, y in enumerate(got))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = [blk(x, router_logits=l)[0] for x, l in zip(xs, logits)]
+    for _ in range(5):
+        for y in captured:
+            y.fill_(7.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for y, w in zip(captured, want))
+
+
 @pytest.mark.parametrize("T", [3, 37, 100])
 @pytest.mark.parametrize("packed", ["gate up down", "gate up", "down"])
 @pytest.mark.parametrize("pairs,scales", [("gate up down", "gate up down"), ("", "gate"), ("up", "up"), ("down", "gate up"), ("gate", "down"), ("gate up", "")])
@@ -499,10 +543,10 @@ def test_null_space_and_input_scales_with_4_bit_backbones(lib, T, packed, pairs,
 
 
 @pytest.mark.parametrize("E,k", [(8, 2), (40, 8), (72, 3), (200, 8)])
-@pytest.mark.parametrize("T", [1, 31, 32, 33, 65, 2100])
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 65, 128, 225, 255, 256, 257, 2100])
 def test_router_and_route_of_the_layer(lib, E, k, T):
-    """One launch up to 32 tokens, two above, runs of several 32-token groups per CTA above 2048; expert counts
-    on both sides of each lane count.  An identity-like layer would hide a wrong order, so whole outputs are compared."""
+    """One CTA up to 32 tokens, a cluster of up to eight to 256 (the last group ragged or full), two launches above, runs of several 32-token
+    groups per CTA above 2048; expert counts on both sides of each lane count.  An identity-like layer would hide a wrong order, so whole outputs are compared."""
     import trismoe_b200 as tm
     import trismoe_oracle as orc
     from trismoe_b200 import synth
