@@ -278,12 +278,14 @@ __global__ void __launch_bounds__(32 * kP4AddWarps) packed4_add_kernel(const __g
   const P4Problem& first = a.p[kSilu ? 0 : blockIdx.z];
   const int N0 = first.w.n_count ? first.w.n_count[e] : first.w.n, N1 = kSilu ? (a.p[1].w.n_count ? a.p[1].w.n_count[e] : a.p[1].w.n) : 0;
   if (n0 >= max(N0, N1)) return;
-  auto pass = [&](const P4Problem& pr, int N, int r0, uint2 (&sum)[2][NT]) {  // old outputs and the product, each four outputs of a row
+  // Old outputs and the product, each four outputs of a row.  Outputs from N on of the second problem keep what lies there: the first one's may
+  // be more.
+  auto pass = [&](const P4Problem& pr, int N, int all, int r0, uint2 (&sum)[2][NT]) {
     uint2 old[2][NT];
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int i = 0; i < NT; ++i) old[m][i] = load4(pr, N, r0 + 8 * i + g, n0 + 16 * m + 8 * (t & 1) + 2 * (t & 2));
+      for (int i = 0; i < NT; ++i) old[m][i] = load4(pr, all, r0 + 8 * i + g, n0 + 16 * m + 8 * (t & 1) + 2 * (t & 2));
     const bool present = pr.w.num_experts > 0 && n0 < N;
     float acc[2][NT][4] = {};
     if (present) product(pr, N, r0, acc);
@@ -291,7 +293,9 @@ __global__ void __launch_bounds__(32 * kP4AddWarps) packed4_add_kernel(const __g
     for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
-        const uint2 v = outputs_of_row(h2_as_u32(__floats2half2_rn(acc[m][i][0], acc[m][i][1])), h2_as_u32(__floats2half2_rn(acc[m][i][2], acc[m][i][3])), t);
+        uint2 v = outputs_of_row(h2_as_u32(__floats2half2_rn(acc[m][i][0], acc[m][i][1])), h2_as_u32(__floats2half2_rn(acc[m][i][2], acc[m][i][3])), t);
+        const int left = N - (n0 + 16 * m + 8 * (t & 1) + 2 * (t & 2));
+        if (kSilu && left < 4) v = make_uint2(left >= 2 ? v.x : (left == 1 ? v.x & 0xFFFFu : 0u), left == 3 ? v.y & 0xFFFFu : 0u);
         if (!a.accumulate) sum[m][i] = v;
         else sum[m][i] = !present ? old[m][i] : make_uint2(h2_as_u32(__hadd2_rn(u32_as_h2(old[m][i].x), u32_as_h2(v.x))), h2_as_u32(__hadd2_rn(u32_as_h2(old[m][i].y), u32_as_h2(v.y))));
       }
@@ -299,10 +303,10 @@ __global__ void __launch_bounds__(32 * kP4AddWarps) packed4_add_kernel(const __g
 #pragma unroll 1
   for (int r0 = 0; r0 < rows; r0 += 8 * NT) {
     uint2 y[2][NT];
-    pass(first, N0, r0, y);
+    pass(first, N0, N0, r0, y);
     if constexpr (kSilu) {
       uint2 up[2][NT];
-      pass(a.p[1], N1, r0, up);
+      pass(a.p[1], N1, max(N0, N1), r0, up);
       auto silu = [](uint32_t f, uint32_t u) {
         const float2 v = __half22float2(u32_as_h2(f));
         return h2_as_u32(__hmul2_rn(__floats2half2_rn(v.x / (1.f + expf(-v.x)), v.y / (1.f + expf(-v.y))), u32_as_h2(u)));

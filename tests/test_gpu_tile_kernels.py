@@ -457,6 +457,40 @@ def test_null_space_and_input_scales_in_one_sequence(lib, T, pairs, scales):
     assert own.dtype == torch.float16 and own.shape == (T, E)
 
 
+@pytest.mark.parametrize("T", [3, 40])
+@pytest.mark.parametrize("counts", [[192, 64, 37, 0, 130, 1, 95, 191]])
+def test_null_space_pair_of_up_with_fewer_outputs_than_gate(lib, T, counts):
+    """Outputs that up's pair does not reach are up's own, and SiLU(gate) * up is theirs as well: the bits of a pair whose scales are zero there."""
+    import trismoe_b200 as tm
+    from trismoe_b200 import synth
+
+    shape = synth.LayerShape(256, 192, 8, 2, rank=96, group_size=32)
+    layer = synth.synth_layer(shape, seed=3)
+    E, H, I = shape.num_experts, shape.hidden_size, shape.intermediate_size
+    x, logits = synth.synth_activations(T, H, seed=T).cuda().view(1, T, -1), synth.synth_router_logits(T, E, seed=T).cuda()
+    outs = []
+    for by_scales in (True, False):
+        rng = np.random.default_rng(19)
+        blk = tm.TrisSparseMoeBlock(H, I, E, shape.top_k, shape.norm_topk_prob)
+        blk.load_grouped_payloads(*({k: v.clone() if isinstance(v, torch.Tensor) else v for k, v in layer[n].items()} for n in ("gate", "up", "down")),
+                                  layer["shared_gate"], layer["shared_up"], layer["shared_down"], layer["router_weight"], device="cuda")
+        pairs = []
+        for which in range(2):
+            ex = [{"c2": synth.packed4_matrix(rng, 32, H, 64, scale_std=0.02), "c1": synth.packed4_matrix(rng, I, 32, 64, scale_std=0.02)} for _ in range(E)]
+            for e in range(E):
+                if which and by_scales:
+                    ex[e]["c1"]["scales"][..., counts[e]:] = 0
+            pairs.append(tm.build_grouped_ns_compensation_payload(ex, "cuda", torch.float16, H, I))
+        blk.load_ns_compensation_payloads(pairs[0], pairs[1], None)
+        blk._layer_extras(x.device)  # prepares the views
+        counts_dev = torch.tensor(counts, dtype=torch.int32, device="cuda")
+        if not by_scales:
+            pairs[1]["_tris_c1_view"].n_count = counts_dev.data_ptr()
+        outs.append(blk(x, router_logits=logits)[0])
+        torch.cuda.synchronize()
+    assert torch.equal(*outs) and outs[0].float().abs().max() > 1e-3
+
+
 @pytest.mark.parametrize("T", [1, 8, 32, 70, 300])
 @pytest.mark.parametrize("pairs,given", [("gate up down", True), ("gate up down", False), ("down", True), ("up", False)])
 def test_null_space_layers_back_to_back(lib, T, pairs, given):
