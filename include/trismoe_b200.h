@@ -164,8 +164,10 @@ const char* tris_last_error(void);
  * default; returns the previous value).  When on, every kernel these entry points launch may start
  * while its predecessor in the stream drains and waits (griddepcontrol.wait) before it touches what
  * the predecessor wrote - the launch gaps of a chain of small kernels (router, route, exchange,
- * grouped kernels, combine) overlap instead of adding up.  tris_moe_layer_forward always launches
- * this way.  No reference counterpart.
+ * grouped kernels, combine) overlap instead of adding up.  The layer entry points always launch
+ * this way, and so do the launches inside tris_qkv_forward.  With the switch on, backbone products of many rows
+ * take the larger tiles that a layer takes (their start is hidden then), which may add an fp32 sum up in another order.
+ * No reference counterpart.
  */
 int tris_set_programmatic_launch(int32_t enable);
 
@@ -479,20 +481,22 @@ int tris_combine_routed(const void* down_out_f16, const int32_t* row_of_flat,
                         int32_t hidden_size, void* final_f16, void* stream);
 
 /*
+ * The three projections of an attention block on the same rows x [num_rows, in], each an ordinary matrix with tile records: q, and
+ * k with v (one launch where their shapes agree, two where not), as tris_linear_forward computes them.  k and v do not wait for
+ * q's results: their launches start as q's ends, whatever tris_set_programmatic_launch says, as inside a layer; what
+ * follows the call is ordered as that switch says.  workspace (16-byte aligned): the largest of what tris_linear_workspace_bytes names
+ * for (q, 1) and for (k, 2), or (k, 1) and (v, 1) in two launches; NULL or fewer bytes: fewer parts of the columns.
+ */
+int tris_qkv_forward(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, const void* x_f16, int32_t num_rows,
+                     void* q_out_f16, void* k_out_f16, void* v_out_f16, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Rows per expert segment (the launch's upper estimate) above which projections without tile
  * records use their tcgen05/TMEM kernel instead of the register kernel; returns the previous value.  The
  * default (2048) lies above the range in which the register kernel measured faster on B200; the
  * tests lower it to exercise the tensor-core kernel.  Process-wide; no reference counterpart
  * (the reference decides per call in run_grouped_structured_expert_forward, QL:2187-2229).
  */
-/*
- * The three projections of an attention block on the same rows x [num_rows, in], each an ordinary matrix with tile records: q, and
- * k with v (one launch where their shapes agree), as tris_linear_forward computes them.  k and v do not wait for q's
- * results: their launches start as q's ends.  workspace: as many bytes as tris_linear_workspace_bytes names for (q, 1) or (k, 2), or NULL.
- */
-int tris_qkv_forward(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, const void* x_f16, int32_t num_rows,
-                     void* q_out_f16, void* k_out_f16, void* v_out_f16, void* workspace, size_t workspace_bytes, void* stream);
-
 int tris_set_grouped_tc_min_rows(int32_t rows);
 
 /*
@@ -609,7 +613,8 @@ int tris_moe_layer_last_status(void* workspace, int32_t clear, void* stream, int
  * stream-ordered launch sequence with no host synchronisation: router (from router_logits
  * [T, E] fp32 when given, else x . router_weight^T), route, both input-side backbones,
  * grouped gate/up with SiLU*mul, down backbone, grouped down, weighted combine.
- * x, y: [T, H] fp16.  router_logits_out (optional) receives the fp32 logits.
+ * x, y: [T, H] fp16, y 16-byte aligned and H a multiple of 8 here and in every other form of the layer.
+ * router_logits_out (optional) receives the fp32 logits.
  */
 int tris_moe_layer_forward(const TrisMoeLayerView* layer, const void* x_f16,
                            const float* router_logits, int32_t num_tokens, void* y_f16,
@@ -645,8 +650,8 @@ int tris_moe_layer_forward_extras_status(const TrisMoeLayerView* layer, const Tr
  * The same launch sequence with one always-on shared expert, the dense MLP of Qwen2-MoE blocks: gate and up [I_s, H] and down
  * [H, I_s] are ordinary compact3 matrices with tile records, joined as tris_shared_expert_add does it
  * (modeling_qwen2_moe.py:815-818).  The workspace holds the expert's rows too
- * (tris_moe_layer_shared_workspace_bytes); scratch: as for tris_linear_forward, as many bytes as
- * tris_linear_workspace_bytes names for either launch, or NULL; not used after the call's last kernel.
+ * (tris_moe_layer_shared_workspace_bytes); scratch (16-byte aligned): as for tris_linear_forward, the larger of what
+ * tris_linear_workspace_bytes names for (gate, 2) and (down, 1), or NULL; not used after the call's last kernel.
  */
 typedef struct TrisSharedExpert {
   const TrisProjView* gate;

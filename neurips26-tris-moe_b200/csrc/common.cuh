@@ -10,6 +10,9 @@
 static_assert(sizeof(TrisProjView) == 224, "TrisProjView layout is part of the ABI");
 static_assert(sizeof(TrisPacked4View) == 112, "TrisPacked4View layout changed: update the ctypes mirror");
 static_assert(sizeof(TrisRouteView) == 80, "TrisRouteView layout is part of the ABI");
+static_assert(sizeof(TrisSharedExpert) == 32, "TrisSharedExpert layout is part of the ABI");
+static_assert(sizeof(TrisPageLaunch) == 24, "TrisPageLaunch layout is part of the ABI");
+static_assert(sizeof(TrisPagedLayer) == 1472, "TrisPagedLayer layout is part of the ABI");
 
 namespace tris {
 
@@ -204,8 +207,9 @@ __device__ __forceinline__ bool elect_one() {
 
 // Programmatic dependent launch: wait for the producer grid's memory to be visible /
 // let the dependent grid start its prologue.
-// What is read ahead of the wait was written by kernels that had ended when this one started (the kernel before waited before it let
-// this one start), at addresses that every layer writes again.  Plain loads are right there: L1 keeps no line of an earlier grid.  Six chains of a grid
+// What is read ahead of the wait was written by kernels that had ended when this one started, at addresses that every layer writes again.
+// (A kernel lets its successor start after its own wait.  One with rows_ready does so before; what its successor reads early is no younger
+// than the rows it has read early itself.)  Plain loads are right there: L1 keeps no line of an earlier grid.  Six chains of a grid
 // that reads 16 KB on all SMs, one that rewrites them on one SM, one or two that still run, and one that reads them ahead of its wait: of 71 M CTAs
 // x 4096 words none was old, where inside one grid all of them were.  Loads by way of L2 for all of it (ld.global.cg, kept in their place)
 // cost 1 to 7 % (attention projections of 512 rows 69.8 -> 75.1 us, blocks of 2048 tokens 151 -> 159).

@@ -154,6 +154,13 @@ static int validate_shared(const TrisMoeLayerView* L, const TrisSharedExpert* S)
   return TRIS_OK;
 }
 
+// The last kernel of a layer stores 16 bytes at a time.
+static int validate_output(const TrisMoeLayerView* L, const void* y) {
+  TRIS_REQUIRE((L->hidden_size & 7) == 0, TRIS_ERR_UNSUPPORTED, "moe layer: hidden_size must be a multiple of 8");
+  TRIS_REQUIRE((reinterpret_cast<uintptr_t>(y) & 15u) == 0, TRIS_ERR_INVALID_ARG, "moe layer: y must be 16-byte aligned");
+  return TRIS_OK;
+}
+
 // The staged projections of a streamed layer: what the grouped entry points ask of them, here before anything is launched, since the record
 // kernels are launched without those entry points.
 static int validate_paged(const TrisMoeLayerView* L, const TrisPagedLayer* P) {
@@ -214,6 +221,8 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
   TRIS_REQUIRE(router_logits || layer->router_weight, TRIS_ERR_INVALID_ARG,
                "tris_moe_layer_forward: need router_logits or a router weight");
   if (num_tokens == 0) return TRIS_OK;
+  st = validate_output(layer, y_f16);
+  if (st != TRIS_OK) return st;
   const int T = num_tokens;
   TRIS_REQUIRE(workspace != nullptr, TRIS_ERR_WORKSPACE, "tris_moe_layer_forward: null workspace");
   LayerWorkspace w = carve(layer, T, static_cast<char*>(workspace), extras, shared.expert);
@@ -457,6 +466,7 @@ extern "C" int tris_moe_layer_forward_paged(const TrisMoeLayerView* layer, const
   TRIS_REQUIRE(!records || paged->slot_ids, TRIS_ERR_INVALID_ARG, "tris_moe_layer_forward_paged: records need slot_ids");
   if (num_tokens == 0) return TRIS_OK;
   st = validate_paged(layer, paged);
+  if (st == TRIS_OK) st = validate_output(layer, y_f16);
   if (st != TRIS_OK) return st;
   const int T = num_tokens, E = layer->num_experts, R = T * layer->top_k;
   LayerWorkspace w = carve(layer, T, static_cast<char*>(workspace));

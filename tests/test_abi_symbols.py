@@ -52,6 +52,10 @@ def test_struct_sizes_match_c_layout(lib):
     assert C.sizeof(tm._native.TrisPacked4View) == 112
     assert tm._native.TrisRouteView.row_gather.offset == 40
     assert tm._native.TrisRouteView.out_row_scatter.offset == 64
+    assert C.sizeof(tm._native.TrisSharedExpert) == 32
+    assert C.sizeof(tm._native.TrisPageLaunch) == 24
+    assert C.sizeof(tm._native.TrisPagedLayer) == 1472
+    assert tm._native.TrisPagedLayer.staged.offset == 24 and tm._native.TrisPagedLayer.timing.offset == 1424
 
 
 def test_cpu_tensors_are_rejected_loudly(lib):
@@ -96,3 +100,28 @@ def test_misaligned_workspace_of_an_ordinary_matrix_is_refused(lib):
     assert need > 0
     st = lib.tris_linear_forward(C.byref(view), None, C.byref(route), 4096, None, 8192, None, 0, 16388, need, None)
     assert st == 1 and b"16-byte aligned" in lib.tris_last_error()
+
+
+def test_outputs_that_the_combine_cannot_store_are_refused(lib):
+    """Rows of y are stored 16 bytes at a time.  Refused before any CUDA call by every form of the layer."""
+    import trismoe_b200 as tm
+
+    def layer(H):
+        v = tm._native.TrisMoeLayerView()
+        v.hidden_size, v.intermediate_size, v.num_experts, v.top_k = H, 96, 1, 1
+        v.gate, v.up, v.down = _record_view(96, 64), _record_view(96, 64), _record_view(H, 64)
+        for name in ("router_weight", "shared_gate", "shared_up", "shared_down"):
+            setattr(v, name, 1 << 20)
+        return v
+
+    def shared(H):
+        views = [_record_view(32, H), _record_view(32, H), _record_view(H, 32)]
+        return tm._native.TrisSharedExpert(*(C.addressof(v) for v in views), 1 << 20), views
+
+    for H, y, status in ((64, (1 << 20) + 8, 1), (100, 1 << 20, 2)):
+        view, (expert, keep) = layer(H), shared(H)
+        calls = [lambda: lib.tris_moe_layer_forward(C.byref(view), 1 << 20, None, 3, y, None, 1 << 20, 1 << 30, None),
+                 lambda: lib.tris_moe_layer_forward_extras(C.byref(view), C.byref(tm._native.TrisMoeLayerExtras()), 1 << 20, None, 3, y, None, 1 << 20, 1 << 30, None),
+                 lambda: lib.tris_moe_layer_forward_shared(C.byref(view), C.byref(expert), 1 << 20, None, 3, y, None, 1 << 20, 1 << 30, None, 0, None)]
+        for call in calls:
+            assert call() == status and (b"aligned" if status == 1 else b"multiple of 8") in lib.tris_last_error()
