@@ -484,9 +484,10 @@ int tris_combine_routed(const void* down_out_f16, const int32_t* row_of_flat,
  * The three projections of an attention block on the same rows x [num_rows, in], each an ordinary matrix with tile records: q, and
  * k with v (one launch where their shapes agree, two where not), as tris_linear_forward computes them.  k and v do not wait for
  * q's results: their launches start as q's ends, whatever tris_set_programmatic_launch says, as inside a layer; what
- * follows the call is ordered as that switch says.  workspace (16-byte aligned): the largest of what tris_linear_workspace_bytes names
- * for (q, 1) and for (k, 2), or (k, 1) and (v, 1) in two launches; NULL or fewer bytes: fewer parts of the columns.
+ * follows the call is ordered as that switch says.  workspace (16-byte aligned): tris_qkv_workspace_bytes, the largest of what
+ * tris_linear_workspace_bytes names for the launches; NULL or fewer bytes: fewer parts of the columns.
  */
+size_t tris_qkv_workspace_bytes(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, int32_t num_rows);
 int tris_qkv_forward(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, const void* x_f16, int32_t num_rows,
                      void* q_out_f16, void* k_out_f16, void* v_out_f16, void* workspace, size_t workspace_bytes, void* stream);
 

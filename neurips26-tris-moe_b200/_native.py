@@ -136,6 +136,7 @@ SIGNATURES = {
     "tris_grouped_pair_forward": (C.c_int, [_P(TrisProjView), _P(TrisProjView), _P(TrisRouteView), _vp, _vp, _vp, _vp, _i32, _vp]),
     "tris_linear_workspace_bytes": (C.c_size_t, [_P(TrisProjView), _i32, _i32]),
     "tris_linear_forward": (C.c_int, [_P(TrisProjView), _P(TrisProjView), _P(TrisRouteView), _vp, _vp, _vp, _vp, _i32, _vp, C.c_size_t, _vp]),
+    "tris_qkv_workspace_bytes": (C.c_size_t, [_P(TrisProjView), _P(TrisProjView), _P(TrisProjView), _i32]),
     "tris_qkv_forward": (C.c_int, [_P(TrisProjView), _P(TrisProjView), _P(TrisProjView), _vp, _i32, _vp, _vp, _vp, _vp, C.c_size_t, _vp]),
     "tris_grouped_hidden_layout": (C.c_int, [_P(TrisProjView), _P(TrisProjView), _i32, _i32, _i32]),
     "tris_set_grouped_tc_min_rows": (C.c_int, [_i32]),

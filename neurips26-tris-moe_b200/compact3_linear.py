@@ -13,7 +13,6 @@ matrix ``[out_features, in_features]`` (the columns are the layer's input featur
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import Optional
 
 import torch
@@ -99,11 +98,11 @@ def run_compact3_qkv_forward(q_proj: Compact3Linear, k_proj: Compact3Linear, v_p
         # the leading dimensions at once; no reshape afterwards
         outs = [torch.empty(lead + (m.out_features,), dtype=torch.float16, device=dev) for m in mods]
         if rows:
-            pair = 2 if _same_shape(k_proj, v_proj) else 1
-            need = 0 if rows <= 32 else max(int(lib.tris_linear_workspace_bytes(C.byref(v), n, rows)) for v, n in zip(views, (1, pair, pair)))
+            # nothing runs on the GPU until the call, so one query for all launches: three took 3 us more before the first of them
+            need = int(lib.tris_qkv_workspace_bytes(*views, rows)) if rows > 32 else 0
             with _native.on_device(dev):
                 ws = torch.empty((need,), dtype=torch.uint8, device=dev) if need else None
-                _native.check(lib.tris_qkv_forward(*(C.byref(v) for v in views), x2.data_ptr(), rows, *(o.data_ptr() for o in outs),
+                _native.check(lib.tris_qkv_forward(*views, x2.data_ptr(), rows, *(o.data_ptr() for o in outs),
                                                    None if ws is None else ws.data_ptr(), need, _native.stream_of(dev)), "qkv_forward")
         return tuple(outs)
     q = run_grouped_structured_expert_forward(q_proj.payload, x2, None, q_proj._route(rows, x2.device))

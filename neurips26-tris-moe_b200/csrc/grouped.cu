@@ -705,6 +705,12 @@ extern "C" int tris_linear_forward(const TrisProjView* proj_a, const TrisProjVie
   return grouped_pair_forward_impl(proj_a, proj_b, route, hidden_a_f16, hidden_b_f16, out_a_f16, out_b_f16, fuse_silu_mul, s, opts);
 }
 
+extern "C" size_t tris_qkv_workspace_bytes(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, int32_t num_rows) {
+  if (!q || !k || !v || num_rows <= 0) return 0;
+  const bool pair = k->out_features == v->out_features;
+  return std::max({grouped_split_bytes(q, 1, num_rows), grouped_split_bytes(k, pair ? 2 : 1, num_rows), pair ? size_t{0} : grouped_split_bytes(v, 1, num_rows)});
+}
+
 extern "C" int tris_qkv_forward(const TrisProjView* q, const TrisProjView* k, const TrisProjView* v, const void* x_f16, int32_t num_rows,
                                 void* q_out_f16, void* k_out_f16, void* v_out_f16, void* workspace, size_t workspace_bytes, void* stream) {
   TRIS_REQUIRE(q && k && v && x_f16 && q_out_f16 && k_out_f16 && v_out_f16, TRIS_ERR_INVALID_ARG, "tris_qkv_forward: null pointer");

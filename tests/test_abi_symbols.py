@@ -90,6 +90,16 @@ def test_column_split_scratch_is_bounded(lib):
             assert n <= 256 << 20 and n % (4 * projections * rows * o) == 0
 
 
+def test_scratch_of_attention_projections_is_that_of_the_largest_launch(lib):
+    one = lambda view, n, rows: lib.tris_linear_workspace_bytes(C.byref(view), n, rows)
+    for widths, rank in (((4096, 1024, 1024), 4096), ((256, 1024, 1024), 2048), ((512, 256, 4096), 2048), ((2048, 128, 64), 4096)):
+        q, k, v = (_record_view(w, rank) for w in widths)
+        for rows in (1, 32, 33, 100, 512, 3000):
+            launches = [(q, 1), (k, 2)] if widths[1] == widths[2] else [(q, 1), (k, 1), (v, 1)]
+            want = max(one(view, n, rows) for view, n in launches)
+            assert lib.tris_qkv_workspace_bytes(q, k, v, rows) == want and (want > 0) == (rows > 32)
+
+
 def test_misaligned_workspace_of_an_ordinary_matrix_is_refused(lib):
     """The sums of the column parts are read 16 bytes at a time.  Refused before any CUDA call, so no GPU is needed."""
     import trismoe_b200 as tm
