@@ -164,10 +164,12 @@ __device__ __forceinline__ uint32_t stream_bits(const uint32_t* words, int rows,
 // tables, planes): in the order of use they took turns with the stores, which may alias them for all the compiler knows.  us for 102 experts
 // of 2048 x 256: 25 in that order, 30 with four outputs to a lane (fewer instructions, too few warps), 24 in this one.
 // In two phases, where only the bitmap is paged: what does not need it while it is still on its way, and then only its bits.
+// The first phase is compiled for six CTAs to an SM: for seven the compiler takes 72 registers and spills some, for six it takes 64 without, and
+// eight fit.  Two streamed layers of 102 experts, 16 tokens: 372.8 / 366 us called from Python, 349 / 346 replayed as a graph.
 enum { BUILD_ALL = 0, BUILD_BASE = 1, BUILD_BITS = 2 };
 constexpr int kBuildWarps = 4, kBuildRows = 2 * kChunkRows;  // packed rows of an item
 template <int PHASE>
-__global__ void __launch_bounds__(32 * kBuildWarps, 7) build_tile_records_kernel(const __grid_constant__ BuildArgs args) {
+__global__ void __launch_bounds__(32 * kBuildWarps, PHASE == BUILD_BASE ? 6 : 7) build_tile_records_kernel(const __grid_constant__ BuildArgs args) {
   __shared__ uint16_t col_of[kBuildWarps][kMaxSteps * 16];
   __shared__ uint32_t stream[kBuildWarps][TRIS_GR_BLOCK_WORDS + 4];    // a block-GR block, with read slack
   __shared__ uint32_t plane[2][4][TRIS_GR_BLOCK_WORDS];                // decoded: [chunk][k block * 2 + out block][row parity][64]
