@@ -9,8 +9,8 @@
 // outputs its pair corrects, each C1 after it; of gate and up in one launch each, SiLU*mul in the epilogue of the second.
 // A shared expert's (TrisSharedExpert) gate/up launch follows the route and its down launch the down backbone.  Both read rows that are older
 // than the kernel before them and, at a few rows, wait only before they store: they run beside the route's one CTA and the down
-// backbone's few.  256 experts of 512, 16 tokens, a call of the whole layer: 121 us with the two linears and the sum as operators of their
-// own, 64 here (GPU 87 / 52 us).
+// backbone's few.  256 experts of 512, 16 tokens, the whole layer with the two linears and the sum as operators of their own / here:
+// replayed as a graph 67.5 / 47.8 us, called from Python, where the host bounds it, 119 / 51.
 #include <algorithm>
 #include <mutex>
 
@@ -354,7 +354,7 @@ static int layer_forward(const TrisMoeLayerView* layer, const TrisMoeLayerExtras
   if (st != TRIS_OK) return st;
   if (ns_gu) {
     // C2 reads x and the route, which are older than the kernel before it: it fills the SMs that the grouped kernel leaves (37 tokens of 64
-    // experts: 82.5 us for the block, 87 with C2 launches ahead of the grouped ones)
+    // experts, the block replayed as a graph: 83 us, 87 with C2 launches ahead of the grouped ones)
     st = packed4_gemm_impl(c2, n2, &route, R, TRIS_OUT_F16, false, false, s, true, /*rows_ready=*/true);
     if (st != TRIS_OK) return st;
     TrisRouteView rows = route;
@@ -449,8 +449,8 @@ extern "C" int tris_moe_layer_forward_shared(const TrisMoeLayerView* layer, cons
 // Two streams: the pages cross the host link on one while the other computes what it has.  The router runs before the backbones, since the
 // pages wait for its route; the backbones run beside them.  Paged experts become tile records, all but the paged bits of them while the
 // pages are on their way: with those bits put in, 8 and 12 us, and the kernels for records, 11 and 15, gate/up and down of 102 experts of 512 x 256
-// (twice) and 2048 x 256 take half of what the kernels for planes did (45 each, 78 beside a pager).  Two such layers, 16 tokens:
-// 416 us with planes and seven calls a layer from Python, 360 here; 1 token 271 / 171.
+// (twice) and 2048 x 256 take half of what the kernels for planes did (45 each, 78 beside a pager).  Two such layers with planes and seven calls
+// a layer from Python / here: replayed as a graph, 16 tokens 402 / 356 us, 1 token 121 / 104; called from Python, 16 tokens 433 / 371.
 extern "C" int tris_moe_layer_forward_paged(const TrisMoeLayerView* layer, const TrisPagedLayer* paged, const void* x_f16, const float* router_logits,
                                             int32_t num_tokens, void* y_f16, float* router_logits_out, void* workspace, size_t workspace_bytes,
                                             int32_t* status_dev, void* stream) {

@@ -19,8 +19,8 @@
 // 8 columns of each, A fragments of two K = 16 steps if step j's K positions are columns 8t + 4j .. + 3;
 // the lane's activations of the slice are then 16 contiguous bytes.  Nibbles and activations are read
 // straight from global memory (L2 / L1) and nothing is staged; four CTAs on an SM hide the latency
-// better than loads four slices ahead in 125 registers (a whole block with null-space pairs, 37 tokens, when C1 took this kernel too:
-// 128 against 148 us).  Staging 32 KB of nibbles and up to 128 KB of activation rows per CTA whatever the
+// better than loads four slices ahead in 125 registers (a whole block with null-space pairs, 37 tokens, called from Python, when C1
+// took this kernel too: 128 against 148 us).  Staging 32 KB of nibbles and up to 128 KB of activation rows per CTA whatever the
 // problem's size let one CTA fill an SM: 64 segments of 5 rows, 2048 -> 64 and 64 -> 1024, took 42 us a
 // launch.  Gate and up share a launch.
 // The eight warps of a CTA split the columns as far as there are slices and take further groups of 16 outputs
@@ -390,7 +390,7 @@ int packed4_gemm_impl(const P4Problem* problems, int num_problems, const TrisRou
   args.rows_ready = pdl && rows_ready;
   const int slices = ceil_div(k, kP4SliceCols);
   // Few columns of many segments (C1 of null-space pairs): a warp per 32 outputs.  64 segments, 37 tokens, pairs of rank 32 and 64, a block
-  // with them on the kernel below / on this one 107 / 87 us, 512 tokens 350 / 208, 1 token 45.9 / 46.4.
+  // with them, replayed as a graph, on the kernel below / on this one 107 / 87 us, 512 tokens 350 / 208, 1 token 45.9 / 46.4.
   TRIS_REQUIRE(args.num_segments <= 65535, TRIS_ERR_UNSUPPORTED, "tris_packed4_grouped_forward: more than 65535 segments");
   if (silu) return dispatch_add<true>(args, hint, stream, pdl);
   if (route && out_mode == TRIS_OUT_F16 && slices <= 4) return dispatch_add<false>(args, hint, stream, pdl);
